@@ -100,8 +100,7 @@ static_assert(sizeof(SmemCtl) <= kCtlBytes, "control block too large");
 struct RoleState {
   uint32_t slot = 0;       // next ring slot
   uint32_t slot_bits = 0;  // phase bit per ring slot
-  uint32_t acc = 0;        // next accumulator buffer
-  uint32_t acc_bits = 0;   // phase bit per accumulator buffer
+  uint32_t acc_bits = 0;   // bits 0, 1: phase bit per accumulator buffer; bit 2: next accumulator buffer
   uint32_t attn_bit = 0;   // phase bit of the attention barriers, pipeline 0
   uint32_t attn_bit1 = 0;  // phase bit of the attention barriers, pipeline 1
   uint32_t ln_bits = 0;    // phase bit per LayerNorm batch buffer
@@ -169,6 +168,9 @@ __device__ bool grid_barrier(const MegaParams& p, const WaitCtl& ctl, int where,
   fence_proxy_async_smem();       // this thread's accesses to shared memory before the next stage's copies into it
   return *ctl.abort_smem == 0;
 }
+
+// The warp's index as a value the compiler knows to be the same in all its lanes (see elect_one).
+__device__ __forceinline__ int uniform_warp(int warp) { return __shfl_sync(0xffffffffu, warp, 0); }
 
 // ------------------------------------------------------------------------------------
 // GEMM stage
@@ -243,23 +245,28 @@ __device__ __forceinline__ void staged_store_64B(uint8_t* sbuf, const uint32_t (
 
 // Swin row maps.  Tokens of an R x R grid are rolled by -shift and cut into (R/win)^2 windows of win*win
 // tokens; the window-major buffers give every window 64 row slots (49 used for win = 7).
+// The divisors are host constants of the stage, so a quotient is one multiply-high (fast_div): with plain divisions,
+// evaluated for five rows per thread, the epilogue of a 128 x 32 tile took 9.5 k cycles, now 2.2 k.
 // token row (b*R*R + ty*R + tx)  ->  window-major row (global window)*64 + position
-__device__ __forceinline__ int swin_token_to_slot(int row, int R, int win, int shift) {
-  const int img = row / (R * R), t = row - img * R * R;
-  const int ty = t / R, tx = t - ty * R;
+__device__ __forceinline__ int swin_token_to_slot(const Stage& st, int row) {
+  const int R = st.seq, win = st.win, shift = st.shift, nwr = st.nwr;
+  const int img = st.mg_seq2 ? (int)__umulhi((uint32_t)row, st.mg_seq2) : row / (R * R), t = row - img * R * R;
+  const int ty = (int)fast_div((uint32_t)t, (uint32_t)R, st.mg_seq), tx = t - ty * R;
   int sy = ty - shift, sx = tx - shift;
   if (sy < 0) sy += R;
   if (sx < 0) sx += R;
-  const int nwr = R / win;
-  const int w = (sy / win) * nwr + sx / win, pos = (sy % win) * win + sx % win;
-  return (img * nwr * nwr + w) * 64 + pos;
+  const int wy = (int)fast_div((uint32_t)sy, (uint32_t)win, st.mg_win), wx = (int)fast_div((uint32_t)sx, (uint32_t)win, st.mg_win);
+  return (img * nwr * nwr + wy * nwr + wx) * 64 + (sy - wy * win) * win + (sx - wx * win);
 }
 // window-major row -> token row, or -1 for a padding slot
-__device__ __forceinline__ int swin_slot_to_token(int slot, int R, int win, int shift, int n_windows) {
+__device__ __forceinline__ int swin_slot_to_token(const Stage& st, int slot, int n_windows) {
+  const int R = st.seq, win = st.win, shift = st.shift, nwr = st.nwr;
   const int wg = slot >> 6, pos = slot & 63;
   if (pos >= win * win || wg >= n_windows) return -1;
-  const int nwr = R / win, img = wg / (nwr * nwr), w = wg - img * nwr * nwr;
-  int ty = (w / nwr) * win + pos / win + shift, tx = (w % nwr) * win + pos % win + shift;
+  const int img = (int)fast_div((uint32_t)wg, (uint32_t)(nwr * nwr), st.mg_nwr2), w = wg - img * nwr * nwr;
+  const int wy = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr), wx = w - wy * nwr;
+  const int py = (int)fast_div((uint32_t)pos, (uint32_t)win, st.mg_win), px = pos - py * win;
+  int ty = wy * win + py + shift, tx = wx * win + px + shift;
   if (ty >= R) ty -= R;
   if (tx >= R) tx -= R;
   return img * R * R + ty * R + tx;
@@ -279,9 +286,9 @@ __device__ __forceinline__ uint32_t epi_row_offset(const Stage& st, const EpiCtx
     return (b * (uint32_t)(st.heads * st.seq) + sq) * (uint32_t)st.head_dim;
   }
   if constexpr (kSwin) {
-    if (e.epi == EPI_SWIN_QKV) return (uint32_t)swin_token_to_slot(row, st.seq, st.win, st.shift) * (uint32_t)e.ldo;
+    if (e.epi == EPI_SWIN_QKV) return (uint32_t)swin_token_to_slot(st, row) * (uint32_t)e.ldo;
     if (e.epi == EPI_SWIN_PROJ) {
-      const int t = swin_slot_to_token(row, st.seq, st.win, st.shift, e.M >> 6);
+      const int t = swin_slot_to_token(st, row, e.M >> 6);
       return t >= 0 ? (uint32_t)t * (uint32_t)e.ldo : kNoRow;
     }
   }
@@ -299,9 +306,8 @@ __device__ __forceinline__ uint32_t epi_col_offset(const Stage& st, const EpiCtx
   if constexpr (kSwin) {
     if (e.epi == EPI_SWIN_QKV) {
       // [3][windows][64][C]: the column picks q/k/v and the channel
-      const int which = col / e.ldo, ch = col - which * e.ldo;
-      const uint32_t plane = (uint32_t)((e.M + st.seq * st.seq - 1) / (st.seq * st.seq)) * (uint32_t)((st.seq / st.win) * (st.seq / st.win) * 64) * (uint32_t)e.ldo;
-      return (uint32_t)which * plane + (uint32_t)ch;
+      const int which = (col >= e.ldo) + (col >= 2 * e.ldo), ch = col - which * e.ldo;
+      return (uint32_t)which * st.plane_elems + (uint32_t)ch;
     }
   }
   return (uint32_t)col;
@@ -462,7 +468,8 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
 // each CTA's epilogue warps drain their own 128 rows and report to the leader's accumulator-free barrier.
 template <bool kSwin, bool kPair = false>
 __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
-                           uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
+                           uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp_id, int lane) {
+  const int warp = uniform_warp(warp_id);
   const MegaParams& p = ca.p;
   GemmGeom g = gemm_geom(st);
   if constexpr (kPair) g.nh = 1;                                       // per CTA: one 128-row half of the pair's tile
@@ -492,13 +499,15 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const CUtensorMap* tmA = map_ptr(ca, st.tm_a);
       const CUtensorMap* tmB = map_ptr(ca, st.tm_b);
       bool ok = true;
-      long long t_wait = 0, t_first = 0;
+      unsigned t_wait = 0;
+      long long t_first = 0;
       const bool prof = p.prof != nullptr;
       uint32_t s = rs.slot, bits = rs.slot_bits;
+      const bool b_mn = st.b_mn_major != 0;
       for (int item = first_item; ok && item < g.items; item += item_step) {
         int mt, nt, ks;
         gemm_item(st, item, mt, nt, ks);
@@ -508,8 +517,8 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         int kk = (int)(rot - fast_div(rot, (uint32_t)g.kchunks, st.mg_kchunks) * (uint32_t)g.kchunks);
         for (int kc = 0; kc < g.kchunks; ++kc) {
           const long long tw = prof ? clock64() : 0;
-          if (!mbar_wait(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 100 + (int)s)) { ok = false; break; }
-          if (prof) t_wait += clock64() - tw;
+          if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 100 + (int)s)) { ok = false; break; }
+          if (prof) t_wait += (unsigned)(clock64() - tw);
           const uint32_t fb = full0 + 8 * s;
           const uint32_t a_dst = ring + s * g.slot_bytes, b_dst = a_dst + a_bytes;
           const int k0 = (kbase + kk) * 64;
@@ -523,7 +532,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           } else {
             mbar_expect_tx(fb, (uint32_t)g.slot_bytes);
             tma_load_2d(a_dst, tmA, fb, k0, m0);                // box rows = bm: both halves in one copy
-            if (!st.b_mn_major) {
+            if (!b_mn) {
               tma_load_2d(b_dst, tmB, fb, k0, n0);
             } else {
               for (int j = 0; j < g.bn / 64; ++j) tma_load_2d(b_dst + j * 8192, tmB, fb, n0 + j * 64, k0);
@@ -545,7 +554,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer (of a pair: the leader's) ----------------
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc = kPair ? umma_idesc_f16_pair((uint32_t)g.bn, (uint32_t)st.b_mn_major)
                                    : umma_idesc_f16((uint32_t)g.bn, (uint32_t)st.b_mn_major);
       const uint32_t tmem = ctl_s.tmem_base;
@@ -556,26 +565,28 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       const uint32_t bstep = st.b_mn_major ? 128u : 2u;       // 16 K-rows = 2048 B, or 16 halves = 32 B
       const bool prof = p.prof != nullptr;
       bool ok = true;
-      long long t_full = 0, t_acc = 0, t_first = 0, t_last = 0;
+      // in registers: `rs` may live in memory
+      uint32_t s = rs.slot, bits = rs.slot_bits, acc_next = rs.acc_bits >> 2, acc_bits = rs.acc_bits & 3u;
+      unsigned t_full = 0, t_acc = 0;
+      long long t_first = 0, t_last = 0;
       for (int item = first_item; ok && item < g.items; item += item_step) {
-        const uint32_t acc0 = g.nh == 2 ? 0u : rs.acc;       // accumulator of half 0; half 1 uses buffer 1
+        const uint32_t acc0 = g.nh == 2 ? 0u : acc_next;       // accumulator of half 0; half 1 uses buffer 1
         const uint32_t d0 = tmem + acc0 * kAccStride, d1 = d0 + kAccStride;
         {                                                      // the epilogue must have drained the buffers
           const long long ta = prof ? clock64() : 0;
           for (int h = 0; h < g.nh; ++h) {
             const uint32_t acc = acc0 + (uint32_t)h;
-            if (!mbar_wait(tempty0 + 8 * acc, ((rs.acc_bits >> acc) & 1u) ^ 1u, ctl, 200 + (int)acc)) { ok = false; break; }
+            if (!mbar_wait_hot(tempty0 + 8 * acc, ((acc_bits >> acc) & 1u) ^ 1u, ctl, 200 + (int)acc)) { ok = false; break; }
           }
           tc_fence_after_sync();
-          if (prof) t_acc += clock64() - ta;
+          if (prof) t_acc += (unsigned)(clock64() - ta);
         }
         for (int kc = 0; ok && kc < g.kchunks; ++kc) {
-          const uint32_t s = rs.slot;
           const long long tw = prof ? clock64() : 0;
-          if (!mbar_wait(full0 + 8 * s, (rs.slot_bits >> s) & 1u, ctl, 300 + (int)s)) { ok = false; break; }
+          if (!mbar_wait_hot(full0 + 8 * s, (bits >> s) & 1u, ctl, 300 + (int)s)) { ok = false; break; }
           if (prof) {
             const long long tn = clock64();
-            t_full += tn - tw;
+            t_full += (unsigned)(tn - tw);
             if (!t_first) t_first = tn;
           }
           tc_fence_after_sync();
@@ -588,19 +599,22 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
             else umma_f16_k64(d0, a_lo, b_lo, bstep, idesc, (uint32_t)(kc != 0));
             umma_commit(empty0 + 8 * s);
           }
-          rs.slot_bits ^= 1u << s;
-          rs.slot = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
+          bits ^= 1u << s;
+          s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
         }
         if (!ok) break;
         for (int h = 0; h < g.nh; ++h) {
           const uint32_t acc = acc0 + (uint32_t)h;
           if constexpr (kPair) umma_commit_pair(tfull0 + 8 * acc);
           else umma_commit(tfull0 + 8 * acc);
-          rs.acc_bits ^= 1u << acc;
+          acc_bits ^= 1u << acc;
         }
         if (prof) t_last = clock64();
-        if (g.nh == 1) rs.acc ^= 1u;
+        if (g.nh == 1) acc_next ^= 1u;
       }
+      rs.slot = s;
+      rs.slot_bits = bits;
+      rs.acc_bits = acc_bits | (acc_next << 2);
       if (p.prof) {
         long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
         pr[3] = t_full;
@@ -627,13 +641,19 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     // a warp's staging: 2 KB of the staging area, or -- for the boxes of TMA stores, which want two buffers -- 4 KB of
     // the vector area and the staging area taken together (a stage that writes planes stages no bias)
     uint8_t* sbuf = e.tm_out ? reinterpret_cast<uint8_t*>(vec_s) + (warp - 2) * 2 * kStageWarp : stage_s + (warp - 2) * kStageWarp;
-    unsigned t_wait = 0, t_busy = 0, t_tmem = 0, t_math = 0, t_store = 0;   // cycle totals (32 bits are plenty)
-    long long t_first = 0;
+    // cycle totals of the profile go straight to its record (no registers held for them over the tiles)
+    auto note = [&](int slot, unsigned cycles) {
+      if (warp == 2 && lane == 0)
+        atomicAdd(reinterpret_cast<unsigned long long*>(p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + slot),
+                  (unsigned long long)cycles);
+    };
+    if (prof && warp == 2 && lane == 0)
+      for (int i = 6; i < 11; ++i) p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + i] = 0;
     int box = 0;
     for (int item = first_item; item < g.items; item += item_step) {
       int mt, nt, ks;
       gemm_item(st, item, mt, nt, ks);
-      const uint32_t acc0 = g.nh == 2 ? 0u : rs.acc;
+      const uint32_t acc0 = g.nh == 2 ? 0u : rs.acc_bits >> 2;
       bool ok = true;
       // TMA-store boxes of the CTA's last tile live in the operand ring: once its accumulator is complete every operand
       // tile of the stage has been consumed, and nothing is loaded before the next stage
@@ -643,6 +663,12 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       if (last_tile) box = 0;
       for (int h = 0; h < g.nh; ++h) {
         const uint32_t acc = acc0 + (uint32_t)h;
+        // output rows first: worked out while the accumulator is still being filled
+        const int row0 = mt * g.bm + (kPair ? (int)rank : h) * 128 + q * 32;
+        const uint32_t own = epi_row_offset<kSwin>(st, e, row0 + lane, ks);
+        uint32_t so[4];                              // rows of the staged stores: each lane has worked out one of the 32
+#pragma unroll
+        for (int i = 0; i < 4; ++i) so[i] = __shfl_sync(0xffffffffu, own, 8 * i + (lane >> 2));
         const unsigned tw = prof ? (unsigned)clock64() : 0u;
         ok = mbar_wait_warp(tfull0 + 8 * acc, (rs.acc_bits >> acc) & 1u, ctl, 400 + (int)acc, lane);
         if (!ok) break;
@@ -650,15 +676,11 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         if (prof) {
           const long long now = clock64();
           tb = (unsigned)now;
-          t_wait += tb - tw;
-          if (!t_first) t_first = now;
+          note(6, tb - tw);
+          if (item == first_item && h == 0 && warp == 2 && lane == 0)
+            p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 14] = now;
         }
         tc_fence_after_sync();
-        const int row0 = mt * g.bm + (kPair ? (int)rank : h) * 128 + q * 32;
-        const uint32_t own = epi_row_offset<kSwin>(st, e, row0 + lane, ks);
-        uint32_t so[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) so[i] = epi_row_offset<kSwin>(st, e, row0 + 8 * i + (lane >> 2), ks);
         const uint32_t t0 = tmem + acc * kAccStride;
         const int colbase = nt * g.bn;
         // this warp takes chunks cpar, cpar+2, ... (its partner warp on the same lane quarter the others)
@@ -670,13 +692,13 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           unsigned tm = 0, tmid = 0;
           if (prof) {
             tm = (unsigned)clock64();
-            t_tmem += tm - tl;
+            note(8, tm - tl);
           }
           epilogue_chunk32<kSwin>(st, e, tile_sbuf, r, own, so, colbase + c * 32, lane, tmid,
                                   row0 < e.M ? (uint32_t)row0 : kNoRow, ks, box, nbox);
           if (prof) {
-            t_math += tmid - tm;
-            t_store += (unsigned)clock64() - tmid;
+            note(9, tmid - tm);
+            note(10, (unsigned)clock64() - tmid);
           }
         }
         if ((g.bn & 16) && (full_chunks & 1) == cpar) {
@@ -693,26 +715,18 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           mbar_arrive(tempty0 + 8 * acc);
         }
         rs.acc_bits ^= 1u << acc;
-        if (prof) t_busy += (unsigned)clock64() - tb;
+        if (prof) note(7, (unsigned)clock64() - tb);
       }
       if (!ok) break;
-      if (g.nh == 1) rs.acc ^= 1u;
+      if (g.nh == 1) rs.acc_bits ^= 4u;
     }
     if (e.tm_out && lane == 0) {          // the planes are complete before the CTA reports the stage done
       bulk_wait_group_all();
       fence_proxy_async_global();
     }
     __syncwarp();
-    if (p.prof && warp == 2 && lane == 0) {
-      long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
-      pr[6] = t_wait;
-      pr[7] = t_busy;
-      pr[8] = t_tmem;
-      pr[9] = t_math;
-      pr[10] = t_store;
-      pr[14] = t_first;
-      pr[15] = clock64();
-    }
+    if (prof && warp == 2 && lane == 0)
+      p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 15] = clock64();
   }
 }
 
@@ -1019,7 +1033,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
   const CUtensorMap* tm = map_ptr(ca, st.tm_qkv);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t bits = rs.attn_bit | (rs.attn_bit1 << 1);
       for (int k = 0; k < my_items; ++k) {
         const int item = item_of(k), g = k & 1;
@@ -1052,7 +1066,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       const uint32_t idesc_s = kPair ? umma_idesc_f16_pair(256u, 0u) : umma_idesc_f16(128u, 0u);
       const uint32_t idesc_o = kPair ? umma_idesc_f16_pair(128u, 1u) : umma_idesc_f16(64u, 1u);
       const uint32_t tmem = ctl_s.tmem_base;
@@ -1915,7 +1929,9 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
 constexpr int kFamilyBert = 0, kFamilyBertCoop = 1, kFamilySwin = 2, kFamilyBertPair = 3;
 __device__ __noinline__ void gemm_stage_ool(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
                                             uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
-  gemm_stage<true>(st, ca, ctl_s, ring, vec_s, stage_s, rs, ctl, warp, lane);
+  RoleState r = rs;                    // a copy the roles can keep in registers
+  gemm_stage<true>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
+  rs = r;
 }
 __device__ __noinline__ void ln_stage_ool(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
                                           __half* vec_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {

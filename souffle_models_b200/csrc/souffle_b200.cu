@@ -420,6 +420,16 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   s.mg_seq = fast_div_magic((uint32_t)(s.seq > 0 ? s.seq : 1));
   s.mg_head_dim = fast_div_magic((uint32_t)(s.head_dim > 0 ? s.head_dim : 1));
   s.mg_heads = fast_div_magic((uint32_t)(s.heads > 0 ? s.heads : 1));
+  if (s.epi == EPI_SWIN_QKV || s.epi == EPI_SWIN_PROJ) {
+    s.nwr = s.seq / s.win;
+    s.plane_elems = (uint32_t)s.batch * (uint32_t)(s.nwr * s.nwr * 64) * (uint32_t)s.ldo;
+    // a token grid too large for an exact 32-bit multiplier (from 256 x 256 tokens on) is divided plainly
+    const unsigned long long grid_tokens = (unsigned long long)s.seq * s.seq;
+    s.mg_seq2 = s.M * grid_tokens < (1ull << 32) ? fast_div_magic((uint32_t)grid_tokens) : 0u;
+    s.mg_win = fast_div_magic((uint32_t)s.win);
+    s.mg_nwr = fast_div_magic((uint32_t)s.nwr);
+    s.mg_nwr2 = fast_div_magic((uint32_t)(s.nwr * s.nwr));
+  }
   const unsigned long long out_elems = (unsigned long long)s.M * (unsigned long long)s.N * (s.epi == EPI_PARTIAL ? s.splitk : 1);
   // 2^20 rows keep every multiply-high division exact (numerator * divisor < 2^32)
   if (s.M > (1 << 20) || out_elems * (s.epi == EPI_SWIN_QKV ? 2 : 1) >= 0xFFFF0000ull || (long long)s.items * 16 >= (1ll << 32))

@@ -79,6 +79,10 @@ struct alignas(16) Stage {      // 16-byte multiples: records are fetched with b
   int tiles_n, kchunks, items, slot_bytes, nslots;
   uint32_t mg_splitk, mg_tiles_n, mg_kchunks;   // magic multipliers, see fast_div()
   uint32_t mg_seq, mg_head_dim, mg_heads;
+  // Swin row maps: windows per side of the grid, elements of one of the Q / K / V planes, and the multipliers of the
+  // divisors seq * seq (0: divide plainly), win, nwr and nwr * nwr
+  int nwr;
+  uint32_t plane_elems, mg_seq2, mg_win, mg_nwr, mg_nwr2;
 };
 
 // q = n / d for n * d < 2^32 as one multiply-high: mg = ceil(2^32 / d); d == 1 has no 32-bit multiplier.
