@@ -4,9 +4,13 @@
 // separated by three grid.sync(): per-channel average pool (the channel's image kept in shared memory), the
 // reduce GEMV with x*sigmoid(x), the expand GEMV with sigmoid, and the broadcast add of the gate onto the image.
 // Here a channel's image is cut into slices handed out per warp, so that small channel counts still fill the GPU
-// and small images cost no CTA-wide synchronisation; every warp keeps its slices in shared memory across the one
-// grid barrier, and both tiny GEMVs are recomputed by every CTA that needs them instead of being exchanged through
-// two more barriers: the input is read from HBM once and the output written once.
+// and small images cost no CTA-wide synchronisation; every warp keeps as many of its slices in shared memory across the
+// one grid barrier as fit, and both tiny GEMVs are recomputed by every CTA that needs them instead of being exchanged
+// through two more barriers: the input is read from HBM once and the output written once.
+// The module is bound by memory: 16 warps of an SM have to keep some 40 KB of loads in flight to draw the full HBM rate,
+// so a warp issues eight 16-byte loads per lane before it touches the first of them, and a CTA's weights are on their way
+// to shared memory before the barrier.  One 4-byte load per lane and four in flight took 139 us of GPU time for
+// 32 x 144 x 56 x 56 (0.83 TB/s of the 116 MB the module cannot do without), this form 32 us (3.6 TB/s).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -16,9 +20,15 @@
 namespace souffle {
 
 constexpr int kSeThreads = 512;
-constexpr int kSeCacheFloats = 49152;         // 192 KiB of image slices per CTA
+constexpr int kSeWarps = kSeThreads / 32;
+constexpr int kSeSmemBytes = 229376;          // 224 KiB of dynamic shared memory at most
 constexpr int kSeMaxReduce = 64;              // reduce channels
 constexpr int kSeMaxChannels = 4096;          // channels (their means are staged in shared memory)
+constexpr int kSeUnroll = 8;                  // 16-byte loads a lane has in flight
+
+// Floats of shared memory a cached slice takes: up to three in front of it, so that the 16-byte pieces of the slice sit on
+// 16-byte boundaries there too, wherever it starts in global memory.
+__host__ __device__ inline int se_slice_floats(int slice_len) { return (slice_len + 3 + 3) & ~3; }
 
 struct SeParams {
   const float* input;      // [batch][channels][hw]
@@ -32,47 +42,102 @@ struct SeParams {
   int batch, channels, hw, reduce;
   int slices, slice_len;   // a channel image = slices pieces of slice_len floats (the last one shorter)
   int items;               // batch * channels * slices
-  int cache;               // 1: the CTA's slices fit its shared memory
+  int per_cta;             // CTA b owns items [b * per_cta, (b + 1) * per_cta): few images per CTA
+  int cached;              // of the (up to ceil(per_cta / 16)) slices of a warp, those kept in shared memory
+  int stage_weights;       // 1: w_reduce is brought to shared memory while the CTA loads its slices
   unsigned long long timeout_ns;
 };
 
 __device__ __forceinline__ float se_sigmoid(float x) { return 1.0f / (1.0f + __expf(-x)); }
 
-// Work is handed out per WARP: an item is one slice of one channel image; warp w of CTA b takes items
-// (b * 16 + w), + gridDim.x * 16, ...  Everything but the grid barrier and the per-image reduce GEMV is
-// warp-local, so a 7 x 7 image costs no CTA-wide synchronisation.
-__global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParams p) {
-  extern __shared__ float se_smem[];
-  constexpr int kWarps = kSeThreads / 32;
-  float* cache = se_smem;                                  // image slices of this CTA, kSeCacheFloats / kWarps per warp
-  float* pooled_s = se_smem + kSeCacheFloats;              // channel means of one image [channels <= kSeMaxChannels]
-  float* gate_in = pooled_s + kSeMaxChannels;              // reduce GEMV outputs of one image [reduce]
-  __shared__ int abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gw = blockIdx.x * kWarps + warp, total_warps = gridDim.x * kWarps;
-  float* my_cache = cache + warp * (kSeCacheFloats / kWarps);
-  if (threadIdx.x == 0) abort_flag = 0;
-  __syncthreads();
+// The first element of a slice that sits on a 16-byte boundary.
+__device__ __forceinline__ int se_head(const float* p, int len) {
+  const int h = (4 - (int)((reinterpret_cast<uintptr_t>(p) >> 2) & 3)) & 3;
+  return h < len ? h : len;
+}
 
-  // ---- phase 1: load this warp's slices (kept in shared memory when they fit) and their partial sums ----
+// Sum of one slice (per lane: the lane's share); the slice is copied to `keep` unless that is null.  `keep` has the slice's
+// own offset from a 16-byte boundary.
+__device__ __forceinline__ float se_load_slice(const float* __restrict__ src, float* keep, int len, int lane) {
+  const int head = se_head(src, len), n4 = (len - head) >> 2, tail = head + 4 * n4;
+  float s = 0.0f, edge = 0.0f;
+  const bool has_edge = lane < head || tail + lane < len;          // up to three floats at either end
+  const int at = lane < head ? lane : tail + lane;
+  if (has_edge) edge = __ldg(src + at);
+  const bool has_edge2 = lane < head && tail + lane < len;         // a lane with one at each end
+  float edge2 = 0.0f;
+  if (has_edge2) edge2 = __ldg(src + tail + lane);
+  const float4* s4 = reinterpret_cast<const float4*>(src + head);
+  float4* k4 = reinterpret_cast<float4*>(keep + head);
+  for (int i0 = lane; i0 < n4; i0 += 32 * kSeUnroll) {
+    float4 v[kSeUnroll];
+#pragma unroll
+    for (int u = 0; u < kSeUnroll; ++u) {
+      const int i = i0 + 32 * u;
+      v[u] = i < n4 ? __ldg(s4 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < kSeUnroll; ++u) {
+      const int i = i0 + 32 * u;
+      if (keep && i < n4) k4[i] = v[u];
+      s += (v[u].x + v[u].y) + (v[u].z + v[u].w);
+    }
+  }
+  if (keep && has_edge) keep[at] = edge;
+  if (keep && has_edge2) keep[tail + lane] = edge2;
+  return s + (edge + edge2);
+}
+
+// dst = src + g over one slice; 16 bytes at a time where src and dst have the same offset from a 16-byte boundary.
+__device__ __forceinline__ void se_add_slice(const float* src, float* __restrict__ dst, int len, float g, int lane) {
+  if (((reinterpret_cast<uintptr_t>(src) ^ reinterpret_cast<uintptr_t>(dst)) & 15) != 0) {
+    for (int i = lane; i < len; i += 32) dst[i] = src[i] + g;
+    return;
+  }
+  const int head = se_head(src, len), n4 = (len - head) >> 2, tail = head + 4 * n4;
+  const float4* s4 = reinterpret_cast<const float4*>(src + head);
+  float4* d4 = reinterpret_cast<float4*>(dst + head);
+  for (int i0 = lane; i0 < n4; i0 += 32 * kSeUnroll) {
+    float4 v[kSeUnroll];
+#pragma unroll
+    for (int u = 0; u < kSeUnroll; ++u)
+      if (i0 + 32 * u < n4) v[u] = s4[i0 + 32 * u];
+#pragma unroll
+    for (int u = 0; u < kSeUnroll; ++u)
+      if (i0 + 32 * u < n4) d4[i0 + 32 * u] = make_float4(v[u].x + g, v[u].y + g, v[u].z + g, v[u].w + g);
+  }
+  if (lane < head) dst[lane] = src[lane] + g;
+  if (tail + lane < len) dst[tail + lane] = src[tail + lane] + g;
+}
+
+// Work is handed out per WARP: an item is one slice of one channel image; warp w of CTA b takes items
+// b * per_cta + w, + 16, ...  Everything but the grid barrier and the per-image reduce GEMV is warp-local, so a 7 x 7
+// image costs no CTA-wide synchronisation.
+__global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParams p) {
+  extern __shared__ __align__(16) float se_smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int keep_floats = se_slice_floats(p.slice_len);
+  float* my_cache = se_smem + (size_t)warp * p.cached * keep_floats;                 // this warp's kept slices
+  float* w_red = se_smem + (size_t)kSeWarps * p.cached * keep_floats;                // [reduce][channels] when staged
+  float* pooled_s = w_red + (p.stage_weights ? p.reduce * p.channels : 0);           // channel means of one image
+  float* gate_in = pooled_s + p.channels;                                            // reduce GEMV outputs of one image
+  __shared__ int abort_flag;
+  const int item0 = blockIdx.x * p.per_cta, item1 = min(item0 + p.per_cta, p.items);
+  if (threadIdx.x == 0) abort_flag = 0;
+
+  // ---- phase 1: this warp's slices, their partial sums ----
   int slot = 0;
-  for (int item = gw; item < p.items; item += total_warps, ++slot) {
+  for (int item = item0 + warp; item < item1; item += kSeWarps, ++slot) {
     const int ch = item / p.slices, sl = item - ch * p.slices;          // ch = image * channels + channel
     const int begin = sl * p.slice_len;
     const int len = min(p.slice_len, p.hw - begin);
     const float* src = p.input + (size_t)ch * p.hw + begin;
-    float* dst = my_cache + (size_t)slot * p.slice_len;
-    float s = 0.0f;
-    for (int i = lane; i < len; i += 32) {
-      const float v = __ldg(src + i);
-      if (p.cache) dst[i] = v;
-      s += v;
-    }
-    s = warp_sum(s);
+    float* keep = slot < p.cached ? my_cache + slot * keep_floats + ((reinterpret_cast<uintptr_t>(src) >> 2) & 3) : nullptr;
+    const float s = warp_sum(se_load_slice(src, keep, len, lane));
     if (lane == 0) p.partial[(size_t)ch * p.slices + sl] = s;
   }
 
-  // ---- the one grid barrier: every partial sum is published ----
+  // ---- the one grid barrier: every partial sum is published; the weights come in while this CTA waits ----
   __syncthreads();
   if (threadIdx.x == 0) {
     red_add_release_u32(p.sync, 1u);
@@ -88,6 +153,9 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
         break;
       }
     }
+  } else if (warp > 0 && p.stage_weights) {
+    const int n = p.reduce * p.channels;
+    for (int i = threadIdx.x - 32; i < n; i += kSeThreads - 32) w_red[i] = __ldg(p.w_reduce + i);
   }
   __syncthreads();
   if (abort_flag) return;
@@ -96,14 +164,11 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
   //      item this channel's gate (expand GEMV row, sigmoid) and the add ----
   const float inv_hw = 1.0f / (float)p.hw;
   const int items_per_img = p.channels * p.slices;
-  // the images this CTA's warps touch: items [blockIdx.x * kWarps, ...) stride total_warps -> a CTA-uniform sequence
-  const int rounds = (p.items + total_warps - 1) / total_warps;
+  const float* wr = p.stage_weights ? w_red : p.w_reduce;
   int cur_img = -1;
   slot = 0;
-  for (int rd = 0; rd < rounds; ++rd, ++slot) {
-    const int first = rd * total_warps + blockIdx.x * kWarps;          // item of warp 0 in this round
-    const int last = min(first + kWarps - 1, p.items - 1);
-    if (first >= p.items) break;
+  for (int first = item0; first < item1; first += kSeWarps, ++slot) {    // item of warp 0 in this round
+    const int last = min(first + kSeWarps, item1) - 1;
     for (int img = first / items_per_img; img <= last / items_per_img; ++img) {
       // a round of one CTA spans at most a few images; (re)build the image's reduce outputs when it changes
       if (img != cur_img) {
@@ -111,13 +176,15 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
         for (int k = threadIdx.x; k < p.channels; k += kSeThreads) {
           const float* pp = p.partial + (size_t)(img * p.channels + k) * p.slices;
           float s = 0.0f;
+#pragma unroll 8
           for (int s2 = 0; s2 < p.slices; ++s2) s += __ldcg(pp + s2);       // written by other CTAs: read at L2
           pooled_s[k] = s * inv_hw;
         }
         __syncthreads();
-        for (int j = warp; j < p.reduce; j += kWarps) {
+        for (int j = warp; j < p.reduce; j += kSeWarps) {
           float acc = 0.0f;
-          for (int k = lane; k < p.channels; k += 32) acc = fmaf(pooled_s[k], __ldg(p.w_reduce + (size_t)j * p.channels + k), acc);
+#pragma unroll 4
+          for (int k = lane; k < p.channels; k += 32) acc = fmaf(pooled_s[k], wr[(size_t)j * p.channels + k], acc);
           acc = warp_sum(acc);
           if (lane == 0) gate_in[j] = acc * se_sigmoid(acc);
         }
@@ -125,7 +192,7 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
         cur_img = img;
       }
       const int item = first + warp;
-      if (item < p.items && item / items_per_img == img) {
+      if (item <= last && item / items_per_img == img) {
         const int ch = item / p.slices, sl = item - ch * p.slices;
         const int c = ch - img * p.channels;
         float g = 0.0f;                                      // expand GEMV row of this channel: lanes over the reduce outputs
@@ -134,9 +201,9 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
         if (p.pooled && sl == 0 && lane == 0) p.pooled[ch] = pooled_s[c];
         const int begin = sl * p.slice_len;
         const int len = min(p.slice_len, p.hw - begin);
-        const float* src = p.cache ? my_cache + (size_t)slot * p.slice_len : p.input + (size_t)ch * p.hw + begin;
-        float* dst = p.out + (size_t)ch * p.hw + begin;
-        for (int i = lane; i < len; i += 32) dst[i] = src[i] + g;
+        const float* src = p.input + (size_t)ch * p.hw + begin;
+        if (slot < p.cached) src = my_cache + slot * keep_floats + ((reinterpret_cast<uintptr_t>(src) >> 2) & 3);
+        se_add_slice(src, p.out + (size_t)ch * p.hw + begin, len, g, lane);
       }
     }
   }

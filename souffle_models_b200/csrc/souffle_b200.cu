@@ -1929,21 +1929,28 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
   unsigned launch = 0;
   int rc = ws_record(workspace, st, false, &launch, &p.status);
   if (rc) return rc;
-  const size_t smem = (size_t)(kSeCacheFloats + kSeMaxChannels + kSeMaxReduce) * sizeof(float);
   static bool attr_set[16] = {};
   if (dev < 16 && !attr_set[dev]) {
-    SF_CUDA(cudaFuncSetAttribute(souffle_se_module, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    SF_CUDA(cudaFuncSetAttribute(souffle_se_module, cudaFuncAttributeMaxDynamicSharedMemorySize, kSeSmemBytes));
     attr_set[dev] = true;
   }
-  const int warps_per_cta = kSeThreads / 32;
-  const int ctas = (p.items + warps_per_cta - 1) / warps_per_cta;
-  const int grid = ctas < sms ? ctas : sms;
-  const int per_warp = (p.items + grid * warps_per_cta - 1) / (grid * warps_per_cta);
+  // Items are dealt out evenly over all SMs, in contiguous runs: a small image is pulled in by as many SMs as it has
+  // slices, and a CTA of a large batch meets one or two images, whose reduce GEMV it recomputes.
+  p.per_cta = (p.items + sms - 1) / sms;
+  const int grid = (p.items + p.per_cta - 1) / p.per_cta;
+  // shared memory: the channel means and reduce outputs, then as many slices per warp as fit, then the reduce weights
+  const int per_warp = (p.per_cta + kSeWarps - 1) / kSeWarps;
+  size_t smem = (size_t)(channels + kSeMaxReduce) * sizeof(float);
+  const size_t keep = (size_t)kSeWarps * se_slice_floats(p.slice_len) * sizeof(float), weights = (size_t)reduce * channels * sizeof(float);
+  p.cached = (int)((kSeSmemBytes - smem) / keep);
+  if (p.cached > per_warp) p.cached = per_warp;
+  smem += p.cached * keep;
+  p.stage_weights = smem + weights <= (size_t)kSeSmemBytes ? 1 : 0;
+  if (p.stage_weights) smem += weights;
   p.input = input; p.w_reduce = w_reduce; p.w_expand = w_expand; p.out = out; p.pooled = pooled;
   p.sync = reinterpret_cast<unsigned*>(workspace) + 8;        // words 8, 9: the SE barrier (the GEMM entries use 0..3)
   p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
   p.batch = batch; p.channels = channels; p.hw = height * width; p.reduce = reduce;
-  p.cache = (long long)per_warp * p.slice_len <= kSeCacheFloats / warps_per_cta ? 1 : 0;
   p.timeout_ns = 2000ull * 1000000ull;
   void* kargs[] = {&p};
   SF_CUDA(cudaLaunchCooperativeKernel((const void*)souffle_se_module, dim3(grid), dim3(kSeThreads), kargs, smem, st));

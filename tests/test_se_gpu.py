@@ -55,3 +55,22 @@ def test_bad_arguments():
         efficientnet.se_module(x.cuda(), we.cuda(), wr.cuda())
     with pytest.raises(Exception):
         efficientnet.se_module(x.cuda(), torch.zeros(80, 16).cuda(), torch.zeros(16, 80).cuda())      # reduce > 64
+
+
+@pytest.mark.parametrize("shape", [(5, 9, 7, 33, 64), (40, 56, 56, 144, 6), (3, 150, 149, 7, 3), (2, 8, 8, 4096, 64), (1, 1, 5, 2, 1)])
+@pytest.mark.parametrize("shift", [0, 1, 3])
+def test_slices_at_every_alignment(shape, shift):
+    """Odd image sizes and inputs that start off a 16-byte boundary (edges of the 16-byte pieces), slices that fit shared
+    memory and that do not, reduce weights too large to stage.  Bound: fp32 sums of n terms are within 1e-6 of the
+    largest term for the orders compared here."""
+    from souffle_models_b200 import efficientnet
+    b, h, w, c, r = shape
+    x, wr, we = _case(b, h, w, c, r, 11 + c)
+    we = we / r ** 0.5
+    flat = torch.zeros(x.numel() + 8)
+    flat[shift:shift + x.numel()] = x.reshape(-1)
+    xin = flat.cuda()[shift:shift + x.numel()].view(b, c, h, w)
+    pooled, out = efficientnet.se_module(xin, wr.cuda(), we.cuda())
+    want_pooled, want = so.se_module(x, wr, we)
+    assert (pooled.cpu() - want_pooled).abs().max() < 1e-5
+    assert (out.cpu() - want).abs().max() < 2e-5
