@@ -5,15 +5,22 @@
 // reference's (python/models/lstm/tf_lstm.py:59-70; cpp/lstm/lstm_reuse_shared_memory.cu:309-318):
 // gates i, j, f, o;  c' = c*sigmoid(f+1) + sigmoid(i)*tanh(j);  h' = tanh(c')*sigmoid(o).
 //
-// Design: every layer is owned by one thread-block cluster of kLstmParts CTAs; a CTA keeps its
-// 4*U gate rows of both weight matrices (fp16, [x;h] concatenated along K) on chip for the whole
-// sequence -- three quarters in the registers of its 512 cell threads (48 each at hidden 256: what 18
-// warps leave room for), the rest in shared memory -- and its units' cell state.  Every path through the (layer, step)
-// grid has steps-1 hops along time and layers-1 hops across layers, so the hop along time is the one
-// that has to be short: a CTA writes its units' new hidden state straight into the shared memory of
-// the eight CTAs of its cluster (distributed shared memory, st.async: the store itself counts as a
-// transfer on the receiver's mbarrier, no fence on either side) -- no trip through L2.  Only the hop to
-// the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
+// Design: every layer is owned by one thread-block cluster of kLstmParts CTAs; a CTA keeps its 4*U gate rows of both
+// weight matrices (fp16) in the registers of its cell warps for the whole sequence, and its units' cell state.  Every
+// path through the (layer, step) grid has steps-1 hops along time and layers-1 hops across layers, so the hop along time
+// is the one that has to be short:
+// * The products run on the tensor cores (mma.sync m16n8k16; tcgen05 has no shape for a one-column product).  A warp owns
+//   one 16-row tile -- the four gates of four units -- over the whole of K, so nothing is reduced across warps.  The fp32
+//   vector enters as three fp16 columns (value, remainder, remainder of the remainder, each scaled by 2^11 against the one
+//   before: 33 bits) of the eight the shape has, so the products are those of the fp32 vector; four accumulators per
+//   half of K keep the chains of additions short.
+// * A step's input half W_in x(t) does not depend on the hidden state: it is multiplied while h(t-1) travels.
+// * Hidden states go straight into the shared memory of the eight CTAs of the cluster (distributed shared memory,
+//   st.async: the store itself counts as a transfer on the receiver's mbarrier, no fence on either side), and every cell
+//   warp waits for them itself: there is no CTA barrier in the step.
+// A step of hidden 256 takes 2.4 k cycles (hidden 64: 1.5 k); with the products on the CUDA cores (128 conversions and FMAs per thread, partial sums by
+// shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps 228 -> 161 us, 12 x 64 x 200 266 -> 180 us.
+// Only the hop to the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
 // Every CTA of a layer publishes its own count of finished steps; the consumer checks all eight, so a CTA whose
 // publication lags cannot be covered by its peers running ahead.
 // Two more warps keep that hop off the cell arithmetic's path: a fetch warp brings the layer's input
@@ -31,15 +38,13 @@
 
 namespace souffle {
 
-constexpr int kLstmThreads = 512;                  // threads of the cell arithmetic
-constexpr int kLstmBlock = kLstmThreads + 64;      // + the fetch warp and the publish warp
 constexpr int kLstmParts = 8;                      // CTAs per layer = cluster size
-constexpr int kLstmMaxHidden = 256;
 constexpr int kLstmXBufs = 4;                      // input vectors the fetch warp may run ahead
-constexpr int kLstmRegChunks = 3;                  // of a thread's (up to 4) weight chunks per gate row, those kept in registers
 constexpr int kLstmMaxLayers = 18;
 constexpr int kLstmDoneWords = 256;                // one set of published-step counters: kLstmMaxLayers * kLstmParts, rounded up
 static_assert(kLstmMaxLayers * kLstmParts <= kLstmDoneWords, "counter block too small");
+// threads of a CTA: a cell warp per 32 hidden units of the layer (it owns four of the CTA's), the fetch and the publish warp
+__host__ __device__ constexpr int lstm_block(int H) { return (H / 32 + 2) * 32; }
 
 struct LstmParams {
   const __half* w_in;     // [4*L][H][H], row = output unit, col = input
@@ -55,14 +60,35 @@ struct LstmParams {
   unsigned long long timeout_ns;
 };
 
-// ex2-based forms: absolute error of a few 1e-7 on values in [-1, 1], far inside the 5e-3 bar on hidden states
+// Both forms are evaluated without a branch: a step is one dependent chain, and its lanes differ.
+// ex2-based sigmoid: absolute error of about 1e-7.
 __device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
-__device__ __forceinline__ float tanh_f(float v) { return 1.0f - __fdividef(2.0f, 1.0f + __expf(2.0f * v)); }
+// tanh = 2 sigmoid(2 v) - 1 keeps only the absolute error, which small arguments (hidden states of deep layers) feel: they
+// take the Taylor series, whose first term left out is below 1e-8 of the result for |v| < 1/4.
+__device__ __forceinline__ float tanh_taylor(float v) {
+  const float q = v * v;
+  float r = fmaf(q, 62.0f / 2835.0f, -17.0f / 315.0f);
+  r = fmaf(q, r, 2.0f / 15.0f);
+  r = fmaf(q, r, -1.0f / 3.0f);
+  return fmaf(v * q, r, v);
+}
+// sigmoid(v), or tanh(v) where is_tanh
+__device__ __forceinline__ float gate_f(float v, bool is_tanh) {
+  const float s = sigmoid_f(is_tanh ? 2.0f * v : v), t = tanh_taylor(v), w = fmaf(2.0f, s, -1.0f);
+  return is_tanh ? (fabsf(v) < 0.25f ? t : w) : s;
+}
 
-// Bounded wait on an mbarrier whose arrivals come from other CTAs of the cluster.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const WaitCtl& c, int where) {
+// Bounded wait of a whole warp on an mbarrier; every lane sees the phase itself.  kCluster: its transfers come from other
+// CTAs of the cluster.
+template <bool kCluster>
+__device__ __forceinline__ bool lstm_try(uint32_t bar, uint32_t parity) {
+  if constexpr (kCluster) return mbar_try_wait_cluster(bar, parity);
+  else return mbar_try_wait(bar, parity);
+}
+template <bool kCluster>
+__device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const WaitCtl& c, int where) {
   uint32_t spins = 0;
-  while (!mbar_try_wait_cluster(bar, parity)) {
+  while (!lstm_try<kCluster>(bar, parity)) {
     if (((++spins) & 0xFF) == 0) {
       if (*c.abort_smem) return false;
       if (globaltimer_ns() > c.deadline_ns) {
@@ -73,84 +99,114 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   }
   return true;
 }
-
-// Position of element e of an input or hidden vector in shared memory: the vector is cut into chunks of eight
-// elements (the columns one 16-byte chunk of fp16 weights multiplies); the first halves of all chunks come first, the
-// second halves after them, so that the sixteen threads of a unit read 16 contiguous bytes each.
-__host__ __device__ inline int lstm_vec_index(int e, int H) { return ((e >> 3) << 2) + (e & 3) + ((e & 4) ? H / 2 : 0); }
-
-// Shared memory of a CTA, in this order: weights [rows = 4*U][2H halves, 64-byte pad per row] (only the chunks the
-// cell threads do not keep in registers are read from it); input vectors
-// [kLstmXBufs][H] fp32; hidden vectors [2][H] fp32 (written by the whole cluster); gate pre-activations
-// [2][rows] fp32; mbarriers xfull[kLstmXBufs], xempty[kLstmXBufs], hfull[2]; abort, verdict (two, by step parity)
-// and produced words.
-__host__ __device__ inline size_t lstm_smem_bytes(int H) {
-  const int rows = 4 * (H / kLstmParts);
-  return (kLstmRegChunks < 4 ? (size_t)rows * (2 * H * 2 + 64) : 0) + (size_t)(kLstmXBufs * H + 2 * H + 2 * rows) * 4 + (2 * kLstmXBufs + 2) * 8 + 32;
+template <bool kCluster>
+__device__ __forceinline__ bool lstm_wait_warp(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, int lane) {
+  if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
+  if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
+  int ok = 1;
+  if (lane == 0) ok = lstm_wait_loop<kCluster>(bar, parity, c, where) ? 1 : 0;
+  if (__shfl_sync(0xffffffffu, ok, 0) == 0) return false;
+  return __all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity));       // complete: lane 0 has seen it
 }
 
-__global__ void __launch_bounds__(kLstmBlock, 1) souffle_lstm_wavefront(const LstmParams p) {
-  extern __shared__ __align__(16) uint8_t lsm[];
-  const int H = p.hidden, L = p.layers, T = p.steps;
-  const int U = H / kLstmParts;                 // units owned by this CTA
-  const int rows = 4 * U;                       // gate rows, row = unit*4 + gate
-  const int row_bytes = 2 * H * 2 + 64;
-  __half* w_s = reinterpret_cast<__half*>(lsm);
-  float* x_s = reinterpret_cast<float*>(lsm + (kLstmRegChunks < 4 ? (size_t)rows * row_bytes : 0));   // [kLstmXBufs][H]
-  float* h_s = x_s + kLstmXBufs * H;                                          // [2][H]
-  float* g_s = h_s + 2 * H;                                                   // [2][rows]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(g_s + 2 * rows);
-  int* abort_s = reinterpret_cast<int*>(bars + 2 * kLstmXBufs + 2);
-  // verdict of step t lives in slot t & 1: thread 0 can only write step t+2's after everyone has read step t's
-  // (it has to pass the barrier of step t+1 first), so all threads leave the loop at the same iteration
-  volatile int* verdict_s = abort_s + 4;
-  const uint32_t produced_a = smem_u32(abort_s + 2);       // steps whose hidden states this CTA has stored to global memory
+// D (16 x 8, fp32) += A (16 x 16, fp16) B (16 x 8, fp16).  Lane 4 g + q holds rows g and g + 8 of A and columns 2 q, 2 q + 1 of
+// D, and column g of B.
+__device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// A vector in shared memory: its three fp16 parts, one row each; the pad puts the rows 16 banks apart.
+constexpr float kLstmPart = 2048.0f;                 // scale of a part against the one before
+constexpr float kLstmHScale = 32768.0f;              // hidden states (at most 1 in magnitude) are scaled by this
+__host__ __device__ constexpr int lstm_row(int H) { return H + 32; }
+
+// v (scaled into the range of fp16) = hi + mid / 2^11 + lo / 2^22.  An infinity has no remainder.
+__device__ __forceinline__ void lstm_split(float v, __half& hi, __half& mid, __half& lo) {
+  hi = __float2half_rn(v);
+  const float r = __hisinf(hi) ? 0.0f : (v - __half2float(hi)) * kLstmPart;
+  mid = __float2half_rn(r);
+  lo = __float2half_rn((r - __half2float(mid)) * kLstmPart);
+}
+
+// One half of the gate rows' products (W_in x or W_state h): K = H in blocks of 32.  The order of K inside a block is
+// chosen so that a lane's weights and vector elements are 16 contiguous bytes: lane q of a row takes elements
+// 8 q .. 8 q + 7, four for each of the block's two MMAs.
+// The first kReg blocks' weights are in registers, the others' come from shared memory (`rest`: this thread's pieces, two
+// per block, `rest_step` apart).
+template <int H, int kReg>
+__device__ __forceinline__ void lstm_product(const uint4 (&w)[2][kReg], const uint4* rest, int rest_step, const __half* vec, int lane, float (&out)[4]) {
+  float acc[4][4];
+#pragma unroll
+  for (int s = 0; s < 4; ++s)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[s][i] = 0.0f;
+  const int n = lane >> 2, q = lane & 3;
+#pragma unroll
+  for (int b = 0; b < H / 32; ++b) {
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (n < 3) v = *reinterpret_cast<const uint4*>(vec + n * lstm_row(H) + b * 32 + q * 8);
+    const uint4 w0 = b < kReg ? w[0][b < kReg ? b : 0] : rest[2 * (b - kReg) * rest_step],
+                w1 = b < kReg ? w[1][b < kReg ? b : 0] : rest[(2 * (b - kReg) + 1) * rest_step];
+    mma_16816(acc[(2 * b) & 3], w0.x, w1.x, w0.y, w1.y, v.x, v.y);
+    mma_16816(acc[(2 * b + 1) & 3], w0.z, w1.z, w0.w, w1.w, v.z, v.w);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) out[i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
+}
+
+// H = 64, 128 or 256 (= p.hidden).
+template <int H>
+__global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const LstmParams p) {
+  constexpr int U = H / kLstmParts;             // units owned by this CTA
+  constexpr int kWarps = H / 32;                // cell warps: four units each
+  constexpr int kRow = lstm_row(H);
+  constexpr uint32_t kStepBytes = 6u * H;       // a hidden vector: three fp16 parts
+  __shared__ __align__(16) __half x_s[kLstmXBufs][3 * kRow];      // input vectors
+  __shared__ __align__(16) __half h_s[2][3 * kRow];               // hidden vectors, written by the whole cluster
+  // Hidden 256: a cell thread's weights are 128 registers of the 168 that ten warps leave it (registers are handed out per
+  // four warps); two blocks of the input half stay in shared memory instead.
+  constexpr int kXReg = H == 256 ? 6 : H / 32;
+  __shared__ uint4 wx_rest[H == 256 ? 2 * (H / 32 - kXReg) * kWarps * 32 : 1];
+  __shared__ float x_scale[kLstmXBufs];
+  __shared__ uint64_t bars[2 * kLstmXBufs + 2];
+  __shared__ int abort_w;
+  __shared__ unsigned produced_w;               // hidden states this CTA has stored to global memory
+  const int L = p.layers, T = p.steps;
   const uint32_t xfull0 = smem_u32(bars), xempty0 = smem_u32(bars + kLstmXBufs), hfull0 = smem_u32(bars + 2 * kLstmXBufs);
   const int layer = blockIdx.x / kLstmParts;
   const int part = (int)cluster_cta_rank();     // == blockIdx.x % kLstmParts for clusters along x
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    *abort_s = 0;
-    verdict_s[0] = 1;
-    verdict_s[1] = 1;
-    abort_s[2] = 0;
+    abort_w = 0;
+    produced_w = 0;
     for (int i = 0; i < kLstmXBufs; ++i) {
       mbar_init(xfull0 + 8 * i, 32);            // the 32 lanes of the fetch warp
-      mbar_init(xempty0 + 8 * i, (uint32_t)(16 * U));   // every thread of the cell arithmetic
+      mbar_init(xempty0 + 8 * i, kWarps);       // one lane of every cell warp
     }
-    for (int i = 0; i < 2; ++i) {               // h(0) and h(1): one local arrival that announces H * 4 bytes
+    for (int i = 0; i < 2; ++i) {               // h(0) and h(1): one local arrival that announces the bytes of a vector
       mbar_init(hfull0 + 8 * i, 1);
-      mbar_expect_tx(hfull0 + 8 * i, (uint32_t)H * 4u);
+      mbar_expect_tx(hfull0 + 8 * i, kStepBytes);
     }
     fence_mbar_init();
   }
   if (blockIdx.x == 0)
-    for (int i = tid; i < L * kLstmParts; i += kLstmBlock) p.done_next[i] = 0u;
-  for (int i = tid; i < 2 * H; i += kLstmBlock) h_s[i] = 0.0f;               // h before the first step
-  // ---- weights -> shared memory (once), unless the cell threads keep all of them in registers ----
-  if (kLstmRegChunks < 4) {
-    const int chunks_per_row = 2 * H / 8;       // 16-byte chunks: first H/8 from w_in, rest from w_state
-    for (int i = tid; i < rows * chunks_per_row; i += kLstmBlock) {
-      const int r = i / chunks_per_row, ch = i % chunks_per_row;
-      const int unit = part * U + r / 4, gate = r % 4;
-      const bool st = ch >= H / 8;
-      const __half* src = (st ? p.w_state : p.w_in) + ((size_t)(layer * 4 + gate) * H + unit) * H + (st ? ch - H / 8 : ch) * 8;
-      *reinterpret_cast<uint4*>(reinterpret_cast<uint8_t*>(w_s) + (size_t)r * row_bytes + ch * 16) =
-          __ldg(reinterpret_cast<const uint4*>(src));
-    }
-  }
+    for (int i = tid; i < L * kLstmParts; i += lstm_block(H)) p.done_next[i] = 0u;
+  for (int i = tid; i < 2 * 3 * kRow; i += lstm_block(H)) (&h_s[0][0])[i] = __ushort_as_half(0);    // h before the first step
   __syncthreads();
   cluster_sync_all();                           // every CTA's barriers exist before anyone arrives on them
 
   WaitCtl ctl;
-  ctl.abort_smem = abort_s;
+  ctl.abort_smem = &abort_w;
   ctl.status_g = p.status;
   ctl.deadline_ns = globaltimer_ns() + p.timeout_ns;
 
-  if (tid >= kLstmThreads + 32) {
+  if (warp == kWarps + 1) {
     // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
-    if (tid == kLstmThreads + 32) {
+    if (lane == 0) {
+      const uint32_t produced_a = smem_u32(&produced_w);
       uint32_t published = 0, spins = 0;
       while (published < (uint32_t)T) {
         const uint32_t n = ld_acquire_cta_shared_u32(produced_a) / (uint32_t)U;     // whole steps only
@@ -167,23 +223,42 @@ __global__ void __launch_bounds__(kLstmBlock, 1) souffle_lstm_wavefront(const Ls
       }
     }
     __syncwarp();
-  } else if (tid >= kLstmThreads) {
+  } else if (warp == kWarps) {
     // ---------------- fetch warp: the layer's input vector of every step -> shared memory ----------------
-    const int lane = tid - kLstmThreads;
+    // Two L2 round trips per step (the counters of the layer below, then the vector) are longer than a step: the counters
+    // are read again only when the steps they announced have been used up, and the next vector is requested before this
+    // one is unpacked.
+    constexpr int E = H / 32;                   // elements of this lane: lane * E ...
+    const unsigned* ctr = p.done + (layer - 1) * kLstmParts + (lane & (kLstmParts - 1));
+    unsigned avail = layer == 0 ? (unsigned)T : 0u;       // steps the layer below is known to have published
+    auto load_vector = [&](int t, float (&v)[E]) {
+      const float* src = nullptr;
+      if (layer == 0) {
+        const int tx = p.ref_input_delay ? t - 1 : t;
+        if (tx >= 0) src = p.x + (size_t)tx * H;
+      } else {
+        src = p.h_all + ((size_t)(layer - 1) * T + t) * H;
+      }
+#pragma unroll
+      for (int i = 0; i < E; i += 2) {
+        const float2 f = src ? __ldcg(reinterpret_cast<const float2*>(src + lane * E + i)) : make_float2(0.f, 0.f);
+        v[i] = f.x;
+        v[i + 1] = f.y;
+      }
+    };
+    float v[E], ahead[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) ahead[i] = 0.0f;
+    bool have = false;                          // `v` holds step t already
     for (int t = 0; t < T; ++t) {
       const int xb = t % kLstmXBufs, use = t / kLstmXBufs;
       int ok = 1;
-      if (lane == 0 && use > 0) ok = mbar_wait(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900) ? 1 : 0;
-      ok = __shfl_sync(0xffffffffu, ok, 0);
-      if (ok && layer > 0) {
-        // lane k < 8 waits until CTA k of the layer below has published step t; the warp-wide vote (which also orders
-        // the other lanes' loads behind these acquires) says when all eight have
-        const unsigned* ctr = p.done + (layer - 1) * kLstmParts + (lane & (kLstmParts - 1));
-        bool mine = lane >= kLstmParts;
+      if ((unsigned)t >= avail) {
+        // lanes read the counter of one CTA of the layer below each; the smallest counts
         uint32_t spins = 0;
         for (;;) {
-          if (!mine) mine = ld_acquire_u32(ctr) >= (unsigned)(t + 1);
-          if (__all_sync(0xffffffffu, mine)) break;
+          avail = __reduce_min_sync(0xffffffffu, ld_acquire_u32(ctr));
+          if (avail > (unsigned)t) break;
           if (((++spins) & 0x3F) == 0) {
             int give_up = 0;
             if (lane == 0) {
@@ -200,139 +275,143 @@ __global__ void __launch_bounds__(kLstmBlock, 1) souffle_lstm_wavefront(const Ls
             }
           }
         }
+        __syncwarp();                           // the other lanes' loads stay behind every lane's acquire
+      }
+      if (ok && !have) load_vector(t, v);
+      const bool next = t + 1 < T && (unsigned)(t + 1) < avail;
+      if (ok && next) load_vector(t + 1, ahead);
+      if (ok && use > 0) {
+        if (lane == 0) ok = mbar_wait(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900) ? 1 : 0;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        __syncwarp();
       }
       if (!ok) {
-        if (lane == 0) *abort_s = 1;
+        if (lane == 0) *ctl.abort_smem = 1;
         break;
       }
-      const float* src = nullptr;
+      // Power-of-two scale that takes the vector into the upper range of fp16: a constant for hidden states; for the
+      // caller's input from its largest element (none for infinities and NaN, which pass through as they are).
+      float up = kLstmHScale, down = 1.0f / kLstmHScale;
       if (layer == 0) {
-        const int tx = p.ref_input_delay ? t - 1 : t;
-        if (tx >= 0) src = p.x + (size_t)tx * H;
-      } else {
-        src = p.h_all + ((size_t)(layer - 1) * T + t) * H;
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < E; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+        m = __reduce_max_sync(0xffffffffu, m);
+        uint32_t e = m >> 23;                   // biased exponent
+        if (e == 255u) {
+          up = down = 1.0f;
+        } else {
+          e = e < 15u ? 15u : e;                // 2^-112 and below need no more than the largest scale
+          up = __uint_as_float((268u - e) << 23);        // 2^(14 - (e - 127))
+          down = __uint_as_float((e - 14u) << 23);
+        }
       }
-      for (int i = lane; i < H / 4; i += 32) {     // elements 4i .. 4i+3 = one half of chunk i / 2 (see lstm_vec_index)
-        const float4 v = src ? __ldcg(reinterpret_cast<const float4*>(src) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-        *reinterpret_cast<float4*>(x_s + xb * H + (i & 1) * (H / 2) + (i >> 1) * 4) = v;
+      __half hi[E], mid[E], lo[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) lstm_split(v[i] * up, hi[i], mid[i], lo[i]);
+#pragma unroll
+      for (int i = 0; i < E; i += 2) {
+        __half* dst = x_s[xb] + lane * E + i;
+        *reinterpret_cast<__half2*>(dst) = __halves2half2(hi[i], hi[i + 1]);
+        *reinterpret_cast<__half2*>(dst + kRow) = __halves2half2(mid[i], mid[i + 1]);
+        *reinterpret_cast<__half2*>(dst + 2 * kRow) = __halves2half2(lo[i], lo[i + 1]);
       }
+      if (lane == 0) x_scale[xb] = down;
       mbar_arrive(xfull0 + 8 * xb);             // release: this lane's stores are visible to whoever waits
+      have = next;
+#pragma unroll
+      for (int i = 0; i < E; ++i) v[i] = ahead[i];
     }
   } else {
     // ---------------- cell arithmetic ----------------
-    // Sixteen threads share a unit: thread (u, q) multiplies the four gate rows of unit u with the 16-byte chunks
-    // q, q + 16, ... of [x ; h], so a chunk of the vector is read once for four rows; the sixteen partial sums meet
-    // by shuffles, and lane q = 0 ends up with the unit's four gate pre-activations in registers -- no second trip
-    // through shared memory, no barrier between the products and the cell update.
-    const int n_act = 16 * U;                   // 128, 256 or 512 threads
-    if (tid < n_act) {
-      const int u = tid >> 4, q = tid & 15;
-      const int nj = H / 64;                    // chunks per thread: 1, 2 or 4
-      float c_state = 0.0f;                     // cell state of unit u (the same value in all sixteen lanes)
-      const int unit = part * U + u;
-      const float bias_u = p.bias ? p.bias[layer * H + unit] : 0.0f;
-      const uint32_t h_s_a = smem_u32(h_s);
-      const uint8_t* wu = reinterpret_cast<const uint8_t*>(w_s) + (size_t)(4 * u) * row_bytes;
-      // this thread's weights: chunk j * 16 + q of the four gate rows of unit u, straight from global memory
-      uint4 wreg[kLstmRegChunks > 0 ? kLstmRegChunks : 1][4];
+    // Rows of a warp's tile: row r < 8 is gate r / 4 (i, j) of unit r % 4, row 8 + r gate 2 + r / 4 (f, o).  So lane 4 g + q
+    // meets the sums of gates g / 4 and 2 + g / 4 of unit g % 4: q = 0 finishes the first, q = 1 the second.
+    const int g = lane >> 2, q = lane & 3, unit0 = part * U + warp * 4, unit = unit0 + (g & 3);
+    const float bias_u = p.bias ? p.bias[layer * H + unit] : 0.0f;
+    const float bias_g = bias_u + (q == 1 && g < 4 ? 1.0f : 0.0f);       // the forget gate's + 1
+    const bool is_tanh = q == 0 && g >= 4;                               // gate j
+    uint4 wx[2][kXReg], wh[2][H / 32];
 #pragma unroll
-      for (int j = 0; j < kLstmRegChunks; ++j) {
+    for (int r = 0; r < 2; ++r) {
+      const size_t row = ((size_t)(layer * 4 + 2 * r + (g >> 2)) * H + unit) * H + q * 8;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          wreg[j][g] = make_uint4(0u, 0u, 0u, 0u);
-          if (j < nj) {
-            const int ch = j * 16 + q;
-            const bool st = ch >= H / 8;
-            const __half* src = (st ? p.w_state : p.w_in) + ((size_t)(layer * 4 + g) * H + unit) * H + (st ? ch - H / 8 : ch) * 8;
-            wreg[j][g] = __ldg(reinterpret_cast<const uint4*>(src));
-          }
-        }
-      }
-      for (int t = 0; t < T; ++t) {
-        const int xb = t % kLstmXBufs, hb = t & 1;          // h(t) goes to h_s[hb]; h(t-1) is in h_s[hb ^ 1]
-        // ---- one thread waits for x(t) and h(t-1); its verdict is the CTA's ----
-        if (tid == 0) {
-          bool ok = mbar_wait(xfull0 + 8 * xb, (uint32_t)(t / kLstmXBufs) & 1u, ctl, 910);
-          if (ok && t > 0) {
-            ok = mbar_wait_cluster(hfull0 + 8 * (hb ^ 1), (uint32_t)((t - 1) >> 1) & 1u, ctl, 800 + layer);
-            // that barrier's next phase receives h(t+1); nobody sends it before having this CTA's h(t)
-            if (ok && t + 1 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), (uint32_t)H * 4u);
-          }
-          if (!ok) *abort_s = 1;
-          verdict_s[t & 1] = ok ? 1 : 0;
-        }
-        named_barrier_sync(1, n_act);
-        if (verdict_s[t & 1] == 0) break;
-        // ---- gate pre-activations: fp16 weights x fp32 vector, fp32 accumulate ----
-        const float* xv = x_s + xb * H;
-        const float* hv = h_s + (hb ^ 1) * H;
-        float acc[4][2];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) acc[g][0] = acc[g][1] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (j < nj) {
-            const int ch = j * 16 + q;                      // chunk of [x ; h]
-            const bool is_h = ch >= H / 8;
-            const float* vec = is_h ? hv : xv;
-            const int cl = is_h ? ch - H / 8 : ch;
-            const float4 a = *reinterpret_cast<const float4*>(vec + cl * 4);
-            const float4 b = *reinterpret_cast<const float4*>(vec + H / 2 + cl * 4);
-#pragma unroll
-            for (int g = 0; g < 4; ++g) {
-              uint4 w;
-              if (j < kLstmRegChunks) {
-                uint4& wr = wreg[j < kLstmRegChunks ? j : 0][g];
-                // opaque to the optimiser: otherwise the fp16 -> fp32 conversions are hoisted out of the step loop
-                // and the weights occupy twice the registers
-                asm volatile("" : "+r"(wr.x), "+r"(wr.y), "+r"(wr.z), "+r"(wr.w));
-                w = wr;
-              } else {
-                w = *reinterpret_cast<const uint4*>(wu + (size_t)g * row_bytes + ch * 16);
-              }
-              const __half2* h2 = reinterpret_cast<const __half2*>(&w);
-              const float2 w0 = __half22float2(h2[0]), w1 = __half22float2(h2[1]), w2 = __half22float2(h2[2]),
-                           w3 = __half22float2(h2[3]);
-              acc[g][0] = fmaf(w0.x, a.x, acc[g][0]); acc[g][1] = fmaf(w0.y, a.y, acc[g][1]);
-              acc[g][0] = fmaf(w1.x, a.z, acc[g][0]); acc[g][1] = fmaf(w1.y, a.w, acc[g][1]);
-              acc[g][0] = fmaf(w2.x, b.x, acc[g][0]); acc[g][1] = fmaf(w2.y, b.y, acc[g][1]);
-              acc[g][0] = fmaf(w3.x, b.z, acc[g][0]); acc[g][1] = fmaf(w3.y, b.w, acc[g][1]);
-            }
-          }
-        }
-        mbar_arrive(xempty0 + 8 * xb);                      // this thread has read x(t)
-        float gsum[4];
-#pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          float v = acc[g][0] + acc[g][1];
-#pragma unroll
-          for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          gsum[g] = v;
-        }
-        // ---- cell update of unit u; h(t) -> the whole cluster and the next layer ----
-        // All sixteen lanes hold the four sums.  Lanes 0..3 of the group take one gate's nonlinearity each (f, i, j, o),
-        // the four results come back by shuffle, and every lane then carries the same cell state and h: the sends to
-        // the eight CTAs of the cluster are issued by eight lanes at once.
-        {
-          const int q4 = q & 3;
-          const float pre = (q4 == 0 ? gsum[2] + 1.0f : q4 == 1 ? gsum[0] : q4 == 2 ? gsum[1] : gsum[3]) + bias_u;
-          const float act = q4 == 2 ? tanh_f(pre) : sigmoid_f(pre);
-          const int base = tid & 16;                        // lane of q == 0 within the warp
-          const float sf = __shfl_sync(0xffffffffu, act, base), si = __shfl_sync(0xffffffffu, act, base + 1);
-          const float tj = __shfl_sync(0xffffffffu, act, base + 2), so = __shfl_sync(0xffffffffu, act, base + 3);
-          c_state = c_state * sf + si * tj;
-          const float h = tanh_f(c_state) * so;
-          const uint32_t off = (uint32_t)(hb * H + lstm_vec_index(unit, H)) * 4u;
-          if (q < kLstmParts)
-            st_async_b32(map_shared_rank(h_s_a + off, (uint32_t)q), __float_as_uint(h), map_shared_rank(hfull0 + 8u * (uint32_t)hb, (uint32_t)q));
-          if (q == 0) {
-            __stcg(p.h_all + ((size_t)layer * T + t) * H + unit, h);
-            if (layer == L - 1) p.y[(size_t)t * H + unit] = h;
-            red_add_release_cta_shared_u32(produced_a, 1u);   // the publish warp takes it from here
-          }
-        }
+      for (int b = 0; b < H / 32; ++b) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.w_in + row + b * 32));
+        if (b < kXReg) wx[r][b < kXReg ? b : 0] = w;
+        else wx_rest[(2 * (b - kXReg) + r) * kWarps * 32 + tid] = w;          // read by this thread only
+        wh[r][b] = __ldg(reinterpret_cast<const uint4*>(p.w_state + row + b * 32));
       }
     }
+    // lane 8 k + d sends part k of the warp's four hidden states to CTA d; lane 24 stores them to global memory
+    const int send_part = lane >> 3;
+    const uint32_t send_to = map_shared_rank(smem_u32(&h_s[0][(send_part < 3 ? send_part : 0) * kRow + unit0]), (uint32_t)(lane & 7));
+    const uint32_t send_bar = map_shared_rank(hfull0, (uint32_t)(lane & 7));
+    const uint32_t produced_a = smem_u32(&produced_w);
+    float c_state = 0.0f;                       // cell state of `unit` (the same value in its eight lanes)
+    float cx[4];                                // W_in x(t), scaled back
+    bool ok = true;
+    auto input_half = [&](int t) {
+      const int xb = t % kLstmXBufs;
+      ok = lstm_wait_warp<false>(xfull0 + 8 * xb, (uint32_t)(t / kLstmXBufs) & 1u, ctl, 910, lane);
+      if (!ok) return;
+      lstm_product<H, kXReg>(wx, wx_rest + (H == 256 ? tid : 0), kWarps * 32, x_s[xb], lane, cx);
+      const float down = x_scale[xb];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cx[i] *= down;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(xempty0 + 8 * xb);       // this warp has read x(t)
+    };
+    input_half(0);
+    for (int t = 0; ok && t < T; ++t) {
+      const int hb = t & 1;                               // h(t) goes to h_s[hb]; h(t-1) is in h_s[hb ^ 1]
+      if (t > 0) {
+        ok = lstm_wait_warp<true>(hfull0 + 8 * (hb ^ 1), (uint32_t)((t - 1) >> 1) & 1u, ctl, 800 + layer, lane);
+        if (!ok) break;
+        // that barrier's next phase receives h(t+1); nobody sends it before having this warp's h(t)
+        if (tid == 0 && t + 1 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), kStepBytes);
+      }
+      float ch[4];
+      lstm_product<H, H / 32>(wh, wx_rest, 0, h_s[hb ^ 1], lane, ch);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ch[i] = fmaf(ch[i], 1.0f / kLstmHScale, cx[i]);
+      // columns 0, 1 (lane q = 0) and 2 (q = 1) are the three parts of the vector
+      const float first = q == 0 ? fmaf(ch[1], 1.0f / kLstmPart, ch[0]) : ch[0] * (1.0f / (kLstmPart * kLstmPart));
+      const float second = q == 0 ? fmaf(ch[3], 1.0f / kLstmPart, ch[2]) : ch[2] * (1.0f / (kLstmPart * kLstmPart));
+      const float other = __shfl_xor_sync(0xffffffffu, q == 0 ? second : first, 1);
+      const float pre = (q == 0 ? first : second) + other + bias_g;
+      const float act = gate_f(pre, is_tanh);
+      const int base = 4 * (g & 3);
+      const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
+      const float gj = __shfl_sync(0xffffffffu, act, base + 16), go = __shfl_sync(0xffffffffu, act, base + 17);
+      c_state = c_state * gf + gi * gj;
+      const float h = gate_f(c_state, true) * go;
+      // lanes 4 u .. 4 u + 3 offer the three parts of unit u's hidden state and the fp32 value itself; lane 8 k + d collects
+      // offer k of all four units
+      uint32_t offer;
+      {
+        const float s0 = h * kLstmHScale;
+        const __half hi = __float2half_rn(s0);
+        const float s1 = (s0 - __half2float(hi)) * kLstmPart;
+        const __half mid = __float2half_rn(s1);
+        const __half lo = __float2half_rn((s1 - __half2float(mid)) * kLstmPart);
+        offer = q == 0 ? __half_as_ushort(hi) : q == 1 ? __half_as_ushort(mid) : q == 2 ? __half_as_ushort(lo) : __float_as_uint(h);
+      }
+      uint32_t got[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) got[i] = __shfl_sync(0xffffffffu, offer, 4 * i + send_part);
+      if (lane < 24) {
+        const uint64_t word = (uint64_t)(got[0] | (got[1] << 16)) | ((uint64_t)(got[2] | (got[3] << 16)) << 32);
+        st_async_b64(send_to + (uint32_t)(hb * 3 * kRow * 2), word, send_bar + 8u * (uint32_t)hb);
+      }
+      if (lane == 24) {
+        const float4 h4 = make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
+        __stcg(reinterpret_cast<float4*>(p.h_all + ((size_t)layer * T + t) * H + unit0), h4);
+        if (layer == L - 1) *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) = h4;
+        red_add_release_cta_shared_u32(produced_a, 4u);   // the publish warp takes it from here
+      }
+      if (t + 1 < T) input_half(t + 1);
+    }
+    if (!ok && lane == 0) *ctl.abort_smem = 1;
   }
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();

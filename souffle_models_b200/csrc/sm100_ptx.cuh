@@ -412,11 +412,11 @@ __device__ __forceinline__ uint32_t map_shared_rank(uint32_t addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-// 4-byte store into the shared memory of any CTA of the cluster that also counts 4 bytes as transferred on an
+// 8-byte store into the shared memory of any CTA of the cluster that also counts 8 bytes as transferred on an
 // mbarrier of that CTA: the value is visible to whoever sees the barrier's phase complete (no fence on either side)
-__device__ __forceinline__ void st_async_b32(uint32_t cluster_addr, uint32_t v, uint32_t cluster_mbar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
-               ::"r"(cluster_addr), "r"(v), "r"(cluster_mbar) : "memory");
+__device__ __forceinline__ void st_async_b64(uint32_t cluster_addr, uint64_t v, uint32_t cluster_mbar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+               ::"r"(cluster_addr), "l"(v), "r"(cluster_mbar) : "memory");
 }
 __device__ __forceinline__ void st_release_cta_shared_u32(uint32_t addr, uint32_t v) {
   asm volatile("st.release.cta.shared::cta.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");

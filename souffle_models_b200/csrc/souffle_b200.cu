@@ -1663,11 +1663,14 @@ static int lstm_coop_default() {
   return (e && e[0] == '1') ? 1 : 0;
 }
 static int g_lstm_coop = lstm_coop_default();
-static void lstm_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int layers, size_t smem, cudaStream_t st, bool coop) {
+static const void* lstm_kernel(int hidden) {
+  return hidden == 64 ? (const void*)souffle_lstm_wavefront<64> : hidden == 128 ? (const void*)souffle_lstm_wavefront<128>
+                                                                                : (const void*)souffle_lstm_wavefront<256>;
+}
+static void lstm_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int layers, int hidden, cudaStream_t st, bool coop) {
   memset(cfg, 0, sizeof(*cfg));
   cfg->gridDim = dim3(layers * kLstmParts);
-  cfg->blockDim = dim3(kLstmBlock);
-  cfg->dynamicSmemBytes = smem;
+  cfg->blockDim = dim3(lstm_block(hidden));
   cfg->stream = st;
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = kLstmParts;
@@ -1678,29 +1681,29 @@ static void lstm_launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at,
   cfg->attrs = at;
   cfg->numAttrs = coop ? 2 : 1;
 }
-static int lstm_check_resident(int layers, size_t smem) {
+static int lstm_check_resident(int layers, int hidden) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
-  lstm_launch_config(&cfg, at, layers, smem, nullptr, false);
+  lstm_launch_config(&cfg, at, layers, hidden, nullptr, false);
   int clusters = 0;
-  SF_CUDA(cudaOccupancyMaxActiveClusters(&clusters, (const void*)souffle_lstm_wavefront, &cfg));
+  SF_CUDA(cudaOccupancyMaxActiveClusters(&clusters, lstm_kernel(hidden), &cfg));
   if (clusters < layers)
     return fail(SOUFFLE_NOT_CORESIDENT, "%d clusters of %d CTAs needed, %d can be resident", layers, kLstmParts, clusters);
   return SOUFFLE_OK;
 }
-static int lstm_launch(const LstmParams& lp, size_t smem, cudaStream_t st) {
+static int lstm_launch(const LstmParams& lp, cudaStream_t st) {
   void* kargs[] = {const_cast<LstmParams*>(&lp)};
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at[2];
   if (g_lstm_coop) {
-    lstm_launch_config(&cfg, at, lp.layers, smem, st, true);
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, (const void*)souffle_lstm_wavefront, kargs);
+    lstm_launch_config(&cfg, at, lp.layers, lp.hidden, st, true);
+    const cudaError_t e = cudaLaunchKernelExC(&cfg, lstm_kernel(lp.hidden), kargs);
     if (e == cudaSuccess) return SOUFFLE_OK;
     cudaGetLastError();          // a refused launch configuration is not sticky
     g_lstm_coop = 0;
   }
-  lstm_launch_config(&cfg, at, lp.layers, smem, st, false);
-  SF_CUDA(cudaLaunchKernelExC(&cfg, (const void*)souffle_lstm_wavefront, kargs));
+  lstm_launch_config(&cfg, at, lp.layers, lp.hidden, st, false);
+  SF_CUDA(cudaLaunchKernelExC(&cfg, lstm_kernel(lp.hidden), kargs));
   return SOUFFLE_OK;
 }
 
@@ -1711,7 +1714,6 @@ struct SouffleLstmPlan {
   unsigned* done = nullptr;   // two sets of kLstmDoneWords counters, used by alternate launches
   int* status = nullptr;
   unsigned launch_id = 0;
-  size_t smem = 0;
 };
 
 int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, const void* w_state, const float* bias,
@@ -1732,14 +1734,12 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
   SouffleLstmPlan* p = new SouffleLstmPlan();
   p->desc = d;
   const int H = d.hidden;
-  p->smem = lstm_smem_bytes(H);
   const size_t wbytes = (size_t)4 * d.layers * H * H * 2;
-  cudaError_t e = cudaFuncSetAttribute(souffle_lstm_wavefront, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_smem_bytes(kLstmMaxHidden));
-  if (e == cudaSuccess && lstm_check_resident(d.layers, p->smem) != SOUFFLE_OK) {
+  if (lstm_check_resident(d.layers, H) != SOUFFLE_OK) {
     delete p;
     return SOUFFLE_NOT_CORESIDENT;
   }
-  if (e == cudaSuccess) e = cudaMalloc((void**)&p->w_in, wbytes);
+  cudaError_t e = cudaMalloc((void**)&p->w_in, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->w_state, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->h_all, (size_t)d.layers * d.steps * H * 4);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->done, 2 * kLstmDoneWords * sizeof(unsigned));
@@ -1778,7 +1778,7 @@ int souffle_lstm_forward(SouffleLstmPlan* plan, const float* x, float* y, souffl
   lp.status = plan->status;
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
-  const int rc = lstm_launch(lp, plan->smem, reinterpret_cast<cudaStream_t>(stream));
+  const int rc = lstm_launch(lp, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
   plan->launch_id++;
   return SOUFFLE_OK;
@@ -1812,8 +1812,6 @@ static int static_lstm_device(int* dev_out, StaticLstmDevice** sd_out) {
     SF_CUDA(cudaDeviceGetAttribute(&sd.sms, cudaDevAttrMultiProcessorCount, dev));
     void* ptr = nullptr;
     SF_CUDA(cudaGetSymbolAddress(&ptr, g_lstm_static_scratch));
-    // the largest shared-memory request any shape makes (plans ask for the same limit)
-    SF_CUDA(cudaFuncSetAttribute(souffle_lstm_wavefront, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lstm_smem_bytes(kLstmMaxHidden)));
     sd.scratch = static_cast<unsigned char*>(ptr);
     sd.ready = true;
   }
@@ -1840,13 +1838,12 @@ int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, c
   int rc = static_lstm_device(&dev, &sdp);
   if (rc) return rc;
   StaticLstmDevice& sd = *sdp;
-  const size_t smem = lstm_smem_bytes(d.hidden);
   {
     // all clusters must be resident at once: asked of the driver once per (device, layers, hidden)
     const int hi = d.hidden == 64 ? 0 : (d.hidden == 128 ? 1 : 2);
     std::lock_guard<std::mutex> lock(sd.mutex);
     if (!(sd.resident_ok[hi] & (1u << d.layers))) {
-      rc = lstm_check_resident(d.layers, smem);
+      rc = lstm_check_resident(d.layers, d.hidden);
       if (rc) return rc;
       sd.resident_ok[hi] |= 1u << d.layers;
     }
@@ -1866,7 +1863,7 @@ int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, c
   lp.status = device_status ? reinterpret_cast<int*>(device_status) : reinterpret_cast<int*>(ctl + kStaticStatusOffset);
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
-  return lstm_launch(lp, smem, st);
+  return lstm_launch(lp, st);
 }
 
 // For callers that passed no device_status: waits for `stream`, then reads the status words the last

@@ -80,6 +80,48 @@ def test_lstm_larger_weights_and_bias():
     assert (y.cpu() - want).abs().max() < 5e-3
 
 
+@pytest.mark.parametrize("layers,hidden,steps,scale", [(1, 64, 1, 1.0), (2, 128, 9, 1e-6), (2, 256, 33, 1e5), (12, 64, 5, 1.0),
+                                                       (3, 256, 6, 1e-40)])
+def test_lstm_against_64_bits(layers, hidden, steps, scale):
+    """Few steps, many layers, inputs outside the range of fp16 (the vector is split into scaled fp16 parts).  fp32 sums
+    and activations good to a few 1e-7 of values of order 0.1 and above; vectors that vanish keep their relative error."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(layers + steps)
+    w = [((torch.rand(4 * layers, hidden, hidden, generator=g) - 0.5) * 2 / hidden ** 0.5).half() for _ in range(2)]
+    x = torch.randn(1, steps, hidden, generator=g) * scale
+    plan = lstm.LstmStack(w[0].cuda(), w[1].cuda(), steps)
+    y = plan.forward(x.cuda()).cpu().double()[0]
+    plan.status()
+    seq = x[0].double()
+    for l in range(layers):
+        wi, ws = (m[4 * l:4 * l + 4].reshape(4 * hidden, hidden).double() for m in w)
+        h = c = torch.zeros(hidden, dtype=torch.float64)
+        rows = []
+        for t in range(steps):
+            z = (wi @ seq[t] + ws @ h).view(4, hidden)                 # gates i, j, f, o
+            c = c * torch.sigmoid(z[2] + 1) + torch.sigmoid(z[0]) * torch.tanh(z[1])
+            h = torch.tanh(c) * torch.sigmoid(z[3])
+            rows.append(h)
+        seq = torch.stack(rows)
+    if seq.norm() > 1e-30:
+        assert (y - seq).norm() / seq.norm() < 5e-6
+    else:
+        assert y.abs().max() < 1e-30
+
+
+def test_lstm_infinities_and_nan_stay_in_their_step():
+    """An infinite input saturates its gates, a NaN spoils every later step and no earlier one."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(5)
+    w = [(torch.rand(4, 64, 64, generator=g) - 0.5).half().cuda() for _ in range(2)]
+    x = torch.randn(1, 5, 64, generator=g)
+    x[0, 2, 3], x[0, 3, 5] = float("inf"), float("nan")
+    plan = lstm.LstmStack(w[0], w[1], 5)
+    y = plan.forward(x.cuda())
+    plan.status()
+    assert torch.isfinite(y[0, :3]).all() and torch.isnan(y[0, 3:]).all()
+
+
 def test_fused_lstm_drop_in_signature():
     from souffle_models_b200 import lstm
     x, w_in, w_st = so.make_lstm_params()
