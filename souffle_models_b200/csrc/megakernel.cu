@@ -1664,7 +1664,7 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
 template <int NJ>
 __device__ __forceinline__ void ln_row_direct(const float* pl, int n_partial, int plane_stride, const __half* res,
                                               const __half* bias, const __half* gamma, const __half* beta, float eps,
-                                              __half* out, int lane) {
+                                              __half* out, __half* sum_out, int lane) {
   constexpr int kG = NJ <= 4 ? 4 : (NJ <= 6 ? 3 : 2);      // planes in flight at once
   float z[NJ][4];
   {
@@ -1702,11 +1702,15 @@ __device__ __forceinline__ void ln_row_direct(const float* pl, int n_partial, in
         for (int g = 0; g < kG; ++g) { z[j][0] += v[g][j].x; z[j][1] += v[g][j].y; z[j][2] += v[g][j].z; z[j][3] += v[g][j].w; }
     }
   }
-  if (eps < 0.0f) {                     // sum only
+  if (sum_out) {                        // the sum itself, as fp16; what is normalised below is the rounded value
 #pragma unroll
-    for (int j = 0; j < NJ; ++j)
-      *reinterpret_cast<uint2*>(out + (lane + 32 * j) * 4) = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
-    return;
+    for (int j = 0; j < NJ; ++j) {
+      const uint2 w = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
+      *reinterpret_cast<uint2*>(sum_out + (lane + 32 * j) * 4) = w;
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+      z[j][0] = f0.x; z[j][1] = f0.y; z[j][2] = f1.x; z[j][3] = f1.y;
+    }
+    if (eps < 0.0f) return;             // sum only
   }
   uint2 ug[NJ], ubt[NJ];
 #pragma unroll
@@ -1763,12 +1767,13 @@ __device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& 
     const float* pl0 = st.partial + (size_t)row * N;
     const __half* ra = resid ? resid + (size_t)row * N : nullptr;
     __half* o0 = out + (size_t)row * N;
+    __half* so = st.eps < 0.0f ? o0 : st.sum_out ? reinterpret_cast<__half*>(st.sum_out) + (size_t)row * N : nullptr;
     switch (N >> 7) {
-      case 1: ln_row_direct<1>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, lane); break;
-      case 2: ln_row_direct<2>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, lane); break;
-      case 4: ln_row_direct<4>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, lane); break;
-      case 6: ln_row_direct<6>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, lane); break;
-      default: ln_row_direct<8>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, lane); break;
+      case 1: ln_row_direct<1>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 2: ln_row_direct<2>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 4: ln_row_direct<4>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 6: ln_row_direct<6>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      default: ln_row_direct<8>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
     }
   }
 }

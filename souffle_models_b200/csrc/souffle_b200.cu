@@ -1513,10 +1513,18 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     const __half* xin = bi == 0 ? nullptr : xbuf[(bi - 1) & 1];
     const bool last = bi == n_blocks - 1;
 
-    Stage s = blank_stage(STAGE_LN);                       // LN1(x)
+    // LN1(x): a stage of its own in the first block; later ones normalise the rows in the stage that adds up the block
+    // before (one grid barrier and one pass over x less per block)
+    Stage s = blank_stage(STAGE_LN);
     s.M = T; s.N = C; s.ldo = C; s.n_partial = 0; s.resid_sel = in_sel; s.resid = xin; s.out = y1; s.gamma = ln1_g; s.beta = ln1_b;
     s.eps = d.eps;
-    p->stages.push_back(s);
+    if (bi == 0) {
+      p->stages.push_back(s);
+    } else {
+      Stage& sum = p->stages.back();
+      sum.sum_out = sum.out;
+      sum.out = y1; sum.gamma = ln1_g; sum.beta = ln1_b; sum.eps = d.eps;
+    }
     s = blank_stage(STAGE_GEMM);                           // QKV, rolled and scattered window-major
     s.tm_a = m_y1; s.tm_b = m_wqkv; s.M = T; s.N = 3 * C; s.K = C; s.bm = t_qkv.bm; s.bn = t_qkv.bn; s.epi = EPI_SWIN_QKV;
     s.bias = qkv_b; s.out = qkvw; s.ldo = C; s.batch = d.batch; s.heads = Hh; s.head_dim = 32; s.seq = R; s.win = ws; s.shift = shift;

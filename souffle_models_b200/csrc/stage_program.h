@@ -63,7 +63,8 @@ struct alignas(16) Stage {      // 16-byte multiples: records are fetched with b
   // ---- layer norm ----
   const void* gamma; // fp16 [N] or null
   const void* beta;  // fp16 [N] or null
-  float eps;
+  float eps;         // < 0: no normalisation, the sum goes to `out`
+  void* sum_out;     // fp16 [M][N] or null: the sum (rounded to fp16, which is then what gets normalised) is stored here as well
   int n_partial;     // number of fp32 partial planes to sum
   int prof_index;    // position of this stage in the program (set by the host when the program is built)
   // ---- weight prefetch: the B matrix of the GEMM stage two stages further on, pulled into L2 by all CTAs while
