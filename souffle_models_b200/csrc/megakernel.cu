@@ -1288,21 +1288,28 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
 }
 
 // ------------------------------------------------------------------------------------
-// Swin window attention: one work item = (window, head).  Q/K/V live window-major as [3][windows][64][C]
-// with the heads side by side in C, so one 64-column TMA box holds a PAIR of 32-wide heads; the MMAs of
-// head h read their half of every 128-byte row (K-major operands: descriptor start +64 B for odd heads)
+// Swin window attention.  Q/K/V live window-major as [3][windows][64][C] with the heads side by side in C, so one box of
+// 128 rows x 64 columns holds two windows of a PAIR of 32-wide heads.  A work item is n consecutive windows x n heads:
+// n = 2  group g of four softmax warps takes head 2 c + g; its upper 64 rows are the first window, the lower 64 the second,
+//        and every product is issued once per window (the rows of the other window in it are dropped), so all eight warps
+//        have rows of their own and a CTA has four (window, head) problems in flight;
+// n = 1  one (window, head): half of group 0's rows are padding and group 1 is idle, but no warp waits for another head.
+// The host takes n = 1 while that gives every CTA one item at most.  Two blocks and a merge, n = 1 -> 2: 16 x 28 x 28 x 256
+// (2048 problems) 281 -> 238 us, 4 x 56 x 56 x 128 (1024) 185 -> 166, 18 blocks of 4 x 14 x 14 x 512 (256) 860 -> 831; below
+// one item per CTA the other way round: 6 blocks of 5 x 7 x 7 x 768 (120) 262 against 280, 2 of 14 x 14 x 512 (64) 79 against 82.
+// The MMAs of head h read their half of every 128-byte row (K-major operands: descriptor start +64 B for odd heads)
 // or their half of the output columns (P.V is computed for the pair, the other half is dropped).
 // Scores get the relative-position bias of the (query, key) offset and, for shifted windows, -100 where
 // query and key come from different sides of the wrap-around.  Slots >= win*win are padding.
 // ------------------------------------------------------------------------------------
-// Softmax of one query row of a WS x WS window (thread = row): reads the 64 score columns from TMEM,
+// Softmax of one query row of a WS x WS window (thread = row, `r_in` = row of the window, `live` = the window exists): reads the 64 score columns from TMEM,
 // adds bias and shift mask, writes the unnormalised probabilities as an fp16 A-operand row (128B swizzle)
 // and returns their sum.  Rows and keys >= WS*WS are padding (probability 0).
 template <int WS>
-__device__ __forceinline__ float swin_softmax_row(uint32_t tmem, const float* bias_s, uint8_t* prow, int r_in, int wy, int wx,
+__device__ __forceinline__ float swin_softmax_row(uint32_t tmem, const float* bias_s, uint8_t* prow, int r_in, bool live, int wy, int wx,
                                                   int R, int shift, float sl2) {
   constexpr int NT = WS * WS, TBL = 2 * WS - 1;
-  const bool rowok = r_in < NT;
+  const bool rowok = live && r_in < NT;
   const int qy = rowok ? r_in / WS : 0, qx = rowok ? r_in - qy * WS : 0;
   // region of a shifted coordinate along one axis: 0 | 1 | 2 (only the last window row/column mixes regions)
   int regy[WS], regx[WS];
@@ -1360,24 +1367,26 @@ __device__ __noinline__ void attn_swin_stage(const Stage& st, const CallArgs& ca
                                 uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
   const int R = st.seq, ws = st.win, shift = st.shift, H = st.heads, C = st.ldo;
   const int nwr = R / ws, nw_img = nwr * nwr, n_windows = st.batch * nw_img, n_tok = ws * ws;
-  const int items = n_windows * H;
-  const uint32_t qk_full = smem_u32(&ctl_s.qk_full), qk_empty = smem_u32(&ctl_s.qk_empty);
-  const uint32_t v_full = smem_u32(&ctl_s.v_full), v_empty = smem_u32(&ctl_s.v_empty);
-  const uint32_t s_full = smem_u32(&ctl_s.s_full), p_full = smem_u32(&ctl_s.p_full), o_full = smem_u32(&ctl_s.o_full);
+  const uint32_t n = (uint32_t)st.bn;                                // windows and heads per item: 1 or 2
+  const int item_h = H / (int)n, items = (n_windows + (int)n - 1) / (int)n * item_h;
+  // scores, probabilities and output have barriers per head (bar(g, ...)), the loads one set; all phases advance once per item
+  const uint32_t bar0 = smem_u32(&ctl_s.qk_full), bar1 = smem_u32(&ctl_s.attn1[0]);
+  auto bar = [&](int g, int which) -> uint32_t { return (g ? bar1 : bar0) + 8u * (uint32_t)which; };
+  const uint32_t qk_full = bar(0, AB_QK_FULL), qk_empty = bar(0, AB_QK_EMPTY), v_full = bar(0, AB_V_FULL), v_empty = bar(0, AB_V_EMPTY);
   const CUtensorMap* tm = map_ptr(ca, st.tm_qkv);
-  // shared memory: Q 16 KiB | K 16 KiB | V 16 KiB | P 16 KiB
+  // shared memory: Q 16 KiB | K 16 KiB | V 16 KiB | P of head 0 16 KiB | P of head 1 16 KiB
+  // TMEM: scores of (head g, window j) at column 64 (2 g + j), outputs 256 further on
   if (warp == 0) {
     if (lane == 0) {
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int h = item % H, w = item / H;
-        const int col = (h >> 1) * 64;
+        const int wp = item / item_h, w0 = wp * (int)n, col = ((item - wp * item_h) * (int)n >> 1) * 64;
         if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 530)) break;
         mbar_expect_tx(qk_full, 2u * kATileBytes);
-        tma_load_2d(ring, tm, qk_full, col, (0 * n_windows + w) * 64);
-        tma_load_2d(ring + kATileBytes, tm, qk_full, col, (1 * n_windows + w) * 64);
+        tma_load_2d(ring, tm, qk_full, col, (0 * n_windows + w0) * 64);
+        tma_load_2d(ring + kATileBytes, tm, qk_full, col, (1 * n_windows + w0) * 64);
         if (!mbar_wait(v_empty, rs.attn_bit ^ 1u, ctl, 531)) break;
         mbar_expect_tx(v_full, (uint32_t)kATileBytes);
-        tma_load_2d(ring + 2 * kATileBytes, tm, v_full, col, (2 * n_windows + w) * 64);
+        tma_load_2d(ring + 2 * kATileBytes, tm, v_full, col, (2 * n_windows + w0) * 64);
         rs.attn_bit ^= 1u;
       }
     }
@@ -1387,63 +1396,76 @@ __device__ __noinline__ void attn_swin_stage(const Stage& st, const CallArgs& ca
       const uint32_t idesc_s = umma_idesc_f16(64u, 0u), idesc_o = umma_idesc_f16(64u, 1u);
       const uint32_t tmem = ctl_s.tmem_base;
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const int h = item % H;
-        const uint32_t half = (uint32_t)(h & 1) * 4u;                  // 64 bytes into every 128-byte row
+        const uint32_t odd = n == 1 ? (uint32_t)(item % item_h) & 1u : 0u;       // a single head may be the pair's second
         if (!mbar_wait(qk_full, rs.attn_bit, ctl, 532)) break;
         tc_fence_after_sync();
-        {
-          // S[128 x 64] = Q_h K_h^T, K = 32: two K=16 steps
-          const uint64_t hi = (uint64_t)kDescHiSw128 << 32;
-          const uint64_t qd = hi | (umma_desc_lo(ring, 16) + half), kd = hi | (umma_desc_lo(ring + kATileBytes, 16) + half);
-          umma_f16(tmem, qd, kd, idesc_s, 0u);
-          umma_f16(tmem, qd + 2u, kd + 2u, idesc_s, 1u);
+        const uint64_t hi = (uint64_t)kDescHiSw128 << 32;
+        for (uint32_t g = 0; g < n; ++g) {
+          // S[128 x 64] = Q_h K_h^T per window, K = 32: two K=16 steps; head g starts 64 bytes into every row, window j
+          // 64 rows (8 KiB) into the K tile
+          const uint64_t qd = hi | (umma_desc_lo(ring, 16) + 4u * (g + odd));
+          for (uint32_t j = 0; j < n; ++j) {
+            const uint64_t kd = hi | (umma_desc_lo(ring + kATileBytes + j * 8192u, 16) + 4u * (g + odd));
+            const uint32_t d = tmem + (2u * g + j) * 64u;
+            umma_f16(d, qd, kd, idesc_s, 0u);
+            umma_f16(d, qd + 2u, kd + 2u, idesc_s, 1u);
+          }
+          umma_commit(bar((int)g, AB_S_FULL));
         }
-        umma_commit(s_full);
         umma_commit(qk_empty);
-        if (!mbar_wait(p_full, rs.attn_bit, ctl, 533)) break;
         if (!mbar_wait(v_full, rs.attn_bit, ctl, 534)) break;
-        tc_fence_after_sync();
-        // O[128 x 64] = P[128 x 64 keys] V_pair[64 keys x 64]: one K chunk of 64
-        umma_f16_k64(tmem + 128, umma_desc_lo(ring + 3 * kATileBytes, 16), umma_desc_lo(ring + 2 * kATileBytes, 8192), 128u,
-                     idesc_o, 0u);
-        umma_commit(o_full);
+        bool ok = true;
+        for (uint32_t g = 0; g < n; ++g) {
+          ok = mbar_wait(bar((int)g, AB_P_FULL), rs.attn_bit, ctl, 533);
+          if (!ok) break;
+          tc_fence_after_sync();
+          // O[128 x 64] = P[128 x 64 keys] V_pair[64 keys x 64] per window: one K chunk of 64
+          for (uint32_t j = 0; j < n; ++j)
+            umma_f16_k64(tmem + 256u + (2u * g + j) * 64u, umma_desc_lo(ring + (3u + g) * kATileBytes, 16),
+                         umma_desc_lo(ring + 2 * kATileBytes + j * 8192u, 8192), 128u, idesc_o, 0u);
+          umma_commit(bar((int)g, AB_O_FULL));
+        }
+        if (!ok) break;
         umma_commit(v_empty);
         rs.attn_bit ^= 1u;
       }
     }
     __syncwarp();
-  } else if (warp < 6) {
-    const int q = warp & 3, r_in = q * 32 + lane;
-    const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
+  } else if (warp < 2 + (int)n * 4) {
+    const int grp = (warp - 2) >> 2, q = warp & 3, r_in = q * 32 + lane;
+    const int j = q >> 1, row = r_in & 63;                           // window of the item, row of the window
+    const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(2 * grp + j) * 64u;
     const float sl2 = st.scale * 1.4426950408889634f, l2e = 1.4426950408889634f;
     const __half* table = reinterpret_cast<const __half*>(st.rel_bias);
     __half* ctx = reinterpret_cast<__half*>(st.out);
     const int tbl = 2 * ws - 1;
-    float* bias_s = reinterpret_cast<float*>(stage_s);               // this head's column of the bias table (x log2 e)
-    uint8_t* prow = ring_ptr + 3 * kATileBytes + r_in * 128;
+    float* bias_s = reinterpret_cast<float*>(stage_s) + grp * 256;   // this head's column of the bias table (x log2 e): at most 225
+    uint8_t* prow = ring_ptr + (3 + grp) * kATileBytes + r_in * 128;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
-      const int h = item % H, wg = item / H, w = wg % nw_img;
+      const int wp = item / item_h, h = (int)n * (item - wp * item_h) + grp;
+      const int wg = (int)n * wp + j, w = wg % nw_img;
+      const bool live = j < (int)n && wg < n_windows;                // an odd number of windows: the last item has one
       const int wy = (w / nwr) * ws, wx = (w % nwr) * ws;
-      named_barrier_sync(2, 128);                                    // previous item's readers are done with bias_s
+      named_barrier_sync(2 + grp, 128);                              // previous item's readers are done with bias_s
       for (int i = r_in; i < tbl * tbl; i += 128) bias_s[i] = __half2float(table[i * H + h]) * l2e;
-      named_barrier_sync(2, 128);
-      if (!mbar_wait_warp(s_full, rs.attn_bit, ctl, 535, lane)) break;
+      named_barrier_sync(2 + grp, 128);
+      if (!mbar_wait_warp(bar(grp, AB_S_FULL), rs.attn_bit, ctl, 535, lane)) break;
       tc_fence_after_sync();
       float sum = 1.0f;
-      if (ws == 7) sum = swin_softmax_row<7>(tmem, bias_s, prow, r_in, wy, wx, R, shift, sl2);
-      else sum = swin_softmax_row<8>(tmem, bias_s, prow, r_in, wy, wx, R, shift, sl2);
+      if (ws == 7) sum = swin_softmax_row<7>(tmem, bias_s, prow, row, live, wy, wx, R, shift, sl2);
+      else sum = swin_softmax_row<8>(tmem, bias_s, prow, row, live, wy, wx, R, shift, sl2);
       const float inv = 1.0f / sum;
       fence_proxy_async_smem();
       tc_fence_before_sync();
-      mbar_arrive(p_full);
-      if (!mbar_wait_warp(o_full, rs.attn_bit, ctl, 536, lane)) break;
+      mbar_arrive(bar(grp, AB_P_FULL));
+      if (!mbar_wait_warp(bar(grp, AB_O_FULL), rs.attn_bit, ctl, 536, lane)) break;
       tc_fence_after_sync();
       {
         uint32_t o[32];
-        tmem_ld32(tmem + 128 + (h & 1) * 32, o);
+        tmem_ld32(tmem + 256u + (uint32_t)(h & 1) * 32u, o);
         tmem_ld_wait(o);
-        if (r_in < n_tok) {
-          uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)wg * 64 + r_in) * C + h * 32);
+        if (live && row < n_tok) {
+          uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)wg * 64 + row) * C + h * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
             dst[i] = make_uint4(pack_h2(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv),

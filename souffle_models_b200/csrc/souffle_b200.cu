@@ -349,7 +349,8 @@ static int stage_items(const Stage& s, bool pair = false) {
   if (s.type == STAGE_GEMM) return ((s.M + s.bm - 1) / s.bm) * (s.N / s.bn) * s.splitk;
   if (s.type == STAGE_ATTN && pair) return s.batch * s.heads / 2;
   if (s.type == STAGE_ATTN) return s.batch * s.heads * ((s.seq + 127) / 128);
-  if (s.type == STAGE_ATTN_SWIN) return s.batch * (s.seq / s.win) * (s.seq / s.win) * s.heads;
+  if (s.type == STAGE_ATTN_SWIN)      // s.bn windows x s.bn heads
+    return (s.batch * (s.seq / s.win) * (s.seq / s.win) + s.bn - 1) / s.bn * (s.heads / s.bn);
   return (s.M + kThreads / 32 - 2) / (kThreads / 32 - 1);       // one row per normalising warp (all warps but the first)
 }
 
@@ -1533,6 +1534,7 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     s = blank_stage(STAGE_ATTN_SWIN);                      // window attention
     s.tm_qkv = m_qkv; s.batch = d.batch; s.heads = Hh; s.head_dim = 32; s.seq = R; s.win = ws; s.shift = shift; s.ldo = C;
     s.scale = 1.0f / sqrtf(32.0f); s.rel_bias = relb; s.out = ctxw;
+    s.bn = nWt * Hh <= sms ? 1 : 2;                        // windows and heads per item, see attn_swin_stage
     p->stages.push_back(s);
     s = blank_stage(STAGE_GEMM);                           // proj, window reverse, roll back, + x
     s.tm_a = m_ctx; s.tm_b = m_wo; s.M = Mw; s.N = C; s.K = C; s.bm = t_proj.bm; s.bn = t_proj.bn; s.epi = EPI_SWIN_PROJ;
