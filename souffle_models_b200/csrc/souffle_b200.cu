@@ -461,7 +461,12 @@ static int status_alloc(int** out) {
     if (~s.used) { slab = &s; break; }
   if (!slab) {
     StatusSlab fresh;
-    SF_CUDA(cudaHostAlloc((void**)&fresh.mem, kStatusSlabBytes, cudaHostAllocPortable | cudaHostAllocMapped));
+    // the first call on a workspace may be one that a stream capture is recording: the allocation is no part of it
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    SF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaHostAlloc((void**)&fresh.mem, kStatusSlabBytes, cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    SF_CUDA(e);
     g_status_slabs.push_back(fresh);
     slab = &g_status_slabs.back();
   }
@@ -1001,9 +1006,11 @@ int souffle_bert_plan_create(const SouffleBertDesc* desc, const SouffleBertLayer
   return SOUFFLE_OK;
 }
 
+static void ws_reclaim();                // see the records of caller-owned workspaces
+
 int souffle_bert_plan_destroy(SouffleBertPlan* plan) {
   if (!plan) return SOUFFLE_OK;
-  cudaDeviceSynchronize();
+  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
   for (void* a : plan->allocs) cudaFree(a);
   status_release(plan->status);
   for (int i = 0; i < 2; ++i) {
@@ -1223,8 +1230,25 @@ static std::mutex g_ws_mutex;
 struct WsRecord {
   unsigned launches = 0;       // of the entry points that alternate between the two barrier pairs
   int* status = nullptr;       // see status_alloc
+  int device = 0;
+  bool forgotten = false;      // the caller has given the workspace up: the next call that is given the address starts afresh
 };
 static std::unordered_map<const void*, WsRecord> g_ws;
+
+// Gives back the status words of forgotten workspaces of the current device, which is idle (nothing can write them).
+static void ws_reclaim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return;
+  std::lock_guard<std::mutex> lock(g_ws_mutex);
+  for (auto it = g_ws.begin(); it != g_ws.end();) {
+    if (it->second.forgotten && it->second.device == dev) {
+      status_release(it->second.status);
+      it = g_ws.erase(it);
+    } else {
+      ++it;
+    }
+  }
+}
 
 // The record of a workspace (`alternate`: counts a launch on the barrier pairs, whose number before it goes to *launch);
 // on first sight its control words are cleared on `st`.
@@ -1233,14 +1257,16 @@ static int ws_record(void* workspace, cudaStream_t st, bool alternate, unsigned*
   auto it = g_ws.find(workspace);
   if (it == g_ws.end()) {
     WsRecord r;
+    SF_CUDA(cudaGetDevice(&r.device));
     int rc = status_alloc(&r.status);
     if (rc) return rc;
-    const cudaError_t e = cudaMemsetAsync(workspace, 0, 128, st);
-    if (e != cudaSuccess) {
-      status_release(r.status);
-      SF_CUDA(e);
-    }
+    r.forgotten = true;
     it = g_ws.emplace(workspace, r).first;
+  }
+  if (it->second.forgotten) {
+    SF_CUDA(cudaMemsetAsync(workspace, 0, 128, st));
+    it->second.launches = 0;
+    it->second.forgotten = false;
   }
   *launch = it->second.launches;
   if (alternate) ++it->second.launches;
@@ -1642,7 +1668,7 @@ int souffle_swin_stage_plan_create(const SouffleSwinDesc* desc, const SouffleSwi
 
 int souffle_swin_block_plan_destroy(SouffleSwinPlan* sp) {
   if (!sp) return SOUFFLE_OK;
-  cudaDeviceSynchronize();
+  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
   for (void* a : sp->base.allocs) cudaFree(a);
   status_release(sp->base.status);
   delete sp;
@@ -1769,7 +1795,7 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
 
 int souffle_lstm_plan_destroy(SouffleLstmPlan* p) {
   if (!p) return SOUFFLE_OK;
-  cudaDeviceSynchronize();
+  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
   cudaFree(p->w_in); cudaFree(p->w_state); cudaFree(p->bias); cudaFree(p->h_all); cudaFree(p->done);
   status_release(p->status);
   delete p;
@@ -1968,10 +1994,9 @@ int souffle_workspace_forget(void* workspace) {
   if (!workspace) return fail(SOUFFLE_BAD_ARGUMENT, "null workspace");
   std::lock_guard<std::mutex> lock(g_ws_mutex);
   auto it = g_ws.find(workspace);
-  if (it == g_ws.end()) return SOUFFLE_OK;
-  cudaDeviceSynchronize();                           // a kernel still running on it may write its status words
-  status_release(it->second.status);
-  g_ws.erase(it);
+  // a kernel still running on it may write its status words: they stay with the address until a plan of the device is
+  // destroyed (which waits for the device)
+  if (it != g_ws.end()) it->second.forgotten = true;
   return SOUFFLE_OK;
 }
 
@@ -1981,12 +2006,9 @@ int souffle_workspace_status(void* workspace, souffle_stream_t stream) {
   int h[4] = {0, 0, 0, 0};
   std::lock_guard<std::mutex> lock(g_ws_mutex);
   auto it = g_ws.find(workspace);
-  if (it == g_ws.end()) return SOUFFLE_OK;           // no call has used it
+  if (it == g_ws.end() || it->second.forgotten) return SOUFFLE_OK;      // no call has used it
   status_take(it->second.status, h);
-  if (h[0] != DEV_OK) {                              // start over: the next call on this workspace clears all of it
-    status_release(it->second.status);
-    g_ws.erase(it);
-  }
+  if (h[0] != DEV_OK) it->second.forgotten = true;   // start over: the next call on this workspace clears all of it
   return decode_status(h, "souffle workspace");
 }
 

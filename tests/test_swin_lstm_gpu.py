@@ -307,3 +307,27 @@ def test_lstm_launch_mode_and_profile_case():
     from souffle_models_b200 import _lib, profile_cases
     assert profile_cases.run("lstm", warmup=1, iters=2) > 0
     assert _lib.load().souffle_lstm_launch_mode() in (0, 1)
+
+
+def test_first_call_on_a_workspace_may_be_captured():
+    """The library's own set-up for a workspace it has not seen is no part of a stream capture, and giving a workspace up
+    does not wait for the device."""
+    from souffle_models_b200 import _lib, swin
+    a, w = _rand((130, 128), 1).cuda(), _rand((128, 192), 2, 0.05).cuda()
+    want = swin.gemm(a, w)
+    dev = torch.cuda.current_device()
+    old = swin._ws[dev]
+    swin._ws[dev] = torch.zeros_like(old)
+    try:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = swin.gemm(a, w, check=False)
+            assert _lib.load().souffle_workspace_forget(old.data_ptr()) == 0
+        for _ in range(3):
+            got.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(got, want)
+    finally:
+        _lib.load().souffle_workspace_forget(swin._ws[dev].data_ptr())
+        swin._ws[dev] = old
