@@ -123,6 +123,21 @@ __device__ __forceinline__ const void* sel_ptr(int sel, const void* plan, const 
 // ------------------------------------------------------------------------------------
 // grid barrier: one monotonic arrival counter per launch, bounded spin
 // ------------------------------------------------------------------------------------
+// The polls in front stand in straight line (a loop's way out costs some 150 cycles, see mbar_wait_hot); a CTA that waits
+// longer than they last goes on out of line.
+__device__ __noinline__ void grid_wait_loop(const unsigned* count, unsigned target, const WaitCtl& ctl, int where) {
+  uint32_t spins = 0;
+  while (ld_acquire_u32(count) < target) {
+    if (((++spins) & 0x3F) == 0) {
+      if (*ctl.abort_smem) break;
+      if (globaltimer_ns() > ctl.deadline_ns) {
+        record_timeout(ctl, DEV_TIMEOUT_GRID, where);
+        break;
+      }
+    }
+  }
+}
+
 __device__ bool grid_barrier(const MegaParams& p, const WaitCtl& ctl, int where, SmemCtl& cs) {
   // The CTA barrier orders every thread's global writes before thread 0, whose gpu-scope release is
   // cumulative and publishes them to the other CTAs.  On the way out thread 0's acquire, the second CTA
@@ -151,17 +166,14 @@ __device__ bool grid_barrier(const MegaParams& p, const WaitCtl& ctl, int where,
       mbar_expect_tx(smem_u32(&cs.rec_full), (uint32_t)sizeof(Stage));
       bulk_load(smem_u32(&cs.stage), p.stages + where + 1, (uint32_t)sizeof(Stage), smem_u32(&cs.rec_full));
     }
-    uint32_t spins = 0;
-    while (!skip && ld_acquire_u32(count) < target) {
-      if (((++spins) & 0x3F) == 0) {
-        if (*ctl.abort_smem) break;
-        if (globaltimer_ns() > ctl.deadline_ns) {
-          record_timeout(ctl, DEV_TIMEOUT_GRID, where);
-          break;
-        }
-      }
+    if (!skip) {
+      bool there = ld_acquire_u32(count) >= target;
+#pragma unroll
+      for (int i = 0; i < 7; ++i)
+        if (!there) there = ld_acquire_u32(count) >= target;
+      if (!there) grid_wait_loop(count, target, ctl, where);
     }
-    if (fetch) mbar_wait(smem_u32(&cs.rec_full), (uint32_t)where & 1u, ctl, 50);
+    if (fetch) mbar_wait_hot(smem_u32(&cs.rec_full), (uint32_t)where & 1u, ctl, 50);
   }
   __syncthreads();
   fence_proxy_async_global();     // the other CTAs' global writes (acquired above) before this CTA's TMA and bulk-copy reads
