@@ -19,7 +19,7 @@
 //   st.async: the store itself counts as a transfer on the receiver's mbarrier, no fence on either side), and every cell
 //   warp waits for them itself: there is no CTA barrier in the step.
 // A step of hidden 256 takes 2.4 k cycles (hidden 64: 1.5 k); with the products on the CUDA cores (128 conversions and FMAs per thread, partial sums by
-// shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps 228 -> 161 us, 12 x 64 x 200 266 -> 180 us.
+// shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps 228 -> 159 us, 12 x 64 x 200 266 -> 178 us.
 // Only the hop to the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
 // Every CTA of a layer publishes its own count of finished steps; the consumer checks all eight, so a CTA whose
 // publication lags cannot be covered by its peers running ahead.
@@ -60,22 +60,11 @@ struct LstmParams {
   unsigned long long timeout_ns;
 };
 
-// Both forms are evaluated without a branch: a step is one dependent chain, and its lanes differ.
-// ex2-based sigmoid: absolute error of about 1e-7.
-__device__ __forceinline__ float sigmoid_f(float v) { return __fdividef(1.0f, 1.0f + __expf(-v)); }
-// tanh = 2 sigmoid(2 v) - 1 keeps only the absolute error, which small arguments (hidden states of deep layers) feel: they
-// take the Taylor series, whose first term left out is below 1e-8 of the result for |v| < 1/4.
-__device__ __forceinline__ float tanh_taylor(float v) {
-  const float q = v * v;
-  float r = fmaf(q, 62.0f / 2835.0f, -17.0f / 315.0f);
-  r = fmaf(q, r, 2.0f / 15.0f);
-  r = fmaf(q, r, -1.0f / 3.0f);
-  return fmaf(v * q, r, v);
-}
-// sigmoid(v), or tanh(v) where is_tanh
+// sigmoid(v) = 1 / (1 + e^-v), or tanh(v) = 1 - 2 / (1 + e^2v) where is_tanh: ex2-based, absolute error of a few 1e-7 on values
+// in [-1, 1].  No branch: a step is one dependent chain, and its lanes differ.
 __device__ __forceinline__ float gate_f(float v, bool is_tanh) {
-  const float s = sigmoid_f(is_tanh ? 2.0f * v : v), t = tanh_taylor(v), w = fmaf(2.0f, s, -1.0f);
-  return is_tanh ? (fabsf(v) < 0.25f ? t : w) : s;
+  const float r = __fdividef(is_tanh ? 2.0f : 1.0f, 1.0f + __expf(is_tanh ? 2.0f * v : -v));
+  return is_tanh ? 1.0f - r : r;
 }
 
 // Bounded wait of a whole warp on an mbarrier; every lane sees the phase itself.  kCluster: its transfers come from other
