@@ -23,14 +23,15 @@ def test_quotients_are_exact(res, win, rows):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("res,window,shift", [(256, 8, 3), (8, 8, 0), (21, 7, 2)])
-def test_block_on_grids_at_the_ends_of_the_range(res, window, shift):
-    """256 x 256 tokens: no exact 32-bit multiplier; one window; an odd number of windows per side."""
+@pytest.mark.parametrize("res,window,shift,dim", [(256, 8, 3, 128), (8, 8, 0, 128), (21, 7, 2, 128), (35, 7, 3, 256), (7, 7, 0, 1024)])
+def test_block_on_grids_at_the_ends_of_the_range(res, window, shift, dim):
+    """256 x 256 tokens: no exact 32-bit multiplier; one window; odd numbers of windows, with one (window, head) per
+    attention item (9 x 4, 1 x 32 problems) and with two by two (25 x 8: the last item has a single window)."""
     from souffle_models_b200 import swin
-    cfg = so.SwinConfig(res=res, dim=128, heads=4, window=window)
+    cfg = so.SwinConfig(res=res, dim=dim, heads=dim // 32, window=window)
     p = so.make_swin_params(cfg, 5, zero_bias=False)
-    x = torch.randn(res * res, 128, generator=torch.Generator().manual_seed(res)).half()
-    blk = swin.SwinBlock(1, res, 128, 4, window, shift, {k: v.cuda() for k, v in p.items()})
+    x = torch.randn(res * res, dim, generator=torch.Generator().manual_seed(res)).half()
+    blk = swin.SwinBlock(1, res, dim, dim // 32, window, shift, {k: v.cuda() for k, v in p.items()})
     y = blk.forward(x.cuda())
     blk.status()
     want = so.swin_block(cfg, x, p, shift)
