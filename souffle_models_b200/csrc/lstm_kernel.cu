@@ -22,7 +22,9 @@
 // shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps 228 -> 159 us, 12 x 64 x 200 266 -> 178 us.
 // Only the hop to the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
 // Every CTA of a layer publishes its own count of finished steps; the consumer checks all eight, so a CTA whose
-// publication lags cannot be covered by its peers running ahead.
+// publication lags cannot be covered by its peers running ahead.  The same holds inside a CTA: a warp sends h(t) to the
+// cluster before it has stored it to global memory, so its peers may be a step further on while that store is still on its
+// way; every cell warp therefore counts its own stored steps, and what the CTA publishes is the smallest of the counts.
 // Two more warps keep that hop off the cell arithmetic's path: a fetch warp brings the layer's input
 // vectors into shared memory up to four steps ahead, and a publish warp pays for the release fence
 // behind the hidden states the cell warps have stored.
@@ -161,7 +163,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   __shared__ float x_scale[kLstmXBufs];
   __shared__ uint64_t bars[2 * kLstmXBufs + 2];
   __shared__ int abort_w;
-  __shared__ unsigned produced_w;               // hidden states this CTA has stored to global memory
+  __shared__ uint32_t stored_s[kWarps];         // steps whose hidden states a cell warp has stored to global memory
   const int L = p.layers, T = p.steps;
   const uint32_t xfull0 = smem_u32(bars), xempty0 = smem_u32(bars + kLstmXBufs), hfull0 = smem_u32(bars + 2 * kLstmXBufs);
   const int layer = blockIdx.x / kLstmParts;
@@ -170,7 +172,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
 
   if (tid == 0) {
     abort_w = 0;
-    produced_w = 0;
+    for (int i = 0; i < kWarps; ++i) stored_s[i] = 0;
     for (int i = 0; i < kLstmXBufs; ++i) {
       mbar_init(xfull0 + 8 * i, 32);            // the 32 lanes of the fetch warp
       mbar_init(xempty0 + 8 * i, kWarps);       // one lane of every cell warp
@@ -194,21 +196,25 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
 
   if (warp == kWarps + 1) {
     // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
-    if (lane == 0) {
-      const uint32_t produced_a = smem_u32(&produced_w);
-      uint32_t published = 0, spins = 0;
-      while (published < (uint32_t)T) {
-        const uint32_t n = ld_acquire_cta_shared_u32(produced_a) / (uint32_t)U;     // whole steps only
-        if (n > published) {
-          st_release_u32(p.done + layer * kLstmParts + part, n);      // this CTA's units of steps < n are in h_all
-          published = n;
-        } else if (((++spins) & 0xFF) == 0) {
-          if (*ctl.abort_smem) break;
-          if (globaltimer_ns() > ctl.deadline_ns) {
+    const uint32_t stored_a = smem_u32(stored_s + (lane & (kWarps - 1)));
+    uint32_t published = 0, spins = 0;
+    while (published < (uint32_t)T) {
+      const uint32_t n = __reduce_min_sync(0xffffffffu, ld_acquire_cta_shared_u32(stored_a));
+      if (n > published) {
+        __syncwarp();                           // every lane's acquire is in front of lane 0's release, which covers them all
+        if (lane == 0) st_release_u32(p.done + layer * kLstmParts + part, n);     // this CTA's units of steps < n are in h_all
+        published = n;
+      } else if (((++spins) & 0xFF) == 0) {
+        int give_up = 0;
+        if (lane == 0) {
+          if (*ctl.abort_smem) {
+            give_up = 1;
+          } else if (globaltimer_ns() > ctl.deadline_ns) {
             record_timeout(ctl, DEV_TIMEOUT_FLAG, 950);
-            break;
+            give_up = 1;
           }
         }
+        if (__shfl_sync(0xffffffffu, give_up, 0)) break;
       }
     }
     __syncwarp();
@@ -335,7 +341,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     const int send_part = lane >> 3;
     const uint32_t send_to = map_shared_rank(smem_u32(&h_s[0][(send_part < 3 ? send_part : 0) * kRow + unit0]), (uint32_t)(lane & 7));
     const uint32_t send_bar = map_shared_rank(hfull0, (uint32_t)(lane & 7));
-    const uint32_t produced_a = smem_u32(&produced_w);
+    const uint32_t stored_a = smem_u32(stored_s + warp);
     float c_state = 0.0f;                       // cell state of `unit` (the same value in its eight lanes)
     float cx[4];                                // W_in x(t), scaled back
     bool ok = true;
@@ -396,7 +402,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         const float4 h4 = make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
         __stcg(reinterpret_cast<float4*>(p.h_all + ((size_t)layer * T + t) * H + unit0), h4);
         if (layer == L - 1) *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) = h4;
-        red_add_release_cta_shared_u32(produced_a, 4u);   // the publish warp takes it from here
+        st_release_cta_shared_u32(stored_a, (uint32_t)t + 1u);      // the publish warp takes it from here
       }
       if (t + 1 < T) input_half(t + 1);
     }

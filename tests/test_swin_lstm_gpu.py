@@ -120,6 +120,29 @@ def test_lstm_infinities_and_nan_stay_in_their_step():
     assert torch.isfinite(y[0, :3]).all() and torch.isnan(y[0, 3:]).all()
 
 
+def test_lstm_next_to_memory_traffic_reads_no_earlier_call():
+    """The layers hand hidden states on through memory that keeps the previous call's values.  With copies on another
+    stream holding that memory up, and inputs that change from call to call, every call returns what a quiet one returns."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(21)
+    L, H, T = 10, 256, 60
+    w = [((torch.rand(4 * L, H, H, generator=g) - 0.5) * 0.5).half().cuda() for _ in range(2)]
+    xs = [torch.randn(1, T, H, generator=g).cuda() for _ in range(2)]
+    plan = lstm.LstmStack(w[0], w[1], T)
+    want = [plan.forward(x).clone() for x in xs]
+    plan.status()
+    assert not torch.equal(*want)
+    src, dst, side = torch.empty(1 << 28, device="cuda"), torch.empty(1 << 28, device="cuda"), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    got = []
+    for k in range(60):
+        got.append(plan.forward(xs[k & 1]).clone())
+        with torch.cuda.stream(side):
+            dst.copy_(src)
+    plan.status()
+    assert all(torch.equal(y, want[k & 1]) for k, y in enumerate(got))
+
+
 def test_fused_lstm_drop_in_signature():
     from souffle_models_b200 import lstm
     x, w_in, w_st = so.make_lstm_params()
