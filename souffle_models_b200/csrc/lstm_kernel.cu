@@ -30,7 +30,9 @@
 // behind the hidden states the cell warps have stored.
 // There is no grid-wide barrier.  All waits in the step loop are bounded; on expiry the CTA records a
 // status word, leaves the loop and waits for its cluster at the final cluster barrier (shared
-// memory must outlive the peers' remote stores).
+// memory must outlive the peers' remote stores).  That barrier does not cover the stores themselves: st.async completes on
+// the receiver's mbarrier only.  So nothing is sent that is not waited for (the last hidden state stays at home), and a CTA
+// that gave up on a wait stays a while longer for whatever is still on its way to it.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -179,7 +181,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     }
     for (int i = 0; i < 2; ++i) {               // h(0) and h(1): one local arrival that announces the bytes of a vector
       mbar_init(hfull0 + 8 * i, 1);
-      mbar_expect_tx(hfull0 + 8 * i, kStepBytes);
+      if (i + 1 < T) mbar_expect_tx(hfull0 + 8 * i, kStepBytes);       // h(T - 1) is not sent
     }
     fence_mbar_init();
   }
@@ -363,7 +365,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         ok = lstm_wait_warp<true>(hfull0 + 8 * (hb ^ 1), (uint32_t)((t - 1) >> 1) & 1u, ctl, 800 + layer, lane);
         if (!ok) break;
         // that barrier's next phase receives h(t+1); nobody sends it before having this warp's h(t)
-        if (tid == 0 && t + 1 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), kStepBytes);
+        if (tid == 0 && t + 2 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), kStepBytes);
       }
       float ch[4];
       lstm_product<H, H / 32>(wh, wx_rest, 0, h_s[hb ^ 1], lane, ch);
@@ -394,7 +396,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
       uint32_t got[4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) got[i] = __shfl_sync(0xffffffffu, offer, 4 * i + send_part);
-      if (lane < 24) {
+      if (lane < 24 && t + 1 < T) {             // the last one has no reader in the cluster
         const uint64_t word = (uint64_t)(got[0] | (got[1] << 16)) | ((uint64_t)(got[2] | (got[3] << 16)) << 32);
         st_async_b64(send_to + (uint32_t)(hb * 3 * kRow * 2), word, send_bar + 8u * (uint32_t)hb);
       }
@@ -411,6 +413,10 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();
   cluster_sync_all();
+  if (*ctl.abort_smem) {                        // sent by peers before they came here, and not waited for: 200 us are ample
+    const unsigned long long t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
+  }
 }
 
 }  // namespace souffle

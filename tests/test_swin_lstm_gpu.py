@@ -63,6 +63,21 @@ def test_lstm_matches_oracle(layers, hidden, steps):
         assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("layers,hidden", [(1, 256), (12, 64), (4, 128)])
+@pytest.mark.parametrize("steps", [1, 2, 3, 4])
+def test_lstm_short_sequences(layers, hidden, steps):
+    """The last hidden state is not sent round the cluster: one step sends none, two and three use one and both buffers
+    once.  Bounds of test_lstm_matches_oracle."""
+    from souffle_models_b200 import lstm
+    x, w_in, w_st = so.make_lstm_params(layers, hidden, steps, seed=77)
+    plan = lstm.LstmStack(w_in.cuda(), w_st.cuda(), steps)
+    want = so.lstm_forward(x, w_in, w_st)
+    for _ in range(3):
+        y = plan.forward(x.float().cuda())
+        plan.status()
+        assert ((y.cpu() - want).abs() <= 2e-5 + 1e-3 * want.abs()).all()
+
+
 def test_lstm_larger_weights_and_bias():
     """Weights large enough that the state does not vanish through the stack."""
     from souffle_models_b200 import lstm
