@@ -31,12 +31,14 @@
 // There is no grid-wide barrier.  All waits in the step loop are bounded; on expiry the CTA records a
 // status word, leaves the loop and waits for its cluster at the final cluster barrier (shared
 // memory must outlive the peers' remote stores).  That barrier does not cover the stores themselves: st.async completes on
-// the receiver's mbarrier only.  So nothing is sent that is not waited for (the last hidden state stays at home), and a CTA
-// that gave up on a wait stays a while longer for whatever is still on its way to it.
+// the receiver's mbarrier only.  So every hidden vector is waited for, the last one too, which nobody reads, and a CTA that
+// gave up on a wait stays a while longer for whatever is still on its way to it.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <type_traits>
 
 #include "sm100_ptx.cuh"
 
@@ -72,18 +74,20 @@ __device__ __forceinline__ float gate_f(float v, bool is_tanh) {
 }
 
 // Bounded wait of a whole warp on an mbarrier; every lane sees the phase itself.  kCluster: its transfers come from other
-// CTAs of the cluster.
+// CTAs of the cluster.  `stop` (0: none) is the address of a shared word: once it is set, a wait whose phase is not
+// complete by then ends as well.
 template <bool kCluster>
 __device__ __forceinline__ bool lstm_try(uint32_t bar, uint32_t parity) {
   if constexpr (kCluster) return mbar_try_wait_cluster(bar, parity);
   else return mbar_try_wait(bar, parity);
 }
 template <bool kCluster>
-__device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const WaitCtl& c, int where) {
+__device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, uint32_t stop) {
   uint32_t spins = 0;
   while (!lstm_try<kCluster>(bar, parity)) {
     if (((++spins) & 0xFF) == 0) {
       if (*c.abort_smem) return false;
+      if (stop && ld_acquire_cta_shared_u32(stop)) return lstm_try<kCluster>(bar, parity);
       if (globaltimer_ns() > c.deadline_ns) {
         record_timeout(c, DEV_TIMEOUT_MBAR, where);
         return false;
@@ -93,11 +97,11 @@ __device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, co
   return true;
 }
 template <bool kCluster>
-__device__ __forceinline__ bool lstm_wait_warp(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, int lane) {
+__device__ __forceinline__ bool lstm_wait_warp(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, int lane, uint32_t stop = 0) {
   if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
   if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
   int ok = 1;
-  if (lane == 0) ok = lstm_wait_loop<kCluster>(bar, parity, c, where) ? 1 : 0;
+  if (lane == 0) ok = lstm_wait_loop<kCluster>(bar, parity, c, where, stop) ? 1 : 0;
   if (__shfl_sync(0xffffffffu, ok, 0) == 0) return false;
   return __all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity));       // complete: lane 0 has seen it
 }
@@ -149,58 +153,213 @@ __device__ __forceinline__ void lstm_product(const uint4 (&w)[2][kReg], const ui
   for (int i = 0; i < 4; ++i) out[i] = (acc[0][i] + acc[1][i]) + (acc[2][i] + acc[3][i]);
 }
 
-// H = 64, 128 or 256 (= p.hidden).
+// The parts of a vector end 2^-61 below its largest element.  Where that may be large enough for a gate to notice (from
+// 2^20 on: the large elements' own weights may be zero), and for infinities and NaN, which have no scale, the caller's vector
+// goes to the cell warps in pieces, largest elements first, whose products add up: a piece takes the elements within 2^37
+// of its largest, all of whose 24 bits the parts hold.  The first such vector moves the cell warps of its layer to a step loop of
+// their own: one more branch in the loop that all others run made a step 150 cycles longer (1 x 256 x 200: 232 -> 248 us).
+constexpr uint32_t kLstmWide = 127u + 20u;           // biased exponent of 2^20
+constexpr uint32_t kLstmPieceRange = 37u;
+
+// What the warps of a CTA share.
 template <int H>
-__global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const LstmParams p) {
-  constexpr int U = H / kLstmParts;             // units owned by this CTA
-  constexpr int kWarps = H / 32;                // cell warps: four units each
-  constexpr int kRow = lstm_row(H);
-  constexpr uint32_t kStepBytes = 6u * H;       // a hidden vector: three fp16 parts
-  __shared__ __align__(16) __half x_s[kLstmXBufs][3 * kRow];      // input vectors
-  __shared__ __align__(16) __half h_s[2][3 * kRow];               // hidden vectors, written by the whole cluster
+struct LstmShared {
+  static constexpr int kWarps = H / 32;         // cell warps: four units each
+  static constexpr int kRow = lstm_row(H);
   // Hidden 256: a cell thread's weights are 128 registers of the 168 that ten warps leave it (registers are handed out per
   // four warps); two blocks of the input half stay in shared memory instead.
-  constexpr int kXReg = H == 256 ? 6 : H / 32;
-  __shared__ uint4 wx_rest[H == 256 ? 2 * (H / 32 - kXReg) * kWarps * 32 : 1];
-  __shared__ float x_scale[kLstmXBufs];
-  __shared__ uint64_t bars[2 * kLstmXBufs + 2];
-  __shared__ int abort_w;
-  __shared__ uint32_t stored_s[kWarps];         // steps whose hidden states a cell warp has stored to global memory
+  static constexpr int kXReg = H == 256 ? 6 : H / 32;
+  alignas(16) __half x[kLstmXBufs][3 * kRow];   // input vectors
+  alignas(16) __half h[2][3 * kRow];            // hidden vectors, written by the whole cluster
+  uint4 wx_rest[H == 256 ? 2 * (H / 32 - kXReg) * kWarps * 32 : 1];
+  float x_scale[kLstmXBufs];                    // takes the products back to the vector's scale; negative: another piece follows
+  uint64_t x_full[kLstmXBufs], x_empty[kLstmXBufs], h_full[2], pieces_ready;
+  unsigned long long deadline_ns;
+  int abort;
+  uint32_t pieces;                              // 1: from the next input vector on, vectors come in pieces
+  int piece[kWarps];                            // then: pieces a cell warp has multiplied so far
+  uint32_t stored[kWarps];                      // steps whose hidden states a cell warp has stored to global memory
+};
+
+// The cell arithmetic of all steps from t on (c_state: the cell state, before step t, of the lane's unit: the same value in its
+// eight lanes); both are brought up to date.
+// kPieces: input vectors may come in several pieces; without, the loop ends (false) in front of the first step whose vector
+// does.  False with the abort flag set: a wait has run out.
+template <int H, bool kPieces>
+__device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& sh, const WaitCtl& ctl, int layer, int part, int tid,
+                                           int& t, float& c_state) {
+  constexpr int U = H / kLstmParts, kWarps = LstmShared<H>::kWarps, kRow = LstmShared<H>::kRow, kXReg = LstmShared<H>::kXReg;
+  constexpr uint32_t kStepBytes = 6u * H;
+  const int L = p.layers, T = p.steps, warp = tid >> 5, lane = tid & 31;
+  const uint32_t xfull0 = smem_u32(sh.x_full), xempty0 = smem_u32(sh.x_empty), hfull0 = smem_u32(sh.h_full);
+  // Rows of a warp's tile: row r < 8 is gate r / 4 (i, j) of unit r % 4, row 8 + r gate 2 + r / 4 (f, o).  So lane 4 g + q
+  // meets the sums of gates g / 4 and 2 + g / 4 of unit g % 4: q = 0 finishes the first, q = 1 the second.
+  const int g = lane >> 2, q = lane & 3, unit0 = part * U + warp * 4, unit = unit0 + (g & 3);
+  const float bias_u = p.bias ? p.bias[layer * H + unit] : 0.0f;
+  const float bias_g = bias_u + (q == 1 && g < 4 ? 1.0f : 0.0f);       // the forget gate's + 1
+  const bool is_tanh = q == 0 && g >= 4;                               // gate j
+  uint4 wx[2][kXReg], wh[2][H / 32];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const size_t row = ((size_t)(layer * 4 + 2 * r + (g >> 2)) * H + unit) * H + q * 8;
+#pragma unroll
+    for (int b = 0; b < H / 32; ++b) {
+      const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.w_in + row + b * 32));
+      if (b < kXReg) wx[r][b < kXReg ? b : 0] = w;
+      else sh.wx_rest[(2 * (b - kXReg) + r) * kWarps * 32 + tid] = w;          // read by this thread only
+      wh[r][b] = __ldg(reinterpret_cast<const uint4*>(p.w_state + row + b * 32));
+    }
+  }
+  // lane 8 k + d sends part k of the warp's four hidden states to CTA d; lane 24 stores them to global memory
+  const int send_part = lane >> 3;
+  const uint32_t send_to = map_shared_rank(smem_u32(&sh.h[0][(send_part < 3 ? send_part : 0) * kRow + unit0]), (uint32_t)(lane & 7));
+  const uint32_t send_bar = map_shared_rank(hfull0, (uint32_t)(lane & 7));
+  const uint32_t stored_a = smem_u32(sh.stored + warp);
+  float cx[4];                                // W_in x(t), scaled back
+  bool ok = true;
+  auto input_half = [&](int step) {
+    if constexpr (!kPieces) {
+      const int xb = step % kLstmXBufs;
+      ok = lstm_wait_warp<false>(xfull0 + 8 * xb, (uint32_t)(step / kLstmXBufs) & 1u, ctl, 910, lane, smem_u32(&sh.pieces));
+      if (!ok) return;
+      lstm_product<H, kXReg>(wx, sh.wx_rest + (H == 256 ? tid : 0), kWarps * 32, sh.x[xb], lane, cx);
+      const float down = sh.x_scale[xb];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cx[i] *= down;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(xempty0 + 8 * xb);       // this warp has read x(step)
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) cx[i] = 0.0f;
+      bool more = true;
+      while (more) {
+        const int piece = *const_cast<volatile int*>(sh.piece + warp), xb = piece % kLstmXBufs;
+        ok = lstm_wait_warp<false>(xfull0 + 8 * xb, (uint32_t)(piece / kLstmXBufs) & 1u, ctl, 910, lane);
+        if (!ok) return;
+        float px[4];
+        lstm_product<H, kXReg>(wx, sh.wx_rest + (H == 256 ? tid : 0), kWarps * 32, sh.x[xb], lane, px);
+        const float down = sh.x_scale[xb];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) cx[i] = fmaf(px[i], fabsf(down), cx[i]);
+        more = __any_sync(0xffffffffu, down < 0.0f);
+        if (lane == 0) {
+          sh.piece[warp] = piece + 1;
+          mbar_arrive(xempty0 + 8 * xb);
+        }
+        __syncwarp();
+      }
+    }
+  };
+  input_half(t);
+  for (; ok && t < T; ++t) {
+    const int hb = t & 1;                               // h(t) goes to sh.h[hb]; h(t-1) is in sh.h[hb ^ 1]
+    if (t > 0) {
+      ok = lstm_wait_warp<true>(hfull0 + 8 * (hb ^ 1), (uint32_t)((t - 1) >> 1) & 1u, ctl, 800 + layer, lane);
+      if (!ok) break;
+      // that barrier's next phase receives h(t+1); nobody sends it before having this warp's h(t)
+      if (tid == 0 && t + 1 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), kStepBytes);
+    }
+    float ch[4];
+    lstm_product<H, H / 32>(wh, sh.wx_rest, 0, sh.h[hb ^ 1], lane, ch);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) ch[i] = fmaf(ch[i], 1.0f / kLstmHScale, cx[i]);
+    // columns 0, 1 (lane q = 0) and 2 (q = 1) are the three parts of the vector
+    const float first = q == 0 ? fmaf(ch[1], 1.0f / kLstmPart, ch[0]) : ch[0] * (1.0f / (kLstmPart * kLstmPart));
+    const float second = q == 0 ? fmaf(ch[3], 1.0f / kLstmPart, ch[2]) : ch[2] * (1.0f / (kLstmPart * kLstmPart));
+    const float other = __shfl_xor_sync(0xffffffffu, q == 0 ? second : first, 1);
+    const float pre = (q == 0 ? first : second) + other + bias_g;
+    const float act = gate_f(pre, is_tanh);
+    const int base = 4 * (g & 3);
+    const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
+    const float gj = __shfl_sync(0xffffffffu, act, base + 16), go = __shfl_sync(0xffffffffu, act, base + 17);
+    c_state = c_state * gf + gi * gj;
+    const float h = gate_f(c_state, true) * go;
+    // lanes 4 u .. 4 u + 3 offer the three parts of unit u's hidden state and the fp32 value itself; lane 8 k + d collects
+    // offer k of all four units
+    uint32_t offer;
+    {
+      const float s0 = h * kLstmHScale;
+      const __half hi = __float2half_rn(s0);
+      const float s1 = (s0 - __half2float(hi)) * kLstmPart;
+      const __half mid = __float2half_rn(s1);
+      const __half lo = __float2half_rn((s1 - __half2float(mid)) * kLstmPart);
+      offer = q == 0 ? __half_as_ushort(hi) : q == 1 ? __half_as_ushort(mid) : q == 2 ? __half_as_ushort(lo) : __float_as_uint(h);
+    }
+    uint32_t got[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) got[i] = __shfl_sync(0xffffffffu, offer, 4 * i + send_part);
+    if (lane < 24) {
+      const uint64_t word = (uint64_t)(got[0] | (got[1] << 16)) | ((uint64_t)(got[2] | (got[3] << 16)) << 32);
+      st_async_b64(send_to + (uint32_t)(hb * 3 * kRow * 2), word, send_bar + 8u * (uint32_t)hb);
+    }
+    if (lane == 24) {
+      const float4 h4 = make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
+      __stcg(reinterpret_cast<float4*>(p.h_all + ((size_t)layer * T + t) * H + unit0), h4);
+      if (layer == L - 1) *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) = h4;
+      st_release_cta_shared_u32(stored_a, (uint32_t)t + 1u);      // the publish warp takes it from here
+    }
+    if (t + 1 < T) input_half(t + 1);
+  }
+  // h(T - 1) has no reader, but it has to be here before this CTA's shared memory goes (not to send it would take a condition
+  // in every step: 10 x 256 x 100 161.4 us against 156.6, 1 x 256 x 200 233.6 against 227.5)
+  if (ok) ok = lstm_wait_warp<true>(hfull0 + 8 * ((T - 1) & 1), (uint32_t)((T - 1) >> 1) & 1u, ctl, 930, lane);
+  return ok;
+}
+// Out of line: rare, and inlined its registers would be taken from the loop above.
+template <int H>
+__device__ __noinline__ void lstm_steps_in_pieces(const LstmParams& p, LstmShared<H>& sh, float c_state) {
+  int t = *const_cast<volatile int*>(sh.piece + (threadIdx.x >> 5));       // every vector before this one came whole
+  WaitCtl ctl;
+  ctl.abort_smem = &sh.abort;
+  ctl.status_g = p.status;
+  ctl.deadline_ns = sh.deadline_ns;
+  lstm_steps<H, true>(p, sh, ctl, blockIdx.x / kLstmParts, (int)cluster_cta_rank(), threadIdx.x, t, c_state);
+}
+
+// H = 64, 128 or 256 (= p.hidden).
+template <int H>
+__global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const __grid_constant__ LstmParams p) {
+  constexpr int kWarps = LstmShared<H>::kWarps, kRow = LstmShared<H>::kRow;
+  constexpr uint32_t kStepBytes = 6u * H;       // a hidden vector: three fp16 parts
+  __shared__ LstmShared<H> sh;
   const int L = p.layers, T = p.steps;
-  const uint32_t xfull0 = smem_u32(bars), xempty0 = smem_u32(bars + kLstmXBufs), hfull0 = smem_u32(bars + 2 * kLstmXBufs);
+  const uint32_t xfull0 = smem_u32(sh.x_full), xempty0 = smem_u32(sh.x_empty), hfull0 = smem_u32(sh.h_full);
   const int layer = blockIdx.x / kLstmParts;
   const int part = (int)cluster_cta_rank();     // == blockIdx.x % kLstmParts for clusters along x
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (tid == 0) {
-    abort_w = 0;
-    for (int i = 0; i < kWarps; ++i) stored_s[i] = 0;
+    sh.abort = 0;
+    sh.deadline_ns = globaltimer_ns() + p.timeout_ns;
+    sh.pieces = 0;
+    for (int i = 0; i < kWarps; ++i) sh.stored[i] = 0;
     for (int i = 0; i < kLstmXBufs; ++i) {
       mbar_init(xfull0 + 8 * i, 32);            // the 32 lanes of the fetch warp
       mbar_init(xempty0 + 8 * i, kWarps);       // one lane of every cell warp
     }
+    mbar_init(smem_u32(&sh.pieces_ready), kWarps);            // one lane of every cell warp
     for (int i = 0; i < 2; ++i) {               // h(0) and h(1): one local arrival that announces the bytes of a vector
       mbar_init(hfull0 + 8 * i, 1);
-      if (i + 1 < T) mbar_expect_tx(hfull0 + 8 * i, kStepBytes);       // h(T - 1) is not sent
+      mbar_expect_tx(hfull0 + 8 * i, kStepBytes);
     }
     fence_mbar_init();
   }
   if (blockIdx.x == 0)
     for (int i = tid; i < L * kLstmParts; i += lstm_block(H)) p.done_next[i] = 0u;
-  for (int i = tid; i < 2 * 3 * kRow; i += lstm_block(H)) (&h_s[0][0])[i] = __ushort_as_half(0);    // h before the first step
+  for (int i = tid; i < 2 * 3 * kRow; i += lstm_block(H)) (&sh.h[0][0])[i] = __ushort_as_half(0);    // h before the first step
   __syncthreads();
   cluster_sync_all();                           // every CTA's barriers exist before anyone arrives on them
 
   WaitCtl ctl;
-  ctl.abort_smem = &abort_w;
+  ctl.abort_smem = &sh.abort;
   ctl.status_g = p.status;
-  ctl.deadline_ns = globaltimer_ns() + p.timeout_ns;
+  ctl.deadline_ns = sh.deadline_ns;
 
   if (warp == kWarps + 1) {
     // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
-    const uint32_t stored_a = smem_u32(stored_s + (lane & (kWarps - 1)));
+    const uint32_t stored_a = smem_u32(sh.stored + (lane & (kWarps - 1)));
     uint32_t published = 0, spins = 0;
-    while (published < (uint32_t)T) {
+    while (layer + 1 < L && published < (uint32_t)T) {      // nobody reads the top layer's count
       const uint32_t n = __reduce_min_sync(0xffffffffu, ld_acquire_cta_shared_u32(stored_a));
       if (n > published) {
         __syncwarp();                           // every lane's acquire is in front of lane 0's release, which covers them all
@@ -243,12 +402,38 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         v[i + 1] = f.y;
       }
     };
+    // vector or piece number n of this CTA: the wait for its slot, and its way into it
+    auto slot_free = [&](int n) -> int {
+      const int xb = n % kLstmXBufs, use = n / kLstmXBufs;
+      if (use == 0) return 1;
+      int free = 1;
+      if (lane == 0) free = mbar_wait(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900) ? 1 : 0;
+      free = __shfl_sync(0xffffffffu, free, 0);
+      __syncwarp();
+      return free;
+    };
+    auto hand_over = [&](int n, const float (&val)[E], float up, float down) {
+      const int xb = n % kLstmXBufs;
+      __half hi[E], mid[E], lo[E];
+#pragma unroll
+      for (int i = 0; i < E; ++i) lstm_split(val[i] * up, hi[i], mid[i], lo[i]);
+#pragma unroll
+      for (int i = 0; i < E; i += 2) {
+        __half* dst = sh.x[xb] + lane * E + i;
+        *reinterpret_cast<__half2*>(dst) = __halves2half2(hi[i], hi[i + 1]);
+        *reinterpret_cast<__half2*>(dst + kRow) = __halves2half2(mid[i], mid[i + 1]);
+        *reinterpret_cast<__half2*>(dst + 2 * kRow) = __halves2half2(lo[i], lo[i + 1]);
+      }
+      if (lane == 0) sh.x_scale[xb] = down;
+      mbar_arrive(xfull0 + 8 * xb);             // release: this lane's stores are visible to whoever waits
+    };
     float v[E], ahead[E];
 #pragma unroll
     for (int i = 0; i < E; ++i) ahead[i] = 0.0f;
     bool have = false;                          // `v` holds step t already
+    int piece = 0;                              // layer 0: pieces handed over so far (the steps so far, unless one had several)
+    bool in_pieces = false;                     // the cell warps expect several
     for (int t = 0; t < T; ++t) {
-      const int xb = t % kLstmXBufs, use = t / kLstmXBufs;
       int ok = 1;
       if ((unsigned)t >= avail) {
         // lanes read the counter of one CTA of the layer below each; the smallest counts
@@ -277,138 +462,70 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
       if (ok && !have) load_vector(t, v);
       const bool next = t + 1 < T && (unsigned)(t + 1) < avail;
       if (ok && next) load_vector(t + 1, ahead);
-      if (ok && use > 0) {
-        if (lane == 0) ok = mbar_wait(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900) ? 1 : 0;
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        __syncwarp();
+      if (layer > 0) {
+        if (ok) ok = slot_free(t);
+        if (ok) hand_over(t, v, kLstmHScale, 1.0f / kLstmHScale);        // hidden states: a constant scale
+      }
+      for (bool more = layer == 0; more && ok;) {
+        // power-of-two scale that takes the piece's largest element into the upper range of fp16
+        uint32_t m = 0;
+#pragma unroll
+        for (int i = 0; i < E; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
+        m = __reduce_max_sync(0xffffffffu, m);
+        uint32_t e = m >> 23, least = 0;        // biased exponents: of the largest element, of the smallest this piece takes
+        more = false;
+        if (e >= kLstmWide) {
+          least = e == 255u ? 255u : e - kLstmPieceRange;
+          bool rest = false;
+#pragma unroll
+          for (int i = 0; i < E; ++i) rest = rest || (v[i] != 0.0f && ((__float_as_uint(v[i]) >> 23) & 255u) < least);
+          more = __any_sync(0xffffffffu, rest);
+          if (more && !in_pieces) {             // the cell warps have to expect it: they stop in front of this vector
+            if (lane == 0) {
+              st_release_cta_shared_u32(smem_u32(&sh.pieces), 1u);
+              ok = mbar_wait(smem_u32(&sh.pieces_ready), 0u, ctl, 920) ? 1 : 0;
+            }
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            in_pieces = true;
+          }
+        }
+        float up = 1.0f, down = 1.0f;           // an infinity or NaN passes through as it is
+        if (e != 255u) {
+          e = e < 15u ? 15u : e;                // 2^-112 and below need no more than the largest scale
+          up = __uint_as_float((268u - e) << 23);        // 2^(14 - (e - 127))
+          down = __uint_as_float((e - 14u) << 23);
+        }
+        float part_v[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) {
+          const bool take = ((__float_as_uint(v[i]) >> 23) & 255u) >= least;
+          part_v[i] = take ? v[i] : 0.0f;
+          if (take) v[i] = 0.0f;
+        }
+        if (ok) ok = slot_free(piece);
+        if (ok) hand_over(piece++, part_v, up, more ? -down : down);
       }
       if (!ok) {
         if (lane == 0) *ctl.abort_smem = 1;
         break;
       }
-      // Power-of-two scale that takes the vector into the upper range of fp16: a constant for hidden states; for the
-      // caller's input from its largest element (none for infinities and NaN, which pass through as they are).
-      float up = kLstmHScale, down = 1.0f / kLstmHScale;
-      if (layer == 0) {
-        uint32_t m = 0;
-#pragma unroll
-        for (int i = 0; i < E; ++i) m = max(m, __float_as_uint(v[i]) & 0x7fffffffu);
-        m = __reduce_max_sync(0xffffffffu, m);
-        uint32_t e = m >> 23;                   // biased exponent
-        if (e == 255u) {
-          up = down = 1.0f;
-        } else {
-          e = e < 15u ? 15u : e;                // 2^-112 and below need no more than the largest scale
-          up = __uint_as_float((268u - e) << 23);        // 2^(14 - (e - 127))
-          down = __uint_as_float((e - 14u) << 23);
-        }
-      }
-      __half hi[E], mid[E], lo[E];
-#pragma unroll
-      for (int i = 0; i < E; ++i) lstm_split(v[i] * up, hi[i], mid[i], lo[i]);
-#pragma unroll
-      for (int i = 0; i < E; i += 2) {
-        __half* dst = x_s[xb] + lane * E + i;
-        *reinterpret_cast<__half2*>(dst) = __halves2half2(hi[i], hi[i + 1]);
-        *reinterpret_cast<__half2*>(dst + kRow) = __halves2half2(mid[i], mid[i + 1]);
-        *reinterpret_cast<__half2*>(dst + 2 * kRow) = __halves2half2(lo[i], lo[i + 1]);
-      }
-      if (lane == 0) x_scale[xb] = down;
-      mbar_arrive(xfull0 + 8 * xb);             // release: this lane's stores are visible to whoever waits
       have = next;
 #pragma unroll
       for (int i = 0; i < E; ++i) v[i] = ahead[i];
     }
   } else {
     // ---------------- cell arithmetic ----------------
-    // Rows of a warp's tile: row r < 8 is gate r / 4 (i, j) of unit r % 4, row 8 + r gate 2 + r / 4 (f, o).  So lane 4 g + q
-    // meets the sums of gates g / 4 and 2 + g / 4 of unit g % 4: q = 0 finishes the first, q = 1 the second.
-    const int g = lane >> 2, q = lane & 3, unit0 = part * U + warp * 4, unit = unit0 + (g & 3);
-    const float bias_u = p.bias ? p.bias[layer * H + unit] : 0.0f;
-    const float bias_g = bias_u + (q == 1 && g < 4 ? 1.0f : 0.0f);       // the forget gate's + 1
-    const bool is_tanh = q == 0 && g >= 4;                               // gate j
-    uint4 wx[2][kXReg], wh[2][H / 32];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const size_t row = ((size_t)(layer * 4 + 2 * r + (g >> 2)) * H + unit) * H + q * 8;
-#pragma unroll
-      for (int b = 0; b < H / 32; ++b) {
-        const uint4 w = __ldg(reinterpret_cast<const uint4*>(p.w_in + row + b * 32));
-        if (b < kXReg) wx[r][b < kXReg ? b : 0] = w;
-        else wx_rest[(2 * (b - kXReg) + r) * kWarps * 32 + tid] = w;          // read by this thread only
-        wh[r][b] = __ldg(reinterpret_cast<const uint4*>(p.w_state + row + b * 32));
+    int t = 0;
+    float c_state = 0.0f;
+    const bool ok = lstm_steps<H, false>(p, sh, ctl, layer, part, tid, t, c_state);
+    if (!ok && *ctl.abort_smem == 0) {          // not given up: vector t comes in pieces, all before it came whole
+      if (lane == 0) {
+        sh.piece[warp] = t;
+        mbar_arrive(smem_u32(&sh.pieces_ready));
       }
-    }
-    // lane 8 k + d sends part k of the warp's four hidden states to CTA d; lane 24 stores them to global memory
-    const int send_part = lane >> 3;
-    const uint32_t send_to = map_shared_rank(smem_u32(&h_s[0][(send_part < 3 ? send_part : 0) * kRow + unit0]), (uint32_t)(lane & 7));
-    const uint32_t send_bar = map_shared_rank(hfull0, (uint32_t)(lane & 7));
-    const uint32_t stored_a = smem_u32(stored_s + warp);
-    float c_state = 0.0f;                       // cell state of `unit` (the same value in its eight lanes)
-    float cx[4];                                // W_in x(t), scaled back
-    bool ok = true;
-    auto input_half = [&](int t) {
-      const int xb = t % kLstmXBufs;
-      ok = lstm_wait_warp<false>(xfull0 + 8 * xb, (uint32_t)(t / kLstmXBufs) & 1u, ctl, 910, lane);
-      if (!ok) return;
-      lstm_product<H, kXReg>(wx, wx_rest + (H == 256 ? tid : 0), kWarps * 32, x_s[xb], lane, cx);
-      const float down = x_scale[xb];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) cx[i] *= down;
       __syncwarp();
-      if (lane == 0) mbar_arrive(xempty0 + 8 * xb);       // this warp has read x(t)
-    };
-    input_half(0);
-    for (int t = 0; ok && t < T; ++t) {
-      const int hb = t & 1;                               // h(t) goes to h_s[hb]; h(t-1) is in h_s[hb ^ 1]
-      if (t > 0) {
-        ok = lstm_wait_warp<true>(hfull0 + 8 * (hb ^ 1), (uint32_t)((t - 1) >> 1) & 1u, ctl, 800 + layer, lane);
-        if (!ok) break;
-        // that barrier's next phase receives h(t+1); nobody sends it before having this warp's h(t)
-        if (tid == 0 && t + 2 < T) mbar_expect_tx(hfull0 + 8 * (hb ^ 1), kStepBytes);
-      }
-      float ch[4];
-      lstm_product<H, H / 32>(wh, wx_rest, 0, h_s[hb ^ 1], lane, ch);
-#pragma unroll
-      for (int i = 0; i < 4; ++i) ch[i] = fmaf(ch[i], 1.0f / kLstmHScale, cx[i]);
-      // columns 0, 1 (lane q = 0) and 2 (q = 1) are the three parts of the vector
-      const float first = q == 0 ? fmaf(ch[1], 1.0f / kLstmPart, ch[0]) : ch[0] * (1.0f / (kLstmPart * kLstmPart));
-      const float second = q == 0 ? fmaf(ch[3], 1.0f / kLstmPart, ch[2]) : ch[2] * (1.0f / (kLstmPart * kLstmPart));
-      const float other = __shfl_xor_sync(0xffffffffu, q == 0 ? second : first, 1);
-      const float pre = (q == 0 ? first : second) + other + bias_g;
-      const float act = gate_f(pre, is_tanh);
-      const int base = 4 * (g & 3);
-      const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
-      const float gj = __shfl_sync(0xffffffffu, act, base + 16), go = __shfl_sync(0xffffffffu, act, base + 17);
-      c_state = c_state * gf + gi * gj;
-      const float h = gate_f(c_state, true) * go;
-      // lanes 4 u .. 4 u + 3 offer the three parts of unit u's hidden state and the fp32 value itself; lane 8 k + d collects
-      // offer k of all four units
-      uint32_t offer;
-      {
-        const float s0 = h * kLstmHScale;
-        const __half hi = __float2half_rn(s0);
-        const float s1 = (s0 - __half2float(hi)) * kLstmPart;
-        const __half mid = __float2half_rn(s1);
-        const __half lo = __float2half_rn((s1 - __half2float(mid)) * kLstmPart);
-        offer = q == 0 ? __half_as_ushort(hi) : q == 1 ? __half_as_ushort(mid) : q == 2 ? __half_as_ushort(lo) : __float_as_uint(h);
-      }
-      uint32_t got[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) got[i] = __shfl_sync(0xffffffffu, offer, 4 * i + send_part);
-      if (lane < 24 && t + 1 < T) {             // the last one has no reader in the cluster
-        const uint64_t word = (uint64_t)(got[0] | (got[1] << 16)) | ((uint64_t)(got[2] | (got[3] << 16)) << 32);
-        st_async_b64(send_to + (uint32_t)(hb * 3 * kRow * 2), word, send_bar + 8u * (uint32_t)hb);
-      }
-      if (lane == 24) {
-        const float4 h4 = make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
-        __stcg(reinterpret_cast<float4*>(p.h_all + ((size_t)layer * T + t) * H + unit0), h4);
-        if (layer == L - 1) *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) = h4;
-        st_release_cta_shared_u32(stored_a, (uint32_t)t + 1u);      // the publish warp takes it from here
-      }
-      if (t + 1 < T) input_half(t + 1);
+      lstm_steps_in_pieces<H>(p, sh, c_state);
     }
-    if (!ok && lane == 0) *ctl.abort_smem = 1;
   }
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();

@@ -66,8 +66,8 @@ def test_lstm_matches_oracle(layers, hidden, steps):
 @pytest.mark.parametrize("layers,hidden", [(1, 256), (12, 64), (4, 128)])
 @pytest.mark.parametrize("steps", [1, 2, 3, 4])
 def test_lstm_short_sequences(layers, hidden, steps):
-    """The last hidden state is not sent round the cluster: one step sends none, two and three use one and both buffers
-    once.  Bounds of test_lstm_matches_oracle."""
+    """The last hidden vector is waited for behind the loop; one, two and three steps use one and both buffers once.  Bounds
+    of test_lstm_matches_oracle."""
     from souffle_models_b200 import lstm
     x, w_in, w_st = so.make_lstm_params(layers, hidden, steps, seed=77)
     plan = lstm.LstmStack(w_in.cuda(), w_st.cuda(), steps)
@@ -95,31 +95,77 @@ def test_lstm_larger_weights_and_bias():
     assert (y.cpu() - want).abs().max() < 5e-3
 
 
-@pytest.mark.parametrize("layers,hidden,steps,scale", [(1, 64, 1, 1.0), (2, 128, 9, 1e-6), (2, 256, 33, 1e5), (12, 64, 5, 1.0),
-                                                       (3, 256, 6, 1e-40)])
-def test_lstm_against_64_bits(layers, hidden, steps, scale):
-    """Few steps, many layers, inputs outside the range of fp16 (the vector is split into scaled fp16 parts).  The sums are
-    fp32 and the activations good to a few 1e-7 absolute, once per gate and layer; an input of 1e5 adds 1e-7 of a
-    pre-activation of that order to gates that are not saturated."""
-    from souffle_models_b200 import lstm
-    g = torch.Generator().manual_seed(layers + steps)
-    w = [((torch.rand(4 * layers, hidden, hidden, generator=g) - 0.5) * 2 / hidden ** 0.5).half() for _ in range(2)]
-    x = torch.randn(1, steps, hidden, generator=g) * scale
-    plan = lstm.LstmStack(w[0].cuda(), w[1].cuda(), steps)
-    y = plan.forward(x.cuda()).cpu().double()[0]
-    plan.status()
-    seq = x[0].double()
-    for l in range(layers):
-        wi, ws = (m[4 * l:4 * l + 4].reshape(4 * hidden, hidden).double() for m in w)
+def _lstm64(w_in, w_state, x):
+    """Top layer's hidden states in 64 bits; x [steps][hidden]."""
+    hidden = x.shape[1]
+    seq = x.double()
+    for l in range(w_in.shape[0] // 4):
+        wi, ws = (m[4 * l:4 * l + 4].reshape(4 * hidden, hidden).double() for m in (w_in, w_state))
         h = c = torch.zeros(hidden, dtype=torch.float64)
         rows = []
-        for t in range(steps):
-            z = (wi @ seq[t] + ws @ h).view(4, hidden)                 # gates i, j, f, o
+        for v in seq:
+            z = (wi @ v + ws @ h).view(4, hidden)                      # gates i, j, f, o
             c = c * torch.sigmoid(z[2] + 1) + torch.sigmoid(z[0]) * torch.tanh(z[1])
             h = torch.tanh(c) * torch.sigmoid(z[3])
             rows.append(h)
         seq = torch.stack(rows)
-    assert (y - seq).abs().max() < (1e-4 if scale > 1 else 2e-6)
+    return seq
+
+
+@pytest.mark.parametrize("layers,hidden,steps,scale,gain", [(1, 64, 1, 1.0, 6), (2, 128, 9, 1e-5, 6), (2, 256, 33, 1e5, 6),
+                                                            (12, 64, 5, 1.0, 10)])
+def test_lstm_against_64_bits(layers, hidden, steps, scale, gain):
+    """Few steps, many layers, inputs outside the range of fp16 (the vector is split into scaled fp16 parts), with weights
+    that bring every layer's pre-activations to order 1.  The sums are fp32 (2^-24 of terms of order 1, hidden of them) and
+    the activations good to 2e-7, once per gate; a layer passes an error on about as large as it came."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(layers + steps)
+    w = [(torch.rand(4 * layers, hidden, hidden, generator=g) - 0.5) * gain / hidden ** 0.5 for _ in range(2)]
+    w[0][:4] *= 0.3 / scale
+    w = [m.half() for m in w]
+    x = torch.randn(1, steps, hidden, generator=g) * scale
+    plan = lstm.LstmStack(w[0].cuda(), w[1].cuda(), steps)
+    y = plan.forward(x.cuda()).cpu().double()[0]
+    plan.status()
+    want = _lstm64(w[0], w[1], x[0])
+    assert want.abs().max() > 0.2
+    assert (y - want).abs().max() < 1e-6 * (layers + 1)
+
+
+def test_lstm_smallest_inputs():
+    """Subnormal inputs: the largest scale is as far as the exponent goes, and nothing but the activations' own error (they
+    are good to 2e-7 absolute) is left of the 1e-38 that comes out of the sums."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(9)
+    w = [((torch.rand(12, 256, 256, generator=g) - 0.5) / 8).half().cuda() for _ in range(2)]
+    plan = lstm.LstmStack(w[0], w[1], 6)
+    y = plan.forward((torch.randn(1, 6, 256, generator=g) * 1e-40).cuda())
+    plan.status()
+    assert (y.abs() < 2e-7).all()
+
+
+@pytest.mark.parametrize("hidden", [64, 128, 256])
+@pytest.mark.parametrize("delay", [False, True])
+def test_lstm_inputs_of_any_range(hidden, delay):
+    """Elements far below the largest one, whose own weights are zero, and finite elements beyond fp16's range next to an
+    infinity: the products are those of the fp32 vector.  Bound of the test against 64 bits for two layers."""
+    from souffle_models_b200 import lstm
+    g = torch.Generator().manual_seed(hidden)
+    w = [((torch.rand(8, hidden, hidden, generator=g) - 0.5) * 4 / hidden ** 0.5).half() for _ in range(2)]
+    w[0][:4, :, 5] = 0
+    w[0][:4, :, 2] = torch.where(w[0][:4, :, 2] == 0, torch.tensor(1e-3).half(), w[0][:4, :, 2])     # inf x 0 is not the point
+    x = torch.randn(1, 9, hidden, generator=g)
+    x[0, 1, 5], x[0, 3, 5], x[0, 6, 5] = 1e30, -3e38, 2.0 ** 20           # zero weights: these steps are the others' alone
+    x[0, 4] *= 2.0 ** 19                                                   # saturate their gates
+    x[0, 7] *= 1e6
+    x[0, 7, 2] = float("inf")
+    plan = lstm.LstmStack(w[0].cuda(), w[1].cuda(), 9, ref_input_delay=delay)
+    y = plan.forward(x.cuda()).cpu().double()[0]
+    plan.status()
+    xd = torch.cat([torch.zeros(1, hidden), x[0, :8]]) if delay else x[0]
+    want = _lstm64(w[0], w[1], xd)
+    assert torch.isfinite(want).all() and want.abs().max() > 0.2
+    assert (y - want).abs().max() < 3e-6
 
 
 def test_lstm_infinities_and_nan_stay_in_their_step():
