@@ -329,7 +329,7 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
                               int32_t batch, int32_t channels, int32_t height, int32_t width, int32_t reduce, void* workspace,
                               size_t workspace_bytes, souffle_stream_t stream);
 
-/* Blocks until `stream` is idle, then decodes the status words the library keeps for `workspace`. */
+/* Blocks until `stream` is idle, then decodes the status words in `workspace`. */
 int souffle_workspace_status(void* workspace, souffle_stream_t stream);
 /* Drops what the library remembers about a caller-owned workspace address (to be called before the memory is
  * freed or re-used for something else); the next call that is given the address clears it again. */

@@ -62,6 +62,7 @@ struct LstmParams {
   unsigned* done;         // [L][kLstmParts] published-step counters of this launch, one per (layer, CTA of its cluster)
   unsigned* done_next;    // the counters the next launch will use (cleared here)
   int* status;
+  int* expired;           // host memory or null: set by a CTA that gave up on a wait
   int layers, hidden, steps, ref_input_delay;
   unsigned long long timeout_ns;
 };
@@ -531,6 +532,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   __syncthreads();
   cluster_sync_all();
   if (*ctl.abort_smem) {                        // sent by peers before they came here, and not waited for: 200 us are ample
+    if (tid == 0 && p.expired) *p.expired = 1;
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }

@@ -58,6 +58,7 @@ struct MegaParams {
   unsigned* sync;       // [0] arrival count, [1] generation used by this launch
   unsigned* sync_next;  // the pair the next launch will use; cleared by this launch
   int* status;        // [0] code, [1] where, [2] cta
+  int* expired;       // host memory or null: set by a CTA that gave up on a wait
   unsigned long long timeout_ns;
   int max_slots;      // experiment knob: cap on operand ring slots, 0 = as many as fit
   int skip_arrival;   // test hook: CTA (skip_arrival-1) leaves at barrier 0 without arriving; 0 = off
@@ -2114,6 +2115,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     pr[4] = (long long)globaltimer_ns();
   }
   if (cs.abort) {
+    if (threadIdx.x == 0 && p.expired) *p.expired = 1;
     // let copies that were already issued land before the CTA's shared memory is released
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);

@@ -39,6 +39,7 @@ struct SeParams {
   float* partial;          // [batch*channels][slices] partial sums of the pool
   unsigned* sync;          // arrival counter of the grid barrier (zero at launch, left zero by the last CTA out)
   int* status;             // [0] code, [1] where, [2] cta
+  int* expired;            // host memory: set by a CTA that gave up on the barrier
   int batch, channels, hw, reduce;
   int slices, slice_len;   // a channel image = slices pieces of slice_len floats (the last one shorter)
   int items;               // batch * channels * slices
@@ -149,6 +150,7 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
           p.status[1] = 900;
           p.status[2] = (int)blockIdx.x;
         }
+        *p.expired = 1;
         abort_flag = 1;
         break;
       }

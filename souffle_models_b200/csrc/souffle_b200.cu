@@ -439,66 +439,39 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
 }
 
 // ------------------------------------------------------------------------------------
-// status words in page-locked host memory that the GPU writes directly (only when a wait expires): once the stream has
-// been waited for, the host reads them with a plain load.  With the words in device memory every synchronous entry
-// point ended with a copy into pageable memory, which cost more than the wait itself (a squeeze-and-excite call on one
-// 112 x 112 x 32 image: 42.4 us with the copy, 29.9 us without; the kernel took 8.6 us of either).
-// Blocks of 64 bytes are cut from 4 KiB slabs; a slab goes back to the driver when its last block is released, except
-// for one that is kept for the next plan.
+// Status words stay in device memory, with the plan or in the caller's workspace, and live and die with it.  Copying them
+// back at the end of every synchronous call costs more than the wait itself (a squeeze-and-excite call on one
+// 112 x 112 x 32 image: 42.4 us with the copy, 29.9 us without; the kernel took 8.6 us of either), so a kernel in which a
+// wait has run out also sets one word in page-locked host memory, for the life of the process: while it is clear, which a
+// plain load tells once the stream has been waited for, there is nothing to copy.
 // ------------------------------------------------------------------------------------
-struct StatusSlab {
-  char* mem = nullptr;
-  unsigned long long used = 0;             // bit i: block i is handed out
-};
-static std::mutex g_status_mutex;
-static std::vector<StatusSlab> g_status_slabs;
-constexpr size_t kStatusBlock = 64, kStatusSlabBytes = 64 * kStatusBlock;
-
-static int status_alloc(int** out) {
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  StatusSlab* slab = nullptr;
-  for (StatusSlab& s : g_status_slabs)
-    if (~s.used) { slab = &s; break; }
-  if (!slab) {
-    StatusSlab fresh;
-    // the first call on a workspace may be one that a stream capture is recording: the allocation is no part of it
+static int expired_word(int** out) {
+  static std::mutex mutex;
+  static int* word = nullptr;
+  std::lock_guard<std::mutex> lock(mutex);
+  if (!word) {
+    // the first call may be one that a stream capture is recording: the allocation is no part of it
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
     SF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-    const cudaError_t e = cudaHostAlloc((void**)&fresh.mem, kStatusSlabBytes, cudaHostAllocPortable | cudaHostAllocMapped);
+    int* fresh = nullptr;
+    const cudaError_t e = cudaHostAlloc((void**)&fresh, 64, cudaHostAllocPortable | cudaHostAllocMapped);
     cudaThreadExchangeStreamCaptureMode(&mode);
     SF_CUDA(e);
-    g_status_slabs.push_back(fresh);
-    slab = &g_status_slabs.back();
+    *fresh = 0;
+    word = fresh;
   }
-  const int i = __builtin_ctzll(~slab->used);
-  slab->used |= 1ull << i;
-  *out = reinterpret_cast<int*>(slab->mem + i * kStatusBlock);
-  memset(*out, 0, kStatusBlock);
+  *out = word;
   return SOUFFLE_OK;
 }
 
-// Nothing that could still write the block may be running (plans synchronise before they are destroyed).
-static void status_release(int* block) {
-  if (!block) return;
-  std::lock_guard<std::mutex> lock(g_status_mutex);
-  for (size_t k = 0; k < g_status_slabs.size(); ++k) {
-    StatusSlab& s = g_status_slabs[k];
-    const char* b = reinterpret_cast<const char*>(block);
-    if (b < s.mem || b >= s.mem + kStatusSlabBytes) continue;
-    s.used &= ~(1ull << ((b - s.mem) / kStatusBlock));
-    if (!s.used && g_status_slabs.size() > 1) {
-      cudaFreeHost(s.mem);
-      g_status_slabs.erase(g_status_slabs.begin() + k);
-    }
-    return;
-  }
-}
-
-// Reads and clears a block; the stream that ran the kernel has been waited for.
-static void status_take(int* block, int h[4]) {
-  volatile int* v = block;
-  for (int i = 0; i < 4; ++i) h[i] = v[i];
-  if (h[0] != DEV_OK) memset(block, 0, kStatusBlock);
+// The status words at `words` (device memory); the stream that ran the kernels has been waited for.
+static int read_status(const int* words, int h[4]) {
+  for (int i = 0; i < 4; ++i) h[i] = 0;
+  int* expired = nullptr;
+  int rc = expired_word(&expired);
+  if (rc) return rc;
+  if (*const_cast<volatile int*>(expired)) SF_CUDA(cudaMemcpy(h, words, 4 * sizeof(int), cudaMemcpyDeviceToHost));
+  return SOUFFLE_OK;
 }
 
 static int decode_status(const int* h, const char* what) {
@@ -528,7 +501,7 @@ struct SouffleBertPlan {
   Stage* d_stages = nullptr;
   CUtensorMap* d_maps = nullptr;
   unsigned* d_sync = nullptr;   // two (count, generation) pairs
-  int* status = nullptr;        // page-locked host memory, see status_alloc
+  int* d_status = nullptr;
   long long* d_prof = nullptr;
   // plan-owned activations
   __half *qkv = nullptr, *ctx = nullptr, *ln1 = nullptr, *fc1 = nullptr, *probs = nullptr, *act[2] = {nullptr, nullptr};
@@ -745,8 +718,9 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     if ((rc = plan_alloc(p, (void**)&p->probs, (size_t)B * Hh * S * S * 2))) return rc;
   }
   if ((rc = plan_alloc(p, (void**)&p->d_sync, 64))) return rc;
-  if ((rc = status_alloc(&p->status))) return rc;
+  if ((rc = plan_alloc(p, (void**)&p->d_status, 64))) return rc;
   SF_CUDA(cudaMemset(p->d_sync, 0, 64));
+  SF_CUDA(cudaMemset(p->d_status, 0, 64));
 
   // ---- tiling ----
   TileChoice t_qkv = choose_tiles(M, 3 * H, H, sms, false, false, 1), t_fc1 = choose_tiles(M, F, H, sms, false, false),
@@ -1006,13 +980,10 @@ int souffle_bert_plan_create(const SouffleBertDesc* desc, const SouffleBertLayer
   return SOUFFLE_OK;
 }
 
-static void ws_reclaim();                // see the records of caller-owned workspaces
-
 int souffle_bert_plan_destroy(SouffleBertPlan* plan) {
   if (!plan) return SOUFFLE_OK;
-  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
+  cudaDeviceSynchronize();
   for (void* a : plan->allocs) cudaFree(a);
-  status_release(plan->status);
   for (int i = 0; i < 2; ++i) {
     if (plan->x_dev[i]) cudaFree(plan->x_dev[i]);
     if (plan->y_dev[i]) cudaFree(plan->y_dev[i]);
@@ -1034,8 +1005,9 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   if (!aligned16(x) || !aligned16(y)) return fail(SOUFFLE_BAD_POINTER, "x and y must be non-null and 16-byte aligned");
   const SouffleBertDesc& d = plan->desc;
   const int M = d.batch * d.seq, H = d.heads * d.head_dim;
+  int rc;
   if (x != plan->last_x) {
-    int rc = make_map(&plan->x_map, x, M, H, (uint32_t)plan->x_box_rows);
+    rc = make_map(&plan->x_map, x, M, H, (uint32_t)plan->x_box_rows);
     if (rc) return rc;
     plan->last_x = x;
   }
@@ -1053,12 +1025,13 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   const unsigned par = plan->launch_id & 1u;
   mp.sync = plan->d_sync + 2 * par;
   mp.sync_next = plan->d_sync + 2 * (par ^ 1u);
-  mp.status = plan->status;
+  mp.status = plan->d_status;
+  if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
   mp.prof = plan->d_prof;
   mp.skip_arrival = d.debug_skip_arrival;
   mp.max_slots = d.debug_max_slots;
-  int rc = launch_mega(args, plan->grid, reinterpret_cast<cudaStream_t>(stream), plan->family);
+  rc = launch_mega(args, plan->grid, reinterpret_cast<cudaStream_t>(stream), plan->family);
   if (rc) return rc;
   plan->launch_id++;
   plan->launches = 1;
@@ -1154,8 +1127,13 @@ int souffle_bert_plan_status(SouffleBertPlan* plan) {
   if (!plan) return fail(SOUFFLE_BAD_ARGUMENT, "null plan");
   SF_CUDA(cudaDeviceSynchronize());
   int h[4];
-  status_take(plan->status, h);
-  if (h[0] != DEV_OK) cudaMemset(plan->d_sync, 0, 64);      // leave the plan usable: clear both barrier pairs
+  const int rc = read_status(plan->d_status, h);
+  if (rc) return rc;
+  if (h[0] != DEV_OK) {
+    // leave the plan usable: clear the status and both barrier pairs
+    cudaMemset(plan->d_status, 0, 64);
+    cudaMemset(plan->d_sync, 0, 64);
+  }
   return decode_status(h, "souffle_bert_forward");
 }
 
@@ -1227,50 +1205,19 @@ size_t souffle_gemm_workspace_bytes(void) { return 256; }
 // memset only the first time this library sees it, and a launch that ended in a device timeout leaves the
 // other pair clean for the call after it.
 static std::mutex g_ws_mutex;
-struct WsRecord {
-  unsigned launches = 0;       // of the entry points that alternate between the two barrier pairs
-  int* status = nullptr;       // see status_alloc
-  int device = 0;
-  bool forgotten = false;      // the caller has given the workspace up: the next call that is given the address starts afresh
-};
-static std::unordered_map<const void*, WsRecord> g_ws;
+static std::unordered_map<const void*, unsigned> g_ws_launches;     // launches of the entry points that alternate between the pairs
+constexpr size_t kWsStatusOffset = 64;
 
-// Gives back the status words of forgotten workspaces of the current device, which is idle (nothing can write them).
-static void ws_reclaim() {
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return;
+// On first sight of a workspace its control words are cleared on `st`.  `launch`: where not null, the number of launches on the barrier
+// pairs so far, which counts up.
+static int ws_enter(void* workspace, cudaStream_t st, unsigned* launch) {
   std::lock_guard<std::mutex> lock(g_ws_mutex);
-  for (auto it = g_ws.begin(); it != g_ws.end();) {
-    if (it->second.forgotten && it->second.device == dev) {
-      status_release(it->second.status);
-      it = g_ws.erase(it);
-    } else {
-      ++it;
-    }
-  }
-}
-
-// The record of a workspace (`alternate`: counts a launch on the barrier pairs, whose number before it goes to *launch);
-// on first sight its control words are cleared on `st`.
-static int ws_record(void* workspace, cudaStream_t st, bool alternate, unsigned* launch, int** status) {
-  std::lock_guard<std::mutex> lock(g_ws_mutex);
-  auto it = g_ws.find(workspace);
-  if (it == g_ws.end()) {
-    WsRecord r;
-    SF_CUDA(cudaGetDevice(&r.device));
-    int rc = status_alloc(&r.status);
-    if (rc) return rc;
-    r.forgotten = true;
-    it = g_ws.emplace(workspace, r).first;
-  }
-  if (it->second.forgotten) {
+  auto it = g_ws_launches.find(workspace);
+  if (it == g_ws_launches.end()) {
     SF_CUDA(cudaMemsetAsync(workspace, 0, 128, st));
-    it->second.launches = 0;
-    it->second.forgotten = false;
+    it = g_ws_launches.emplace(workspace, 0u).first;
   }
-  *launch = it->second.launches;
-  if (alternate) ++it->second.launches;
-  *status = it->second.status;
+  if (launch) *launch = it->second++;
   return SOUFFLE_OK;
 }
 
@@ -1278,11 +1225,12 @@ static int ws_prepare(void* workspace, size_t ws_bytes, cudaStream_t st, MegaPar
   if (!aligned16(workspace) || ws_bytes < souffle_gemm_workspace_bytes())
     return fail(SOUFFLE_BAD_POINTER, "workspace must be 16-byte aligned and hold %zu bytes", souffle_gemm_workspace_bytes());
   unsigned launch = 0;
-  int rc = ws_record(workspace, st, true, &launch, &mp->status);
-  if (rc) return rc;
+  int rc = ws_enter(workspace, st, &launch);
+  if (rc || (rc = expired_word(&mp->expired))) return rc;
   const unsigned par = launch & 1u;
   mp->sync = reinterpret_cast<unsigned*>(workspace) + 2 * par;
   mp->sync_next = reinterpret_cast<unsigned*>(workspace) + 2 * (par ^ 1u);
+  mp->status = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsStatusOffset);
   mp->timeout_ns = 2000ull * 1000000ull;
   return SOUFFLE_OK;
 }
@@ -1419,6 +1367,7 @@ struct SouffleSwinPlan {
 };
 
 static int launch_plan(SouffleBertPlan* plan, const void* x, void* y, const int32_t* lens, int timeout_ms, cudaStream_t st) {
+  int rc;
   CallArgs args;
   memset(&args, 0, sizeof(args));
   args.call_maps[0] = plan->x_map;
@@ -1433,9 +1382,10 @@ static int launch_plan(SouffleBertPlan* plan, const void* x, void* y, const int3
   const unsigned par = plan->launch_id & 1u;
   mp.sync = plan->d_sync + 2 * par;
   mp.sync_next = plan->d_sync + 2 * (par ^ 1u);
-  mp.status = plan->status;
+  mp.status = plan->d_status;
+  if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
-  int rc = launch_mega(args, plan->grid, st, kFamilySwin);
+  rc = launch_mega(args, plan->grid, st, kFamilySwin);
   if (rc) return rc;
   plan->launch_id++;
   plan->launches = 1;
@@ -1485,8 +1435,9 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
   __half* xlast = nullptr;          // output of the last block when patch merging follows inside the launch
   if (sp->has_merge && (rc = plan_alloc(p, (void**)&xlast, (size_t)T * C * 2))) return rc;
   if ((rc = plan_alloc(p, (void**)&p->d_sync, 64))) return rc;
-  if ((rc = status_alloc(&p->status))) return rc;
+  if ((rc = plan_alloc(p, (void**)&p->d_status, 64))) return rc;
   SF_CUDA(cudaMemset(p->d_sync, 0, 64));
+  SF_CUDA(cudaMemset(p->d_status, 0, 64));
   SF_CUDA(cudaMemset(qkvw, 0, (size_t)3 * Mw * C * 2));     // padding slots stay zero for ever
   SF_CUDA(cudaMemset(ctxw, 0, (size_t)Mw * C * 2));
   int m_y1, m_ctx, m_y2, m_hid, m_qkv;
@@ -1668,9 +1619,8 @@ int souffle_swin_stage_plan_create(const SouffleSwinDesc* desc, const SouffleSwi
 
 int souffle_swin_block_plan_destroy(SouffleSwinPlan* sp) {
   if (!sp) return SOUFFLE_OK;
-  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
+  cudaDeviceSynchronize();
   for (void* a : sp->base.allocs) cudaFree(a);
-  status_release(sp->base.status);
   delete sp;
   return SOUFFLE_OK;
 }
@@ -1779,12 +1729,13 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->w_state, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->h_all, (size_t)d.layers * d.steps * H * 4);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->done, 2 * kLstmDoneWords * sizeof(unsigned));
-  if (e == cudaSuccess && status_alloc(&p->status) != SOUFFLE_OK) e = cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = cudaMalloc((void**)&p->status, 64);
   if (e == cudaSuccess && bias) e = cudaMalloc((void**)&p->bias, (size_t)d.layers * H * 4);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_in, w_in, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_state, w_state, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess && bias) e = cudaMemcpy(p->bias, bias, (size_t)d.layers * H * 4, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaMemset(p->done, 0, 2 * kLstmDoneWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(p->status, 0, 64);
   if (e != cudaSuccess) {
     souffle_lstm_plan_destroy(p);
     return fail(SOUFFLE_CUDA_ERROR, "LSTM plan set-up failed: %s", cudaGetErrorString(e));
@@ -1795,9 +1746,8 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
 
 int souffle_lstm_plan_destroy(SouffleLstmPlan* p) {
   if (!p) return SOUFFLE_OK;
-  if (cudaDeviceSynchronize() == cudaSuccess) ws_reclaim();
-  cudaFree(p->w_in); cudaFree(p->w_state); cudaFree(p->bias); cudaFree(p->h_all); cudaFree(p->done);
-  status_release(p->status);
+  cudaDeviceSynchronize();
+  cudaFree(p->w_in); cudaFree(p->w_state); cudaFree(p->bias); cudaFree(p->h_all); cudaFree(p->done); cudaFree(p->status);
   delete p;
   return SOUFFLE_OK;
 }
@@ -1812,9 +1762,11 @@ int souffle_lstm_forward(SouffleLstmPlan* plan, const float* x, float* y, souffl
   lp.done = plan->done + kLstmDoneWords * par;
   lp.done_next = plan->done + kLstmDoneWords * (par ^ 1u);
   lp.status = plan->status;
+  int rc = expired_word(&lp.expired);
+  if (rc) return rc;
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
-  const int rc = lstm_launch(lp, reinterpret_cast<cudaStream_t>(stream));
+  rc = lstm_launch(lp, reinterpret_cast<cudaStream_t>(stream));
   if (rc) return rc;
   plan->launch_id++;
   return SOUFFLE_OK;
@@ -1826,8 +1778,10 @@ int souffle_lstm_plan_status(SouffleLstmPlan* plan) {
   if (!plan) return fail(SOUFFLE_BAD_ARGUMENT, "null plan");
   SF_CUDA(cudaDeviceSynchronize());
   int h[4];
-  status_take(plan->status, h);
+  const int rc = read_status(plan->status, h);
+  if (rc) return rc;
   if (h[0] != DEV_OK) {
+    cudaMemset(plan->status, 0, 64);
     cudaMemset(plan->done, 0, 2 * kLstmDoneWords * sizeof(unsigned));
   }
   return decode_status(h, "souffle_lstm_forward");
@@ -1896,6 +1850,7 @@ int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, c
   lp.h_all = reinterpret_cast<float*>(sd.scratch);
   lp.done = reinterpret_cast<unsigned*>(ctl);
   lp.done_next = reinterpret_cast<unsigned*>(ctl) + kLstmDoneWords;
+  lp.expired = nullptr;                  // the words below are read unasked; nothing is allocated here
   lp.status = device_status ? reinterpret_cast<int*>(device_status) : reinterpret_cast<int*>(ctl + kStaticStatusOffset);
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
@@ -1959,9 +1914,9 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
   if (!aligned16(workspace) || workspace_bytes < need)
     return fail(SOUFFLE_BAD_POINTER, "workspace must be 16-byte aligned and hold %zu bytes", need);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  unsigned launch = 0;
-  int rc = ws_record(workspace, st, false, &launch, &p.status);
-  if (rc) return rc;
+  int rc = ws_enter(workspace, st, nullptr);
+  if (rc || (rc = expired_word(&p.expired))) return rc;
+  p.status = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsStatusOffset);
   static bool attr_set[16] = {};
   if (dev < 16 && !attr_set[dev]) {
     SF_CUDA(cudaFuncSetAttribute(souffle_se_module, cudaFuncAttributeMaxDynamicSharedMemorySize, kSeSmemBytes));
@@ -1993,22 +1948,20 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
 int souffle_workspace_forget(void* workspace) {
   if (!workspace) return fail(SOUFFLE_BAD_ARGUMENT, "null workspace");
   std::lock_guard<std::mutex> lock(g_ws_mutex);
-  auto it = g_ws.find(workspace);
-  // a kernel still running on it may write its status words: they stay with the address until a plan of the device is
-  // destroyed (which waits for the device)
-  if (it != g_ws.end()) it->second.forgotten = true;
+  g_ws_launches.erase(workspace);
   return SOUFFLE_OK;
 }
 
 int souffle_workspace_status(void* workspace, souffle_stream_t stream) {
   if (!workspace) return fail(SOUFFLE_BAD_ARGUMENT, "null workspace");
   SF_CUDA(cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream)));
-  int h[4] = {0, 0, 0, 0};
-  std::lock_guard<std::mutex> lock(g_ws_mutex);
-  auto it = g_ws.find(workspace);
-  if (it == g_ws.end() || it->second.forgotten) return SOUFFLE_OK;      // no call has used it
-  status_take(it->second.status, h);
-  if (h[0] != DEV_OK) it->second.forgotten = true;   // start over: the next call on this workspace clears all of it
+  int h[4];
+  const int rc = read_status(reinterpret_cast<const int*>(reinterpret_cast<const char*>(workspace) + kWsStatusOffset), h);
+  if (rc) return rc;
+  if (h[0] != DEV_OK) {                 // start over: the next call on this workspace clears all of it
+    std::lock_guard<std::mutex> lock(g_ws_mutex);
+    g_ws_launches.erase(workspace);
+  }
   return decode_status(h, "souffle workspace");
 }
 
