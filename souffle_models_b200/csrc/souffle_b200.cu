@@ -464,6 +464,26 @@ static int expired_word(int** out) {
   return SOUFFLE_OK;
 }
 
+// Barrier words that alternate between launches are tracked here on the host, which a captured call must not take part in:
+// its launch runs when the graph is replayed, any number of times, with calls of any kind in between.  It has words of
+// its own, and the graph clears them in front of every replay.
+static int is_captured(cudaStream_t st, bool* captured) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  SF_CUDA(cudaStreamIsCapturing(st, &status));
+  *captured = status != cudaStreamCaptureStatusNone;
+  return SOUFFLE_OK;
+}
+
+// words: the pairs of alternate launches (0-3), a captured launch's pair (4, 5) and the pair it clears for nobody (6, 7).
+constexpr int kCapturedPair = 4;
+static int pick_barrier_words(unsigned* words, unsigned launches, bool captured, cudaStream_t st, MegaParams* mp) {
+  if (captured && mp->n_stages > 1) SF_CUDA(cudaMemsetAsync(words + kCapturedPair, 0, 2 * sizeof(unsigned), st));
+  const unsigned at = captured ? kCapturedPair : 2u * (launches & 1u);
+  mp->sync = words + at;
+  mp->sync_next = words + (at ^ 2u);
+  return SOUFFLE_OK;
+}
+
 // The status words at `words` (device memory); the stream that ran the kernels has been waited for.
 static int read_status(const int* words, int h[4]) {
   for (int i = 0; i < 4; ++i) h[i] = 0;
@@ -500,7 +520,7 @@ struct SouffleBertPlan {
   std::vector<void*> allocs;
   Stage* d_stages = nullptr;
   CUtensorMap* d_maps = nullptr;
-  unsigned* d_sync = nullptr;   // two (count, generation) pairs
+  unsigned* d_sync = nullptr;   // see pick_barrier_words
   int* d_status = nullptr;
   long long* d_prof = nullptr;
   // plan-owned activations
@@ -1022,9 +1042,8 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   mp.x = x;
   mp.y = y;
   mp.lens = seq_lens;
-  const unsigned par = plan->launch_id & 1u;
-  mp.sync = plan->d_sync + 2 * par;
-  mp.sync_next = plan->d_sync + 2 * (par ^ 1u);
+  bool captured = false;
+  if ((rc = is_captured(reinterpret_cast<cudaStream_t>(stream), &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, reinterpret_cast<cudaStream_t>(stream), &mp))) return rc;
   mp.status = plan->d_status;
   if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
@@ -1033,7 +1052,7 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   mp.max_slots = d.debug_max_slots;
   rc = launch_mega(args, plan->grid, reinterpret_cast<cudaStream_t>(stream), plan->family);
   if (rc) return rc;
-  plan->launch_id++;
+  if (!captured) plan->launch_id++;
   plan->launches = 1;
   return SOUFFLE_OK;
 }
@@ -1208,30 +1227,48 @@ static std::mutex g_ws_mutex;
 static std::unordered_map<const void*, unsigned> g_ws_launches;     // launches of the entry points that alternate between the pairs
 constexpr size_t kWsStatusOffset = 64;
 
-// On first sight of a workspace its control words are cleared on `st`.  `launch`: where not null, the number of launches on the barrier
-// pairs so far, which counts up.
-static int ws_enter(void* workspace, cudaStream_t st, unsigned* launch) {
+// On first sight of a workspace its control words are cleared: on `st`, or, where that is being captured, there and then
+// (the captured launch may be replayed after other calls).  `launches`: launches on the barrier pairs so far.
+static int ws_enter(void* workspace, cudaStream_t st, bool captured, unsigned* launches) {
   std::lock_guard<std::mutex> lock(g_ws_mutex);
   auto it = g_ws_launches.find(workspace);
   if (it == g_ws_launches.end()) {
-    SF_CUDA(cudaMemsetAsync(workspace, 0, 128, st));
+    if (captured) {
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      SF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+      cudaStream_t own = nullptr;
+      cudaError_t e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaMemsetAsync(workspace, 0, 128, own);
+      if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+      if (own) cudaStreamDestroy(own);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      SF_CUDA(e);
+    } else {
+      SF_CUDA(cudaMemsetAsync(workspace, 0, 128, st));
+    }
     it = g_ws_launches.emplace(workspace, 0u).first;
   }
-  if (launch) *launch = it->second++;
+  if (launches) *launches = it->second;
   return SOUFFLE_OK;
 }
 
-static int ws_prepare(void* workspace, size_t ws_bytes, cudaStream_t st, MegaParams* mp) {
+// Fills in what a launch takes from its workspace; args->p.n_stages is set.
+static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes, cudaStream_t st) {
   if (!aligned16(workspace) || ws_bytes < souffle_gemm_workspace_bytes())
     return fail(SOUFFLE_BAD_POINTER, "workspace must be 16-byte aligned and hold %zu bytes", souffle_gemm_workspace_bytes());
-  unsigned launch = 0;
-  int rc = ws_enter(workspace, st, &launch);
-  if (rc || (rc = expired_word(&mp->expired))) return rc;
-  const unsigned par = launch & 1u;
-  mp->sync = reinterpret_cast<unsigned*>(workspace) + 2 * par;
-  mp->sync_next = reinterpret_cast<unsigned*>(workspace) + 2 * (par ^ 1u);
+  MegaParams* mp = &args->p;
+  unsigned launches = 0;
+  bool captured = false;
+  int rc = is_captured(st, &captured);
+  if (rc || (rc = ws_enter(workspace, st, captured, &launches)) || (rc = expired_word(&mp->expired)) ||
+      (rc = pick_barrier_words(reinterpret_cast<unsigned*>(workspace), launches, captured, st, mp)))
+    return rc;
   mp->status = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsStatusOffset);
   mp->timeout_ns = 2000ull * 1000000ull;
+  if ((rc = launch_mega(*args, grid, st)) || captured) return rc;
+  std::lock_guard<std::mutex> lock(g_ws_mutex);
+  auto it = g_ws_launches.find(workspace);
+  if (it != g_ws_launches.end()) ++it->second;          // only now: a call that was refused has used neither pair
   return SOUFFLE_OK;
 }
 
@@ -1255,14 +1292,13 @@ int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CallArgs args;
   memset(&args, 0, sizeof(args));
-  if ((rc = ws_prepare(workspace, workspace_bytes, st, &args.p))) return rc;
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
   if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, c, M, N, K, sms))) return rc;
   if ((rc = make_map(&args.call_maps[0], a, M, K, (uint32_t)args.inline_stages[0].bm))) return rc;
   if ((rc = make_map(&args.call_maps[1], w_kn, K, N, 64))) return rc;     // [K][N]: box 64 (N) x 64 (K rows)
   args.p.n_stages = 1;
   const int items = stage_items(args.inline_stages[0]);
-  return launch_mega(args, items < sms ? items : sms, st);
+  return ws_launch(&args, items < sms ? items : sms, workspace, workspace_bytes, st);
 }
 
 // FC2 of the MLP has few output tiles and a long K (256 x 512 outputs, K = 2048 in the reference's shape), so
@@ -1290,7 +1326,6 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CallArgs args;
   memset(&args, 0, sizeof(args));
-  if ((rc = ws_prepare(workspace, workspace_bytes, st, &args.p))) return rc;
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
   if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, hidden, M, F, C, sms))) return rc;
   // split FC2 when the caller's workspace has room for the planes and the reduction stage supports the width
@@ -1325,7 +1360,7 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
     s3.eps = -1.0f;                                    // sum only
     if ((rc = finalize_stage(s3, 0, grid))) return rc;
   }
-  return launch_mega(args, grid, st);
+  return ws_launch(&args, grid, workspace, workspace_bytes, st);
 }
 
 int souffle_layernorm_forward(const float* partial, int32_t n_partial, const void* bias, const void* resid,
@@ -1343,7 +1378,6 @@ int souffle_layernorm_forward(const float* partial, int32_t n_partial, const voi
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   CallArgs args;
   memset(&args, 0, sizeof(args));
-  if ((rc = ws_prepare(workspace, workspace_bytes, st, &args.p))) return rc;
   Stage& s = args.inline_stages[0];
   s = blank_stage(STAGE_LN);
   s.M = M; s.N = N; s.ldo = N; s.partial = const_cast<float*>(partial); s.n_partial = n_partial; s.bias = bias;
@@ -1353,7 +1387,7 @@ int souffle_layernorm_forward(const float* partial, int32_t n_partial, const voi
   const int items = stage_items(s);
   const int grid = items < sms ? items : sms;
   if ((rc = finalize_stage(s, 0, grid))) return rc;
-  return launch_mega(args, grid, st);
+  return ws_launch(&args, grid, workspace, workspace_bytes, st);
 }
 
 // ======================================================================================
@@ -1379,15 +1413,14 @@ static int launch_plan(SouffleBertPlan* plan, const void* x, void* y, const int3
   mp.x = x;
   mp.y = y;
   mp.lens = lens;
-  const unsigned par = plan->launch_id & 1u;
-  mp.sync = plan->d_sync + 2 * par;
-  mp.sync_next = plan->d_sync + 2 * (par ^ 1u);
+  bool captured = false;
+  if ((rc = is_captured(st, &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, st, &mp))) return rc;
   mp.status = plan->d_status;
   if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
   rc = launch_mega(args, plan->grid, st, kFamilySwin);
   if (rc) return rc;
-  plan->launch_id++;
+  if (!captured) plan->launch_id++;
   plan->launches = 1;
   return SOUFFLE_OK;
 }
@@ -1697,7 +1730,7 @@ struct SouffleLstmPlan {
   SouffleLstmDesc desc;
   __half *w_in = nullptr, *w_state = nullptr;
   float *bias = nullptr, *h_all = nullptr;
-  unsigned* done = nullptr;   // two sets of kLstmDoneWords counters, used by alternate launches
+  unsigned* done = nullptr;   // four sets of kLstmDoneWords counters: two for alternate launches, one for captured ones, one they clear for nobody
   int* status = nullptr;
   unsigned launch_id = 0;
 };
@@ -1728,13 +1761,13 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
   cudaError_t e = cudaMalloc((void**)&p->w_in, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->w_state, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->h_all, (size_t)d.layers * d.steps * H * 4);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&p->done, 2 * kLstmDoneWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&p->done, 4 * kLstmDoneWords * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->status, 64);
   if (e == cudaSuccess && bias) e = cudaMalloc((void**)&p->bias, (size_t)d.layers * H * 4);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_in, w_in, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_state, w_state, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess && bias) e = cudaMemcpy(p->bias, bias, (size_t)d.layers * H * 4, cudaMemcpyDeviceToDevice);
-  if (e == cudaSuccess) e = cudaMemset(p->done, 0, 2 * kLstmDoneWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(p->done, 0, 4 * kLstmDoneWords * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(p->status, 0, 64);
   if (e != cudaSuccess) {
     souffle_lstm_plan_destroy(p);
@@ -1758,17 +1791,21 @@ int souffle_lstm_forward(SouffleLstmPlan* plan, const float* x, float* y, souffl
   const SouffleLstmDesc& d = plan->desc;
   LstmParams lp;
   lp.w_in = plan->w_in; lp.w_state = plan->w_state; lp.bias = plan->bias; lp.x = x; lp.y = y; lp.h_all = plan->h_all;
-  const unsigned par = plan->launch_id & 1u;
-  lp.done = plan->done + kLstmDoneWords * par;
-  lp.done_next = plan->done + kLstmDoneWords * (par ^ 1u);
-  lp.status = plan->status;
-  int rc = expired_word(&lp.expired);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  bool captured = false;
+  int rc = is_captured(st, &captured);
   if (rc) return rc;
+  const unsigned set = captured ? 2u : plan->launch_id & 1u;
+  lp.done = plan->done + kLstmDoneWords * set;
+  lp.done_next = plan->done + kLstmDoneWords * (set ^ 1u);
+  if (captured) SF_CUDA(cudaMemsetAsync(lp.done, 0, kLstmDoneWords * sizeof(unsigned), st));
+  lp.status = plan->status;
+  if ((rc = expired_word(&lp.expired))) return rc;
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
-  rc = lstm_launch(lp, reinterpret_cast<cudaStream_t>(stream));
+  rc = lstm_launch(lp, st);
   if (rc) return rc;
-  plan->launch_id++;
+  if (!captured) plan->launch_id++;
   return SOUFFLE_OK;
 }
 
@@ -1914,8 +1951,9 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
   if (!aligned16(workspace) || workspace_bytes < need)
     return fail(SOUFFLE_BAD_POINTER, "workspace must be 16-byte aligned and hold %zu bytes", need);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  int rc = ws_enter(workspace, st, nullptr);
-  if (rc || (rc = expired_word(&p.expired))) return rc;
+  bool captured = false;
+  int rc = is_captured(st, &captured);
+  if (rc || (rc = ws_enter(workspace, st, captured, nullptr)) || (rc = expired_word(&p.expired))) return rc;
   p.status = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsStatusOffset);
   static bool attr_set[16] = {};
   if (dev < 16 && !attr_set[dev]) {
