@@ -243,6 +243,8 @@ int souffle_lstm_static_status(souffle_stream_t stream);
  * workspace, or hands its memory to another use, tells the library with souffle_workspace_forget() before the
  * address can come back with other contents: barrier words the library believes consistent but that were
  * overwritten make the next call's result undefined (the barriers may pass at once), not merely a timeout.
+ * A call may be recorded by a stream capture, the first one on a workspace too, and replayed between ordinary calls
+ * (so may the plans' forward calls); a workspace that the library has not seen is cleared when the call is recorded.
  * ------------------------------------------------------------------------------------------ */
 size_t souffle_gemm_workspace_bytes(void);
 int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_t N, int32_t K,

@@ -1,25 +1,48 @@
-"""The multiply-high quotients of the Swin row maps are exact over the sizes a plan takes (host arithmetic: the kernel
-uses the same 32-bit formula), and a token grid past that range goes through the plain divisions."""
+"""The multiply-high quotients of the Swin row maps are exact over the sizes a plan takes (the library's own multipliers,
+with the kernel's multiply-high in 64 bits), and a token grid past that range goes through the plain divisions."""
+import os
+import shutil
+import subprocess
+
 import pytest
 import torch
 
 from oracle import souffle_oracle as so
 
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "souffle_models_b200", "csrc")
+PROGRAM = """
+#include <cstdio>
+#include <cstdlib>
+#include "stage_program.h"
+int main(int argc, char** argv) {       // pairs: divisor, number of numerators
+  for (int i = 1; i + 1 < argc; i += 2) {
+    const uint32_t d = (uint32_t)atol(argv[i]), top = (uint32_t)atol(argv[i + 1]), mg = souffle::fast_div_magic(d);
+    for (uint32_t n = 0; n < top; ++n)
+      if ((d <= 1 ? n : (uint32_t)(((uint64_t)n * mg) >> 32)) != n / d) { printf("%u / %u", n, d); return 1; }
+  }
+  return 0;
+}
+"""
 
-def _magic(d):
-    return 0 if d <= 1 else (2 ** 32 + d - 1) // d
+
+@pytest.fixture(scope="module")
+def quotients(tmp_path_factory):
+    if not shutil.which("g++"):
+        pytest.skip("no g++")
+    tmp = tmp_path_factory.mktemp("quotients")
+    (tmp / "q.cpp").write_text(PROGRAM)
+    subprocess.run(["g++", "-O2", "-I", CSRC, "-o", str(tmp / "q"), str(tmp / "q.cpp")], check=True)
+    return str(tmp / "q")
 
 
 @pytest.mark.parametrize("res,win,rows", [(7, 7, 1 << 20), (14, 7, 1 << 20), (56, 7, 1 << 20), (64, 8, (1 << 20) - 4096), (120, 8, 291600),
                                           (252, 7, 63504)])
-def test_quotients_are_exact(res, win, rows):
-    import numpy as np
+def test_quotients_are_exact(quotients, res, win, rows):
     nwr = res // win
     assert rows * res * res < 2 ** 32            # the rule by which the host hands out a multiplier at all
-    for d, top in ((res * res, rows), (res, res * res), (win, res), (nwr * nwr, rows // 64 + 1), (nwr, nwr * nwr), (win, 64)):
-        if d > 1:
-            n = np.arange(top, dtype=np.uint64)
-            assert ((n * np.uint64(_magic(d))) >> np.uint64(32) == n // np.uint64(d)).all(), (d, top)
+    pairs = ((res * res, rows), (res, res * res), (win, res), (nwr * nwr, rows // 64 + 1), (nwr, nwr * nwr), (win, 64))
+    run = subprocess.run([quotients] + [str(v) for pair in pairs for v in pair], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
 
 
 @pytest.mark.gpu
