@@ -86,9 +86,10 @@ template <bool kCluster>
 __device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, uint32_t stop) {
   uint32_t spins = 0;
   while (!lstm_try<kCluster>(bar, parity)) {
-    if (((++spins) & 0xFF) == 0) {
+    ++spins;
+    if (stop && (spins & 0xF) == 0 && ld_acquire_cta_shared_u32(stop)) return lstm_try<kCluster>(bar, parity);
+    if ((spins & 0xFF) == 0) {
       if (*c.abort_smem) return false;
-      if (stop && ld_acquire_cta_shared_u32(stop)) return lstm_try<kCluster>(bar, parity);
       if (globaltimer_ns() > c.deadline_ns) {
         record_timeout(c, DEV_TIMEOUT_MBAR, where);
         return false;
