@@ -8,9 +8,13 @@
 // one grid barrier as fit, and both tiny GEMVs are recomputed by every CTA that needs them instead of being exchanged
 // through two more barriers: the input is read from HBM once and the output written once.
 // The module is bound by memory: 16 warps of an SM have to keep some 40 KB of loads in flight to draw the full HBM rate,
-// so a warp issues eight 16-byte loads per lane before it touches the first of them, and a CTA's weights are on their way
-// to shared memory before the barrier.  One 4-byte load per lane and four in flight took 139 us of GPU time for
-// 32 x 144 x 56 x 56 (0.83 TB/s of the 116 MB the module cannot do without), this form 32 us (3.6 TB/s).
+// so a warp issues eight 16-byte loads per lane before it touches the first of them.  One 4-byte load per lane and four in
+// flight took 107-114 us of GPU time for 32 x 144 x 56 x 56 (1.1 TB/s of the 116 MB the module cannot do without), this
+// form 33 us (3.6 TB/s).
+// Small images with many channels are bound by the reduce weights instead (1 x 1152 x 7 x 7: 221 KB, which every CTA needs,
+// against 0.2 MB of image): a CTA brings them to shared memory while it waits at the barrier, 16 bytes at a time, eight
+// loads in flight (19.7 us under ncu with the rows of the GEMV read from L2 four 4-byte loads at a time, 13.8 so; 1 x 4096 x 8 x 8, whose 1 MB of
+// weights stay in L2, 62 us four 4-byte loads at a time, 24.5 so).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -21,7 +25,7 @@ namespace souffle {
 
 constexpr int kSeThreads = 512;
 constexpr int kSeWarps = kSeThreads / 32;
-constexpr int kSeSmemBytes = 229376;          // 224 KiB of dynamic shared memory at most
+constexpr int kSeSmemBytes = 231424;          // 226 KiB of dynamic shared memory at most
 constexpr int kSeMaxReduce = 64;              // reduce channels
 constexpr int kSeMaxChannels = 4096;          // channels (their means are staged in shared memory)
 constexpr int kSeUnroll = 8;                  // 16-byte loads a lane has in flight
@@ -156,8 +160,18 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
       }
     }
   } else if (warp > 0 && p.stage_weights) {
-    const int n = p.reduce * p.channels;
-    for (int i = threadIdx.x - 32; i < n; i += kSeThreads - 32) w_red[i] = __ldg(p.w_reduce + i);
+    const int n = p.reduce * p.channels, n4 = (reinterpret_cast<uintptr_t>(p.w_reduce) & 15) == 0 ? n >> 2 : 0;
+    constexpr int kStep = kSeThreads - 32;
+    for (int i0 = threadIdx.x - 32; i0 < n4; i0 += kStep * kSeUnroll) {
+      float4 v[kSeUnroll];
+#pragma unroll
+      for (int u = 0; u < kSeUnroll; ++u)
+        if (i0 + u * kStep < n4) v[u] = __ldg(reinterpret_cast<const float4*>(p.w_reduce) + i0 + u * kStep);
+#pragma unroll
+      for (int u = 0; u < kSeUnroll; ++u)
+        if (i0 + u * kStep < n4) reinterpret_cast<float4*>(w_red)[i0 + u * kStep] = v[u];
+    }
+    for (int i = 4 * n4 + threadIdx.x - 32; i < n; i += kStep) w_red[i] = __ldg(p.w_reduce + i);
   }
   __syncthreads();
   if (abort_flag) return;
@@ -166,7 +180,6 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
   //      item this channel's gate (expand GEMV row, sigmoid) and the add ----
   const float inv_hw = 1.0f / (float)p.hw;
   const int items_per_img = p.channels * p.slices;
-  const float* wr = p.stage_weights ? w_red : p.w_reduce;
   int cur_img = -1;
   slot = 0;
   for (int first = item0; first < item1; first += kSeWarps, ++slot) {    // item of warp 0 in this round
@@ -185,8 +198,22 @@ __global__ void __launch_bounds__(kSeThreads, 1) souffle_se_module(const SeParam
         __syncthreads();
         for (int j = warp; j < p.reduce; j += kSeWarps) {
           float acc = 0.0f;
+          if (p.stage_weights) {
 #pragma unroll 4
-          for (int k = lane; k < p.channels; k += 32) acc = fmaf(pooled_s[k], wr[(size_t)j * p.channels + k], acc);
+            for (int k = lane; k < p.channels; k += 32) acc = fmaf(pooled_s[k], w_red[j * p.channels + k], acc);
+          } else {                                           // too large to stage: rows from L2, eight loads in flight
+            const float* row = p.w_reduce + (size_t)j * p.channels;
+            if (p.channels % 4 == 0 && (reinterpret_cast<uintptr_t>(row) & 15) == 0) {
+#pragma unroll 8
+              for (int k = lane; k < p.channels / 4; k += 32) {
+                const float4 w = __ldg(reinterpret_cast<const float4*>(row) + k), m = reinterpret_cast<const float4*>(pooled_s)[k];
+                acc = fmaf(m.w, w.w, fmaf(m.z, w.z, fmaf(m.y, w.y, fmaf(m.x, w.x, acc))));
+              }
+            } else {
+#pragma unroll 8
+              for (int k = lane; k < p.channels; k += 32) acc = fmaf(pooled_s[k], __ldg(row + k), acc);
+            }
+          }
           acc = warp_sum(acc);
           if (lane == 0) gate_in[j] = acc * se_sigmoid(acc);
         }

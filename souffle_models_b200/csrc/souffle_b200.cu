@@ -1963,11 +1963,20 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
   // Items are dealt out evenly over all SMs, in contiguous runs: a small image is pulled in by as many SMs as it has
   // slices, and a CTA of a large batch meets one or two images, whose reduce GEMV it recomputes.
   p.per_cta = (p.items + sms - 1) / sms;
+  const size_t weights = (size_t)reduce * channels * sizeof(float);
+  const int per_image = channels * p.slices;
+  if (batch > 1 && p.per_cta < per_image && p.per_cta * (size_t)p.slice_len * sizeof(float) < 2 * weights) {
+    // The GEMV counts for more than the slices: where a run up to a quarter longer divides the image, no CTA meets two
+    // images (2 x 672 x 14 x 14: 12.4 -> 10.0 us, 8 x 1152 x 7 x 7: 27.7 -> 20.5; where the slices are the larger part,
+    // as in 32 x 144 x 56 x 56, idle SMs would cost more than the second GEMV)
+    for (int d = p.per_cta; d <= p.per_cta + p.per_cta / 4 && d <= per_image; ++d)
+      if (per_image % d == 0) { p.per_cta = d; break; }
+  }
   const int grid = (p.items + p.per_cta - 1) / p.per_cta;
   // shared memory: the channel means and reduce outputs, then as many slices per warp as fit, then the reduce weights
   const int per_warp = (p.per_cta + kSeWarps - 1) / kSeWarps;
   size_t smem = (size_t)(channels + kSeMaxReduce) * sizeof(float);
-  const size_t keep = (size_t)kSeWarps * se_slice_floats(p.slice_len) * sizeof(float), weights = (size_t)reduce * channels * sizeof(float);
+  const size_t keep = (size_t)kSeWarps * se_slice_floats(p.slice_len) * sizeof(float);
   p.cached = (int)((kSeSmemBytes - smem) / keep);
   if (p.cached > per_warp) p.cached = per_warp;
   smem += p.cached * keep;

@@ -74,3 +74,21 @@ def test_slices_at_every_alignment(shape, shift):
     want_pooled, want = so.se_module(x, wr, we)
     assert (pooled.cpu() - want_pooled).abs().max() < 1e-5
     assert (out.cpu() - want).abs().max() < 2e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 7, 7, 1152, 48), (2, 14, 14, 672, 28), (8, 14, 14, 240, 10), (2, 8, 8, 4096, 64), (3, 3, 3, 1801, 64),
+                                   (5, 7, 7, 101, 64)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_reduce_weights_staged_and_not_at_every_alignment(shape, shift):
+    """Reduce weights that fill shared memory to the last hundred bytes, that do not fit, that start off a 16-byte boundary,
+    rows that are no multiple of four; runs of items that divide an image and runs that cannot.  Bound of the test above."""
+    from souffle_models_b200 import efficientnet
+    b, h, w, c, r = shape
+    x, wr, we = _case(b, h, w, c, r, 23 + c)
+    we = we / r ** 0.5
+    flat = torch.zeros(wr.numel() + 4)
+    flat[shift:shift + wr.numel()] = wr.reshape(-1)
+    pooled, out = efficientnet.se_module(x.cuda(), flat.cuda()[shift:shift + wr.numel()].view(r, c), we.cuda())
+    want_pooled, want = so.se_module(x, wr, we)
+    assert (pooled.cpu() - want_pooled).abs().max() < 1e-5
+    assert (out.cpu() - want).abs().max() < 2e-5
