@@ -18,8 +18,9 @@
 // * Hidden states go straight into the shared memory of the eight CTAs of the cluster (distributed shared memory,
 //   st.async: the store itself counts as a transfer on the receiver's mbarrier, no fence on either side), and every cell
 //   warp waits for them itself: there is no CTA barrier in the step.
-// A step of hidden 256 takes 2.4 k cycles (hidden 64: 1.5 k); with the products on the CUDA cores (128 conversions and FMAs per thread, partial sums by
-// shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps 228 -> 159 us, 12 x 64 x 200 266 -> 178 us.
+// A step of hidden 256 takes 2.3 k cycles (hidden 64: 1.5 k); with the products on the CUDA cores (128 conversions and FMAs
+// per thread, partial sums by shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps
+// 228 -> 155 us, 12 x 64 x 200 266 -> 175 us.
 // Only the hop to the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
 // Every CTA of a layer publishes its own count of finished steps; the consumer checks all eight, so a CTA whose
 // publication lags cannot be covered by its peers running ahead.  The same holds inside a CTA: a warp sends h(t) to the

@@ -1315,9 +1315,9 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
 // Scores get the relative-position bias of the (query, key) offset and, for shifted windows, -100 where
 // query and key come from different sides of the wrap-around.  Slots >= win*win are padding.
 // ------------------------------------------------------------------------------------
-// Softmax of one query row of a WS x WS window (thread = row, `r_in` = row of the window, `live` = the window exists): reads the 64 score columns from TMEM,
-// adds bias and shift mask, writes the unnormalised probabilities as an fp16 A-operand row (128B swizzle)
-// and returns their sum.  Rows and keys >= WS*WS are padding (probability 0).
+// Softmax of one query row of a WS x WS window (thread = row, `r_in` = row of the window, `live` = the window exists):
+// reads the 64 score columns from TMEM, adds bias and shift mask, writes the unnormalised probabilities as an fp16
+// A-operand row (128B swizzle) and returns their sum.  Rows and keys >= WS*WS are padding (probability 0).
 template <int WS>
 __device__ __forceinline__ float swin_softmax_row(uint32_t tmem, const float* bias_s, uint8_t* prow, int r_in, bool live, int wy, int wx,
                                                   int R, int shift, float sl2) {

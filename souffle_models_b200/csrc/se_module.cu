@@ -13,8 +13,8 @@
 // form 33 us (3.6 TB/s).
 // Small images with many channels are bound by the reduce weights instead (1 x 1152 x 7 x 7: 221 KB, which every CTA needs,
 // against 0.2 MB of image): a CTA brings them to shared memory while it waits at the barrier, 16 bytes at a time, eight
-// loads in flight (19.7 us under ncu with the rows of the GEMV read from L2 four 4-byte loads at a time, 13.8 so; 1 x 4096 x 8 x 8, whose 1 MB of
-// weights stay in L2, 62 us four 4-byte loads at a time, 24.5 so).
+// loads in flight (19.7 us under ncu with the rows of the GEMV read from L2 four 4-byte loads at a time, 13.8 so).  Larger
+// weights stay in L2 and are read 16 bytes at a time (1 x 4096 x 8 x 8, 1 MB of weights: 62 us by 4-byte loads, 24.5 so).
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -1043,7 +1043,8 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   mp.y = y;
   mp.lens = seq_lens;
   bool captured = false;
-  if ((rc = is_captured(reinterpret_cast<cudaStream_t>(stream), &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, reinterpret_cast<cudaStream_t>(stream), &mp))) return rc;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if ((rc = is_captured(st, &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, st, &mp))) return rc;
   mp.status = plan->d_status;
   if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
@@ -1730,7 +1731,8 @@ struct SouffleLstmPlan {
   SouffleLstmDesc desc;
   __half *w_in = nullptr, *w_state = nullptr;
   float *bias = nullptr, *h_all = nullptr;
-  unsigned* done = nullptr;   // four sets of kLstmDoneWords counters: two for alternate launches, one for captured ones, one they clear for nobody
+  // four sets of kLstmDoneWords counters: two for alternate launches, one for captured ones, one these clear for nobody
+  unsigned* done = nullptr;
   int* status = nullptr;
   unsigned launch_id = 0;
 };
