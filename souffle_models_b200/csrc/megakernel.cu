@@ -32,8 +32,9 @@ constexpr int kThreads = 384;               // warp 0 TMA, warp 1 MMA, warps 2..
                                             // the LayerNorm stages only (registers are handed out per four warps: a block of
                                             // ten warps is charged for twelve, so the two extra warps cost nothing)
 constexpr int kEpiWarps = 8, kEpiThreads = kEpiWarps * 32;
+constexpr int kSpareWarp = 2 + kEpiWarps, kWeightWarp = kSpareWarp + 1;
 constexpr int kRingBytes = 196608;          // 192 KiB operand ring (4 x 48 KiB, 3 x 64 KiB or 6 x 32 KiB slots)
-constexpr int kCtlBytes = 1024;             // barriers + control words
+constexpr int kCtlBytes = 2048;             // barriers, control words, two stage records
 constexpr int kVecBytes = 16384;             // per-stage vectors staged in shared memory (a GEMM's bias as fp32: N <= 4096)
 constexpr int kStageRow = 64;                // bytes per staged row; the 16-byte pieces of a row are XOR-swizzled (see below)
 constexpr int kStageWarp = 32 * kStageRow;   // one epilogue warp's transpose buffer
@@ -89,15 +90,18 @@ struct __align__(8) SmemCtl {
   uint64_t attn1[7];                                                     // attention, pipeline 1 (same order)
   uint64_t o_empty[2];                                                   // pair attention: output accumulator read out
   uint64_t ln_full[4], ln_empty[4];
-  uint64_t rec_full;                // the next stage's record has landed (bulk copy issued inside the grid barrier)
   uint32_t tmem_base;
   int abort;
-  unsigned long long deadline_ns;   // read from the global timer once per CTA
-  alignas(16) Stage stage;   // current stage; plan-owned programs fetch the next record while the CTA waits at the barrier
+  int leave[2];                     // a wait has run out: all warps leave the stage loop together
+  uint32_t arrived;                 // stages whose arrival this CTA has sent
+  uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go)
+  WaitCtl wait;                     // here and not on the stack: see RoleState
+  alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their position
 };
 static_assert(sizeof(SmemCtl) <= kCtlBytes, "control block too large");
 
-// Per-thread view of the pipelines; identical arithmetic in every role keeps them in step.
+// Per-thread view of the pipelines; identical arithmetic in every role keeps them in step.  Out-of-line stage functions take and
+// return it packed into one register: every grid barrier's acquire empties L1, so a word on the stack costs a round trip to L2.
 struct RoleState {
   uint32_t slot = 0;       // next ring slot
   uint32_t slot_bits = 0;  // phase bit per ring slot
@@ -106,7 +110,17 @@ struct RoleState {
   uint32_t attn_bit1 = 0;  // phase bit of the attention barriers, pipeline 1
   uint32_t ln_bits = 0;    // phase bit per LayerNorm batch buffer
   uint32_t o_bits = 0;     // pair attention: phase bit of the o_empty barrier of each pipeline (MMA lane)
+  __device__ __forceinline__ uint32_t pack() const {
+    return slot | (slot_bits << 4) | (acc_bits << 12) | (attn_bit << 15) | (attn_bit1 << 16) | (ln_bits << 17) | (o_bits << 21);
+  }
+  static __device__ __forceinline__ RoleState unpack(uint32_t w) {
+    RoleState r;
+    r.slot = w & 15u; r.slot_bits = (w >> 4) & 255u; r.acc_bits = (w >> 12) & 7u; r.attn_bit = (w >> 15) & 1u;
+    r.attn_bit1 = (w >> 16) & 1u; r.ln_bits = (w >> 17) & 15u; r.o_bits = (w >> 21) & 3u;
+    return r;
+  }
 };
+static_assert(kMaxSlots <= 8, "a slot index and a phase bit per slot are packed into four and eight bits");
 
 // SM clock for the stage-level stamps of the in-kernel profile.  The memory clobber keeps the read where it is
 // written: a plain clock64() may be scheduled above a preceding barrier, which charges a stage's work to the wait
@@ -123,63 +137,72 @@ __device__ __forceinline__ const void* sel_ptr(int sel, const void* plan, const 
 
 // ------------------------------------------------------------------------------------
 // grid barrier: one monotonic arrival counter per launch, bounded spin
+//
+// Its two halves lie with different warps, so that a stage's set-up runs while the CTA waits.  At the end of a stage all
+// threads of a CTA meet once (the end of the stage loop); a lane of a spare warp then adds the CTA's arrival to the counter,
+// whose release covers every thread's writes and takes ~1 k cycles.  Meanwhile every warp has gone on to the next stage: the
+// epilogue warps stage the bias, the row warps load gamma and beta, and the feeder (the lone lane of warp 0 that issues the
+// stage's copies) requests the first weight tiles, none of which the stage before has written.  Only the feeder looks at the
+// counter (grid_wait), and what it does next is issue the stage's first activation copy.  All other warps of a GEMM or
+// attention stage are behind the data the feeder asks for; warps that read what earlier stages wrote by themselves wait for
+// the feeder's word (wait_go).
 // ------------------------------------------------------------------------------------
 // The polls in front stand in straight line (a loop's way out costs some 150 cycles, see mbar_wait_hot); a CTA that waits
 // longer than they last goes on out of line.
-__device__ __noinline__ void grid_wait_loop(const unsigned* count, unsigned target, const WaitCtl& ctl, int where) {
+__device__ __noinline__ bool grid_wait_loop(const unsigned* count, unsigned target, const WaitCtl& ctl, int where) {
   uint32_t spins = 0;
   while (ld_acquire_u32(count) < target) {
     if (((++spins) & 0x3F) == 0) {
-      if (*ctl.abort_smem) break;
+      if (*ctl.abort_smem) return false;
       if (globaltimer_ns() > ctl.deadline_ns) {
         record_timeout(ctl, DEV_TIMEOUT_GRID, where);
-        break;
+        return false;
       }
     }
   }
+  return true;
 }
-
-__device__ bool grid_barrier(const MegaParams& p, const WaitCtl& ctl, int where, SmemCtl& cs) {
-  // The CTA barrier orders every thread's global writes before thread 0, whose gpu-scope release is
-  // cumulative and publishes them to the other CTAs.  On the way out thread 0's acquire, the second CTA
-  // barrier and a proxy fence order the other CTAs' writes before this CTA's TMA and bulk-copy reads.
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (p.prof) p.prof[((size_t)where * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
-    // The counter only grows during a launch: barrier number `where` is passed once every CTA
+// One thread: waits until every CTA has finished stage si - 1.  Its acquire and the proxy fence order the other CTAs'
+// writes before this thread's TMA and bulk copies.  False: the wait has run out.
+__device__ __forceinline__ bool grid_wait(const MegaParams& p, const WaitCtl& ctl, int si) {
+  bool there = si == 0;
+  if (!there) {
+    // The counter only grows during a launch: barrier number `si - 1` is passed once every CTA
     // has added 1 for it.  (The launch that runs next clears the other counter, see the prologue.)
-    unsigned* count = p.sync;
-    const unsigned target = (unsigned)(where + 1) * gridDim.x;
-    const bool skip = p.skip_arrival > 0 && where == 0 && (int)blockIdx.x == p.skip_arrival - 1;
-    if (skip) *ctl.abort_smem = 1; else red_add_release_u32(count, 1u);
-    // Nobody reads the current stage record any more (the CTA barrier above): the next one is fetched by a bulk
-    // copy while this thread waits for the other CTAs, so its round trip to L2 costs the stage nothing.
-    const bool fetch = p.stages != nullptr;
-    if (fetch) {
-      // first this CTA's slice of the weights of the GEMM stage after next -> L2 (they come from HBM when the program's
-      // weights exceed L2; without this every GEMM stage starts with all CTAs waiting on the same DRAM rows)
-      const uint32_t pf_bytes = cs.stage.pf_bytes;
-      if (pf_bytes) {
-        const uint32_t per = ((pf_bytes + gridDim.x - 1) / gridDim.x + 15u) & ~15u, off = blockIdx.x * per;
-        if (off < pf_bytes)
-          bulk_prefetch_l2(reinterpret_cast<const char*>(cs.stage.pf_ptr) + off, off + per <= pf_bytes ? per : pf_bytes - off);
-      }
-      mbar_expect_tx(smem_u32(&cs.rec_full), (uint32_t)sizeof(Stage));
-      bulk_load(smem_u32(&cs.stage), p.stages + where + 1, (uint32_t)sizeof(Stage), smem_u32(&cs.rec_full));
-    }
-    if (!skip) {
-      bool there = ld_acquire_u32(count) >= target;
+    const unsigned* count = p.sync;
+    const unsigned target = (unsigned)si * gridDim.x;
 #pragma unroll
-      for (int i = 0; i < 7; ++i)
-        if (!there) there = ld_acquire_u32(count) >= target;
-      if (!there) grid_wait_loop(count, target, ctl, where);
-    }
-    if (fetch) mbar_wait_hot(smem_u32(&cs.rec_full), (uint32_t)where & 1u, ctl, 50);
+    for (int i = 0; i < 8; ++i)
+      if (!there) there = ld_acquire_u32(count) >= target;
+    if (!there) there = grid_wait_loop(count, target, ctl, si - 1);
+    fence_proxy_async_global();
   }
-  __syncthreads();
-  fence_proxy_async_global();     // the other CTAs' global writes (acquired above) before this CTA's TMA and bulk-copy reads
-  fence_proxy_async_smem();       // this thread's accesses to shared memory before the next stage's copies into it
-  return *ctl.abort_smem == 0;
+  if (p.prof) {
+    const long long now = clock_now();
+    p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 0] = now;
+    if (si > 0) p.prof[((size_t)(si - 1) * gridDim.x + blockIdx.x) * kProfSlots + 2] = now;
+  }
+  return there;
+}
+// Bounded wait for a word of this CTA's shared memory that only grows.  (It records nothing: its writer's own waits have the same
+// limit and do.)
+__device__ __noinline__ bool wait_word_loop(uint32_t word, uint32_t want, const WaitCtl& ctl) {
+  uint32_t spins = 0;
+  while (ld_acquire_cta_shared_u32(word) < want) {
+    if (((++spins) & 0xFF) == 0 && (*ctl.abort_smem || globaltimer_ns() > ctl.deadline_ns)) return false;
+  }
+  return true;
+}
+__device__ __forceinline__ bool wait_word(uint32_t word, uint32_t want, const WaitCtl& ctl) {
+  return ld_acquire_cta_shared_u32(word) >= want || wait_word_loop(word, want, ctl);
+}
+// One thread: this CTA's arrival for stage si - 1 is on its way.  Copies issued before that would delay it: its release waits for
+// them too.
+__device__ __forceinline__ bool wait_arrived(SmemCtl& cs, int si, const WaitCtl& ctl) { return wait_word(smem_u32(&cs.arrived), (uint32_t)si, ctl); }
+// The feeder's word that stage si may start, for warps that read global memory by themselves.
+__device__ __forceinline__ void publish_go(SmemCtl& cs, int si) { st_release_cta_shared_u32(smem_u32(&cs.go), (uint32_t)si + 1u); }
+__device__ __forceinline__ bool wait_go(SmemCtl& cs, int si, const WaitCtl& ctl) {      // whole warps
+  return __all_sync(0xffffffffu, wait_word(smem_u32(&cs.go), (uint32_t)si + 1u, ctl));
 }
 
 // The warp's index as a value the compiler knows to be the same in all its lanes (see elect_one).
@@ -510,45 +533,83 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     named_barrier_sync(1, kEpiThreads);
   }
 
+  // CTAs start at different K chunks so they do not all pull the same A tile at once
+  auto first_chunk = [&](int item) {
+    const uint32_t rot = (uint32_t)first_item + (uint32_t)item;
+    return (int)(rot - fast_div(rot, (uint32_t)g.kchunks, st.mg_kchunks) * (uint32_t)g.kchunks);
+  };
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
+    // ---------------- feeder: activation tiles, behind the grid barrier ----------------
     if (elect_one()) {
       const CUtensorMap* tmA = map_ptr(ca, st.tm_a);
-      const CUtensorMap* tmB = map_ptr(ca, st.tm_b);
-      bool ok = true;
       unsigned t_wait = 0;
-      long long t_first = 0;
       const bool prof = p.prof != nullptr;
       uint32_t s = rs.slot, bits = rs.slot_bits;
-      const bool b_mn = st.b_mn_major != 0;
-      for (int item = first_item; ok && item < g.items; item += item_step) {
-        int mt, nt, ks;
-        gemm_item(st, item, mt, nt, ks);
-        const int m0 = mt * g.bm + (int)rank * 128, n0 = nt * g.bn + (int)rank * (g.bn >> 1), kbase = ks * g.kchunks;
-        // CTAs start at different K chunks so they do not all pull the same A tile at once
-        const uint32_t rot = (uint32_t)first_item + (uint32_t)item;
-        int kk = (int)(rot - fast_div(rot, (uint32_t)g.kchunks, st.mg_kchunks) * (uint32_t)g.kchunks);
+      int mt, nt, ks;
+      gemm_item(st, first_item, mt, nt, ks);
+      int kk = first_chunk(first_item);
+      bool ok = grid_wait(p, ctl, st.prof_index);
+      const long long t_first = prof ? clock64() : 0;
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      for (int item = first_item; ok && item < g.items;) {
+        const int m0 = mt * g.bm + (int)rank * 128, kbase = ks * g.kchunks;
         for (int kc = 0; kc < g.kchunks; ++kc) {
           const long long tw = prof ? clock64() : 0;
           if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 100 + (int)s)) { ok = false; break; }
           if (prof) t_wait += (unsigned)(clock64() - tw);
-          const uint32_t fb = full0 + 8 * s;
-          const uint32_t a_dst = ring + s * g.slot_bytes, b_dst = a_dst + a_bytes;
-          const int k0 = (kbase + kk) * 64;
-          if (prof && !t_first) t_first = clock64();
+          const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes;
           if constexpr (kPair) {
             // both CTAs' bytes are counted on the leader's barrier, which only the leader arms
-            if (rank == 0) mbar_expect_tx(fb, 2u * (uint32_t)g.slot_bytes);
-            const uint32_t fbl = map_shared_rank(fb, 0);
-            tma_load_2d_pair(a_dst, tmA, fbl, k0, m0);          // box rows = 128: this CTA's half of the rows
-            tma_load_2d_pair(b_dst, tmB, fbl, k0, n0);          // box rows = bn / 2: this CTA's half of the columns
+            if (rank == 0) mbar_expect_tx(fb, 2u * a_bytes);
+            tma_load_2d_pair(dst, tmA, map_shared_rank(fb, 0), (kbase + kk) * 64, m0);      // box rows = 128: this CTA's half of the rows
           } else {
-            mbar_expect_tx(fb, (uint32_t)g.slot_bytes);
-            tma_load_2d(a_dst, tmA, fb, k0, m0);                // box rows = bm: both halves in one copy
+            mbar_expect_tx(fb, a_bytes);
+            tma_load_2d(dst, tmA, fb, (kbase + kk) * 64, m0);      // box rows = bm: both halves in one copy
+          }
+          bits ^= 1u << s;
+          s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
+          kk = (kk + 1 == g.kchunks) ? 0 : kk + 1;
+        }
+        item += item_step;
+        gemm_item(st, item, mt, nt, ks);
+        kk = first_chunk(item);
+      }
+      rs.slot = s;
+      rs.slot_bits = bits;
+      if (p.prof) {
+        long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
+        pr[5] = t_wait;
+        pr[11] = t_first;
+      }
+    }
+    __syncwarp();
+  } else if (warp == kWeightWarp) {
+    // ---------------- weight tiles: no stage writes them, so they are requested as soon as there are slots ----------------
+    // (a lane of its own: a copy takes the issuing thread 100 cycles and more, which behind the barrier is the stage's latency)
+    if (elect_one()) {
+      const CUtensorMap* tmB = map_ptr(ca, st.tm_b);
+      uint32_t s = rs.slot, bits = rs.slot_bits;
+      const bool b_mn = st.b_mn_major != 0;
+      const uint32_t b_bytes = (uint32_t)g.slot_bytes - a_bytes;
+      bool ok = wait_arrived(ctl_s, st.prof_index, ctl);
+      for (int item = first_item; ok && item < g.items; item += item_step) {
+        int mt, nt, ks;
+        gemm_item(st, item, mt, nt, ks);
+        const int n0 = nt * g.bn + (int)rank * (g.bn >> 1), kbase = ks * g.kchunks;
+        int kk = first_chunk(item);
+        for (int kc = 0; kc < g.kchunks; ++kc) {
+          if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 110 + (int)s)) { ok = false; break; }
+          const int k0 = (kbase + kk) * 64;
+          const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes + a_bytes;
+          if constexpr (kPair) {
+            if (rank == 0) mbar_expect_tx(fb, 2u * b_bytes);
+            tma_load_2d_pair(dst, tmB, map_shared_rank(fb, 0), k0, n0);          // box rows = bn / 2: this CTA's half of the columns
+          } else {
+            mbar_expect_tx(fb, b_bytes);
             if (!b_mn) {
-              tma_load_2d(b_dst, tmB, fb, k0, n0);
+              tma_load_2d(dst, tmB, fb, k0, n0);
             } else {
-              for (int j = 0; j < g.bn / 64; ++j) tma_load_2d(b_dst + j * 8192, tmB, fb, n0 + j * 64, k0);
+              for (int j = 0; j < g.bn / 64; ++j) tma_load_2d(dst + j * 8192, tmB, fb, n0 + j * 64, k0);
             }
           }
           bits ^= 1u << s;
@@ -558,11 +619,6 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       }
       rs.slot = s;
       rs.slot_bits = bits;
-      if (p.prof) {
-        long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
-        pr[5] = t_wait;
-        pr[11] = t_first;
-      }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -821,7 +877,9 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
 
   if (warp == 0) {
     if (lane == 0) {
-      for (int item = blockIdx.x; item < items; item += gridDim.x) {
+      const bool ok = grid_wait(p, ctl, st.prof_index);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
         const int qt = item % n_kb, h = (item / n_kb) % H, b = item / (n_kb * H);
         const int rq = ((0 * B + b) * H + h) * S, rk = ((1 * B + b) * H + h) * S, rv = ((2 * B + b) * H + h) * S;
         if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 500)) break;
@@ -1048,7 +1106,9 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
   if (warp == 0) {
     if (elect_one()) {
       uint32_t bits = rs.attn_bit | (rs.attn_bit1 << 1);
-      for (int k = 0; k < my_items; ++k) {
+      const bool ok = grid_wait(p, ctl, st.prof_index);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      for (int k = 0; ok && k < my_items; ++k) {
         const int item = item_of(k), g = k & 1;
         const int h = item % H, b = item / H;
         const int rq = ((0 * B + b) * H + h) * S, rk = ((1 * B + b) * H + h) * S, rv = ((2 * B + b) * H + h) * S;
@@ -1376,8 +1436,9 @@ __device__ __forceinline__ float swin_softmax_row(uint32_t tmem, const float* bi
   return rowok ? sum : 1.0f;
 }
 
-__device__ __noinline__ void attn_swin_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, uint8_t* ring_ptr,
-                                uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
+__device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, uint8_t* ring_ptr,
+                                uint8_t* stage_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
+  RoleState rs = RoleState::unpack(state);
   const int R = st.seq, ws = st.win, shift = st.shift, H = st.heads, C = st.ldo;
   const int nwr = R / ws, nw_img = nwr * nwr, n_windows = st.batch * nw_img, n_tok = ws * ws;
   const uint32_t n = (uint32_t)st.bn;                                // windows and heads per item: 1 or 2
@@ -1391,7 +1452,9 @@ __device__ __noinline__ void attn_swin_stage(const Stage& st, const CallArgs& ca
   // TMEM: scores of (head g, window j) at column 64 (2 g + j), outputs 256 further on
   if (warp == 0) {
     if (lane == 0) {
-      for (int item = blockIdx.x; item < items; item += gridDim.x) {
+      const bool ok = grid_wait(ca.p, ctl, st.prof_index);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
         const int wp = item / item_h, w0 = wp * (int)n, col = ((item - wp * item_h) * (int)n >> 1) * 64;
         if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 530)) break;
         mbar_expect_tx(qk_full, 2u * kATileBytes);
@@ -1490,6 +1553,23 @@ __device__ __noinline__ void attn_swin_stage(const Stage& st, const CallArgs& ca
       tc_fence_before_sync();
       rs.attn_bit ^= 1u;
     }
+  }
+  return rs.pack();
+}
+
+// Intermediates that the previous stage read for the last time (the barrier behind it has been passed by every CTA):
+// this CTA's share of their lines is dropped from L2 before anything evicts them to DRAM.  Out of line: a few
+// instructions per thread and stage, whose registers are not charged to the stages.
+// Threads tid0 .. tid0 + nthr - 1 of every CTA share the work: all of them in a LayerNorm stage, a spare warp in the other
+// stages.
+__device__ __noinline__ void drop_dead_buffers(const Stage& st, int tid0, int nthr) {
+  const int tid = (int)threadIdx.x - tid0;
+#pragma unroll 1
+  for (int b = 0; b < 2; ++b) {
+    const uint32_t lines = st.dead_bytes[b] >> 7;
+    if (!lines) continue;
+    const char* base = reinterpret_cast<const char*>(st.dead_ptr[b]);
+    for (uint32_t i = blockIdx.x * nthr + tid; i < lines; i += gridDim.x * nthr) discard_l2_128(base + ((size_t)i << 7));
   }
 }
 
@@ -1692,123 +1772,155 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
   }
 }
 
-// One row of the direct form: the lanes of a warp read the row straight from L2.  Every round trip costs ~800 cycles,
-// so the loads are issued in as few dependent rounds as the registers allow: bias, residual and the first planes
-// together, further planes kG at a time, gamma and beta just before the statistics (they land while the shuffles run).
-// With the loads strung one behind the other a row of six planes took 6.2 k cycles.
-template <int NJ>
-__device__ __forceinline__ void ln_row_direct(const float* pl, int n_partial, int plane_stride, const __half* res,
-                                              const __half* bias, const __half* gamma, const __half* beta, float eps,
-                                              __half* out, __half* sum_out, int lane) {
-  constexpr int kG = NJ <= 4 ? 4 : (NJ <= 6 ? 3 : 2);      // planes in flight at once
-  float z[NJ][4];
-  {
-    uint2 ub[NJ], ur[NJ];
-    float4 v[kG][NJ];
+// Rows read straight from L2.  W = N / 256 warps share a row (one for a row of 128 columns): lane l of part w holds columns
+// 256 w + 4 l .. + 3 and those 128 further on.  So 12 / W rows are in flight per CTA, dealt out over the CTAs first.  What a row
+// costs is latency: one L2 round trip for its planes, then a dependent chain in code that is cold when a CTA has one row, and
+// both the chain and the code grow with the columns a lane holds; with fewer columns than eight the shuffles of all the warps
+// cost more than they save.  The next row's loads are issued as soon as this row's sum is formed, and bias, gamma and beta are
+// loaded once per stage, in front of the wait for the stage's start.  Sets of columns are merged as (mean, squared deviations
+// from it), which is as exact as a second pass over the row (Chan, Golub, LeVeque) and needs one chain of shuffles and one
+// exchange between the parts.
+// Out of line: its registers are not charged to the stage interpreter.  `red`: 192 bytes of shared memory.
+__device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
+  constexpr int NJ = 2, kG = 2;                           // blocks of 128 columns per warp, planes in flight at once
+  const int N = st.N, M = st.M, P = st.n_partial, W = st.splitk, G = (kThreads / 32) / W;
+  const int grp = (int)fast_div((uint32_t)warp, (uint32_t)W, st.mg_splitk), part = warp - grp * W;
+  const int col = part * NJ * 128 + lane * 4;
+  const bool both = N > 128;
+  const size_t plane = (size_t)M * N;
+  const float* planes = st.partial + col;
+  const __half* resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
+  __half* out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p))) + col;
+  __half* sum_out = st.sum_out ? reinterpret_cast<__half*>(st.sum_out) + col : nullptr;
+  const float eps = st.eps;
+  const int step = (int)gridDim.x * G;
+  int row = grp < G ? grp * (int)gridDim.x + (int)blockIdx.x : M;
+  uint2 ub[NJ], ug[NJ], ubt[NJ], ur[NJ];
+  float4 v[kG][NJ];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      ub[j] = bias ? __ldg(reinterpret_cast<const uint2*>(bias + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
-      ur[j] = res ? __ldcg(reinterpret_cast<const uint2*>(res + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
-    }
+  for (int j = 0; j < NJ; ++j) {
+    const __half *bias = reinterpret_cast<const __half*>(st.bias), *gamma = reinterpret_cast<const __half*>(st.gamma),
+                 *beta = reinterpret_cast<const __half*>(st.beta);
+    ub[j] = bias && (j == 0 || both) ? __ldg(reinterpret_cast<const uint2*>(bias + col + 128 * j)) : make_uint2(0u, 0u);
+    ug[j] = gamma && (j == 0 || both) ? __ldg(reinterpret_cast<const uint2*>(gamma + col + 128 * j)) : make_uint2(0u, 0u);
+    ubt[j] = gamma && (j == 0 || both) ? __ldg(reinterpret_cast<const uint2*>(beta + col + 128 * j)) : make_uint2(0u, 0u);
+  }
+  const bool affine = st.gamma != nullptr;
+  const float inv_n = 1.0f / (float)N;
+  red += grp * W;
+  bool go = true;
+  if (warp == 0) {
+    if (lane == 0) go = grid_wait(p, ctl, st.prof_index);
+    if (lane == 0 && go) publish_go(cs, st.prof_index);
+    go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
+  } else {
+    go = wait_go(cs, st.prof_index, ctl);
+  }
+  if (!go) return;
+  auto load_planes = [&](int r, int g0) {
+    const float* src = planes + (size_t)r * N + (size_t)g0 * plane;
 #pragma unroll
-    for (int g = 0; g < kG; ++g)
+    for (int g = 0; g < kG; ++g, src += plane)
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
-        v[g][j] = g < n_partial ? __ldcg(reinterpret_cast<const float4*>(pl + (size_t)g * plane_stride + (lane + 32 * j) * 4))
-                                : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[g][j] = g0 + g < P && (j == 0 || both) ? __ldcg(reinterpret_cast<const float4*>(src + 128 * j)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto load_row = [&](int r) {
+    load_planes(r, 0);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+      ur[j] = resid && (j == 0 || both) ? __ldcg(reinterpret_cast<const uint2*>(resid + (size_t)r * N + col + 128 * j)) : make_uint2(0u, 0u);
+  };
+  if (row < M) load_row(row);
+  if (st.dead_bytes[0]) drop_dead_buffers(st, 0, kThreads);       // while the first rows are on their way
+#pragma unroll 1
+  for (uint32_t turn = 0; row < M; row += step, turn ^= 1u) {
+    float z[NJ][4];
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
       const float2 b0 = __half22float2(*reinterpret_cast<const __half2*>(&ub[j].x)), b1 = __half22float2(*reinterpret_cast<const __half2*>(&ub[j].y));
       const float2 r0 = __half22float2(*reinterpret_cast<const __half2*>(&ur[j].x)), r1 = __half22float2(*reinterpret_cast<const __half2*>(&ur[j].y));
       z[j][0] = b0.x + r0.x; z[j][1] = b0.y + r0.y; z[j][2] = b1.x + r1.x; z[j][3] = b1.y + r1.y;
-#pragma unroll
-      for (int g = 0; g < kG; ++g) { z[j][0] += v[g][j].x; z[j][1] += v[g][j].y; z[j][2] += v[g][j].z; z[j][3] += v[g][j].w; }
     }
-    for (int p0 = kG; p0 < n_partial; p0 += kG) {
-#pragma unroll
-      for (int g = 0; g < kG; ++g)
-#pragma unroll
-        for (int j = 0; j < NJ; ++j)
-          v[g][j] = p0 + g < n_partial ? __ldcg(reinterpret_cast<const float4*>(pl + (size_t)(p0 + g) * plane_stride + (lane + 32 * j) * 4))
-                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int g0 = 0;;) {                                  // deep splits: further rounds
 #pragma unroll
       for (int j = 0; j < NJ; ++j)
 #pragma unroll
         for (int g = 0; g < kG; ++g) { z[j][0] += v[g][j].x; z[j][1] += v[g][j].y; z[j][2] += v[g][j].z; z[j][3] += v[g][j].w; }
+      g0 += kG;
+      if (g0 >= P) break;
+      load_planes(row, g0);
     }
-  }
-  if (sum_out) {                        // the sum itself, as fp16; what is normalised below is the rounded value
+    if (row + step < M) load_row(row + step);
+    __half* o = out + (size_t)row * N;
+    if (eps < 0.0f || sum_out) {        // the sum itself, as fp16; what is normalised below is the rounded value
+      __half* so = eps < 0.0f ? o : sum_out + (size_t)row * N;
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        const uint2 w = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
+        if (j == 0 || both) *reinterpret_cast<uint2*>(so + 128 * j) = w;
+        const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+        z[j][0] = f0.x; z[j][1] = f0.y; z[j][2] = f1.x; z[j][3] = f1.y;
+      }
+      if (eps < 0.0f) continue;         // sum only
+    }
+    // (mean, sum of squared deviations from it) of the lane's columns, then of twice as many with every step: a pair of
+    // equally large sets has the mean of the means, and its deviations grow by (difference of the means)^2 n / 2
+    float row_mean = 0.0f, va = 0.0f;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) row_mean += (z[j][0] + z[j][1]) + (z[j][2] + z[j][3]);
+    row_mean *= both ? 0.125f : 0.25f;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float d = z[j][i] - row_mean;
+        if (j == 0 || both) va = fmaf(d, d, va);
+      }
+    const float half_n = both ? 4.0f : 2.0f;
+#pragma unroll
+    for (int o2 = 1; o2 < 32; o2 <<= 1) {
+      const float m2 = __shfl_xor_sync(0xffffffffu, row_mean, o2), v2 = __shfl_xor_sync(0xffffffffu, va, o2);
+      const float d = m2 - row_mean;
+      va = fmaf(d * d, half_n * (float)o2, va + v2);
+      row_mean = 0.5f * (row_mean + m2);
+    }
+    if (W > 1) {
+      float2* slot = red + turn * (kThreads / 32);        // two sets, used by alternate rows: one barrier per row is enough
+      if (lane == 0) slot[part] = make_float2(row_mean, va);
+      named_barrier_sync(4 + grp, W * 32);
+      float2 t[8];                                        // W <= 8
+      float total = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        t[i] = i < W ? slot[i] : make_float2(0.f, 0.f);
+        total += t[i].x;
+      }
+      row_mean = total * ((float)(NJ * 128) * inv_n);
+      va = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float d = i < W ? t[i].x - row_mean : 0.0f;
+        va += fmaf(d * d, (float)(NJ * 128), t[i].y);
+      }
+    }
+    const float rstd = rsqrtf(va * inv_n + eps), nm = -row_mean * rstd;
+    // (z - mean) * rstd in fp32 (one FMA), rounded to fp16 pairs; gamma and beta are applied on the pairs (one packed
+    // FMA per two elements, no conversions).  With gamma = 1, beta = 0 that last step is exact.
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      const uint2 w = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
-      *reinterpret_cast<uint2*>(sum_out + (lane + 32 * j) * 4) = w;
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
-      z[j][0] = f0.x; z[j][1] = f0.y; z[j][2] = f1.x; z[j][3] = f1.y;
-    }
-    if (eps < 0.0f) return;             // sum only
-  }
-  uint2 ug[NJ], ubt[NJ];
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    ug[j] = gamma ? __ldg(reinterpret_cast<const uint2*>(gamma + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
-    ubt[j] = gamma ? __ldg(reinterpret_cast<const uint2*>(beta + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
-  }
-  const float inv_n = 1.0f / (float)(NJ * 128);
-  float sa = 0.0f;
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) sa += (z[j][0] + z[j][1]) + (z[j][2] + z[j][3]);
-  sa = warp_sum(sa);
-  const float mean = sa * inv_n;
-  float va = 0.0f;
-#pragma unroll
-  for (int j = 0; j < NJ; ++j)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float d0 = z[j][i] - mean;
-      va = fmaf(d0, d0, va);
-    }
-  va = warp_sum(va);
-  const float rstd = rsqrtf(va * inv_n + eps), nm = -mean * rstd;
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    uint32_t w0 = pack_h2(fmaf(z[j][0], rstd, nm), fmaf(z[j][1], rstd, nm));
-    uint32_t w1 = pack_h2(fmaf(z[j][2], rstd, nm), fmaf(z[j][3], rstd, nm));
-    if (gamma) {
-      const __half2 y0 = __hfma2(*reinterpret_cast<const __half2*>(&w0), *reinterpret_cast<const __half2*>(&ug[j].x),
-                                 *reinterpret_cast<const __half2*>(&ubt[j].x));
-      const __half2 y1 = __hfma2(*reinterpret_cast<const __half2*>(&w1), *reinterpret_cast<const __half2*>(&ug[j].y),
-                                 *reinterpret_cast<const __half2*>(&ubt[j].y));
-      w0 = *reinterpret_cast<const uint32_t*>(&y0);
-      w1 = *reinterpret_cast<const uint32_t*>(&y1);
-    }
-    *reinterpret_cast<uint2*>(out + (lane + 32 * j) * 4) = make_uint2(w0, w1);
-  }
-}
-
-// Direct form of the LayerNorm stage (the host picks it when a CTA has at most one row per normalising warp): every
-// warp reads its row from global memory itself -- no copy issue, copy latency and barrier wait of the staging ring.
-// Out of line: its registers are not charged to the stage interpreter.
-__device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& p, int warp, int lane) {
-  const int N = st.N, M = st.M, P = st.n_partial, rb = st.bm, n_batches = st.items;
-  if (warp >= rb) return;
-  const __half* resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
-  __half* out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p)));
-  const __half* bias = reinterpret_cast<const __half*>(st.bias);
-  const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
-  const __half* beta = reinterpret_cast<const __half*>(st.beta);
-  for (int blk = blockIdx.x; blk < n_batches; blk += gridDim.x) {
-    const int row = blk * rb + warp;
-    if (row >= M) break;
-    const float* pl0 = st.partial + (size_t)row * N;
-    const __half* ra = resid ? resid + (size_t)row * N : nullptr;
-    __half* o0 = out + (size_t)row * N;
-    __half* so = st.eps < 0.0f ? o0 : st.sum_out ? reinterpret_cast<__half*>(st.sum_out) + (size_t)row * N : nullptr;
-    switch (N >> 7) {
-      case 1: ln_row_direct<1>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
-      case 2: ln_row_direct<2>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
-      case 4: ln_row_direct<4>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
-      case 6: ln_row_direct<6>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
-      default: ln_row_direct<8>(pl0, P, M * N, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      uint32_t w0 = pack_h2(fmaf(z[j][0], rstd, nm), fmaf(z[j][1], rstd, nm));
+      uint32_t w1 = pack_h2(fmaf(z[j][2], rstd, nm), fmaf(z[j][3], rstd, nm));
+      if (affine) {
+        const __half2 y0 = __hfma2(*reinterpret_cast<const __half2*>(&w0), *reinterpret_cast<const __half2*>(&ug[j].x),
+                                   *reinterpret_cast<const __half2*>(&ubt[j].x));
+        const __half2 y1 = __hfma2(*reinterpret_cast<const __half2*>(&w1), *reinterpret_cast<const __half2*>(&ug[j].y),
+                                   *reinterpret_cast<const __half2*>(&ubt[j].y));
+        w0 = *reinterpret_cast<const uint32_t*>(&y0);
+        w1 = *reinterpret_cast<const uint32_t*>(&y1);
+      }
+      if (j == 0 || both) *reinterpret_cast<uint2*>(o + 128 * j) = make_uint2(w0, w1);
     }
   }
 }
@@ -1833,10 +1945,6 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
   // in flight, at most two rows per warp, and few enough that every CTA gets work -- buffers, batch count.
   const int row_bytes = (P * 4 + (resid ? 2 : 0)) * N;
   const int rb = st.bm, batch_bytes = st.slot_bytes, nbuf = st.nslots, n_batches = st.items;
-  if (nbuf == 0) {          // direct form: see ln_stage_direct
-    ln_stage_direct(st, p, warp, lane);
-    return;
-  }
   const bool stage_vecs = st.kchunks != 0;   // bias | gamma | beta side by side in shared memory
   const int my_batches = n_batches > (int)blockIdx.x ? (n_batches - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const uint32_t full0 = smem_u32(&cs.ln_full[0]), empty0 = smem_u32(&cs.ln_empty[0]);
@@ -1845,9 +1953,10 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
 
   if (warp == 0) {
     if (lane == 0) {
+      const bool go = grid_wait(p, ctl, st.prof_index);
       if (prof) p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 9] = clock64();
       int buf = 0;
-      for (int k = 0; k < my_batches; ++k) {
+      for (int k = 0; go && k < my_batches; ++k) {
         const int batch = blockIdx.x + k * gridDim.x;
         if (!mbar_wait(empty0 + 8 * buf, ((bits >> buf) & 1u) ^ 1u, ctl, 610 + buf)) break;
         const int row0 = batch * rb;
@@ -1911,10 +2020,7 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
         __half* o0 = out + (size_t)(row0 + r) * N;
         __half* o1 = two ? out + (size_t)(row0 + r2) * N : nullptr;
         switch (N >> 7) {
-          case 1: ln_rows2<1>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
-          case 2: ln_rows2<2>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
           case 4: ln_rows2<4>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
-          case 6: ln_rows2<6>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
           case 16:
             if constexpr (kMerge) {
               ln_row_wide(ra, gamma, beta, st.eps, o0, lane);
@@ -1967,31 +2073,23 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
 //                    weight-tile traffic per FLOP of the GEMM stages; the attention stage takes two heads per pair.
 //                    Launched with a cluster dimension of two.
 constexpr int kFamilyBert = 0, kFamilyBertCoop = 1, kFamilySwin = 2, kFamilyBertPair = 3;
-__device__ __noinline__ void gemm_stage_ool(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
-                                            uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
-  RoleState r = rs;                    // a copy the roles can keep in registers
+__device__ __noinline__ uint32_t gemm_stage_ool(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
+                                            uint8_t* stage_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
+  RoleState r = RoleState::unpack(state);
   gemm_stage<true>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
-  rs = r;
+  return r.pack();
 }
-__device__ __noinline__ void ln_stage_ool(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
-                                          __half* vec_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
-  ln_stage<true>(st, p, cs, ring, ring_ptr, vec_s, rs, ctl, warp, lane);
+__device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
+                                          __half* vec_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
+  RoleState r = RoleState::unpack(state);
+  ln_stage<true>(st, p, cs, ring, ring_ptr, vec_s, r, ctl, warp, lane);
+  return r.pack();
 }
 
-// Intermediates that the previous stage read for the last time (the barrier behind it has been passed by every CTA):
-// this CTA's share of their lines is dropped from L2 before anything evicts them to DRAM.  Out of line: a few
-// instructions per thread and stage, whose registers are not charged to the stages.
-// Threads tid0 .. kThreads - 1 of every CTA share the work: all of them in front of a LayerNorm stage, the two spare
-// warps alone in front of the other stages, whose roles then start without it.
-__device__ __noinline__ void drop_dead_buffers(const Stage& st, int tid0) {
-  const int nthr = kThreads - tid0, tid = (int)threadIdx.x - tid0;
-#pragma unroll 1
-  for (int b = 0; b < 2; ++b) {
-    const uint32_t lines = st.dead_bytes[b] >> 7;
-    if (!lines) continue;
-    const char* base = reinterpret_cast<const char*>(st.dead_ptr[b]);
-    for (uint32_t i = blockIdx.x * nthr + tid; i < lines; i += gridDim.x * nthr) discard_l2_128(base + ((size_t)i << 7));
-  }
+// One warp copies a stage record to shared memory.
+__device__ __forceinline__ void copy_record(Stage* to, const Stage* from, int lane) {
+  static_assert(sizeof(Stage) % 16 == 0, "records are copied 16 bytes at a time");
+  for (int i = lane; i < (int)(sizeof(Stage) / 16); i += 32) reinterpret_cast<uint4*>(to)[i] = reinterpret_cast<const uint4*>(from)[i];
 }
 
 template <int kFamily>
@@ -2015,7 +2113,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kMaxSlots; ++i) {
-      mbar_init(smem_u32(&cs.full[i]), 1);
+      mbar_init(smem_u32(&cs.full[i]), 2);        // armed by the feeder and by the weight warp
       mbar_init(smem_u32(&cs.empty[i]), 1);
     }
     constexpr bool kPairK = kFamily == kFamilyBertPair;
@@ -2025,7 +2123,6 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       mbar_init(smem_u32(&cs.tmem_empty[i]), kPairK ? 2 * kEpiWarps : kEpiThreads);
       mbar_init(smem_u32(&cs.o_empty[i]), 8);
     }
-    mbar_init(smem_u32(&cs.rec_full), 1);
     mbar_init(smem_u32(&cs.qk_full), 1);
     mbar_init(smem_u32(&cs.qk_empty), 1);
     mbar_init(smem_u32(&cs.v_full), 1);
@@ -2039,7 +2136,11 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       mbar_init(smem_u32(&cs.ln_empty[i]), kThreads / 32 - 1);
     }
     cs.abort = 0;
-    cs.deadline_ns = globaltimer_ns() + p.timeout_ns;
+    cs.leave[0] = cs.leave[1] = 0;
+    cs.go = cs.arrived = 0u;
+    cs.wait.abort_smem = &cs.abort;
+    cs.wait.status_g = p.status;
+    cs.wait.deadline_ns = globaltimer_ns() + p.timeout_ns;      // read once per CTA
     fence_mbar_init();
     if (blockIdx.x == 0) {          // the other launch parity's barrier words start clean
       p.sync_next[0] = 0u;
@@ -2051,6 +2152,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   } else {
     if (warp == 1) tmem_alloc(smem_u32(&cs.tmem_base), kTmemCols);
   }
+  if (warp == 0) copy_record(&cs.stage[0], p.stages ? p.stages : &ca.inline_stages[0], lane);
   if (warp >= 2 && p.maps) {               // warm the descriptor cache while the CTA sets up
     for (int i = (int)threadIdx.x - 64; i < p.n_maps; i += kThreads - 64) tma_prefetch_desc(p.maps + i);
   }
@@ -2059,10 +2161,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   if constexpr (kFamily == kFamilyBertPair) cluster_sync_all();     // the peer's barriers exist before anything arrives on them
   tc_fence_after_sync();
 
-  WaitCtl ctl;
-  ctl.abort_smem = &cs.abort;
-  ctl.status_g = p.status;
-  ctl.deadline_ns = cs.deadline_ns;
+  const WaitCtl& ctl = cs.wait;
   if (p.prof && threadIdx.x == 0) {          // one record past the stages: kernel entry, prologue done, ...
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[1] = clock64();
@@ -2070,23 +2169,29 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
 
   RoleState rs;
   for (int si = 0; si < p.n_stages; ++si) {
-    // stage record -> shared memory (uniform, read-only afterwards).  Records of a plan-owned program arrive during
-    // the barrier before the stage (grid_barrier), except the first; the stages of the plan-less entry points travel
-    // in the launch parameters and are copied here.
-    if (si == 0 || !p.stages) {
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(p.stages ? p.stages + si : &ca.inline_stages[si]);
-      uint32_t* dst = reinterpret_cast<uint32_t*>(&cs.stage);
-      for (int i = threadIdx.x; i < (int)(sizeof(Stage) / 4); i += kThreads) dst[i] = src[i];
+    const Stage& st = cs.stage[si & 1];
+    // The spare warps' part, in front of anything that waits: the next stage's record (constant since the launch: plan-owned
+    // programs lie in global memory, the stages of the plan-less entry points in the launch parameters) goes to shared
+    // memory, and this CTA's slice of the next stage's weights to L2 (they come from HBM when the program's weights exceed
+    // L2; without this every GEMM stage starts with all CTAs waiting on the same DRAM rows).
+    if (warp == kWeightWarp && si + 1 < p.n_stages) copy_record(&cs.stage[(si + 1) & 1], p.stages ? p.stages + si + 1 : &ca.inline_stages[si + 1], lane);
+    if (warp == kSpareWarp && lane == 0) {
+      const uint32_t pf_bytes = st.pf_bytes;
+      if (pf_bytes) {
+        const uint32_t per = ((pf_bytes + gridDim.x - 1) / gridDim.x + 15u) & ~15u, off = blockIdx.x * per;
+        if (off < pf_bytes)
+          bulk_prefetch_l2(reinterpret_cast<const char*>(st.pf_ptr) + off, off + per <= pf_bytes ? per : pf_bytes - off);
+      }
     }
-    __syncthreads();
-    if (p.prof && threadIdx.x == 0) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 0] = clock_now();
-    const Stage& st = cs.stage;
-    if (st.type == STAGE_LN) drop_dead_buffers(st, 0);
-    else if (warp >= 2 + kEpiWarps) drop_dead_buffers(st, (2 + kEpiWarps) * 32);
+    __syncwarp();
+    if (st.type != STAGE_LN && warp == kSpareWarp && st.dead_bytes[0]) {
+      if (wait_go(cs, si, ctl)) drop_dead_buffers(st, warp * 32, 32);
+    }
     if constexpr (kFamily == kFamilySwin) {
-      if (st.type == STAGE_GEMM) gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
-      else if (st.type == STAGE_ATTN_SWIN) attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
-      else if (st.type == STAGE_LN) ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, rs, ctl, warp, lane);
+      if (st.type == STAGE_GEMM) rs = RoleState::unpack(gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, rs.pack(), ctl, warp, lane));
+      else if (st.type == STAGE_ATTN_SWIN) rs = RoleState::unpack(attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, rs.pack(), ctl, warp, lane));
+      else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+      else if (st.type == STAGE_LN) rs = RoleState::unpack(ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, rs.pack(), ctl, warp, lane));
     } else {
       if (st.type == STAGE_GEMM) {
         gemm_stage<false, kFamily == kFamilyBertPair>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
@@ -2095,17 +2200,24 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
         else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
         else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
       } else if (st.type == STAGE_LN) {
-        ln_stage<false>(st, p, cs, ring, ring_ptr, vec_s, rs, ctl, warp, lane);
+        ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
       }
     }
-    if (si + 1 < p.n_stages) {
-      if (!grid_barrier(p, ctl, si, cs)) break;
-    } else {
-      __syncthreads();
-      if (p.prof && threadIdx.x == 0) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
+    // Every thread comes by here once per stage, whatever became of its waits, and all leave the loop together.
+    fence_proxy_async_smem();             // this thread's accesses to shared memory before the next stage's copies into it
+    if (*ctl.abort_smem) cs.leave[si & 1] = 1;       // two words in turn: the next stage's is not written before all have read this one
+    __syncthreads();
+    if (*const_cast<volatile int*>(&cs.leave[si & 1])) break;
+    if (warp == kSpareWarp && lane == 0) {
+      if (p.prof) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
+      if (si + 1 < p.n_stages) {
+        if (p.skip_arrival > 0 && si == 0 && (int)blockIdx.x == p.skip_arrival - 1) *ctl.abort_smem = 1;      // test hook
+        else red_add_release_u32(p.sync, 1u);
+        st_release_cta_shared_u32(smem_u32(&cs.arrived), (uint32_t)si + 1u);
+      } else if (p.prof) {
+        p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 2] = clock_now();
+      }
     }
-    if (p.prof && threadIdx.x == 0) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 2] = clock_now();
-    if (cs.abort) break;
   }
 
   __syncthreads();

@@ -351,7 +351,7 @@ static int stage_items(const Stage& s, bool pair = false) {
   if (s.type == STAGE_ATTN) return s.batch * s.heads * ((s.seq + 127) / 128);
   if (s.type == STAGE_ATTN_SWIN)      // s.bn windows x s.bn heads
     return (s.batch * (s.seq / s.win) * (s.seq / s.win) + s.bn - 1) / s.bn * (s.heads / s.bn);
-  return (s.M + kThreads / 32 - 2) / (kThreads / 32 - 1);       // one row per normalising warp (all warps but the first)
+  return s.M;       // rows are dealt out over the CTAs first
 }
 
 // Fills the derived fields of a GEMM stage (tile counts, ring geometry, magic divisors) and checks that its
@@ -374,13 +374,13 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
     s.nslots = 196608 / s.slot_bytes > 4 ? 4 : 196608 / s.slot_bytes;
     s.items = (s.M + rb - 1) / rb;
     s.kchunks = (3 * s.N * 2 <= kVecBytes) ? 1 : 0;
-    // Rows of up to 1024 columns that need no gather: the warps read their rows from L2 themselves, one row per
-    // normalising warp and pass (no staging ring).  Measured faster than the ring at every batch size: twelve layers
-    // at 16 sequences 0.87 against 0.93 ms, equal at 64.
+    // Rows of up to 1024 columns that need no gather: the warps read them from L2 themselves, s.splitk warps per row
+    // (ln_stage_direct).
     if (s.seq == 0 && s.N <= 1024) {
-      if (per_cta > comp + 1) per_cta = comp + 1;       // every warp takes a row
-      s.bm = per_cta;
-      s.items = (s.M + per_cta - 1) / per_cta;
+      s.splitk = s.N <= 256 ? 1 : s.N / 256;
+      s.mg_splitk = fast_div_magic((uint32_t)s.splitk);
+      s.bm = 1;
+      s.items = s.M;
       s.nslots = 0;
       s.kchunks = 0;
       return SOUFFLE_OK;
@@ -544,24 +544,33 @@ namespace souffle {
 
 static int plan_alloc(SouffleBertPlan* p, void** ptr, size_t bytes);
 
+constexpr size_t kL2Bytes = (size_t)126 << 20, kStagesPerLayer = 7;
+
 // Numbers the stages and copies the program and its tensor maps to the device.
 static int upload_program(SouffleBertPlan* p) {
   int rc;
   for (size_t i = 0; i < p->stages.size(); ++i) {
     Stage& s = p->stages[i];
     s.prof_index = (int)i;
-    // the weights of the GEMM stage after next are prefetched into L2 at the barrier that ends this stage
+    // the weights of the GEMM stage that comes next are prefetched into L2 while this stage runs
     s.pf_ptr = nullptr;
     s.pf_bytes = 0;
-    if (i + 2 < p->stages.size() && p->stages[i + 2].type == STAGE_GEMM && p->stage_weights.size() > i + 2 && p->stage_weights[i + 2]) {
-      const Stage& g = p->stages[i + 2];
-      s.pf_ptr = p->stage_weights[i + 2];
+    if (i + 1 < p->stages.size() && p->stages[i + 1].type == STAGE_GEMM && p->stage_weights.size() > i + 1 && p->stage_weights[i + 1]) {
+      const Stage& g = p->stages[i + 1];
+      s.pf_ptr = p->stage_weights[i + 1];
       s.pf_bytes = (uint32_t)((size_t)g.N * g.K * 2) & ~15u;
     }
     s.dead_bytes[0] = s.dead_bytes[1] = 0;
     s.dead_ptr[0] = s.dead_ptr[1] = nullptr;
   }
+  // Buffers are dropped from L2 only where a layer's intermediates together are larger than it: smaller ones are written anew
+  // before anything evicts them, and the drops cost time (twelve layers at 32 sequences, 88 MB: 1130 us with them, 1110
+  // without; at 16, 44 MB: 787 and 770).  Beyond that they keep dead data from being written to DRAM.
+  size_t live = 0;
+  for (const SouffleBertPlan::Dead& dd : p->dead_after)
+    if (dd.after_stage < kStagesPerLayer) live += dd.bytes;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {
+    if (live <= kL2Bytes) break;
     if (dd.after_stage + 1 >= p->stages.size()) continue;          // nothing runs after it inside the launch
     Stage& nx = p->stages[dd.after_stage + 1];
     const int k = nx.dead_bytes[0] ? 1 : 0;

@@ -30,7 +30,7 @@ enum Activation : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2 };
 // Pointer selectors: a stage either carries a plan-owned pointer or names a per-call argument.
 enum PtrSel : int { PTR_PLAN = 0, PTR_CALL_X = 1, PTR_CALL_Y = 2 };
 
-struct alignas(16) Stage {      // 16-byte multiples: records are fetched with bulk copies
+struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 bytes at a time
   int type;
   // ---- GEMM ----
   int tm_a;          // tensor-map index of the A operand ([M][K], box 64 x bm); negative = per-call map
@@ -67,8 +67,8 @@ struct alignas(16) Stage {      // 16-byte multiples: records are fetched with b
   void* sum_out;     // fp16 [M][N] or null: the sum (rounded to fp16, which is then what gets normalised) is stored here as well
   int n_partial;     // number of fp32 partial planes to sum
   int prof_index;    // position of this stage in the program (set by the host when the program is built)
-  // ---- weight prefetch: the B matrix of the GEMM stage two stages further on, pulled into L2 by all CTAs while
-  //      they wait at the barrier that ends this stage (weights never depend on an earlier stage) ----
+  // ---- weight prefetch: the B matrix of the next stage, a GEMM, pulled into L2 by all CTAs at the start of this one
+  //      (weights never depend on an earlier stage) ----
   uint32_t pf_bytes;
   const void* pf_ptr;
   // ---- buffers whose last reader was the stage before this one (multiples of 128 bytes, 128-byte aligned): their
