@@ -216,7 +216,7 @@ __device__ __forceinline__ uint32_t fast_div(uint32_t n, uint32_t d, uint32_t mg
 }
 
 struct GemmGeom {
-  int tiles_n, splitk, items, kchunks, bn, bm, nh, slot_bytes, nslots;
+  int tiles_n, splitk, items, kchunks, kper, bn, bm, nh, slot_bytes, nslots;
 };
 __device__ __forceinline__ GemmGeom gemm_geom(const Stage& st) {
   GemmGeom g;
@@ -227,6 +227,7 @@ __device__ __forceinline__ GemmGeom gemm_geom(const Stage& st) {
   g.splitk = st.splitk;
   g.items = st.items;
   g.kchunks = st.kchunks;
+  g.kper = st.kper;
   g.slot_bytes = st.slot_bytes;
   g.nslots = st.nslots;
   return g;
@@ -513,6 +514,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
   const uint32_t full0 = smem_u32(&ctl_s.full[0]), empty0 = smem_u32(&ctl_s.empty[0]);
   const uint32_t tfull0 = smem_u32(&ctl_s.tmem_full[0]), tempty0 = smem_u32(&ctl_s.tmem_empty[0]);
   const uint32_t a_bytes = (uint32_t)(g.nh * kATileBytes);
+  const uint32_t sub_bytes = (uint32_t)g.slot_bytes >> (g.kper - 1);       // a slot holds one or two K steps of 64, each its A tile and its B tile
   const uint32_t rank = kPair ? cluster_cta_rank() : 0u;               // 0 = the pair's leader
   const int first_item = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int item_step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -558,13 +560,15 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 100 + (int)s)) { ok = false; break; }
           if (prof) t_wait += (unsigned)(clock64() - tw);
           const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes;
+          const int k0 = (kbase + kk) * g.kper * 64;
           if constexpr (kPair) {
             // both CTAs' bytes are counted on the leader's barrier, which only the leader arms
             if (rank == 0) mbar_expect_tx(fb, 2u * a_bytes);
-            tma_load_2d_pair(dst, tmA, map_shared_rank(fb, 0), (kbase + kk) * 64, m0);      // box rows = 128: this CTA's half of the rows
+            tma_load_2d_pair(dst, tmA, map_shared_rank(fb, 0), k0, m0);      // box rows = 128: this CTA's half of the rows
           } else {
-            mbar_expect_tx(fb, a_bytes);
-            tma_load_2d(dst, tmA, fb, (kbase + kk) * 64, m0);      // box rows = bm: both halves in one copy
+            mbar_expect_tx(fb, a_bytes * (uint32_t)g.kper);
+            tma_load_2d(dst, tmA, fb, k0, m0);      // box rows = bm: both halves in one copy
+            if (g.kper == 2) tma_load_2d(dst + sub_bytes, tmA, fb, k0 + 64, m0);
           }
           bits ^= 1u << s;
           s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
@@ -590,7 +594,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       const CUtensorMap* tmB = map_ptr(ca, st.tm_b);
       uint32_t s = rs.slot, bits = rs.slot_bits;
       const bool b_mn = st.b_mn_major != 0;
-      const uint32_t b_bytes = (uint32_t)g.slot_bytes - a_bytes;
+      const uint32_t b_bytes = sub_bytes - a_bytes;
       bool ok = wait_arrived(ctl_s, st.prof_index, ctl);
       for (int item = first_item; ok && item < g.items; item += item_step) {
         int mt, nt, ks;
@@ -599,17 +603,20 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         int kk = first_chunk(item);
         for (int kc = 0; kc < g.kchunks; ++kc) {
           if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 110 + (int)s)) { ok = false; break; }
-          const int k0 = (kbase + kk) * 64;
+          const int k0 = (kbase + kk) * g.kper * 64;
           const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes + a_bytes;
           if constexpr (kPair) {
             if (rank == 0) mbar_expect_tx(fb, 2u * b_bytes);
             tma_load_2d_pair(dst, tmB, map_shared_rank(fb, 0), k0, n0);          // box rows = bn / 2: this CTA's half of the columns
           } else {
-            mbar_expect_tx(fb, b_bytes);
-            if (!b_mn) {
-              tma_load_2d(dst, tmB, fb, k0, n0);
-            } else {
-              for (int j = 0; j < g.bn / 64; ++j) tma_load_2d(dst + j * 8192, tmB, fb, n0 + j * 64, k0);
+            mbar_expect_tx(fb, b_bytes * (uint32_t)g.kper);
+            for (int sub = 0; sub < g.kper; ++sub) {
+              const uint32_t to = dst + (uint32_t)sub * sub_bytes;
+              if (!b_mn) {
+                tma_load_2d(to, tmB, fb, k0 + sub * 64, n0);
+              } else {
+                for (int j = 0; j < g.bn / 64; ++j) tma_load_2d(to + j * 8192, tmB, fb, n0 + j * 64, k0 + sub * 64);
+              }
             }
           }
           bits ^= 1u << s;
@@ -666,6 +673,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           } else {
             if (g.nh == 2) umma_f16_k64_x2(d0, d1, a_lo, b_lo, bstep, idesc, (uint32_t)(kc != 0));
             else umma_f16_k64(d0, a_lo, b_lo, bstep, idesc, (uint32_t)(kc != 0));
+            if (g.kper == 2) umma_f16_k64(d0, a_lo + (sub_bytes >> 4), b_lo + (sub_bytes >> 4), bstep, idesc, 1u);
             umma_commit(empty0 + 8 * s);
           }
           bits ^= 1u << s;

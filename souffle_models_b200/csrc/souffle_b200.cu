@@ -411,6 +411,14 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   s.items = stage_items(s);
   // per CTA and K chunk: the A rows (all of the tile's, or one 128-row half of a pair's) and the B rows (all, or half)
   s.slot_bytes = pair ? 16384 + s.bn * 64 : (s.bm / 128) * 16384 + s.bn * 128;
+  // Two steps of 64 per slot where three such slots fit: the lone lanes' wait, commit and bookkeeping are paid once per slot (a
+  // 128 x 16 tile: 390 -> 295 cycles per step).  With two slots left the copies no longer run ahead (16 sequences: 743 -> 774 us).
+  s.kper = 1;
+  if (!pair && max_slots == 0 && s.bm == 128 && s.kchunks % 2 == 0 && 196608 / (2 * s.slot_bytes) >= 3) {
+    s.kper = 2;
+    s.kchunks /= 2;
+    s.slot_bytes *= 2;
+  }
   int n = 196608 / s.slot_bytes;
   if (n > 8) n = 8;
   if (max_slots > 0 && n > max_slots) n = max_slots;
@@ -1220,7 +1228,7 @@ int souffle_bert_plan_stage_info(SouffleBertPlan* plan, int index, int out[6]) {
   if (index < 0 || index >= (int)plan->stages.size()) return fail(SOUFFLE_BAD_ARGUMENT, "stage index %d out of range", index);
   const Stage& s = plan->stages[index];
   out[0] = s.type; out[1] = s.bm; out[2] = s.bn; out[3] = s.splitk; out[4] = stage_items(s, plan->pair);
-  out[5] = s.type == STAGE_GEMM ? s.nslots : 0;
+  out[5] = s.type == STAGE_GEMM ? s.nslots * s.kper : 0;      // slots of one K step of 64
   return SOUFFLE_OK;
 }
 
@@ -1263,7 +1271,7 @@ static int ws_enter(void* workspace, cudaStream_t st, bool captured, unsigned* l
 }
 
 // Fills in what a launch takes from its workspace; args->p.n_stages is set.
-static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes, cudaStream_t st) {
+static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes, cudaStream_t st, int family = kFamilyBert) {
   if (!aligned16(workspace) || ws_bytes < souffle_gemm_workspace_bytes())
     return fail(SOUFFLE_BAD_POINTER, "workspace must be 16-byte aligned and hold %zu bytes", souffle_gemm_workspace_bytes());
   MegaParams* mp = &args->p;
@@ -1275,12 +1283,16 @@ static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes,
     return rc;
   mp->status = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsStatusOffset);
   mp->timeout_ns = 2000ull * 1000000ull;
-  if ((rc = launch_mega(*args, grid, st)) || captured) return rc;
+  if ((rc = launch_mega(*args, grid, st, family)) || captured) return rc;
   std::lock_guard<std::mutex> lock(g_ws_mutex);
   auto it = g_ws_launches.find(workspace);
   if (it != g_ws_launches.end()) ++it->second;          // only now: a call that was refused has used neither pair
   return SOUFFLE_OK;
 }
+
+// The build for a plan-less launch that sums or normalises M rows: with few rows per CTA the one that spreads a row over
+// several warps.
+static int row_family(int M, int grid) { return M <= grid * (kThreads / 32) ? kFamilyBertCoop : kFamilyBert; }
 
 static int fill_gemm_stage(Stage* s, int tm_a, int tm_b, const void* out, int M, int N, int K, int sms) {
   *s = blank_stage(STAGE_GEMM);
@@ -1370,7 +1382,7 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
     s3.eps = -1.0f;                                    // sum only
     if ((rc = finalize_stage(s3, 0, grid))) return rc;
   }
-  return ws_launch(&args, grid, workspace, workspace_bytes, st);
+  return ws_launch(&args, grid, workspace, workspace_bytes, st, row_family(M, grid));
 }
 
 int souffle_layernorm_forward(const float* partial, int32_t n_partial, const void* bias, const void* resid,
@@ -1397,7 +1409,7 @@ int souffle_layernorm_forward(const float* partial, int32_t n_partial, const voi
   const int items = stage_items(s);
   const int grid = items < sms ? items : sms;
   if ((rc = finalize_stage(s, 0, grid))) return rc;
-  return ws_launch(&args, grid, workspace, workspace_bytes, st);
+  return ws_launch(&args, grid, workspace, workspace_bytes, st, row_family(M, grid));
 }
 
 // ======================================================================================

@@ -77,7 +77,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   const void* dead_ptr[2];
   // ---- derived on the host by finalize_stage(): the kernel's lone producer / MMA lanes would otherwise
   //      spend a few thousand cycles per stage in integer divisions ----
-  int tiles_n, kchunks, items, slot_bytes, nslots;
+  int tiles_n, kchunks, kper, items, slot_bytes, nslots;   // a K chunk: kper steps of 64
   uint32_t mg_splitk, mg_tiles_n, mg_kchunks;   // magic multipliers, see fast_div()
   uint32_t mg_seq, mg_head_dim, mg_heads;
   // Swin row maps: windows per side of the grid, elements of one of the Q / K / V planes, and the multipliers of the

@@ -32,6 +32,18 @@ def test_gemm_matches_oracle(M, N, K):
     assert (c.float().cpu() - want).abs().max() < 2e-3 * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.parametrize("K", [64, 128, 192, 256, 320, 1024, 1088])
+@pytest.mark.parametrize("M,N", [(129, 64), (200, 192)])
+def test_gemm_slots_of_one_and_two_k_steps(M, N, K):
+    """Operand slots hold one step of 64 along K or, where the number of steps is even, two; one step alone, fewer steps than
+    slots, and more.  fp16 output of magnitude <= 8 (half an ulp: 4e-3 at 8, 2e-3 below 4) and fp32 sums of at most 1088 terms."""
+    from souffle_models_b200 import swin
+    a, w = _rand((M, K), K), _rand((K, N), K + 1, 1.0 / K ** 0.5)
+    c = swin.swin_ffn(a.cuda(), w.cuda(), M, N, K)
+    want = so.gemm_kn(a, w)
+    assert (c.float().cpu() - want).abs().max() < 2e-3 * max(1.0, want.abs().max().item())
+
+
 def test_swin_fused_mlp_and_fc2():
     from souffle_models_b200 import swin
     src, w1, w2 = _rand((256, 512), 3), _rand((512, 2048), 4, 0.02), _rand((2048, 512), 5, 0.02)
