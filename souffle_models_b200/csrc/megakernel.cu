@@ -1933,6 +1933,134 @@ __device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& 
   }
 }
 
+// The same for many rows per CTA: a warp per row, nothing exchanged between warps, twelve rows in flight (the form above has four of
+// 768 columns and is bound by its chain: 64 sequences 21.2 k cycles a stage against 16.3 k).  Every round trip costs ~800 cycles,
+// so the loads are issued in as few dependent rounds as the registers allow: bias, residual and the first planes
+// together, further planes kG at a time, gamma and beta just before the statistics (they land while the shuffles run).
+// With the loads strung one behind the other a row of six planes took 6.2 k cycles.
+template <int NJ>
+__device__ __forceinline__ void ln_row_alone(const float* pl, int n_partial, size_t plane_stride, const __half* res,
+                                              const __half* bias, const __half* gamma, const __half* beta, float eps,
+                                              __half* out, __half* sum_out, int lane) {
+  constexpr int kG = NJ <= 4 ? 4 : (NJ <= 6 ? 3 : 2);      // planes in flight at once
+  float z[NJ][4];
+  {
+    uint2 ub[NJ], ur[NJ];
+    float4 v[kG][NJ];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      ub[j] = bias ? __ldg(reinterpret_cast<const uint2*>(bias + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
+      ur[j] = res ? __ldcg(reinterpret_cast<const uint2*>(res + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int g = 0; g < kG; ++g)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+        v[g][j] = g < n_partial ? __ldcg(reinterpret_cast<const float4*>(pl + (size_t)g * plane_stride + (lane + 32 * j) * 4))
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const float2 b0 = __half22float2(*reinterpret_cast<const __half2*>(&ub[j].x)), b1 = __half22float2(*reinterpret_cast<const __half2*>(&ub[j].y));
+      const float2 r0 = __half22float2(*reinterpret_cast<const __half2*>(&ur[j].x)), r1 = __half22float2(*reinterpret_cast<const __half2*>(&ur[j].y));
+      z[j][0] = b0.x + r0.x; z[j][1] = b0.y + r0.y; z[j][2] = b1.x + r1.x; z[j][3] = b1.y + r1.y;
+#pragma unroll
+      for (int g = 0; g < kG; ++g) { z[j][0] += v[g][j].x; z[j][1] += v[g][j].y; z[j][2] += v[g][j].z; z[j][3] += v[g][j].w; }
+    }
+    for (int p0 = kG; p0 < n_partial; p0 += kG) {
+#pragma unroll
+      for (int g = 0; g < kG; ++g)
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+          v[g][j] = p0 + g < n_partial ? __ldcg(reinterpret_cast<const float4*>(pl + (size_t)(p0 + g) * plane_stride + (lane + 32 * j) * 4))
+                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int g = 0; g < kG; ++g) { z[j][0] += v[g][j].x; z[j][1] += v[g][j].y; z[j][2] += v[g][j].z; z[j][3] += v[g][j].w; }
+    }
+  }
+  if (sum_out) {                        // the sum itself, as fp16; what is normalised below is the rounded value
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const uint2 w = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
+      *reinterpret_cast<uint2*>(sum_out + (lane + 32 * j) * 4) = w;
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&w.x)), f1 = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
+      z[j][0] = f0.x; z[j][1] = f0.y; z[j][2] = f1.x; z[j][3] = f1.y;
+    }
+    if (eps < 0.0f) return;             // sum only
+  }
+  uint2 ug[NJ], ubt[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    ug[j] = gamma ? __ldg(reinterpret_cast<const uint2*>(gamma + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
+    ubt[j] = gamma ? __ldg(reinterpret_cast<const uint2*>(beta + (lane + 32 * j) * 4)) : make_uint2(0u, 0u);
+  }
+  const float inv_n = 1.0f / (float)(NJ * 128);
+  float sa = 0.0f;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) sa += (z[j][0] + z[j][1]) + (z[j][2] + z[j][3]);
+  sa = warp_sum(sa);
+  const float mean = sa * inv_n;
+  float va = 0.0f;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float d0 = z[j][i] - mean;
+      va = fmaf(d0, d0, va);
+    }
+  va = warp_sum(va);
+  const float rstd = rsqrtf(va * inv_n + eps), nm = -mean * rstd;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    uint32_t w0 = pack_h2(fmaf(z[j][0], rstd, nm), fmaf(z[j][1], rstd, nm));
+    uint32_t w1 = pack_h2(fmaf(z[j][2], rstd, nm), fmaf(z[j][3], rstd, nm));
+    if (gamma) {
+      const __half2 y0 = __hfma2(*reinterpret_cast<const __half2*>(&w0), *reinterpret_cast<const __half2*>(&ug[j].x),
+                                 *reinterpret_cast<const __half2*>(&ubt[j].x));
+      const __half2 y1 = __hfma2(*reinterpret_cast<const __half2*>(&w1), *reinterpret_cast<const __half2*>(&ug[j].y),
+                                 *reinterpret_cast<const __half2*>(&ubt[j].y));
+      w0 = *reinterpret_cast<const uint32_t*>(&y0);
+      w1 = *reinterpret_cast<const uint32_t*>(&y1);
+    }
+    *reinterpret_cast<uint2*>(out + (lane + 32 * j) * 4) = make_uint2(w0, w1);
+  }
+}
+
+// Out of line; a build has this form or the other one, not both: with both, their registers spill into one another's callers.
+__device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p, SmemCtl& cs, const WaitCtl& ctl, int warp, int lane) {
+  const int N = st.N, M = st.M, P = st.n_partial;
+  const size_t plane = (size_t)M * N;
+  const __half* resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
+  __half* out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p)));
+  const __half* bias = reinterpret_cast<const __half*>(st.bias);
+  const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
+  const __half* beta = reinterpret_cast<const __half*>(st.beta);
+  bool go = true;
+  if (warp == 0) {
+    if (lane == 0) go = grid_wait(p, ctl, st.prof_index);
+    if (lane == 0 && go) publish_go(cs, st.prof_index);
+    go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
+  } else {
+    go = wait_go(cs, st.prof_index, ctl);
+  }
+  if (!go) return;
+  if (st.dead_bytes[0]) drop_dead_buffers(st, 0, kThreads);
+  for (int row = warp * (int)gridDim.x + (int)blockIdx.x; row < M; row += (int)gridDim.x * (kThreads / 32)) {
+    const float* pl0 = st.partial + (size_t)row * N;
+    const __half* ra = resid ? resid + (size_t)row * N : nullptr;
+    __half* o0 = out + (size_t)row * N;
+    __half* so = st.eps < 0.0f ? o0 : st.sum_out ? reinterpret_cast<__half*>(st.sum_out) + (size_t)row * N : nullptr;
+    switch (N >> 7) {
+      case 1: ln_row_alone<1>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 2: ln_row_alone<2>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 4: ln_row_alone<4>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      case 6: ln_row_alone<6>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+      default: ln_row_alone<8>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
+    }
+  }
+}
+
 // kMerge builds add the patch-merging form (Swin, python/models/swin_transformer/swin_patch_merge.py:1-17): with
 // st.seq = R > 0 the fp16 input is a [batch][R][R][N/4] token grid and row (b, h, w) of the normalised matrix is the
 // concatenation of tokens (2h, 2w), (2h+1, 2w), (2h, 2w+1), (2h+1, 2w+1), fetched as four bulk copies; rows of 2048
@@ -2208,7 +2336,8 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
         else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
         else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
       } else if (st.type == STAGE_LN) {
-        ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+        if constexpr (kFamily == kFamilyBertCoop) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+        else ln_stage_many(st, p, cs, ctl, warp, lane);
       }
     }
     // Every thread comes by here once per stage, whatever became of its waits, and all leave the loop together.
