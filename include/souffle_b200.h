@@ -158,6 +158,9 @@ int souffle_bert_plan_buffer(SouffleBertPlan* plan, int which, void** ptr_out, s
 /* Copies one of those buffers into caller memory (device pointer, `dst_bytes` >= its size) on `stream`. */
 int souffle_bert_plan_copy_buffer(SouffleBertPlan* plan, int which, void* dst, size_t dst_bytes,
                                   souffle_stream_t stream);
+/* The same for `n` (0..8) of them as one launch; destinations 16-byte aligned. */
+int souffle_bert_plan_copy_buffers(SouffleBertPlan* plan, int n, const int* which, void* const* dst, const size_t* dst_bytes,
+                                   souffle_stream_t stream);
 
 /* Synchronises the plan's device and reports the device-side status of the last launch:
  * SOUFFLE_OK, or SOUFFLE_DEVICE_TIMEOUT with the stage/CTA in souffle_last_error(). */

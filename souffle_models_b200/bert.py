@@ -123,11 +123,22 @@ class BertEncoder:
         _lib.check(self._lib.souffle_bert_plan_read_profile(self._h, out.data_ptr(), out.numel()))
         return out
 
+    def _buffer_shape(self, name: str) -> tuple:
+        B, S, h, d, H, F = self.batch, self.seq, self.heads, self.head_dim, self.hidden, self.ffn
+        return dict(qkv=(3, B, h, S, d), probs=(B * h, S, S), ctx=(B * S, H), ln1=(B * S, H), fc1=(B * S, F))[name]
+
+    def buffers(self, *names: str) -> List[torch.Tensor]:
+        """Copies of several stage outputs (see buffer), made by one launch."""
+        outs = [torch.empty(self._buffer_shape(k), dtype=torch.float16, device="cuda") for k in names]
+        n = len(outs)
+        _lib.check(self._lib.souffle_bert_plan_copy_buffers(
+            self._h, n, (C.c_int * n)(*(_BUF[k] for k in names)), (C.c_void_p * n)(*(t.data_ptr() for t in outs)),
+            (C.c_size_t * n)(*(2 * t.numel() for t in outs)), _stream_ptr()))
+        return outs
+
     def buffer(self, name: str) -> torch.Tensor:
         """Copy of a last-layer stage output (see SouffleBertBuffer in the header)."""
-        B, S, h, d, H, F = self.batch, self.seq, self.heads, self.head_dim, self.hidden, self.ffn
-        shape = dict(qkv=(3, B, h, S, d), probs=(B * h, S, S), ctx=(B * S, H), ln1=(B * S, H), fc1=(B * S, F))[name]
-        out = torch.empty(shape, dtype=torch.float16, device="cuda")
+        out = torch.empty(self._buffer_shape(name), dtype=torch.float16, device="cuda")
         _lib.check(self._lib.souffle_bert_plan_copy_buffer(self._h, _BUF[name], out.data_ptr(), out.numel() * 2,
                                                            _stream_ptr()))
         return out
@@ -174,9 +185,9 @@ def souffle_bert_layer(src: torch.Tensor, qkv_weight: torch.Tensor, attn_fc_weig
         _layer_cache[key] = hit
     enc = hit[0]
     out = enc.forward(src).reshape(B * S, H)
-    # the copies of the intermediates are queued behind the launch while it runs; one wait at the end
-    outs = [enc.buffer("qkv").reshape(3 * B, heads, S, 64), enc.buffer("probs"), enc.buffer("ctx"),
-            enc.buffer("ln1"), enc.buffer("fc1"), out]
+    # the copy of the intermediates is queued behind the launch while it runs; one wait at the end
+    qkv, *rest = enc.buffers("qkv", "probs", "ctx", "ln1", "fc1")
+    outs = [qkv.reshape(3 * B, heads, S, 64), *rest, out]
     enc.status()                                   # blocks, as the reference call does (bert_binding.cu:532)
     return outs
 

@@ -147,6 +147,41 @@ __global__ void transpose_kn_to_nk(const __half* __restrict__ src, __half* __res
 }
 
 // ------------------------------------------------------------------------------------
+// several device-to-device copies as one launch: the five intermediates of the drop-in layer (8.9 MB at 384 tokens, out of L2).
+// Bound by the launch: as five copies of the driver's they took 12 us of GPU time behind a 43 us kernel.  Four 16-byte loads per
+// thread are in flight.
+// ------------------------------------------------------------------------------------
+constexpr int kMaxCopies = 8, kCopyThreads = 256;
+struct CopyList {
+  const uint4* src[kMaxCopies];
+  uint4* dst[kMaxCopies];
+  unsigned long long end[kMaxCopies];        // running totals of 16-byte pieces
+  int n;
+};
+__global__ void __launch_bounds__(kCopyThreads) souffle_copy_list(const __grid_constant__ CopyList list) {
+  const unsigned long long total = list.end[list.n - 1], step = (unsigned long long)gridDim.x * kCopyThreads;
+  for (unsigned long long i0 = (unsigned long long)blockIdx.x * kCopyThreads + threadIdx.x; i0 < total; i0 += 4 * step) {
+    uint4 v[4];
+    uint4* to[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned long long i = i0 + k * step;
+      to[k] = nullptr;
+      if (i < total) {
+        int b = 0;
+        while (i >= list.end[b]) ++b;
+        const unsigned long long at = i - (b ? list.end[b - 1] : 0ull);
+        v[k] = __ldcg(list.src[b] + at);
+        to[k] = list.dst[b] + at;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (to[k]) *to[k] = v[k];
+  }
+}
+
+// ------------------------------------------------------------------------------------
 // tiling choice: a small cycle model of one CTA, fitted to the in-kernel stage profile on a B200.
 // A K chunk costs the larger of its tensor-core time (bm*bn/64 cycles) and its shared-memory traffic
 // (operands written once by TMA and read by the tensor core, B once per 128-row half, at 128 B/clk).
@@ -1157,6 +1192,33 @@ int souffle_bert_plan_copy_buffer(SouffleBertPlan* plan, int which, void* dst, s
   if (rc) return rc;
   if (!dst || dst_bytes < bytes) return fail(SOUFFLE_BAD_ARGUMENT, "destination holds %zu bytes, buffer has %zu", dst_bytes, bytes);
   SF_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, reinterpret_cast<cudaStream_t>(stream)));
+  return SOUFFLE_OK;
+}
+
+int souffle_bert_plan_copy_buffers(SouffleBertPlan* plan, int n, const int* which, void* const* dst, const size_t* dst_bytes,
+                                   souffle_stream_t stream) {
+  if (n < 0 || n > kMaxCopies) return fail(SOUFFLE_BAD_ARGUMENT, "%d buffers (0..%d can be copied at once)", n, kMaxCopies);
+  if (n > 0 && (!which || !dst || !dst_bytes)) return fail(SOUFFLE_BAD_ARGUMENT, "null argument");
+  CopyList list;
+  memset(&list, 0, sizeof(list));
+  unsigned long long total = 0;
+  for (int i = 0; i < n; ++i) {
+    void* src = nullptr;
+    size_t bytes = 0;
+    int rc = souffle_bert_plan_buffer(plan, which[i], &src, &bytes);
+    if (rc) return rc;
+    if (!dst[i] || dst_bytes[i] < bytes) return fail(SOUFFLE_BAD_ARGUMENT, "destination holds %zu bytes, buffer has %zu", dst_bytes[i], bytes);
+    if (!aligned16(dst[i])) return fail(SOUFFLE_BAD_POINTER, "destinations must be 16-byte aligned");
+    total += bytes / 16;                                 // every buffer is a whole number of 16-byte pieces: S and H are multiples of 16
+    list.src[i] = reinterpret_cast<const uint4*>(src);
+    list.dst[i] = reinterpret_cast<uint4*>(dst[i]);
+    list.end[i] = total;
+  }
+  list.n = n;
+  if (total == 0) return SOUFFLE_OK;
+  const unsigned long long blocks = (total + 4ull * kCopyThreads - 1) / (4ull * kCopyThreads);
+  souffle_copy_list<<<(unsigned)(blocks < 148ull * 8 ? blocks : 148ull * 8), kCopyThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(list);
+  SF_CUDA(cudaGetLastError());
   return SOUFFLE_OK;
 }
 

@@ -193,6 +193,16 @@ def test_autotuned_plan_matches_the_oracle():
     assert (fixed.stage_info(4)["bm"], fixed.stage_info(4)["bn"]) == (128, 64)
 
 
+@pytest.mark.parametrize("B,S,heads,ffn", [(1, 16, 2, 128), (3, 48, 4, 320), (1, 384, 12, 3072)])
+def test_buffers_copied_at_once_equal_the_single_copies(B, S, heads, ffn):
+    """One launch that copies several stage outputs: smallest sizes, sizes that are no multiple of a block's work, the drop-in's."""
+    cfg = so.BertConfig(B, S, heads, 64, ffn, "std")
+    enc, _, _, _, _ = _run(cfg, 31, keep_probs=True)
+    for names in (("qkv", "probs", "ctx", "ln1", "fc1"), ("fc1",), ("ctx", "ctx", "probs"), ()):
+        for name, got in zip(names, enc.buffers(*names)):
+            assert torch.equal(got, enc.buffer(name)), name
+
+
 def test_stage_info_reports_the_tiling():
     cfg = so.BertConfig(2, 128, 12, 64, 3072, "std")
     layers = so.make_bert_weights(cfg, 5, 1)
