@@ -375,6 +375,11 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
   const void* fn = family == kFamilySwin ? (const void*)souffle_megakernel<kFamilySwin>
                    : family == kFamilyBertCoop ? (const void*)souffle_megakernel<kFamilyBertCoop>
                                                : (const void*)souffle_megakernel<kFamilyBert>;
+  // (a single stage waits for no other CTA: a plain launch does)
+  if (args.p.n_stages == 1) {
+    SF_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), kargs, (size_t)kSmemBytes, stream));
+    return SOUFFLE_OK;
+  }
   SF_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), kargs, (size_t)kSmemBytes, stream));
   return SOUFFLE_OK;
 }
