@@ -12,10 +12,10 @@
 //   cpp/swin_transformer/kernels/swin_fused_ffn_m256n2048k512_m256n512k2048.cu:9-769 fc1 -> fc2
 //   cpp/swin_transformer/kernels/gemm_three_stages.h:8-379 and kernels/gemm_k6.cu:9-339 single GEMMs
 //
-// Warp roles (384 threads): warp 0 = TMA producer (one elected lane), warp 1 = MMA issuer and
+// Warp roles (384 threads): warp 0 = feeder (a lone lane: grid barrier, activation tiles), warp 1 = MMA issuer and
 // TMEM owner, warps 2..9 = epilogue (warp w reads TMEM lanes 32*(w%4) .. +31; two warps share a
-// lane quarter and take alternate 32-column chunks) and attention softmax warps; warps 10..11 are spare:
-// they take LayerNorm rows like every other warp and drop dead buffers from L2 in front of the other stages.
+// lane quarter and take alternate 32-column chunks) and attention softmax warps, warp 10 = arrivals, L2 prefetch and drops,
+// warp 11 = weight tiles and stage records.  All twelve take rows of the LayerNorm stages.
 // Every wait (mbarrier, grid barrier) is bounded by a wall-clock deadline; on expiry the CTA
 // records a status word, drains and returns, so a fault never leaves the GPU spinning.
 #include <cuda.h>
@@ -28,9 +28,8 @@
 
 namespace souffle {
 
-constexpr int kThreads = 384;               // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue / softmax, warps 10..11 take rows of
-                                            // the LayerNorm stages only (registers are handed out per four warps: a block of
-                                            // ten warps is charged for twelve, so the two extra warps cost nothing)
+constexpr int kThreads = 384;               // registers are handed out per four warps: a block of ten warps is charged for
+                                            // twelve, so the last two cost nothing
 constexpr int kEpiWarps = 8, kEpiThreads = kEpiWarps * 32;
 constexpr int kSpareWarp = 2 + kEpiWarps, kWeightWarp = kSpareWarp + 1;
 constexpr int kRingBytes = 196608;          // 192 KiB operand ring (4 x 48 KiB, 3 x 64 KiB or 6 x 32 KiB slots)

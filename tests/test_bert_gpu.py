@@ -193,6 +193,24 @@ def test_autotuned_plan_matches_the_oracle():
     assert (fixed.stage_info(4)["bm"], fixed.stage_info(4)["bn"]) == (128, 64)
 
 
+@pytest.mark.parametrize("B,S,heads,ffn", [
+    (1, 16, 2, 128),       # rows of 128 columns: one warp, the second block of columns is absent
+    (9, 384, 2, 256),      # the same in two passes, the second one ragged
+    (3, 144, 4, 256),      # 256 columns, one warp
+    (4, 256, 8, 512),      # 512 columns on two warps, several rows per group
+    (4, 256, 16, 1024),    # 1024 columns on four warps, three passes
+    (12, 128, 16, 1024),   # many attention items: a warp per row
+])
+def test_layernorm_rows_shared_by_warps(B, S, heads, ffn):
+    """The two LayerNorm forms over the row widths a plan takes, with one and with several rows per group of warps: LayerNorm 1
+    (planes + bias + residual) and the layer's output against the oracle."""
+    cfg = so.BertConfig(B, S, heads, 64, ffn, "std")
+    enc, layers, x, lens, y = _run(cfg, 57, zero_bias=False, keep_probs=True)
+    r = so.bert_layer(cfg, x, layers[0], lens)
+    assert _err(enc.buffer("ln1"), r["ln1"]) < TOL_LAYER
+    assert _err(y, r["out"]) < TOL_LAYER
+
+
 @pytest.mark.parametrize("B,S,heads,ffn", [(1, 16, 2, 128), (3, 48, 4, 320), (1, 384, 12, 3072)])
 def test_buffers_copied_at_once_equal_the_single_copies(B, S, heads, ffn):
     """One launch that copies several stage outputs: smallest sizes, sizes that are no multiple of a block's work, the drop-in's."""
