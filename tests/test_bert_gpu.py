@@ -196,7 +196,7 @@ def test_autotuned_plan_matches_the_oracle():
 @pytest.mark.parametrize("B,S,heads,ffn", [
     (1, 16, 2, 128),       # rows of 128 columns: one warp, the second block of columns is absent
     (9, 384, 2, 256),      # the same in two passes, the second one ragged
-    (3, 144, 4, 256),      # 256 columns, one warp
+    (3, 256, 4, 256),      # 256 columns, one warp
     (4, 256, 8, 512),      # 512 columns on two warps, several rows per group
     (4, 256, 16, 1024),    # 1024 columns on four warps, three passes
     (12, 128, 16, 1024),   # many attention items: a warp per row
