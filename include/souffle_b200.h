@@ -74,9 +74,10 @@ typedef struct SouffleBertDesc {
   int32_t profile;    /* 1: record per-stage, per-CTA SM clock stamps (souffle_bert_plan_read_profile) */
   int32_t bm_qkv, bm_fc1, bm_proj, bm_fc2; /* tile heights (128 or 256), 0 = choose automatically */
   int32_t debug_max_slots;    /* experiment knob: cap on operand ring slots per CTA, 0 = as many as fit */
-  int32_t debug_skip_arrival; /* failure-detection test hook, 0 = off: CTA (value-1) leaves at the first grid
-                                 barrier without arriving, so the others run into the wait limit and the
-                                 launch ends with SOUFFLE_DEVICE_TIMEOUT (nothing is in flight at that point) */
+  int32_t debug_skip_arrival; /* failure-detection test hook, 0 = off: CTA (low 16 bits - 1) leaves at the grid
+                                 barrier behind stage (high 16 bits) without arriving, so the others run into the
+                                 wait limit and the launch ends with SOUFFLE_DEVICE_TIMEOUT (nothing is in flight
+                                 at that point) */
   int32_t autotune;   /* 1: plan creation times the likeliest tilings of every GEMM stage on the device (a few
                          launches each on the plan's own buffers, tens of milliseconds in all) and keeps the
                          fastest; stages with an explicit bm_ / bn_ / split_ setting are left alone.  0: tiles come

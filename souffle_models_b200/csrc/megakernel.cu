@@ -61,7 +61,7 @@ struct MegaParams {
   int* expired;       // host memory or null: set by a CTA that gave up on a wait
   unsigned long long timeout_ns;
   int max_slots;      // experiment knob: cap on operand ring slots, 0 = as many as fit
-  int skip_arrival;   // test hook: CTA (skip_arrival-1) leaves at barrier 0 without arriving; 0 = off
+  int skip_arrival;   // test hook: CTA (low 16 bits - 1) leaves without arriving after stage (high 16 bits); 0 = off
   long long* prof;    // optional [n_stages][grid][8]: clock64 at stage start, work done, barrier left, then GEMM
                       // role cycles: MMA waiting for operands, MMA waiting for a free accumulator, producer
                       // waiting for a free slot, epilogue waiting for an accumulator, epilogue busy
@@ -93,7 +93,7 @@ struct __align__(8) SmemCtl {
   int abort;
   int leave[2];                     // a wait has run out: all warps leave the stage loop together
   uint32_t arrived;                 // stages whose arrival this CTA has sent
-  uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go)
+  uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go / stage_go)
   WaitCtl wait;                     // here and not on the stack: see RoleState
   alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their position
 };
@@ -140,11 +140,11 @@ __device__ __forceinline__ const void* sel_ptr(int sel, const void* plan, const 
 // Its two halves lie with different warps, so that a stage's set-up runs while the CTA waits.  At the end of a stage all
 // threads of a CTA meet once (the end of the stage loop); a lane of a spare warp then adds the CTA's arrival to the counter,
 // whose release covers every thread's writes and takes ~1 k cycles.  Meanwhile every warp has gone on to the next stage: the
-// epilogue warps stage the bias, the row warps load gamma and beta, and the feeder (the lone lane of warp 0 that issues the
-// stage's copies) requests the first weight tiles, none of which the stage before has written.  Only the feeder looks at the
+// epilogue warps stage the bias, the row warps load gamma and beta, and the weight warp requests the first weight tiles, none of
+// which the stage before has written.  Only the feeder (the lone lane of warp 0 that issues the stage's copies) looks at the
 // counter (grid_wait), and what it does next is issue the stage's first activation copy.  All other warps of a GEMM or
-// attention stage are behind the data the feeder asks for; warps that read what earlier stages wrote by themselves wait for
-// the feeder's word (wait_go).
+// attention stage are behind the data the feeder asks for; the warps of a LayerNorm stage, which read what earlier stages wrote
+// by themselves, all get the feeder's one verdict (stage_go).
 // ------------------------------------------------------------------------------------
 // The polls in front stand in straight line (a loop's way out costs some 150 cycles, see mbar_wait_hot); a CTA that waits
 // longer than they last goes on out of line.
@@ -183,25 +183,43 @@ __device__ __forceinline__ bool grid_wait(const MegaParams& p, const WaitCtl& ct
   }
   return there;
 }
-// Bounded wait for a word of this CTA's shared memory that only grows.  (It records nothing: its writer's own waits have the same
-// limit and do.)
-__device__ __noinline__ bool wait_word_loop(uint32_t word, uint32_t want, const WaitCtl& ctl) {
+// Bounded wait for a word of this CTA's shared memory that only grows.
+__device__ __noinline__ bool wait_word_loop(uint32_t word, uint32_t want, const WaitCtl& ctl, int where) {
   uint32_t spins = 0;
   while (ld_acquire_cta_shared_u32(word) < want) {
-    if (((++spins) & 0xFF) == 0 && (*ctl.abort_smem || globaltimer_ns() > ctl.deadline_ns)) return false;
+    if (((++spins) & 0xFF) == 0) {
+      if (*ctl.abort_smem) return false;
+      if (globaltimer_ns() > ctl.deadline_ns) {
+        record_timeout(ctl, DEV_TIMEOUT_FLAG, where);
+        return false;
+      }
+    }
   }
   return true;
 }
-__device__ __forceinline__ bool wait_word(uint32_t word, uint32_t want, const WaitCtl& ctl) {
-  return ld_acquire_cta_shared_u32(word) >= want || wait_word_loop(word, want, ctl);
+__device__ __forceinline__ bool wait_word(uint32_t word, uint32_t want, const WaitCtl& ctl, int where) {
+  return ld_acquire_cta_shared_u32(word) >= want || wait_word_loop(word, want, ctl, where);
 }
 // One thread: this CTA's arrival for stage si - 1 is on its way.  Copies issued before that would delay it: its release waits for
 // them too.
-__device__ __forceinline__ bool wait_arrived(SmemCtl& cs, int si, const WaitCtl& ctl) { return wait_word(smem_u32(&cs.arrived), (uint32_t)si, ctl); }
-// The feeder's word that stage si may start, for warps that read global memory by themselves.
+__device__ __forceinline__ bool wait_arrived(SmemCtl& cs, int si, const WaitCtl& ctl) { return wait_word(smem_u32(&cs.arrived), (uint32_t)si, ctl, 700); }
+// The feeder's word that stage si may start.
 __device__ __forceinline__ void publish_go(SmemCtl& cs, int si) { st_release_cta_shared_u32(smem_u32(&cs.go), (uint32_t)si + 1u); }
-__device__ __forceinline__ bool wait_go(SmemCtl& cs, int si, const WaitCtl& ctl) {      // whole warps
-  return __all_sync(0xffffffffu, wait_word(smem_u32(&cs.go), (uint32_t)si + 1u, ctl));
+// For a warp whose part the stage's result does not depend on (what it skips when it gives up is a drop from L2).
+__device__ __forceinline__ bool wait_go(SmemCtl& cs, int si, const WaitCtl& ctl) {
+  return __all_sync(0xffffffffu, wait_word(smem_u32(&cs.go), (uint32_t)si + 1u, ctl, 701));
+}
+// All threads of the CTA: true if stage si may start.  The feeder alone looks at the clock, and its verdict reaches every warp
+// through a barrier: warps that judged the limit one by one could part ways when it passes, and those that went on would miss
+// the others' rows or wait for them in a barrier.
+constexpr int kGoBarrier = 15;
+__device__ __forceinline__ bool stage_go(const MegaParams& p, SmemCtl& cs, int si, const WaitCtl& ctl, int warp, int lane) {
+  if (warp == 0) {
+    if (lane == 0 && grid_wait(p, ctl, si)) publish_go(cs, si);
+    __syncwarp();
+  }
+  named_barrier_sync(kGoBarrier, kThreads);
+  return ld_acquire_cta_shared_u32(smem_u32(&cs.go)) > (uint32_t)si;      // not written again before all have met at the stage's end
 }
 
 // The warp's index as a value the compiler knows to be the same in all its lanes (see elect_one).
@@ -1815,15 +1833,7 @@ __device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& 
   const bool affine = st.gamma != nullptr;
   const float inv_n = 1.0f / (float)N;
   red += grp * W;
-  bool go = true;
-  if (warp == 0) {
-    if (lane == 0) go = grid_wait(p, ctl, st.prof_index);
-    if (lane == 0 && go) publish_go(cs, st.prof_index);
-    go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
-  } else {
-    go = wait_go(cs, st.prof_index, ctl);
-  }
-  if (!go) return;
+  if (!stage_go(p, cs, st.prof_index, ctl, warp, lane)) return;
   auto load_planes = [&](int r, int g0) {
     const float* src = planes + (size_t)r * N + (size_t)g0 * plane;
 #pragma unroll
@@ -2035,15 +2045,7 @@ __device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p,
   const __half* bias = reinterpret_cast<const __half*>(st.bias);
   const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
   const __half* beta = reinterpret_cast<const __half*>(st.beta);
-  bool go = true;
-  if (warp == 0) {
-    if (lane == 0) go = grid_wait(p, ctl, st.prof_index);
-    if (lane == 0 && go) publish_go(cs, st.prof_index);
-    go = __shfl_sync(0xffffffffu, (int)go, 0) != 0;
-  } else {
-    go = wait_go(cs, st.prof_index, ctl);
-  }
-  if (!go) return;
+  if (!stage_go(p, cs, st.prof_index, ctl, warp, lane)) return;
   if (st.dead_bytes[0]) drop_dead_buffers(st, 0, kThreads);
   for (int row = warp * (int)gridDim.x + (int)blockIdx.x; row < M; row += (int)gridDim.x * (kThreads / 32)) {
     const float* pl0 = st.partial + (size_t)row * N;
@@ -2347,7 +2349,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     if (warp == kSpareWarp && lane == 0) {
       if (p.prof) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
       if (si + 1 < p.n_stages) {
-        if (p.skip_arrival > 0 && si == 0 && (int)blockIdx.x == p.skip_arrival - 1) *ctl.abort_smem = 1;      // test hook
+        if (p.skip_arrival > 0 && si == p.skip_arrival >> 16 && (int)blockIdx.x == (p.skip_arrival & 0xFFFF) - 1) *ctl.abort_smem = 1;      // test hook
         else red_add_release_u32(p.sync, 1u);
         st_release_cta_shared_u32(smem_u32(&cs.arrived), (uint32_t)si + 1u);
       } else if (p.prof) {

@@ -303,3 +303,28 @@ def test_device_side_wait_limit_reports_status_without_hanging():
     y = good.forward(x.cuda())
     good.status()
     assert _err(y, so.bert_layer(cfg, x, layers[0])["out"]) < TOL_LAYER
+
+
+@pytest.mark.parametrize("stage", [0, 1, 2, 5])       # the wait in front of attention, proj, LayerNorm 1, LayerNorm 2
+@pytest.mark.parametrize("B,S,heads", [
+    (1, 64, 2),            # LayerNorm: a warp per row, few rows
+    (1, 128, 12),          # three warps per row
+    (2, 384, 12),          # the same, several rows per group of warps
+    (13, 128, 12),         # more attention items than CTAs: a warp per row, many rows
+])
+def test_wait_limit_in_front_of_every_kind_of_stage(B, S, heads, stage):
+    """The stage behind the barrier that one CTA leaves out is entered by all warps of a CTA or by none: the launch ends by itself
+    after the 20 ms limit with a status.  In front of a LayerNorm stage only the feeder waits, so the status names that barrier; in
+    the other stages the warps behind the feeder's copies look at the same limit."""
+    from souffle_models_b200 import _lib
+    cfg = so.BertConfig(B, S, heads, 64, 512, "std")
+    layers = so.make_bert_weights(cfg, 3, 1)
+    x, _ = so.make_bert_input(cfg, 3)
+    bad = _encoder(cfg, layers, tuning=dict(timeout_ms=20, debug_skip_arrival=(stage << 16) | 2))
+    bad.forward(x.cuda())
+    with pytest.raises(_lib.SouffleError) as ei:
+        bad.status()
+    assert ei.value.code == 6 and "wait expired" in str(ei.value)
+    if stage in (2, 5):
+        assert f"code 2, where {stage}," in str(ei.value)
+    bad.close()
