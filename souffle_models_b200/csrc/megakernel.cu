@@ -964,11 +964,13 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
     // staging areas behind it, which no one else uses during attention; the exchange buffer sits at their very end.
     static_assert(13 * kATileBytes <= kRingBytes + kVecBytes + kStageBytes - 2048, "attention tiles overlap the exchange buffer");
     float* red = reinterpret_cast<float*>(stage_s + kStageBytes - 2048);   // [2 groups][128 rows] maxima, then [2][128] sums
+    // The warps look at the wait limit one by one and meet in barriers, so none leaves the loop early: one that has given up goes
+    // through the remaining items without waiting again and without storing.
+    bool ok = true;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int qt = item % n_kb, h = (item / n_kb) % H, b = item / (n_kb * H);
       const int kv_len = lens ? lens[b] : S;
-      bool ok = mbar_wait_warp(s_full, rs.attn_bit, ctl, 520, lane);
-      if (!ok) break;
+      ok = ok && mbar_wait_warp(s_full, rs.attn_bit, ctl, 520, lane);
       tc_fence_after_sync();
       // Keys >= kv_len carry the additive -1e4 mask: probability 0 in fp32, never the maximum -> only the blocks
       // with valid keys are visited; the other P blocks are written as zeros.
@@ -1073,14 +1075,13 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
                               S - qt * 128 < 128 ? S - qt * 128 : 128, (int)threadIdx.x - 64);
         named_barrier_sync(3, 256);
       }
-      ok = mbar_wait_warp(o_full, rs.attn_bit, ctl, 521, lane);
-      if (!ok) break;
+      ok = ok && mbar_wait_warp(o_full, rs.attn_bit, ctl, 521, lane);
       tc_fence_after_sync();
       {
         uint32_t r0[32];
         tmem_ld32(tmem + kOCol + grp * 32, r0);               // this group's 32 of the 64 output columns
         tmem_ld_wait(r0);
-        if (qrow < S) {
+        if (ok && qrow < S) {
           uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)b * S + qrow) * hidden + h * st.head_dim + grp * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -1542,6 +1543,7 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
     const int tbl = 2 * ws - 1;
     float* bias_s = reinterpret_cast<float*>(stage_s) + grp * 256;   // this head's column of the bias table (x log2 e): at most 225
     uint8_t* prow = ring_ptr + (3 + grp) * kATileBytes + r_in * 128;
+    bool ok = true;                                                  // false: given up, see attn_stage
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int wp = item / item_h, h = (int)n * (item - wp * item_h) + grp;
       const int wg = (int)n * wp + j, w = wg % nw_img;
@@ -1550,7 +1552,7 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
       named_barrier_sync(2 + grp, 128);                              // previous item's readers are done with bias_s
       for (int i = r_in; i < tbl * tbl; i += 128) bias_s[i] = __half2float(table[i * H + h]) * l2e;
       named_barrier_sync(2 + grp, 128);
-      if (!mbar_wait_warp(bar(grp, AB_S_FULL), rs.attn_bit, ctl, 535, lane)) break;
+      ok = ok && mbar_wait_warp(bar(grp, AB_S_FULL), rs.attn_bit, ctl, 535, lane);
       tc_fence_after_sync();
       float sum = 1.0f;
       if (ws == 7) sum = swin_softmax_row<7>(tmem, bias_s, prow, row, live, wy, wx, R, shift, sl2);
@@ -1559,13 +1561,13 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
       fence_proxy_async_smem();
       tc_fence_before_sync();
       mbar_arrive(bar(grp, AB_P_FULL));
-      if (!mbar_wait_warp(bar(grp, AB_O_FULL), rs.attn_bit, ctl, 536, lane)) break;
+      ok = ok && mbar_wait_warp(bar(grp, AB_O_FULL), rs.attn_bit, ctl, 536, lane);
       tc_fence_after_sync();
       {
         uint32_t o[32];
         tmem_ld32(tmem + 256u + (uint32_t)(h & 1) * 32u, o);
         tmem_ld_wait(o);
-        if (live && row < n_tok) {
+        if (ok && live && row < n_tok) {
           uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)wg * 64 + row) * C + h * 32);
 #pragma unroll
           for (int i = 0; i < 4; ++i)

@@ -310,6 +310,7 @@ def test_device_side_wait_limit_reports_status_without_hanging():
     (1, 64, 2),            # LayerNorm: a warp per row, few rows
     (1, 128, 12),          # three warps per row
     (2, 384, 12),          # the same, several rows per group of warps
+    (8, 384, 12),          # several attention items per CTA, whose softmax warps meet in barriers
     (13, 128, 12),         # more attention items than CTAs: a warp per row, many rows
 ])
 def test_wait_limit_in_front_of_every_kind_of_stage(B, S, heads, stage):
