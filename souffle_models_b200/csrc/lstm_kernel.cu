@@ -177,7 +177,7 @@ struct LstmShared {
   uint4 wx_rest[H == 256 ? 2 * (H / 32 - kXReg) * kWarps * 32 : 1];
   float x_scale[kLstmXBufs];                    // takes the products back to the vector's scale; negative: another piece follows
   uint64_t x_full[kLstmXBufs], x_empty[kLstmXBufs], h_full[2], pieces_ready;
-  WaitCtl wait;                                 // here and not on the stack: the step loop's registers are full
+  unsigned long long deadline_ns;
   int abort;
   uint32_t pieces;                              // 1: from the next input vector on, vectors come in pieces
   int piece[kWarps];                            // then: pieces a cell warp has multiplied so far
@@ -312,7 +312,10 @@ __device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& s
 template <int H>
 __device__ __noinline__ void lstm_steps_in_pieces(const LstmParams& p, LstmShared<H>& sh, float c_state) {
   int t = *const_cast<volatile int*>(sh.piece + (threadIdx.x >> 5));       // every vector before this one came whole
-  const WaitCtl& ctl = sh.wait;
+  WaitCtl ctl;
+  ctl.abort_smem = &sh.abort;
+  ctl.status_g = p.status;
+  ctl.deadline_ns = sh.deadline_ns;
   lstm_steps<H, true>(p, sh, ctl, blockIdx.x / kLstmParts, (int)cluster_cta_rank(), threadIdx.x, t, c_state);
 }
 
@@ -330,9 +333,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
 
   if (tid == 0) {
     sh.abort = 0;
-    sh.wait.abort_smem = &sh.abort;
-    sh.wait.status_g = p.status;
-    sh.wait.deadline_ns = globaltimer_ns() + p.timeout_ns;
+    sh.deadline_ns = globaltimer_ns() + p.timeout_ns;
     sh.pieces = 0;
     for (int i = 0; i < kWarps; ++i) sh.stored[i] = 0;
     for (int i = 0; i < kLstmXBufs; ++i) {
@@ -352,7 +353,10 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   __syncthreads();
   cluster_sync_all();                           // every CTA's barriers exist before anyone arrives on them
 
-  const WaitCtl& ctl = sh.wait;
+  WaitCtl ctl;
+  ctl.abort_smem = &sh.abort;
+  ctl.status_g = p.status;
+  ctl.deadline_ns = sh.deadline_ns;
 
   if (warp == kWarps + 1) {
     // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
