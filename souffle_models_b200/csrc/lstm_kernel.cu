@@ -75,6 +75,34 @@ __device__ __forceinline__ float gate_f(float v, bool is_tanh) {
   return is_tanh ? 1.0f - r : r;
 }
 
+// What the bounded waits look at.  Hidden 64 and 128: a WaitCtl on the stack (in shared memory every step was slower, 3 x 128 x 37
+// 38.1 -> 38.9 us, 8 x 128 x 150 161.7 -> 163.8; recording a timeout without one, 163.0).  Hidden 256, whose step loop has no register left: places known at
+// compile time and no call, where the WaitCtl spilled a word (12 x 256 x 200 284.5 -> 281.5 us).
+struct LstmWait {
+  int* abort;                                   // of the CTA, in shared memory
+  const unsigned long long* deadline_ns;        // in shared memory
+  int* status;
+};
+template <int H>
+using LstmWaitOf = std::conditional_t<(H < 256), WaitCtl, LstmWait>;
+// One thread, now and then: true if it has to give up.
+__device__ __forceinline__ bool lstm_expired(const WaitCtl& w, int code, int where) {
+  if (*w.abort_smem) return true;
+  if (globaltimer_ns() <= w.deadline_ns) return false;
+  record_timeout(w, code, where);
+  return true;
+}
+__device__ __forceinline__ bool lstm_expired(const LstmWait& w, int code, int where) {
+  if (*const_cast<volatile int*>(w.abort)) return true;
+  if (globaltimer_ns() <= *const_cast<const volatile unsigned long long*>(w.deadline_ns)) return false;
+  *const_cast<volatile int*>(w.abort) = 1;
+  if (atomicCAS(w.status, 0, code) == 0) {
+    w.status[1] = where;
+    w.status[2] = (int)blockIdx.x;
+  }
+  return true;
+}
+
 // Bounded wait of a whole warp on an mbarrier; every lane sees the phase itself.  kCluster: its transfers come from other
 // CTAs of the cluster.  `stop` (0: none) is the address of a shared word: once it is set, a wait whose phase is not
 // complete by then ends as well.
@@ -83,28 +111,22 @@ __device__ __forceinline__ bool lstm_try(uint32_t bar, uint32_t parity) {
   if constexpr (kCluster) return mbar_try_wait_cluster(bar, parity);
   else return mbar_try_wait(bar, parity);
 }
-template <bool kCluster>
-__device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, uint32_t stop) {
+template <bool kCluster, class W>
+__device__ __forceinline__ bool lstm_wait_loop(uint32_t bar, uint32_t parity, const W& w, int where, uint32_t stop) {
   uint32_t spins = 0;
   while (!lstm_try<kCluster>(bar, parity)) {
     ++spins;
     if (stop && (spins & 0xF) == 0 && ld_acquire_cta_shared_u32(stop)) return lstm_try<kCluster>(bar, parity);
-    if ((spins & 0xFF) == 0) {
-      if (*c.abort_smem) return false;
-      if (globaltimer_ns() > c.deadline_ns) {
-        record_timeout(c, DEV_TIMEOUT_MBAR, where);
-        return false;
-      }
-    }
+    if ((spins & 0xFF) == 0 && lstm_expired(w, DEV_TIMEOUT_MBAR, where)) return false;
   }
   return true;
 }
-template <bool kCluster>
-__device__ __forceinline__ bool lstm_wait_warp(uint32_t bar, uint32_t parity, const WaitCtl& c, int where, int lane, uint32_t stop = 0) {
+template <bool kCluster, class W>
+__device__ __forceinline__ bool lstm_wait_warp(uint32_t bar, uint32_t parity, const W& w, int where, int lane, uint32_t stop = 0) {
   if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
   if (__all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity))) return true;
   int ok = 1;
-  if (lane == 0) ok = lstm_wait_loop<kCluster>(bar, parity, c, where, stop) ? 1 : 0;
+  if (lane == 0) ok = lstm_wait_loop<kCluster>(bar, parity, w, where, stop) ? 1 : 0;
   if (__shfl_sync(0xffffffffu, ok, 0) == 0) return false;
   return __all_sync(0xffffffffu, lstm_try<kCluster>(bar, parity));       // complete: lane 0 has seen it
 }
@@ -184,12 +206,25 @@ struct LstmShared {
   uint32_t stored[kWarps];                      // steps whose hidden states a cell warp has stored to global memory
 };
 
+template <int H>
+__device__ __forceinline__ void lstm_wait_set(LstmWaitOf<H>& w, LstmShared<H>& sh, const LstmParams& p) {
+  if constexpr (H < 256) {
+    w.abort_smem = &sh.abort;
+    w.status_g = p.status;
+    w.deadline_ns = sh.deadline_ns;
+  } else {
+    w.abort = &sh.abort;
+    w.deadline_ns = &sh.deadline_ns;
+    w.status = p.status;
+  }
+}
+
 // The cell arithmetic of all steps from t on (c_state: the cell state, before step t, of the lane's unit: the same value in its
 // eight lanes); both are brought up to date.
 // kPieces: input vectors may come in several pieces; without, the loop ends (false) in front of the first step whose vector
 // does.  False with the abort flag set: a wait has run out.
 template <int H, bool kPieces>
-__device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& sh, const WaitCtl& ctl, int layer, int part, int tid,
+__device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& sh, const LstmWaitOf<H>& ctl, int layer, int part, int tid,
                                            int& t, float& c_state) {
   constexpr int U = H / kLstmParts, kWarps = LstmShared<H>::kWarps, kRow = LstmShared<H>::kRow, kXReg = LstmShared<H>::kXReg;
   constexpr uint32_t kStepBytes = 6u * H;
@@ -312,10 +347,8 @@ __device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& s
 template <int H>
 __device__ __noinline__ void lstm_steps_in_pieces(const LstmParams& p, LstmShared<H>& sh, float c_state) {
   int t = *const_cast<volatile int*>(sh.piece + (threadIdx.x >> 5));       // every vector before this one came whole
-  WaitCtl ctl;
-  ctl.abort_smem = &sh.abort;
-  ctl.status_g = p.status;
-  ctl.deadline_ns = sh.deadline_ns;
+  LstmWaitOf<H> ctl;
+  lstm_wait_set<H>(ctl, sh, p);
   lstm_steps<H, true>(p, sh, ctl, blockIdx.x / kLstmParts, (int)cluster_cta_rank(), threadIdx.x, t, c_state);
 }
 
@@ -353,10 +386,8 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   __syncthreads();
   cluster_sync_all();                           // every CTA's barriers exist before anyone arrives on them
 
-  WaitCtl ctl;
-  ctl.abort_smem = &sh.abort;
-  ctl.status_g = p.status;
-  ctl.deadline_ns = sh.deadline_ns;
+  LstmWaitOf<H> ctl;
+  lstm_wait_set<H>(ctl, sh, p);
 
   if (warp == kWarps + 1) {
     // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
@@ -370,14 +401,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         published = n;
       } else if (((++spins) & 0xFF) == 0) {
         int give_up = 0;
-        if (lane == 0) {
-          if (*ctl.abort_smem) {
-            give_up = 1;
-          } else if (globaltimer_ns() > ctl.deadline_ns) {
-            record_timeout(ctl, DEV_TIMEOUT_FLAG, 950);
-            give_up = 1;
-          }
-        }
+        if (lane == 0) give_up = lstm_expired(ctl, DEV_TIMEOUT_FLAG, 950) ? 1 : 0;
         if (__shfl_sync(0xffffffffu, give_up, 0)) break;
       }
     }
@@ -410,7 +434,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
       const int xb = n % kLstmXBufs, use = n / kLstmXBufs;
       if (use == 0) return 1;
       int free = 1;
-      if (lane == 0) free = mbar_wait(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900) ? 1 : 0;
+      if (lane == 0) free = lstm_wait_loop<false>(xempty0 + 8 * xb, (uint32_t)(use - 1) & 1u, ctl, 900, 0) ? 1 : 0;
       free = __shfl_sync(0xffffffffu, free, 0);
       __syncwarp();
       return free;
@@ -446,14 +470,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
           if (avail > (unsigned)t) break;
           if (((++spins) & 0x3F) == 0) {
             int give_up = 0;
-            if (lane == 0) {
-              if (*ctl.abort_smem) {
-                give_up = 1;
-              } else if (globaltimer_ns() > ctl.deadline_ns) {
-                record_timeout(ctl, DEV_TIMEOUT_FLAG, 700 + layer);
-                give_up = 1;
-              }
-            }
+            if (lane == 0) give_up = lstm_expired(ctl, DEV_TIMEOUT_FLAG, 700 + layer) ? 1 : 0;
             if (__shfl_sync(0xffffffffu, give_up, 0)) {
               ok = 0;
               break;
@@ -486,7 +503,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
           if (more && !in_pieces) {             // the cell warps have to expect it: they stop in front of this vector
             if (lane == 0) {
               st_release_cta_shared_u32(smem_u32(&sh.pieces), 1u);
-              ok = mbar_wait(smem_u32(&sh.pieces_ready), 0u, ctl, 920) ? 1 : 0;
+              ok = lstm_wait_loop<false>(smem_u32(&sh.pieces_ready), 0u, ctl, 920, 0) ? 1 : 0;
             }
             ok = __shfl_sync(0xffffffffu, ok, 0);
             in_pieces = true;
@@ -509,7 +526,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         if (ok) hand_over(piece++, part_v, up, more ? -down : down);
       }
       if (!ok) {
-        if (lane == 0) *ctl.abort_smem = 1;
+        if (lane == 0) *const_cast<volatile int*>(&sh.abort) = 1;
         break;
       }
       have = next;
@@ -521,7 +538,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     int t = 0;
     float c_state = 0.0f;
     const bool ok = lstm_steps<H, false>(p, sh, ctl, layer, part, tid, t, c_state);
-    if (!ok && *ctl.abort_smem == 0) {          // not given up: vector t comes in pieces, all before it came whole
+    if (!ok && *const_cast<volatile int*>(&sh.abort) == 0) {          // not given up: vector t comes in pieces, all before it came whole
       if (lane == 0) {
         sh.piece[warp] = t;
         mbar_arrive(smem_u32(&sh.pieces_ready));
@@ -533,7 +550,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();
   cluster_sync_all();
-  if (*ctl.abort_smem) {                        // sent by peers before they came here, and not waited for: 200 us are ample
+  if (*const_cast<volatile int*>(&sh.abort)) {   // sent by peers before they came here, and not waited for: 200 us are ample
     if (tid == 0 && p.expired) *p.expired = 1;
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
