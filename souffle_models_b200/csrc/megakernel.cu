@@ -1807,8 +1807,8 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
 // loaded once per stage, in front of the wait for the stage's start.  Sets of columns are merged as (mean, squared deviations
 // from it), which is as exact as a second pass over the row (Chan, Golub, LeVeque) and needs one chain of shuffles and one
 // exchange between the parts.
-// Out of line: its registers are not charged to the stage interpreter.  `red`: 192 bytes of shared memory.
-__device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
+// `red`: 192 bytes of shared memory.
+__device__ __forceinline__ void ln_shared_rows(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
   constexpr int NJ = 2, kG = 2;                           // blocks of 128 columns per warp, planes in flight at once
   const int N = st.N, M = st.M, P = st.n_partial, W = st.splitk, G = (kThreads / 32) / W;
   const int grp = (int)fast_div((uint32_t)warp, (uint32_t)W, st.mg_splitk), part = warp - grp * W;
@@ -2038,8 +2038,9 @@ __device__ __forceinline__ void ln_row_alone(const float* pl, int n_partial, siz
   }
 }
 
-// Out of line; a build has this form or the other one, not both: with both, their registers spill into one another's callers.
-__device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p, SmemCtl& cs, const WaitCtl& ctl, int warp, int lane) {
+// kNJ: the row's blocks of 128 columns, or 0: any.
+template <int kNJ>
+__device__ __forceinline__ void ln_lone_rows(const Stage& st, const MegaParams& p, SmemCtl& cs, const WaitCtl& ctl, int warp, int lane) {
   const int N = st.N, M = st.M, P = st.n_partial;
   const size_t plane = (size_t)M * N;
   const __half* resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
@@ -2054,6 +2055,10 @@ __device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p,
     const __half* ra = resid ? resid + (size_t)row * N : nullptr;
     __half* o0 = out + (size_t)row * N;
     __half* so = st.eps < 0.0f ? o0 : st.sum_out ? reinterpret_cast<__half*>(st.sum_out) + (size_t)row * N : nullptr;
+    if constexpr (kNJ > 0) {
+      ln_row_alone<kNJ>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane);
+      continue;
+    }
     switch (N >> 7) {
       case 1: ln_row_alone<1>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
       case 2: ln_row_alone<2>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
@@ -2062,6 +2067,23 @@ __device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p,
       default: ln_row_alone<8>(pl0, P, plane, ra, bias, gamma, beta, st.eps, o0, so, lane); break;
     }
   }
+}
+
+// The LayerNorm stages of the builds, out of line: their registers are not charged to the stage interpreter.
+__device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
+  ln_shared_rows(st, p, cs, red, ctl, warp, lane);
+}
+__device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p, SmemCtl& cs, const WaitCtl& ctl, int warp, int lane) {
+  ln_lone_rows<0>(st, p, cs, ctl, warp, lane);
+}
+// Both forms, for the build that runs long sequences as well as small batches.  Rows of 768 columns, which leave the shared form
+// four in flight, go one to a warp where a CTA has more than 16 of them (layers of 256 tokens: at 13 rows per CTA 277.6 us shared,
+// 277.8 alone, at 27 395.3 / 389.1, at 69 854.0 / 830.0, at 110 1358 / 1296); narrower rows and rows of 1024 columns are
+// faster shared at any number (512 columns, 110 per CTA: 737.7 / 740.4; 256: 360.2 / 390.4; 1024: 2149 / 2197).  The
+// lone form for all widths would spill here.
+__device__ __noinline__ void ln_stage_either(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
+  if (st.N == 768 && st.M > 16 * (int)gridDim.x) ln_lone_rows<6>(st, p, cs, ctl, warp, lane);
+  else ln_shared_rows(st, p, cs, red, ctl, warp, lane);
 }
 
 // kMerge builds add the patch-merging form (Swin, python/models/swin_transformer/swin_patch_merge.py:1-17): with
@@ -2339,7 +2361,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
         else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
         else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
       } else if (st.type == STAGE_LN) {
-        if constexpr (kFamily == kFamilyBertCoop) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+        if constexpr (kFamily == kFamilyBertCoop) ln_stage_either(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
         else ln_stage_many(st, p, cs, ctl, warp, lane);
       }
     }

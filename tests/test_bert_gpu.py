@@ -200,6 +200,8 @@ def test_autotuned_plan_matches_the_oracle():
     (4, 256, 8, 512),      # 512 columns on two warps, several rows per group
     (4, 256, 16, 1024),    # 1024 columns on four warps, three passes
     (12, 128, 16, 1024),   # many attention items: a warp per row
+    (7, 384, 12, 768),     # long sequences, 18 rows of 768 columns per CTA: a warp per row there too
+    (6, 384, 12, 768),     # 15.6: shared
 ])
 def test_layernorm_rows_shared_by_warps(B, S, heads, ffn):
     """The two LayerNorm forms over the row widths a plan takes, with one and with several rows per group of warps: LayerNorm 1
