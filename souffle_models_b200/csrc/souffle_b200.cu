@@ -695,9 +695,11 @@ static Stage blank_stage(int type) {
 // the plan will build it (shape, epilogue, output pointers) without tile fields; its operands are read through
 // per-call tensor maps over `a` ([M][K]) and `w` ([N][K]), whose contents do not matter for the timing.  A stage
 // that writes split-K planes is timed together with the LayerNorm stage that sums them (`ln_proto`), since more
-// planes make that one slower.  Failures of any kind leave `*choice` as the cycle model set it.
+// planes make that one slower: in the plan's own build of the kernel (`family`), whose LayerNorm stages differ.  Failures of any
+// kind leave `*choice` as the cycle model set it.
 static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void* a, const void* w, int sms, bool allow_split,
-                          int head_split, int max_split, void* tune_ws, TileChoice* choice, bool pair = false) {
+                          int head_split, int max_split, void* tune_ws, TileChoice* choice, int family) {
+  const bool pair = family == kFamilyBertPair;
   std::vector<RankedTile> ranked;
   if (pair) choose_tiles_pair(proto.M, proto.N, proto.K, sms / 2, allow_split, &ranked);
   else choose_tiles(proto.M, proto.N, proto.K, sms, allow_split, false, head_split, &ranked);
@@ -741,7 +743,7 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
     for (int it = 0; it < 26 && ok; ++it) {                // two warm-up launches, twenty-four timed ones
       ok = cudaMemsetAsync(tune_ws, 0, 128, nullptr) == cudaSuccess;
       if (it == 2) ok = ok && cudaEventRecord(e0, nullptr) == cudaSuccess;
-      ok = ok && launch_mega(args, grid, nullptr, pair ? kFamilyBertPair : kFamilyBert) == SOUFFLE_OK;
+      ok = ok && launch_mega(args, grid, nullptr, family) == SOUFFLE_OK;
     }
     float ms = 0.0f;
     int h[4] = {0, 0, 0, 0};
@@ -781,6 +783,9 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   const bool pair = d.pair_mma == 1 && npairs >= 1 && S <= 128 && Hh % 2 == 0 && B * Hh > sms && M >= 2048;
   p->pair = pair;
   if (pair) sms = 2 * npairs;
+  // one attention item per CTA at most, or a long sequence: the stage in which all softmax warps share an item (the grid is at least
+  // as large as there are such items, or all SMs)
+  p->family = pair ? kFamilyBertPair : (S > 128 || B * Hh <= sms) ? kFamilyBertCoop : kFamilyBert;
 
   // ---- buffers ----
   if ((rc = plan_alloc(p, (void**)&p->qkv, (size_t)3 * M * H * 2))) return rc;
@@ -835,22 +840,22 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
       if (!d.bm_qkv && !d.bn_qkv) {
         Stage q = g;
         q.N = 3 * H; q.K = H; q.epi = EPI_QKV; q.out = p->qkv; q.ldo = H;
-        autotune_gemm(q, nullptr, p->ln1, w_tmp, sms, false, 1, 1, tune_ws, &t_qkv, pair);
+        autotune_gemm(q, nullptr, p->ln1, w_tmp, sms, false, 1, 1, tune_ws, &t_qkv, p->family);
       }
       if (!d.bm_fc1 && !d.bn_fc1) {
         Stage f = g;
         f.N = F; f.K = H; f.epi = EPI_F16; f.act = std_variant ? ACT_GELU : ACT_RELU; f.out = p->fc1; f.ldo = F;
-        autotune_gemm(f, nullptr, p->ln1, w_tmp, sms, false, 0, 1, tune_ws, &t_fc1, pair);
+        autotune_gemm(f, nullptr, p->ln1, w_tmp, sms, false, 0, 1, tune_ws, &t_fc1, p->family);
       }
       if (!d.bm_proj && !d.bn_proj && !d.split_proj) {
         Stage f = g;
         f.N = H; f.K = H; f.epi = EPI_PARTIAL; f.partial = reinterpret_cast<float*>(planes); f.ldo = H;
-        autotune_gemm(f, &ln, p->ctx, w_tmp, sms, true, 0, max_split, tune_ws, &t_proj, pair);
+        autotune_gemm(f, &ln, p->ctx, w_tmp, sms, true, 0, max_split, tune_ws, &t_proj, p->family);
       }
       if (!d.bm_fc2 && !d.bn_fc2 && !d.split_fc2) {
         Stage f = g;
         f.N = H; f.K = F; f.epi = EPI_PARTIAL; f.partial = reinterpret_cast<float*>(planes); f.ldo = H;
-        autotune_gemm(f, &ln, p->fc1, w_tmp, sms, true, 0, max_split, tune_ws, &t_fc2, pair);
+        autotune_gemm(f, &ln, p->fc1, w_tmp, sms, true, 0, max_split, tune_ws, &t_fc2, p->family);
       }
     }
     cudaDeviceSynchronize();
@@ -1014,8 +1019,6 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     if ((rc = plan_alloc(p, (void**)&p->d_prof, pb))) return rc;
     SF_CUDA(cudaMemset(p->d_prof, 0, pb));
   }
-  // one attention item per CTA at most, or a long sequence: the stage in which all softmax warps share an item
-  p->family = pair ? kFamilyBertPair : (d.seq > 128 || d.batch * d.heads <= p->grid) ? kFamilyBertCoop : kFamilyBert;
   for (Stage& fs : p->stages)
     if ((rc = finalize_stage(fs, p->desc.debug_max_slots, p->grid, pair))) return rc;
   return upload_program(p);
