@@ -277,7 +277,7 @@ static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_
 // launch helper shared by every entry point
 // ------------------------------------------------------------------------------------
 struct DeviceInfo {
-  int device = -1, sms = 0, cc_major = 0, max_ctas = 0;
+  int device = -1, sms = 0, cc_major = 0, max_ctas = 0, l2_bytes = 0;
   int max_pairs = 0;             // clusters of two CTAs of the pair build that can be resident at once
   int pair_coop = 1;             // the pair launch still carries the cooperative attribute on top of the cluster dimension
   bool attr_set = false;
@@ -292,6 +292,7 @@ static int device_info(DeviceInfo** out) {
   if (d.device < 0) {
     SF_CUDA(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev));
     SF_CUDA(cudaDeviceGetAttribute(&d.cc_major, cudaDevAttrComputeCapabilityMajor, dev));
+    SF_CUDA(cudaDeviceGetAttribute(&d.l2_bytes, cudaDevAttrL2CacheSize, dev));
     if (d.cc_major != 10)
       return fail(SOUFFLE_BAD_DEVICE, "device %d has compute capability %d.x; this library needs sm_100", dev, d.cc_major);
     const void* fns[3] = {(const void*)souffle_megakernel<kFamilyBert>, (const void*)souffle_megakernel<kFamilyBertCoop>,
@@ -592,7 +593,7 @@ namespace souffle {
 
 static int plan_alloc(SouffleBertPlan* p, void** ptr, size_t bytes);
 
-constexpr size_t kL2Bytes = (size_t)126 << 20, kStagesPerLayer = 7;
+constexpr size_t kStagesPerLayer = 7;
 
 // Numbers the stages and copies the program and its tensor maps to the device.
 static int upload_program(SouffleBertPlan* p) {
@@ -612,13 +613,16 @@ static int upload_program(SouffleBertPlan* p) {
     s.dead_ptr[0] = s.dead_ptr[1] = nullptr;
   }
   // Buffers are dropped from L2 only where a layer's intermediates together are larger than it: smaller ones are written anew
-  // before anything evicts them, and the drops cost time (twelve layers at 32 sequences, 88 MB: 1130 us with them, 1110
-  // without; at 16, 44 MB: 787 and 770).  Beyond that they keep dead data from being written to DRAM.
+  // before anything evicts them, and the drops cost time.  Beyond that they keep dead data from being written to DRAM.  Twelve layers
+  // of 128 tokens, hidden 768, with drops / without: 32 sequences (88 MB) 1063 / 1053 us, 40 (110 MB) 1273 / 1269, 44 (121 MB) 1322 /
+  // 1323, 48 (132 MB) 1374 / 1383, 52 (143 MB) 1597 / 1636, 64 (176 MB) 1843 / 1879.
+  DeviceInfo* di = nullptr;
+  if ((rc = device_info(&di))) return rc;
   size_t live = 0;
   for (const SouffleBertPlan::Dead& dd : p->dead_after)
     if (dd.after_stage < kStagesPerLayer) live += dd.bytes;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {
-    if (live <= kL2Bytes) break;
+    if (live <= (size_t)di->l2_bytes) break;
     if (dd.after_stage + 1 >= p->stages.size()) continue;          // nothing runs after it inside the launch
     Stage& nx = p->stages[dd.after_stage + 1];
     const int k = nx.dead_bytes[0] ? 1 : 0;
@@ -1224,8 +1228,11 @@ int souffle_bert_plan_copy_buffers(SouffleBertPlan* plan, int n, const int* whic
   }
   list.n = n;
   if (total == 0) return SOUFFLE_OK;
-  const unsigned long long blocks = (total + 4ull * kCopyThreads - 1) / (4ull * kCopyThreads);
-  souffle_copy_list<<<(unsigned)(blocks < 148ull * 8 ? blocks : 148ull * 8), kCopyThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(list);
+  DeviceInfo* di = nullptr;
+  const int rc = device_info(&di);
+  if (rc) return rc;
+  const unsigned long long blocks = (total + 4ull * kCopyThreads - 1) / (4ull * kCopyThreads), most = 8ull * di->sms;
+  souffle_copy_list<<<(unsigned)(blocks < most ? blocks : most), kCopyThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(list);
   SF_CUDA(cudaGetLastError());
   return SOUFFLE_OK;
 }
