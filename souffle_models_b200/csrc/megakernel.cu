@@ -567,9 +567,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       int mt, nt, ks;
       gemm_item(st, first_item, mt, nt, ks);
       int kk = first_chunk(first_item);
-      bool ok = grid_wait(p, ctl, st.prof_index);
+      bool ok = grid_wait(p, ctl, st.position);
       const long long t_first = prof ? clock64() : 0;
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
       for (int item = first_item; ok && item < g.items;) {
         const int m0 = mt * g.bm + (int)rank * 128, kbase = ks * g.kchunks;
         for (int kc = 0; kc < g.kchunks; ++kc) {
@@ -598,7 +598,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       rs.slot = s;
       rs.slot_bits = bits;
       if (p.prof) {
-        long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
+        long long* pr = p.prof + ((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots;
         pr[5] = t_wait;
         pr[11] = t_first;
       }
@@ -612,7 +612,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       uint32_t s = rs.slot, bits = rs.slot_bits;
       const bool b_mn = st.b_mn_major != 0;
       const uint32_t b_bytes = sub_bytes - a_bytes;
-      bool ok = wait_arrived(ctl_s, st.prof_index, ctl);
+      bool ok = wait_arrived(ctl_s, st.position, ctl);
       for (int item = first_item; ok && item < g.items; item += item_step) {
         int mt, nt, ks;
         gemm_item(st, item, mt, nt, ks);
@@ -710,7 +710,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       rs.slot_bits = bits;
       rs.acc_bits = acc_bits | (acc_next << 2);
       if (p.prof) {
-        long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
+        long long* pr = p.prof + ((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots;
         pr[3] = t_full;
         pr[4] = t_acc;
         pr[12] = t_first;
@@ -738,11 +738,11 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     // cycle totals of the profile go straight to its record (no registers held for them over the tiles)
     auto note = [&](int slot, unsigned cycles) {
       if (warp == 2 && lane == 0)
-        atomicAdd(reinterpret_cast<unsigned long long*>(p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + slot),
+        atomicAdd(reinterpret_cast<unsigned long long*>(p.prof + ((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + slot),
                   (unsigned long long)cycles);
     };
     if (prof && warp == 2 && lane == 0)
-      for (int i = 6; i < 11; ++i) p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + i] = 0;
+      for (int i = 6; i < 11; ++i) p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + i] = 0;
     int box = 0;
     for (int item = first_item; item < g.items; item += item_step) {
       int mt, nt, ks;
@@ -772,7 +772,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           tb = (unsigned)now;
           note(6, tb - tw);
           if (item == first_item && h == 0 && warp == 2 && lane == 0)
-            p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 14] = now;
+            p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 14] = now;
         }
         tc_fence_after_sync();
         const uint32_t t0 = tmem + acc * kAccStride;
@@ -820,7 +820,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     }
     __syncwarp();
     if (prof && warp == 2 && lane == 0)
-      p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 15] = clock64();
+      p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 15] = clock64();
   }
 }
 
@@ -902,8 +902,8 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
 
   if (warp == 0) {
     if (lane == 0) {
-      const bool ok = grid_wait(p, ctl, st.prof_index);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      const bool ok = grid_wait(p, ctl, st.position);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
       for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
         const int qt = item % n_kb, h = (item / n_kb) % H, b = item / (n_kb * H);
         const int rq = ((0 * B + b) * H + h) * S, rk = ((1 * B + b) * H + h) * S, rv = ((2 * B + b) * H + h) * S;
@@ -1132,8 +1132,8 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
   if (warp == 0) {
     if (elect_one()) {
       uint32_t bits = rs.attn_bit | (rs.attn_bit1 << 1);
-      const bool ok = grid_wait(p, ctl, st.prof_index);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      const bool ok = grid_wait(p, ctl, st.position);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
       for (int k = 0; ok && k < my_items; ++k) {
         const int item = item_of(k), g = k & 1;
         const int h = item % H, b = item / H;
@@ -1376,7 +1376,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       if (prof) { const long long c4 = clock64(); t_ws += c1 - c0; t_sm += c2 - c1; t_wo += c3 - c2; t_ep += c4 - c3; t_p1 += c1a - c1; }
     }
     if (prof && warp == 2 && lane == 0) {  // [3] waiting for scores, [4] softmax, [5] waiting for P.V, [6] output
-      long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
+      long long* pr = p.prof + ((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots;
       pr[3] = t_ws; pr[4] = t_sm; pr[5] = t_wo; pr[6] = t_ep; pr[7] = t_p1;
     }
     if (g) rs.attn_bit1 = bit; else rs.attn_bit = bit;
@@ -1478,8 +1478,8 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
   // TMEM: scores of (head g, window j) at column 64 (2 g + j), outputs 256 further on
   if (warp == 0) {
     if (lane == 0) {
-      const bool ok = grid_wait(ca.p, ctl, st.prof_index);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.prof_index);
+      const bool ok = grid_wait(ca.p, ctl, st.position);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
       for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
         const int wp = item / item_h, w0 = wp * (int)n, col = ((item - wp * item_h) * (int)n >> 1) * 64;
         if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 530)) break;
@@ -1601,84 +1601,26 @@ __device__ __noinline__ void drop_dead_buffers(const Stage& st, int tid0, int nt
 }
 
 // ------------------------------------------------------------------------------------
-// LayerNorm stage.  Rows stream through shared memory in batches fetched by bulk copies (all
-// split-K planes plus the residual of a batch are in flight together, several batches deep), so
-// the stage is bound by memory bandwidth rather than by per-warp load latency.  A warp owns a
-// row: z = sum of planes + bias + residual, two-pass statistics in fp32, fp16 output.
+// LayerNorm stages: z = sum of planes + bias + residual, two-pass statistics (or their merged equivalent) in fp32, fp16 output.
+// Rows are read straight from L2, except the patch-merging form (ln_stage_ool), whose rows are gathered from four tokens each by
+// bulk copies into a ring of batches in shared memory.
 // ------------------------------------------------------------------------------------
-constexpr int kLnMaxBufs = 4;
-
-// Two rows per call (the second optional): their instruction streams interleave, which hides the
+// Two gathered rows per call (the second optional): their instruction streams interleave, which hides the
 // shared-memory, shuffle and MUFU latencies a single row's dependent chain exposes.
-// kCg: the rows are read straight from global memory (L2: they were written by other SMs a stage ago).
-template <bool kCg>
-__device__ __forceinline__ float4 ln_ld4(const float* p) {
-  if constexpr (kCg) return __ldcg(reinterpret_cast<const float4*>(p));
-  else return *reinterpret_cast<const float4*>(p);
-}
-template <bool kCg>
-__device__ __forceinline__ uint2 ln_ld2(const __half* p) {
-  if constexpr (kCg) return __ldcg(reinterpret_cast<const uint2*>(p));
-  else return *reinterpret_cast<const uint2*>(p);
-}
-
-template <int NJ, bool kCg = false>
-__device__ __forceinline__ void ln_rows2(const float* pl0, const float* pl1, int n_partial, int plane_stride,
-                                         const __half* res0, const __half* res1, const __half* bias,
-                                         const __half* gamma, const __half* beta, float eps, __half* out0, __half* out1,
-                                         int lane) {
+template <int NJ>
+__device__ __forceinline__ void ln_rows2(const __half* row0, const __half* row1, const __half* gamma, const __half* beta, float eps,
+                                         __half* out0, __half* out1, int lane) {
   const bool two = out1 != nullptr;
   float z[2][NJ][4];
 #pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 a = n_partial > 0 ? ln_ld4<kCg>(pl0 + (lane + 32 * j) * 4) : zero4;
-    const float4 b = (two && n_partial > 0) ? ln_ld4<kCg>(pl1 + (lane + 32 * j) * 4) : zero4;
-    z[0][j][0] = a.x; z[0][j][1] = a.y; z[0][j][2] = a.z; z[0][j][3] = a.w;
-    z[1][j][0] = b.x; z[1][j][1] = b.y; z[1][j][2] = b.z; z[1][j][3] = b.w;
-  }
-  for (int pl = 1; pl < n_partial; ++pl) {
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      const float4 a = ln_ld4<kCg>(pl0 + (size_t)pl * plane_stride + (lane + 32 * j) * 4);
-      z[0][j][0] += a.x; z[0][j][1] += a.y; z[0][j][2] += a.z; z[0][j][3] += a.w;
-      if (two) {
-        const float4 b = ln_ld4<kCg>(pl1 + (size_t)pl * plane_stride + (lane + 32 * j) * 4);
-        z[1][j][0] += b.x; z[1][j][1] += b.y; z[1][j][2] += b.z; z[1][j][3] += b.w;
-      }
-    }
-  }
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    float add[4] = {0.f, 0.f, 0.f, 0.f};
-    if (bias) {
-      const uint2 u = *reinterpret_cast<const uint2*>(bias + (lane + 32 * j) * 4);
-      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-      const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-      add[0] = f0.x; add[1] = f0.y; add[2] = f1.x; add[3] = f1.y;
-    }
+  for (int j = 0; j < NJ; ++j)
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const __half* res = r ? res1 : res0;
-      float rr[4] = {0.f, 0.f, 0.f, 0.f};
-      if (res && (r == 0 || two)) {
-        const uint2 u = ln_ld2<kCg>(res + (lane + 32 * j) * 4);
-        const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
-        const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
-        rr[0] = f0.x; rr[1] = f0.y; rr[2] = f1.x; rr[3] = f1.y;
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) z[r][j][i] += add[i] + rr[i];
+      const uint2 u = r == 0 || two ? *reinterpret_cast<const uint2*>((r ? row1 : row0) + (lane + 32 * j) * 4) : make_uint2(0u, 0u);
+      const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&u.x));
+      const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&u.y));
+      z[r][j][0] = f0.x; z[r][j][1] = f0.y; z[r][j][2] = f1.x; z[r][j][3] = f1.y;
     }
-  }
-  if (eps < 0.0f) {                     // sum only: the split-K reduction of a GEMM whose consumer reads fp16
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      *reinterpret_cast<uint2*>(out0 + (lane + 32 * j) * 4) = make_uint2(pack_h2(z[0][j][0], z[0][j][1]), pack_h2(z[0][j][2], z[0][j][3]));
-      if (two) *reinterpret_cast<uint2*>(out1 + (lane + 32 * j) * 4) = make_uint2(pack_h2(z[1][j][0], z[1][j][1]), pack_h2(z[1][j][2], z[1][j][3]));
-    }
-    return;
-  }
   const float inv_n = 1.0f / (float)(NJ * 128);
   float sa = 0.0f, sb = 0.0f;
 #pragma unroll
@@ -1835,7 +1777,7 @@ __device__ __forceinline__ void ln_shared_rows(const Stage& st, const MegaParams
   const bool affine = st.gamma != nullptr;
   const float inv_n = 1.0f / (float)N;
   red += grp * W;
-  if (!stage_go(p, cs, st.prof_index, ctl, warp, lane)) return;
+  if (!stage_go(p, cs, st.position, ctl, warp, lane)) return;
   auto load_planes = [&](int r, int g0) {
     const float* src = planes + (size_t)r * N + (size_t)g0 * plane;
 #pragma unroll
@@ -2048,7 +1990,7 @@ __device__ __forceinline__ void ln_lone_rows(const Stage& st, const MegaParams& 
   const __half* bias = reinterpret_cast<const __half*>(st.bias);
   const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
   const __half* beta = reinterpret_cast<const __half*>(st.beta);
-  if (!stage_go(p, cs, st.prof_index, ctl, warp, lane)) return;
+  if (!stage_go(p, cs, st.position, ctl, warp, lane)) return;
   if (st.dead_bytes[0]) drop_dead_buffers(st, 0, kThreads);
   for (int row = warp * (int)gridDim.x + (int)blockIdx.x; row < M; row += (int)gridDim.x * (kThreads / 32)) {
     const float* pl0 = st.partial + (size_t)row * N;
@@ -2086,36 +2028,30 @@ __device__ __noinline__ void ln_stage_either(const Stage& st, const MegaParams& 
   else ln_shared_rows(st, p, cs, red, ctl, warp, lane);
 }
 
-// kMerge builds add the patch-merging form (Swin, python/models/swin_transformer/swin_patch_merge.py:1-17): with
-// st.seq = R > 0 the fp16 input is a [batch][R][R][N/4] token grid and row (b, h, w) of the normalised matrix is the
-// concatenation of tokens (2h, 2w), (2h+1, 2w), (2h, 2w+1), (2h+1, 2w+1), fetched as four bulk copies; rows of 2048
+// The patch-merging form (Swin, python/models/swin_transformer/swin_patch_merge.py:1-17): the fp16 input is a
+// [batch][R][R][N/4] token grid (R = st.seq), and row (b, h, w) of the normalised matrix is the concatenation of tokens
+// (2h, 2w), (2h+1, 2w), (2h, 2w+1), (2h+1, 2w+1), fetched as four bulk copies.  N = 512, 1024 or 2048; rows of 2048
 // columns are normalised one per warp and call.
-template <bool kMerge>
-__device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
-                                         __half* vec_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
-  const int N = st.N, M = st.M, P = st.n_partial;
-  const __half* resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
+__device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
+                                              __half* vec_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
+  RoleState rs = RoleState::unpack(state);
+  const int N = st.N, M = st.M;
+  const __half* src = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
   __half* out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p)));
-  const __half* bias = reinterpret_cast<const __half*>(st.bias);
   const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
   const __half* beta = reinterpret_cast<const __half*>(st.beta);
   // Warp 0 only feeds the ring (issuing a bulk copy of tens of KB stalls the issuing thread until the copy
   // engine has taken the previous ones); the other warps normalise rows, two per warp and round.
   constexpr int kComp = kThreads / 32 - 1;
-  // Batch geometry comes from the host (finalize_stage): rows per batch -- up to 96 KB so that two batches are
-  // in flight, at most two rows per warp, and few enough that every CTA gets work -- buffers, batch count.
-  const int row_bytes = (P * 4 + (resid ? 2 : 0)) * N;
+  // batch geometry from the host (finalize_stage)
   const int rb = st.bm, batch_bytes = st.slot_bytes, nbuf = st.nslots, n_batches = st.items;
-  const bool stage_vecs = st.kchunks != 0;   // bias | gamma | beta side by side in shared memory
   const int my_batches = n_batches > (int)blockIdx.x ? (n_batches - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const uint32_t full0 = smem_u32(&cs.ln_full[0]), empty0 = smem_u32(&cs.ln_empty[0]);
   uint32_t bits = rs.ln_bits;
-  const bool prof = p.prof != nullptr;
 
   if (warp == 0) {
     if (lane == 0) {
-      const bool go = grid_wait(p, ctl, st.prof_index);
-      if (prof) p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 9] = clock64();
+      const bool go = grid_wait(p, ctl, st.position);
       int buf = 0;
       for (int k = 0; go && k < my_batches; ++k) {
         const int batch = blockIdx.x + k * gridDim.x;
@@ -2123,90 +2059,56 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
         const int row0 = batch * rb;
         const int rows = (M - row0) < rb ? (M - row0) : rb;
         const uint32_t bar = full0 + 8 * buf;
-        const uint32_t dst = ring + buf * batch_bytes;
-        mbar_expect_tx(bar, (uint32_t)(rows * row_bytes));
-        if (kMerge && st.seq > 0) {
-          ln_gather_rows(dst, resid, row0, rows, N, st.seq, bar);
-          bits ^= 1u << buf;
-          buf = buf + 1 == nbuf ? 0 : buf + 1;
-          continue;
-        }
-        for (int pl = 0; pl < P; ++pl)
-          bulk_load(dst + pl * rb * N * 4, st.partial + ((size_t)pl * M + row0) * N, (uint32_t)(rows * N * 4), bar);
-        if (resid) bulk_load(dst + P * rb * N * 4, resid + (size_t)row0 * N, (uint32_t)(rows * N * 2), bar);
+        mbar_expect_tx(bar, (uint32_t)(rows * N * 2));
+        ln_gather_rows(ring + buf * batch_bytes, src, row0, rows, N, st.seq, bar);
         bits ^= 1u << buf;
         buf = buf + 1 == nbuf ? 0 : buf + 1;
       }
-      if (prof) p.prof[((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 10] = clock64();
     }
     __syncwarp();
   } else {
     const int cw = warp - 1;
-    // The per-column vectors go to shared memory once (while the first batches are in flight): read from global
-    // memory inside the row loop, a miss in the small L1 costs an L2 round trip in the middle of every row.
-    if (stage_vecs) {
-      const __half* srcs[3] = {bias, gamma, beta};
+    // gamma and beta go to shared memory once (while the first batches are in flight): read from global
+    // memory inside the row loop, a miss in the small L1 costs an L2 round trip in the middle of every row
+    if (gamma) {
 #pragma unroll
-      for (int v = 0; v < 3; ++v) {
-        if (!srcs[v]) continue;
-        const uint2* src = reinterpret_cast<const uint2*>(srcs[v]);
-        uint2* dst = reinterpret_cast<uint2*>(vec_s + v * N);
-        for (int i = threadIdx.x - 32; i < N / 4; i += kThreads - 32) dst[i] = __ldg(src + i);
+      for (int v = 0; v < 2; ++v) {
+        const uint2* from = reinterpret_cast<const uint2*>(v ? beta : gamma);
+        uint2* to = reinterpret_cast<uint2*>(vec_s + v * N);
+        for (int i = threadIdx.x - 32; i < N / 4; i += kThreads - 32) to[i] = __ldg(from + i);
       }
       named_barrier_sync(2, kThreads - 32);
-      if (bias) bias = vec_s;
-      if (gamma) { gamma = vec_s + N; beta = vec_s + 2 * N; }
+      gamma = vec_s;
+      beta = vec_s + N;
     }
-    unsigned t_wait = 0, t_comp = 0;
     int buf = 0;
     for (int k = 0; k < my_batches; ++k) {
       const int batch = blockIdx.x + k * gridDim.x;
-      const unsigned tw = prof ? (unsigned)clock64() : 0u;
       const bool ok = mbar_wait_warp(full0 + 8 * buf, (bits >> buf) & 1u, ctl, 600 + buf, lane);
-      const unsigned tc = prof ? (unsigned)clock64() : 0u;
-      t_wait += tc - tw;
       bits ^= 1u << buf;
       if (!ok) break;
       const int row0 = batch * rb;
       const int rows = (M - row0) < rb ? (M - row0) : rb;
-      const float* base = reinterpret_cast<const float*>(ring_ptr + buf * batch_bytes);
-      const __half* rbase = reinterpret_cast<const __half*>(ring_ptr + buf * batch_bytes + P * rb * N * 4);
+      const __half* base = reinterpret_cast<const __half*>(ring_ptr + buf * batch_bytes);
       for (int r = cw; r < rows; r += 2 * kComp) {
         const int r2 = r + kComp;
         const bool two = r2 < rows;
-        const float* pl0 = base + (size_t)r * N;
-        const float* pl1 = two ? base + (size_t)r2 * N : nullptr;
-        const __half* ra = resid ? rbase + (size_t)r * N : nullptr;
-        const __half* rb2 = (resid && two) ? rbase + (size_t)r2 * N : nullptr;
+        const __half* a = base + (size_t)r * N;
+        const __half* b = two ? base + (size_t)r2 * N : nullptr;
         __half* o0 = out + (size_t)(row0 + r) * N;
         __half* o1 = two ? out + (size_t)(row0 + r2) * N : nullptr;
         switch (N >> 7) {
-          case 4: ln_rows2<4>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
-          case 16:
-            if constexpr (kMerge) {
-              ln_row_wide(ra, gamma, beta, st.eps, o0, lane);
-              if (two) ln_row_wide(rb2, gamma, beta, st.eps, o1, lane);
-            }
+          case 4: ln_rows2<4>(a, b, gamma, beta, st.eps, o0, o1, lane); break;
+          case 8: ln_rows2<8>(a, b, gamma, beta, st.eps, o0, o1, lane); break;
+          default:
+            ln_row_wide(a, gamma, beta, st.eps, o0, lane);
+            if (two) ln_row_wide(b, gamma, beta, st.eps, o1, lane);
             break;
-          default: ln_rows2<8>(pl0, pl1, P, rb * N, ra, rb2, bias, gamma, beta, st.eps, o0, o1, lane); break;
         }
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + 8 * buf);    // this warp is done with the buffer
-      if (prof) t_comp += (unsigned)clock64() - tc;
       buf = buf + 1 == nbuf ? 0 : buf + 1;
-    }
-    if (prof && lane == 0)
-      atomicMax(reinterpret_cast<unsigned long long*>(p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots + 11),
-                (unsigned long long)clock64());
-    if (prof && warp == 2 && lane == 0) {    // [3] waiting for a batch, [7] normalising
-      long long* pr = p.prof + ((size_t)st.prof_index * gridDim.x + blockIdx.x) * kProfSlots;
-      pr[3] = t_wait;
-      pr[4] = 0;
-      pr[5] = rb;
-      pr[6] = nbuf;
-      pr[7] = t_comp;
-      pr[8] = my_batches;
     }
   }
   // every thread leaves with the same view of the buffers' phase bits
@@ -2216,6 +2118,7 @@ __device__ __forceinline__ void ln_stage(const Stage& st, const MegaParams& p, S
     if (rem) flip ^= (1u << rem) - 1u;
     rs.ln_bits ^= flip;
   }
+  return rs.pack();
 }
 
 // ------------------------------------------------------------------------------------
@@ -2240,13 +2143,6 @@ __device__ __noinline__ uint32_t gemm_stage_ool(const Stage& st, const CallArgs&
   gemm_stage<true>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
   return r.pack();
 }
-__device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams& p, SmemCtl& cs, uint32_t ring, uint8_t* ring_ptr,
-                                          __half* vec_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
-  RoleState r = RoleState::unpack(state);
-  ln_stage<true>(st, p, cs, ring, ring_ptr, vec_s, r, ctl, warp, lane);
-  return r.pack();
-}
-
 // One warp copies a stage record to shared memory.
 __device__ __forceinline__ void copy_record(Stage* to, const Stage* from, int lane) {
   static_assert(sizeof(Stage) % 16 == 0, "records are copied 16 bytes at a time");

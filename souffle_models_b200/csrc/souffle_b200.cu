@@ -337,7 +337,7 @@ static int device_info(DeviceInfo** out) {
 // `family` selects the build of the kernel (see souffle_megakernel).
 static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, int family = kFamilyBert) {
   CallArgs args = args_in;
-  for (int i = 0; i < 3; ++i) args.inline_stages[i].prof_index = i;      // stages that travel in the launch parameters
+  for (int i = 0; i < 3; ++i) args.inline_stages[i].position = i;      // stages that travel in the launch parameters
   void* kargs[] = {&args};
   if (family == kFamilyBertPair) {
     // Clusters of two CTAs.  All CTAs must be resident at once (the grid barrier): the grid never exceeds what
@@ -399,33 +399,28 @@ static int stage_items(const Stage& s, bool pair = false) {
 // output fits the kernel's 32-bit element offsets.
 static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) {
   if (s.type == STAGE_LN) {
-    // Rows per batch: up to 96 KB (two batches in flight), at most two rows per normalising warp, and few
-    // enough that every CTA gets work.  The per-column vectors are staged in shared memory when a CTA
-    // normalises enough rows to pay for the copy.
-    const int comp = kThreads / 32 - 1;
-    const bool has_resid = s.resid != nullptr || s.resid_sel != PTR_PLAN;
-    const int row_bytes = (s.n_partial * 4 + (has_resid ? 2 : 0)) * s.N;
+    // Rows that need no gather: the warps read them from L2 themselves (nslots = 0), s.splitk warps per row where rows are shared
+    // (ln_shared_rows).
+    if (s.seq == 0) {
+      s.splitk = s.N <= 256 ? 1 : s.N / 256;
+      s.mg_splitk = fast_div_magic((uint32_t)s.splitk);
+      s.bm = 1;
+      s.items = s.M;
+      s.nslots = 0;
+      return SOUFFLE_OK;
+    }
+    // Gathered rows, per batch: up to 96 KB (two batches in flight), at most two rows per normalising warp, and few enough that every
+    // CTA gets work.
+    const int comp = kThreads / 32 - 1, row_bytes = 2 * s.N;
     int rb = 98304 / row_bytes;
     rb = rb > 2 * comp ? 2 * comp : (rb < 1 ? 1 : rb);
-    int per_cta = (s.M + grid - 1) / grid;
+    const int per_cta = (s.M + grid - 1) / grid;
     if (rb > per_cta) rb = per_cta;
     if (rb > comp) rb -= rb % comp;
     s.bm = rb;
     s.slot_bytes = rb * row_bytes;
     s.nslots = 196608 / s.slot_bytes > 4 ? 4 : 196608 / s.slot_bytes;
     s.items = (s.M + rb - 1) / rb;
-    s.kchunks = (3 * s.N * 2 <= kVecBytes) ? 1 : 0;
-    // Rows of up to 1024 columns that need no gather: the warps read them from L2 themselves, s.splitk warps per row
-    // (ln_stage_direct).
-    if (s.seq == 0 && s.N <= 1024) {
-      s.splitk = s.N <= 256 ? 1 : s.N / 256;
-      s.mg_splitk = fast_div_magic((uint32_t)s.splitk);
-      s.bm = 1;
-      s.items = s.M;
-      s.nslots = 0;
-      s.kchunks = 0;
-      return SOUFFLE_OK;
-    }
     if (s.nslots < 1) return fail(SOUFFLE_BAD_SHAPE, "LayerNorm rows of %d bytes do not fit the staging ring", row_bytes);
     return SOUFFLE_OK;
   }
@@ -600,7 +595,7 @@ static int upload_program(SouffleBertPlan* p) {
   int rc;
   for (size_t i = 0; i < p->stages.size(); ++i) {
     Stage& s = p->stages[i];
-    s.prof_index = (int)i;
+    s.position = (int)i;
     // the weights of the GEMM stage that comes next are prefetched into L2 while this stage runs
     s.pf_ptr = nullptr;
     s.pf_bytes = 0;

@@ -40,7 +40,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   int M, N, K;
   int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile)
   int bn;            // tile width in N (multiple of 16, <= 256, divides N)
-  int splitk;        // K is cut into this many independent partial products
+  int splitk;        // K is cut into this many independent partial products (STAGE_LN: warps that may share a row)
   int b_mn_major;    // 0: B stored [N][K] (K contiguous); 1: B stored [K][N] (N contiguous, bn % 64 == 0)
   int epi;           // EpilogueKind
   int act;           // Activation
@@ -66,7 +66,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   float eps;         // < 0: no normalisation, the sum goes to `out`
   void* sum_out;     // fp16 [M][N] or null: the sum (rounded to fp16, which is then what gets normalised) is stored here as well
   int n_partial;     // number of fp32 partial planes to sum
-  int prof_index;    // position of this stage in the program (set by the host when the program is built)
+  int position;      // of this stage in the program, set by the host: the grid barrier counts arrivals against it
   // ---- weight prefetch: the B matrix of the next stage, a GEMM, pulled into L2 by all CTAs at the start of this one
   //      (weights never depend on an earlier stage) ----
   uint32_t pf_bytes;
