@@ -6,7 +6,9 @@ reference (cpp/bert/setup.py:11-46): one command builds everything the bindings 
 """
 from __future__ import annotations
 
+import functools
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -58,12 +60,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     return LIB_PATH
 
 
-def resource_usage() -> dict:
-    """Compiles without linking and returns {function: (registers, spill_store_bytes, spill_load_bytes)} from
-    `ptxas -v`: the kernels, and the out-of-line device functions they call (registers 0 for those: ptxas reports
-    none per function).  The persistent kernels must not spill in their stages: a spilling epilogue cost 10-25%
-    end to end."""
-    import re
+@functools.lru_cache(maxsize=None)
+def _ptxas_log() -> str:
+    """What `ptxas -v` prints for the library's one source file, compiled without linking."""
     import tempfile
     with tempfile.TemporaryDirectory() as tmp:
         cmd = [_nvcc(), "-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-Xptxas", "-v", "-c",
@@ -71,9 +70,30 @@ def resource_usage() -> dict:
         res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
+    return res.stderr
+
+
+def stack_frames() -> dict:
+    """{function: largest stack frame in bytes} of the kernels and their out-of-line device functions."""
+    out, func = {}, None
+    for line in _ptxas_log().splitlines():
+        m = re.search(r"Function properties for (\w+)", line)
+        if m:
+            func = m.group(1)
+        m = re.search(r"(\d+) bytes stack frame", line)
+        if m and func:
+            out[func] = max(out.get(func, 0), int(m.group(1)))
+    return out
+
+
+def resource_usage() -> dict:
+    """Compiles without linking and returns {function: (registers, spill_store_bytes, spill_load_bytes)} from
+    `ptxas -v`: the kernels, and the out-of-line device functions they call (registers 0 for those: ptxas reports
+    none per function).  The persistent kernels must not spill in their stages: a spilling epilogue cost 10-25%
+    end to end."""
     out, name, func = {}, None, None
     spills = (0, 0)
-    for line in res.stderr.splitlines():
+    for line in _ptxas_log().splitlines():
         m = re.search(r"Compiling entry function '(\w+)'", line)
         if m:
             name = m.group(1)

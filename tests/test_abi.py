@@ -91,6 +91,20 @@ def test_persistent_kernels_do_not_spill():
     assert all(v[0] <= 168 for v in mega.values())    # 384 threads per CTA leave 168 registers per thread
 
 
+def test_megakernels_have_no_stack_frame():
+    """Every grid barrier's acquire empties L1, so a word on the stack costs a round trip to L2: neither the four builds nor any
+    function that they call may have one, or a spill."""
+    usage, frames = build.resource_usage(), build.stack_frames()
+    names = ("souffle_megakernel", "gemm_stage_ool", "ln_stage_ool", "ln_stage_direct", "ln_stage_many", "ln_stage_either",
+             "drop_dead_buffers", "attn_swin_stage", "ln_row_wide", "ln_gather_rows", "attn_store_probs", "attn_copy_probs",
+             "grid_wait_loop", "wait_word_loop", "mbar_wait_loop", "record_timeout")
+    for n in names:
+        assert any(n in k for k in frames), n
+    for k in frames:
+        if any(n in k for n in names):
+            assert frames[k] == 0 and usage[k][1:] == (0, 0), (k, frames[k], usage[k])
+
+
 def test_packed_parameter_block_layout():
     """Offsets of the reference's packed 12-layer parameter block (cpp/bert/bert_base_impl.cu:536-572): host-only
     arithmetic, checked on a made-up base address."""
