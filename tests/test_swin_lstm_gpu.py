@@ -1,4 +1,5 @@
 """Parity of the GEMM / Swin MLP / LSTM entry points (through the C ABI) with the oracle."""
+import math
 import os
 
 import pytest
@@ -304,6 +305,23 @@ def test_swin_block_batch2_window8():
     want = torch.cat([so.swin_block(cfg, x[:256], p, 4), so.swin_block(cfg, x[256:], p, 4)])
     _report("Swin block batch 2, window 8: max-abs vs fp32 oracle", (y.float().cpu() - want).abs().max().item())
     assert (y.float().cpu() - want).abs().max() < 1e-2
+
+
+@pytest.mark.parametrize("batch", [1, 12])          # 49 rows, and 588: four per CTA on three groups of warps
+def test_swin_block_with_four_warps_per_row(batch):
+    """The widest rows a block has: 1024 columns, shared by four warps.  Against the oracle that rounds to fp16 where the kernel
+    does; three units in the last place of the largest output for the roundings that fall the other way."""
+    from souffle_models_b200 import swin
+    cfg = so.SwinConfig(res=7, dim=1024, heads=32, window=7)
+    p = so.make_swin_params(cfg, 91, zero_bias=False)
+    x = _rand((batch * 49, 1024), 43)
+    blk = swin.SwinBlock(batch, 7, 1024, 32, 7, 0, {k: v.cuda() for k, v in p.items()})
+    y = blk.forward(x.cuda())
+    blk.status()
+    want = torch.cat([so.swin_block(cfg, x[49 * i:49 * i + 49], p, 0, emulate_fp16=True) for i in range(batch)]).float()
+    err = (y.float().cpu() - want).abs().max().item()
+    _report(f"Swin block, dim 1024, batch {batch}: max-abs vs fp16-storage oracle", err)
+    assert err < 3 * 2.0 ** (math.floor(math.log2(want.abs().max().item())) - 10)
 
 
 @pytest.mark.parametrize("batch,res,dim,heads,window", [(1, 14, 512, 16, 7), (2, 16, 256, 8, 8), (3, 14, 128, 4, 7)])
