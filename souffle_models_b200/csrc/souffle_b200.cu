@@ -558,6 +558,7 @@ struct SouffleBertPlan {
   unsigned launch_id = 0;
   std::vector<Stage> stages;
   std::vector<const void*> stage_weights;   // per stage: the repacked [N][K] weight matrix of a GEMM stage, else null
+  size_t layer_bytes = 0;                   // a layer's intermediates together
   struct Dead { size_t after_stage; const void* ptr; uint32_t bytes; };
   std::vector<Dead> dead_after;             // buffers nobody reads again once stage `after_stage` has run
   std::vector<CUtensorMap> maps;
@@ -588,8 +589,6 @@ namespace souffle {
 
 static int plan_alloc(SouffleBertPlan* p, void** ptr, size_t bytes);
 
-constexpr size_t kStagesPerLayer = 7;
-
 // Numbers the stages and copies the program and its tensor maps to the device.
 static int upload_program(SouffleBertPlan* p) {
   int rc;
@@ -607,17 +606,15 @@ static int upload_program(SouffleBertPlan* p) {
     s.dead_bytes[0] = s.dead_bytes[1] = 0;
     s.dead_ptr[0] = s.dead_ptr[1] = nullptr;
   }
-  // Buffers are dropped from L2 only where a layer's intermediates together are larger than it: smaller ones are written anew
-  // before anything evicts them, and the drops cost time.  Beyond that they keep dead data from being written to DRAM.  Twelve layers
-  // of 128 tokens, hidden 768, with drops / without: 32 sequences (88 MB) 1063 / 1053 us, 40 (110 MB) 1273 / 1269, 44 (121 MB) 1322 /
-  // 1323, 48 (132 MB) 1374 / 1383, 52 (143 MB) 1597 / 1636, 64 (176 MB) 1843 / 1879.
+  // Buffers are dropped from L2 only where a layer's intermediates are larger than half of it: smaller ones are written anew
+  // before anything evicts them, and the drops cost time.  Beyond that they keep dead data from being written to DRAM.  128 tokens,
+  // inputs that change from call to call, with drops / without: twelve layers of hidden 512 at 24 sequences (41 MB) 681 / 669 us,
+  // of hidden 768 at 16 (41 MB) 748 / 740, 24 (61 MB) 895 / 896, 32 (82 MB) 1133 / 1143, 40 (102 MB) 1358 / 1379; one layer at 16
+  // 66.0 / 65.9, 32 99.6 / 101.0, 48 (122 MB) 131.7 / 134.9, 64 (163 MB) 172.2 / 176.1.
   DeviceInfo* di = nullptr;
   if ((rc = device_info(&di))) return rc;
-  size_t live = 0;
-  for (const SouffleBertPlan::Dead& dd : p->dead_after)
-    if (dd.after_stage < kStagesPerLayer) live += dd.bytes;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {
-    if (live <= (size_t)di->l2_bytes) break;
+    if (p->layer_bytes <= (size_t)di->l2_bytes / 2) break;
     if (dd.after_stage + 1 >= p->stages.size()) continue;          // nothing runs after it inside the launch
     Stage& nx = p->stages[dd.after_stage + 1];
     const int k = nx.dead_bytes[0] ? 1 : 0;
@@ -880,6 +877,8 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
             sp_fc2 = t_fc2.split;
   const int max_split = sp_proj > sp_fc2 ? sp_proj : sp_fc2;
   if ((rc = plan_alloc(p, (void**)&p->partial, (size_t)max_split * M * H * 4))) return rc;
+  // Q, K, V, attention output, LayerNorm 1 output, FFN hidden layer and both products' planes
+  p->layer_bytes = (size_t)M * (5 * (size_t)H + F) * 2 + (size_t)(sp_proj + sp_fc2) * M * H * 4;
   // rows of an A box: the tile's height, or one CTA's 128-row half of a pair's tile; rows of a B box: the tile's
   // width, or one CTA's half of it
   auto a_rows = [pair](const TileChoice& t) { return (uint32_t)(pair ? 128 : t.bm); };
