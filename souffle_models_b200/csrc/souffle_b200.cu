@@ -1184,7 +1184,7 @@ int souffle_bert_plan_buffer(SouffleBertPlan* plan, int which, void** ptr_out, s
   }
   if (!ptr) return fail(SOUFFLE_BAD_ARGUMENT, "buffer %d was not requested at plan creation", which);
   if (!d.keep_probs)
-    return fail(SOUFFLE_BAD_ARGUMENT, "stage outputs are kept readable only by plans created with keep_probs (others drop them from L2 once consumed)");
+    return fail(SOUFFLE_BAD_ARGUMENT, "stage outputs are kept readable only by plans created with keep_probs (others may drop them from L2 once consumed)");
   *ptr_out = ptr;
   if (bytes_out) *bytes_out = bytes;
   return SOUFFLE_OK;
