@@ -75,9 +75,10 @@ __device__ __forceinline__ float gate_f(float v, bool is_tanh) {
   return is_tanh ? 1.0f - r : r;
 }
 
-// What the bounded waits look at.  Hidden 64 and 128: a WaitCtl on the stack (in shared memory every step was slower, 3 x 128 x 37
-// 38.1 -> 38.9 us, 8 x 128 x 150 161.7 -> 163.8; recording a timeout without one, 163.0).  Hidden 256, whose step loop has no register left: places known at
-// compile time and no call, where the WaitCtl spilled a word (12 x 256 x 200 284.5 -> 281.5 us).
+// What the bounded waits look at.  Hidden 64 and 128: a WaitCtl on the stack.  In shared memory every step was slower (3 x 128 x 37
+// 38.1 -> 38.9 us, 8 x 128 x 150 161.7 -> 163.8), and so were the places below (163.0 with a call at the limit, 167 without).  Hidden 256,
+// whose step loop has no register left: places known at compile time and no call, where the WaitCtl spilled a word
+// (12 x 256 x 200 284.5 -> 281.5 us).
 struct LstmWait {
   int* abort;                                   // of the CTA, in shared memory
   const unsigned long long* deadline_ns;        // in shared memory
