@@ -830,15 +830,18 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
 // Tile form (the cooperative attention stage): the unnormalised probabilities already sit in shared memory as the
 // fp16 A-operand tiles of P.V ([128 rows][64 keys] per tile, 128-byte rows with the 16-byte pieces XOR-swizzled by
 // row & 7); the 256 softmax threads copy them out scaled by 1 / rowsum: eight threads per row, 32 rows per pass, so a
-// store instruction writes four rows of 128 contiguous bytes.  `sums` = the two groups' partial row sums [2][128].
-__device__ __noinline__ void attn_copy_probs_tiles(const uint8_t* ptiles, const float* sums, __half* mat, int S, int rows, int t8) {
-  const int sub = t8 & 7, rsub = t8 >> 3;
+// store instruction writes four rows of 128 contiguous bytes.  An item has `qrows` query rows, each in 128 / qrows copies
+// (see attn_stage); `sums` = the partial row sums [2][copies][qrows].
+__device__ __noinline__ void attn_copy_probs_tiles(const uint8_t* ptiles, const float* sums, __half* mat, int S, int qrows, int rows, int t8) {
+  const int sub = t8 & 7, rsub = t8 >> 3, copies = 128 / qrows;
   for (int r = rsub; r < rows; r += 32) {
-    const float inv = 1.0f / (sums[r] + sums[128 + r]);
-    const uint8_t* src = ptiles + r * 128 + ((sub ^ (r & 7)) << 4);
+    float sum = 0.0f;
+    for (int i = r; i < 256; i += qrows) sum += sums[i];
+    const float inv = 1.0f / sum;
     __half* dst = mat + (size_t)r * S + sub * 8;
     for (int tile = 0; tile * 64 + sub * 8 + 8 <= S; ++tile) {
-      const uint4 v = *reinterpret_cast<const uint4*>(src + tile * kATileBytes);
+      const int prow = ((tile * 4 + (sub >> 1)) & (copies - 1)) * qrows + r;       // the copy that holds these keys
+      const uint4 v = *reinterpret_cast<const uint4*>(ptiles + tile * kATileBytes + prow * 128 + ((sub ^ (prow & 7)) << 4));
       const uint32_t in[4] = {v.x, v.y, v.z, v.w};
       uint32_t w[4];
 #pragma unroll
@@ -884,14 +887,23 @@ __device__ __noinline__ void attn_store_probs_staged(uint32_t ts, uint8_t* sbuf,
 }
 
 // ------------------------------------------------------------------------------------
-// attention stage: one work item = (sequence, head, 128-query tile); S <= 384, head_dim 64
+// attention stage: one work item = (sequence, head, query tile); S <= 384, head_dim 64
+//
+// A tile has st.bm = 128, 64 or 32 query rows (the smallest for which every CTA has one item at most), and the MMA has 128: a
+// tile of fewer rows is loaded 128 / bm times, one copy below the other, and every copy takes its own share of the keys.  A copy
+// leaves 0 where another copy's keys are, so P.V gives each copy's part of the output, and the parts are added up at the end.
+// So all eight softmax warps have work, and one sequence's attention lies on four times as many CTAs: a layer of one sequence
+// (bm = 32 against 128, the lone lanes' loops as they are) 36.0 -> 34.8 us at 128 tokens, the stage 9.7 k -> 7.2 k cycles; at 384
+// tokens 16.4 k -> 10.3 k.  What is left is latency: 2.7 k until the scores are there, 0.4 k for the maxima, 0.5 k for their
+// exchange, 0.7 k for the exponentials, 0.9 k for P.V, 1.1 k for the output.
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, uint8_t* ring_ptr,
                                            uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
   const MegaParams& p = ca.p;
   const int S = st.seq, B = st.batch, H = st.heads;
+  const int qrows = st.bm, copies = 128 / qrows, n_qt = (S + qrows - 1) / qrows;
   const int n_kb = (S + 127) / 128;
-  const int items = B * H * n_kb;
+  const int items = B * H * n_qt;
   const uint32_t q_off = 0, k_off = kATileBytes, v_off = k_off + n_kb * kATileBytes,
                  p_off = v_off + n_kb * kATileBytes;
   const uint32_t qk_full = smem_u32(&ctl_s.qk_full), qk_empty = smem_u32(&ctl_s.qk_empty);
@@ -901,59 +913,69 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
   const CUtensorMap* tm = map_ptr(ca, st.tm_qkv);
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
+      const CUtensorMap* tmq = map_ptr(ca, st.tm_a);
+      uint32_t bit = rs.attn_bit;
+      int qt = (int)blockIdx.x % n_qt, bh = (int)blockIdx.x / n_qt;          // in front of the wait: divisions
       const bool ok = grid_wait(p, ctl, st.position);
       if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
-      for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-        const int qt = item % n_kb, h = (item / n_kb) % H, b = item / (n_kb * H);
-        const int rq = ((0 * B + b) * H + h) * S, rk = ((1 * B + b) * H + h) * S, rv = ((2 * B + b) * H + h) * S;
-        if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 500)) break;
+      for (int item = blockIdx.x; ok && item < items;) {
+        const int rq = bh * S, rk = (B * H + bh) * S, rv = (2 * B * H + bh) * S;
+        if (!mbar_wait_hot(qk_empty, bit ^ 1u, ctl, 500)) break;
         mbar_expect_tx(qk_full, (uint32_t)(kATileBytes * (1 + n_kb)));
-        tma_load_2d(ring + q_off, tm, qk_full, 0, rq + qt * 128);
+#pragma unroll 1
+        for (int c = 0; c < copies; ++c) tma_load_2d(ring + q_off + c * qrows * 128, tmq, qk_full, 0, rq + qt * qrows);
+#pragma unroll 1
         for (int kb = 0; kb < n_kb; ++kb) tma_load_2d(ring + k_off + kb * kATileBytes, tm, qk_full, 0, rk + kb * 128);
-        if (!mbar_wait(v_empty, rs.attn_bit ^ 1u, ctl, 501)) break;
+        if (!mbar_wait_hot(v_empty, bit ^ 1u, ctl, 501)) break;
         mbar_expect_tx(v_full, (uint32_t)(kATileBytes * n_kb));
+#pragma unroll 1
         for (int kb = 0; kb < n_kb; ++kb) tma_load_2d(ring + v_off + kb * kATileBytes, tm, v_full, 0, rv + kb * 128);
-        rs.attn_bit ^= 1u;
+        bit ^= 1u;
+        item += gridDim.x;
+        qt = item % n_qt;
+        bh = item / n_qt;
       }
+      rs.attn_bit = bit;
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc_f16(128u, 0u);
       const uint32_t idesc_o = umma_idesc_f16(64u, 1u);
       const uint32_t tmem = ctl_s.tmem_base;
+      const uint32_t q_lo = umma_desc_lo(ring + q_off, 16), k_lo = umma_desc_lo(ring + k_off, 16), p_lo = umma_desc_lo(ring + p_off, 16),
+                     v_lo = umma_desc_lo(ring + v_off, 8192);
+      uint32_t bit = rs.attn_bit;
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        if (!mbar_wait(qk_full, rs.attn_bit, ctl, 510)) break;
+        if (!mbar_wait_hot(qk_full, bit, ctl, 510)) break;
         tc_fence_after_sync();
-        const uint64_t qd = umma_desc_sw128(ring + q_off, 16, 1024);
-        for (int kb = 0; kb < n_kb; ++kb) {
-          const uint64_t kd = umma_desc_sw128(ring + k_off + kb * kATileBytes, 16, 1024);
-#pragma unroll
-          for (uint32_t k = 0; k < 4; ++k) umma_f16(tmem + kb * 128, qd + 2u * k, kd + 2u * k, idesc_s, (uint32_t)(k != 0));
-        }
+#pragma unroll 1
+        for (int kb = 0; kb < n_kb; ++kb) umma_f16_k64(tmem + kb * 128, q_lo, k_lo + kb * (kATileBytes >> 4), 2u, idesc_s, 0u);
         umma_commit(s_full);
         umma_commit(qk_empty);
-        if (!mbar_wait(p_full, rs.attn_bit, ctl, 511)) break;
-        if (!mbar_wait(v_full, rs.attn_bit, ctl, 512)) break;
+        if (!mbar_wait_hot(v_full, bit, ctl, 512)) break;
+        if (!mbar_wait_hot(p_full, bit, ctl, 511)) break;
         tc_fence_after_sync();
-        for (int kk = 0; kk < n_kb * 8; ++kk) {
-          const uint64_t pd = umma_desc_sw128(ring + p_off + (kk >> 2) * kATileBytes, 16, 1024) + 2u * (kk & 3);
-          const uint64_t vd = umma_desc_sw128(ring + v_off + (kk >> 3) * kATileBytes, 8192, 1024) + 128u * (kk & 7);
-          umma_f16(tmem + kOCol, pd, vd, idesc_o, (uint32_t)(kk != 0));
-        }
+        // 64 keys per chunk: a tile of P, half a tile of V
+#pragma unroll 1
+        for (int c = 0; c < 2 * n_kb; ++c)
+          umma_f16_k64(tmem + kOCol, p_lo + c * (kATileBytes >> 4), v_lo + c * (8192 >> 4), 128u, idesc_o, (uint32_t)(c != 0));
         umma_commit(o_full);
         umma_commit(v_empty);
-        rs.attn_bit ^= 1u;
+        bit ^= 1u;
       }
+      rs.attn_bit = bit;
     }
     __syncwarp();
   } else if (warp < 2 + kEpiWarps) {
-    // Both groups of four warps work on the same item: group 0 takes the first half of the 16-key blocks, group 1
-    // the second half (a thread of each group owns query row r_in); row maxima and row sums are exchanged through
-    // shared memory around two 256-thread barriers.  The output columns are split 32 / 32 likewise.
+    // Both groups of four warps work on the same item.  Of the 16-key blocks, copy c takes numbers c, c + copies, ...,
+    // group 0 and group 1 in turn (a thread of each group owns row r_in); row maxima and row sums are exchanged through
+    // shared memory around two 256-thread barriers.  The output columns are split 32 / 32 between the groups.
     const int grp = (warp - 2) >> 2, q = warp & 3;
     const int r_in = q * 32 + lane;
+    const int copy = r_in / qrows, row = r_in & (qrows - 1);
+    const int blk0 = copy + grp * copies, stepb = 2 * copies;
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const float sl2 = st.scale * 1.4426950408889634f;
     const int* lens = st.lens_from_call ? p.lens : st.lens;
@@ -967,17 +989,28 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
     // The warps look at the wait limit one by one and meet in barriers, so none leaves the loop early: one that has given up goes
     // through the remaining items without waiting again and without storing.
     bool ok = true;
+    uint8_t* pbase = ring_ptr + p_off + r_in * 128;
+    auto zero16 = [&](int blk) {
+      uint8_t* base = pbase + (blk >> 2) * kATileBytes;
+      const int j = (blk & 3) * 2;
+      *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+      *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+    };
+    const int nb_all = n_kb * 8;
+    if (copies > 1 && (int)blockIdx.x < items) {               // the other copies' keys, while nothing has arrived yet; there is one item
+#pragma unroll 1
+      for (int blk = grp; blk < nb_all; blk += 2)
+        if ((blk & (copies - 1)) != copy) zero16(blk);
+    }
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
-      const int qt = item % n_kb, h = (item / n_kb) % H, b = item / (n_kb * H);
+      const int qt = item % n_qt, h = (item / n_qt) % H, b = item / (n_qt * H);
       const int kv_len = lens ? lens[b] : S;
       ok = ok && mbar_wait_warp(s_full, rs.attn_bit, ctl, 520, lane);
       tc_fence_after_sync();
       // Keys >= kv_len carry the additive -1e4 mask: probability 0 in fp32, never the maximum -> only the blocks
       // with valid keys are visited; the other P blocks are written as zeros.
       const int kvl = kv_len < 1 ? 1 : (kv_len > S ? S : kv_len);
-      const int nb = (kvl + 15) >> 4, nb_all = n_kb * 8;
-      const int nb_half = (nb + 1) >> 1;
-      const int blk0 = grp ? nb_half : 0, blk1 = grp ? nb : nb_half;       // this group's valid blocks
+      const int nb = (kvl + 15) >> 4;
       uint32_t ra[16], rb[16];
       // ---- pass 1: maximum of the raw scores of the valid keys (the scale is positive) ----
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
@@ -994,26 +1027,28 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
           for (int i = 0; i < 16; ++i) m0 = fmaxf(m0, key0 + i < kvl ? __uint_as_float(r[i]) : -INFINITY);
         }
       };
-      if (blk0 < blk1) {
+      if (blk0 < nb) {
         tmem_ld16(tmem + blk0 * 16, ra);
         tmem_ld_wait(ra);
       }
-      for (int blk = blk0; blk < blk1; blk += 2) {
-        if (blk + 1 < blk1) tmem_ld16(tmem + (blk + 1) * 16, rb);
+      for (int blk = blk0; blk < nb; blk += 2 * stepb) {
+        if (blk + stepb < nb) tmem_ld16(tmem + (blk + stepb) * 16, rb);
         max16(ra, blk);
-        if (blk + 1 < blk1) {
+        if (blk + stepb < nb) {
           tmem_ld_wait(rb);
-          if (blk + 2 < blk1) tmem_ld16(tmem + (blk + 2) * 16, ra);
-          max16(rb, blk + 1);
-          if (blk + 2 < blk1) tmem_ld_wait(ra);
+          if (blk + 2 * stepb < nb) tmem_ld16(tmem + (blk + 2 * stepb) * 16, ra);
+          max16(rb, blk + stepb);
+          if (blk + 2 * stepb < nb) tmem_ld_wait(ra);
         }
       }
       red[grp * 128 + r_in] = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
       named_barrier_sync(3, 256);
-      const float mx = fmaxf(red[r_in], red[128 + r_in]) * sl2;
+      float mx = red[row];
+#pragma unroll 1
+      for (int i = row + qrows; i < 256; i += qrows) mx = fmaxf(mx, red[i]);
+      mx *= sl2;
       // ---- pass 2: unnormalised probabilities -> fp16 A-operand tiles (128B-swizzled rows, 64 keys per tile) ----
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      uint8_t* pbase = ring_ptr + p_off + r_in * 128;
       auto exp16 = [&](const uint32_t (&r)[16], int blk) {
         const int key0 = blk * 16;
         uint32_t w[8];
@@ -1040,57 +1075,75 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
         *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
       };
-      if (blk0 < blk1) {
+      if (blk0 < nb) {
         tmem_ld16(tmem + blk0 * 16, ra);
         tmem_ld_wait(ra);
       }
-      for (int blk = blk0; blk < blk1; blk += 2) {
-        if (blk + 1 < blk1) tmem_ld16(tmem + (blk + 1) * 16, rb);
+      for (int blk = blk0; blk < nb; blk += 2 * stepb) {
+        if (blk + stepb < nb) tmem_ld16(tmem + (blk + stepb) * 16, rb);
         exp16(ra, blk);
-        if (blk + 1 < blk1) {
+        if (blk + stepb < nb) {
           tmem_ld_wait(rb);
-          if (blk + 2 < blk1) tmem_ld16(tmem + (blk + 2) * 16, ra);
-          exp16(rb, blk + 1);
-          if (blk + 2 < blk1) tmem_ld_wait(ra);
+          if (blk + 2 * stepb < nb) tmem_ld16(tmem + (blk + 2 * stepb) * 16, ra);
+          exp16(rb, blk + stepb);
+          if (blk + 2 * stepb < nb) tmem_ld_wait(ra);
         }
       }
-      // keys past the valid ones: probability 0 (the two groups share the blocks alternately)
-      for (int blk = nb + grp; blk < nb_all; blk += 2) {
-        uint8_t* base = pbase + (blk >> 2) * kATileBytes;
-        const int j = (blk & 3) * 2;
-        *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-      }
+#pragma unroll 1
+      for (int blk = blk0; blk < nb_all; blk += stepb)        // keys past the valid ones: probability 0
+        if (blk >= nb) zero16(blk);
       red[256 + grp * 128 + r_in] = (s0 + s1) + (s2 + s3);
       fence_proxy_async_smem();                               // this thread's P rows -> visible to the MMA
       named_barrier_sync(3, 256);
-      const float inv = 1.0f / (red[256 + r_in] + red[384 + r_in]);
-      const int qrow = qt * 128 + r_in;
+      float sum = 0.0f;
+#pragma unroll 1
+      for (int i = row; i < 256; i += qrows) sum += red[256 + i];
+      const float inv = 1.0f / sum;
+      const int row0 = qt * qrows;
       tc_fence_before_sync();
       if (grp == 0) mbar_arrive(p_full);                      // 128 arrivals: group 1's rows are behind the barrier above
       if (probs) {
         // parity output: normalised probabilities [B*heads][S][S], copied from the P tiles while P.V runs; nobody may
         // start the next item's P rows or row sums before every thread has copied
-        attn_copy_probs_tiles(ring_ptr + p_off, red + 256, probs + ((size_t)(b * H + h) * S + qt * 128) * S, S,
-                              S - qt * 128 < 128 ? S - qt * 128 : 128, (int)threadIdx.x - 64);
+        attn_copy_probs_tiles(ring_ptr + p_off, red + 256, probs + ((size_t)(b * H + h) * S + row0) * S, S, qrows,
+                              S - row0 < qrows ? S - row0 : qrows, (int)threadIdx.x - 64);
         named_barrier_sync(3, 256);
       }
       ok = ok && mbar_wait_warp(o_full, rs.attn_bit, ctl, 521, lane);
       tc_fence_after_sync();
       {
+        // This group's 32 of the 64 output columns.  The P tiles have been consumed: a warp hands its rows over through 4 KB of
+        // them (16-byte pieces XOR-swizzled by the row), and a thread adds up the copies of eight columns of a row, so that a store
+        // instruction writes eight rows of 64 contiguous bytes.
         uint32_t r0[32];
-        tmem_ld32(tmem + kOCol + grp * 32, r0);               // this group's 32 of the 64 output columns
+        tmem_ld32(tmem + kOCol + grp * 32, r0);
         tmem_ld_wait(r0);
-        if (ok && qrow < S) {
-          uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)b * S + qrow) * hidden + h * st.head_dim + grp * 32);
+        uint8_t* part = ring_ptr + p_off + grp * kATileBytes;
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            dst[i] = make_uint4(pack_h2(__uint_as_float(r0[8 * i]) * inv, __uint_as_float(r0[8 * i + 1]) * inv),
-                                pack_h2(__uint_as_float(r0[8 * i + 2]) * inv, __uint_as_float(r0[8 * i + 3]) * inv),
-                                pack_h2(__uint_as_float(r0[8 * i + 4]) * inv, __uint_as_float(r0[8 * i + 5]) * inv),
-                                pack_h2(__uint_as_float(r0[8 * i + 6]) * inv, __uint_as_float(r0[8 * i + 7]) * inv));
+        for (int i = 0; i < 8; ++i)
+          *reinterpret_cast<float4*>(part + r_in * 128 + ((i ^ (r_in & 7)) << 4)) =
+              make_float4(__uint_as_float(r0[4 * i]) * inv, __uint_as_float(r0[4 * i + 1]) * inv, __uint_as_float(r0[4 * i + 2]) * inv,
+                          __uint_as_float(r0[4 * i + 3]) * inv);
+        if (copies > 1) named_barrier_sync(4 + grp, 128);      // a copy's rows lie with other warps
+        else __syncwarp();
+        // threads 4 r .. 4 r + 3 of the group (of the warp, where it owns its rows alone): columns 8 j .. 8 j + 7
+        const int j = lane & 3;
+        for (int rr = q * 8 + (lane >> 2) + (copies > 1 ? 0 : q * 24); rr < (copies > 1 ? qrows : q * 32 + 32); rr += copies > 1 ? 32 : 8) {
+          float o[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = 0.0f;
+#pragma unroll 1
+          for (int pr = rr; pr < 128; pr += qrows) {
+            const float4 u0 = *reinterpret_cast<const float4*>(part + pr * 128 + (((2 * j) ^ (pr & 7)) << 4));
+            const float4 u1 = *reinterpret_cast<const float4*>(part + pr * 128 + (((2 * j + 1) ^ (pr & 7)) << 4));
+            o[0] += u0.x; o[1] += u0.y; o[2] += u0.z; o[3] += u0.w; o[4] += u1.x; o[5] += u1.y; o[6] += u1.z; o[7] += u1.w;
+          }
+          if (ok && row0 + rr < S)
+            *reinterpret_cast<uint4*>(ctx + ((size_t)b * S + row0 + rr) * hidden + h * st.head_dim + grp * 32 + j * 8) =
+                make_uint4(pack_h2(o[0], o[1]), pack_h2(o[2], o[3]), pack_h2(o[4], o[5]), pack_h2(o[6], o[7]));
         }
       }
+      // (the next item's P rows go over the parts just read, but behind the barrier of its maxima)
       tc_fence_before_sync();
       rs.attn_bit ^= 1u;
     }
@@ -2162,10 +2215,6 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;      // 1024-byte alignment for swizzled tiles
   SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + pad);
-  uint8_t* ring_ptr = smem_raw + pad + kCtlBytes;
-  __half* vec_s = reinterpret_cast<__half*>(ring_ptr + kRingBytes);
-  uint8_t* stage_s = ring_ptr + kRingBytes + kVecBytes;
-  const uint32_t ring = raw + pad + kCtlBytes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -2218,14 +2267,24 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   if constexpr (kFamily == kFamilyBertPair) cluster_sync_all();     // the peer's barriers exist before anything arrives on them
   tc_fence_after_sync();
 
-  const WaitCtl& ctl = cs.wait;
   if (p.prof && threadIdx.x == 0) {          // one record past the stages: kernel entry, prologue done, ...
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[1] = clock64();
   }
 
-  RoleState rs;
+  uint32_t state = RoleState().pack();
   for (int si = 0; si < p.n_stages; ++si) {
+    // Addresses and the warp's role are worked out anew for every stage, the roles' state is packed between them: the compiler would
+    // keep what follows from them in registers over all stages, and the stages that need most of them would spill.
+    uint32_t off = pad, tid = threadIdx.x;
+    asm volatile("" : "+r"(off), "+r"(tid));
+    SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + off);
+    const WaitCtl& ctl = cs.wait;
+    uint8_t* ring_ptr = smem_raw + off + kCtlBytes;
+    __half* vec_s = reinterpret_cast<__half*>(ring_ptr + kRingBytes);
+    uint8_t* stage_s = ring_ptr + kRingBytes + kVecBytes;
+    const uint32_t ring = smem_u32(smem_raw) + off + kCtlBytes;
+    const int warp = (int)(tid >> 5), lane = (int)(tid & 31u);
     const Stage& st = cs.stage[si & 1];
     // The spare warps' part, in front of anything that waits: the next stage's record (constant since the launch: plan-owned
     // programs lie in global memory, the stages of the plan-less entry points in the launch parameters) goes to shared
@@ -2245,17 +2304,21 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       if (wait_go(cs, si, ctl)) drop_dead_buffers(st, warp * 32, 32);
     }
     if constexpr (kFamily == kFamilySwin) {
-      if (st.type == STAGE_GEMM) rs = RoleState::unpack(gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, rs.pack(), ctl, warp, lane));
-      else if (st.type == STAGE_ATTN_SWIN) rs = RoleState::unpack(attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, rs.pack(), ctl, warp, lane));
+      if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
+      else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, state, ctl, warp, lane);
       else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
-      else if (st.type == STAGE_LN) rs = RoleState::unpack(ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, rs.pack(), ctl, warp, lane));
+      else if (st.type == STAGE_LN) state = ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, state, ctl, warp, lane);
     } else {
       if (st.type == STAGE_GEMM) {
+        RoleState rs = RoleState::unpack(state);
         gemm_stage<false, kFamily == kFamilyBertPair>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
+        state = rs.pack();
       } else if (st.type == STAGE_ATTN) {
+        RoleState rs = RoleState::unpack(state);
         if constexpr (kFamily == kFamilyBert) attn_stage_pp<false>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
         else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
         else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
+        state = rs.pack();
       } else if (st.type == STAGE_LN) {
         if constexpr (kFamily == kFamilyBertCoop) ln_stage_either(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
         else ln_stage_many(st, p, cs, ctl, warp, lane);

@@ -389,7 +389,7 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
 static int stage_items(const Stage& s, bool pair = false) {
   if (s.type == STAGE_GEMM) return ((s.M + s.bm - 1) / s.bm) * (s.N / s.bn) * s.splitk;
   if (s.type == STAGE_ATTN && pair) return s.batch * s.heads / 2;
-  if (s.type == STAGE_ATTN) return s.batch * s.heads * ((s.seq + 127) / 128);
+  if (s.type == STAGE_ATTN) return s.batch * s.heads * ((s.seq + s.bm - 1) / s.bm);
   if (s.type == STAGE_ATTN_SWIN)      // s.bn windows x s.bn heads
     return (s.batch * (s.seq / s.win) * (s.seq / s.win) + s.bn - 1) / s.bn * (s.heads / s.bn);
   return s.M;       // rows are dealt out over the CTAs first
@@ -886,13 +886,19 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   p->x_box_rows = (int)a_rows(t_qkv);
 
   // ---- activation maps (A operands, box 64 x 128) ----
-  int m_ctx, m_ln1, m_fc1, m_act[2] = {-1, -1}, m_qkv;
+  int m_ctx, m_ln1, m_fc1, m_act[2] = {-1, -1}, m_qkv, m_q;
   if ((rc = add_map(p, p->ctx, M, H, a_rows(t_proj), &m_ctx))) return rc;
   if ((rc = add_map(p, p->ln1, M, H, a_rows(t_fc1), &m_ln1))) return rc;
   if ((rc = add_map(p, p->fc1, M, F, a_rows(t_fc2), &m_fc1))) return rc;
   for (int i = 0; i < 2; ++i)
     if (p->act[i] && (rc = add_map(p, p->act[i], M, H, a_rows(t_qkv), &m_act[i]))) return rc;
   if ((rc = add_map(p, p->qkv, (uint64_t)3 * B * Hh * S, hd, 128, &m_qkv))) return rc;
+  // query rows per attention item (see attn_stage): as few as leave every CTA one item at most
+  int q_rows = 128;
+  if (p->family == kFamilyBertCoop)
+    while (q_rows > 32 && B * Hh * ((S + q_rows / 2 - 1) / (q_rows / 2)) <= sms) q_rows /= 2;
+  m_q = m_qkv;
+  if (q_rows < 128 && (rc = add_map(p, p->qkv, (uint64_t)3 * B * Hh * S, hd, (uint32_t)q_rows, &m_q))) return rc;
 
   // ---- per layer: repack weights, maps, stages ----
   for (int l = 0; l < L; ++l) {
@@ -958,7 +964,7 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     note_weights(p, wqkv_t);
 
     s = blank_stage(STAGE_ATTN);                       // softmax(QK^T) V
-    s.tm_qkv = m_qkv; s.batch = B; s.heads = Hh; s.seq = S; s.head_dim = hd; s.scale = scale;
+    s.tm_qkv = m_qkv; s.tm_a = m_q; s.bm = q_rows; s.batch = B; s.heads = Hh; s.seq = S; s.head_dim = hd; s.scale = scale;
     s.lens_from_call = 1; s.out = p->ctx; s.probs = (last && d.keep_probs) ? p->probs : nullptr;
     p->stages.push_back(s);
     if (!keep) note_dead(p, p->qkv, (size_t)3 * M * H * 2);            // Q, K, V: read by the attention stage only

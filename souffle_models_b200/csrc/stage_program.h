@@ -33,12 +33,12 @@ enum PtrSel : int { PTR_PLAN = 0, PTR_CALL_X = 1, PTR_CALL_Y = 2 };
 struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 bytes at a time
   int type;
   // ---- GEMM ----
-  int tm_a;          // tensor-map index of the A operand ([M][K], box 64 x bm); negative = per-call map
+  int tm_a;          // tensor-map index of the A operand ([M][K], box 64 x bm; STAGE_ATTN: of Q); negative = per-call map
   int tm_b;          // tensor-map index of the B operand
   int tm_out;        // EPI_PARTIAL with out_tma: tensor-map index of the fp32 planes viewed as [splitk][M][N] (box 16 columns x
   int out_tma;       // 32 rows x 1 plane, 64B swizzle) through which the epilogue stores them; out_tma = 0: plain stores
   int M, N, K;
-  int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile)
+  int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile); STAGE_ATTN: query rows per item
   int bn;            // tile width in N (multiple of 16, <= 256, divides N)
   int splitk;        // K is cut into this many independent partial products (STAGE_LN: warps that may share a row)
   int b_mn_major;    // 0: B stored [N][K] (K contiguous); 1: B stored [K][N] (N contiguous, bn % 64 == 0)

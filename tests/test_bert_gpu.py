@@ -70,6 +70,35 @@ def test_layer_matches_fp32_golden(B, S, heads, ffn, ragged, zero_bias):
     assert torch.isfinite(y).all()
 
 
+@pytest.mark.parametrize("B,S,heads,rows", [
+    (1, 384, 12, 32),                  # 144 items of four copies each, three key blocks per warp
+    (1, 384, 16, 64),                  # two copies
+    (2, 256, 16, 64),
+    (3, 256, 16, 128),                 # one copy, two key blocks
+    (3, 112, 12, 32),                  # the last tile of a sequence has 16 rows, seven key blocks for eight warps
+    (5, 48, 16, 64),                   # fewer keys than a copy has blocks, rows past the sequence
+    (7, 112, 12, 128),
+    (1, 16, 2, 32),
+])
+def test_attention_tiles_of_few_query_rows(B, S, heads, rows):
+    """The attention stage of few items: tiles of 32, 64 and 128 query rows, the shortest valid lengths among them."""
+    cfg = so.BertConfig(B, S, heads, 64, 128, "std")
+    layers = so.make_bert_weights(cfg, 1250, 1, zero_bias=False)
+    x, lens = so.make_bert_input(cfg, 1250, ragged=True)
+    lens[0] = 1
+    lens[-1] = S if B > 1 else min(17, S)
+    for keep in (True, False):
+        enc = _encoder(cfg, layers, keep_probs=keep)
+        assert enc.stage_info(1)["bm"] == rows
+        y = enc.forward(x.cuda(), lens.cuda()).float().cpu().reshape(B * S, -1)
+        enc.status()
+        r = so.bert_layer(cfg, x, layers[0], lens)
+        assert _err(y, r["out"]) < TOL_LAYER
+        if keep:
+            assert _err(enc.buffer("probs"), r["probs"]) < TOL_LAYER
+            assert _err(enc.buffer("ctx"), r["ctx"]) < TOL_LAYER
+
+
 def test_ref_compat_s384_matches_oracle_and_reference_cuda(golden_dir):
     """Drop-in entry (six tensors, REF_COMPAT, S=384) vs the oracle and vs the stored outputs of the
     reference's own kernels on a B200."""
