@@ -33,14 +33,15 @@ constexpr int kThreads = 384;               // registers are handed out per four
 constexpr int kEpiWarps = 8, kEpiThreads = kEpiWarps * 32;
 constexpr int kSpareWarp = 2 + kEpiWarps, kWeightWarp = kSpareWarp + 1;
 constexpr int kRingBytes = 196608;          // 192 KiB operand ring (4 x 48 KiB, 3 x 64 KiB or 6 x 32 KiB slots)
-constexpr int kCtlBytes = 2048;             // barriers, control words, two stage records
-constexpr int kVecBytes = 16384;             // per-stage vectors staged in shared memory (a GEMM's bias as fp32: N <= 4096)
+constexpr int kCtlBytes = 3072;             // barriers, control words, two stage records, two tiles' bias
+constexpr int kVecBytes = 16384;             // per-stage vectors (LayerNorm stages)
 constexpr int kStageRow = 64;                // bytes per staged row; the 16-byte pieces of a row are XOR-swizzled (see below)
 constexpr int kStageWarp = 32 * kStageRow;   // one epilogue warp's transpose buffer
 constexpr int kStageBytes = 8 * kStageWarp;  // 16 KiB
-// Layout after the control block: ring | bias vector | store staging.  The attention stage with three
-// key blocks needs 208 KiB and simply runs over all three regions (it uses neither of the other two).
-constexpr int kSmemBytes = kCtlBytes + kRingBytes + kVecBytes + kStageBytes + 1024;  // + alignment slack
+// Layout after the control block: ring | vectors | store staging.  The attention stage with three
+// key blocks needs 208 KiB and simply runs over all three regions (it uses neither of the other two); the boxes of a GEMM stage's
+// TMA stores take the last two together.
+constexpr int kSmemBytes = kCtlBytes + kRingBytes + kVecBytes + kStageBytes;
 constexpr int kMaxSlots = 8;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kATileBytes = 128 * 64 * 2;   // 128 rows x 64 halves
@@ -70,7 +71,7 @@ struct MegaParams {
 // Everything a launch needs, passed in parameter space: per-call tensor maps (negative map
 // indices: -1 -> call_maps[0], -2 -> call_maps[1], ...), up to two inline stages for the
 // plan-less entry points, and the pointers above.
-constexpr int kCallMaps = 4;
+constexpr int kCallMaps = 6;
 struct CallArgs {
   CUtensorMap call_maps[kCallMaps];
   Stage inline_stages[3];
@@ -95,6 +96,7 @@ struct __align__(8) SmemCtl {
   uint32_t arrived;                 // stages whose arrival this CTA has sent
   uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go / stage_go)
   WaitCtl wait;                     // here and not on the stack: see RoleState
+  alignas(16) float bias[2][256];   // of this tile's and the next tile's columns
   alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their position
 };
 static_assert(sizeof(SmemCtl) <= kCtlBytes, "control block too large");
@@ -262,11 +264,10 @@ __device__ __forceinline__ void gemm_item(const Stage& st, int item, int& mt, in
 // shared memory and would otherwise be re-read around every asm statement).
 struct EpiCtx {
   int epi, act, M, N, ldo;
-  const float* bias_s;     // bias staged in shared memory as fp32 (converted once per stage), or null
   const __half* resid;
   __half* out;
   float* partial;
-  const CUtensorMap* tm_out;   // store map of the fp32 planes, or null: plain stores
+  const CUtensorMap* tm_out;   // store map, or null: plain stores
   bool prof;
 };
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;      // "this row is outside the matrix"
@@ -367,77 +368,70 @@ __device__ __forceinline__ uint32_t epi_col_offset(const Stage& st, const EpiCtx
   return (uint32_t)col;
 }
 
-// One 32-column chunk of the accumulator block: r[i] = column col+i of this thread's own row, whose output
-// offset is `own`; `so[i]` = output offset of row (8*i + lane/4) of the same 32-row block (staged stores).
-template <bool kSwin>
-__device__ __forceinline__ void epilogue_chunk32(const Stage& st, const EpiCtx& e, uint8_t* sbuf, const uint32_t (&r)[32],
-                                                 uint32_t own, const uint32_t (&so)[4], int col, int lane, unsigned& t_mid,
-                                                 uint32_t tma_row, int tma_plane, int& box, int nbox) {
-  if (e.epi == EPI_PARTIAL) {
-    // fp32 planes: two halves of 16 columns = 64 bytes per row each.  (Storing each thread's own 128-byte
-    // row segment directly measured twice as slow: an instruction's cost grows with the lines it touches.)
-    if (e.prof) t_mid = (unsigned)clock64();
-    if (e.tm_out) {
-      // Through the TMA: the thread writes its row's 64 bytes into a staging box (the layout of a 64B-swizzled box of
-      // 16 columns x 32 rows) and one lane hands the box to the copy engine.  A warp has `nbox` boxes, used round
-      // robin: two beside the operand ring while the main loop runs, twelve inside the ring for the CTA's last tile
-      // (whose operands have all been consumed) -- a box is rewritten once the copy issued from it has read it.
-      const int sw_w = (lane >> 1) & 3;
+// Bias, activation and conversion of a 32-column chunk: r[i] = column i of this thread's own row, `bias` = the chunk's in shared
+// memory.  Written phase by phase over the whole chunk -- every loop is 16 independent operations -- instead of element by
+// element: an epilogue warp has at most one other warp on its scheduler, so a dependent chain per element (add, pack, seven GELU
+// steps) runs at one instruction per ALU latency.
+__device__ __forceinline__ void epilogue_values32(const EpiCtx& e, const uint32_t (&r)[32], const float* bias, uint32_t (&w)[16]) {
+  const float4* b4 = reinterpret_cast<const float4*>(bias);     // fp32: no conversions here
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint8_t* buf = sbuf + box * kStageWarp;
-        if (lane == 0) {
-          if (nbox == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<11>();
-        }
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(buf + lane * kStageRow + ((i ^ sw_w) << 4)) =
-              make_uint4(r[16 * half + 4 * i], r[16 * half + 4 * i + 1], r[16 * half + 4 * i + 2], r[16 * half + 4 * i + 3]);
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0 && tma_row != kNoRow) {
-          tma_store_3d(e.tm_out, smem_u32(buf), col + 16 * half, (int)tma_row, tma_plane);
-          bulk_commit_group();
-        }
-        box = box + 1 == nbox ? 0 : box + 1;
-      }
-      return;
-    }
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint8_t* rowptr[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        rowptr[i] = so[i] != kNoRow ? reinterpret_cast<uint8_t*>(e.partial + (so[i] + (uint32_t)(col + 16 * half))) : nullptr;
-      uint32_t w[16];
-#pragma unroll
-      for (int i = 0; i < 16; ++i) w[i] = r[16 * half + i];
-      staged_store_64B(sbuf, w, rowptr, lane);
-    }
-    return;
+  for (int i = 0; i < 8; ++i) {
+    const float4 b = b4[i];
+    w[2 * i] = pack_h2_sum(r[4 * i], r[4 * i + 1], b.x, b.y);
+    w[2 * i + 1] = pack_h2_sum(r[4 * i + 2], r[4 * i + 3], b.z, b.w);
   }
-  // The arithmetic below is written phase by phase over the whole chunk -- every loop is 16 or 32 independent
-  // operations -- instead of element by element: an epilogue warp has at most one other warp on its scheduler, so
-  // a dependent chain per element (conversion, add, pack, seven GELU steps) runs at one instruction per ALU latency.
+  if (e.act == ACT_RELU) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) w[i] = relu_h2(w[i]);
+  } else if (e.act == ACT_GELU) {
+    gelu_tanh_h2x16(w);                                          // on fp16 pairs
+  }
+}
+
+// Stores through the TMA: a lane writes 64 bytes of its row (32 fp16 or 16 fp32 columns) into a box of 32 rows (the layout of a
+// 64B-swizzled box), one lane hands the box to the copy engine.  A warp has kRingBoxes boxes inside the operand ring for the CTA's
+// last tile, whose operands have all been consumed, and two beside the ring before that, used round robin; a box is
+// written again once the copy issued from it has read it, for which the issuing lane waits right behind the next copy.
+// With fp16 outputs going through shared memory twice (written by rows, read back and stored by eight rows of 64 bytes), addresses
+// per chunk and the stage's whole bias vector read from there, a chunk of 32 columns took ~1.9 k cycles of its warp, now ~1.0 k
+// (without GELU 0.9 k): 7 x 112 QKV 13.5 k -> 12.7 k cycles, FC1 17.0 k -> 15.5 k; 64 x 128 FC1 61.9 k -> 59.6 k, on pairs 56.9 k -> 53.2 k.
+constexpr int kRingBoxes = 12;
+struct StoreBoxes {
+  uint8_t* base;
+  int box, n;
+};
+template <class Issue>
+__device__ __forceinline__ void store_box(StoreBoxes& sb, const uint32_t* w, int lane, Issue issue) {
+  uint8_t* buf = sb.base + sb.box * kStageWarp;
+  const int sw = (lane >> 1) & 3;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<uint4*>(buf + lane * kStageRow + ((i ^ sw) << 4)) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+  fence_proxy_async_smem();
+  __syncwarp();
+  if (elect_one()) {
+    issue(smem_u32(buf));
+    bulk_commit_group();
+    if (sb.n == 2) bulk_wait_group_read<1>(); else bulk_wait_group_read<kRingBoxes - 1>();
+  }
+  __syncwarp();
+  sb.box = sb.box + 1 == sb.n ? 0 : sb.box + 1;
+}
+
+// One 32-column chunk of the row-permuting epilogues: r[i] = column col+i of this thread's own row, whose output
+// offset is `own`; `so[i]` = output offset of row (8*i + lane/4) of the same 32-row block (staged stores).
+__device__ __forceinline__ void epilogue_permuted32(const Stage& st, const EpiCtx& e, uint8_t* sbuf, const uint32_t (&r)[32], const float* bias,
+                                                    uint32_t own, const uint32_t (&so)[4], int col, int lane) {
   float v[32];
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-  if (e.bias_s) {               // fp32 in shared memory: no conversions here (they run on the narrow XU pipe)
-    const float4* b4 = reinterpret_cast<const float4*>(e.bias_s + col);
+  {
+    const float4* b4 = reinterpret_cast<const float4*>(bias);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const float4 b = b4[i];
       v[4 * i] += b.x; v[4 * i + 1] += b.y; v[4 * i + 2] += b.z; v[4 * i + 3] += b.w;
     }
-  }
-  const bool gelu_packed = e.act == ACT_GELU && e.resid == nullptr;   // GELU on fp16 pairs after packing (below)
-  if (e.act == ACT_RELU) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = fmaxf(v[i], 0.0f);
-  } else if (e.act == ACT_GELU && !gelu_packed) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = gelu_tanh(v[i]);
   }
   if (e.resid && own != kNoRow) {
     const uint4* r4 = reinterpret_cast<const uint4*>(e.resid + own + col);
@@ -455,21 +449,19 @@ __device__ __forceinline__ void epilogue_chunk32(const Stage& st, const EpiCtx& 
       v[2 * i + 1] += fr[i].y;
     }
   }
-  const uint32_t coff = epi_col_offset<kSwin>(st, e, col);
+  const uint32_t coff = epi_col_offset<true>(st, e, col);
   uint8_t* rowptr[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) rowptr[i] = so[i] != kNoRow ? reinterpret_cast<uint8_t*>(e.out + (so[i] + coff)) : nullptr;
   uint32_t w[16];
 #pragma unroll
   for (int i = 0; i < 16; ++i) w[i] = pack_h2(v[2 * i], v[2 * i + 1]);
-  if (gelu_packed) gelu_tanh_h2x16(w);
-  if (e.prof) t_mid = (unsigned)clock64();
   staged_store_64B(sbuf, w, rowptr, lane);
 }
 
 // 16-column tail chunk (tile widths that are an odd multiple of 16): direct stores.
 template <bool kSwin>
-__device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& e, const uint32_t (&r)[16], uint32_t own, int col) {
+__device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& e, const uint32_t (&r)[16], const float* bias, uint32_t own, int col) {
   if (own == kNoRow) return;
   if (e.epi == EPI_PARTIAL) {
     float4* dst = reinterpret_cast<float4*>(e.partial + own + col);
@@ -481,31 +473,13 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
   }
   float v[16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-  if (e.bias_s) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] += e.bias_s[col + i];
-  }
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]) + bias[i];
   if (e.act == ACT_RELU) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
   } else if (e.act == ACT_GELU) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = gelu_tanh(v[i]);
-  }
-  if (e.resid) {
-    const uint4* r4 = reinterpret_cast<const uint4*>(e.resid + own + col);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint4 u = r4[i];
-      const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 f = __half22float2(h[j]);
-        v[8 * i + 2 * j] += f.x;
-        v[8 * i + 2 * j + 1] += f.y;
-      }
-    }
   }
   uint4* d4 = reinterpret_cast<uint4*>(e.out + (own + epi_col_offset<kSwin>(st, e, col)));
   d4[0] = make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
@@ -535,23 +509,6 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
   const uint32_t rank = kPair ? cluster_cta_rank() : 0u;               // 0 = the pair's leader
   const int first_item = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int item_step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
-  // the stage's bias vector -> shared memory (one global read per CTA instead of one per tile chunk)
-  // (done by the epilogue warps alone; the producer and MMA warps start the main loop meanwhile)
-  const float* bias_s = nullptr;
-  if (warp >= 2 && warp < 2 + kEpiWarps && st.bias && st.epi != EPI_PARTIAL && st.N * 4 <= kVecBytes) {
-    const uint4* src = reinterpret_cast<const uint4*>(st.bias);
-    float4* dst = reinterpret_cast<float4*>(vec_s);
-    for (int i = threadIdx.x - 64; i < st.N / 8; i += kEpiThreads) {
-      const uint4 u = __ldg(src + i);
-      const __half2* h = reinterpret_cast<const __half2*>(&u);
-      const float2 f0 = __half22float2(h[0]), f1 = __half22float2(h[1]), f2 = __half22float2(h[2]), f3 = __half22float2(h[3]);
-      dst[2 * i] = make_float4(f0.x, f0.y, f1.x, f1.y);
-      dst[2 * i + 1] = make_float4(f2.x, f2.y, f3.x, f3.y);
-    }
-    bias_s = reinterpret_cast<const float*>(vec_s);
-    named_barrier_sync(1, kEpiThreads);
-  }
-
   // CTAs start at different K chunks so they do not all pull the same A tile at once
   auto first_chunk = [&](int item) {
     const uint32_t rot = (uint32_t)first_item + (uint32_t)item;
@@ -725,16 +682,12 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     const int full_chunks = g.bn >> 5;
     EpiCtx e;
     e.epi = st.epi; e.act = st.act; e.M = st.M; e.N = st.N; e.ldo = st.ldo;
-    e.bias_s = bias_s;
     e.resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
     e.out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p)));
     e.partial = st.partial;
-    e.tm_out = (st.epi == EPI_PARTIAL && st.out_tma) ? map_ptr(ca, st.tm_out) : nullptr;
+    e.tm_out = st.out_stores ? map_ptr(ca, st.tm_out) : nullptr;
     const bool prof = p.prof != nullptr;
     e.prof = prof;
-    // a warp's staging: 2 KB of the staging area, or -- for the boxes of TMA stores, which want two buffers -- 4 KB of
-    // the vector area and the staging area taken together (a stage that writes planes stages no bias)
-    uint8_t* sbuf = e.tm_out ? reinterpret_cast<uint8_t*>(vec_s) + (warp - 2) * 2 * kStageWarp : stage_s + (warp - 2) * kStageWarp;
     // cycle totals of the profile go straight to its record (no registers held for them over the tiles)
     auto note = [&](int slot, unsigned cycles) {
       if (warp == 2 && lane == 0)
@@ -743,28 +696,60 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     };
     if (prof && warp == 2 && lane == 0)
       for (int i = 6; i < 11; ++i) p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + i] = 0;
-    int box = 0;
-    for (int item = first_item; item < g.items; item += item_step) {
-      int mt, nt, ks;
-      gemm_item(st, item, mt, nt, ks);
+    StoreBoxes sb;
+    sb.base = reinterpret_cast<uint8_t*>(vec_s) + (warp - 2) * 2 * kStageWarp;
+    sb.box = 0;
+    sb.n = 2;
+    // The bias of a tile's columns goes to shared memory as fp32 in front of the tile: a thread loads one column's (0 where there is
+    // none) while the tile before is being stored, and one barrier per tile separates the two buffers' uses.
+    const int my_col = (int)threadIdx.x - 64;
+    const __half* bias = e.epi != EPI_PARTIAL ? reinterpret_cast<const __half*>(st.bias) : nullptr;
+    auto load_bias = [&](int nt) -> float { return bias && my_col < g.bn ? __half2float(__ldg(bias + nt * g.bn + my_col)) : 0.0f; };
+    int mt, nt, ks;
+    gemm_item(st, first_item, mt, nt, ks);
+    float next_bias = first_item < g.items ? load_bias(nt) : 0.0f;
+    uint32_t turn = 0;
+    // The warps look at the wait limit one by one and meet in a barrier per tile: one that has given up goes through the remaining
+    // tiles without waiting again and without storing.
+    bool ok = true;
+#pragma unroll 1
+    for (int item = first_item; item < g.items; item += item_step, turn ^= 1u) {
       const uint32_t acc0 = g.nh == 2 ? 0u : rs.acc_bits >> 2;
-      bool ok = true;
+      const int row_tile = mt * g.bm, colbase = nt * g.bn, plane = ks;
+      const float* bias_t = ctl_s.bias[turn];
+      if (e.epi != EPI_PARTIAL) {
+        ctl_s.bias[turn][my_col] = next_bias;
+        named_barrier_sync(1, kEpiThreads);
+      }
       // TMA-store boxes of the CTA's last tile live in the operand ring: once its accumulator is complete every operand
       // tile of the stage has been consumed, and nothing is loaded before the next stage
-      const bool last_tile = e.tm_out != nullptr && item + item_step >= g.items;
-      uint8_t* tile_sbuf = last_tile ? stage_s - kVecBytes - kRingBytes + (warp - 2) * 12 * kStageWarp : sbuf;
-      const int nbox = last_tile ? 12 : 2;
-      if (last_tile) box = 0;
+      if (item + item_step >= g.items) {
+        sb.base = stage_s - kVecBytes - kRingBytes + (warp - 2) * kRingBoxes * kStageWarp;
+        sb.box = 0;
+        sb.n = kRingBoxes;
+      } else {
+        gemm_item(st, item + item_step, mt, nt, ks);
+        next_bias = load_bias(nt);
+      }
       for (int h = 0; h < g.nh; ++h) {
         const uint32_t acc = acc0 + (uint32_t)h;
         // output rows first: worked out while the accumulator is still being filled
-        const int row0 = mt * g.bm + (kPair ? (int)rank : h) * 128 + q * 32;
-        const uint32_t own = epi_row_offset<kSwin>(st, e, row0 + lane, ks);
+        const int row0 = row_tile + (kPair ? (int)rank : h) * 128 + q * 32;
+        const uint32_t own = epi_row_offset<kSwin>(st, e, row0 + lane, plane);
         uint32_t so[4];                              // rows of the staged stores: each lane has worked out one of the 32
+        if constexpr (kSwin) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) so[i] = __shfl_sync(0xffffffffu, own, 8 * i + (lane >> 2));
+          for (int i = 0; i < 4; ++i) so[i] = __shfl_sync(0xffffffffu, own, 8 * i + (lane >> 2));
+        }
+        // head-split stores: rows of the [3 B heads S][64] view at which the block's two halves of 16 rows begin
+        uint32_t tok0 = 0, tok1 = 0;
+        if (e.epi == EPI_QKV) {
+          tok0 = __shfl_sync(0xffffffffu, own, 0) >> 6;
+          tok1 = __shfl_sync(0xffffffffu, own, 16);
+          tok1 = tok1 == kNoRow ? kNoRow : tok1 >> 6;
+        }
         const unsigned tw = prof ? (unsigned)clock64() : 0u;
-        ok = mbar_wait_warp(tfull0 + 8 * acc, (rs.acc_bits >> acc) & 1u, ctl, 400 + (int)acc, lane);
+        ok = ok && mbar_wait_warp(tfull0 + 8 * acc, (rs.acc_bits >> acc) & 1u, ctl, 400 + (int)acc, lane);
         if (!ok) break;
         unsigned tb = 0;
         if (prof) {
@@ -776,7 +761,6 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         }
         tc_fence_after_sync();
         const uint32_t t0 = tmem + acc * kAccStride;
-        const int colbase = nt * g.bn;
         // this warp takes chunks cpar, cpar+2, ... (its partner warp on the same lane quarter the others)
         for (int c = cpar; c < full_chunks; c += 2) {
           uint32_t r[32];
@@ -788,8 +772,35 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
             tm = (unsigned)clock64();
             note(8, tm - tl);
           }
-          epilogue_chunk32<kSwin>(st, e, tile_sbuf, r, own, so, colbase + c * 32, lane, tmid,
-                                  row0 < e.M ? (uint32_t)row0 : kNoRow, ks, box, nbox);
+          const int col = colbase + c * 32;
+          if (e.epi == EPI_PARTIAL) {
+            // fp32 planes: two boxes of 16 columns.  (Storing each thread's own 128-byte row segment directly measured twice as
+            // slow: an instruction's cost grows with the lines it touches.)
+            if (prof) tmid = (unsigned)clock64();
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+              store_box(sb, r + 16 * half, lane, [&](uint32_t buf) {
+                if (row0 < e.M) tma_store_3d(e.tm_out, buf, col + 16 * half, row0, plane);
+              });
+          } else if (kSwin && !e.tm_out) {
+            epilogue_permuted32(st, e, stage_s + (warp - 2) * kStageWarp, r, bias_t + c * 32, own, so, col, lane);
+          } else {
+            uint32_t w[16];
+            epilogue_values32(e, r, bias_t + c * 32, w);
+            if (prof) tmid = (unsigned)clock64();
+            store_box(sb, w, lane, [&](uint32_t buf) {
+              if (row0 < e.M) {
+                if (!kSwin && e.epi == EPI_QKV) {
+                  const uint32_t gq = (uint32_t)col >> 6, which = fast_div(gq, (uint32_t)st.heads, st.mg_heads), hh = gq - which * (uint32_t)st.heads;
+                  const uint32_t head_row = (which * (uint32_t)(st.batch * st.heads) + hh) * (uint32_t)st.seq;
+                  tma_store_2d(e.tm_out, buf, col & 63, (int)(head_row + tok0));
+                  if (st.out_stores == 2 && tok1 != kNoRow) tma_store_2d(e.tm_out, buf + 16 * kStageRow, col & 63, (int)(head_row + tok1));
+                } else {
+                  tma_store_2d(e.tm_out, buf, col, row0);
+                }
+              }
+            });
+          }
           if (prof) {
             note(9, tmid - tm);
             note(10, (unsigned)clock64() - tmid);
@@ -799,7 +810,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           uint32_t r[16];
           tmem_ld16(t0 + full_chunks * 32, r);
           tmem_ld_wait(r);
-          epilogue_chunk16<kSwin>(st, e, r, own, colbase + full_chunks * 32);
+          epilogue_chunk16<kSwin>(st, e, r, bias_t + full_chunks * 32, own, colbase + full_chunks * 32);
         }
         tc_fence_before_sync();
         if constexpr (kPair) {                      // one arrival per warp on the leader's barrier (16 in all)
@@ -811,10 +822,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         rs.acc_bits ^= 1u << acc;
         if (prof) note(7, (unsigned)clock64() - tb);
       }
-      if (!ok) break;
       if (g.nh == 1) rs.acc_bits ^= 4u;
     }
-    if (e.tm_out && lane == 0) {          // the planes are complete before the CTA reports the stage done
+    if (e.tm_out && elect_one()) {        // the stores are complete before the CTA reports the stage done
       bulk_wait_group_all();
       fence_proxy_async_global();
     }
@@ -978,7 +988,7 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
     const int blk0 = copy + grp * copies, stepb = 2 * copies;
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const float sl2 = st.scale * 1.4426950408889634f;
-    const int* lens = st.lens_from_call ? p.lens : st.lens;
+    const int* lens = p.lens;
     __half* ctx = reinterpret_cast<__half*>(st.out);
     __half* probs = reinterpret_cast<__half*>(st.probs);
     const int hidden = H * st.head_dim;
@@ -1011,7 +1021,7 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
       // with valid keys are visited; the other P blocks are written as zeros.
       const int kvl = kv_len < 1 ? 1 : (kv_len > S ? S : kv_len);
       const int nb = (kvl + 15) >> 4;
-      uint32_t ra[16], rb[16];
+      uint32_t ra[16];                     // (one block at a time: two in flight would spill in this build)
       // ---- pass 1: maximum of the raw scores of the valid keys (the scale is positive) ----
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
       auto max16 = [&](const uint32_t (&r)[16], int blk) {
@@ -1027,19 +1037,10 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
           for (int i = 0; i < 16; ++i) m0 = fmaxf(m0, key0 + i < kvl ? __uint_as_float(r[i]) : -INFINITY);
         }
       };
-      if (blk0 < nb) {
-        tmem_ld16(tmem + blk0 * 16, ra);
+      for (int blk = blk0; blk < nb; blk += stepb) {
+        tmem_ld16(tmem + blk * 16, ra);
         tmem_ld_wait(ra);
-      }
-      for (int blk = blk0; blk < nb; blk += 2 * stepb) {
-        if (blk + stepb < nb) tmem_ld16(tmem + (blk + stepb) * 16, rb);
         max16(ra, blk);
-        if (blk + stepb < nb) {
-          tmem_ld_wait(rb);
-          if (blk + 2 * stepb < nb) tmem_ld16(tmem + (blk + 2 * stepb) * 16, ra);
-          max16(rb, blk + stepb);
-          if (blk + 2 * stepb < nb) tmem_ld_wait(ra);
-        }
       }
       red[grp * 128 + r_in] = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
       named_barrier_sync(3, 256);
@@ -1075,19 +1076,10 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
         *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
       };
-      if (blk0 < nb) {
-        tmem_ld16(tmem + blk0 * 16, ra);
+      for (int blk = blk0; blk < nb; blk += stepb) {
+        tmem_ld16(tmem + blk * 16, ra);
         tmem_ld_wait(ra);
-      }
-      for (int blk = blk0; blk < nb; blk += 2 * stepb) {
-        if (blk + stepb < nb) tmem_ld16(tmem + (blk + stepb) * 16, rb);
         exp16(ra, blk);
-        if (blk + stepb < nb) {
-          tmem_ld_wait(rb);
-          if (blk + 2 * stepb < nb) tmem_ld16(tmem + (blk + 2 * stepb) * 16, ra);
-          exp16(rb, blk + stepb);
-          if (blk + 2 * stepb < nb) tmem_ld_wait(ra);
-        }
       }
 #pragma unroll 1
       for (int blk = blk0; blk < nb_all; blk += stepb)        // keys past the valid ones: probability 0
@@ -1285,7 +1277,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const float sl2 = st.scale * 1.4426950408889634f;
     const float mask_l2 = -10000.0f * 1.4426950408889634f;
-    const int* lens = st.lens_from_call ? p.lens : st.lens;
+    const int* lens = p.lens;
     __half* ctx = reinterpret_cast<__half*>(st.out);
     __half* probs = reinterpret_cast<__half*>(st.probs);
     const int hd = st.head_dim, hidden = H * hd;
@@ -2206,15 +2198,13 @@ template <int kFamily>
 __global__ void __launch_bounds__(kThreads, 1)
 souffle_megakernel(const __grid_constant__ CallArgs ca) {
   const MegaParams& p = ca.p;
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];      // swizzled tiles need 1024-byte alignment
   if (p.prof && threadIdx.x == 0) {
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[0] = clock64();
     pr[3] = (long long)globaltimer_ns();        // wall clock shared by all SMs: launch skew between CTAs
   }
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t pad = ((raw + 1023u) & ~1023u) - raw;      // 1024-byte alignment for swizzled tiles
-  SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + pad);
+  SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
@@ -2276,60 +2266,66 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   for (int si = 0; si < p.n_stages; ++si) {
     // Addresses and the warp's role are worked out anew for every stage, the roles' state is packed between them: the compiler would
     // keep what follows from them in registers over all stages, and the stages that need most of them would spill.
-    uint32_t off = pad, tid = threadIdx.x;
-    asm volatile("" : "+r"(off), "+r"(tid));
-    SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + off);
-    const WaitCtl& ctl = cs.wait;
-    uint8_t* ring_ptr = smem_raw + off + kCtlBytes;
-    __half* vec_s = reinterpret_cast<__half*>(ring_ptr + kRingBytes);
-    uint8_t* stage_s = ring_ptr + kRingBytes + kVecBytes;
-    const uint32_t ring = smem_u32(smem_raw) + off + kCtlBytes;
-    const int warp = (int)(tid >> 5), lane = (int)(tid & 31u);
-    const Stage& st = cs.stage[si & 1];
-    // The spare warps' part, in front of anything that waits: the next stage's record (constant since the launch: plan-owned
-    // programs lie in global memory, the stages of the plan-less entry points in the launch parameters) goes to shared
-    // memory, and this CTA's slice of the next stage's weights to L2 (they come from HBM when the program's weights exceed
-    // L2; without this every GEMM stage starts with all CTAs waiting on the same DRAM rows).
-    if (warp == kWeightWarp && si + 1 < p.n_stages) copy_record(&cs.stage[(si + 1) & 1], p.stages ? p.stages + si + 1 : &ca.inline_stages[si + 1], lane);
-    if (warp == kSpareWarp && lane == 0) {
-      const uint32_t pf_bytes = st.pf_bytes;
-      if (pf_bytes) {
-        const uint32_t per = ((pf_bytes + gridDim.x - 1) / gridDim.x + 15u) & ~15u, off = blockIdx.x * per;
-        if (off < pf_bytes)
-          bulk_prefetch_l2(reinterpret_cast<const char*>(st.pf_ptr) + off, off + per <= pf_bytes ? per : pf_bytes - off);
+    {
+      uint32_t off = 0, tid = threadIdx.x;
+      asm volatile("" : "+r"(off), "+r"(tid));
+      SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + off);
+      const WaitCtl& ctl = cs.wait;
+      uint8_t* ring_ptr = smem_raw + off + kCtlBytes;
+      __half* vec_s = reinterpret_cast<__half*>(ring_ptr + kRingBytes);
+      uint8_t* stage_s = ring_ptr + kRingBytes + kVecBytes;
+      const uint32_t ring = smem_u32(smem_raw) + off + kCtlBytes;
+      const int warp = (int)(tid >> 5), lane = (int)(tid & 31u);
+      const Stage& st = cs.stage[si & 1];
+      // The spare warps' part, in front of anything that waits: the next stage's record (constant since the launch: plan-owned
+      // programs lie in global memory, the stages of the plan-less entry points in the launch parameters) goes to shared
+      // memory, and this CTA's slice of the next stage's weights to L2 (they come from HBM when the program's weights exceed
+      // L2; without this every GEMM stage starts with all CTAs waiting on the same DRAM rows).
+      if (warp == kWeightWarp && si + 1 < p.n_stages) copy_record(&cs.stage[(si + 1) & 1], p.stages ? p.stages + si + 1 : &ca.inline_stages[si + 1], lane);
+      if (warp == kSpareWarp && lane == 0) {
+        const uint32_t pf_bytes = st.pf_bytes;
+        if (pf_bytes) {
+          const uint32_t per = ((pf_bytes + gridDim.x - 1) / gridDim.x + 15u) & ~15u, off = blockIdx.x * per;
+          if (off < pf_bytes)
+            bulk_prefetch_l2(reinterpret_cast<const char*>(st.pf_ptr) + off, off + per <= pf_bytes ? per : pf_bytes - off);
+        }
       }
-    }
-    __syncwarp();
-    if (st.type != STAGE_LN && warp == kSpareWarp && st.dead_bytes[0]) {
-      if (wait_go(cs, si, ctl)) drop_dead_buffers(st, warp * 32, 32);
-    }
-    if constexpr (kFamily == kFamilySwin) {
-      if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
-      else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, state, ctl, warp, lane);
-      else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
-      else if (st.type == STAGE_LN) state = ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, state, ctl, warp, lane);
-    } else {
-      if (st.type == STAGE_GEMM) {
-        RoleState rs = RoleState::unpack(state);
-        gemm_stage<false, kFamily == kFamilyBertPair>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
-        state = rs.pack();
-      } else if (st.type == STAGE_ATTN) {
-        RoleState rs = RoleState::unpack(state);
-        if constexpr (kFamily == kFamilyBert) attn_stage_pp<false>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
-        else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
-        else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
-        state = rs.pack();
-      } else if (st.type == STAGE_LN) {
-        if constexpr (kFamily == kFamilyBertCoop) ln_stage_either(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
-        else ln_stage_many(st, p, cs, ctl, warp, lane);
+      __syncwarp();
+      if (st.type != STAGE_LN && warp == kSpareWarp && st.dead_bytes[0]) {
+        if (wait_go(cs, si, ctl)) drop_dead_buffers(st, warp * 32, 32);
+      }
+      if constexpr (kFamily == kFamilySwin) {
+        if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
+        else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, state, ctl, warp, lane);
+        else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+        else if (st.type == STAGE_LN) state = ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, state, ctl, warp, lane);
+      } else {
+        if (st.type == STAGE_GEMM) {
+          RoleState rs = RoleState::unpack(state);
+          gemm_stage<false, kFamily == kFamilyBertPair>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
+          state = rs.pack();
+        } else if (st.type == STAGE_ATTN) {
+          RoleState rs = RoleState::unpack(state);
+          if constexpr (kFamily == kFamilyBert) attn_stage_pp<false>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
+          else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
+          else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
+          state = rs.pack();
+        } else if (st.type == STAGE_LN) {
+          if constexpr (kFamily == kFamilyBertCoop) ln_stage_either(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
+          else ln_stage_many(st, p, cs, ctl, warp, lane);
+        }
       }
     }
     // Every thread comes by here once per stage, whatever became of its waits, and all leave the loop together.
+    uint32_t off = 0, tid = threadIdx.x;
+    asm volatile("" : "+r"(off), "+r"(tid));
+    SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + off);
+    const WaitCtl& ctl = cs.wait;
     fence_proxy_async_smem();             // this thread's accesses to shared memory before the next stage's copies into it
     if (*ctl.abort_smem) cs.leave[si & 1] = 1;       // two words in turn: the next stage's is not written before all have read this one
     __syncthreads();
     if (*const_cast<volatile int*>(&cs.leave[si & 1])) break;
-    if (warp == kSpareWarp && lane == 0) {
+    if (tid == kSpareWarp * 32) {
       if (p.prof) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
       if (si + 1 < p.n_stages) {
         if (p.skip_arrival > 0 && si == p.skip_arrival >> 16 && (int)blockIdx.x == (p.skip_arrival & 0xFFFF) - 1) *ctl.abort_smem = 1;      // test hook

@@ -171,6 +171,12 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, uint32_t src, int
                ::"l"(tmap), "r"(src), "r"(x), "r"(y), "r"(z)
                : "memory");
 }
+// The same, 2-D.
+__device__ __forceinline__ void tma_store_2d(const void* tmap, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(tmap), "r"(src), "r"(x), "r"(y)
+               : "memory");
+}
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Waits until at most kPending of this thread's bulk groups have not yet READ their shared-memory source.
 template <int kPending>
@@ -513,6 +519,17 @@ __device__ __forceinline__ void gelu_tanh_h2x16(uint32_t (&w)[16]) {
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
   __half2 h = __floats2half2_rn(a, b);
   return *reinterpret_cast<uint32_t*>(&h);
+}
+// fp16 pair of (a + x, b + y): one packed fp32 addition, one conversion
+__device__ __forceinline__ uint32_t pack_h2_sum(uint32_t a, uint32_t b, float x, float y) {
+  float sx, sy;
+  asm("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%2, %3};\n\tmov.b64 v, {%4, %5};\n\tadd.rn.f32x2 u, u, v;\n\tmov.b64 {%0, %1}, u;\n\t}"
+      : "=f"(sx), "=f"(sy) : "r"(a), "r"(b), "f"(x), "f"(y));
+  return pack_h2(sx, sy);
+}
+__device__ __forceinline__ uint32_t relu_h2(uint32_t w) {
+  const __half2 y = __hmax2(*reinterpret_cast<const __half2*>(&w), __float2half2_rn(0.0f));
+  return *reinterpret_cast<const uint32_t*>(&y);
 }
 
 }  // namespace souffle

@@ -69,51 +69,69 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// fp16 matrix [rows][cols] (cols contiguous), box = 64 columns x box_rows rows, 128B swizzle,
-// out-of-range elements read as zero.
-static int make_map_uncached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows);
-
-// A tensor map is a pure function of (address, extents, box): the plan-less entry points, which encode four of
-// them per call, keep the last few per thread.
-static int make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
-  struct Entry { const void* ptr; uint64_t rows, cols; uint32_t box; CUtensorMap map; };
-  constexpr int kEntries = 16;
-  static thread_local Entry cache[kEntries];
-  static thread_local int used = 0, next = 0;
-  for (int i = 0; i < used; ++i) {
-    const Entry& e = cache[i];
-    if (e.ptr == ptr && e.rows == rows && e.cols == cols && e.box == box_rows) {
-      *m = e.map;
-      return SOUFFLE_OK;
-    }
-  }
-  const int rc = make_map_uncached(m, ptr, rows, cols, box_rows);
-  if (rc) return rc;
-  Entry& e = cache[next];
-  e.ptr = ptr; e.rows = rows; e.cols = cols; e.box = box_rows; e.map = *m;
-  next = (next + 1) % kEntries;
-  if (used < kEntries) ++used;
-  return SOUFFLE_OK;
-}
-
-static int make_map_uncached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+// fp16 matrix [rows][cols] (cols contiguous), out-of-range elements read as zero; operand tiles are boxes of 64 columns x box_rows
+// rows, 128B swizzle.
+static int make_map_boxed(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows,
+                          CUtensorMapSwizzle swizzle) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from the driver");
   if (!aligned16(ptr) || (cols * 2) % 16 != 0) return fail(SOUFFLE_BAD_POINTER, "tensor map needs 16-byte alignment");
   cuuint64_t dims[2] = {cols, rows};
   cuuint64_t strides[1] = {cols * 2};
-  cuuint32_t box[2] = {64, box_rows};
+  cuuint32_t box[2] = {box_cols, box_rows};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return SOUFFLE_OK;
+}
+static int make_map_uncached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_map_boxed(m, ptr, rows, cols, 64, box_rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+static int make_store_map_uncached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows);
+static int make_plane_map_uncached(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols);
+
+// A tensor map is a pure function of (address, extents, box): the plan-less entry points, which encode up to six of
+// them per call, keep the last few per thread.
+enum MapKind { MAP_LOAD, MAP_STORE, MAP_PLANES };       // `size`: rows of the box, or the number of planes
+static int make_map_cached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t size, MapKind kind) {
+  struct Entry { const void* ptr; uint64_t rows, cols; uint32_t size; MapKind kind; CUtensorMap map; };
+  constexpr int kEntries = 16;
+  static thread_local Entry cache[kEntries];
+  static thread_local int used = 0, next = 0;
+  for (int i = 0; i < used; ++i) {
+    const Entry& e = cache[i];
+    if (e.ptr == ptr && e.rows == rows && e.cols == cols && e.size == size && e.kind == kind) {
+      *m = e.map;
+      return SOUFFLE_OK;
+    }
+  }
+  const int rc = kind == MAP_LOAD    ? make_map_uncached(m, ptr, rows, cols, size)
+                 : kind == MAP_STORE ? make_store_map_uncached(m, ptr, rows, cols, size)
+                                     : make_plane_map_uncached(m, ptr, size, rows, cols);
+  if (rc) return rc;
+  Entry& e = cache[next];
+  e.ptr = ptr; e.rows = rows; e.cols = cols; e.size = size; e.kind = kind; e.map = *m;
+  next = (next + 1) % kEntries;
+  if (used < kEntries) ++used;
+  return SOUFFLE_OK;
+}
+static int make_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_map_cached(m, ptr, rows, cols, box_rows, MAP_LOAD);
+}
+
+// fp16 matrix [rows][cols] as a store target: box = 32 columns x box_rows rows (64-byte rows in shared memory, 64B swizzle); rows
+// of a box past `rows` are not written.
+static int make_store_map_uncached(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols, uint32_t box_rows) {
+  return make_map_boxed(m, ptr, rows, cols, 32, box_rows, CU_TENSOR_MAP_SWIZZLE_64B);
+}
+static int make_store_map(CUtensorMap* m, const void* ptr, uint64_t rows, uint64_t cols) {
+  return make_map_cached(m, ptr, rows, cols, 32u, MAP_STORE);
 }
 
 // fp32 planes [planes][rows][cols] as a store target: box = 16 columns x 32 rows x 1 plane (64-byte rows in shared
 // memory, 64B swizzle); rows of a box past `rows` are not written.
-static int make_plane_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols) {
+static int make_plane_map_uncached(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from the driver");
   if (!aligned16(ptr) || (cols * 4) % 16 != 0) return fail(SOUFFLE_BAD_POINTER, "tensor map needs 16-byte alignment");
@@ -126,6 +144,9 @@ static int make_plane_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled (planes) failed with CUresult %d", (int)r);
   return SOUFFLE_OK;
+}
+static int make_plane_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols) {
+  return make_map_cached(m, ptr, rows, cols, (uint32_t)planes, MAP_PLANES);
 }
 
 // ------------------------------------------------------------------------------------
@@ -440,8 +461,8 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
       (s.win < 1 || s.win * s.win > 64 || s.seq % s.win || s.heads * 32 != s.ldo ||
        s.M != (s.epi == EPI_SWIN_QKV ? s.batch * s.seq * s.seq : s.batch * (s.seq / s.win) * (s.seq / s.win) * 64)))
     return fail(SOUFFLE_BAD_SHAPE, "window-major epilogue: %d rows do not match batch %d, grid %d, window %d", s.M, s.batch, s.seq, s.win);
-  if (s.bias && s.epi != EPI_PARTIAL && s.N * 4 > kVecBytes)
-    return fail(SOUFFLE_BAD_SHAPE, "a GEMM stage with a bias vector is limited to %d output columns (got %d)", kVecBytes / 4, s.N);
+  if (s.bias && s.epi != EPI_PARTIAL && s.N > 4096)
+    return fail(SOUFFLE_BAD_SHAPE, "a GEMM stage with a bias vector is limited to 4096 output columns (got %d)", s.N);
   s.tiles_n = s.N / s.bn;
   s.kchunks = s.K / 64 / s.splitk;
   s.items = stage_items(s);
@@ -646,22 +667,39 @@ static int add_map(SouffleBertPlan* p, const void* ptr, uint64_t rows, uint64_t 
   return SOUFFLE_OK;
 }
 
-// The store map of a split-K GEMM stage's planes (see make_plane_map); sets the stage's tm_out / out_tma.
-static int add_plane_map(SouffleBertPlan* p, Stage& s) {
-  if ((int)p->maps.size() >= kMaxTensorMaps) return fail(SOUFFLE_BAD_SHAPE, "too many tensor maps");
-  if (s.N % 16) return SOUFFLE_OK;                     // (cannot happen: tile widths are multiples of 16) plain stores
-  CUtensorMap m;
-  int rc = make_plane_map(&m, s.partial, (uint64_t)s.splitk, (uint64_t)s.M, (uint64_t)s.N);
-  if (rc) return rc;
-  s.out_tma = 1;
-  for (size_t i = 0; i < p->maps.size(); ++i)          // the layers of a stack share their planes: one map serves them all
+// Sets a stage's store map: `m` is new to the plan or one it has already (the layers of a stack share their buffers).
+static int set_store_map(SouffleBertPlan* p, Stage& s, const CUtensorMap& m, int stores) {
+  s.out_stores = stores;
+  for (size_t i = 0; i < p->maps.size(); ++i)
     if (memcmp(&p->maps[i], &m, sizeof(m)) == 0) {
       s.tm_out = (int)i;
       return SOUFFLE_OK;
     }
+  if ((int)p->maps.size() >= kMaxTensorMaps) return fail(SOUFFLE_BAD_SHAPE, "too many tensor maps");
   s.tm_out = (int)p->maps.size();
   p->maps.push_back(m);
   return SOUFFLE_OK;
+}
+// The store map of a stage with fp16 output (see make_store_map).  A block of 32 rows of a head-split output may lie in two
+// sequences, whose lengths are multiples of 16.
+static int head_split_stores(int seq) { return seq % 32 ? 2 : 1; }
+static int add_f16_out_map(SouffleBertPlan* p, Stage& s) {
+  CUtensorMap m;
+  int rc;
+  if (s.epi == EPI_QKV) {
+    const int stores = head_split_stores(s.seq);
+    if ((rc = make_store_map_uncached(&m, s.out, (uint64_t)3 * s.batch * s.heads * s.seq, (uint64_t)s.head_dim, (uint32_t)(32 / stores)))) return rc;
+    return set_store_map(p, s, m, stores);
+  }
+  if ((rc = make_store_map_uncached(&m, s.out, (uint64_t)s.M, (uint64_t)s.N, 32u))) return rc;
+  return set_store_map(p, s, m, 1);
+}
+// The store map of a split-K GEMM stage's planes (see make_plane_map).
+static int add_plane_map(SouffleBertPlan* p, Stage& s) {
+  CUtensorMap m;
+  int rc = make_plane_map(&m, s.partial, (uint64_t)s.splitk, (uint64_t)s.M, (uint64_t)s.N);
+  if (rc) return rc;
+  return set_store_map(p, s, m, 1);
 }
 
 // Marks `ptr` (`bytes` long) as dead once the stage just appended has run: the stage appended NEXT drops its lines from
@@ -715,10 +753,16 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
     if (make_map_uncached(&args.call_maps[0], a, (uint64_t)proto.M, (uint64_t)proto.K, (uint32_t)(pair ? 128 : t.bm))) continue;
     if (make_map_uncached(&args.call_maps[1], w, (uint64_t)proto.N, (uint64_t)proto.K, (uint32_t)(pair ? t.bn / 2 : t.bn))) continue;
     if (g.epi == EPI_PARTIAL) {
+      g.out_stores = 1;
       if (make_plane_map(&args.call_maps[2], g.partial, (uint64_t)t.split, (uint64_t)proto.M, (uint64_t)proto.N)) continue;
-      g.tm_out = -3;
-      g.out_tma = 1;
+    } else {
+      const bool split = g.epi == EPI_QKV;
+      g.out_stores = split ? head_split_stores(g.seq) : 1;
+      if (make_store_map_uncached(&args.call_maps[2], g.out, split ? (uint64_t)3 * g.batch * g.heads * g.seq : (uint64_t)g.M,
+                                  split ? (uint64_t)g.head_dim : (uint64_t)g.N, (uint32_t)(32 / g.out_stores)))
+        continue;
     }
+    g.tm_out = -3;
     int items = stage_items(g) * (pair ? 2 : 1);                // CTAs that have work
     args.p.n_stages = 1;
     if (ln_proto) {
@@ -960,12 +1004,13 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     Stage s = blank_stage(STAGE_GEMM);                 // QKV projection, head-split store
     s.tm_a = in_map; s.tm_b = m_wqkv; s.M = M; s.N = 3 * H; s.K = H; s.bm = t_qkv.bm; s.bn = bn_qkv;
     s.epi = EPI_QKV; s.bias = qkv_b; s.out = p->qkv; s.batch = B; s.heads = Hh; s.seq = S; s.head_dim = hd;
+    if ((rc = add_f16_out_map(p, s))) return rc;
     p->stages.push_back(s);
     note_weights(p, wqkv_t);
 
     s = blank_stage(STAGE_ATTN);                       // softmax(QK^T) V
     s.tm_qkv = m_qkv; s.tm_a = m_q; s.bm = q_rows; s.batch = B; s.heads = Hh; s.seq = S; s.head_dim = hd; s.scale = scale;
-    s.lens_from_call = 1; s.out = p->ctx; s.probs = (last && d.keep_probs) ? p->probs : nullptr;
+    s.out = p->ctx; s.probs = (last && d.keep_probs) ? p->probs : nullptr;
     p->stages.push_back(s);
     if (!keep) note_dead(p, p->qkv, (size_t)3 * M * H * 2);            // Q, K, V: read by the attention stage only
 
@@ -987,6 +1032,7 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     s = blank_stage(STAGE_GEMM);                       // FC1 + bias + activation
     s.tm_a = m_ln1; s.tm_b = m_w1; s.M = M; s.N = F; s.K = H; s.bm = t_fc1.bm; s.bn = bn_fc1;
     s.epi = EPI_F16; s.act = std_variant ? ACT_GELU : ACT_RELU; s.bias = fc1_b; s.out = p->fc1; s.ldo = F;
+    if ((rc = add_f16_out_map(p, s))) return rc;
     p->stages.push_back(s);
     note_weights(p, w1_t);
 
@@ -1395,6 +1441,9 @@ int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_
   if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, c, M, N, K, sms))) return rc;
   if ((rc = make_map(&args.call_maps[0], a, M, K, (uint32_t)args.inline_stages[0].bm))) return rc;
   if ((rc = make_map(&args.call_maps[1], w_kn, K, N, 64))) return rc;     // [K][N]: box 64 (N) x 64 (K rows)
+  if ((rc = make_store_map(&args.call_maps[2], c, M, N))) return rc;
+  args.inline_stages[0].tm_out = -3;
+  args.inline_stages[0].out_stores = 1;
   args.p.n_stages = 1;
   const int items = stage_items(args.inline_stages[0]);
   return ws_launch(&args, items < sms ? items : sms, workspace, workspace_bytes, st);
@@ -1447,6 +1496,13 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
   if ((rc = make_map(&args.call_maps[1], fc1_w, C, F, 64))) return rc;
   if ((rc = make_map(&args.call_maps[2], hidden, M, F, (uint32_t)s2.bm))) return rc;
   if ((rc = make_map(&args.call_maps[3], fc2_w, F, C, 64))) return rc;
+  if ((rc = make_store_map(&args.call_maps[4], hidden, M, F))) return rc;
+  args.inline_stages[0].tm_out = -5;
+  if ((rc = split > 1 ? make_plane_map(&args.call_maps[5], s2.partial, (uint64_t)split, (uint64_t)M, (uint64_t)C)
+                      : make_store_map(&args.call_maps[5], out, M, C)))
+    return rc;
+  s2.tm_out = -6;
+  args.inline_stages[0].out_stores = s2.out_stores = 1;
   args.p.n_stages = split > 1 ? 3 : 2;
   int items = stage_items(args.inline_stages[0]);
   const int i2 = stage_items(s2);
@@ -1657,6 +1713,7 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     s = blank_stage(STAGE_GEMM);                           // FC1 + GELU
     s.tm_a = m_y2; s.tm_b = m_w1; s.M = T; s.N = F; s.K = C; s.bm = t_fc1.bm; s.bn = t_fc1.bn; s.epi = EPI_F16; s.act = ACT_GELU;
     s.bias = fc1_b; s.out = hid; s.ldo = F;
+    if ((rc = add_f16_out_map(p, s))) return rc;
     p->stages.push_back(s);
     note_weights(p, w1_t);
     s = blank_stage(STAGE_GEMM);                           // FC2 -> fp32 planes

@@ -35,8 +35,10 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   // ---- GEMM ----
   int tm_a;          // tensor-map index of the A operand ([M][K], box 64 x bm; STAGE_ATTN: of Q); negative = per-call map
   int tm_b;          // tensor-map index of the B operand
-  int tm_out;        // EPI_PARTIAL with out_tma: tensor-map index of the fp32 planes viewed as [splitk][M][N] (box 16 columns x
-  int out_tma;       // 32 rows x 1 plane, 64B swizzle) through which the epilogue stores them; out_tma = 0: plain stores
+  int tm_out;        // with out_stores: tensor-map index of the output, 64B swizzle.  EPI_PARTIAL: the fp32 planes as
+                     // [splitk][M][N], box 16 columns x 32 rows x 1 plane; EPI_F16: [M][N], box 32 x 32; EPI_QKV: [3 B heads S][d],
+                     // box 32 columns x 32 / out_stores rows
+  int out_stores;    // copies per box of 32 rows (2 where a sequence ends inside one); 0: the row-permuting epilogues' plain stores
   int M, N, K;
   int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile); STAGE_ATTN: query rows per item
   int bn;            // tile width in N (multiple of 16, <= 256, divides N)
@@ -54,8 +56,6 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   // ---- attention / head split ----
   int batch, heads, seq, head_dim;
   float scale;       // softmax scale applied to Q.K
-  const int* lens;   // per-sequence valid length or null (selected at call time when lens_from_call)
-  int lens_from_call;
   int tm_qkv;        // tensor map over the head-split buffer viewed as [3*B*heads*S][d], box 64 x 128
   int win, shift;    // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
   const void* rel_bias;  // Swin: fp16 [(2*win-1)^2][heads] relative-position bias table

@@ -45,6 +45,23 @@ def test_gemm_slots_of_one_and_two_k_steps(M, N, K):
     assert (c.float().cpu() - want).abs().max() < 2e-3 * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 64, 64), (31, 64, 128), (33, 192, 64), (127, 320, 64), (129, 64, 192), (1000, 448, 64), (4131, 3072, 64)])
+def test_gemm_stores_end_with_the_matrix(M, N, K):
+    """Outputs leave in boxes of 32 rows: the last rows of a ragged matrix are there and nothing behind them is touched."""
+    from souffle_models_b200 import _lib, swin
+    g = torch.Generator().manual_seed(M)
+    a, w = torch.randn(M, K, generator=g).half(), (torch.randn(K, N, generator=g) * 0.05).half()
+    buf = torch.full((M + 64, N), 7.0, dtype=torch.float16, device="cuda")
+    ws, lib, ac, wc = swin._workspace(), _lib.load(), a.cuda(), w.cuda()
+    stream = torch.cuda.current_stream().cuda_stream
+    _lib.check(lib.souffle_gemm_f16(ac.data_ptr(), wc.data_ptr(), buf.data_ptr(), M, N, K, ws.data_ptr(), ws.numel(), stream))
+    _lib.check(lib.souffle_workspace_status(ws.data_ptr(), stream))
+    out = buf.float().cpu()
+    want = a.float() @ w.float()
+    assert (out[:M] - want).abs().max() < 1e-3 * max(1.0, want.abs().max().item())        # half an ulp of fp16 and fp32 sums
+    assert (out[M:] == 7.0).all()
+
+
 def test_swin_fused_mlp_and_fc2():
     from souffle_models_b200 import swin
     src, w1, w2 = _rand((256, 512), 3), _rand((512, 2048), 4, 0.02), _rand((2048, 512), 5, 0.02)
