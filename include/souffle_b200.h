@@ -183,7 +183,7 @@ int souffle_bert_plan_info(SouffleBertPlan* plan, int* launches_out, int* grid_o
 /* 1 if the plan's launch runs on CTA pairs (see SouffleBertDesc.pair_mma), else 0. */
 int souffle_bert_plan_uses_pairs(SouffleBertPlan* plan);
 /* The tiling chosen for stage `index` of the program: out[0..5] = {stage type (0 GEMM, 1 attention, 2 LayerNorm),
- * tile rows, tile columns, split-K factor, work items, ring slots}.  The reference fixes these at compile time
+ * tile rows, tile columns, split-K factor, work items (0: a LayerNorm that the GEMM stage before it does), ring slots}.  The reference fixes these at compile time
  * (cpp/bert/kernels/bert.h:18-52); here they depend on the shape and on the SM count. */
 int souffle_bert_plan_stage_info(SouffleBertPlan* plan, int index, int out[6]);
 

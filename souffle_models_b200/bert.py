@@ -110,7 +110,8 @@ class BertEncoder:
         return dict(launches=a.value, grid=b.value, stages=c.value, pairs=int(self._lib.souffle_bert_plan_uses_pairs(self._h)))
 
     def stage_info(self, index: int) -> Dict[str, int]:
-        """Tiling of stage `index`: type (0 GEMM, 1 attention, 2 LayerNorm), tile rows/columns, split-K, items, ring slots."""
+        """Tiling of stage `index`: type (0 GEMM, 1 attention, 2 LayerNorm), tile rows/columns, split-K, items
+        (0: the GEMM stage before does this LayerNorm in its epilogue), ring slots."""
         out = (C.c_int * 6)()
         _lib.check(self._lib.souffle_bert_plan_stage_info(self._h, index, out))
         return dict(type=out[0], bm=out[1], bn=out[2], splitk=out[3], items=out[4], slots=out[5])

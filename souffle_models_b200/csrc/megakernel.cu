@@ -46,6 +46,7 @@ constexpr int kMaxSlots = 8;
 constexpr uint32_t kTmemCols = 512;
 constexpr int kATileBytes = 128 * 64 * 2;   // 128 rows x 64 halves
 constexpr int kAccStride = 256;             // TMEM columns between the two accumulator buffers
+constexpr int kUnitBytes = 64 * 64 * 2;     // the unit matrix that adds residuals (of a pair: each CTA has half)
 constexpr int kOCol = 384;                  // TMEM column of the attention output accumulator
 
 struct MegaParams {
@@ -58,6 +59,7 @@ struct MegaParams {
   const int* lens;
   unsigned* sync;       // [0] arrival count, [1] generation used by this launch
   unsigned* sync_next;  // the pair the next launch will use; cleared by this launch
+  unsigned* epoch;      // plan-owned word that this launch increments at its end (EPI_LN tags), or null
   int* status;        // [0] code, [1] where, [2] cta
   int* expired;       // host memory or null: set by a CTA that gave up on a wait
   unsigned long long timeout_ns;
@@ -81,6 +83,8 @@ __device__ __forceinline__ const CUtensorMap* map_ptr(const CallArgs& a, int idx
   return idx < 0 ? &a.call_maps[-idx - 1] : a.p.maps + idx;
 }
 
+extern __shared__ __align__(1024) uint8_t smem_raw[];      // swizzled tiles need 1024-byte alignment
+
 struct __align__(8) SmemCtl {
   uint64_t full[kMaxSlots];
   uint64_t empty[kMaxSlots];
@@ -95,9 +99,10 @@ struct __align__(8) SmemCtl {
   int leave[2];                     // a wait has run out: all warps leave the stage loop together
   uint32_t arrived;                 // stages whose arrival this CTA has sent
   uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go / stage_go)
+  uint32_t epoch;                   // of this launch, see RowStat
   WaitCtl wait;                     // here and not on the stack: see RoleState
   alignas(16) float bias[2][256];   // of this tile's and the next tile's columns
-  alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their position
+  alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their ordinals
 };
 static_assert(sizeof(SmemCtl) <= kCtlBytes, "control block too large");
 
@@ -163,25 +168,25 @@ __device__ __noinline__ bool grid_wait_loop(const unsigned* count, unsigned targ
   }
   return true;
 }
-// One thread: waits until every CTA has finished stage si - 1.  Its acquire and the proxy fence order the other CTAs'
+// One thread: waits until every CTA has finished the stage before `st`.  Its acquire and the proxy fence order the other CTAs'
 // writes before this thread's TMA and bulk copies.  False: the wait has run out.
-__device__ __forceinline__ bool grid_wait(const MegaParams& p, const WaitCtl& ctl, int si) {
-  bool there = si == 0;
+__device__ __forceinline__ bool grid_wait(const MegaParams& p, const WaitCtl& ctl, const Stage& st) {
+  bool there = st.ordinal == 0;
   if (!there) {
-    // The counter only grows during a launch: barrier number `si - 1` is passed once every CTA
-    // has added 1 for it.  (The launch that runs next clears the other counter, see the prologue.)
+    // The counter only grows during a launch: the barrier in front of `st` is passed once every CTA has added 1 for each stage
+    // that runs before it.  (The launch that runs next clears the other counter, see the prologue.)
     const unsigned* count = p.sync;
-    const unsigned target = (unsigned)si * gridDim.x;
+    const unsigned target = (unsigned)st.ordinal * gridDim.x;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
       if (!there) there = ld_acquire_u32(count) >= target;
-    if (!there) there = grid_wait_loop(count, target, ctl, si - 1);
+    if (!there) there = grid_wait_loop(count, target, ctl, st.prev);
     fence_proxy_async_global();
   }
   if (p.prof) {
     const long long now = clock_now();
-    p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 0] = now;
-    if (si > 0) p.prof[((size_t)(si - 1) * gridDim.x + blockIdx.x) * kProfSlots + 2] = now;
+    p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 0] = now;
+    if (st.ordinal > 0) p.prof[((size_t)st.prev * gridDim.x + blockIdx.x) * kProfSlots + 2] = now;
   }
   return there;
 }
@@ -191,7 +196,7 @@ __device__ __noinline__ bool wait_word_loop(uint32_t word, uint32_t want, const 
   while (ld_acquire_cta_shared_u32(word) < want) {
     if (((++spins) & 0xFF) == 0) {
       if (*ctl.abort_smem) return false;
-      if (globaltimer_ns() > ctl.deadline_ns) {
+      if (globaltimer_ns() > ctl.deadline_ns + kWaitGraceNs) {
         record_timeout(ctl, DEV_TIMEOUT_FLAG, where);
         return false;
       }
@@ -202,7 +207,7 @@ __device__ __noinline__ bool wait_word_loop(uint32_t word, uint32_t want, const 
 __device__ __forceinline__ bool wait_word(uint32_t word, uint32_t want, const WaitCtl& ctl, int where) {
   return ld_acquire_cta_shared_u32(word) >= want || wait_word_loop(word, want, ctl, where);
 }
-// One thread: this CTA's arrival for stage si - 1 is on its way.  Copies issued before that would delay it: its release waits for
+// One thread: this CTA's arrival for the stage before the one of ordinal si is on its way.  Copies issued before that would delay it: its release waits for
 // them too.
 __device__ __forceinline__ bool wait_arrived(SmemCtl& cs, int si, const WaitCtl& ctl) { return wait_word(smem_u32(&cs.arrived), (uint32_t)si, ctl, 700); }
 // The feeder's word that stage si may start.
@@ -215,13 +220,13 @@ __device__ __forceinline__ bool wait_go(SmemCtl& cs, int si, const WaitCtl& ctl)
 // through a barrier: warps that judged the limit one by one could part ways when it passes, and those that went on would miss
 // the others' rows or wait for them in a barrier.
 constexpr int kGoBarrier = 15;
-__device__ __forceinline__ bool stage_go(const MegaParams& p, SmemCtl& cs, int si, const WaitCtl& ctl, int warp, int lane) {
+__device__ __forceinline__ bool stage_go(const MegaParams& p, SmemCtl& cs, const Stage& st, const WaitCtl& ctl, int warp, int lane) {
   if (warp == 0) {
-    if (lane == 0 && grid_wait(p, ctl, si)) publish_go(cs, si);
+    if (lane == 0 && grid_wait(p, ctl, st)) publish_go(cs, st.ordinal);
     __syncwarp();
   }
   named_barrier_sync(kGoBarrier, kThreads);
-  return ld_acquire_cta_shared_u32(smem_u32(&cs.go)) > (uint32_t)si;      // not written again before all have met at the stage's end
+  return ld_acquire_cta_shared_u32(smem_u32(&cs.go)) > (uint32_t)st.ordinal;      // not written again before all have met at the stage's end
 }
 
 // The warp's index as a value the compiler knows to be the same in all its lanes (see elect_one).
@@ -486,6 +491,221 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
   d4[1] = make_uint4(pack_h2(v[8], v[9]), pack_h2(v[10], v[11]), pack_h2(v[12], v[13]), pack_h2(v[14], v[15]));
 }
 
+// LayerNorm in the epilogue of a product whose K is not cut: out = LayerNorm(acc + bias + residual) without a plane in memory and
+// without a stage of its own.  A row's columns lie in tiles_n tiles of as many CTAs (or pairs), all of which are running or have run:
+// items are dealt out in order, every CTA takes its own in order, and a CTA has at most one tile of a row block (the host checks that
+// tiles_n is not larger than the grid), so the tile of the lowest number that has not been published never waits for another.
+//   0. The residual is added by the tensor core: behind the last step along K come steps of 64 columns of it times a unit matrix
+//      (exact products, fp32 sums).  Read by the epilogue warps, 16 bytes of a row at a time, it cost 1.5 k cycles per 32 columns.
+//   1. A thread adds the bias to its row's columns, puts the sum back into tensor memory and forms (mean, squared deviations
+//      from it); sets of columns are merged as in ln_shared_rows.
+//   2. The tile's pair is published as a RowStat per row: value and tag in one 64-bit word, so neither a fence in front of the store
+//      nor a flag behind it is needed, and who finds the tags has the values.
+//   3. A thread reads the pairs of all of its row's tiles (bounded), normalises the sums and stores fp16 rows as boxes.
+// Out of line: its registers are not charged to the other stages.  Few arguments: they have to live beside the caller's values.
+// `acc_bits`: see RoleState; bit 31: the stage's record is the second one.
+template <bool kPair>
+__device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) {
+  SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw);
+  const Stage& st = cs.stage[acc_bits >> 31];
+  acc_bits &= 7u;
+  const WaitCtl& ctl = cs.wait;
+  uint8_t* boxes = smem_raw + kCtlBytes + kRingBytes;
+  const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
+  const MegaParams& p = ca.p;
+  const int q = warp & 3, cpar = (warp - 2) >> 2, my_col = (int)threadIdx.x - 64;
+  const int bn = st.bn, chunks = bn >> 5, tiles_n = st.tiles_n, nh = kPair ? 1 : st.bm >> 7, M = st.M;
+  const uint32_t rank = kPair ? cluster_cta_rank() : 0u;
+  const int first_item = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, item_step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+  const uint32_t tfull0 = smem_u32(&cs.tmem_full[0]), tempty0 = smem_u32(&cs.tmem_empty[0]);
+  const uint32_t tmem = cs.tmem_base + ((uint32_t)(q * 32) << 16);
+  const CUtensorMap* tm_out = map_ptr(ca, st.tm_out);
+  const uint32_t tag = (cs.epoch << 8) | st.ordinal;
+  const float inv_n = 1.0f / (float)st.N;
+  const bool prof = p.prof != nullptr, affine = st.gamma != nullptr;
+  float* bias_s = cs.bias[0];
+  __half* gamma_s = reinterpret_cast<__half*>(cs.bias[1]);          // gamma of the tile's columns, then beta
+  // statistics of the warps that have the other chunks of these rows, in their boxes (written again only once all tiles of the row
+  // have been published, and so after they have been read)
+  float2* other = reinterpret_cast<float2*>(boxes + (4 + q) * 2 * kStageWarp);
+  StoreBoxes sb;
+  sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+  sb.box = 0;
+  sb.n = 2;
+  bool ok = true;            // a warp that has given up goes through the remaining tiles, whose barriers the others wait in
+#pragma unroll 1
+  for (int item = first_item; item < st.items; item += item_step) {
+    const int mt = (int)fast_div((uint32_t)item, (uint32_t)tiles_n, st.mg_tiles_n), nt = item - mt * tiles_n;
+    const int colbase = nt * bn;
+    float b = 0.0f;
+    __half gm = __ushort_as_half(0), bt = gm;
+    if (my_col < bn) {
+      if (st.bias) b = __half2float(__ldg(reinterpret_cast<const __half*>(st.bias) + colbase + my_col));
+      if (affine) {
+        gm = __ldg(reinterpret_cast<const __half*>(st.gamma) + colbase + my_col);
+        bt = __ldg(reinterpret_cast<const __half*>(st.beta) + colbase + my_col);
+      }
+    }
+    named_barrier_sync(1, kEpiThreads);                              // the tile before has been read
+    bias_s[my_col] = b;
+    gamma_s[my_col] = gm;
+    gamma_s[256 + my_col] = bt;
+    if (elect_one()) bulk_wait_group_read<0>();
+    named_barrier_sync(1, kEpiThreads);
+    if (item + item_step >= st.items) {                              // boxes inside the operand ring, see StoreBoxes
+      sb.base = boxes - kRingBytes + (warp - 2) * kRingBoxes * kStageWarp;
+      sb.box = 0;
+      sb.n = kRingBoxes;
+    }
+    const uint32_t acc0 = nh == 2 ? 0u : acc_bits >> 2;
+#pragma unroll 1
+    for (int h = 0; h < nh; ++h) {
+      const uint32_t acc = acc0 + (uint32_t)h, t0 = tmem + acc * kAccStride;
+      const int row0 = mt * st.bm + (kPair ? (int)rank : h) * 128 + q * 32;
+      ok = ok && mbar_wait_warp(tfull0 + 8 * acc, (acc_bits >> acc) & 1u, ctl, 400 + (int)acc, lane);
+      tc_fence_after_sync();
+      if (prof && item == first_item && h == 0 && warp == 2 && lane == 0)
+        p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 14] = clock64();
+      float mean = 0.0f, dev = 0.0f, sets = 0.0f;                    // of `sets` chunks of 32 columns
+#pragma unroll 1
+      for (int c = cpar; c < chunks; c += 2) {
+        uint32_t r[32];
+        tmem_ld32(t0 + c * 32, r);
+        tmem_ld_wait(r);
+        float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        const float4* b4 = reinterpret_cast<const float4*>(bias_s + c * 32);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float4 bb = b4[i];
+          const float z0 = __uint_as_float(r[4 * i]) + bb.x, z1 = __uint_as_float(r[4 * i + 1]) + bb.y;
+          const float z2 = __uint_as_float(r[4 * i + 2]) + bb.z, z3 = __uint_as_float(r[4 * i + 3]) + bb.w;
+          sum[0] += z0; sum[1] += z1; sum[2] += z2; sum[3] += z3;
+          r[4 * i] = __float_as_uint(z0); r[4 * i + 1] = __float_as_uint(z1);
+          r[4 * i + 2] = __float_as_uint(z2); r[4 * i + 3] = __float_as_uint(z3);
+        }
+        tmem_st32(t0 + c * 32, r);
+        const float cm = ((sum[0] + sum[1]) + (sum[2] + sum[3])) * (1.0f / 32.0f);
+        float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const float d = __uint_as_float(r[i]) - cm;
+          v[i & 3] = fmaf(d, d, v[i & 3]);
+        }
+        const float w = 1.0f / (sets + 1.0f), d = cm - mean;
+        dev += ((v[0] + v[1]) + (v[2] + v[3])) + d * d * (32.0f * sets * w);
+        mean = fmaf(d, w, mean);
+        sets += 1.0f;
+      }
+      tmem_st_wait();
+      if (chunks > 1) {
+        if (cpar == 1) other[h * 32 + lane] = make_float2(mean, dev);
+        named_barrier_sync(4 + q, 64);
+        if (cpar == 0) {
+          const float2 o = other[h * 32 + lane];
+          const float os = (float)(chunks >> 1), w = os / (sets + os), d = o.x - mean;
+          dev += o.y + d * d * (32.0f * sets * w);
+          mean = fmaf(d, w, mean);
+        }
+      }
+      if (cpar == 0 && ok)
+        st_relaxed_2x64(st.stats + ((size_t)(row0 >> 5) * tiles_n + nt) * 32 + lane, (uint64_t)__float_as_uint(mean) | ((uint64_t)tag << 32),
+                        (uint64_t)__float_as_uint(dev) | ((uint64_t)tag << 32));
+    }
+#pragma unroll 1
+    for (int h = 0; h < nh; ++h) {
+      const uint32_t acc = acc0 + (uint32_t)h, t0 = tmem + acc * kAccStride;
+      const int row0 = mt * st.bm + (kPair ? (int)rank : h) * 128 + q * 32;
+      float mean = 0.0f, dev = 0.0f;
+      const RowStat* from = st.stats + (size_t)(row0 >> 5) * tiles_n * 32 + lane;
+      uint32_t spins = 0;
+#pragma unroll 1
+      for (int s0 = 0; ok && s0 < tiles_n;) {
+        constexpr int kG = 4;                                        // tiles whose pairs are on their way at once
+        uint64_t a[kG], v[kG];
+        bool there = true;
+#pragma unroll
+        for (int i = 0; i < kG; ++i)
+          if (s0 + i < tiles_n) ld_relaxed_2x64(from + (s0 + i) * 32, a[i], v[i]);
+#pragma unroll
+        for (int i = 0; i < kG; ++i)
+          if (s0 + i < tiles_n) there = there && (uint32_t)(a[i] >> 32) == tag && (uint32_t)(v[i] >> 32) == tag;
+        if (!__all_sync(0xffffffffu, there)) {
+          if (((++spins) & 0x3F) == 0) {
+            int give_up = 0;
+            if (lane == 0) {
+              give_up = *ctl.abort_smem;
+              if (!give_up && globaltimer_ns() > ctl.deadline_ns + kWaitGraceNs) {
+                record_timeout(ctl, DEV_TIMEOUT_FLAG, 750);
+                give_up = 1;
+              }
+            }
+            if (__shfl_sync(0xffffffffu, give_up, 0)) ok = false;
+          }
+          continue;
+        }
+        // sets of bn columns each: those of this round among themselves, then with the rounds before
+        const int n = tiles_n - s0 < kG ? tiles_n - s0 : kG;
+        float m = 0.0f, e = 0.0f, sq = 0.0f;
+#pragma unroll
+        for (int i = 0; i < kG; ++i) m += i < n ? __uint_as_float((uint32_t)a[i]) : 0.0f;
+        m *= 1.0f / (float)n;
+#pragma unroll
+        for (int i = 0; i < kG; ++i)
+          if (i < n) {
+            const float d = __uint_as_float((uint32_t)a[i]) - m;
+            e += __uint_as_float((uint32_t)v[i]);
+            sq = fmaf(d, d, sq);
+          }
+        const float w = (float)n / (float)(s0 + n), d = m - mean;
+        dev += e + (float)bn * (sq + d * d * ((float)s0 * w));
+        mean = fmaf(d, w, mean);
+        s0 += kG;
+      }
+      const float rstd = rsqrtf(dev * inv_n + st.eps), nm = -mean * rstd;
+#pragma unroll 1
+      for (int c = cpar; ok && c < chunks; c += 2) {
+        uint32_t r[32], w[16];
+        tmem_ld32(t0 + c * 32, r);
+        tmem_ld_wait(r);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) w[i] = pack_h2(fmaf(__uint_as_float(r[2 * i]), rstd, nm), fmaf(__uint_as_float(r[2 * i + 1]), rstd, nm));
+        if (affine) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 ug = *(reinterpret_cast<const uint4*>(gamma_s + c * 32) + i), ub = *(reinterpret_cast<const uint4*>(gamma_s + 256 + c * 32) + i);
+            const uint32_t g4[4] = {ug.x, ug.y, ug.z, ug.w}, b4[4] = {ub.x, ub.y, ub.z, ub.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const __half2 y = __hfma2(*reinterpret_cast<const __half2*>(&w[4 * i + j]), *reinterpret_cast<const __half2*>(&g4[j]),
+                                        *reinterpret_cast<const __half2*>(&b4[j]));
+              w[4 * i + j] = *reinterpret_cast<const uint32_t*>(&y);
+            }
+          }
+        }
+        store_box(sb, w, lane, [&](uint32_t buf) {
+          if (row0 < M) tma_store_2d(tm_out, buf, colbase + c * 32, row0);
+        });
+      }
+      tc_fence_before_sync();
+      if constexpr (kPair) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster_relaxed(map_shared_rank(tempty0 + 8 * acc, 0));
+      } else {
+        mbar_arrive(tempty0 + 8 * acc);
+      }
+      acc_bits ^= 1u << acc;
+    }
+    if (nh == 1) acc_bits ^= 4u;
+  }
+  if (elect_one()) {                      // the stores are complete before the CTA reports the stage done
+    bulk_wait_group_all();
+    fence_proxy_async_global();
+  }
+  __syncwarp();
+  if (prof && warp == 2 && lane == 0) p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 15] = clock64();
+  return acc_bits;
+}
+
 // Tiles are bm x bn with bm = 128 (two accumulators used alternately, so the epilogue of one tile
 // overlaps the main loop of the next) or bm = 256 (two 128-row halves share every B tile, which
 // halves the B traffic per FLOP; each half has its own accumulator and hand-shake).
@@ -494,7 +714,7 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
 // shared memory -- half the B traffic per FLOP of the single-CTA form -- with every copy's completion counted on the
 // leader's full barrier; the leader's MMA lane issues for both and its commits arrive on the barriers of both CTAs;
 // each CTA's epilogue warps drain their own 128 rows and report to the leader's accumulator-free barrier.
-template <bool kSwin, bool kPair = false>
+template <bool kSwin, bool kPair = false, bool kLnEpi = false>
 __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
                            uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp_id, int lane) {
   const int warp = uniform_warp(warp_id);
@@ -524,9 +744,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       int mt, nt, ks;
       gemm_item(st, first_item, mt, nt, ks);
       int kk = first_chunk(first_item);
-      bool ok = grid_wait(p, ctl, st.position);
+      bool ok = grid_wait(p, ctl, st);
       const long long t_first = prof ? clock64() : 0;
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
       for (int item = first_item; ok && item < g.items;) {
         const int m0 = mt * g.bm + (int)rank * 128, kbase = ks * g.kchunks;
         for (int kc = 0; kc < g.kchunks; ++kc) {
@@ -547,6 +767,23 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           bits ^= 1u << s;
           s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
           kk = (kk + 1 == g.kchunks) ? 0 : kk + 1;
+        }
+        if constexpr (kLnEpi) {          // the tile's residual, one step of 64 columns per slot (see gemm_ln_epilogue)
+          const int steps = st.epi == EPI_LN ? (g.bn + 63) >> 6 : 0;
+          for (int i = 0; ok && i < steps; ++i) {
+            if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 120 + (int)s)) { ok = false; break; }
+            const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes;
+            const CUtensorMap* tmR = map_ptr(ca, st.tm_resid);
+            if constexpr (kPair) {
+              if (rank == 0) mbar_expect_tx(fb, 2u * a_bytes);
+              tma_load_2d_pair(dst, tmR, map_shared_rank(fb, 0), nt * g.bn + i * 64, m0);
+            } else {
+              mbar_expect_tx(fb, a_bytes);
+              tma_load_2d(dst, tmR, fb, nt * g.bn + i * 64, m0);
+            }
+            bits ^= 1u << s;
+            s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
+          }
         }
         item += item_step;
         gemm_item(st, item, mt, nt, ks);
@@ -569,7 +806,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       uint32_t s = rs.slot, bits = rs.slot_bits;
       const bool b_mn = st.b_mn_major != 0;
       const uint32_t b_bytes = sub_bytes - a_bytes;
-      bool ok = wait_arrived(ctl_s, st.position, ctl);
+      bool ok = wait_arrived(ctl_s, st.ordinal, ctl);
       for (int item = first_item; ok && item < g.items; item += item_step) {
         int mt, nt, ks;
         gemm_item(st, item, mt, nt, ks);
@@ -596,6 +833,24 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           bits ^= 1u << s;
           s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
           kk = (kk + 1 == g.kchunks) ? 0 : kk + 1;
+        }
+        if constexpr (kLnEpi) {          // unit matrices for the residual
+          const int steps = st.epi == EPI_LN ? (g.bn + 63) >> 6 : 0;
+          for (int i = 0; ok && i < steps; ++i) {
+            if (!mbar_wait_hot(empty0 + 8 * s, ((bits >> s) & 1u) ^ 1u, ctl, 130 + (int)s)) { ok = false; break; }
+            const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes + a_bytes;
+            const CUtensorMap* tmU = map_ptr(ca, st.tm_unit);
+            if constexpr (kPair) {
+              if (rank == 0) mbar_expect_tx(fb, 2u * kUnitBytes / 2u);
+              const int n = g.bn - 64 * i < 64 ? g.bn - 64 * i : 64;      // the pair MMA's columns: each CTA has half of them
+              tma_load_2d_pair(dst, tmU, map_shared_rank(fb, 0), 0, (int)rank * (n >> 1));
+            } else {
+              mbar_expect_tx(fb, kUnitBytes);
+              tma_load_2d(dst, tmU, fb, 0, 0);
+            }
+            bits ^= 1u << s;
+            s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
+          }
         }
       }
       rs.slot = s;
@@ -653,6 +908,25 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           bits ^= 1u << s;
           s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
         }
+        if constexpr (kLnEpi) {          // + residual x unit matrix, 64 columns at a time
+          const int steps = st.epi == EPI_LN ? (g.bn + 63) >> 6 : 0;
+          for (int i = 0; ok && i < steps; ++i) {
+            const uint32_t n = g.bn - 64 * i < 64 ? (uint32_t)(g.bn - 64 * i) : 64u;
+            if (!mbar_wait_hot(full0 + 8 * s, (bits >> s) & 1u, ctl, 310 + (int)s)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t a_lo = a_lo0 + s * slot16, b_lo = b_lo0 + s * slot16, d = d0 + 64u * (uint32_t)i;
+            if constexpr (kPair) {
+              umma_f16_k64_pair(d, a_lo, b_lo, 2u, umma_idesc_f16_pair(n, 0u), 1u);
+              umma_commit_pair(empty0 + 8 * s);
+            } else {
+              if (g.nh == 2) umma_f16_k64_x2(d, d + kAccStride, a_lo, b_lo, 2u, umma_idesc_f16(n, 0u), 1u);
+              else umma_f16_k64(d, a_lo, b_lo, 2u, umma_idesc_f16(n, 0u), 1u);
+              umma_commit(empty0 + 8 * s);
+            }
+            bits ^= 1u << s;
+            s = (s + 1 == (uint32_t)g.nslots) ? 0 : s + 1;
+          }
+        }
         if (!ok) break;
         for (int h = 0; h < g.nh; ++h) {
           const uint32_t acc = acc0 + (uint32_t)h;
@@ -680,6 +954,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     const int q = warp & 3, cpar = (warp - 2) >> 2;
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const int full_chunks = g.bn >> 5;
+    if (kLnEpi && st.epi == EPI_LN) {
+      rs.acc_bits = gemm_ln_epilogue<kPair>(ca, rs.acc_bits | (uint32_t)(&st == &ctl_s.stage[1]) << 31);
+    } else {
     EpiCtx e;
     e.epi = st.epi; e.act = st.act; e.M = st.M; e.N = st.N; e.ldo = st.ldo;
     e.resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
@@ -831,6 +1108,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     __syncwarp();
     if (prof && warp == 2 && lane == 0)
       p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 15] = clock64();
+    }
   }
 }
 
@@ -927,8 +1205,8 @@ __device__ __forceinline__ void attn_stage(const Stage& st, const CallArgs& ca, 
       const CUtensorMap* tmq = map_ptr(ca, st.tm_a);
       uint32_t bit = rs.attn_bit;
       int qt = (int)blockIdx.x % n_qt, bh = (int)blockIdx.x / n_qt;          // in front of the wait: divisions
-      const bool ok = grid_wait(p, ctl, st.position);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
+      const bool ok = grid_wait(p, ctl, st);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
       for (int item = blockIdx.x; ok && item < items;) {
         const int rq = bh * S, rk = (B * H + bh) * S, rv = (2 * B * H + bh) * S;
         if (!mbar_wait_hot(qk_empty, bit ^ 1u, ctl, 500)) break;
@@ -1177,8 +1455,8 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
   if (warp == 0) {
     if (elect_one()) {
       uint32_t bits = rs.attn_bit | (rs.attn_bit1 << 1);
-      const bool ok = grid_wait(p, ctl, st.position);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
+      const bool ok = grid_wait(p, ctl, st);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
       for (int k = 0; ok && k < my_items; ++k) {
         const int item = item_of(k), g = k & 1;
         const int h = item % H, b = item / H;
@@ -1523,8 +1801,8 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
   // TMEM: scores of (head g, window j) at column 64 (2 g + j), outputs 256 further on
   if (warp == 0) {
     if (lane == 0) {
-      const bool ok = grid_wait(ca.p, ctl, st.position);
-      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.position);
+      const bool ok = grid_wait(ca.p, ctl, st);
+      if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
       for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
         const int wp = item / item_h, w0 = wp * (int)n, col = ((item - wp * item_h) * (int)n >> 1) * 64;
         if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 530)) break;
@@ -1822,7 +2100,7 @@ __device__ __forceinline__ void ln_shared_rows(const Stage& st, const MegaParams
   const bool affine = st.gamma != nullptr;
   const float inv_n = 1.0f / (float)N;
   red += grp * W;
-  if (!stage_go(p, cs, st.position, ctl, warp, lane)) return;
+  if (!stage_go(p, cs, st, ctl, warp, lane)) return;
   auto load_planes = [&](int r, int g0) {
     const float* src = planes + (size_t)r * N + (size_t)g0 * plane;
 #pragma unroll
@@ -2035,7 +2313,7 @@ __device__ __forceinline__ void ln_lone_rows(const Stage& st, const MegaParams& 
   const __half* bias = reinterpret_cast<const __half*>(st.bias);
   const __half* gamma = reinterpret_cast<const __half*>(st.gamma);
   const __half* beta = reinterpret_cast<const __half*>(st.beta);
-  if (!stage_go(p, cs, st.position, ctl, warp, lane)) return;
+  if (!stage_go(p, cs, st, ctl, warp, lane)) return;
   if (st.dead_bytes[0]) drop_dead_buffers(st, 0, kThreads);
   for (int row = warp * (int)gridDim.x + (int)blockIdx.x; row < M; row += (int)gridDim.x * (kThreads / 32)) {
     const float* pl0 = st.partial + (size_t)row * N;
@@ -2096,7 +2374,7 @@ __device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams&
 
   if (warp == 0) {
     if (lane == 0) {
-      const bool go = grid_wait(p, ctl, st.position);
+      const bool go = grid_wait(p, ctl, st);
       int buf = 0;
       for (int k = 0; go && k < my_batches; ++k) {
         const int batch = blockIdx.x + k * gridDim.x;
@@ -2198,7 +2476,6 @@ template <int kFamily>
 __global__ void __launch_bounds__(kThreads, 1)
 souffle_megakernel(const __grid_constant__ CallArgs ca) {
   const MegaParams& p = ca.p;
-  extern __shared__ __align__(1024) uint8_t smem_raw[];      // swizzled tiles need 1024-byte alignment
   if (p.prof && threadIdx.x == 0) {
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[0] = clock64();
@@ -2234,6 +2511,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     cs.abort = 0;
     cs.leave[0] = cs.leave[1] = 0;
     cs.go = cs.arrived = 0u;
+    cs.epoch = p.epoch ? *p.epoch : 0u;
     cs.wait.abort_smem = &cs.abort;
     cs.wait.status_g = p.status;
     cs.wait.deadline_ns = globaltimer_ns() + p.timeout_ns;      // read once per CTA
@@ -2263,7 +2541,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   }
 
   uint32_t state = RoleState().pack();
-  for (int si = 0; si < p.n_stages; ++si) {
+  for (int si = 0, ord = 0, next; si < p.n_stages; si = next, ++ord) {
     // Addresses and the warp's role are worked out anew for every stage, the roles' state is packed between them: the compiler would
     // keep what follows from them in registers over all stages, and the stages that need most of them would spill.
     {
@@ -2276,12 +2554,13 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       uint8_t* stage_s = ring_ptr + kRingBytes + kVecBytes;
       const uint32_t ring = smem_u32(smem_raw) + off + kCtlBytes;
       const int warp = (int)(tid >> 5), lane = (int)(tid & 31u);
-      const Stage& st = cs.stage[si & 1];
+      const Stage& st = cs.stage[ord & 1];
+      next = st.next;
       // The spare warps' part, in front of anything that waits: the next stage's record (constant since the launch: plan-owned
       // programs lie in global memory, the stages of the plan-less entry points in the launch parameters) goes to shared
       // memory, and this CTA's slice of the next stage's weights to L2 (they come from HBM when the program's weights exceed
       // L2; without this every GEMM stage starts with all CTAs waiting on the same DRAM rows).
-      if (warp == kWeightWarp && si + 1 < p.n_stages) copy_record(&cs.stage[(si + 1) & 1], p.stages ? p.stages + si + 1 : &ca.inline_stages[si + 1], lane);
+      if (warp == kWeightWarp && next < p.n_stages) copy_record(&cs.stage[(ord + 1) & 1], p.stages ? p.stages + next : &ca.inline_stages[next], lane);
       if (warp == kSpareWarp && lane == 0) {
         const uint32_t pf_bytes = st.pf_bytes;
         if (pf_bytes) {
@@ -2292,7 +2571,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       }
       __syncwarp();
       if (st.type != STAGE_LN && warp == kSpareWarp && st.dead_bytes[0]) {
-        if (wait_go(cs, si, ctl)) drop_dead_buffers(st, warp * 32, 32);
+        if (wait_go(cs, ord, ctl)) drop_dead_buffers(st, warp * 32, 32);
       }
       if constexpr (kFamily == kFamilySwin) {
         if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
@@ -2302,7 +2581,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       } else {
         if (st.type == STAGE_GEMM) {
           RoleState rs = RoleState::unpack(state);
-          gemm_stage<false, kFamily == kFamilyBertPair>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
+          gemm_stage<false, kFamily == kFamilyBertPair, kFamily != kFamilyBertCoop>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
           state = rs.pack();
         } else if (st.type == STAGE_ATTN) {
           RoleState rs = RoleState::unpack(state);
@@ -2322,15 +2601,15 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw + off);
     const WaitCtl& ctl = cs.wait;
     fence_proxy_async_smem();             // this thread's accesses to shared memory before the next stage's copies into it
-    if (*ctl.abort_smem) cs.leave[si & 1] = 1;       // two words in turn: the next stage's is not written before all have read this one
+    if (*ctl.abort_smem) cs.leave[ord & 1] = 1;       // two words in turn: the next stage's is not written before all have read this one
     __syncthreads();
-    if (*const_cast<volatile int*>(&cs.leave[si & 1])) break;
+    if (*const_cast<volatile int*>(&cs.leave[ord & 1])) break;
     if (tid == kSpareWarp * 32) {
       if (p.prof) p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 1] = clock_now();
-      if (si + 1 < p.n_stages) {
+      if (next < p.n_stages) {
         if (p.skip_arrival > 0 && si == p.skip_arrival >> 16 && (int)blockIdx.x == (p.skip_arrival & 0xFFFF) - 1) *ctl.abort_smem = 1;      // test hook
         else red_add_release_u32(p.sync, 1u);
-        st_release_cta_shared_u32(smem_u32(&cs.arrived), (uint32_t)si + 1u);
+        st_release_cta_shared_u32(smem_u32(&cs.arrived), (uint32_t)ord + 1u);
       } else if (p.prof) {
         p.prof[((size_t)si * gridDim.x + blockIdx.x) * kProfSlots + 2] = clock_now();
       }
@@ -2338,6 +2617,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   }
 
   __syncthreads();
+  if (p.epoch && blockIdx.x == 0 && threadIdx.x == 0) *p.epoch = cs.epoch + 1u;      // every CTA has read it: all have been in a grid barrier
   if (p.prof && threadIdx.x == 0) {
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[2] = clock64();

@@ -358,7 +358,12 @@ static int device_info(DeviceInfo** out) {
 // `family` selects the build of the kernel (see souffle_megakernel).
 static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, int family = kFamilyBert) {
   CallArgs args = args_in;
-  for (int i = 0; i < 3; ++i) args.inline_stages[i].position = i;      // stages that travel in the launch parameters
+  for (int i = 0; i < 3; ++i) {      // stages that travel in the launch parameters
+    Stage& s = args.inline_stages[i];
+    s.position = s.ordinal = (uint8_t)i;
+    s.prev = (uint8_t)(i > 0 ? i - 1 : 0);
+    s.next = (uint8_t)(i + 1);
+  }
   void* kargs[] = {&args};
   if (family == kFamilyBertPair) {
     // Clusters of two CTAs.  All CTAs must be resident at once (the grid barrier): the grid never exceeds what
@@ -541,6 +546,7 @@ static int is_captured(cudaStream_t st, bool* captured) {
 
 // words: the pairs of alternate launches (0-3), a captured launch's pair (4, 5) and the pair it clears for nobody (6, 7).
 constexpr int kCapturedPair = 4;
+constexpr int kEpochWord = 8;          // behind them, in a plan: MegaParams::epoch
 static int pick_barrier_words(unsigned* words, unsigned launches, bool captured, cudaStream_t st, MegaParams* mp) {
   if (captured && mp->n_stages > 1) SF_CUDA(cudaMemsetAsync(words + kCapturedPair, 0, 2 * sizeof(unsigned), st));
   const unsigned at = captured ? kCapturedPair : 2u * (launches & 1u);
@@ -604,6 +610,8 @@ struct SouffleBertPlan {
   const void* last_x = nullptr;
   CUtensorMap x_map;
   int x_box_rows = 128;
+  int x_res_rows = 0;            // rows of the boxes in which the first layer's input is read as a residual, or 0
+  bool y_map = false;            // the last stage stores the output through a tensor map of the call's
 };
 
 namespace souffle {
@@ -613,15 +621,23 @@ static int plan_alloc(SouffleBertPlan* p, void** ptr, size_t bytes);
 // Numbers the stages and copies the program and its tensor maps to the device.
 static int upload_program(SouffleBertPlan* p) {
   int rc;
-  for (size_t i = 0; i < p->stages.size(); ++i) {
+  const size_t n = p->stages.size();
+  auto next_of = [&](size_t i) { do ++i; while (i < n && p->stages[i].fused); return i; };
+  for (size_t i = 0, prev = 0, ordinal = 0; i < n; prev = i, i = next_of(i), ++ordinal) {
+    p->stages[i].prev = (uint8_t)prev;
+    p->stages[i].ordinal = (uint8_t)ordinal;
+  }
+  for (size_t i = 0; i < n; ++i) {
     Stage& s = p->stages[i];
-    s.position = (int)i;
+    s.position = (uint8_t)i;
+    const size_t next = next_of(i);
+    s.next = (uint8_t)next;
     // the weights of the GEMM stage that comes next are prefetched into L2 while this stage runs
     s.pf_ptr = nullptr;
     s.pf_bytes = 0;
-    if (i + 1 < p->stages.size() && p->stages[i + 1].type == STAGE_GEMM && p->stage_weights.size() > i + 1 && p->stage_weights[i + 1]) {
-      const Stage& g = p->stages[i + 1];
-      s.pf_ptr = p->stage_weights[i + 1];
+    if (next < n && p->stages[next].type == STAGE_GEMM && p->stage_weights.size() > next && p->stage_weights[next]) {
+      const Stage& g = p->stages[next];
+      s.pf_ptr = p->stage_weights[next];
       s.pf_bytes = (uint32_t)((size_t)g.N * g.K * 2) & ~15u;
     }
     s.dead_bytes[0] = s.dead_bytes[1] = 0;
@@ -636,8 +652,9 @@ static int upload_program(SouffleBertPlan* p) {
   if ((rc = device_info(&di))) return rc;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {
     if (p->layer_bytes <= (size_t)di->l2_bytes / 2) break;
-    if (dd.after_stage + 1 >= p->stages.size()) continue;          // nothing runs after it inside the launch
-    Stage& nx = p->stages[dd.after_stage + 1];
+    const size_t next = next_of(dd.after_stage);
+    if (next >= n) continue;                                       // nothing runs after it inside the launch
+    Stage& nx = p->stages[next];
     const int k = nx.dead_bytes[0] ? 1 : 0;
     if (nx.dead_bytes[k]) continue;                                // both slots taken: the buffer is written back as before
     nx.dead_ptr[k] = dd.ptr;
@@ -920,9 +937,24 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   const int bn_qkv = t_qkv.bn, bn_fc1 = t_fc1.bn, bn_proj = t_proj.bn, sp_proj = t_proj.split, bn_fc2 = t_fc2.bn,
             sp_fc2 = t_fc2.split;
   const int max_split = sp_proj > sp_fc2 ? sp_proj : sp_fc2;
-  if ((rc = plan_alloc(p, (void**)&p->partial, (size_t)max_split * M * H * 4))) return rc;
+  // LayerNorm in the product's epilogue (see gemm_ln_epilogue) where the product is not cut along K, from 2048 rows on: below, products
+  // that are not cut have more tiles per row and shorter LayerNorm stages (twelve layers of 128 tokens, as planes / in the epilogue:
+  // 13 sequences 676 / 675 us, 16 732 / 660, 32 1044 / 946, 64 1795 / 1550; six layers of 30 x 80 at hidden 512 310 / 276).  The
+  // build for few attention items does not have it: it would spill.
+  auto can_fuse = [&](const TileChoice& t) {
+    return M >= 2048 && p->family != kFamilyBertCoop && t.split == 1 && t.bn % 32 == 0 && t.bn >= 64 && H / t.bn <= (pair ? npairs : sms);
+  };
+  const bool fuse_proj = can_fuse(t_proj), fuse_fc2 = can_fuse(t_fc2);
+  RowStat* stats[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2; ++i)
+    if (i ? fuse_fc2 : fuse_proj) {
+      const size_t bytes = (size_t)((M + 255) / 256) * 256 * (H / (i ? bn_fc2 : bn_proj)) * sizeof(RowStat);
+      if ((rc = plan_alloc(p, (void**)&stats[i], bytes))) return rc;
+      SF_CUDA(cudaMemset(stats[i], 0xff, bytes));
+    }
+  if ((!fuse_proj || !fuse_fc2) && (rc = plan_alloc(p, (void**)&p->partial, (size_t)max_split * M * H * 4))) return rc;
   // Q, K, V, attention output, LayerNorm 1 output, FFN hidden layer and both products' planes
-  p->layer_bytes = (size_t)M * (5 * (size_t)H + F) * 2 + (size_t)(sp_proj + sp_fc2) * M * H * 4;
+  p->layer_bytes = (size_t)M * (5 * (size_t)H + F) * 2 + (size_t)((fuse_proj ? 0 : sp_proj) + (fuse_fc2 ? 0 : sp_fc2)) * M * H * 4;
   // rows of an A box: the tile's height, or one CTA's 128-row half of a pair's tile; rows of a B box: the tile's
   // width, or one CTA's half of it
   auto a_rows = [pair](const TileChoice& t) { return (uint32_t)(pair ? 128 : t.bm); };
@@ -943,6 +975,45 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     while (q_rows > 32 && B * Hh * ((S + q_rows / 2 - 1) / (q_rows / 2)) <= sms) q_rows /= 2;
   m_q = m_qkv;
   if (q_rows < 128 && (rc = add_map(p, p->qkv, (uint64_t)3 * B * Hh * S, hd, (uint32_t)q_rows, &m_q))) return rc;
+
+  // what a product with LayerNorm in its epilogue reads besides its operands: a unit matrix and the residuals (the layer's input and
+  // LayerNorm 1's output) in boxes as high as its own tiles
+  int m_unit = 0, m_res_act[2] = {-1, -1}, m_res_ln1 = -1;
+  if (fuse_proj || fuse_fc2) {
+    __half* unit = nullptr;
+    std::vector<uint16_t> host(64 * 64, 0);
+    for (int i = 0; i < 64; ++i) host[65 * i] = 0x3C00;
+    if ((rc = plan_alloc(p, (void**)&unit, kUnitBytes))) return rc;
+    SF_CUDA(cudaMemcpy(unit, host.data(), kUnitBytes, cudaMemcpyHostToDevice));
+    if ((rc = add_map(p, unit, 64, 64, pair ? 32 : 64, &m_unit))) return rc;
+    for (int i = 0; i < 2; ++i)
+      if (fuse_proj && p->act[i] && (rc = add_map(p, p->act[i], M, H, a_rows(t_proj), &m_res_act[i]))) return rc;
+    if (fuse_fc2 && (rc = add_map(p, p->ln1, M, H, a_rows(t_fc2), &m_res_ln1))) return rc;
+    if (fuse_proj) p->x_res_rows = (int)a_rows(t_proj);
+  }
+  // A product and the LayerNorm of its sum with bias and residual: as fp32 planes that the LayerNorm stage adds up, or in the
+  // product's epilogue.
+  auto add_product_and_ln = [&](Stage s, Stage ln, bool fuse, RowStat* row_stats, int resid_map, const void* w) -> int {
+    if (fuse) {
+      s.epi = EPI_LN; s.stats = row_stats; s.ldo = ln.ldo; s.bias = ln.bias; s.tm_resid = resid_map; s.tm_unit = m_unit;
+      s.out = ln.out; s.out_sel = ln.out_sel; s.gamma = ln.gamma; s.beta = ln.beta; s.eps = ln.eps;
+      ln.fused = 1;
+      if (s.out_sel == PTR_CALL_Y) {
+        s.out_stores = 1;
+        s.tm_out = -2;
+        p->y_map = true;
+      } else if (const int r = add_f16_out_map(p, s)) {
+        return r;
+      }
+    } else {
+      s.epi = EPI_PARTIAL; s.partial = p->partial;
+      if (const int r = add_plane_map(p, s)) return r;
+    }
+    p->stages.push_back(s);
+    note_weights(p, w);
+    p->stages.push_back(ln);
+    return SOUFFLE_OK;
+  };
 
   // ---- per layer: repack weights, maps, stages ----
   for (int l = 0; l < L; ++l) {
@@ -1016,17 +1087,12 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
 
     s = blank_stage(STAGE_GEMM);                       // output projection -> fp32 partials
     s.tm_a = m_ctx; s.tm_b = m_wo; s.M = M; s.N = H; s.K = H; s.bm = t_proj.bm; s.bn = bn_proj; s.splitk = sp_proj;
-    s.epi = EPI_PARTIAL; s.partial = p->partial;
-    if ((rc = add_plane_map(p, s))) return rc;
-    p->stages.push_back(s);
-    note_weights(p, wo_t);
-    if (!keep) note_dead(p, p->ctx, (size_t)M * H * 2);               // attention output: read by the projection only
-
-    s = blank_stage(STAGE_LN);                         // + bias + residual, LayerNorm 1
-    s.M = M; s.N = H; s.ldo = H; s.partial = p->partial; s.n_partial = sp_proj; s.bias = proj_b;
-    s.resid = in_ptr; s.resid_sel = in_sel; s.out = p->ln1; s.gamma = ln1_g; s.beta = ln1_b; s.eps = d.eps;
-    p->stages.push_back(s);
-    note_dead(p, p->partial, (size_t)sp_proj * M * H * 4);             // the projection's planes
+    Stage ln = blank_stage(STAGE_LN);                  // + bias + residual, LayerNorm 1
+    ln.M = M; ln.N = H; ln.ldo = H; ln.partial = p->partial; ln.n_partial = (uint8_t)sp_proj; ln.bias = proj_b;
+    ln.resid = in_ptr; ln.resid_sel = in_sel; ln.out = p->ln1; ln.gamma = ln1_g; ln.beta = ln1_b; ln.eps = d.eps;
+    if ((rc = add_product_and_ln(s, ln, fuse_proj, stats[0], first ? -3 : m_res_act[(l - 1) & 1], wo_t))) return rc;
+    if (!keep) p->dead_after.push_back({p->stages.size() - 2, p->ctx, (uint32_t)((size_t)M * H * 2)});      // attention output: read by the projection only
+    if (!fuse_proj) note_dead(p, p->partial, (size_t)sp_proj * M * H * 4);             // the projection's planes
     if (!first) note_dead(p, in_ptr, (size_t)M * H * 2);               // the previous layer's output: QKV and this residual were its readers
 
     s = blank_stage(STAGE_GEMM);                       // FC1 + bias + activation
@@ -1038,19 +1104,14 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
 
     s = blank_stage(STAGE_GEMM);                       // FC2 -> fp32 partials
     s.tm_a = m_fc1; s.tm_b = m_w2; s.M = M; s.N = H; s.K = F; s.bm = t_fc2.bm; s.bn = bn_fc2; s.splitk = sp_fc2;
-    s.epi = EPI_PARTIAL; s.partial = p->partial;
-    if ((rc = add_plane_map(p, s))) return rc;
-    p->stages.push_back(s);
-    note_weights(p, w2_t);
-    if (!keep) note_dead(p, p->fc1, (size_t)M * F * 2);               // FFN hidden layer: read by FC2 only
-
-    s = blank_stage(STAGE_LN);                         // + bias + residual, LayerNorm 2
-    s.M = M; s.N = H; s.ldo = H; s.partial = p->partial; s.n_partial = sp_fc2; s.bias = fc2_b;
-    s.resid = p->ln1; s.resid_sel = PTR_PLAN; s.out = out_ptr; s.out_sel = out_sel;
-    s.gamma = ln2_g; s.beta = ln2_b; s.eps = d.eps;
-    p->stages.push_back(s);
+    ln = blank_stage(STAGE_LN);                        // + bias + residual, LayerNorm 2
+    ln.M = M; ln.N = H; ln.ldo = H; ln.partial = p->partial; ln.n_partial = (uint8_t)sp_fc2; ln.bias = fc2_b;
+    ln.resid = p->ln1; ln.resid_sel = PTR_PLAN; ln.out = out_ptr; ln.out_sel = out_sel;
+    ln.gamma = ln2_g; ln.beta = ln2_b; ln.eps = d.eps;
+    if ((rc = add_product_and_ln(s, ln, fuse_fc2, stats[1], m_res_ln1, w2_t))) return rc;
+    if (!keep) p->dead_after.push_back({p->stages.size() - 2, p->fc1, (uint32_t)((size_t)M * F * 2)});      // FFN hidden layer: read by FC2 only
     if (!last) {
-      note_dead(p, p->partial, (size_t)sp_fc2 * M * H * 4);            // FC2's planes
+      if (!fuse_fc2) note_dead(p, p->partial, (size_t)sp_fc2 * M * H * 4);            // FC2's planes
       note_dead(p, p->ln1, (size_t)M * H * 2);                         // LayerNorm 1 output: FC1 and this residual were its readers
     }
   }
@@ -1058,6 +1119,7 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
 
   int max_items = 1;
   for (const Stage& s : p->stages) {
+    if (s.fused) continue;
     const int it = stage_items(s, pair) * ((pair && s.type != STAGE_LN) ? 2 : 1);      // CTAs that have work
     if (it > max_items) max_items = it;
   }
@@ -1159,6 +1221,9 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
   mp.prof = plan->d_prof;
+  mp.epoch = plan->d_sync + kEpochWord;
+  if (plan->x_res_rows && (rc = make_map(&args.call_maps[2], x, M, H, (uint32_t)plan->x_res_rows))) return rc;
+  if (plan->y_map && (rc = make_store_map(&args.call_maps[1], y, M, H))) return rc;
   mp.skip_arrival = d.debug_skip_arrival;
   mp.max_slots = d.debug_max_slots;
   rc = launch_mega(args, plan->grid, reinterpret_cast<cudaStream_t>(stream), plan->family);
@@ -1292,7 +1357,7 @@ int souffle_bert_plan_status(SouffleBertPlan* plan) {
   if (h[0] != DEV_OK) {
     // leave the plan usable: clear the status and both barrier pairs
     cudaMemset(plan->d_status, 0, 64);
-    cudaMemset(plan->d_sync, 0, 64);
+    cudaMemset(plan->d_sync, 0, kEpochWord * sizeof(unsigned));        // the epoch goes on: tags of the launch that failed may lie in the plan's memory
   }
   return decode_status(h, "souffle_bert_forward");
 }
@@ -1350,7 +1415,7 @@ int souffle_bert_plan_stage_info(SouffleBertPlan* plan, int index, int out[6]) {
   if (!plan || !out) return fail(SOUFFLE_BAD_ARGUMENT, "null argument");
   if (index < 0 || index >= (int)plan->stages.size()) return fail(SOUFFLE_BAD_ARGUMENT, "stage index %d out of range", index);
   const Stage& s = plan->stages[index];
-  out[0] = s.type; out[1] = s.bm; out[2] = s.bn; out[3] = s.splitk; out[4] = stage_items(s, plan->pair);
+  out[0] = s.type; out[1] = s.bm; out[2] = s.bn; out[3] = s.splitk; out[4] = s.fused ? 0 : stage_items(s, plan->pair);
   out[5] = s.type == STAGE_GEMM ? s.nslots * s.kper : 0;      // slots of one K step of 64
   return SOUFFLE_OK;
 }

@@ -23,12 +23,22 @@ enum EpilogueKind : int {
   EPI_PARTIAL = 2,  // raw fp32 accumulators to partial[split][row][col]
   EPI_SWIN_QKV = 3, // rows (tokens) are rolled by -shift and scattered window-major: [3][windows][64][C]
   EPI_SWIN_PROJ = 4,// rows arrive window-major, are rolled back to token order; + bias + residual[token]
+  EPI_LN = 5,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it
 };
 
 enum Activation : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2 };
 
 // Pointer selectors: a stage either carries a plan-owned pointer or names a per-call argument.
 enum PtrSel : int { PTR_PLAN = 0, PTR_CALL_X = 1, PTR_CALL_Y = 2 };
+
+// Mean and sum of squared deviations of a row's columns in one tile, each beside a tag that tells when it was written: a word of
+// 64 bits is written as a whole, so a reader that finds the tag has the value.
+struct alignas(16) RowStat {
+  float mean;
+  uint32_t tag0;
+  float dev;
+  uint32_t tag1;
+};
 
 struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 bytes at a time
   int type;
@@ -52,12 +62,18 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   const void* bias;  // fp16 [N] or null
   const void* resid; // fp16 [M][ldo] or null
   void* out;         // fp16 output
-  float* partial;    // fp32 [splitk][M][N] (EPI_PARTIAL and STAGE_LN)
+  union {
+    float* partial;  // fp32 [splitk][M][N] (EPI_PARTIAL and STAGE_LN)
+    RowStat* stats;  // EPI_LN: [blocks of 32 rows][tiles_n][32]
+  };
   // ---- attention / head split ----
   int batch, heads, seq, head_dim;
   float scale;       // softmax scale applied to Q.K
   int tm_qkv;        // tensor map over the head-split buffer viewed as [3*B*heads*S][d], box 64 x 128
-  int win, shift;    // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
+  union {
+    struct { int win, shift; };        // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
+    struct { int tm_resid, tm_unit; }; // EPI_LN: tensor maps of the residual ([M][N], box 64 x bm) and of the unit matrix ([64][64])
+  };
   const void* rel_bias;  // Swin: fp16 [(2*win-1)^2][heads] relative-position bias table
   void* probs;       // optional fp16 [B*heads][S][S] normalised probabilities (debug / parity output)
   // ---- layer norm ----
@@ -65,8 +81,13 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   const void* beta;  // fp16 [N] or null
   float eps;         // < 0: no normalisation, the sum goes to `out`
   void* sum_out;     // fp16 [M][N] or null: the sum (rounded to fp16, which is then what gets normalised) is stored here as well
-  int n_partial;     // number of fp32 partial planes to sum
-  int position;      // of this stage in the program, set by the host: the grid barrier counts arrivals against it
+  uint8_t n_partial; // number of fp32 partial planes to sum
+  // ---- order, set by the host.  A LayerNorm stage that the GEMM stage in front of it does in its epilogue keeps its place in the
+  //      program, but nothing runs there ----
+  uint8_t fused;     // STAGE_LN: done by the stage before
+  uint8_t position;  // of this stage in the program
+  uint8_t prev, next;// positions of the stages that run before and after it (the number of stages: none)
+  uint8_t ordinal;   // stages that run before it: the grid barrier counts arrivals against it
   // ---- weight prefetch: the B matrix of the next stage, a GEMM, pulled into L2 by all CTAs at the start of this one
   //      (weights never depend on an earlier stage) ----
   uint32_t pf_bytes;
@@ -90,7 +111,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
 inline uint32_t fast_div_magic(uint32_t d) { return d <= 1 ? 0u : (uint32_t)((0x100000000ull + d - 1) / d); }
 
 constexpr int kMaxTensorMaps = 96;
-constexpr int kMaxStages = 160;
+constexpr int kMaxStages = 160;   // positions fit a byte
 constexpr int kProfSlots = 16;   // int64 words per (stage, CTA) record of the in-kernel profile
 
 }  // namespace souffle

@@ -222,6 +222,53 @@ def test_autotuned_plan_matches_the_oracle():
     assert (fixed.stage_info(4)["bm"], fixed.stage_info(4)["bn"]) == (128, 64)
 
 
+LN_TILES = lambda bm1, bn1, bm2, bn2, **kw: dict(bm_proj=bm1, bn_proj=bn1, split_proj=1, bm_fc2=bm2, bn_fc2=bn2, split_fc2=1, **kw)
+
+
+@pytest.mark.parametrize("B,S,heads,ffn,tuning", [
+    (20, 112, 16, 256, {}),                                     # 2240 rows: the last tile of rows is ragged
+    (16, 128, 12, 128, LN_TILES(256, 192, 128, 64)),            # two halves per CTA; twelve tiles per row, one 64-column residual step
+    (17, 128, 12, 128, LN_TILES(128, 256, 256, 96)),            # eight tiles per row (two rounds of four), a residual step of 32 columns
+    (64, 48, 4, 64, LN_TILES(128, 64, 128, 256)),               # several tiles per CTA; one tile per row
+    (64, 128, 12, 64, LN_TILES(128, 64, 128, 128)),             # 768 tiles on 148 CTAs: rows whose tiles are in different turns
+    (17, 128, 12, 128, LN_TILES(256, 192, 256, 64, pair_mma=1)),
+    (64, 80, 12, 128, LN_TILES(256, 96, 256, 256, pair_mma=1)),
+])
+def test_layernorm_in_the_epilogue(B, S, heads, ffn, tuning):
+    """Products that are not cut along K normalise their rows themselves, with statistics from all tiles of a row."""
+    cfg = so.BertConfig(B, S, heads, 64, ffn, "std")
+    enc, layers, x, lens, y = _run(cfg, 1260, n_layers=2, ragged=True, zero_bias=False, tuning=tuning)
+    if tuning:
+        assert enc.stage_info(2)["items"] > 0 and enc.stage_info(3)["items"] == 0 and enc.stage_info(6)["items"] == 0
+    assert _err(y, so.bert_stack(cfg, x, layers, lens)) < TOL_STACK_FP32
+    xs, ls = x.cuda(), lens.cuda()
+    first, out = enc.forward(xs, ls).clone(), torch.empty_like(xs)
+    graph = torch.cuda.CUDAGraph()                  # a captured launch runs as often as its graph, with calls in between
+    with torch.cuda.graph(graph):
+        enc.forward(xs, ls, out)
+    for _ in range(3):
+        out.zero_()
+        graph.replay()
+        assert torch.equal(out, first)
+        assert torch.equal(enc.forward(xs, ls), first)
+    enc.status()
+
+
+@pytest.mark.parametrize("stage", [0, 1, 2, 4])      # in front of attention, proj with LayerNorm 1, FC1, FC2 with LayerNorm 2
+def test_wait_limit_around_layernorm_in_the_epilogue(stage):
+    from souffle_models_b200 import _lib
+    cfg = so.BertConfig(16, 128, 12, 64, 128, "std")
+    layers = so.make_bert_weights(cfg, 3, 1)
+    x, _ = so.make_bert_input(cfg, 3)
+    bad = _encoder(cfg, layers, tuning=LN_TILES(128, 96, 128, 96, timeout_ms=20, debug_skip_arrival=(stage << 16) | 2))
+    for _ in range(2):
+        bad.forward(x.cuda())
+        with pytest.raises(_lib.SouffleError) as ei:
+            bad.status()
+        assert ei.value.code == 6 and f"code 2, where {stage}," in str(ei.value)
+    bad.close()
+
+
 @pytest.mark.parametrize("B,S,heads,ffn", [
     (1, 16, 2, 128),       # rows of 128 columns: one warp, the second block of columns is absent
     (9, 384, 2, 256),      # the same in two passes, the second one ragged
