@@ -1433,7 +1433,7 @@ constexpr int kPipeOCol = 256;                   // TMEM: scores at 0 / 128, out
 
 template <bool kPair>
 __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, uint8_t* ring_ptr,
-                              uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
+                              uint8_t* boxes, RoleState& rs, const WaitCtl& ctl, int warp, int lane) {
   const MegaParams& p = ca.p;
   const int S = st.seq, B = st.batch, H = st.heads;
   // kPair: the two CTAs of a pair take the two heads 2c, 2c + 1 of one sequence (same valid length) and the leader
@@ -1447,6 +1447,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
   const int first = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   const int my_items = units > first ? (units - 1 - first) / step + 1 : 0;
   auto item_of = [&](int k) -> int { const int u = first + k * step; return kPair ? 2 * u + (int)rank : u; };
+  auto seq_of = [&](int item) -> int { return (int)fast_div((uint32_t)item, (uint32_t)H, st.mg_heads); };
   const uint32_t bar0 = smem_u32(&ctl_s.qk_full), bar1 = smem_u32(&ctl_s.attn1[0]);
   auto bar = [&](int g, int which) -> uint32_t { return (g ? bar1 : bar0) + 8u * (uint32_t)which; };
   const uint32_t oempty0 = smem_u32(&ctl_s.o_empty[0]);
@@ -1459,10 +1460,9 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
       for (int k = 0; ok && k < my_items; ++k) {
         const int item = item_of(k), g = k & 1;
-        const int h = item % H, b = item / H;
-        const int rq = ((0 * B + b) * H + h) * S, rk = ((1 * B + b) * H + h) * S, rv = ((2 * B + b) * H + h) * S;
+        const int rq = item * S, rk = (B * H + item) * S, rv = (2 * B * H + item) * S;
         const uint32_t base = ring + g * kPipeBytes, bit = (bits >> g) & 1u;
-        if (!mbar_wait(bar(g, AB_QK_EMPTY), bit ^ 1u, ctl, 500 + g)) break;
+        if (!mbar_wait_hot(bar(g, AB_QK_EMPTY), bit ^ 1u, ctl, 500 + g)) break;
         if constexpr (kPair) {            // both CTAs' tiles are counted on the leader's barriers
           if (rank == 0) mbar_expect_tx(bar(g, AB_QK_FULL), 4u * kATileBytes);
           const uint32_t fl = map_shared_rank(bar(g, AB_QK_FULL), 0);
@@ -1473,7 +1473,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
           tma_load_2d(base, tm, bar(g, AB_QK_FULL), 0, rq);
           tma_load_2d(base + kATileBytes, tm, bar(g, AB_QK_FULL), 0, rk);
         }
-        if (!mbar_wait(bar(g, AB_V_EMPTY), bit ^ 1u, ctl, 502 + g)) break;
+        if (!mbar_wait_hot(bar(g, AB_V_EMPTY), bit ^ 1u, ctl, 502 + g)) break;
         if constexpr (kPair) {
           if (rank == 0) mbar_expect_tx(bar(g, AB_V_FULL), 2u * kATileBytes);
           tma_load_2d_pair(base + 2 * kATileBytes, tm, map_shared_rank(bar(g, AB_V_FULL), 0), 0, rv);
@@ -1498,7 +1498,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       auto issue_s = [&](int k) {                              // scores of item k: S = Q K^T
         const int g = k & 1;
         const uint32_t base = ring + g * kPipeBytes;
-        if (!mbar_wait(bar(g, AB_QK_FULL), (bits >> g) & 1u, ctl, 510 + g)) { ok = false; return; }
+        if (!mbar_wait_hot(bar(g, AB_QK_FULL), (bits >> g) & 1u, ctl, 510 + g)) { ok = false; return; }
         tc_fence_after_sync();
         if constexpr (kPair) {
           umma_f16_k64_pair(tmem + g * 256, umma_desc_lo(base, 16), umma_desc_lo(base + kATileBytes, 16), 2u, idesc_s, 0u);
@@ -1515,8 +1515,8 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       for (int k = 0; ok && k < my_items; ++k) {
         const int g = k & 1;
         const uint32_t base = ring + g * kPipeBytes, bit = (bits >> g) & 1u;
-        if (!mbar_wait(bar(g, AB_P_FULL), bit, ctl, 512 + g)) break;
-        if (!mbar_wait(bar(g, AB_V_FULL), bit, ctl, 514 + g)) break;
+        if (!mbar_wait_hot(bar(g, AB_P_FULL), bit, ctl, 512 + g)) break;
+        if (!mbar_wait_hot(bar(g, AB_V_FULL), bit, ctl, 514 + g)) break;
         tc_fence_after_sync();
         // O = P V: K = 128 keys = two chunks of 64; V is an MN-major B operand (16 keys = 2048 B per step)
         if constexpr (kPair) {
@@ -1537,7 +1537,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
         bits ^= 1u << g;
         if (k + 2 < my_items) {
           if constexpr (kPair) {          // the next scores of this pipeline overwrite the output just issued: wait for its readers
-            if (!mbar_wait(oempty0 + 8 * g, (obits >> g) & 1u, ctl, 516 + g)) break;
+            if (!mbar_wait_hot(oempty0 + 8 * g, (obits >> g) & 1u, ctl, 516 + g)) break;
             tc_fence_after_sync();
           }
           issue_s(k + 2);
@@ -1556,17 +1556,19 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
     const float sl2 = st.scale * 1.4426950408889634f;
     const float mask_l2 = -10000.0f * 1.4426950408889634f;
     const int* lens = p.lens;
-    __half* ctx = reinterpret_cast<__half*>(st.out);
     __half* probs = reinterpret_cast<__half*>(st.probs);
-    const int hd = st.head_dim, hidden = H * hd;
-    uint8_t* sbuf = stage_s + (warp - 2) * kStageWarp;
+    const CUtensorMap* tm_out = map_ptr(ca, st.tm_out);
+    StoreBoxes sb;                                            // a row's 64 columns are two boxes
+    sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+    sb.box = 0;
+    sb.n = 2;
     uint8_t* pbase = ring_ptr + g * kPipeBytes + 3 * kATileBytes + r_in * 128;
     uint32_t bit = g ? rs.attn_bit1 : rs.attn_bit;
     const bool prof = p.prof != nullptr;
     long long t_ws = 0, t_sm = 0, t_wo = 0, t_ep = 0, t_p1 = 0;
     for (int k = g; k < my_items; k += 2) {
       const int item = item_of(k);
-      const int h = item % H, b = item / H;
+      const int b = seq_of(item), h = item - b * H;
       const int kv_len = lens ? lens[b] : S;
       const long long c0 = prof ? clock64() : 0;
       if (!mbar_wait_warp(bar(g, AB_S_FULL), bit, ctl, 520 + g, lane)) break;
@@ -1574,48 +1576,49 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       tc_fence_after_sync();
       const uint32_t ts = kPair ? tmem + g * 256 + rank * 128 : tmem + g * 128;
       // Masked keys (>= kv_len) get -10000 added, which underflows to probability 0 in fp32 and never wins
-      // the maximum, so both passes only visit the 16-column blocks that hold valid keys.  TMEM loads are
-      // double-buffered 16 columns at a time: the next block is in flight while this one is processed.
+      // the maximum, so both passes only visit the 32-column blocks that hold valid keys.  The next block is requested as soon
+      // as this one's values have been used (16 columns at a time left the exponentials waiting for one another: softmax of
+      // 64 x 128 4.0 k cycles an item).
       const int kvl = kv_len < 1 ? 1 : (kv_len > S ? S : kv_len);
-      const int nb = (kvl + 15) >> 4;
-      uint32_t ra[16], rb[16];
+      const int nb = (kvl + 31) >> 5;
+      uint32_t r[32];
       // ---- pass 1: row maximum of the raw scores of the valid keys (the scale is positive) ----
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
-      auto max16 = [&](const uint32_t (&r)[16], int blk) {
-        const int key0 = blk * 16;
-        if (key0 + 16 <= kvl) {
+      auto max32 = [&](int blk) {
+        const int left = kvl - blk * 32;
+        if (left >= 32) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
-            m0 = fmaxf(m0, __uint_as_float(r[i])); m1 = fmaxf(m1, __uint_as_float(r[i + 1]));
-            m2 = fmaxf(m2, __uint_as_float(r[i + 2])); m3 = fmaxf(m3, __uint_as_float(r[i + 3]));
+          for (int i = 0; i < 32; i += 8) {
+            m0 = fmaxf(m0, fmaxf(__uint_as_float(r[i]), __uint_as_float(r[i + 4])));
+            m1 = fmaxf(m1, fmaxf(__uint_as_float(r[i + 1]), __uint_as_float(r[i + 5])));
+            m2 = fmaxf(m2, fmaxf(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 6])));
+            m3 = fmaxf(m3, fmaxf(__uint_as_float(r[i + 3]), __uint_as_float(r[i + 7])));
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) m0 = fmaxf(m0, key0 + i < kvl ? __uint_as_float(r[i]) : -INFINITY);
+          for (int i = 0; i < 32; i += 2) {
+            m0 = fmaxf(m0, i < left ? __uint_as_float(r[i]) : -INFINITY);
+            m1 = fmaxf(m1, i + 1 < left ? __uint_as_float(r[i + 1]) : -INFINITY);
+          }
         }
+        if (left > 32) tmem_ld32(ts + (blk + 1) * 32, r);
       };
-      tmem_ld16(ts, ra);
-      tmem_ld_wait(ra);
-      for (int blk = 0; blk < nb; blk += 2) {
-        if (blk + 1 < nb) tmem_ld16(ts + (blk + 1) * 16, rb);
-        max16(ra, blk);
-        if (blk + 1 < nb) {
-          tmem_ld_wait(rb);
-          if (blk + 2 < nb) tmem_ld16(ts + (blk + 2) * 16, ra);
-          max16(rb, blk + 1);
-          if (blk + 2 < nb) tmem_ld_wait(ra);
-        }
+      tmem_ld32(ts, r);
+#pragma unroll 1
+      for (int blk = 0; blk < nb; ++blk) {
+        tmem_ld_wait(r);
+        max32(blk);
       }
       const float mx = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)) * sl2;
       const long long c1a = prof ? clock64() : 0;
       // ---- pass 2: unnormalised probabilities -> fp16 A-operand tile (128B-swizzled rows) ----
       float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
-      auto exp16 = [&](const uint32_t (&r)[16], int blk) {
-        const int key0 = blk * 16;
-        uint32_t w[8];
-        if (key0 + 16 <= kvl) {
+      auto exp32 = [&](int blk) {
+        const int left = kvl - blk * 32;
+        uint32_t w[16];
+        if (left >= 32) {
 #pragma unroll
-          for (int i = 0; i < 16; i += 4) {
+          for (int i = 0; i < 32; i += 4) {
             const float p0 = ex2_fast(fmaf(__uint_as_float(r[i]), sl2, -mx)), p1 = ex2_fast(fmaf(__uint_as_float(r[i + 1]), sl2, -mx));
             const float p2 = ex2_fast(fmaf(__uint_as_float(r[i + 2]), sl2, -mx)), p3 = ex2_fast(fmaf(__uint_as_float(r[i + 3]), sl2, -mx));
             s0 += p0; s1 += p1; s2 += p2; s3 += p3;
@@ -1624,45 +1627,41 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
           }
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; i += 2) {
-            const float p0 = key0 + i < kvl ? ex2_fast(fmaf(__uint_as_float(r[i]), sl2, -mx)) : 0.f;
-            const float p1 = key0 + i + 1 < kvl ? ex2_fast(fmaf(__uint_as_float(r[i + 1]), sl2, -mx)) : 0.f;
+          for (int i = 0; i < 32; i += 2) {
+            const float p0 = i < left ? ex2_fast(fmaf(__uint_as_float(r[i]), sl2, -mx)) : 0.f;
+            const float p1 = i + 1 < left ? ex2_fast(fmaf(__uint_as_float(r[i + 1]), sl2, -mx)) : 0.f;
             s0 += p0; s1 += p1;
             w[i >> 1] = pack_h2(p0, p1);
           }
         }
-        uint8_t* base = pbase + (blk >> 2) * kATileBytes;
-        const int j = (blk & 3) * 2;
-        *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+        if (left > 32) tmem_ld32(ts + (blk + 1) * 32, r);
+        uint8_t* base = pbase + (blk >> 1) * kATileBytes;
+        const int j = (blk & 1) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          *reinterpret_cast<uint4*>(base + (((j + i) ^ (r_in & 7)) << 4)) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
       };
-      tmem_ld16(ts, ra);
-      tmem_ld_wait(ra);
-      for (int blk = 0; blk < nb; blk += 2) {
-        if (blk + 1 < nb) tmem_ld16(ts + (blk + 1) * 16, rb);
-        exp16(ra, blk);
-        if (blk + 1 < nb) {
-          tmem_ld_wait(rb);
-          if (blk + 2 < nb) tmem_ld16(ts + (blk + 2) * 16, ra);
-          exp16(rb, blk + 1);
-          if (blk + 2 < nb) tmem_ld_wait(ra);
-        }
+      tmem_ld32(ts, r);
+#pragma unroll 1
+      for (int blk = 0; blk < nb; ++blk) {
+        tmem_ld_wait(r);
+        exp32(blk);
       }
-      for (int blk = nb; blk < 8; ++blk) {                    // keys past the valid ones: probability 0
-        uint8_t* base = pbase + (blk >> 2) * kATileBytes;
-        const int j = (blk & 3) * 2;
-        *reinterpret_cast<uint4*>(base + ((j ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(base + (((j + 1) ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
+      for (int blk = nb; blk < 4; ++blk) {                    // keys past the valid ones: probability 0
+        uint8_t* base = pbase + (blk >> 1) * kATileBytes;
+        const int j = (blk & 1) * 4;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *reinterpret_cast<uint4*>(base + (((j + i) ^ (r_in & 7)) << 4)) = make_uint4(0u, 0u, 0u, 0u);
       }
       const float inv = 1.0f / ((s0 + s1) + (s2 + s3));
       if (probs) {                                            // parity output: normalised probabilities
-        attn_store_probs_staged(ts, sbuf, probs + (size_t)(b * H + h) * S * S, q * 32, S, kv_len, sl2, mask_l2, mx, inv, lane);
+        attn_store_probs_staged(ts, sb.base, probs + (size_t)(b * H + h) * S * S, q * 32, S, kv_len, sl2, mask_l2, mx, inv, lane);
       }
       fence_proxy_async_smem();
       tc_fence_before_sync();
       if constexpr (kPair) {                                  // one arrival per warp on the leader's barrier (8 in all)
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster(map_shared_rank(bar(g, AB_P_FULL), 0));
+        if (lane == 0) mbar_arrive_cluster_relaxed(map_shared_rank(bar(g, AB_P_FULL), 0));      // P is read by this SM's own tensor core
       } else {
         mbar_arrive(bar(g, AB_P_FULL));
       }
@@ -1670,25 +1669,19 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       if (!mbar_wait_warp(bar(g, AB_O_FULL), bit, ctl, 522 + g, lane)) break;
       const long long c3 = prof ? clock64() : 0;
       tc_fence_after_sync();
-      {
-        // O rows are 128 bytes: two staged stores of 64 bytes per row
-        const int row0 = q * 32;
-        uint8_t* rowptr[4];
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          uint32_t r[32];
-          tmem_ld32((kPair ? tmem + g * 256 + rank * 64 : tmem + kPipeOCol + g * 64) + half * 32, r);
-          tmem_ld_wait(r);
+      for (int half = 0; half < 2; ++half) {                  // (no plain stores: a pair's arrivals would wait for them)
+        uint32_t w[16];
+        tmem_ld32((kPair ? tmem + g * 256 + rank * 64 : tmem + kPipeOCol + g * 64) + half * 32, r);
+        tmem_ld_wait(r);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const int rr = row0 + 8 * i + (lane >> 2);
-            rowptr[i] = rr < S ? reinterpret_cast<uint8_t*>(ctx + ((size_t)b * S + rr) * hidden + h * hd + half * 32) : nullptr;
-          }
-          uint32_t w[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) w[i] = pack_h2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
-          staged_store_64B(sbuf, w, rowptr, lane);
-        }
+        for (int i = 0; i < 16; ++i) w[i] = pack_h2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+        store_box(sb, w, lane, [&](uint32_t buf) {
+          // 16 rows of the block where the sequence ends inside it
+          const int row0 = q * 32, y = b * S + row0, x = h * 64 + half * 32;
+          if (row0 < S) tma_store_2d(tm_out, buf, x, y);
+          if (st.out_stores == 2 && row0 + 16 < S) tma_store_2d(tm_out, buf + 16 * kStageRow, x, y + 16);
+        });
       }
       tc_fence_before_sync();
       if constexpr (kPair) {                                  // this warp has read its rows of the output accumulator
@@ -1702,6 +1695,11 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       long long* pr = p.prof + ((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots;
       pr[3] = t_ws; pr[4] = t_sm; pr[5] = t_wo; pr[6] = t_ep; pr[7] = t_p1;
     }
+    if (elect_one()) {                     // the stores are complete before the CTA reports the stage done
+      bulk_wait_group_all();
+      fence_proxy_async_global();
+    }
+    __syncwarp();
     if (g) rs.attn_bit1 = bit; else rs.attn_bit = bit;
     // the other pipeline's bit advances with that pipeline's item count
     const int n_other = (my_items + (g ? 1 : 0)) >> 1;        // items handled by pipeline 1-g
@@ -2585,8 +2583,8 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
           state = rs.pack();
         } else if (st.type == STAGE_ATTN) {
           RoleState rs = RoleState::unpack(state);
-          if constexpr (kFamily == kFamilyBert) attn_stage_pp<false>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
-          else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
+          if constexpr (kFamily == kFamilyBert) attn_stage_pp<false>(st, ca, cs, ring, ring_ptr, reinterpret_cast<uint8_t*>(vec_s), rs, ctl, warp, lane);
+          else if constexpr (kFamily == kFamilyBertPair) attn_stage_pp<true>(st, ca, cs, ring, ring_ptr, reinterpret_cast<uint8_t*>(vec_s), rs, ctl, warp, lane);
           else attn_stage(st, ca, cs, ring, ring_ptr, stage_s, rs, ctl, warp, lane);
           state = rs.pack();
         } else if (st.type == STAGE_LN) {

@@ -461,6 +461,7 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
                   s.win, s.seq, s.heads, s.ldo);
     return SOUFFLE_OK;
   }
+  s.mg_heads = fast_div_magic((uint32_t)(s.heads > 0 ? s.heads : 1));
   if (s.type != STAGE_GEMM) return SOUFFLE_OK;
   if ((s.epi == EPI_SWIN_QKV || s.epi == EPI_SWIN_PROJ) &&
       (s.win < 1 || s.win * s.win > 64 || s.seq % s.win || s.heads * 32 != s.ldo ||
@@ -490,7 +491,6 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   s.mg_kchunks = fast_div_magic((uint32_t)s.kchunks);
   s.mg_seq = fast_div_magic((uint32_t)(s.seq > 0 ? s.seq : 1));
   s.mg_head_dim = fast_div_magic((uint32_t)(s.head_dim > 0 ? s.head_dim : 1));
-  s.mg_heads = fast_div_magic((uint32_t)(s.heads > 0 ? s.heads : 1));
   if (s.epi == EPI_SWIN_QKV || s.epi == EPI_SWIN_PROJ) {
     s.nwr = s.seq / s.win;
     s.plane_elems = (uint32_t)s.batch * (uint32_t)(s.nwr * s.nwr * 64) * (uint32_t)s.ldo;
@@ -1082,6 +1082,11 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     s = blank_stage(STAGE_ATTN);                       // softmax(QK^T) V
     s.tm_qkv = m_qkv; s.tm_a = m_q; s.bm = q_rows; s.batch = B; s.heads = Hh; s.seq = S; s.head_dim = hd; s.scale = scale;
     s.out = p->ctx; s.probs = (last && d.keep_probs) ? p->probs : nullptr;
+    if (p->family != kFamilyBertCoop) {               // stored in boxes of a head's columns
+      const int stores = head_split_stores(S);
+      CUtensorMap m;
+      if ((rc = make_store_map_uncached(&m, p->ctx, (uint64_t)M, (uint64_t)H, (uint32_t)(32 / stores))) || (rc = set_store_map(p, s, m, stores))) return rc;
+    }
     p->stages.push_back(s);
     if (!keep) note_dead(p, p->qkv, (size_t)3 * M * H * 2);            // Q, K, V: read by the attention stage only
 
