@@ -86,9 +86,10 @@ typedef struct SouffleBertDesc {
   int32_t pair_mma;   /* 1: run on CTA pairs where the shape qualifies (seq <= 128, an even number of heads, more
                          (sequence, head) items than CTAs, at least 2048 rows): clusters of two CTAs share every
                          tensor-core instruction (cta_group::2), each CTA loads half of every weight tile and the
-                         attention stage takes two heads per pair.  0 (default): single-CTA MMAs.  Pairs measure the
-                         same on twelve layers of 64 x 128 and 3 to 8 % faster on mid-sized batches (32 x 128,
-                         40 x 112 at hidden 1024).  souffle_bert_plan_uses_pairs reports what a plan uses. */
+                         attention stage takes two heads per pair.  0 (default): where that is faster, which is from
+                         3072 rows of 768 columns on (twelve layers of 32 x 128 10 %, of 64 x 128 6 %), unless a
+                         bm_ / bn_ setting asks for a tile that pairs do not have.  -1: never.
+                         souffle_bert_plan_uses_pairs reports what a plan uses. */
 } SouffleBertDesc;
 
 /* Device pointers to one layer's parameters, fp16.  Matrices use the reference's [K][N]

@@ -833,11 +833,19 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   int sms = di->sms;
   if (d.max_ctas > 0 && d.max_ctas < sms) sms = d.max_ctas;
   if (sms > di->max_ctas) sms = di->max_ctas;
-  // CTA pairs (opt-in): for shapes whose GEMM stages have many tiles per CTA and whose attention stage has more
-  // (sequence, head) items than CTAs (its two-pipeline form, which the pair build has; the one-item form exists for
-  // single CTAs only)
+  // CTA pairs: for shapes whose GEMM stages have many tiles per CTA and whose attention stage has more (sequence, head) items than
+  // CTAs (its two-pipeline form, which the pair build has; the one-item form exists for single CTAs only).  Unless the caller decides, from
+  // 3072 rows of 768 and more columns on, where a K step of 128 x 256 outputs per CTA is bound by the tensor core (512 cycles) instead of by
+  // the operands' way into shared memory (700).  Twelve layers of 128 tokens, single CTAs / pairs: 32 sequences 926 / 835 us, 64
+  // 1576 / 1485; six of 60 x 64 498 / 434, of 64 x 48 400 / 397; three of 40 x 112 at hidden 1024 360 / 332.  With fewer rows a pair has
+  // one or two tiles (16 x 128 647 / 630) or loses in its lock-step attention (64 x 32, three layers 178 / 182); narrower layers are as fast
+  // either way (64 x 96 at hidden 512 113 / 115, 64 x 128 at 256 247 / 247).
   int npairs = sms / 2 < di->max_pairs ? sms / 2 : di->max_pairs;
-  const bool pair = d.pair_mma == 1 && npairs >= 1 && S <= 128 && Hh % 2 == 0 && B * Hh > sms && M >= 2048;
+  const bool pair_fits = npairs >= 1 && S <= 128 && Hh % 2 == 0 && B * Hh > sms && M >= 2048;
+  // explicit settings that a pair cannot follow
+  const bool pair_tiles = d.bm_qkv != 128 && d.bm_fc1 != 128 && d.bm_proj != 128 && d.bm_fc2 != 128 && d.bn_qkv % 32 == 0 && d.bn_fc1 % 32 == 0 &&
+                          d.bn_proj % 32 == 0 && d.bn_fc2 % 32 == 0;
+  const bool pair = pair_fits && (d.pair_mma == 1 || (d.pair_mma == 0 && M >= 3072 && H >= 768 && pair_tiles));
   p->pair = pair;
   if (pair) sms = 2 * npairs;
   // one attention item per CTA at most, or a long sequence: the stage in which all softmax warps share an item (the grid is at least
