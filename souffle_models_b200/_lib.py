@@ -7,6 +7,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 from . import build as _build
 
 STATUS_NAMES = {0: "OK", 1: "BAD_SHAPE", 2: "BAD_POINTER", 3: "BAD_DEVICE", 4: "NOT_CORESIDENT",
@@ -122,6 +124,18 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+# torch.cuda.current_stream() builds a Stream object, 3.2 us a call; the handle alone takes 0.3 us.  A blocking call on a small input
+# asks twice: squeeze-and-excite of 1 x 32 x 112 x 112, 8 us of kernel, took 32 us.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
+def stream_ptr() -> int:
+    """Handle of the current stream of the current device."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(torch.cuda.current_device())
 
 
 def check(code: int) -> None:

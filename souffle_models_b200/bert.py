@@ -21,10 +21,6 @@ _VEC_KEYS = ("qkv_b", "proj_b", "ln1_g", "ln1_b", "fc1_b", "fc2_b", "ln2_g", "ln
 _MAT_KEYS = ("qkv_w", "proj_w", "fc1_w", "fc2_w")
 
 
-def _stream_ptr() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
 def _check_f16_cuda(t: torch.Tensor, name: str) -> None:
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
@@ -88,7 +84,7 @@ class BertEncoder:
             if seq_lens.dtype != torch.int32 or not seq_lens.is_cuda or seq_lens.numel() != self.batch:
                 raise ValueError("seq_lens must be an int32 CUDA tensor of length batch")
             lens_ptr = seq_lens.data_ptr()
-        _lib.check(self._lib.souffle_bert_forward(self._h, x.data_ptr(), lens_ptr, out.data_ptr(), _stream_ptr()))
+        _lib.check(self._lib.souffle_bert_forward(self._h, x.data_ptr(), lens_ptr, out.data_ptr(), _lib.stream_ptr()))
         return out
 
     def forward_host(self, x_host: torch.Tensor, seq_lens_host: Optional[torch.Tensor], y_host: torch.Tensor,
@@ -98,7 +94,7 @@ class BertEncoder:
         caught up (x_host and y_host must be left alone until then)."""
         lens_ptr = seq_lens_host.data_ptr() if seq_lens_host is not None else None
         fn = self._lib.souffle_bert_forward_host if wait else self._lib.souffle_bert_forward_host_async
-        _lib.check(fn(self._h, x_host.data_ptr(), lens_ptr, y_host.data_ptr(), _stream_ptr()))
+        _lib.check(fn(self._h, x_host.data_ptr(), lens_ptr, y_host.data_ptr(), _lib.stream_ptr()))
 
     def status(self) -> None:
         """Synchronises and raises SouffleError if a device-side wait expired."""
@@ -134,14 +130,14 @@ class BertEncoder:
         n = len(outs)
         _lib.check(self._lib.souffle_bert_plan_copy_buffers(
             self._h, n, (C.c_int * n)(*(_BUF[k] for k in names)), (C.c_void_p * n)(*(t.data_ptr() for t in outs)),
-            (C.c_size_t * n)(*(2 * t.numel() for t in outs)), _stream_ptr()))
+            (C.c_size_t * n)(*(2 * t.numel() for t in outs)), _lib.stream_ptr()))
         return outs
 
     def buffer(self, name: str) -> torch.Tensor:
         """Copy of a last-layer stage output (see SouffleBertBuffer in the header)."""
         out = torch.empty(self._buffer_shape(name), dtype=torch.float16, device="cuda")
         _lib.check(self._lib.souffle_bert_plan_copy_buffer(self._h, _BUF[name], out.data_ptr(), out.numel() * 2,
-                                                           _stream_ptr()))
+                                                           _lib.stream_ptr()))
         return out
 
 

@@ -1,5 +1,6 @@
 """EfficientNet squeeze-and-excite module: host-side mirror of the reference binding
 (cpp/efficientnet/efficientnet_se_module_binding.cu:164-233) over souffle_se_module_forward."""
+import functools
 from typing import Dict, List
 
 import torch
@@ -9,8 +10,9 @@ from . import _lib
 _ws: Dict[int, torch.Tensor] = {}
 
 
-def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+@functools.lru_cache(maxsize=64)
+def _workspace_bytes(batch: int, channels: int, height: int, width: int) -> int:
+    return _lib.load().souffle_se_module_workspace_bytes(batch, channels, height, width)
 
 
 def _workspace(nbytes: int) -> torch.Tensor:
@@ -40,11 +42,11 @@ def se_module(x: torch.Tensor, se_reduce_weight: torch.Tensor, se_expand_weight:
     lib = _lib.load()
     out = torch.empty_like(x)
     pooled = torch.empty(B, Cc, dtype=torch.float32, device=x.device)
-    ws = _workspace(lib.souffle_se_module_workspace_bytes(B, Cc, H, W))
+    ws, stream = _workspace(_workspace_bytes(B, Cc, H, W)), _lib.stream_ptr()
     _lib.check(lib.souffle_se_module_forward(x.data_ptr(), se_reduce_weight.data_ptr(), se_expand_weight.data_ptr(), out.data_ptr(),
-                                             pooled.data_ptr(), B, Cc, H, W, R, ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                             pooled.data_ptr(), B, Cc, H, W, R, ws.data_ptr(), ws.numel(), stream))
     if check:
-        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), _stream_ptr()))
+        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), stream))
     return [pooled, out]
 
 

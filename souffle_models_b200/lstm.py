@@ -8,7 +8,6 @@ from typing import Dict, Optional
 import torch
 
 from . import _lib
-from .bert import _stream_ptr
 
 
 class LstmStack:
@@ -50,7 +49,7 @@ class LstmStack:
         if x.numel() != self.steps * self.hidden:
             raise ValueError(f"x must hold {self.steps}x{self.hidden} values")
         y = torch.empty_like(x)
-        _lib.check(self._lib.souffle_lstm_forward(self._h, x.data_ptr(), y.data_ptr(), _stream_ptr()))
+        _lib.check(self._lib.souffle_lstm_forward(self._h, x.data_ptr(), y.data_ptr(), _lib.stream_ptr()))
         return y
 
     def status(self) -> None:

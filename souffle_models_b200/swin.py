@@ -3,21 +3,30 @@
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import List
 
 import torch
 
 from . import _lib
-from .bert import _check_f16_cuda, _stream_ptr
+from .bert import _check_f16_cuda
 
 _ws = {}
+
+
+@functools.lru_cache(maxsize=64)
+def _workspace_bytes(rows: int, dim: int, ffn: int) -> int:
+    return _lib.load().souffle_swin_mlp_workspace_bytes(rows, dim, ffn)
 
 
 def _workspace(nbytes: int = 0) -> torch.Tensor:
     """Per-device scratch for the plan-less entry points (barrier words, then split-K planes); grows on demand."""
     dev = torch.cuda.current_device()
+    have = _ws.get(dev)
+    if have is not None and nbytes <= have.numel():
+        return have
     need = max(int(nbytes), int(_lib.load().souffle_gemm_workspace_bytes()))
-    if dev not in _ws or _ws[dev].numel() < need:
+    if have is None or have.numel() < need:
         if dev in _ws:          # the old block goes back to the allocator: the library must not trust its address any more
             _lib.load().souffle_workspace_forget(_ws[dev].data_ptr())
         _ws[dev] = torch.zeros(need, dtype=torch.uint8, device="cuda")
@@ -34,12 +43,12 @@ def gemm(a: torch.Tensor, w_kn: torch.Tensor, check: bool = True) -> torch.Tenso
     if K2 != K:
         raise ValueError(f"inner dimensions differ: {K} vs {K2}")
     c = torch.empty(M, N, dtype=torch.float16, device=a.device)
-    ws = _workspace()
+    ws, stream = _workspace(), _lib.stream_ptr()
     lib = _lib.load()
     _lib.check(lib.souffle_gemm_f16(a.data_ptr(), w_kn.data_ptr(), c.data_ptr(), M, N, K, ws.data_ptr(),
-                                    ws.numel(), _stream_ptr()))
+                                    ws.numel(), stream))
     if check:
-        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), _stream_ptr()))
+        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), stream))
     return c
 
 
@@ -70,12 +79,12 @@ def swin_fused_feed_mlp(src: torch.Tensor, fc1_weight: torch.Tensor, fc2_weight:
     hidden = torch.empty(M, F, dtype=torch.float16, device=src.device)
     out = torch.empty(M, Cc, dtype=torch.float16, device=src.device)
     lib = _lib.load()
-    ws = _workspace(lib.souffle_swin_mlp_workspace_bytes(M, Cc, F))
+    ws, stream = _workspace(_workspace_bytes(M, Cc, F)), _lib.stream_ptr()
     _lib.check(lib.souffle_swin_mlp_forward(src.data_ptr(), fc1_weight.data_ptr(), fc2_weight.data_ptr(),
                                             hidden.data_ptr(), out.data_ptr(), M, Cc, F, ws.data_ptr(), ws.numel(),
-                                            _stream_ptr()))
+                                            stream))
     if check:
-        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), _stream_ptr()))
+        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), stream))
     return [hidden, out]
 
 
@@ -121,13 +130,13 @@ def layernorm(partial: torch.Tensor, resid=None, bias=None, gamma=None, beta=Non
         raise ValueError("partial must be a float32 CUDA tensor [P, M, N]")
     P, M, N = partial.shape
     out = torch.empty(M, N, dtype=torch.float16, device=partial.device)
-    ws = _workspace()
+    ws, stream = _workspace(), _lib.stream_ptr()
     lib = _lib.load()
     ptr = lambda t: t.data_ptr() if t is not None else None
     _lib.check(lib.souffle_layernorm_forward(partial.data_ptr(), P, ptr(bias), ptr(resid), ptr(gamma), ptr(beta),
-                                             out.data_ptr(), M, N, eps, ws.data_ptr(), ws.numel(), _stream_ptr()))
+                                             out.data_ptr(), M, N, eps, ws.data_ptr(), ws.numel(), stream))
     if check:
-        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), _stream_ptr()))
+        _lib.check(lib.souffle_workspace_status(ws.data_ptr(), stream))
     return out
 
 
@@ -189,7 +198,7 @@ class SwinBlock:
         if x.numel() != self.batch * self.res * self.res * self.dim:
             raise ValueError("x has the wrong number of elements for this plan")
         y = torch.empty(self.out_shape, dtype=torch.float16, device=x.device)
-        _lib.check(self._lib.souffle_swin_block_forward(self._h, x.data_ptr(), y.data_ptr(), _stream_ptr()))
+        _lib.check(self._lib.souffle_swin_block_forward(self._h, x.data_ptr(), y.data_ptr(), _lib.stream_ptr()))
         return y
 
     def status(self) -> None:
