@@ -818,7 +818,11 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           const uint32_t fb = full0 + 8 * s, dst = ring + s * g.slot_bytes + a_bytes;
           if constexpr (kPair) {
             if (rank == 0) mbar_expect_tx(fb, 2u * b_bytes);
-            tma_load_2d_pair(dst, tmB, map_shared_rank(fb, 0), k0, n0);          // box rows = bn / 2: this CTA's half of the columns
+            if (!b_mn) {
+              tma_load_2d_pair(dst, tmB, map_shared_rank(fb, 0), k0, n0);          // box rows = bn / 2: this CTA's half of the columns
+            } else {
+              for (int j = 0; j < g.bn / 128; ++j) tma_load_2d_pair(dst + j * 8192, tmB, map_shared_rank(fb, 0), n0 + j * 64, k0);
+            }
           } else {
             mbar_expect_tx(fb, b_bytes * (uint32_t)g.kper);
             for (int sub = 0; sub < g.kper; ++sub) {

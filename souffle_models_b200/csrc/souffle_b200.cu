@@ -260,7 +260,7 @@ static TileChoice choose_tiles(int M, int N, int K, int sms, bool allow_split, b
 
 // The same for a plan on CTA pairs: a pair owns a 256 x bn tile, each CTA loads 128 rows of A and bn/2 rows of B per
 // K chunk and runs MMAs of bn/2 cycles; both accumulator buffers of a CTA alternate, so the epilogue overlaps.
-static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_split, std::vector<RankedTile>* ranked = nullptr) {
+static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_split, bool b_mn = false, std::vector<RankedTile>* ranked = nullptr) {
   const int kch = K / 64;
   double best = 1e300;
   TileChoice bt;
@@ -269,6 +269,7 @@ static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_
   for (int ci = 0; ci < 6; ++ci) {
     const int bn = cands[ci];
     if (N % bn) continue;
+    if (b_mn && bn % 128) continue;             // each CTA loads its half in blocks of 64 columns
     for (int split = 1; split <= (allow_split ? 16 : 1); ++split) {
       if (kch % split) continue;
       const long items = (long)((M + 255) / 256) * (N / bn) * split;
@@ -292,6 +293,26 @@ static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_
   }
   if (ranked) std::stable_sort(ranked->begin(), ranked->end(), [](const RankedTile& a, const RankedTile& b) { return a.cost < b.cost; });
   return bt;
+}
+
+// Cycles of one GEMM with fp16 output on single CTAs or on pairs, to choose between the two for a launch.  A K step of 64 takes its MMAs' time
+// or the operands' way into shared memory (70 B per cycle and SM), a pair's at least 450 (the hand-shakes across the cluster); a tile's
+// epilogue of ~950 cycles per 64 columns overlaps the next tile's main loop, except that of a 256-row tile of a single CTA; ~3.5 k
+// until the first operands have arrived (5.5 k on pairs), 8 k until the CTAs run.  Checked against kernel times under ncu, single CTAs /
+// pairs: 8192 x 3072 x 768 40.7 / 35.0 us (model 64 / 54 k cycles), 4096 x 3072 x 768 22.9 / 21.2 (41 / 36), 4096 x 4096 x 1024 36.7 / 31.2,
+// 8192 x 1024 x 1024 20.2 / 19.4, 2048 x 3072 x 768 15.9 / 16.1 (28 / 30); and back to back 8192 x 768 x 3072 32.8 / 38.7 (57 / 66),
+// 1024 x 4096 x 4096 32.1 / 28.9.
+static double gemm_cycles(const TileChoice& t, int M, int N, int K, int ctas, bool pair) {
+  const long items = (long)((M + t.bm - 1) / t.bm) * (N / t.bn) * t.split;
+  const long at_once = pair ? ctas / 2 : ctas, waves = (items + at_once - 1) / at_once;
+  const double steps = K / 64 / t.split, epilogue = t.bn / 64.0 * 950.0;
+  if (pair) {
+    const double step = std::max(450.0, std::max(2.0 * t.bn, (16384.0 + 64.0 * t.bn) / 70.0));
+    return waves * std::max(steps * step, epilogue) + epilogue + 13500.0;
+  }
+  const double step = std::max(t.bm / 128 * 2.0 * t.bn, (128.0 * t.bm + 128.0 * t.bn) / 70.0);
+  if (t.bm == 256) return waves * (steps * step + 2.0 * epilogue) + 11500.0;
+  return waves * std::max(steps * step, epilogue) + epilogue + 11500.0;
 }
 
 // ------------------------------------------------------------------------------------
@@ -389,7 +410,7 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
     at[1].val.cooperative = 1;
     cfg.attrs = at;
     const void* fn = (const void*)souffle_megakernel<kFamilyBertPair>;
-    if (env_coop && di->pair_coop) {
+    if (env_coop && di->pair_coop && args.p.n_stages > 1) {          // (a single stage waits for no CTA outside its pair)
       cfg.numAttrs = 2;
       if (cudaLaunchKernelExC(&cfg, fn, kargs) == cudaSuccess) return SOUFFLE_OK;
       cudaGetLastError();          // a refused launch configuration is not sticky
@@ -752,7 +773,7 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
                           int head_split, int max_split, void* tune_ws, TileChoice* choice, int family) {
   const bool pair = family == kFamilyBertPair;
   std::vector<RankedTile> ranked;
-  if (pair) choose_tiles_pair(proto.M, proto.N, proto.K, sms / 2, allow_split, &ranked);
+  if (pair) choose_tiles_pair(proto.M, proto.N, proto.K, sms / 2, allow_split, false, &ranked);
   else choose_tiles(proto.M, proto.N, proto.K, sms, allow_split, false, head_split, &ranked);
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (cudaEventCreate(&e0) != cudaSuccess || cudaEventCreate(&e1) != cudaSuccess) return;
@@ -1495,13 +1516,24 @@ static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes,
 // several warps.
 static int row_family(int M, int grid) { return M <= grid * (kThreads / 32) ? kFamilyBertCoop : kFamilyBert; }
 
-static int fill_gemm_stage(Stage* s, int tm_a, int tm_b, const void* out, int M, int N, int K, int sms) {
+// Cycles that pairs save in a GEMM of [K][N] weights with fp16 output (negative: they lose), or 0 where they cannot run or come out above
+// `share` of a single CTAs' time.
+static double gemm_saved_by_pairs(int M, int N, int K, int sms, int npairs, double share) {
+  if (npairs < 1 || N % 128) return 0.0;
+  const TileChoice s = choose_tiles(M, N, K, sms, false, true), t = choose_tiles_pair(M, N, K, npairs, false, true);
+  if (!s.bn || !t.bn) return 0.0;
+  const double single = gemm_cycles(s, M, N, K, sms, false), pairs = gemm_cycles(t, M, N, K, 2 * npairs, true);
+  return pairs < share * single ? single - pairs : 0.0;
+}
+
+// `npairs` > 0: for a launch on CTA pairs.
+static int fill_gemm_stage(Stage* s, int tm_a, int tm_b, const void* out, int M, int N, int K, int sms, int npairs = 0) {
   *s = blank_stage(STAGE_GEMM);
-  const TileChoice t = choose_tiles(M, N, K, sms, false, true);
+  const TileChoice t = npairs ? choose_tiles_pair(M, N, K, npairs, false, true) : choose_tiles(M, N, K, sms, false, true);
   if (!t.bn) return fail(SOUFFLE_BAD_SHAPE, "N=%d must be a multiple of 64", N);
   s->tm_a = tm_a; s->tm_b = tm_b; s->M = M; s->N = N; s->K = K; s->bm = t.bm; s->bn = t.bn; s->b_mn_major = 1;
   s->epi = EPI_F16; s->out = const_cast<void*>(out); s->ldo = N;
-  return finalize_stage(*s, 0, 1);
+  return finalize_stage(*s, 0, 1, npairs > 0);
 }
 
 int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_t N, int32_t K, void* workspace,
@@ -1516,14 +1548,17 @@ int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_
   CallArgs args;
   memset(&args, 0, sizeof(args));
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
-  if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, c, M, N, K, sms))) return rc;
-  if ((rc = make_map(&args.call_maps[0], a, M, K, (uint32_t)args.inline_stages[0].bm))) return rc;
+  const int npairs = sms / 2 < di->max_pairs ? sms / 2 : di->max_pairs;
+  const bool pair = gemm_saved_by_pairs(M, N, K, sms, npairs, 0.95) > 0.0;
+  if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, c, M, N, K, sms, pair ? npairs : 0))) return rc;
+  if ((rc = make_map(&args.call_maps[0], a, M, K, pair ? 128u : (uint32_t)args.inline_stages[0].bm))) return rc;
   if ((rc = make_map(&args.call_maps[1], w_kn, K, N, 64))) return rc;     // [K][N]: box 64 (N) x 64 (K rows)
   if ((rc = make_store_map(&args.call_maps[2], c, M, N))) return rc;
   args.inline_stages[0].tm_out = -3;
   args.inline_stages[0].out_stores = 1;
   args.p.n_stages = 1;
   const int items = stage_items(args.inline_stages[0]);
+  if (pair) return ws_launch(&args, 2 * (items < npairs ? items : npairs), workspace, workspace_bytes, st, kFamilyBertPair);
   return ws_launch(&args, items < sms ? items : sms, workspace, workspace_bytes, st);
 }
 

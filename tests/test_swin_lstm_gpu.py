@@ -62,6 +62,17 @@ def test_gemm_stores_end_with_the_matrix(M, N, K):
     assert (out[M:] == 7.0).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(2500, 4096, 1024), (8191, 3072, 768), (1000, 4096, 4096), (8000, 128, 192), (6000, 3200, 512)])
+def test_gemm_of_many_tiles(M, N, K):
+    """Large products run on CTA pairs (256-row tiles, each CTA with half of the [K][N] weights' columns): ragged rows, tiles of 256 and 128
+    columns, several per pair.  fp16 output (half an ulp) and fp32 sums."""
+    from souffle_models_b200 import swin
+    a, w = _rand((M, K), K), _rand((K, N), K + 1, 1.0 / K ** 0.5)
+    c = swin.gemm(a.cuda(), w.cuda())
+    want = (a.cuda().double() @ w.cuda().double()).float()
+    assert (c.float() - want).abs().max() < 2e-3 * max(1.0, want.abs().max().item())
+
+
 def test_swin_fused_mlp_and_fc2():
     from souffle_models_b200 import swin
     src, w1, w2 = _rand((256, 512), 3), _rand((512, 2048), 4, 0.02), _rand((2048, 512), 5, 0.02)
