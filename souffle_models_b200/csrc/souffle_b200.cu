@@ -1516,14 +1516,11 @@ static int ws_launch(CallArgs* args, int grid, void* workspace, size_t ws_bytes,
 // several warps.
 static int row_family(int M, int grid) { return M <= grid * (kThreads / 32) ? kFamilyBertCoop : kFamilyBert; }
 
-// Cycles that pairs save in a GEMM of [K][N] weights with fp16 output (negative: they lose), or 0 where they cannot run or come out above
-// `share` of a single CTAs' time.
-static double gemm_saved_by_pairs(int M, int N, int K, int sms, int npairs, double share) {
-  if (npairs < 1 || N % 128) return 0.0;
+// Whether a GEMM of [K][N] weights with fp16 output is faster on pairs.
+static bool gemm_on_pairs(int M, int N, int K, int sms, int npairs) {
+  if (npairs < 1 || N % 128) return false;
   const TileChoice s = choose_tiles(M, N, K, sms, false, true), t = choose_tiles_pair(M, N, K, npairs, false, true);
-  if (!s.bn || !t.bn) return 0.0;
-  const double single = gemm_cycles(s, M, N, K, sms, false), pairs = gemm_cycles(t, M, N, K, 2 * npairs, true);
-  return pairs < share * single ? single - pairs : 0.0;
+  return s.bn && t.bn && gemm_cycles(t, M, N, K, 2 * npairs, true) < 0.95 * gemm_cycles(s, M, N, K, sms, false);
 }
 
 // `npairs` > 0: for a launch on CTA pairs.
@@ -1549,7 +1546,7 @@ int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_
   memset(&args, 0, sizeof(args));
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
   const int npairs = sms / 2 < di->max_pairs ? sms / 2 : di->max_pairs;
-  const bool pair = gemm_saved_by_pairs(M, N, K, sms, npairs, 0.95) > 0.0;
+  const bool pair = gemm_on_pairs(M, N, K, sms, npairs);
   if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, c, M, N, K, sms, pair ? npairs : 0))) return rc;
   if ((rc = make_map(&args.call_maps[0], a, M, K, pair ? 128u : (uint32_t)args.inline_stages[0].bm))) return rc;
   if ((rc = make_map(&args.call_maps[1], w_kn, K, N, 64))) return rc;     // [K][N]: box 64 (N) x 64 (K rows)
@@ -1565,11 +1562,6 @@ int souffle_gemm_f16(const void* a, const void* w_kn, void* c, int32_t M, int32_
 // FC2 of the MLP has few output tiles and a long K (256 x 512 outputs, K = 2048 in the reference's shape), so
 // it is cut along K into fp32 planes and a third stage sums them: the LayerNorm stage in its sum-only mode.
 // The planes live behind the barrier words of the workspace.
-static int swin_mlp_split(int M, int C, int F, int sms) {
-  const TileChoice t = choose_tiles(M, C, F, sms, true, true);
-  return t.bn ? t.split : 1;
-}
-
 size_t souffle_swin_mlp_workspace_bytes(int32_t M, int32_t C, int32_t F) {
   if (M < 1 || C < 64 || F < 64) return souffle_gemm_workspace_bytes();
   return souffle_gemm_workspace_bytes() + (size_t)16 * M * C * sizeof(float);      // room for the deepest split
@@ -1588,26 +1580,45 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
   CallArgs args;
   memset(&args, 0, sizeof(args));
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
-  if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, hidden, M, F, C, sms))) return rc;
-  // split FC2 when the caller's workspace has room for the planes and the reduction stage supports the width
-  int split = swin_mlp_split(M, C, F, sms);
+  // FC2's tiles: cut along K when the caller's workspace has room for the planes and the reduction stage supports the width
   const bool can_reduce = C == 128 || C == 256 || C == 512 || C == 768 || C == 1024;
   const size_t plane_bytes = (size_t)M * C * sizeof(float);
-  if (!can_reduce || workspace_bytes < souffle_gemm_workspace_bytes() + (size_t)split * plane_bytes) split = 1;
-  Stage& s2 = args.inline_stages[1];
-  if (split > 1) {
-    const TileChoice t = choose_tiles(M, C, F, sms, true, true);
-    s2 = blank_stage(STAGE_GEMM);
-    s2.tm_a = -3; s2.tm_b = -4; s2.M = M; s2.N = C; s2.K = F; s2.bm = t.bm; s2.bn = t.bn; s2.splitk = split; s2.b_mn_major = 1;
-    s2.epi = EPI_PARTIAL; s2.ldo = C;
-    s2.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + souffle_gemm_workspace_bytes());
-    if ((rc = finalize_stage(s2, 0, 1))) return rc;
-  } else if ((rc = fill_gemm_stage(&s2, -3, -4, out, M, C, F, sms))) {
-    return rc;
+  auto fc2_tiles = [&](int npairs) {
+    TileChoice t = npairs ? choose_tiles_pair(M, C, F, npairs, true, true) : choose_tiles(M, C, F, sms, true, true);
+    if (t.split > 1 && (!can_reduce || workspace_bytes < souffle_gemm_workspace_bytes() + (size_t)t.split * plane_bytes))
+      t = npairs ? choose_tiles_pair(M, C, F, npairs, false, true) : choose_tiles(M, C, F, sms, false, true);
+    return t;
+  };
+  TileChoice t2 = fc2_tiles(0);
+  // both products on CTA pairs where they take less time together (see gemm_cycles)
+  int npairs = sms / 2 < di->max_pairs ? sms / 2 : di->max_pairs;
+  if (npairs >= 1 && C % 128 == 0 && F % 128 == 0 && t2.bn) {
+    const TileChoice p2 = fc2_tiles(npairs);
+    const double pairs = gemm_cycles(choose_tiles_pair(M, F, C, npairs, false, true), M, F, C, 2 * npairs, true) + gemm_cycles(p2, M, C, F, 2 * npairs, true);
+    const double single = gemm_cycles(choose_tiles(M, F, C, sms, false, true), M, F, C, sms, false) + gemm_cycles(t2, M, C, F, sms, false);
+    if (pairs < 0.95 * single) t2 = p2;
+    else npairs = 0;
+  } else {
+    npairs = 0;
   }
-  if ((rc = make_map(&args.call_maps[0], src, M, C, (uint32_t)args.inline_stages[0].bm))) return rc;
+  const bool pair = npairs > 0;
+  if ((rc = fill_gemm_stage(&args.inline_stages[0], -1, -2, hidden, M, F, C, sms, npairs))) return rc;
+  if (!t2.bn) return fail(SOUFFLE_BAD_SHAPE, "N=%d must be a multiple of 64", C);
+  const int split = t2.split;
+  Stage& s2 = args.inline_stages[1];
+  s2 = blank_stage(STAGE_GEMM);
+  s2.tm_a = -3; s2.tm_b = -4; s2.M = M; s2.N = C; s2.K = F; s2.bm = t2.bm; s2.bn = t2.bn; s2.splitk = split; s2.b_mn_major = 1; s2.ldo = C;
+  if (split > 1) {
+    s2.epi = EPI_PARTIAL;
+    s2.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + souffle_gemm_workspace_bytes());
+  } else {
+    s2.epi = EPI_F16;
+    s2.out = out;
+  }
+  if ((rc = finalize_stage(s2, 0, 1, pair))) return rc;
+  if ((rc = make_map(&args.call_maps[0], src, M, C, pair ? 128u : (uint32_t)args.inline_stages[0].bm))) return rc;
   if ((rc = make_map(&args.call_maps[1], fc1_w, C, F, 64))) return rc;
-  if ((rc = make_map(&args.call_maps[2], hidden, M, F, (uint32_t)s2.bm))) return rc;
+  if ((rc = make_map(&args.call_maps[2], hidden, M, F, pair ? 128u : (uint32_t)s2.bm))) return rc;
   if ((rc = make_map(&args.call_maps[3], fc2_w, F, C, 64))) return rc;
   if ((rc = make_store_map(&args.call_maps[4], hidden, M, F))) return rc;
   args.inline_stages[0].tm_out = -5;
@@ -1620,14 +1631,15 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
   int items = stage_items(args.inline_stages[0]);
   const int i2 = stage_items(s2);
   if (i2 > items) items = i2;
-  const int grid = items < sms ? items : sms;
+  const int grid = pair ? 2 * (items < npairs ? items : npairs) : items < sms ? items : sms;
   if (split > 1) {
     Stage& s3 = args.inline_stages[2];
     s3 = blank_stage(STAGE_LN);
-    s3.M = M; s3.N = C; s3.ldo = C; s3.partial = s2.partial; s3.n_partial = split; s3.out = out;
+    s3.M = M; s3.N = C; s3.ldo = C; s3.partial = s2.partial; s3.n_partial = (uint8_t)split; s3.out = out;
     s3.eps = -1.0f;                                    // sum only
     if ((rc = finalize_stage(s3, 0, grid))) return rc;
   }
+  if (pair) return ws_launch(&args, grid, workspace, workspace_bytes, st, kFamilyBertPair);
   return ws_launch(&args, grid, workspace, workspace_bytes, st, row_family(M, grid));
 }
 

@@ -73,6 +73,20 @@ def test_gemm_of_many_tiles(M, N, K):
     assert (c.float() - want).abs().max() < 2e-3 * max(1.0, want.abs().max().item())
 
 
+@pytest.mark.parametrize("M,C,F", [(7001, 768, 3072), (8000, 512, 2048), (4000, 1024, 4096), (3000, 128, 256), (5000, 640, 2560)])
+def test_mlp_of_many_rows(M, C, F):
+    """Both products on CTA pairs (or, the smallest, on single CTAs), with and without planes, ragged rows.  The second product is
+    compared from the hidden layer as stored."""
+    from souffle_models_b200 import swin
+    a, w1, w2 = _rand((M, C), 3), _rand((C, F), 4, 1.0 / C ** 0.5), _rand((F, C), 5, 1.0 / F ** 0.5)
+    for _ in range(2):
+        hidden, out = swin.swin_fused_feed_mlp(a.cuda(), w1.cuda(), w2.cuda())
+        h = (a.cuda().double() @ w1.cuda().double()).float()
+        assert (hidden.float() - h).abs().max() < 2e-3 * max(1.0, h.abs().max().item())
+        o = (hidden.double() @ w2.cuda().double()).float()
+        assert (out.float() - o).abs().max() < 2e-3 * max(1.0, o.abs().max().item())
+
+
 def test_swin_fused_mlp_and_fc2():
     from souffle_models_b200 import swin
     src, w1, w2 = _rand((256, 512), 3), _rand((512, 2048), 4, 0.02), _rand((2048, 512), 5, 0.02)
