@@ -219,8 +219,8 @@ int souffle_lstm_launch_mode(void);
 /* Has no counterpart in the reference.  The same stacked-LSTM forward for callers that must not allocate
  * device memory (a server whose memory pool owns the whole GPU, a plugin inside someone else's process, a
  * loop that cannot take the device-wide synchronisation cudaMalloc/cudaFree imply): no plan, no cudaMalloc,
- * cudaFree or other allocating call.  The kernel's scratch -- every published hidden state, the per-layer
- * arrival counters, the status words -- sits in a fixed array inside the library image (about 1.5 MB held
+ * cudaFree or other allocating call.  The kernel's scratch -- every published hidden state beside its
+ * launch's tag, the launch counter, the status words -- sits in a fixed array inside the library image (about 3 MB held
  * by every GPU that loads the library, until the process exits), so layers * steps * hidden must not exceed
  * 12 * 128 * 256 = 393,216; larger shapes are rejected with SOUFFLE_BAD_SHAPE (use a plan for those).
  * w_in / w_state (fp16 [4*layers][hidden][hidden]), bias (fp32 [layers][hidden] or null), x and y (fp32
@@ -228,7 +228,7 @@ int souffle_lstm_launch_mode(void);
  * `stream` has run.  `device_status` is optional: 4 device ints that receive {code, where, cta, 0}, code 0
  * meaning every bounded wait was satisfied.  The first call on a device also looks up the array's device
  * address and sets the kernel's attributes; make that first call before any stream capture begins.
- * All calls share the one array and it keeps the previous call's contents: the counters and status words
+ * All calls share the one array and it keeps the previous call's contents: the status words
  * are cleared on `stream` at the start of each call, and two calls that overlap on the GPU (different
  * streams, or different host threads) would race on it -- serialise them. */
 int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, const void* w_state, const float* bias,

@@ -21,14 +21,13 @@
 // A step of hidden 256 takes 2.3 k cycles (hidden 64: 1.5 k); with the products on the CUDA cores (128 conversions and FMAs
 // per thread, partial sums by shuffle, one waiting thread and a CTA barrier) it took 3.5 k (2.4 k): 10 layers x 100 steps
 // 228 -> 155 us, 12 x 64 x 200 266 -> 175 us.
-// Only the hop to the next layer goes through global memory: one slot per (layer, step) and per-layer arrival counters.
-// Every CTA of a layer publishes its own count of finished steps; the consumer checks all eight, so a CTA whose
-// publication lags cannot be covered by its peers running ahead.  The same holds inside a CTA: a warp sends h(t) to the
-// cluster before it has stored it to global memory, so its peers may be a step further on while that store is still on its
-// way; every cell warp therefore counts its own stored steps, and what the CTA publishes is the smallest of the counts.
-// Two more warps keep that hop off the cell arithmetic's path: a fetch warp brings the layer's input
-// vectors into shared memory up to four steps ahead, and a publish warp pays for the release fence
-// behind the hidden states the cell warps have stored.
+// Only the hop to the next layer goes through global memory: one slot per (layer, step) and unit, a 64-bit word of the hidden
+// state and the launch's tag.  A word is written as a whole, so the reader, which polls the vector itself, needs neither a
+// fence in front of the store nor a counter behind it, and a unit that lags cannot be covered by its peers.  With counters (a release
+// behind the stored states, a poll of eight counters, then the vector) a hop took a fence and a round trip through L2 more:
+// 10 layers x 100 steps of hidden 256 155 -> 141 us, 3 x 37 of hidden 128 38.7 -> 34.8 a call.
+// A fetch warp keeps that hop off the cell arithmetic's path: it brings the layer's input vectors into shared memory up to four steps
+// ahead.
 // There is no grid-wide barrier.  All waits in the step loop are bounded; on expiry the CTA records a
 // status word, leaves the loop and waits for its cluster at the final cluster barrier (shared
 // memory must outlive the peers' remote stores).  That barrier does not cover the stores themselves: st.async completes on
@@ -48,10 +47,8 @@ namespace souffle {
 constexpr int kLstmParts = 8;                      // CTAs per layer = cluster size
 constexpr int kLstmXBufs = 4;                      // input vectors the fetch warp may run ahead
 constexpr int kLstmMaxLayers = 18;
-constexpr int kLstmDoneWords = 256;                // one set of published-step counters: kLstmMaxLayers * kLstmParts, rounded up
-static_assert(kLstmMaxLayers * kLstmParts <= kLstmDoneWords, "counter block too small");
-// threads of a CTA: a cell warp per 32 hidden units of the layer (it owns four of the CTA's), the fetch and the publish warp
-__host__ __device__ constexpr int lstm_block(int H) { return (H / 32 + 2) * 32; }
+// threads of a CTA: a cell warp per 32 hidden units of the layer (it owns four of the CTA's), and the fetch warp
+__host__ __device__ constexpr int lstm_block(int H) { return (H / 32 + 1) * 32; }
 
 struct LstmParams {
   const __half* w_in;     // [4*L][H][H], row = output unit, col = input
@@ -59,9 +56,8 @@ struct LstmParams {
   const float* bias;      // [L][H] or null; added to all four gates of a unit (reference layout)
   const float* x;         // [T][H]
   float* y;               // [T][H]: top layer's h per step
-  float* h_all;           // [L][T][H] scratch: every published hidden state
-  unsigned* done;         // [L][kLstmParts] published-step counters of this launch, one per (layer, CTA of its cluster)
-  unsigned* done_next;    // the counters the next launch will use (cleared here)
+  uint64_t* h_all;        // [L][T][H] scratch: every published hidden state (low half) beside the launch's tag
+  unsigned* epoch;        // launches on this scratch so far; the tag is one more, which no word of the scratch holds yet
   int* status;
   int* expired;           // host memory or null: set by a CTA that gave up on a wait
   int layers, hidden, steps, ref_input_delay;
@@ -192,7 +188,7 @@ template <int H>
 struct LstmShared {
   static constexpr int kWarps = H / 32;         // cell warps: four units each
   static constexpr int kRow = lstm_row(H);
-  // Hidden 256: a cell thread's weights are 128 registers of the 168 that ten warps leave it (registers are handed out per
+  // Hidden 256: a cell thread's weights are 128 registers of the 168 that nine warps leave it (registers are handed out per
   // four warps); two blocks of the input half stay in shared memory instead.
   static constexpr int kXReg = H == 256 ? 6 : H / 32;
   alignas(16) __half x[kLstmXBufs][3 * kRow];   // input vectors
@@ -204,7 +200,7 @@ struct LstmShared {
   int abort;
   uint32_t pieces;                              // 1: from the next input vector on, vectors come in pieces
   int piece[kWarps];                            // then: pieces a cell warp has multiplied so far
-  uint32_t stored[kWarps];                      // steps whose hidden states a cell warp has stored to global memory
+  uint32_t tag;                                 // of this launch's words in h_all
 };
 
 template <int H>
@@ -253,7 +249,6 @@ __device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& s
   const int send_part = lane >> 3;
   const uint32_t send_to = map_shared_rank(smem_u32(&sh.h[0][(send_part < 3 ? send_part : 0) * kRow + unit0]), (uint32_t)(lane & 7));
   const uint32_t send_bar = map_shared_rank(hfull0, (uint32_t)(lane & 7));
-  const uint32_t stored_a = smem_u32(sh.stored + warp);
   float cx[4];                                // W_in x(t), scaled back
   bool ok = true;
   auto input_half = [&](int step) {
@@ -332,10 +327,16 @@ __device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& s
       st_async_b64(send_to + (uint32_t)(hb * 3 * kRow * 2), word, send_bar + 8u * (uint32_t)hb);
     }
     if (lane == 24) {
-      const float4 h4 = make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
-      __stcg(reinterpret_cast<float4*>(p.h_all + ((size_t)layer * T + t) * H + unit0), h4);
-      if (layer == L - 1) *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) = h4;
-      st_release_cta_shared_u32(stored_a, (uint32_t)t + 1u);      // the publish warp takes it from here
+      if (layer == L - 1) {
+        *reinterpret_cast<float4*>(p.y + (size_t)t * H + unit0) =
+            make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
+      } else {                                  // for the next layer
+        const uint32_t tag = *const_cast<volatile uint32_t*>(&sh.tag);
+        uint64_t* to = p.h_all + (uint32_t)(t * H + unit0);         // (a 64-bit step index would spill at hidden 256)
+        to += (size_t)(uint32_t)(layer * T) * H;
+        st_relaxed_tagged(to, got[0], got[1], tag);
+        st_relaxed_tagged(to + 2, got[2], got[3], tag);
+      }
     }
     if (t + 1 < T) input_half(t + 1);
   }
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     sh.abort = 0;
     sh.deadline_ns = globaltimer_ns() + p.timeout_ns;
     sh.pieces = 0;
-    for (int i = 0; i < kWarps; ++i) sh.stored[i] = 0;
+    sh.tag = *const_cast<volatile unsigned*>(p.epoch) + 1u;
     for (int i = 0; i < kLstmXBufs; ++i) {
       mbar_init(xfull0 + 8 * i, 32);            // the 32 lanes of the fetch warp
       mbar_init(xempty0 + 8 * i, kWarps);       // one lane of every cell warp
@@ -381,8 +382,6 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     }
     fence_mbar_init();
   }
-  if (blockIdx.x == 0)
-    for (int i = tid; i < L * kLstmParts; i += lstm_block(H)) p.done_next[i] = 0u;
   for (int i = tid; i < 2 * 3 * kRow; i += lstm_block(H)) (&sh.h[0][0])[i] = __ushort_as_half(0);    // h before the first step
   __syncthreads();
   cluster_sync_all();                           // every CTA's barriers exist before anyone arrives on them
@@ -390,46 +389,11 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   LstmWaitOf<H> ctl;
   lstm_wait_set<H>(ctl, sh, p);
 
-  if (warp == kWarps + 1) {
-    // ---------------- publish warp: makes the stored hidden states visible to the next layer ----------------
-    const uint32_t stored_a = smem_u32(sh.stored + (lane & (kWarps - 1)));
-    uint32_t published = 0, spins = 0;
-    while (layer + 1 < L && published < (uint32_t)T) {      // nobody reads the top layer's count
-      const uint32_t n = __reduce_min_sync(0xffffffffu, ld_acquire_cta_shared_u32(stored_a));
-      if (n > published) {
-        __syncwarp();                           // every lane's acquire is in front of lane 0's release, which covers them all
-        if (lane == 0) st_release_u32(p.done + layer * kLstmParts + part, n);     // this CTA's units of steps < n are in h_all
-        published = n;
-      } else if (((++spins) & 0xFF) == 0) {
-        int give_up = 0;
-        if (lane == 0) give_up = lstm_expired(ctl, DEV_TIMEOUT_FLAG, 950) ? 1 : 0;
-        if (__shfl_sync(0xffffffffu, give_up, 0)) break;
-      }
-    }
-    __syncwarp();
-  } else if (warp == kWarps) {
+  if (warp == kWarps) {
     // ---------------- fetch warp: the layer's input vector of every step -> shared memory ----------------
-    // Two L2 round trips per step (the counters of the layer below, then the vector) are longer than a step: the counters
-    // are read again only when the steps they announced have been used up, and the next vector is requested before this
-    // one is unpacked.
+    // The vector of the layer below is polled as a whole, and the next one is requested before this one is unpacked: where the layer
+    // below is ahead, a step costs no round trip.
     constexpr int E = H / 32;                   // elements of this lane: lane * E ...
-    const unsigned* ctr = p.done + (layer - 1) * kLstmParts + (lane & (kLstmParts - 1));
-    unsigned avail = layer == 0 ? (unsigned)T : 0u;       // steps the layer below is known to have published
-    auto load_vector = [&](int t, float (&v)[E]) {
-      const float* src = nullptr;
-      if (layer == 0) {
-        const int tx = p.ref_input_delay ? t - 1 : t;
-        if (tx >= 0) src = p.x + (size_t)tx * H;
-      } else {
-        src = p.h_all + ((size_t)(layer - 1) * T + t) * H;
-      }
-#pragma unroll
-      for (int i = 0; i < E; i += 2) {
-        const float2 f = src ? __ldcg(reinterpret_cast<const float2*>(src + lane * E + i)) : make_float2(0.f, 0.f);
-        v[i] = f.x;
-        v[i + 1] = f.y;
-      }
-    };
     // vector or piece number n of this CTA: the wait for its slot, and its way into it
     auto slot_free = [&](int n) -> int {
       const int xb = n % kLstmXBufs, use = n / kLstmXBufs;
@@ -455,20 +419,23 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
       if (lane == 0) sh.x_scale[xb] = down;
       mbar_arrive(xfull0 + 8 * xb);             // release: this lane's stores are visible to whoever waits
     };
-    float v[E], ahead[E];
+    if (layer > 0) {
+      const uint64_t* src = p.h_all + (size_t)(layer - 1) * T * H + lane * E;
+      const uint32_t tag = *const_cast<volatile uint32_t*>(&sh.tag);
+      uint64_t word[E];
+      auto request = [&](const uint64_t* from, uint64_t (&w)[E]) {
 #pragma unroll
-    for (int i = 0; i < E; ++i) ahead[i] = 0.0f;
-    bool have = false;                          // `v` holds step t already
-    int piece = 0;                              // layer 0: pieces handed over so far (the steps so far, unless one had several)
-    bool in_pieces = false;                     // the cell warps expect several
-    for (int t = 0; t < T; ++t) {
-      int ok = 1;
-      if ((unsigned)t >= avail) {
-        // lanes read the counter of one CTA of the layer below each; the smallest counts
+        for (int i = 0; i < E; i += 2) ld_relaxed_2x64(from + i, w[i], w[i + 1]);
+      };
+      request(src, word);
+      for (int t = 0; t < T; ++t, src += H) {
+        int ok = 1;
         uint32_t spins = 0;
         for (;;) {
-          avail = __reduce_min_sync(0xffffffffu, ld_acquire_u32(ctr));
-          if (avail > (unsigned)t) break;
+          bool there = true;
+#pragma unroll
+          for (int i = 0; i < E; ++i) there = there && (uint32_t)(word[i] >> 32) == tag;
+          if (__all_sync(0xffffffffu, there)) break;
           if (((++spins) & 0x3F) == 0) {
             int give_up = 0;
             if (lane == 0) give_up = lstm_expired(ctl, DEV_TIMEOUT_FLAG, 700 + layer) ? 1 : 0;
@@ -477,17 +444,34 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
               break;
             }
           }
+          request(src, word);
         }
-        __syncwarp();                           // the other lanes' loads stay behind every lane's acquire
-      }
-      if (ok && !have) load_vector(t, v);
-      const bool next = t + 1 < T && (unsigned)(t + 1) < avail;
-      if (ok && next) load_vector(t + 1, ahead);
-      if (layer > 0) {
+        float v[E];
+#pragma unroll
+        for (int i = 0; i < E; ++i) v[i] = __uint_as_float((uint32_t)word[i]);
+        if (ok && t + 1 < T) request(src + H, word);
         if (ok) ok = slot_free(t);
-        if (ok) hand_over(t, v, kLstmHScale, 1.0f / kLstmHScale);        // hidden states: a constant scale
+        if (!ok) {
+          if (lane == 0) *const_cast<volatile int*>(&sh.abort) = 1;
+          break;
+        }
+        hand_over(t, v, kLstmHScale, 1.0f / kLstmHScale);          // hidden states: a constant scale
       }
-      for (bool more = layer == 0; more && ok;) {
+    }
+    int piece = 0;                              // layer 0: pieces handed over so far (the steps so far, unless one had several)
+    bool in_pieces = false;                     // the cell warps expect several
+    for (int t = 0; layer == 0 && t < T; ++t) {
+      const int tx = p.ref_input_delay ? t - 1 : t;
+      const float* src = p.x + (size_t)tx * H + lane * E;
+      float v[E];
+#pragma unroll
+      for (int i = 0; i < E; i += 2) {
+        const float2 f = tx >= 0 ? __ldcg(reinterpret_cast<const float2*>(src + i)) : make_float2(0.f, 0.f);
+        v[i] = f.x;
+        v[i + 1] = f.y;
+      }
+      int ok = 1;
+      for (bool more = true; more && ok;) {
         // power-of-two scale that takes the piece's largest element into the upper range of fp16
         uint32_t m = 0;
 #pragma unroll
@@ -530,9 +514,6 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
         if (lane == 0) *const_cast<volatile int*>(&sh.abort) = 1;
         break;
       }
-      have = next;
-#pragma unroll
-      for (int i = 0; i < E; ++i) v[i] = ahead[i];
     }
   } else {
     // ---------------- cell arithmetic ----------------
@@ -551,6 +532,8 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();
   cluster_sync_all();
+  // the top layer has had every word of the layers below, so every CTA has read the epoch
+  if (layer == L - 1 && part == 0 && tid == 0) *p.epoch = sh.tag;
   if (*const_cast<volatile int*>(&sh.abort)) {   // sent by peers before they came here, and not waited for: 200 us are ample
     if (tid == 0 && p.expired) *p.expired = 1;
     const unsigned long long t0 = globaltimer_ns();

@@ -4,7 +4,7 @@
 // all device memory to its own pool, a plugin loaded into a process whose allocator it does not
 // own, or a latency-critical loop where the implicit device synchronisation of cudaMalloc/cudaFree
 // is not acceptable.  For them the wavefront kernel's scratch (the published hidden states of every
-// (layer, step), the per-layer arrival counters and the status words) lives in a fixed array that
+// (layer, step), the launch counter their tags come from and the status words) lives in a fixed array that
 // is part of the library image.  Every GPU that loads the library holds these kStaticScratchBytes
 // until the process exits.
 #pragma once
@@ -17,9 +17,9 @@
 namespace souffle {
 
 constexpr size_t kStaticHiddenFloats = (size_t)12 * 128 * 256;      // layers * steps * hidden <= this
-constexpr size_t kStaticStatusOffset = 2 * kLstmDoneWords * sizeof(unsigned);   // two sets of counters, then the status words
-constexpr size_t kStaticCtlBytes = kStaticStatusOffset + 256;
-constexpr size_t kStaticScratchBytes = kStaticHiddenFloats * 4 + kStaticCtlBytes;
+constexpr size_t kStaticStatusOffset = kStaticHiddenFloats * 8;      // a word per hidden state, then the status words, then the launch counter
+constexpr size_t kStaticEpochOffset = kStaticStatusOffset + 256;
+constexpr size_t kStaticScratchBytes = kStaticEpochOffset + 256;     // zero when the library is loaded
 
 // In host code this name is only a handle for cudaGetSymbolAddress; it is not a device address.
 static __device__ __align__(256) unsigned char g_lstm_static_scratch[kStaticScratchBytes];

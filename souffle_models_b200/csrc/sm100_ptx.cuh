@@ -407,6 +407,11 @@ __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
 __device__ __forceinline__ void st_relaxed_2x64(void* p, uint64_t a, uint64_t b) {
   asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
 }
+// a and b, each beside `tag` in the upper half of its word.
+__device__ __forceinline__ void st_relaxed_tagged(void* p, uint32_t a, uint32_t b, uint32_t tag) {
+  asm volatile("{\n\t.reg .b64 u, v;\n\tmov.b64 u, {%1, %3};\n\tmov.b64 v, {%2, %3};\n\tst.relaxed.gpu.global.v2.b64 [%0], {u, v};\n\t}"
+               ::"l"(p), "r"(a), "r"(b), "r"(tag) : "memory");
+}
 __device__ __forceinline__ void ld_relaxed_2x64(const void* p, uint64_t& a, uint64_t& b) {
   asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }

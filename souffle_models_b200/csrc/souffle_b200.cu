@@ -2010,11 +2010,10 @@ static int lstm_launch(const LstmParams& lp, cudaStream_t st) {
 struct SouffleLstmPlan {
   SouffleLstmDesc desc;
   __half *w_in = nullptr, *w_state = nullptr;
-  float *bias = nullptr, *h_all = nullptr;
-  // four sets of kLstmDoneWords counters: two for alternate launches, one for captured ones, one these clear for nobody
-  unsigned* done = nullptr;
+  float* bias = nullptr;
+  uint64_t* h_all = nullptr;
+  unsigned* epoch = nullptr;
   int* status = nullptr;
-  unsigned launch_id = 0;
 };
 
 int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, const void* w_state, const float* bias,
@@ -2042,14 +2041,15 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
   }
   cudaError_t e = cudaMalloc((void**)&p->w_in, wbytes);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->w_state, wbytes);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&p->h_all, (size_t)d.layers * d.steps * H * 4);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&p->done, 4 * kLstmDoneWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&p->h_all, (size_t)d.layers * d.steps * H * 8);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&p->epoch, 64);
   if (e == cudaSuccess) e = cudaMalloc((void**)&p->status, 64);
   if (e == cudaSuccess && bias) e = cudaMalloc((void**)&p->bias, (size_t)d.layers * H * 4);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_in, w_in, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->w_state, w_state, wbytes, cudaMemcpyDeviceToDevice);
   if (e == cudaSuccess && bias) e = cudaMemcpy(p->bias, bias, (size_t)d.layers * H * 4, cudaMemcpyDeviceToDevice);
-  if (e == cudaSuccess) e = cudaMemset(p->done, 0, 4 * kLstmDoneWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMemset(p->h_all, 0, (size_t)d.layers * d.steps * H * 8);
+  if (e == cudaSuccess) e = cudaMemset(p->epoch, 0, 64);
   if (e == cudaSuccess) e = cudaMemset(p->status, 0, 64);
   if (e != cudaSuccess) {
     souffle_lstm_plan_destroy(p);
@@ -2062,7 +2062,7 @@ int souffle_lstm_plan_create(const SouffleLstmDesc* desc, const void* w_in, cons
 int souffle_lstm_plan_destroy(SouffleLstmPlan* p) {
   if (!p) return SOUFFLE_OK;
   cudaDeviceSynchronize();
-  cudaFree(p->w_in); cudaFree(p->w_state); cudaFree(p->bias); cudaFree(p->h_all); cudaFree(p->done); cudaFree(p->status);
+  cudaFree(p->w_in); cudaFree(p->w_state); cudaFree(p->bias); cudaFree(p->h_all); cudaFree(p->epoch); cudaFree(p->status);
   delete p;
   return SOUFFLE_OK;
 }
@@ -2074,21 +2074,13 @@ int souffle_lstm_forward(SouffleLstmPlan* plan, const float* x, float* y, souffl
   LstmParams lp;
   lp.w_in = plan->w_in; lp.w_state = plan->w_state; lp.bias = plan->bias; lp.x = x; lp.y = y; lp.h_all = plan->h_all;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  bool captured = false;
-  int rc = is_captured(st, &captured);
-  if (rc) return rc;
-  const unsigned set = captured ? 2u : plan->launch_id & 1u;
-  lp.done = plan->done + kLstmDoneWords * set;
-  lp.done_next = plan->done + kLstmDoneWords * (set ^ 1u);
-  if (captured) SF_CUDA(cudaMemsetAsync(lp.done, 0, kLstmDoneWords * sizeof(unsigned), st));
+  lp.epoch = plan->epoch;
+  int rc = SOUFFLE_OK;
   lp.status = plan->status;
   if ((rc = expired_word(&lp.expired))) return rc;
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
-  rc = lstm_launch(lp, st);
-  if (rc) return rc;
-  if (!captured) plan->launch_id++;
-  return SOUFFLE_OK;
+  return lstm_launch(lp, st);
 }
 
 int souffle_lstm_launch_mode(void) { return g_lstm_coop; }
@@ -2101,7 +2093,6 @@ int souffle_lstm_plan_status(SouffleLstmPlan* plan) {
   if (rc) return rc;
   if (h[0] != DEV_OK) {
     cudaMemset(plan->status, 0, 64);
-    cudaMemset(plan->done, 0, 2 * kLstmDoneWords * sizeof(unsigned));
   }
   return decode_status(h, "souffle_lstm_forward");
 }
@@ -2158,19 +2149,17 @@ int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, c
     }
   }
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  unsigned char* ctl = sd.scratch + kStaticHiddenFloats * 4;
-  // counters and status must start at zero; the hidden-state slots are all written before they are read
-  SF_CUDA(cudaMemsetAsync(ctl, 0, kStaticCtlBytes, st));
+  // hidden states are recognised by this launch's tag; only the status words have to start at zero
+  if (!device_status) SF_CUDA(cudaMemsetAsync(sd.scratch + kStaticStatusOffset, 0, 16, st));
   if (device_status) SF_CUDA(cudaMemsetAsync(device_status, 0, 16, st));
   LstmParams lp;
   lp.w_in = reinterpret_cast<const __half*>(w_in);
   lp.w_state = reinterpret_cast<const __half*>(w_state);
   lp.bias = bias; lp.x = x; lp.y = y;
-  lp.h_all = reinterpret_cast<float*>(sd.scratch);
-  lp.done = reinterpret_cast<unsigned*>(ctl);
-  lp.done_next = reinterpret_cast<unsigned*>(ctl) + kLstmDoneWords;
+  lp.h_all = reinterpret_cast<uint64_t*>(sd.scratch);
+  lp.epoch = reinterpret_cast<unsigned*>(sd.scratch + kStaticEpochOffset);
   lp.expired = nullptr;                  // the words below are read unasked; nothing is allocated here
-  lp.status = device_status ? reinterpret_cast<int*>(device_status) : reinterpret_cast<int*>(ctl + kStaticStatusOffset);
+  lp.status = device_status ? reinterpret_cast<int*>(device_status) : reinterpret_cast<int*>(sd.scratch + kStaticStatusOffset);
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;
   lp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
   return lstm_launch(lp, st);
@@ -2185,7 +2174,7 @@ int souffle_lstm_static_status(souffle_stream_t stream) {
   if (rc) return rc;
   SF_CUDA(cudaStreamSynchronize(reinterpret_cast<cudaStream_t>(stream)));
   int h[4] = {0, 0, 0, 0};
-  SF_CUDA(cudaMemcpy(h, sd->scratch + kStaticHiddenFloats * 4 + kStaticStatusOffset, sizeof(h), cudaMemcpyDeviceToHost));
+  SF_CUDA(cudaMemcpy(h, sd->scratch + kStaticStatusOffset, sizeof(h), cudaMemcpyDeviceToHost));
   return decode_status(h, "souffle_lstm_forward_static");
 }
 

@@ -1,4 +1,5 @@
 """Parity of the GEMM / Swin MLP / LSTM entry points (through the C ABI) with the oracle."""
+import ctypes as C
 import math
 import os
 
@@ -485,3 +486,25 @@ def test_first_call_on_a_workspace_may_be_captured():
     finally:
         _lib.load().souffle_workspace_forget(swin._ws[dev].data_ptr())
         swin._ws[dev] = old
+
+
+@pytest.mark.parametrize("layers,hidden,steps", [(18, 64, 3), (12, 256, 40), (5, 128, 64)])
+def test_lstm_calls_do_not_read_one_another(layers, hidden, steps):
+    """Hidden states of a call are told from those of the calls before by their tag alone: calls on changing inputs, plan and
+    allocation-free entry in turn (the latter's scratch is shared by all shapes), each against the oracle."""
+    from souffle_models_b200 import _lib, lstm
+    _, w_in, w_st = so.make_lstm_params(layers, hidden, steps, seed=9)
+    plan = lstm.LstmStack(w_in.cuda(), w_st.cuda(), steps)
+    wi, ws = w_in.half().cuda(), w_st.half().cuda()
+    desc = _lib.LstmDesc(layers=layers, hidden=hidden, steps=steps)
+    for i in range(4):
+        x = torch.randn(1, steps, hidden, generator=torch.Generator().manual_seed(i))
+        want = so.lstm_forward(x, w_in, w_st)[0].reshape(steps, hidden)
+        xd = x.cuda()
+        y = plan.forward(xd).reshape(steps, hidden)
+        s = torch.empty_like(y)
+        _lib.check(_lib.load().souffle_lstm_forward_static(C.byref(desc), wi.data_ptr(), ws.data_ptr(), None, xd.data_ptr(), s.data_ptr(),
+                                                           None, torch.cuda.current_stream().cuda_stream))
+        plan.status()
+        assert torch.equal(y, s)
+        assert (y.cpu() - want).abs().max() < 2e-5 + 1e-3 * want.abs().max()
