@@ -269,10 +269,9 @@ __device__ __forceinline__ void gemm_item(const Stage& st, int item, int& mt, in
 // shared memory and would otherwise be re-read around every asm statement).
 struct EpiCtx {
   int epi, act, M, N, ldo;
-  const __half* resid;
   __half* out;
   float* partial;
-  const CUtensorMap* tm_out;   // store map, or null: plain stores
+  const CUtensorMap* tm_out;   // store map
   bool prof;
 };
 constexpr uint32_t kNoRow = 0xFFFFFFFFu;      // "this row is outside the matrix"
@@ -303,40 +302,9 @@ __device__ __forceinline__ void staged_store_64B(uint8_t* sbuf, const uint32_t (
   __syncwarp();
 }
 
-// Swin row maps.  Tokens of an R x R grid are rolled by -shift and cut into (R/win)^2 windows of win*win
-// tokens; the window-major buffers give every window 64 row slots (49 used for win = 7).
-// The divisors are host constants of the stage, so a quotient is one multiply-high (fast_div): with plain divisions,
-// evaluated for five rows per thread, the epilogue of a 128 x 32 tile took 9.5 k cycles, now 2.2 k.
-// token row (b*R*R + ty*R + tx)  ->  window-major row (global window)*64 + position
-__device__ __forceinline__ int swin_token_to_slot(const Stage& st, int row) {
-  const int R = st.seq, win = st.win, shift = st.shift, nwr = st.nwr;
-  const int img = st.mg_seq2 ? (int)__umulhi((uint32_t)row, st.mg_seq2) : row / (R * R), t = row - img * R * R;
-  const int ty = (int)fast_div((uint32_t)t, (uint32_t)R, st.mg_seq), tx = t - ty * R;
-  int sy = ty - shift, sx = tx - shift;
-  if (sy < 0) sy += R;
-  if (sx < 0) sx += R;
-  const int wy = (int)fast_div((uint32_t)sy, (uint32_t)win, st.mg_win), wx = (int)fast_div((uint32_t)sx, (uint32_t)win, st.mg_win);
-  return (img * nwr * nwr + wy * nwr + wx) * 64 + (sy - wy * win) * win + (sx - wx * win);
-}
-// window-major row -> token row, or -1 for a padding slot
-__device__ __forceinline__ int swin_slot_to_token(const Stage& st, int slot, int n_windows) {
-  const int R = st.seq, win = st.win, shift = st.shift, nwr = st.nwr;
-  const int wg = slot >> 6, pos = slot & 63;
-  if (pos >= win * win || wg >= n_windows) return -1;
-  const int img = (int)fast_div((uint32_t)wg, (uint32_t)(nwr * nwr), st.mg_nwr2), w = wg - img * nwr * nwr;
-  const int wy = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr), wx = w - wy * nwr;
-  const int py = (int)fast_div((uint32_t)pos, (uint32_t)win, st.mg_win), px = pos - py * win;
-  int ty = wy * win + py + shift, tx = wx * win + px + shift;
-  if (ty >= R) ty -= R;
-  if (tx >= R) tx -= R;
-  return img * R * R + ty * R + tx;
-}
-
 // Output addressing is split into a row part, computed once per tile, and a column part, computed once
 // per chunk; both are element offsets that fit 32 bits (the host rejects larger buffers).
-// Row part: offset of matrix row `row` in the stage's output (kNoRow past the end).  The residual, where a
-// stage has one, is laid out like the output, so the same offset addresses it.
-template <bool kSwin>
+// Row part: offset of matrix row `row` in the stage's output (kNoRow past the end).
 __device__ __forceinline__ uint32_t epi_row_offset(const Stage& st, const EpiCtx& e, int row, int ks) {
   if (row >= e.M) return kNoRow;
   if (e.epi == EPI_PARTIAL) return (uint32_t)(ks * e.M + row) * (uint32_t)e.N;
@@ -345,30 +313,15 @@ __device__ __forceinline__ uint32_t epi_row_offset(const Stage& st, const EpiCtx
     const uint32_t b = fast_div((uint32_t)row, (uint32_t)st.seq, st.mg_seq), sq = (uint32_t)row - b * (uint32_t)st.seq;
     return (b * (uint32_t)(st.heads * st.seq) + sq) * (uint32_t)st.head_dim;
   }
-  if constexpr (kSwin) {
-    if (e.epi == EPI_SWIN_QKV) return (uint32_t)swin_token_to_slot(st, row) * (uint32_t)e.ldo;
-    if (e.epi == EPI_SWIN_PROJ) {
-      const int t = swin_slot_to_token(st, row, e.M >> 6);
-      return t >= 0 ? (uint32_t)t * (uint32_t)e.ldo : kNoRow;
-    }
-  }
   return (uint32_t)row * (uint32_t)e.ldo;
 }
 // Column part: offset of column `col` (a multiple of 16; a chunk never straddles a head or a q/k/v plane).
-template <bool kSwin>
 __device__ __forceinline__ uint32_t epi_col_offset(const Stage& st, const EpiCtx& e, int col) {
   if (e.epi == EPI_QKV) {
     const uint32_t g = fast_div((uint32_t)col, (uint32_t)st.head_dim, st.mg_head_dim), dd = (uint32_t)col - g * (uint32_t)st.head_dim;
     const uint32_t which = fast_div(g, (uint32_t)st.heads, st.mg_heads), hh = g - which * (uint32_t)st.heads;
     const uint32_t head_plane = (uint32_t)(st.seq * st.head_dim);
     return (which * (uint32_t)(st.batch * st.heads) + hh) * head_plane + dd;
-  }
-  if constexpr (kSwin) {
-    if (e.epi == EPI_SWIN_QKV) {
-      // [3][windows][64][C]: the column picks q/k/v and the channel
-      const int which = (col >= e.ldo) + (col >= 2 * e.ldo), ch = col - which * e.ldo;
-      return (uint32_t)which * st.plane_elems + (uint32_t)ch;
-    }
   }
   return (uint32_t)col;
 }
@@ -423,49 +376,7 @@ __device__ __forceinline__ void store_box(StoreBoxes& sb, const uint32_t* w, int
   sb.box = sb.box + 1 == sb.n ? 0 : sb.box + 1;
 }
 
-// One 32-column chunk of the row-permuting epilogues: r[i] = column col+i of this thread's own row, whose output
-// offset is `own`; `so[i]` = output offset of row (8*i + lane/4) of the same 32-row block (staged stores).
-__device__ __forceinline__ void epilogue_permuted32(const Stage& st, const EpiCtx& e, uint8_t* sbuf, const uint32_t (&r)[32], const float* bias,
-                                                    uint32_t own, const uint32_t (&so)[4], int col, int lane) {
-  float v[32];
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-  {
-    const float4* b4 = reinterpret_cast<const float4*>(bias);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 b = b4[i];
-      v[4 * i] += b.x; v[4 * i + 1] += b.y; v[4 * i + 2] += b.z; v[4 * i + 3] += b.w;
-    }
-  }
-  if (e.resid && own != kNoRow) {
-    const uint4* r4 = reinterpret_cast<const uint4*>(e.resid + own + col);
-    float2 fr[16];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 u = r4[i];
-      const __half2* h = reinterpret_cast<const __half2*>(&u);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) fr[4 * i + j] = __half22float2(h[j]);
-    }
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      v[2 * i] += fr[i].x;
-      v[2 * i + 1] += fr[i].y;
-    }
-  }
-  const uint32_t coff = epi_col_offset<true>(st, e, col);
-  uint8_t* rowptr[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) rowptr[i] = so[i] != kNoRow ? reinterpret_cast<uint8_t*>(e.out + (so[i] + coff)) : nullptr;
-  uint32_t w[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) w[i] = pack_h2(v[2 * i], v[2 * i + 1]);
-  staged_store_64B(sbuf, w, rowptr, lane);
-}
-
 // 16-column tail chunk (tile widths that are an odd multiple of 16): direct stores.
-template <bool kSwin>
 __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& e, const uint32_t (&r)[16], const float* bias, uint32_t own, int col) {
   if (own == kNoRow) return;
   if (e.epi == EPI_PARTIAL) {
@@ -486,7 +397,7 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
 #pragma unroll
     for (int i = 0; i < 16; ++i) v[i] = gelu_tanh(v[i]);
   }
-  uint4* d4 = reinterpret_cast<uint4*>(e.out + (own + epi_col_offset<kSwin>(st, e, col)));
+  uint4* d4 = reinterpret_cast<uint4*>(e.out + (own + epi_col_offset(st, e, col)));
   d4[0] = make_uint4(pack_h2(v[0], v[1]), pack_h2(v[2], v[3]), pack_h2(v[4], v[5]), pack_h2(v[6], v[7]));
   d4[1] = make_uint4(pack_h2(v[8], v[9]), pack_h2(v[10], v[11]), pack_h2(v[12], v[13]), pack_h2(v[14], v[15]));
 }
@@ -714,7 +625,7 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
 // shared memory -- half the B traffic per FLOP of the single-CTA form -- with every copy's completion counted on the
 // leader's full barrier; the leader's MMA lane issues for both and its commits arrive on the barriers of both CTAs;
 // each CTA's epilogue warps drain their own 128 rows and report to the leader's accumulator-free barrier.
-template <bool kSwin, bool kPair = false, bool kLnEpi = false>
+template <bool kPair = false, bool kLnEpi = false>
 __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
                            uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp_id, int lane) {
   const int warp = uniform_warp(warp_id);
@@ -963,10 +874,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     } else {
     EpiCtx e;
     e.epi = st.epi; e.act = st.act; e.M = st.M; e.N = st.N; e.ldo = st.ldo;
-    e.resid = reinterpret_cast<const __half*>(sel_ptr(st.resid_sel, st.resid, p));
     e.out = reinterpret_cast<__half*>(const_cast<void*>(sel_ptr(st.out_sel, st.out, p)));
     e.partial = st.partial;
-    e.tm_out = st.out_stores ? map_ptr(ca, st.tm_out) : nullptr;
+    e.tm_out = map_ptr(ca, st.tm_out);
     const bool prof = p.prof != nullptr;
     e.prof = prof;
     // cycle totals of the profile go straight to its record (no registers held for them over the tiles)
@@ -1016,12 +926,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         const uint32_t acc = acc0 + (uint32_t)h;
         // output rows first: worked out while the accumulator is still being filled
         const int row0 = row_tile + (kPair ? (int)rank : h) * 128 + q * 32;
-        const uint32_t own = epi_row_offset<kSwin>(st, e, row0 + lane, plane);
-        uint32_t so[4];                              // rows of the staged stores: each lane has worked out one of the 32
-        if constexpr (kSwin) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) so[i] = __shfl_sync(0xffffffffu, own, 8 * i + (lane >> 2));
-        }
+        const uint32_t own = epi_row_offset(st, e, row0 + lane, plane);
         // head-split stores: rows of the [3 B heads S][64] view at which the block's two halves of 16 rows begin
         uint32_t tok0 = 0, tok1 = 0;
         if (e.epi == EPI_QKV) {
@@ -1063,15 +968,13 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
               store_box(sb, r + 16 * half, lane, [&](uint32_t buf) {
                 if (row0 < e.M) tma_store_3d(e.tm_out, buf, col + 16 * half, row0, plane);
               });
-          } else if (kSwin && !e.tm_out) {
-            epilogue_permuted32(st, e, stage_s + (warp - 2) * kStageWarp, r, bias_t + c * 32, own, so, col, lane);
           } else {
             uint32_t w[16];
             epilogue_values32(e, r, bias_t + c * 32, w);
             if (prof) tmid = (unsigned)clock64();
             store_box(sb, w, lane, [&](uint32_t buf) {
               if (row0 < e.M) {
-                if (!kSwin && e.epi == EPI_QKV) {
+                if (e.epi == EPI_QKV) {
                   const uint32_t gq = (uint32_t)col >> 6, which = fast_div(gq, (uint32_t)st.heads, st.mg_heads), hh = gq - which * (uint32_t)st.heads;
                   const uint32_t head_row = (which * (uint32_t)(st.batch * st.heads) + hh) * (uint32_t)st.seq;
                   tma_store_2d(e.tm_out, buf, col & 63, (int)(head_row + tok0));
@@ -1091,7 +994,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
           uint32_t r[16];
           tmem_ld16(t0 + full_chunks * 32, r);
           tmem_ld_wait(r);
-          epilogue_chunk16<kSwin>(st, e, r, bias_t + full_chunks * 32, own, colbase + full_chunks * 32);
+          epilogue_chunk16(st, e, r, bias_t + full_chunks * 32, own, colbase + full_chunks * 32);
         }
         tc_fence_before_sync();
         if constexpr (kPair) {                      // one arrival per warp on the leader's barrier (16 in all)
@@ -1105,7 +1008,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
       }
       if (g.nh == 1) rs.acc_bits ^= 4u;
     }
-    if (e.tm_out && elect_one()) {        // the stores are complete before the CTA reports the stage done
+    if (elect_one()) {        // the stores are complete before the CTA reports the stage done
       bulk_wait_group_all();
       fence_proxy_async_global();
     }
@@ -1712,8 +1615,10 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
 }
 
 // ------------------------------------------------------------------------------------
-// Swin window attention.  Q/K/V live window-major as [3][windows][64][C] with the heads side by side in C, so one box of
-// 128 rows x 64 columns holds two windows of a PAIR of 32-wide heads.  A work item is n consecutive windows x n heads:
+// Swin window attention.  The rows of Q, K and V, side by side in [tokens][3 C], and of the output are in the order of the block's
+// windows, win * win rows each, with the heads side by side in C.  Seen as [windows][win * win][columns], a box of 64 rows of one window x 64
+// columns of a PAIR of 32-wide heads is a tile whose rows past the window read as zero and are not written.  A work item is n
+// consecutive windows x n heads:
 // n = 2  group g of four softmax warps takes head 2 c + g; its upper 64 rows are the first window, the lower 64 the second,
 //        and every product is issued once per window (the rows of the other window in it are dropped), so all eight warps
 //        have rows of their own and a CTA has four (window, head) problems in flight;
@@ -1788,51 +1693,60 @@ __device__ __forceinline__ float swin_softmax_row(uint32_t tmem, const float* bi
 }
 
 __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, uint8_t* ring_ptr,
-                                uint8_t* stage_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
+                                uint8_t* boxes, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
   RoleState rs = RoleState::unpack(state);
   const int R = st.seq, ws = st.win, shift = st.shift, H = st.heads, C = st.ldo;
-  const int nwr = R / ws, nw_img = nwr * nwr, n_windows = st.batch * nw_img, n_tok = ws * ws;
+  const int nwr = st.nwr, nw_img = nwr * nwr, n_windows = st.batch * nw_img, n_tok = ws * ws;
   const uint32_t n = (uint32_t)st.bn;                                // windows and heads per item: 1 or 2
   const int item_h = H / (int)n, items = (n_windows + (int)n - 1) / (int)n * item_h;
+  auto wp_of = [&](int item) -> int { return (int)fast_div((uint32_t)item, (uint32_t)item_h, st.mg_heads); };
   // scores, probabilities and output have barriers per head (bar(g, ...)), the loads one set; all phases advance once per item
   const uint32_t bar0 = smem_u32(&ctl_s.qk_full), bar1 = smem_u32(&ctl_s.attn1[0]);
   auto bar = [&](int g, int which) -> uint32_t { return (g ? bar1 : bar0) + 8u * (uint32_t)which; };
   const uint32_t qk_full = bar(0, AB_QK_FULL), qk_empty = bar(0, AB_QK_EMPTY), v_full = bar(0, AB_V_FULL), v_empty = bar(0, AB_V_EMPTY);
-  const CUtensorMap* tm = map_ptr(ca, st.tm_qkv);
-  // shared memory: Q 16 KiB | K 16 KiB | V 16 KiB | P of head 0 16 KiB | P of head 1 16 KiB
+  // shared memory: Q 16 KiB | K 16 KiB | V 16 KiB | P of head 0 16 KiB | P of head 1 16 KiB | bias tables
   // TMEM: scores of (head g, window j) at column 64 (2 g + j), outputs 256 further on
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
+      const CUtensorMap* tm = map_ptr(ca, st.tm_qkv);
+      uint32_t bit = rs.attn_bit;
+      int wp = wp_of((int)blockIdx.x), col = (((int)blockIdx.x - wp * item_h) * (int)n >> 1) * 64;
       const bool ok = grid_wait(ca.p, ctl, st);
       if (ok && st.dead_bytes[0]) publish_go(ctl_s, st.ordinal);
-      for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
-        const int wp = item / item_h, w0 = wp * (int)n, col = ((item - wp * item_h) * (int)n >> 1) * 64;
-        if (!mbar_wait(qk_empty, rs.attn_bit ^ 1u, ctl, 530)) break;
-        mbar_expect_tx(qk_full, 2u * kATileBytes);
-        tma_load_2d(ring, tm, qk_full, col, (0 * n_windows + w0) * 64);
-        tma_load_2d(ring + kATileBytes, tm, qk_full, col, (1 * n_windows + w0) * 64);
-        if (!mbar_wait(v_empty, rs.attn_bit ^ 1u, ctl, 531)) break;
-        mbar_expect_tx(v_full, (uint32_t)kATileBytes);
-        tma_load_2d(ring + 2 * kATileBytes, tm, v_full, col, (2 * n_windows + w0) * 64);
-        rs.attn_bit ^= 1u;
+      for (int item = blockIdx.x; ok && item < items;) {
+        if (!mbar_wait_hot(qk_empty, bit ^ 1u, ctl, 530)) break;
+        mbar_expect_tx(qk_full, n * kATileBytes);                    // two tiles of n windows of 64 rows
+        tma_load_3d(ring, tm, qk_full, col, 0, wp * (int)n);
+        tma_load_3d(ring + kATileBytes, tm, qk_full, C + col, 0, wp * (int)n);
+        if (!mbar_wait_hot(v_empty, bit ^ 1u, ctl, 531)) break;
+        mbar_expect_tx(v_full, n * (kATileBytes / 2));
+        tma_load_3d(ring + 2 * kATileBytes, tm, v_full, 2 * C + col, 0, wp * (int)n);
+        bit ^= 1u;
+        item += gridDim.x;
+        wp = wp_of(item);
+        col = ((item - wp * item_h) * (int)n >> 1) * 64;
       }
+      rs.attn_bit = bit;
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc_s = umma_idesc_f16(64u, 0u), idesc_o = umma_idesc_f16(64u, 1u);
-      const uint32_t tmem = ctl_s.tmem_base;
+      const uint32_t tmem = ctl_s.tmem_base, q_lo = umma_desc_lo(ring, 16), k_lo = umma_desc_lo(ring + kATileBytes, 16);
+      const uint64_t hi = (uint64_t)kDescHiSw128 << 32;
+      uint32_t bit = rs.attn_bit;
       for (int item = blockIdx.x; item < items; item += gridDim.x) {
-        const uint32_t odd = n == 1 ? (uint32_t)(item % item_h) & 1u : 0u;       // a single head may be the pair's second
-        if (!mbar_wait(qk_full, rs.attn_bit, ctl, 532)) break;
+        const uint32_t odd = n == 1 ? (uint32_t)(item - wp_of(item) * item_h) & 1u : 0u;       // a single head may be the pair's second
+        if (!mbar_wait_hot(qk_full, bit, ctl, 532)) break;
         tc_fence_after_sync();
-        const uint64_t hi = (uint64_t)kDescHiSw128 << 32;
+#pragma unroll 1
         for (uint32_t g = 0; g < n; ++g) {
           // S[128 x 64] = Q_h K_h^T per window, K = 32: two K=16 steps; head g starts 64 bytes into every row, window j
           // 64 rows (8 KiB) into the K tile
-          const uint64_t qd = hi | (umma_desc_lo(ring, 16) + 4u * (g + odd));
+          const uint64_t qd = hi | (q_lo + 4u * (g + odd));
+#pragma unroll 1
           for (uint32_t j = 0; j < n; ++j) {
-            const uint64_t kd = hi | (umma_desc_lo(ring + kATileBytes + j * 8192u, 16) + 4u * (g + odd));
+            const uint64_t kd = hi | (k_lo + j * (8192u >> 4) + 4u * (g + odd));
             const uint32_t d = tmem + (2u * g + j) * 64u;
             umma_f16(d, qd, kd, idesc_s, 0u);
             umma_f16(d, qd + 2u, kd + 2u, idesc_s, 1u);
@@ -1840,13 +1754,15 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
           umma_commit(bar((int)g, AB_S_FULL));
         }
         umma_commit(qk_empty);
-        if (!mbar_wait(v_full, rs.attn_bit, ctl, 534)) break;
+        if (!mbar_wait_hot(v_full, bit, ctl, 534)) break;
         bool ok = true;
+#pragma unroll 1
         for (uint32_t g = 0; g < n; ++g) {
-          ok = mbar_wait(bar((int)g, AB_P_FULL), rs.attn_bit, ctl, 533);
+          ok = mbar_wait_hot(bar((int)g, AB_P_FULL), bit, ctl, 533);
           if (!ok) break;
           tc_fence_after_sync();
           // O[128 x 64] = P[128 x 64 keys] V_pair[64 keys x 64] per window: one K chunk of 64
+#pragma unroll 1
           for (uint32_t j = 0; j < n; ++j)
             umma_f16_k64(tmem + 256u + (2u * g + j) * 64u, umma_desc_lo(ring + (3u + g) * kATileBytes, 16),
                          umma_desc_lo(ring + 2 * kATileBytes + j * 8192u, 8192), 128u, idesc_o, 0u);
@@ -1854,8 +1770,9 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
         }
         if (!ok) break;
         umma_commit(v_empty);
-        rs.attn_bit ^= 1u;
+        bit ^= 1u;
       }
+      rs.attn_bit = bit;
     }
     __syncwarp();
   } else if (warp < 2 + (int)n * 4) {
@@ -1864,19 +1781,35 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(2 * grp + j) * 64u;
     const float sl2 = st.scale * 1.4426950408889634f, l2e = 1.4426950408889634f;
     const __half* table = reinterpret_cast<const __half*>(st.rel_bias);
-    __half* ctx = reinterpret_cast<__half*>(st.out);
-    const int tbl = 2 * ws - 1;
-    float* bias_s = reinterpret_cast<float*>(stage_s) + grp * 256;   // this head's column of the bias table (x log2 e): at most 225
+    const CUtensorMap* tm_out = map_ptr(ca, st.tm_out);
+    const int tbl2 = (2 * ws - 1) * (2 * ws - 1);                    // at most 225
+    float* bias_s = reinterpret_cast<float*>(ring_ptr + 5 * kATileBytes) + grp * 256;      // this head's column of the bias table (x log2 e)
     uint8_t* prow = ring_ptr + (3 + grp) * kATileBytes + r_in * 128;
+    StoreBoxes sb;
+    sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+    sb.box = 0;
+    sb.n = 2;
+    // the table's column of the next item is requested while this one is worked on
+    auto load_bias = [&](int i, int h) -> float { return i < tbl2 ? __half2float(__ldg(table + i * H + h)) * l2e : 0.0f; };
+    int wp = wp_of((int)blockIdx.x), h = (int)n * ((int)blockIdx.x - wp * item_h) + grp;
+    float b0 = 0.0f, b1 = 0.0f;
+    if ((int)blockIdx.x < items) { b0 = load_bias(r_in, h); b1 = load_bias(r_in + 128, h); }
     bool ok = true;                                                  // false: given up, see attn_stage
-    for (int item = blockIdx.x; item < items; item += gridDim.x) {
-      const int wp = item / item_h, h = (int)n * (item - wp * item_h) + grp;
-      const int wg = (int)n * wp + j, w = wg % nw_img;
+#pragma unroll 1
+    for (int item = blockIdx.x; item < items;) {
+      const int wg = (int)n * wp + j;
+      const int w = wg - (int)fast_div((uint32_t)wg, (uint32_t)nw_img, st.mg_nwr2) * nw_img;
       const bool live = j < (int)n && wg < n_windows;                // an odd number of windows: the last item has one
-      const int wy = (w / nwr) * ws, wx = (w % nwr) * ws;
+      const int wrow = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr), wy = wrow * ws, wx = (w - wrow * nwr) * ws;
       named_barrier_sync(2 + grp, 128);                              // previous item's readers are done with bias_s
-      for (int i = r_in; i < tbl * tbl; i += 128) bias_s[i] = __half2float(table[i * H + h]) * l2e;
+      bias_s[r_in] = b0;
+      bias_s[r_in + 128] = b1;
       named_barrier_sync(2 + grp, 128);
+      const int this_h = h;
+      item += gridDim.x;
+      wp = wp_of(item);
+      h = (int)n * (item - wp * item_h) + grp;
+      if (item < items) { b0 = load_bias(r_in, h); b1 = load_bias(r_in + 128, h); }
       ok = ok && mbar_wait_warp(bar(grp, AB_S_FULL), rs.attn_bit, ctl, 535, lane);
       tc_fence_after_sync();
       float sum = 1.0f;
@@ -1889,22 +1822,23 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
       ok = ok && mbar_wait_warp(bar(grp, AB_O_FULL), rs.attn_bit, ctl, 536, lane);
       tc_fence_after_sync();
       {
-        uint32_t o[32];
-        tmem_ld32(tmem + 256u + (uint32_t)(h & 1) * 32u, o);
+        uint32_t o[32], wv[16];
+        tmem_ld32(tmem + 256u + (uint32_t)(this_h & 1) * 32u, o);
         tmem_ld_wait(o);
-        if (ok && live && row < n_tok) {
-          uint4* dst = reinterpret_cast<uint4*>(ctx + ((size_t)wg * 64 + row) * C + h * 32);
 #pragma unroll
-          for (int i = 0; i < 4; ++i)
-            dst[i] = make_uint4(pack_h2(__uint_as_float(o[8 * i]) * inv, __uint_as_float(o[8 * i + 1]) * inv),
-                                pack_h2(__uint_as_float(o[8 * i + 2]) * inv, __uint_as_float(o[8 * i + 3]) * inv),
-                                pack_h2(__uint_as_float(o[8 * i + 4]) * inv, __uint_as_float(o[8 * i + 5]) * inv),
-                                pack_h2(__uint_as_float(o[8 * i + 6]) * inv, __uint_as_float(o[8 * i + 7]) * inv));
-        }
+        for (int i = 0; i < 16; ++i) wv[i] = pack_h2(__uint_as_float(o[2 * i]) * inv, __uint_as_float(o[2 * i + 1]) * inv);
+        store_box(sb, wv, lane, [&](uint32_t buf) {                   // (rows past the window are outside the map's extent)
+          if (ok && live && (q & 1) * 32 < n_tok) tma_store_3d(tm_out, buf, this_h * 32, (q & 1) * 32, wg);
+        });
       }
       tc_fence_before_sync();
       rs.attn_bit ^= 1u;
     }
+    if (elect_one()) {                     // the stores are complete before the CTA reports the stage done
+      bulk_wait_group_all();
+      fence_proxy_async_global();
+    }
+    __syncwarp();
   }
   return rs.pack();
 }
@@ -2066,6 +2000,38 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
   }
 }
 
+// Rows of Swin blocks change their order where a block's windows lie differently from those before: a LayerNorm stage writes row `row` to
+// the place that its token has in the order it leaves in (Stage::tok_grid), so that all products and the attention stage have rows that
+// are adjacent.  (When the products permuted, an epilogue took 1.9 k cycles per 32 columns, and windows of 49 tokens took 64 rows of
+// the projection.)  The divisors are host constants, so a quotient is one multiply-high.
+__device__ __forceinline__ int ln_out_row(const Stage& st, int row) {
+  const int R = st.tok_grid;
+  if (!R) return row;
+  const int win = st.win, nwr = st.nwr, n_tok = win * win;
+  int img, ty, tx;
+  if (st.shift < 0) {                      // rows come in the order of the tokens
+    img = st.mg_seq2 ? (int)__umulhi((uint32_t)row, st.mg_seq2) : row / (R * R);
+    const int t = row - img * R * R;
+    ty = (int)fast_div((uint32_t)t, (uint32_t)R, st.mg_seq);
+    tx = t - ty * R;
+  } else {
+    const int wg = (int)fast_div((uint32_t)row, (uint32_t)n_tok, st.mg_tok), pos = row - wg * n_tok;
+    img = (int)fast_div((uint32_t)wg, (uint32_t)(nwr * nwr), st.mg_nwr2);
+    const int w = wg - img * nwr * nwr, wy = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr);
+    const int py = (int)fast_div((uint32_t)pos, (uint32_t)win, st.mg_win);
+    ty = wy * win + py + st.shift;
+    tx = (w - wy * nwr) * win + (pos - py * win) + st.shift;
+    if (ty >= R) ty -= R;
+    if (tx >= R) tx -= R;
+  }
+  if (st.to_shift < 0) return (img * R + ty) * R + tx;
+  int sy = ty - st.to_shift, sx = tx - st.to_shift;
+  if (sy < 0) sy += R;
+  if (sx < 0) sx += R;
+  const int wy = (int)fast_div((uint32_t)sy, (uint32_t)win, st.mg_win), wx = (int)fast_div((uint32_t)sx, (uint32_t)win, st.mg_win);
+  return ((img * nwr + wy) * nwr + wx) * n_tok + (sy - wy * win) * win + (sx - wx * win);
+}
+
 // Rows read straight from L2.  W = N / 256 warps share a row (one for a row of 128 columns): lane l of part w holds columns
 // 256 w + 4 l .. + 3 and those 128 further on.  So 12 / W rows are in flight per CTA, dealt out over the CTAs first.  What a row
 // costs is latency: one L2 round trip for its planes, then a dependent chain in code that is cold when a CTA has one row, and
@@ -2075,6 +2041,7 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
 // from it), which is as exact as a second pass over the row (Chan, Golub, LeVeque) and needs one chain of shuffles and one
 // exchange between the parts.
 // `red`: 192 bytes of shared memory.
+template <bool kPermute>
 __device__ __forceinline__ void ln_shared_rows(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
   constexpr int NJ = 2, kG = 2;                           // blocks of 128 columns per warp, planes in flight at once
   const int N = st.N, M = st.M, P = st.n_partial, W = st.splitk, G = (kThreads / 32) / W;
@@ -2139,9 +2106,10 @@ __device__ __forceinline__ void ln_shared_rows(const Stage& st, const MegaParams
       load_planes(row, g0);
     }
     if (row + step < M) load_row(row + step);
-    __half* o = out + (size_t)row * N;
+    const size_t to = (size_t)(kPermute ? ln_out_row(st, row) : row) * N;
+    __half* o = out + to;
     if (eps < 0.0f || sum_out) {        // the sum itself, as fp16; what is normalised below is the rounded value
-      __half* so = eps < 0.0f ? o : sum_out + (size_t)row * N;
+      __half* so = eps < 0.0f ? o : sum_out + to;
 #pragma unroll
       for (int j = 0; j < NJ; ++j) {
         const uint2 w = make_uint2(pack_h2(z[j][0], z[j][1]), pack_h2(z[j][2], z[j][3]));
@@ -2338,7 +2306,7 @@ __device__ __forceinline__ void ln_lone_rows(const Stage& st, const MegaParams& 
 
 // The LayerNorm stages of the builds, out of line: their registers are not charged to the stage interpreter.
 __device__ __noinline__ void ln_stage_direct(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
-  ln_shared_rows(st, p, cs, red, ctl, warp, lane);
+  ln_shared_rows<true>(st, p, cs, red, ctl, warp, lane);
 }
 __device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p, SmemCtl& cs, const WaitCtl& ctl, int warp, int lane) {
   ln_lone_rows<0>(st, p, cs, ctl, warp, lane);
@@ -2350,7 +2318,7 @@ __device__ __noinline__ void ln_stage_many(const Stage& st, const MegaParams& p,
 // lone form for all widths would spill here.
 __device__ __noinline__ void ln_stage_either(const Stage& st, const MegaParams& p, SmemCtl& cs, float2* red, const WaitCtl& ctl, int warp, int lane) {
   if (st.N == 768 && st.M > 16 * (int)gridDim.x) ln_lone_rows<6>(st, p, cs, ctl, warp, lane);
-  else ln_shared_rows(st, p, cs, red, ctl, warp, lane);
+  else ln_shared_rows<false>(st, p, cs, red, ctl, warp, lane);
 }
 
 // The patch-merging form (Swin, python/models/swin_transformer/swin_patch_merge.py:1-17): the fp16 input is a
@@ -2465,7 +2433,7 @@ constexpr int kFamilyBert = 0, kFamilyBertCoop = 1, kFamilySwin = 2, kFamilyBert
 __device__ __noinline__ uint32_t gemm_stage_ool(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
                                             uint8_t* stage_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
   RoleState r = RoleState::unpack(state);
-  gemm_stage<true>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
+  gemm_stage<>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
   return r.pack();
 }
 // One warp copies a stage record to shared memory.
@@ -2577,13 +2545,13 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
       }
       if constexpr (kFamily == kFamilySwin) {
         if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
-        else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, stage_s, state, ctl, warp, lane);
+        else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, reinterpret_cast<uint8_t*>(vec_s), state, ctl, warp, lane);
         else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
         else if (st.type == STAGE_LN) state = ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, state, ctl, warp, lane);
       } else {
         if (st.type == STAGE_GEMM) {
           RoleState rs = RoleState::unpack(state);
-          gemm_stage<false, kFamily == kFamilyBertPair, kFamily != kFamilyBertCoop>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
+          gemm_stage<kFamily == kFamilyBertPair, kFamily != kFamilyBertCoop>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
           state = rs.pack();
         } else if (st.type == STAGE_ATTN) {
           RoleState rs = RoleState::unpack(state);

@@ -145,6 +145,22 @@ static int make_plane_map_uncached(CUtensorMap* m, const void* ptr, uint64_t pla
   if (r != CUDA_SUCCESS) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled (planes) failed with CUresult %d", (int)r);
   return SOUFFLE_OK;
 }
+// fp16 rows of windows, [windows][rows][cols]: box = box_cols columns x box_rows rows x box_windows windows; rows past a window's read as
+// zero and are not written.
+static int make_window_map(CUtensorMap* m, const void* ptr, uint64_t windows, uint64_t rows, uint64_t cols, uint32_t box_cols, uint32_t box_rows,
+                           uint32_t box_windows, CUtensorMapSwizzle swizzle) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled is not available from the driver");
+  if (!aligned16(ptr) || (cols * 2) % 16 != 0) return fail(SOUFFLE_BAD_POINTER, "tensor map needs 16-byte alignment");
+  cuuint64_t dims[3] = {cols, rows, windows};
+  cuuint64_t strides[2] = {cols * 2, rows * cols * 2};
+  cuuint32_t box[3] = {box_cols, box_rows, box_windows};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(SOUFFLE_CUDA_ERROR, "cuTensorMapEncodeTiled (windows) failed with CUresult %d", (int)r);
+  return SOUFFLE_OK;
+}
 static int make_plane_map(CUtensorMap* m, const void* ptr, uint64_t planes, uint64_t rows, uint64_t cols) {
   return make_map_cached(m, ptr, rows, cols, (uint32_t)planes, MAP_PLANES);
 }
@@ -230,7 +246,6 @@ static TileChoice choose_tiles(int M, int N, int K, int sms, bool allow_split, b
       if (N % bn) continue;
       if (b_mn && bn % 64) continue;
       if (head_split == 1 && bn != 16 && bn % 32) continue;   // 32-column epilogue chunks must not straddle a head
-      if (head_split == 2 && bn % 32) continue;               // row-permuting epilogues have no 16-column path
       if (196608 / ((bm + bn) * 128) < 2) continue;
       for (int split = 1; split <= (allow_split ? 16 : 1); ++split) {
         if (kch % split) continue;
@@ -442,12 +457,26 @@ static int stage_items(const Stage& s, bool pair = false) {
   return s.M;       // rows are dealt out over the CTAs first
 }
 
+// What the row maps of a Swin block divide by, for a grid of R x R tokens in M / (R * R) images.
+static void window_divisors(Stage* s, int R) {
+  s->nwr = R / s->win;
+  // a token grid too large for an exact 32-bit multiplier (from 256 x 256 tokens on) is divided plainly
+  const unsigned long long grid_tokens = (unsigned long long)R * R;
+  s->mg_seq2 = s->M * grid_tokens < (1ull << 32) ? fast_div_magic((uint32_t)grid_tokens) : 0u;
+  s->mg_seq = fast_div_magic((uint32_t)R);
+  s->mg_win = fast_div_magic((uint32_t)s->win);
+  s->mg_nwr = fast_div_magic((uint32_t)s->nwr);
+  s->mg_nwr2 = fast_div_magic((uint32_t)(s->nwr * s->nwr));
+  s->mg_tok = fast_div_magic((uint32_t)(s->win * s->win));
+}
+
 // Fills the derived fields of a GEMM stage (tile counts, ring geometry, magic divisors) and checks that its
 // output fits the kernel's 32-bit element offsets.
 static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) {
   if (s.type == STAGE_LN) {
     // Rows that need no gather: the warps read them from L2 themselves (nslots = 0), s.splitk warps per row where rows are shared
     // (ln_shared_rows).
+    if (s.tok_grid) window_divisors(&s, s.tok_grid);
     if (s.seq == 0) {
       s.splitk = s.N <= 256 ? 1 : s.N / 256;
       s.mg_splitk = fast_div_magic((uint32_t)s.splitk);
@@ -473,21 +502,18 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   }
   if (s.type == STAGE_ATTN_SWIN) {
     // The extents the window-attention stage relies on: a window's tokens fit the 64 rows of its Q/K/V/P tiles,
-    // one head's column of the relative-position table fits the staging area as fp32, the two heads of a
-    // 64-column pair exist, and the window-major buffers hold whole 64-row windows.
+    // one head's column of the relative-position table fits its 256 words, and the two heads of a 64-column pair exist.
     const int tbl = 2 * s.win - 1;
-    if (s.win < 1 || s.win * s.win > 64 || s.seq % s.win || tbl * tbl * 4 > kStageBytes || s.head_dim != 32 || (s.heads & 1) ||
+    if (s.win < 1 || s.win * s.win > 64 || s.seq % s.win || tbl * tbl > 256 || s.head_dim != 32 || (s.heads & 1) ||
         s.heads * 32 != s.ldo || s.shift < 0 || s.shift >= s.win)
       return fail(SOUFFLE_BAD_SHAPE, "window attention: window %d, grid %d, heads %d, row length %d are outside what the stage addresses",
                   s.win, s.seq, s.heads, s.ldo);
+    window_divisors(&s, s.seq);
+    s.mg_heads = fast_div_magic((uint32_t)(s.heads / s.bn));
     return SOUFFLE_OK;
   }
   s.mg_heads = fast_div_magic((uint32_t)(s.heads > 0 ? s.heads : 1));
   if (s.type != STAGE_GEMM) return SOUFFLE_OK;
-  if ((s.epi == EPI_SWIN_QKV || s.epi == EPI_SWIN_PROJ) &&
-      (s.win < 1 || s.win * s.win > 64 || s.seq % s.win || s.heads * 32 != s.ldo ||
-       s.M != (s.epi == EPI_SWIN_QKV ? s.batch * s.seq * s.seq : s.batch * (s.seq / s.win) * (s.seq / s.win) * 64)))
-    return fail(SOUFFLE_BAD_SHAPE, "window-major epilogue: %d rows do not match batch %d, grid %d, window %d", s.M, s.batch, s.seq, s.win);
   if (s.bias && s.epi != EPI_PARTIAL && s.N > 4096)
     return fail(SOUFFLE_BAD_SHAPE, "a GEMM stage with a bias vector is limited to 4096 output columns (got %d)", s.N);
   s.tiles_n = s.N / s.bn;
@@ -512,19 +538,9 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   s.mg_kchunks = fast_div_magic((uint32_t)s.kchunks);
   s.mg_seq = fast_div_magic((uint32_t)(s.seq > 0 ? s.seq : 1));
   s.mg_head_dim = fast_div_magic((uint32_t)(s.head_dim > 0 ? s.head_dim : 1));
-  if (s.epi == EPI_SWIN_QKV || s.epi == EPI_SWIN_PROJ) {
-    s.nwr = s.seq / s.win;
-    s.plane_elems = (uint32_t)s.batch * (uint32_t)(s.nwr * s.nwr * 64) * (uint32_t)s.ldo;
-    // a token grid too large for an exact 32-bit multiplier (from 256 x 256 tokens on) is divided plainly
-    const unsigned long long grid_tokens = (unsigned long long)s.seq * s.seq;
-    s.mg_seq2 = s.M * grid_tokens < (1ull << 32) ? fast_div_magic((uint32_t)grid_tokens) : 0u;
-    s.mg_win = fast_div_magic((uint32_t)s.win);
-    s.mg_nwr = fast_div_magic((uint32_t)s.nwr);
-    s.mg_nwr2 = fast_div_magic((uint32_t)(s.nwr * s.nwr));
-  }
   const unsigned long long out_elems = (unsigned long long)s.M * (unsigned long long)s.N * (s.epi == EPI_PARTIAL ? s.splitk : 1);
   // 2^20 rows keep every multiply-high division exact (numerator * divisor < 2^32)
-  if (s.M > (1 << 20) || out_elems * (s.epi == EPI_SWIN_QKV ? 2 : 1) >= 0xFFFF0000ull || (long long)s.items * 16 >= (1ll << 32))
+  if (s.M > (1 << 20) || out_elems >= 0xFFFF0000ull || (long long)s.items * 16 >= (1ll << 32))
     return fail(SOUFFLE_BAD_SHAPE, "GEMM stage %d x %d (split %d) is too large for 32-bit output offsets", s.M, s.N, s.splitk);
   return SOUFFLE_OK;
 }
@@ -1727,37 +1743,42 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
   p->device = di->device;
   const int sms = di->sms < di->max_ctas ? di->sms : di->max_ctas;
   const int R = d.res, C = d.dim, Hh = d.heads, ws = d.window, F = C * d.mlp_ratio;
-  const int T = d.batch * R * R, nWt = d.batch * (R / ws) * (R / ws), Mw = nWt * 64;
+  const int T = d.batch * R * R, nWt = d.batch * (R / ws) * (R / ws), n_tok = ws * ws;
   const int n_blocks = d.n_blocks > 0 ? d.n_blocks : 1;
-  // FC2 has few output tiles and the longest K of the block: it is cut along K into fp32 planes, and a sum-only
-  // LayerNorm stage adds them, the bias and the residual (the block's output).
-  const TileChoice t_qkv = choose_tiles(T, 3 * C, C, sms, false, false, 2), t_proj = choose_tiles(Mw, C, C, sms, false, false, 2),
+  // proj and FC2 are cut along K into fp32 planes, which the LayerNorm stage behind them adds up together with bias and residual
+  const TileChoice t_qkv = choose_tiles(T, 3 * C, C, sms, false, false, 0), t_proj = choose_tiles(T, C, C, sms, true, false, 0),
                    t_fc1 = choose_tiles(T, F, C, sms, false, false, 0), t_fc2 = choose_tiles(T, C, F, sms, true, false, 0);
-  // activations, shared by all blocks of the chain (stages run one after the other)
-  __half *y1, *qkvw, *ctxw, *x1, *y2, *hid, *xbuf[2] = {nullptr, nullptr};
+  // Activations, shared by all blocks of the chain (stages run one after the other).  Inside a block all rows are in the order of its
+  // windows (see ln_out_row); x is the block's input, x1 the sum of its attention half.
+  __half *y1, *qkv, *ctx, *x, *x1, *y2, *hid;
   float* planes;
   if ((rc = plan_alloc(p, (void**)&y1, (size_t)T * C * 2))) return rc;
-  if ((rc = plan_alloc(p, (void**)&qkvw, (size_t)3 * Mw * C * 2))) return rc;
-  if ((rc = plan_alloc(p, (void**)&ctxw, (size_t)Mw * C * 2))) return rc;
+  if ((rc = plan_alloc(p, (void**)&qkv, (size_t)3 * T * C * 2))) return rc;
+  if ((rc = plan_alloc(p, (void**)&ctx, (size_t)T * C * 2))) return rc;
+  if ((rc = plan_alloc(p, (void**)&x, (size_t)T * C * 2))) return rc;
   if ((rc = plan_alloc(p, (void**)&x1, (size_t)T * C * 2))) return rc;
   if ((rc = plan_alloc(p, (void**)&y2, (size_t)T * C * 2))) return rc;
   if ((rc = plan_alloc(p, (void**)&hid, (size_t)T * F * 2))) return rc;
-  if ((rc = plan_alloc(p, (void**)&planes, (size_t)t_fc2.split * T * C * 4))) return rc;
-  for (int i = 0; i < 2 && i < n_blocks - 1; ++i)
-    if ((rc = plan_alloc(p, (void**)&xbuf[i], (size_t)T * C * 2))) return rc;
+  if ((rc = plan_alloc(p, (void**)&planes, (size_t)(t_fc2.split > t_proj.split ? t_fc2.split : t_proj.split) * T * C * 4))) return rc;
   __half* xlast = nullptr;          // output of the last block when patch merging follows inside the launch
   if (sp->has_merge && (rc = plan_alloc(p, (void**)&xlast, (size_t)T * C * 2))) return rc;
   if ((rc = plan_alloc(p, (void**)&p->d_sync, 64))) return rc;
   if ((rc = plan_alloc(p, (void**)&p->d_status, 64))) return rc;
   SF_CUDA(cudaMemset(p->d_sync, 0, 64));
   SF_CUDA(cudaMemset(p->d_status, 0, 64));
-  SF_CUDA(cudaMemset(qkvw, 0, (size_t)3 * Mw * C * 2));     // padding slots stay zero for ever
-  SF_CUDA(cudaMemset(ctxw, 0, (size_t)Mw * C * 2));
+  const int attn_n = nWt * Hh <= sms ? 1 : 2;             // windows and heads per item, see attn_swin_stage
   int m_y1, m_ctx, m_y2, m_hid, m_qkv;
-  if ((rc = add_map(p, y1, T, C, t_qkv.bm, &m_y1)) || (rc = add_map(p, ctxw, Mw, C, t_proj.bm, &m_ctx)) ||
-      (rc = add_map(p, y2, T, C, t_fc1.bm, &m_y2)) || (rc = add_map(p, hid, T, F, t_fc2.bm, &m_hid)) ||
-      (rc = add_map(p, qkvw, (uint64_t)3 * Mw, C, 128, &m_qkv)))
+  CUtensorMap ctx_out;
+  if ((rc = add_map(p, y1, T, C, t_qkv.bm, &m_y1)) || (rc = add_map(p, ctx, T, C, t_proj.bm, &m_ctx)) ||
+      (rc = add_map(p, y2, T, C, t_fc1.bm, &m_y2)) || (rc = add_map(p, hid, T, F, t_fc2.bm, &m_hid)))
     return rc;
+  {
+    CUtensorMap m;
+    if ((rc = make_window_map(&m, qkv, nWt, n_tok, 3 * C, 64, 64, attn_n, CU_TENSOR_MAP_SWIZZLE_128B))) return rc;
+    m_qkv = (int)p->maps.size();
+    p->maps.push_back(m);
+    if ((rc = make_window_map(&ctx_out, ctx, nWt, n_tok, C, 32, 32, 1, CU_TENSOR_MAP_SWIZZLE_64B))) return rc;
+  }
   auto copy_vec = [&](const void* src, size_t n, const void** dst) -> int {
     *dst = nullptr;
     if (!src) return SOUFFLE_OK;
@@ -1799,41 +1820,44 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     if ((rc = add_map(p, wqkv_t, 3 * C, C, t_qkv.bn, &m_wqkv)) || (rc = add_map(p, wo_t, C, C, t_proj.bn, &m_wo)) ||
         (rc = add_map(p, w1_t, F, C, t_fc1.bn, &m_w1)) || (rc = add_map(p, w2_t, C, F, t_fc2.bn, &m_w2)))
       return rc;
-    // the block's input (also the residual of its attention half) and output
-    const int in_sel = bi == 0 ? PTR_CALL_X : PTR_PLAN;
-    const __half* xin = bi == 0 ? nullptr : xbuf[(bi - 1) & 1];
     const bool last = bi == n_blocks - 1;
+    // rows of a stage that leave in another order
+    auto reorder = [&](Stage* st, int from, int to) {
+      if (from == to) return;
+      st->tok_grid = R; st->win = ws; st->shift = from; st->to_shift = to;
+    };
 
-    // LN1(x): a stage of its own in the first block; later ones normalise the rows in the stage that adds up the block
-    // before (one grid barrier and one pass over x less per block)
     Stage s = blank_stage(STAGE_LN);
-    s.M = T; s.N = C; s.ldo = C; s.n_partial = 0; s.resid_sel = in_sel; s.resid = xin; s.out = y1; s.gamma = ln1_g; s.beta = ln1_b;
-    s.eps = d.eps;
-    if (bi == 0) {
+    if (bi == 0) {                                         // LN1(x) and x in the order of the first block's windows
+      s.M = T; s.N = C; s.ldo = C; s.n_partial = 0; s.resid_sel = PTR_CALL_X; s.sum_out = x; s.out = y1; s.gamma = ln1_g; s.beta = ln1_b;
+      s.eps = d.eps;
+      reorder(&s, -1, shift);
       p->stages.push_back(s);
-    } else {
+    } else {       // later blocks' rows are normalised by the stage that adds up the block before (one barrier and one pass over x less)
       Stage& sum = p->stages.back();
-      sum.sum_out = sum.out;
+      sum.sum_out = x;
       sum.out = y1; sum.gamma = ln1_g; sum.beta = ln1_b; sum.eps = d.eps;
     }
-    s = blank_stage(STAGE_GEMM);                           // QKV, rolled and scattered window-major
-    s.tm_a = m_y1; s.tm_b = m_wqkv; s.M = T; s.N = 3 * C; s.K = C; s.bm = t_qkv.bm; s.bn = t_qkv.bn; s.epi = EPI_SWIN_QKV;
-    s.bias = qkv_b; s.out = qkvw; s.ldo = C; s.batch = d.batch; s.heads = Hh; s.head_dim = 32; s.seq = R; s.win = ws; s.shift = shift;
+    s = blank_stage(STAGE_GEMM);                           // QKV
+    s.tm_a = m_y1; s.tm_b = m_wqkv; s.M = T; s.N = 3 * C; s.K = C; s.bm = t_qkv.bm; s.bn = t_qkv.bn; s.epi = EPI_F16;
+    s.bias = qkv_b; s.out = qkv; s.ldo = 3 * C;
+    if ((rc = add_f16_out_map(p, s))) return rc;
     p->stages.push_back(s);
     note_weights(p, wqkv_t);
     s = blank_stage(STAGE_ATTN_SWIN);                      // window attention
-    s.tm_qkv = m_qkv; s.batch = d.batch; s.heads = Hh; s.head_dim = 32; s.seq = R; s.win = ws; s.shift = shift; s.ldo = C;
-    s.scale = 1.0f / sqrtf(32.0f); s.rel_bias = relb; s.out = ctxw;
-    s.bn = nWt * Hh <= sms ? 1 : 2;                        // windows and heads per item, see attn_swin_stage
+    s.tm_qkv = m_qkv; s.batch = d.batch; s.heads = Hh; s.head_dim = 32; s.seq = R; s.win = ws; s.shift = shift; s.ldo = C; s.M = T;
+    s.scale = 1.0f / sqrtf(32.0f); s.rel_bias = relb; s.bn = attn_n;
+    if ((rc = set_store_map(p, s, ctx_out, 1))) return rc;
     p->stages.push_back(s);
-    s = blank_stage(STAGE_GEMM);                           // proj, window reverse, roll back, + x
-    s.tm_a = m_ctx; s.tm_b = m_wo; s.M = Mw; s.N = C; s.K = C; s.bm = t_proj.bm; s.bn = t_proj.bn; s.epi = EPI_SWIN_PROJ;
-    s.bias = proj_b; s.resid_sel = in_sel; s.resid = xin; s.out = x1; s.ldo = C; s.batch = d.batch; s.heads = Hh; s.head_dim = 32;
-    s.seq = R; s.win = ws; s.shift = shift;
+    s = blank_stage(STAGE_GEMM);                           // proj -> fp32 planes
+    s.tm_a = m_ctx; s.tm_b = m_wo; s.M = T; s.N = C; s.K = C; s.bm = t_proj.bm; s.bn = t_proj.bn; s.splitk = t_proj.split;
+    s.epi = EPI_PARTIAL; s.partial = planes; s.ldo = C;
+    if ((rc = add_plane_map(p, s))) return rc;
     p->stages.push_back(s);
     note_weights(p, wo_t);
-    s = blank_stage(STAGE_LN);                             // LN2(x1)
-    s.M = T; s.N = C; s.ldo = C; s.n_partial = 0; s.resid = x1; s.out = y2; s.gamma = ln2_g; s.beta = ln2_b; s.eps = d.eps;
+    s = blank_stage(STAGE_LN);                             // x1 = planes + bias + x, LN2(x1)
+    s.M = T; s.N = C; s.ldo = C; s.partial = planes; s.n_partial = (uint8_t)t_proj.split; s.bias = proj_b; s.resid = x; s.sum_out = x1;
+    s.out = y2; s.gamma = ln2_g; s.beta = ln2_b; s.eps = d.eps;
     p->stages.push_back(s);
     s = blank_stage(STAGE_GEMM);                           // FC1 + GELU
     s.tm_a = m_y2; s.tm_b = m_w1; s.M = T; s.N = F; s.K = C; s.bm = t_fc1.bm; s.bn = t_fc1.bn; s.epi = EPI_F16; s.act = ACT_GELU;
@@ -1848,8 +1872,9 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     p->stages.push_back(s);
     note_weights(p, w2_t);
     s = blank_stage(STAGE_LN);                             // planes + bias + x1 -> block output (no normalisation)
-    s.M = T; s.N = C; s.ldo = C; s.partial = planes; s.n_partial = t_fc2.split; s.bias = fc2_b; s.resid = x1; s.eps = -1.0f;
-    if (last && !sp->has_merge) s.out_sel = PTR_CALL_Y; else s.out = last ? xlast : xbuf[bi & 1];
+    s.M = T; s.N = C; s.ldo = C; s.partial = planes; s.n_partial = (uint8_t)t_fc2.split; s.bias = fc2_b; s.resid = x1; s.eps = -1.0f;
+    if (last && !sp->has_merge) s.out_sel = PTR_CALL_Y; else s.out = xlast;
+    reorder(&s, shift, last ? -1 : ((bi + 1) & 1) ? d.shift_alt : d.shift);
     p->stages.push_back(s);
   }
   if (sp->has_merge) {

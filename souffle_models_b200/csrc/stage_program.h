@@ -21,9 +21,7 @@ enum EpilogueKind : int {
   EPI_F16 = 0,      // out[row, col] = f16(act(acc + bias)) (+ resid)
   EPI_QKV = 1,      // like EPI_F16 but scattered head-split to [3][B][heads][S][d]
   EPI_PARTIAL = 2,  // raw fp32 accumulators to partial[split][row][col]
-  EPI_SWIN_QKV = 3, // rows (tokens) are rolled by -shift and scattered window-major: [3][windows][64][C]
-  EPI_SWIN_PROJ = 4,// rows arrive window-major, are rolled back to token order; + bias + residual[token]
-  EPI_LN = 5,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it
+  EPI_LN = 3,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it
 };
 
 enum Activation : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2 };
@@ -48,7 +46,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   int tm_out;        // with out_stores: tensor-map index of the output, 64B swizzle.  EPI_PARTIAL: the fp32 planes as
                      // [splitk][M][N], box 16 columns x 32 rows x 1 plane; EPI_F16: [M][N], box 32 x 32; EPI_QKV: [3 B heads S][d],
                      // box 32 columns x 32 / out_stores rows
-  int out_stores;    // copies per box of 32 rows (2 where a sequence ends inside one); 0: the row-permuting epilogues' plain stores
+  int out_stores;    // copies per box of 32 rows (2 where a sequence ends inside one)
   int M, N, K;
   int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile); STAGE_ATTN: query rows per item
   int bn;            // tile width in N (multiple of 16, <= 256, divides N)
@@ -68,8 +66,14 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   };
   // ---- attention / head split ----
   int batch, heads, seq, head_dim;
-  float scale;       // softmax scale applied to Q.K
-  int tm_qkv;        // tensor map over the head-split buffer viewed as [3*B*heads*S][d], box 64 x 128
+  union {
+    float scale;     // softmax scale applied to Q.K
+    int to_shift;    // STAGE_LN of a Swin block, see tok_grid
+  };
+  union {
+    int tm_qkv;      // tensor map over the head-split buffer viewed as [3*B*heads*S][d], box 64 x 128; Swin: see attn_swin_stage
+    int tok_grid;    // STAGE_LN: 0, or the side of the token grid whose rows leave in another order than they come in: in the order of the
+  };                 // windows of `win` x `win` tokens after a shift, to_shift and `shift`, or in that of the tokens (-1)
   union {
     struct { int win, shift; };        // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
     struct { int tm_resid, tm_unit; }; // EPI_LN: tensor maps of the residual ([M][N], box 64 x bm) and of the unit matrix ([64][64])
@@ -101,10 +105,10 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   int tiles_n, kchunks, kper, items, slot_bytes, nslots;   // a K chunk: kper steps of 64
   uint32_t mg_splitk, mg_tiles_n, mg_kchunks;   // magic multipliers, see fast_div()
   uint32_t mg_seq, mg_head_dim, mg_heads;
-  // Swin row maps: windows per side of the grid, elements of one of the Q / K / V planes, and the multipliers of the
-  // divisors seq * seq (0: divide plainly), win, nwr and nwr * nwr
+  // Swin row maps: windows per side of the grid, and the multipliers of the divisors grid * grid (0: divide plainly), win, nwr,
+  // nwr * nwr and win * win
   int nwr;
-  uint32_t plane_elems, mg_seq2, mg_win, mg_nwr, mg_nwr2;
+  uint32_t mg_seq2, mg_win, mg_nwr, mg_nwr2, mg_tok;
 };
 
 // q = n / d for n * d < 2^32 as one multiply-high: mg = ceil(2^32 / d); d == 1 has no 32-bit multiplier.
