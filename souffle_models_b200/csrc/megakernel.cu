@@ -402,6 +402,38 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
   d4[1] = make_uint4(pack_h2(v[8], v[9]), pack_h2(v[10], v[11]), pack_h2(v[12], v[13]), pack_h2(v[14], v[15]));
 }
 
+// Rows of Swin blocks change their order where a block's windows lie differently from those before: a LayerNorm stage writes row `row` to
+// the place that its token has in the order it leaves in (Stage::tok_grid), so that all products and the attention stage have rows that
+// are adjacent.  (When the products permuted, an epilogue took 1.9 k cycles per 32 columns, and windows of 49 tokens took 64 rows of
+// the projection.)  The divisors are host constants, so a quotient is one multiply-high.
+__device__ __forceinline__ int ln_out_row(const Stage& st, int row) {
+  const int R = st.tok_grid;
+  if (!R) return row;
+  const int win = st.win, nwr = st.nwr, n_tok = win * win;
+  int img, ty, tx;
+  if (st.shift < 0) {                      // rows come in the order of the tokens
+    img = st.mg_seq2 ? (int)__umulhi((uint32_t)row, st.mg_seq2) : row / (R * R);
+    const int t = row - img * R * R;
+    ty = (int)fast_div((uint32_t)t, (uint32_t)R, st.mg_seq);
+    tx = t - ty * R;
+  } else {
+    const int wg = (int)fast_div((uint32_t)row, (uint32_t)n_tok, st.mg_tok), pos = row - wg * n_tok;
+    img = (int)fast_div((uint32_t)wg, (uint32_t)(nwr * nwr), st.mg_nwr2);
+    const int w = wg - img * nwr * nwr, wy = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr);
+    const int py = (int)fast_div((uint32_t)pos, (uint32_t)win, st.mg_win);
+    ty = wy * win + py + st.shift;
+    tx = (w - wy * nwr) * win + (pos - py * win) + st.shift;
+    if (ty >= R) ty -= R;
+    if (tx >= R) tx -= R;
+  }
+  if (st.to_shift < 0) return (img * R + ty) * R + tx;
+  int sy = ty - st.to_shift, sx = tx - st.to_shift;
+  if (sy < 0) sy += R;
+  if (sx < 0) sx += R;
+  const int wy = (int)fast_div((uint32_t)sy, (uint32_t)win, st.mg_win), wx = (int)fast_div((uint32_t)sx, (uint32_t)win, st.mg_win);
+  return ((img * nwr + wy) * nwr + wx) * n_tok + (sy - wy * win) * win + (sx - wx * win);
+}
+
 // LayerNorm in the epilogue of a product whose K is not cut: out = LayerNorm(acc + bias + residual) without a plane in memory and
 // without a stage of its own.  A row's columns lie in tiles_n tiles of as many CTAs (or pairs), all of which are running or have run:
 // items are dealt out in order, every CTA takes its own in order, and a CTA has at most one tile of a row block (the host checks that
@@ -415,8 +447,10 @@ __device__ __forceinline__ void epilogue_chunk16(const Stage& st, const EpiCtx& 
 //   3. A thread reads the pairs of all of its row's tiles (bounded), normalises the sums and stores fp16 rows as boxes.
 // Out of line: its registers are not charged to the other stages.  Few arguments: they have to live beside the caller's values.
 // `acc_bits`: see RoleState; bit 31: the stage's record is the second one.
-template <bool kPair>
-__device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) {
+// kSwin: the sum leaves as well, rounded to fp16, which is then what gets normalised (or leaves alone: eps < 0), and rows may leave in
+// another order; such stores are plain ones.
+template <bool kPair, bool kSwin>
+__device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint32_t acc_bits) {
   SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw);
   const Stage& st = cs.stage[acc_bits >> 31];
   acc_bits &= 7u;
@@ -431,14 +465,26 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
   const uint32_t tfull0 = smem_u32(&cs.tmem_full[0]), tempty0 = smem_u32(&cs.tmem_empty[0]);
   const uint32_t tmem = cs.tmem_base + ((uint32_t)(q * 32) << 16);
   const CUtensorMap* tm_out = map_ptr(ca, st.tm_out);
+  const bool sum_only = kSwin && st.eps < 0.0f;
+  // plain stores: offset of output row row0 + lane; a lane's rows of the staged pieces are other lanes' (see staged_store_64B)
+  auto out_row = [&](int row0) -> uint32_t { return row0 + lane < M ? (uint32_t)ln_out_row(st, row0 + lane) * (uint32_t)st.ldo : kNoRow; };
+  auto store_rows = [&](uint8_t* sbuf, __half* to, uint32_t own, int col, const uint32_t (&w)[16]) {
+    uint32_t so[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) so[i] = __shfl_sync(0xffffffffu, own, 8 * i + (lane >> 2));
+    uint8_t* rowptr[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) rowptr[i] = so[i] != kNoRow ? reinterpret_cast<uint8_t*>(to + (so[i] + (uint32_t)col)) : nullptr;
+    staged_store_64B(sbuf, w, rowptr, lane);
+  };
   const uint32_t tag = (cs.epoch << 8) | st.ordinal;
   const float inv_n = 1.0f / (float)st.N;
   const bool prof = p.prof != nullptr, affine = st.gamma != nullptr;
   float* bias_s = cs.bias[0];
   __half* gamma_s = reinterpret_cast<__half*>(cs.bias[1]);          // gamma of the tile's columns, then beta
-  // statistics of the warps that have the other chunks of these rows, in their boxes (written again only once all tiles of the row
-  // have been published, and so after they have been read)
-  float2* other = reinterpret_cast<float2*>(boxes + (4 + q) * 2 * kStageWarp);
+  // statistics of the warps that have the other chunks of these rows, in their second boxes (written again only once all tiles of the
+  // row have been published, and so after they have been read; plain stores pass through the first)
+  float2* other = reinterpret_cast<float2*>(boxes + ((4 + q) * 2 + 1) * kStageWarp);
   StoreBoxes sb;
   sb.base = boxes + (warp - 2) * 2 * kStageWarp;
   sb.box = 0;
@@ -478,6 +524,7 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
       if (prof && item == first_item && h == 0 && warp == 2 && lane == 0)
         p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + 14] = clock64();
       float mean = 0.0f, dev = 0.0f, sets = 0.0f;                    // of `sets` chunks of 32 columns
+      const uint32_t own = kSwin ? out_row(row0) : 0u;
 #pragma unroll 1
       for (int c = cpar; c < chunks; c += 2) {
         uint32_t r[32];
@@ -490,9 +537,23 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
           const float4 bb = b4[i];
           const float z0 = __uint_as_float(r[4 * i]) + bb.x, z1 = __uint_as_float(r[4 * i + 1]) + bb.y;
           const float z2 = __uint_as_float(r[4 * i + 2]) + bb.z, z3 = __uint_as_float(r[4 * i + 3]) + bb.w;
-          sum[0] += z0; sum[1] += z1; sum[2] += z2; sum[3] += z3;
+          if constexpr (!kSwin) { sum[0] += z0; sum[1] += z1; sum[2] += z2; sum[3] += z3; }
           r[4 * i] = __float_as_uint(z0); r[4 * i + 1] = __float_as_uint(z1);
           r[4 * i + 2] = __float_as_uint(z2); r[4 * i + 3] = __float_as_uint(z3);
+        }
+        if constexpr (kSwin) {
+          uint32_t w[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) w[i] = pack_h2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          if (ok) store_rows(sb.base, reinterpret_cast<__half*>(sum_only ? const_cast<void*>(sel_ptr(st.out_sel, st.out, p)) : st.sum_out), own, colbase + c * 32, w);
+          if (sum_only) continue;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
+            r[2 * i] = __float_as_uint(f.x);
+            r[2 * i + 1] = __float_as_uint(f.y);
+            sum[i & 3] += f.x + f.y;
+          }
         }
         tmem_st32(t0 + c * 32, r);
         const float cm = ((sum[0] + sum[1]) + (sum[2] + sum[3])) * (1.0f / 32.0f);
@@ -507,6 +568,7 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
         mean = fmaf(d, w, mean);
         sets += 1.0f;
       }
+      if (sum_only) continue;
       tmem_st_wait();
       if (chunks > 1) {
         if (cpar == 1) other[h * 32 + lane] = make_float2(mean, dev);
@@ -522,16 +584,20 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
         st_relaxed_2x64(st.stats + ((size_t)(row0 >> 5) * tiles_n + nt) * 32 + lane, (uint64_t)__float_as_uint(mean) | ((uint64_t)tag << 32),
                         (uint64_t)__float_as_uint(dev) | ((uint64_t)tag << 32));
     }
+    // the second half's statistics have been read before the first half's boxes go over them (the first half's have been read before they
+    // are published)
+    if (nh == 2) named_barrier_sync(4 + q, 64);
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
       const uint32_t acc = acc0 + (uint32_t)h, t0 = tmem + acc * kAccStride;
       const int row0 = mt * st.bm + (kPair ? (int)rank : h) * 128 + q * 32;
       float mean = 0.0f, dev = 0.0f;
+      const uint32_t own = kSwin && st.tok_grid ? out_row(row0) : 0u;
       const RowStat* from = st.stats + (size_t)(row0 >> 5) * tiles_n * 32 + lane;
       uint32_t spins = 0;
 #pragma unroll 1
-      for (int s0 = 0; ok && s0 < tiles_n;) {
-        constexpr int kG = 4;                                        // tiles whose pairs are on their way at once
+      for (int s0 = 0; ok && !sum_only && s0 < tiles_n;) {
+        constexpr int kG = kSwin ? 2 : 4;                            // tiles whose pairs are on their way at once (more would spill)
         uint64_t a[kG], v[kG];
         bool there = true;
 #pragma unroll
@@ -574,7 +640,7 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
       }
       const float rstd = rsqrtf(dev * inv_n + st.eps), nm = -mean * rstd;
 #pragma unroll 1
-      for (int c = cpar; ok && c < chunks; c += 2) {
+      for (int c = cpar; ok && !sum_only && c < chunks; c += 2) {
         uint32_t r[32], w[16];
         tmem_ld32(t0 + c * 32, r);
         tmem_ld_wait(r);
@@ -593,9 +659,13 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
             }
           }
         }
-        store_box(sb, w, lane, [&](uint32_t buf) {
-          if (row0 < M) tma_store_2d(tm_out, buf, colbase + c * 32, row0);
-        });
+        if (kSwin && st.tok_grid) {
+          store_rows(sb.base, reinterpret_cast<__half*>(st.out), own, colbase + c * 32, w);
+        } else {
+          store_box(sb, w, lane, [&](uint32_t buf) {
+            if (row0 < M) tma_store_2d(tm_out, buf, colbase + c * 32, row0);
+          });
+        }
       }
       tc_fence_before_sync();
       if constexpr (kPair) {
@@ -617,6 +687,11 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
   return acc_bits;
 }
 
+// The Swin build's: sums and reordered rows.
+__device__ __noinline__ uint32_t gemm_stage_ool(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<false, true>(ca, acc_bits); }
+template <bool kPair>
+__device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<kPair, false>(ca, acc_bits); }
+
 // Tiles are bm x bn with bm = 128 (two accumulators used alternately, so the epilogue of one tile
 // overlaps the main loop of the next) or bm = 256 (two 128-row halves share every B tile, which
 // halves the B traffic per FLOP; each half has its own accumulator and hand-shake).
@@ -625,7 +700,7 @@ __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t a
 // shared memory -- half the B traffic per FLOP of the single-CTA form -- with every copy's completion counted on the
 // leader's full barrier; the leader's MMA lane issues for both and its commits arrive on the barriers of both CTAs;
 // each CTA's epilogue warps drain their own 128 rows and report to the leader's accumulator-free barrier.
-template <bool kPair = false, bool kLnEpi = false>
+template <bool kPair = false, bool kLnEpi = false, bool kSwin = false>
 __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
                            uint8_t* stage_s, RoleState& rs, const WaitCtl& ctl, int warp_id, int lane) {
   const int warp = uniform_warp(warp_id);
@@ -870,7 +945,9 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const int full_chunks = g.bn >> 5;
     if (kLnEpi && st.epi == EPI_LN) {
-      rs.acc_bits = gemm_ln_epilogue<kPair>(ca, rs.acc_bits | (uint32_t)(&st == &ctl_s.stage[1]) << 31);
+      const uint32_t which = (uint32_t)(&st == &ctl_s.stage[1]) << 31;
+      if constexpr (kSwin) rs.acc_bits = gemm_stage_ool(ca, rs.acc_bits | which);
+      else rs.acc_bits = gemm_ln_epilogue<kPair>(ca, rs.acc_bits | which);
     } else {
     EpiCtx e;
     e.epi = st.epi; e.act = st.act; e.M = st.M; e.N = st.N; e.ldo = st.ldo;
@@ -2000,38 +2077,6 @@ __device__ __noinline__ void ln_row_wide(const __half* row, const __half* gamma,
   }
 }
 
-// Rows of Swin blocks change their order where a block's windows lie differently from those before: a LayerNorm stage writes row `row` to
-// the place that its token has in the order it leaves in (Stage::tok_grid), so that all products and the attention stage have rows that
-// are adjacent.  (When the products permuted, an epilogue took 1.9 k cycles per 32 columns, and windows of 49 tokens took 64 rows of
-// the projection.)  The divisors are host constants, so a quotient is one multiply-high.
-__device__ __forceinline__ int ln_out_row(const Stage& st, int row) {
-  const int R = st.tok_grid;
-  if (!R) return row;
-  const int win = st.win, nwr = st.nwr, n_tok = win * win;
-  int img, ty, tx;
-  if (st.shift < 0) {                      // rows come in the order of the tokens
-    img = st.mg_seq2 ? (int)__umulhi((uint32_t)row, st.mg_seq2) : row / (R * R);
-    const int t = row - img * R * R;
-    ty = (int)fast_div((uint32_t)t, (uint32_t)R, st.mg_seq);
-    tx = t - ty * R;
-  } else {
-    const int wg = (int)fast_div((uint32_t)row, (uint32_t)n_tok, st.mg_tok), pos = row - wg * n_tok;
-    img = (int)fast_div((uint32_t)wg, (uint32_t)(nwr * nwr), st.mg_nwr2);
-    const int w = wg - img * nwr * nwr, wy = (int)fast_div((uint32_t)w, (uint32_t)nwr, st.mg_nwr);
-    const int py = (int)fast_div((uint32_t)pos, (uint32_t)win, st.mg_win);
-    ty = wy * win + py + st.shift;
-    tx = (w - wy * nwr) * win + (pos - py * win) + st.shift;
-    if (ty >= R) ty -= R;
-    if (tx >= R) tx -= R;
-  }
-  if (st.to_shift < 0) return (img * R + ty) * R + tx;
-  int sy = ty - st.to_shift, sx = tx - st.to_shift;
-  if (sy < 0) sy += R;
-  if (sx < 0) sx += R;
-  const int wy = (int)fast_div((uint32_t)sy, (uint32_t)win, st.mg_win), wx = (int)fast_div((uint32_t)sx, (uint32_t)win, st.mg_win);
-  return ((img * nwr + wy) * nwr + wx) * n_tok + (sy - wy * win) * win + (sx - wx * win);
-}
-
 // Rows read straight from L2.  W = N / 256 warps share a row (one for a row of 128 columns): lane l of part w holds columns
 // 256 w + 4 l .. + 3 and those 128 further on.  So 12 / W rows are in flight per CTA, dealt out over the CTAs first.  What a row
 // costs is latency: one L2 round trip for its planes, then a dependent chain in code that is cold when a CTA has one row, and
@@ -2430,12 +2475,6 @@ __device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams&
 //                    weight-tile traffic per FLOP of the GEMM stages; the attention stage takes two heads per pair.
 //                    Launched with a cluster dimension of two.
 constexpr int kFamilyBert = 0, kFamilyBertCoop = 1, kFamilySwin = 2, kFamilyBertPair = 3;
-__device__ __noinline__ uint32_t gemm_stage_ool(const Stage& st, const CallArgs& ca, SmemCtl& ctl_s, uint32_t ring, __half* vec_s,
-                                            uint8_t* stage_s, uint32_t state, const WaitCtl& ctl, int warp, int lane) {
-  RoleState r = RoleState::unpack(state);
-  gemm_stage<>(st, ca, ctl_s, ring, vec_s, stage_s, r, ctl, warp, lane);
-  return r.pack();
-}
 // One warp copies a stage record to shared memory.
 __device__ __forceinline__ void copy_record(Stage* to, const Stage* from, int lane) {
   static_assert(sizeof(Stage) % 16 == 0, "records are copied 16 bytes at a time");
@@ -2544,7 +2583,11 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
         if (wait_go(cs, ord, ctl)) drop_dead_buffers(st, warp * 32, 32);
       }
       if constexpr (kFamily == kFamilySwin) {
-        if (st.type == STAGE_GEMM) state = gemm_stage_ool(st, ca, cs, ring, vec_s, stage_s, state, ctl, warp, lane);
+        if (st.type == STAGE_GEMM) {
+          RoleState rs = RoleState::unpack(state);
+          gemm_stage<false, true, true>(st, ca, cs, ring, vec_s, stage_s, rs, ctl, warp, lane);
+          state = rs.pack();
+        }
         else if (st.type == STAGE_ATTN_SWIN) state = attn_swin_stage(st, ca, cs, ring, ring_ptr, reinterpret_cast<uint8_t*>(vec_s), state, ctl, warp, lane);
         else if (st.type == STAGE_LN && st.nslots == 0) ln_stage_direct(st, p, cs, reinterpret_cast<float2*>(vec_s), ctl, warp, lane);
         else if (st.type == STAGE_LN) state = ln_stage_ool(st, p, cs, ring, ring_ptr, vec_s, state, ctl, warp, lane);

@@ -538,6 +538,7 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   s.mg_kchunks = fast_div_magic((uint32_t)s.kchunks);
   s.mg_seq = fast_div_magic((uint32_t)(s.seq > 0 ? s.seq : 1));
   s.mg_head_dim = fast_div_magic((uint32_t)(s.head_dim > 0 ? s.head_dim : 1));
+  if (s.epi == EPI_LN && s.tok_grid) window_divisors(&s, s.tok_grid);
   const unsigned long long out_elems = (unsigned long long)s.M * (unsigned long long)s.N * (s.epi == EPI_PARTIAL ? s.splitk : 1);
   // 2^20 rows keep every multiply-high division exact (numerator * divisor < 2^32)
   if (s.M > (1 << 20) || out_elems >= 0xFFFF0000ull || (long long)s.items * 16 >= (1ll << 32))
@@ -754,6 +755,17 @@ static int add_plane_map(SouffleBertPlan* p, Stage& s) {
   int rc = make_plane_map(&m, s.partial, (uint64_t)s.splitk, (uint64_t)s.M, (uint64_t)s.N);
   if (rc) return rc;
   return set_store_map(p, s, m, 1);
+}
+
+// The map of a unit matrix, which adds residuals (see gemm_ln_epilogue).
+static int add_unit_map(SouffleBertPlan* p, uint32_t box_rows, int* idx) {
+  void* unit = nullptr;
+  std::vector<uint16_t> host(64 * 64, 0);
+  for (int i = 0; i < 64; ++i) host[65 * i] = 0x3C00;
+  int rc = plan_alloc(p, &unit, kUnitBytes);
+  if (rc) return rc;
+  SF_CUDA(cudaMemcpy(unit, host.data(), kUnitBytes, cudaMemcpyHostToDevice));
+  return add_map(p, unit, 64, 64, box_rows, idx);
 }
 
 // Marks `ptr` (`bytes` long) as dead once the stage just appended has run: the stage appended NEXT drops its lines from
@@ -1025,12 +1037,7 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   // LayerNorm 1's output) in boxes as high as its own tiles
   int m_unit = 0, m_res_act[2] = {-1, -1}, m_res_ln1 = -1;
   if (fuse_proj || fuse_fc2) {
-    __half* unit = nullptr;
-    std::vector<uint16_t> host(64 * 64, 0);
-    for (int i = 0; i < 64; ++i) host[65 * i] = 0x3C00;
-    if ((rc = plan_alloc(p, (void**)&unit, kUnitBytes))) return rc;
-    SF_CUDA(cudaMemcpy(unit, host.data(), kUnitBytes, cudaMemcpyHostToDevice));
-    if ((rc = add_map(p, unit, 64, 64, pair ? 32 : 64, &m_unit))) return rc;
+    if ((rc = add_unit_map(p, pair ? 32 : 64, &m_unit))) return rc;
     for (int i = 0; i < 2; ++i)
       if (fuse_proj && p->act[i] && (rc = add_map(p, p->act[i], M, H, a_rows(t_proj), &m_res_act[i]))) return rc;
     if (fuse_fc2 && (rc = add_map(p, p->ln1, M, H, a_rows(t_fc2), &m_res_ln1))) return rc;
@@ -1713,6 +1720,7 @@ static int launch_plan(SouffleBertPlan* plan, const void* x, void* y, const int3
   if ((rc = is_captured(st, &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, st, &mp))) return rc;
   mp.status = plan->d_status;
   if ((rc = expired_word(&mp.expired))) return rc;
+  mp.epoch = plan->d_sync + kEpochWord;
   mp.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
   rc = launch_mega(args, plan->grid, st, kFamilySwin);
   if (rc) return rc;
@@ -1725,7 +1733,7 @@ static int finish_plan(SouffleBertPlan* p, int sms) {
   int rc;
   int max_items = 1;
   for (const Stage& s : p->stages) {
-    const int it = stage_items(s);
+    const int it = s.fused ? 0 : stage_items(s);
     if (it > max_items) max_items = it;
   }
   p->grid = max_items < sms ? max_items : sms;
@@ -1767,6 +1775,22 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
   SF_CUDA(cudaMemset(p->d_sync, 0, 64));
   SF_CUDA(cudaMemset(p->d_status, 0, 64));
   const int attn_n = nWt * Hh <= sms ? 1 : 2;             // windows and heads per item, see attn_swin_stage
+  // LayerNorm (and the block's sum) in the epilogue of proj and FC2 from 2048 rows on, as in the encoder's plan (as planes / in the epilogue:
+  // 8 x 56 x 56 x 128 164 / 140 us, 16 x 28 x 28 x 256 with merging 179 / 168, six blocks of 16 x 14 x 14 x 512 374 / 347, of 11 283 / 273;
+  // below, 16 x 7 x 7 x 1024 111 / 118)
+  auto can_fuse = [&](const TileChoice& t) { return T >= 2048 && t.split == 1 && t.bn % 32 == 0 && t.bn >= 64 && C / t.bn <= sms; };
+  const bool fuse_proj = can_fuse(t_proj), fuse_fc2 = can_fuse(t_fc2);
+  RowStat* stats[2] = {nullptr, nullptr};
+  int m_unit = 0, m_resid[2] = {-1, -1};
+  for (int i = 0; i < 2; ++i)
+    if (i ? fuse_fc2 : fuse_proj) {
+      const TileChoice& t = i ? t_fc2 : t_proj;
+      const size_t bytes = (size_t)((T + 255) / 256) * 256 * (C / t.bn) * sizeof(RowStat);
+      if ((rc = plan_alloc(p, (void**)&stats[i], bytes))) return rc;
+      SF_CUDA(cudaMemset(stats[i], 0xff, bytes));
+      if ((rc = add_map(p, i ? x1 : x, T, C, (uint32_t)t.bm, &m_resid[i]))) return rc;
+    }
+  if ((fuse_proj || fuse_fc2) && (rc = add_unit_map(p, 64, &m_unit))) return rc;
   int m_y1, m_ctx, m_y2, m_hid, m_qkv;
   CUtensorMap ctx_out;
   if ((rc = add_map(p, y1, T, C, t_qkv.bm, &m_y1)) || (rc = add_map(p, ctx, T, C, t_proj.bm, &m_ctx)) ||
@@ -1821,6 +1845,29 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
         (rc = add_map(p, w1_t, F, C, t_fc1.bn, &m_w1)) || (rc = add_map(p, w2_t, C, F, t_fc2.bn, &m_w2)))
       return rc;
     const bool last = bi == n_blocks - 1;
+    const void *next_ln1_g = nullptr, *next_ln1_b = nullptr;
+    if (!last) {
+      const SouffleSwinWeights& nw = blocks[bi + 1];
+      if ((rc = copy_vec(nw.ln1_g, C, &next_ln1_g)) || (rc = copy_vec(nw.ln1_b, C, &next_ln1_b))) return rc;
+      if ((next_ln1_g == nullptr) != (next_ln1_b == nullptr)) return fail(SOUFFLE_BAD_ARGUMENT, "gamma and beta must be given together");
+    }
+    // a product and the LayerNorm stage behind it, or both in one (`i`: 0 proj, 1 FC2); leaves rc
+    auto add_product = [&](Stage g, Stage ln, bool fuse, int i, const void* w) {
+      g.ldo = C;
+      if (fuse) {
+        g.epi = EPI_LN; g.stats = stats[i]; g.tm_resid = m_resid[i]; g.tm_unit = m_unit;
+        g.bias = ln.bias; g.gamma = ln.gamma; g.beta = ln.beta; g.eps = ln.eps; g.sum_out = ln.sum_out; g.out = ln.out; g.out_sel = ln.out_sel;
+        g.tok_grid = ln.tok_grid; g.win = ln.win; g.shift = ln.shift; g.to_shift = ln.to_shift;
+        ln.fused = 1;
+        if (g.out && (rc = add_f16_out_map(p, g))) return;
+      } else {
+        g.epi = EPI_PARTIAL; g.partial = planes;
+        if ((rc = add_plane_map(p, g))) return;
+      }
+      p->stages.push_back(g);
+      note_weights(p, w);
+      p->stages.push_back(ln);
+    };
     // rows of a stage that leave in another order
     auto reorder = [&](Stage* st, int from, int to) {
       if (from == to) return;
@@ -1833,11 +1880,7 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
       s.eps = d.eps;
       reorder(&s, -1, shift);
       p->stages.push_back(s);
-    } else {       // later blocks' rows are normalised by the stage that adds up the block before (one barrier and one pass over x less)
-      Stage& sum = p->stages.back();
-      sum.sum_out = x;
-      sum.out = y1; sum.gamma = ln1_g; sum.beta = ln1_b; sum.eps = d.eps;
-    }
+    }              // (later blocks' rows are normalised by the stage that adds up the block before: one barrier and one pass over x less)
     s = blank_stage(STAGE_GEMM);                           // QKV
     s.tm_a = m_y1; s.tm_b = m_wqkv; s.M = T; s.N = 3 * C; s.K = C; s.bm = t_qkv.bm; s.bn = t_qkv.bn; s.epi = EPI_F16;
     s.bias = qkv_b; s.out = qkv; s.ldo = 3 * C;
@@ -1851,14 +1894,11 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     p->stages.push_back(s);
     s = blank_stage(STAGE_GEMM);                           // proj -> fp32 planes
     s.tm_a = m_ctx; s.tm_b = m_wo; s.M = T; s.N = C; s.K = C; s.bm = t_proj.bm; s.bn = t_proj.bn; s.splitk = t_proj.split;
-    s.epi = EPI_PARTIAL; s.partial = planes; s.ldo = C;
-    if ((rc = add_plane_map(p, s))) return rc;
-    p->stages.push_back(s);
-    note_weights(p, wo_t);
-    s = blank_stage(STAGE_LN);                             // x1 = planes + bias + x, LN2(x1)
-    s.M = T; s.N = C; s.ldo = C; s.partial = planes; s.n_partial = (uint8_t)t_proj.split; s.bias = proj_b; s.resid = x; s.sum_out = x1;
-    s.out = y2; s.gamma = ln2_g; s.beta = ln2_b; s.eps = d.eps;
-    p->stages.push_back(s);
+    Stage ln = blank_stage(STAGE_LN);                      // x1 = planes + bias + x, LN2(x1)
+    ln.M = T; ln.N = C; ln.ldo = C; ln.partial = planes; ln.n_partial = (uint8_t)t_proj.split; ln.bias = proj_b; ln.resid = x; ln.sum_out = x1;
+    ln.out = y2; ln.gamma = ln2_g; ln.beta = ln2_b; ln.eps = d.eps;
+    add_product(s, ln, fuse_proj, 0, wo_t);
+    if (rc) return rc;
     s = blank_stage(STAGE_GEMM);                           // FC1 + GELU
     s.tm_a = m_y2; s.tm_b = m_w1; s.M = T; s.N = F; s.K = C; s.bm = t_fc1.bm; s.bn = t_fc1.bn; s.epi = EPI_F16; s.act = ACT_GELU;
     s.bias = fc1_b; s.out = hid; s.ldo = F;
@@ -1867,15 +1907,19 @@ static int build_swin_plan(SouffleSwinPlan* sp, const SouffleSwinWeights* blocks
     note_weights(p, w1_t);
     s = blank_stage(STAGE_GEMM);                           // FC2 -> fp32 planes
     s.tm_a = m_hid; s.tm_b = m_w2; s.M = T; s.N = C; s.K = F; s.bm = t_fc2.bm; s.bn = t_fc2.bn; s.splitk = t_fc2.split;
-    s.epi = EPI_PARTIAL; s.partial = planes; s.ldo = C;
-    if ((rc = add_plane_map(p, s))) return rc;
-    p->stages.push_back(s);
-    note_weights(p, w2_t);
-    s = blank_stage(STAGE_LN);                             // planes + bias + x1 -> block output (no normalisation)
-    s.M = T; s.N = C; s.ldo = C; s.partial = planes; s.n_partial = (uint8_t)t_fc2.split; s.bias = fc2_b; s.resid = x1; s.eps = -1.0f;
-    if (last && !sp->has_merge) s.out_sel = PTR_CALL_Y; else s.out = xlast;
-    reorder(&s, shift, last ? -1 : ((bi + 1) & 1) ? d.shift_alt : d.shift);
-    p->stages.push_back(s);
+    ln = blank_stage(STAGE_LN);          // planes + bias + x1 -> the block's output or, with LN1 of the next one, its input
+    ln.M = T; ln.N = C; ln.ldo = C; ln.partial = planes; ln.n_partial = (uint8_t)t_fc2.split; ln.bias = fc2_b; ln.resid = x1; ln.eps = -1.0f;
+    if (!last) {
+      ln.sum_out = x;
+      ln.out = y1; ln.gamma = next_ln1_g; ln.beta = next_ln1_b; ln.eps = d.eps;
+    } else if (!sp->has_merge) {
+      ln.out_sel = PTR_CALL_Y;
+    } else {
+      ln.out = xlast;
+    }
+    reorder(&ln, shift, last ? -1 : ((bi + 1) & 1) ? d.shift_alt : d.shift);
+    add_product(s, ln, fuse_fc2, 1, w2_t);
+    if (rc) return rc;
   }
   if (sp->has_merge) {
     // Patch merging (python/models/swin_transformer/swin_patch_merge.py:1-17): 2 x 2 neighbourhoods concatenated to

@@ -21,7 +21,8 @@ enum EpilogueKind : int {
   EPI_F16 = 0,      // out[row, col] = f16(act(acc + bias)) (+ resid)
   EPI_QKV = 1,      // like EPI_F16 but scattered head-split to [3][B][heads][S][d]
   EPI_PARTIAL = 2,  // raw fp32 accumulators to partial[split][row][col]
-  EPI_LN = 3,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it
+  EPI_LN = 3,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it; sum_out, eps < 0 and
+                    // tok_grid as in a LayerNorm stage (Swin build)
 };
 
 enum Activation : int { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU = 2 };
@@ -65,19 +66,19 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
     RowStat* stats;  // EPI_LN: [blocks of 32 rows][tiles_n][32]
   };
   // ---- attention / head split ----
-  int batch, heads, seq, head_dim;
+  union {
+    struct { int batch, heads, seq, head_dim; };
+    struct { int tm_resid, tm_unit; };  // EPI_LN: tensor maps of the residual ([M][N], box 64 x bm) and of the unit matrix ([64][64])
+  };
   union {
     float scale;     // softmax scale applied to Q.K
-    int to_shift;    // STAGE_LN of a Swin block, see tok_grid
+    int to_shift;    // STAGE_LN and EPI_LN of a Swin block, see tok_grid
   };
   union {
     int tm_qkv;      // tensor map over the head-split buffer viewed as [3*B*heads*S][d], box 64 x 128; Swin: see attn_swin_stage
-    int tok_grid;    // STAGE_LN: 0, or the side of the token grid whose rows leave in another order than they come in: in the order of the
+    int tok_grid;    // STAGE_LN, EPI_LN: 0, or the side of the token grid whose rows leave in another order than they come in: in the order of the
   };                 // windows of `win` x `win` tokens after a shift, to_shift and `shift`, or in that of the tokens (-1)
-  union {
-    struct { int win, shift; };        // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
-    struct { int tm_resid, tm_unit; }; // EPI_LN: tensor maps of the residual ([M][N], box 64 x bm) and of the unit matrix ([64][64])
-  };
+  int win, shift;    // Swin: window size (7) and cyclic shift; `seq` is then the side of the token grid
   const void* rel_bias;  // Swin: fp16 [(2*win-1)^2][heads] relative-position bias table
   void* probs;       // optional fp16 [B*heads][S][S] normalised probabilities (debug / parity output)
   // ---- layer norm ----

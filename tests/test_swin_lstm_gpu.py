@@ -508,3 +508,43 @@ def test_lstm_calls_do_not_read_one_another(layers, hidden, steps):
         plan.status()
         assert torch.equal(y, s)
         assert (y.cpu() - want).abs().max() < 2e-5 + 1e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("batch,res,dim,window,shift,merge", [
+    (11, 14, 512, 7, 3, False),        # 2156 rows: the last tile of rows is ragged
+    (42, 7, 256, 7, 0, False),         # one window per image: 2058 rows
+    (3, 28, 256, 7, 3, True),          # the last block's rows go to the merging in the order of the tokens
+    (5, 24, 128, 8, 4, False),         # one tile per row
+    (1, 56, 512, 7, 2, False),         # tiles of 256 rows, several tiles per row
+])
+def test_swin_layernorm_in_the_epilogue(batch, res, dim, window, shift, merge):
+    """From 2048 rows on proj and FC2 add the residual, store the sum and normalise the rows in their epilogues, FC2's in the order of
+    the next block's windows.  Three blocks, twice, and from a graph."""
+    from souffle_models_b200 import swin
+    cfg = so.SwinConfig(res=res, dim=dim, heads=dim // 32, window=window)
+    blocks = [so.make_swin_params(cfg, 70 + i, zero_bias=False) for i in range(3)]
+    g = torch.Generator().manual_seed(res)
+    x = torch.randn(batch * res * res, dim, generator=g).half()
+    mg = so.make_swin_merge_params(cfg, 88, zero_bias=False) if merge else None
+    plan = swin.SwinBlock(batch, res, dim, dim // 32, window, 0, [{k: v.cuda() for k, v in p.items()} for p in blocks], shift_alt=shift,
+                          merge={k: v.cuda() for k, v in mg.items()} if mg else None)
+    xd = x.cuda()
+    y = plan.forward(xd).clone()
+    out = []
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out.append(plan.forward(xd))
+    for _ in range(2):
+        graph.replay()
+        assert torch.equal(out[0], y) and torch.equal(plan.forward(xd), y)
+    plan.status()
+    n = res * res
+    for b in {0, batch - 1}:
+        want = x[b * n:(b + 1) * n]
+        for i, p in enumerate(blocks):
+            want = so.swin_block(cfg, want, p, shift if i & 1 else 0).half()
+        if merge:
+            want = so.swin_patch_merge(cfg, want.float(), mg)
+        rows = y.shape[0] // batch
+        err = (y[b * rows:(b + 1) * rows].float().cpu() - want.float()).abs()
+        assert err.max() < 1.5e-2 and err.pow(2).mean().sqrt() < 2e-3          # the bounds of the block and stage tests
