@@ -2298,6 +2298,7 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
   static bool attr_set[16] = {};
   if (dev < 16 && !attr_set[dev]) {
     SF_CUDA(cudaFuncSetAttribute(souffle_se_module, cudaFuncAttributeMaxDynamicSharedMemorySize, kSeSmemBytes));
+    SF_CUDA(cudaFuncSetAttribute(souffle_se_module_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSeSmemBytes));
     attr_set[dev] = true;
   }
   // Items are dealt out evenly over all SMs, in contiguous runs: a small image is pulled in by as many SMs as it has
@@ -2313,22 +2314,37 @@ int souffle_se_module_forward(const float* input, const float* w_reduce, const f
       if (per_image % d == 0) { p.per_cta = d; break; }
   }
   const int grid = (p.items + p.per_cta - 1) / p.per_cta;
-  // shared memory: the channel means and reduce outputs, then as many slices per warp as fit, then the reduce weights
-  const int per_warp = (p.per_cta + kSeWarps - 1) / kSeWarps;
-  size_t smem = (size_t)(channels + kSeMaxReduce) * sizeof(float);
-  const size_t keep = (size_t)kSeWarps * se_slice_floats(p.slice_len) * sizeof(float);
-  p.cached = (int)((kSeSmemBytes - smem) / keep);
-  if (p.cached > per_warp) p.cached = per_warp;
-  smem += p.cached * keep;
+  // Images that a CTA meets are worked on together, as many as 4096 means allow: their means and GEMVs are one chain of reads then
+  // instead of one per image (32 x 144 x 56 x 56, 31 channels a CTA: a second image had cost 6 us of 30).
+  p.group = per_image % p.per_cta == 0 ? 1 : (p.per_cta + per_image - 2) / per_image + 1;
+  if (p.group > batch) p.group = batch;
+  if (p.group > kSeMaxChannels / (channels + kSeMaxReduce)) p.group = kSeMaxChannels / (channels + kSeMaxReduce);
+  if (p.group < 1) p.group = 1;
+  // shared memory: the channel means and reduce outputs, then as many slices per warp as fit, then the reduce weights, then the rows of the
+  // expand weights
+  p.per_warp = (p.per_cta + kSeWarps - 1) / kSeWarps;
+  const int image = height * width;          // (a warp keeps at most 3616 floats: the quotients by the multiplier are exact)
+  p.mg_hw = image > 1 && image < 512 ? fast_div_magic((uint32_t)image) : 0u;
+  const bool small = p.per_warp == 1 && p.slice_len <= 32 * 4 * kSeUnroll;          // a slice per warp: in registers
+  size_t smem = (size_t)p.group * (channels + kSeMaxReduce) * sizeof(float);
+  const int room = (int)((kSeSmemBytes - smem) / (kSeWarps * sizeof(float)));       // floats per warp
+  p.cached = small || room < 8 ? 0 : (room - 6) / p.slice_len;
+  if (p.cached > p.per_warp) p.cached = p.per_warp;
+  smem += (size_t)kSeWarps * se_run_floats(p.cached, p.slice_len) * sizeof(float);
   p.stage_weights = smem + weights <= (size_t)kSeSmemBytes ? 1 : 0;
   if (p.stage_weights) smem += weights;
+  const int rows = (p.per_cta + p.slices - 2) / p.slices + 1;                          // channels that a run of slices can touch
+  const size_t expand = (size_t)rows * (reduce | 1) * sizeof(float);
+  // (up to four floats a thread: one round trip to L2 in the shadow of the barrier; more of them would outlast it)
+  p.expand_rows = !small && rows * reduce <= 4 * (kSeThreads - 32) && smem + expand <= (size_t)kSeSmemBytes ? rows : 0;
+  if (p.expand_rows) smem += expand;
   p.input = input; p.w_reduce = w_reduce; p.w_expand = w_expand; p.out = out; p.pooled = pooled;
   p.sync = reinterpret_cast<unsigned*>(workspace) + 8;        // words 8, 9: the SE barrier (the GEMM entries use 0..3)
   p.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + 256);
   p.batch = batch; p.channels = channels; p.hw = height * width; p.reduce = reduce;
   p.timeout_ns = 2000ull * 1000000ull;
   void* kargs[] = {&p};
-  SF_CUDA(cudaLaunchCooperativeKernel((const void*)souffle_se_module, dim3(grid), dim3(kSeThreads), kargs, smem, st));
+  SF_CUDA(cudaLaunchCooperativeKernel(small ? (const void*)souffle_se_module_small : (const void*)souffle_se_module, dim3(grid), dim3(kSeThreads), kargs, smem, st));
   return SOUFFLE_OK;
 }
 

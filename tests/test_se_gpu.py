@@ -92,3 +92,25 @@ def test_reduce_weights_staged_and_not_at_every_alignment(shape, shift):
     want_pooled, want = so.se_module(x, wr, we)
     assert (pooled.cpu() - want_pooled).abs().max() < 1e-5
     assert (out.cpu() - want).abs().max() < 2e-5
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 3, 2368, 64), (1, 3, 3, 2369, 64), (1, 32, 32, 2368, 7), (1, 25, 41, 2368, 7), (300, 5, 5, 2, 3),
+                                   (3000, 5, 5, 2, 3), (12000, 1, 3, 1, 64), (20, 7, 73, 160, 9), (20, 16, 32, 160, 9), (33, 19, 27, 37, 5)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_one_slice_a_warp_and_many_images_a_block(shape, shift):
+    """As many slices as a B200 has warps, one more, a slice of 1024 floats and the next longer one (kept in registers or in
+    shared memory); blocks that meet two images, twenty, more than are worked on together; images just under and over the
+    512 floats from where they are added one by one.  Bound of the tests above; the same call twice gives the same bits."""
+    from souffle_models_b200 import efficientnet
+    b, h, w, c, r = shape
+    x, wr, we = _case(b, h, w, c, r, 31 + c)
+    wr, we = wr * (32.0 / c) ** 0.5 if c > 32 else wr, we / r ** 0.5
+    flat = torch.zeros(x.numel() + 4)
+    flat[shift:shift + x.numel()] = x.reshape(-1)
+    xin, wr_d, we_d = flat.cuda()[shift:shift + x.numel()].view(b, c, h, w), wr.cuda(), we.cuda()
+    pooled, out = efficientnet.se_module(xin, wr_d, we_d)
+    want_pooled, want = so.se_module(x, wr, we)
+    assert (pooled.cpu() - want_pooled).abs().max() < 1e-5
+    assert (out.cpu() - want).abs().max() < 2e-5
+    pooled2, out2 = efficientnet.se_module(xin, wr_d, we_d)
+    assert torch.equal(out, out2) and torch.equal(pooled, pooled2)
