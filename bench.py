@@ -36,9 +36,10 @@ HIDDEN = HEADS * HEAD_DIM
 # {sequences per GPU: bytes}, each from a one-pass capture of the 12-layer launch of that many sequences
 #   ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none \
 #       -k regex:souffle_megakernel -s 4 -c 1 --csv python -m souffle_models_b200.profile_cases bert_base_b<n>
+# (with SOUFFLE_PAIR_COOPERATIVE=0: a launch that is clustered and cooperative cannot be captured)
 # (the library as of the commit that last changed this table; tilings chosen by the cycle model, not timed)
-DRAM_BYTES_PER_LAUNCH = {64: 333_930_496 + 496_672_000, 32: 178_450_176 + 14_552_576, 16: 173_403_136 + 54_248_192,
-                         8: 172_171_264 + 4_679_424}
+DRAM_BYTES_PER_LAUNCH = {64: 412_645_632 + 565_328_384, 32: 180_741_888 + 572_626_688, 16: 173_494_528 + 15_390_464,
+                         8: 171_802_112 + 6_097_920}
 METRIC = "bert_base_12layer_seq128_batch64_sequences_per_second"
 WORKLOAD = "BERT-base 12-layer encoder, batch 64 (sharded by sequence), seq 128, lengths U[32,128]"
 SEED = 1239

@@ -686,6 +686,8 @@ static int upload_program(SouffleBertPlan* p) {
   // inputs that change from call to call, with drops / without: twelve layers of hidden 512 at 24 sequences (41 MB) 681 / 669 us,
   // of hidden 768 at 16 (41 MB) 748 / 740, 24 (61 MB) 895 / 896, 32 (82 MB) 1133 / 1143, 40 (102 MB) 1358 / 1379; one layer at 16
   // 66.0 / 65.9, 32 99.6 / 101.0, 48 (122 MB) 131.7 / 134.9, 64 (163 MB) 172.2 / 176.1.
+  // (With planes.  Where LayerNorm is in the products' epilogues a layer has less, and the drops decide little: twelve layers at 64
+  // sequences, 113 MB, 1426..1466 / 1434..1481 us, at 32, 57 MB, 827..863 / 829..849.)
   DeviceInfo* di = nullptr;
   if ((rc = device_info(&di))) return rc;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {

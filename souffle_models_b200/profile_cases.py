@@ -10,8 +10,8 @@ python/models/tee:1-2).  The counterpart here:
 
 Every case builds its plan on seeded random parameters, makes 3 warm-up calls and 5 timed ones (CUDA events) and
 prints the mean time per call.  Cases: bert_layer (1 x 128, one layer), bert_base (1 x 128, 12 layers), bert_layer_b64 (64 x 128
-with ragged lengths, one layer), bert_layer_b64_pairs (the same on CTA pairs, desc.pair_mma; set SOUFFLE_PAIR_COOPERATIVE=0
-under Nsight Compute, which cannot capture a launch that is both clustered and cooperative), bert_base_b<n> (12 layers
+with ragged lengths, one layer, on CTA pairs as by default; set SOUFFLE_PAIR_COOPERATIVE=0 under Nsight Compute, which cannot
+capture a launch that is both clustered and cooperative), bert_layer_b64_pairs (the same asked for by desc.pair_mma), bert_base_b<n> (12 layers
 at n sequences, e.g. bert_base_b64, _b32, _b16, _b8: one GPU's share of the benchmark step on 1, 2, 4 and 8 GPUs),
 gemm_fc1 (one 8192 x 3072 x 768 product through the plan-less GEMM entry: main loop and plain fp16 epilogue alone),
 bert_layer_s384
