@@ -972,7 +972,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     // none) while the tile before is being stored, and one barrier per tile separates the two buffers' uses.
     const int my_col = (int)threadIdx.x - 64;
     const __half* bias = e.epi != EPI_PARTIAL ? reinterpret_cast<const __half*>(st.bias) : nullptr;
-    auto load_bias = [&](int nt) -> float { return bias && my_col < g.bn ? __half2float(__ldg(bias + nt * g.bn + my_col)) : 0.0f; };
+    auto load_bias = [&](int nt) -> float { return bias && my_col < g.bn && nt * g.bn + my_col < e.N ? __half2float(__ldg(bias + nt * g.bn + my_col)) : 0.0f; };
     int mt, nt, ks;
     gemm_item(st, first_item, mt, nt, ks);
     float next_bias = first_item < g.items ? load_bias(nt) : 0.0f;
@@ -984,6 +984,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     for (int item = first_item; item < g.items; item += item_step, turn ^= 1u) {
       const uint32_t acc0 = g.nh == 2 ? 0u : rs.acc_bits >> 2;
       const int row_tile = mt * g.bm, colbase = nt * g.bn, plane = ks;
+      const int left = (e.N - colbase) >> 5, chunks = left < full_chunks ? left : full_chunks;
       const float* bias_t = ctl_s.bias[turn];
       if (e.epi != EPI_PARTIAL) {
         ctl_s.bias[turn][my_col] = next_bias;
@@ -1025,7 +1026,8 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
         tc_fence_after_sync();
         const uint32_t t0 = tmem + acc * kAccStride;
         // this warp takes chunks cpar, cpar+2, ... (its partner warp on the same lane quarter the others)
-        for (int c = cpar; c < full_chunks; c += 2) {
+        // and a last tile that is wider than what is left of the matrix (a multiple of 64 columns) ends with it
+        for (int c = cpar; c < chunks; c += 2) {
           uint32_t r[32];
           const unsigned tl = prof ? (unsigned)clock64() : 0u;
           tmem_ld32(t0 + c * 32, r);

@@ -233,6 +233,20 @@ struct RankedTile {
   double cost;
   TileChoice t;
 };
+// A tile width that does not divide N, or a split that does not divide K's chunks: the copy engine reads zeros past the matrix and writes
+// nothing there, so the last tile or the last split just has less to do.  Widths: where no tile of 256 columns divides N, nor one of 192
+// ([K][N] weights: 256, a pair cannot read 192 of them), for products that are not cut along K, whose outputs are plain rows; an odd multiple of 64
+// had tiles of 64, an odd multiple of 128 of 128 at best.  Splits: where the number of chunks is no multiple of four; a last split without a
+// chunk is of no use.  Back to back in us, dividing tiles only / now: products of 8000 x 3392 x 768 80.3 / 38.7, 4096 x 3008 x 768
+// 35.1 / 21.6, 4096 x 2944 x 768 26.2 / 21.7; MLP 196 x 1024 x 3904 27 / 18.7; three encoder layers of 40 x 128 at 768 with a hidden layer
+// of 3008 308 / 257, 7 x 112 of 2368 143.7 / 125.1, 1 x 128 of 1856 106.6 / 93.2, 40 x 128 of 2432 247 / 236.
+// Not for plans whose tilings are timed: those may be handed on to other ranks as settings, which have to divide.
+static bool ragged_width(int N, int bn, bool takes_192 = true) {
+  return N % 256 != 0 && !(takes_192 && N % 192 == 0) && bn >= 96 && bn < N;
+}
+static int chunks_per_split(int kch, int split) { return (kch + split - 1) / split; }
+static bool ragged_split(int kch, int split) { return kch % 4 != 0 && (split - 1) * chunks_per_split(kch, split) < kch; }
+
 static TileChoice choose_tiles(int M, int N, int K, int sms, bool allow_split, bool b_mn, int head_split = 0,
                                std::vector<RankedTile>* ranked = nullptr) {
   const int kch = K / 64;
@@ -243,18 +257,18 @@ static TileChoice choose_tiles(int M, int N, int K, int sms, bool allow_split, b
     if (bm == 256 && M <= 128) continue;
     for (int ci = 0; ci < 8; ++ci) {
       const int bn = cands[ci];
-      if (N % bn) continue;
+      if (N % bn && (ranked || allow_split || !ragged_width(N, bn, !b_mn))) continue;
       if (b_mn && bn % 64) continue;
       if (head_split == 1 && bn != 16 && bn % 32) continue;   // 32-column epilogue chunks must not straddle a head
       if (196608 / ((bm + bn) * 128) < 2) continue;
       for (int split = 1; split <= (allow_split ? 16 : 1); ++split) {
-        if (kch % split) continue;
-        const long items = (long)((M + bm - 1) / bm) * (N / bn) * split;
+        if (kch % split && (ranked || !ragged_split(kch, split))) continue;
+        const long items = (long)((M + bm - 1) / bm) * ((N + bn - 1) / bn) * split;
         const long waves = (items + sms - 1) / sms;
         const double smem = 2.0 * bm + (bm / 128 + 1.0) * bn, mma = bm * bn / 64.0;
         const double chunk = 1.1 * (smem > mma ? smem : mma);
         const double epilogue = bm * bn * (allow_split ? 0.2 : 0.35);      // fp32 planes need no math
-        const double tile = (kch / split) * chunk + (bm == 256 ? 0.7 : 0.45) * epilogue + 1500.0;
+        const double tile = chunks_per_split(kch, split) * chunk + (bm == 256 ? 0.7 : 0.45) * epilogue + 1500.0;
         double cost = waves * tile;
         if (allow_split) cost += (double)split * M * N * 8.0 / sms / 12.0;
         if (ranked) {
@@ -283,16 +297,16 @@ static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_
   const int cands[6] = {256, 192, 128, 96, 64, 32};
   for (int ci = 0; ci < 6; ++ci) {
     const int bn = cands[ci];
-    if (N % bn) continue;
+    if (N % bn && (ranked || allow_split || !ragged_width(N, bn, !b_mn))) continue;
     if (b_mn && bn % 128) continue;             // each CTA loads its half in blocks of 64 columns
     for (int split = 1; split <= (allow_split ? 16 : 1); ++split) {
-      if (kch % split) continue;
-      const long items = (long)((M + 255) / 256) * (N / bn) * split;
+      if (kch % split && (ranked || !ragged_split(kch, split))) continue;
+      const long items = (long)((M + 255) / 256) * ((N + bn - 1) / bn) * split;
       const long waves = (items + npairs - 1) / npairs;
       const double load = (16384.0 + 64.0 * bn) / 55.0, mma = 2.0 * bn;
       const double chunk = 1.05 * (load > mma ? load : mma);
       const double epilogue = 128.0 * bn * (allow_split ? 0.2 : 0.35);
-      const double tile = (kch / split) * chunk + 0.45 * epilogue + 1500.0;
+      const double tile = chunks_per_split(kch, split) * chunk + 0.45 * epilogue + 1500.0;
       double cost = waves * tile;
       if (allow_split) cost += (double)split * M * N * 8.0 / (2.0 * npairs) / 12.0;
       if (ranked) {
@@ -318,9 +332,9 @@ static TileChoice choose_tiles_pair(int M, int N, int K, int npairs, bool allow_
 // 8192 x 1024 x 1024 20.2 / 19.4, 2048 x 3072 x 768 15.9 / 16.1 (28 / 30); and back to back 8192 x 768 x 3072 32.8 / 38.7 (57 / 66),
 // 1024 x 4096 x 4096 32.1 / 28.9.
 static double gemm_cycles(const TileChoice& t, int M, int N, int K, int ctas, bool pair) {
-  const long items = (long)((M + t.bm - 1) / t.bm) * (N / t.bn) * t.split;
+  const long items = (long)((M + t.bm - 1) / t.bm) * ((N + t.bn - 1) / t.bn) * t.split;
   const long at_once = pair ? ctas / 2 : ctas, waves = (items + at_once - 1) / at_once;
-  const double steps = K / 64 / t.split, epilogue = t.bn / 64.0 * 950.0;
+  const double steps = chunks_per_split(K / 64, t.split), epilogue = t.bn / 64.0 * 950.0;
   if (pair) {
     const double step = std::max(450.0, std::max(2.0 * t.bn, (16384.0 + 64.0 * t.bn) / 70.0));
     return waves * std::max(steps * step, epilogue) + epilogue + 13500.0;
@@ -449,7 +463,7 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
 
 // Work items of a stage; for a plan on CTA pairs GEMM tiles and attention couples are per PAIR (bm = 256).
 static int stage_items(const Stage& s, bool pair = false) {
-  if (s.type == STAGE_GEMM) return ((s.M + s.bm - 1) / s.bm) * (s.N / s.bn) * s.splitk;
+  if (s.type == STAGE_GEMM) return ((s.M + s.bm - 1) / s.bm) * ((s.N + s.bn - 1) / s.bn) * s.splitk;
   if (s.type == STAGE_ATTN && pair) return s.batch * s.heads / 2;
   if (s.type == STAGE_ATTN) return s.batch * s.heads * ((s.seq + s.bm - 1) / s.bm);
   if (s.type == STAGE_ATTN_SWIN)      // s.bn windows x s.bn heads
@@ -516,17 +530,20 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   if (s.type != STAGE_GEMM) return SOUFFLE_OK;
   if (s.bias && s.epi != EPI_PARTIAL && s.N > 4096)
     return fail(SOUFFLE_BAD_SHAPE, "a GEMM stage with a bias vector is limited to 4096 output columns (got %d)", s.N);
-  s.tiles_n = s.N / s.bn;
-  s.kchunks = s.K / 64 / s.splitk;
+  s.tiles_n = (s.N + s.bn - 1) / s.bn;
+  s.kchunks = chunks_per_split(s.K / 64, s.splitk);
   s.items = stage_items(s);
   // per CTA and K chunk: the A rows (all of the tile's, or one 128-row half of a pair's) and the B rows (all, or half)
   s.slot_bytes = pair ? 16384 + s.bn * 64 : (s.bm / 128) * 16384 + s.bn * 128;
   // Two steps of 64 per slot where three such slots fit: the lone lanes' wait, commit and bookkeeping are paid once per slot (a
   // 128 x 16 tile: 390 -> 295 cycles per step).  With two slots left the copies no longer run ahead (16 sequences: 743 -> 774 us).
   s.kper = 1;
-  if (!pair && max_slots == 0 && s.bm == 128 && s.kchunks % 2 == 0 && 196608 / (2 * s.slot_bytes) >= 3) {
+  // An odd number of steps gets one more, of zeros, where narrow tiles make it pay (256 x 512 x 1856 13.3 -> 12.4 us a call, two layers of
+  // 4 x 384 at 512 with FC2 of 27 steps 90.0 -> 87.1).
+  const bool even = s.kchunks % 2 == 0 || (s.bn <= 64 && s.kchunks >= 8);
+  if (!pair && max_slots == 0 && s.bm == 128 && even && 196608 / (2 * s.slot_bytes) >= 3) {
     s.kper = 2;
-    s.kchunks /= 2;
+    s.kchunks = (s.kchunks + 1) / 2;
     s.slot_bytes *= 2;
   }
   int n = 196608 / s.slot_bytes;
@@ -981,17 +998,18 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     if (tune_ws) cudaFree(tune_ws);
   }
   if (pair) t_qkv.bm = t_fc1.bm = t_proj.bm = t_fc2.bm = 256;      // a pair's tile is 256 rows: 128 per CTA
-  auto bad_tile = [pair](const TileChoice& t, int N) {
-    if (pair) return t.bn < 32 || t.bn > 256 || t.bn % 32 || N % t.bn;     // each CTA holds bn / 2 rows of the B tile
-    return (t.bm != 128 && t.bm != 256) || t.bn < 16 || t.bn > 256 || t.bn % 16 || N % t.bn ||
+  auto bad_tile = [pair](const TileChoice& t, int N, bool divides = true) {
+    if (divides && t.bn > 0 && N % t.bn) return true;
+    if (pair) return t.bn < 32 || t.bn > 256 || t.bn % 32 != 0;            // each CTA holds bn / 2 rows of the B tile
+    return (t.bm != 128 && t.bm != 256) || t.bn < 16 || t.bn > 256 || t.bn % 16 ||
            196608 / ((t.bm + t.bn) * 128) < 2;
   };
   if (t_qkv.bn != 16 && t_qkv.bn % 32) return fail(SOUFFLE_BAD_SHAPE, "bn_qkv must be 16 or a multiple of 32");
-  if (bad_tile(t_qkv, 3 * H) || bad_tile(t_fc1, F) || bad_tile(t_proj, H) || bad_tile(t_fc2, H))
+  if (bad_tile(t_qkv, 3 * H) || bad_tile(t_fc1, F, d.bn_fc1 != 0) || bad_tile(t_proj, H) || bad_tile(t_fc2, H))
     return fail(SOUFFLE_BAD_SHAPE, "tile shapes (%dx%d, %dx%d, %dx%d, %dx%d) do not fit the layer", t_qkv.bm, t_qkv.bn,
                 t_fc1.bm, t_fc1.bn, t_proj.bm, t_proj.bn, t_fc2.bm, t_fc2.bn);
   if (t_proj.split < 1 || t_fc2.split < 1 || t_proj.split > 16 || t_fc2.split > 16 || (H / 64) % t_proj.split ||
-      (F / 64) % t_fc2.split)
+      (d.split_fc2 && (F / 64) % t_fc2.split))
     return fail(SOUFFLE_BAD_SHAPE, "split-K factors must be in 1..16 and divide K/64");
   const int bn_qkv = t_qkv.bn, bn_fc1 = t_fc1.bn, bn_proj = t_proj.bn, sp_proj = t_proj.split, bn_fc2 = t_fc2.bn,
             sp_fc2 = t_fc2.split;
@@ -1543,7 +1561,7 @@ static int row_family(int M, int grid) { return M <= grid * (kThreads / 32) ? kF
 
 // Whether a GEMM of [K][N] weights with fp16 output is faster on pairs.
 static bool gemm_on_pairs(int M, int N, int K, int sms, int npairs) {
-  if (npairs < 1 || N % 128) return false;
+  if (npairs < 1) return false;
   const TileChoice s = choose_tiles(M, N, K, sms, false, true), t = choose_tiles_pair(M, N, K, npairs, false, true);
   return s.bn && t.bn && gemm_cycles(t, M, N, K, 2 * npairs, true) < 0.95 * gemm_cycles(s, M, N, K, sms, false);
 }
@@ -1609,17 +1627,17 @@ int souffle_swin_mlp_forward(const void* src, const void* fc1_w, const void* fc2
   const bool can_reduce = C == 128 || C == 256 || C == 512 || C == 768 || C == 1024;
   const size_t plane_bytes = (size_t)M * C * sizeof(float);
   auto fc2_tiles = [&](int npairs) {
-    TileChoice t = npairs ? choose_tiles_pair(M, C, F, npairs, true, true) : choose_tiles(M, C, F, sms, true, true);
-    if (t.split > 1 && (!can_reduce || workspace_bytes < souffle_gemm_workspace_bytes() + (size_t)t.split * plane_bytes))
+    TileChoice t = npairs ? choose_tiles_pair(M, C, F, npairs, can_reduce, true) : choose_tiles(M, C, F, sms, can_reduce, true);
+    if (t.split > 1 && workspace_bytes < souffle_gemm_workspace_bytes() + (size_t)t.split * plane_bytes)
       t = npairs ? choose_tiles_pair(M, C, F, npairs, false, true) : choose_tiles(M, C, F, sms, false, true);
     return t;
   };
   TileChoice t2 = fc2_tiles(0);
   // both products on CTA pairs where they take less time together (see gemm_cycles)
   int npairs = sms / 2 < di->max_pairs ? sms / 2 : di->max_pairs;
-  if (npairs >= 1 && C % 128 == 0 && F % 128 == 0 && t2.bn) {
-    const TileChoice p2 = fc2_tiles(npairs);
-    const double pairs = gemm_cycles(choose_tiles_pair(M, F, C, npairs, false, true), M, F, C, 2 * npairs, true) + gemm_cycles(p2, M, C, F, 2 * npairs, true);
+  const TileChoice p1 = npairs >= 1 ? choose_tiles_pair(M, F, C, npairs, false, true) : TileChoice(), p2 = npairs >= 1 ? fc2_tiles(npairs) : TileChoice();
+  if (p1.bn && p2.bn && t2.bn) {
+    const double pairs = gemm_cycles(p1, M, F, C, 2 * npairs, true) + gemm_cycles(p2, M, C, F, 2 * npairs, true);
     const double single = gemm_cycles(choose_tiles(M, F, C, sms, false, true), M, F, C, sms, false) + gemm_cycles(t2, M, C, F, sms, false);
     if (pairs < 0.95 * single) t2 = p2;
     else npairs = 0;

@@ -407,3 +407,19 @@ def test_wait_limit_in_front_of_every_kind_of_stage(B, S, heads, stage):
     if stage in (2, 5):
         assert f"code 2, where {stage}," in str(ei.value)
     bad.close()
+
+
+@pytest.mark.parametrize("B,S,heads,ffn", [
+    (2, 128, 12, 1856),    # 29 steps and column blocks of 64: FC2 cut along K with a shorter last part
+    (7, 112, 12, 2368),    # 37
+    (30, 128, 12, 832),    # 13, on CTA pairs
+    (16, 128, 12, 448),    # 7, LayerNorm in the epilogues
+    (1, 384, 2, 320),      # 5
+])
+def test_ffn_of_an_odd_multiple_of_64(B, S, heads, ffn):
+    """FC1's tiles do not divide its columns, FC2's parts do not divide its steps: hidden layer and output against the oracle."""
+    cfg = so.BertConfig(B, S, heads, 64, ffn, "std")
+    enc, layers, x, lens, y = _run(cfg, 91, zero_bias=False, keep_probs=True)
+    r = so.bert_layer(cfg, x, layers[0], lens)
+    assert _err(enc.buffer("fc1"), r["fc1"]) < TOL_LAYER
+    assert _err(y, r["out"]) < TOL_LAYER

@@ -548,3 +548,30 @@ def test_swin_layernorm_in_the_epilogue(batch, res, dim, window, shift, merge):
         rows = y.shape[0] // batch
         err = (y[b * rows:(b + 1) * rows].float().cpu() - want.float()).abs()
         assert err.max() < 1.5e-2 and err.pow(2).mean().sqrt() < 2e-3          # the bounds of the block and stage tests
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (300, 1856, 704),      # N an odd multiple of 64: the last tile has 64 columns of it; K an odd number of steps
+    (4000, 3008, 576),     # the same on CTA pairs
+    (129, 320, 832),       # few tiles, two steps per slot: the last slot's second step is all zeros
+    (1, 64, 1856),         # one column block, narrower than the tile that would be taken
+    (1000, 1664, 448),     # N an odd multiple of 128
+])
+def test_gemm_of_odd_multiples_of_64(M, N, K):
+    """Tile widths that do not divide the output and step counts that are padded with zeros.  Values in memory around the output stay as
+    they are.  Bound: fp16 rounding of the result and fp32 sums of K products of fp16 values."""
+    from souffle_models_b200 import swin
+    g = torch.Generator().manual_seed(N + K)
+    a, w = torch.randn(M, K, generator=g).half(), (torch.randn(K, N, generator=g) * 0.05).half()
+    want = a.float() @ w.float()
+    got = swin.gemm(a.cuda(), w.cuda()).float().cpu()
+    assert ((got - want).abs() <= 2.0 ** -11 * want.abs() + K * 2.0 ** -24 * (a.float().abs() @ w.float().abs()) + 1e-6).all()
+    x, w2 = torch.randn(M, 320, generator=g).half(), (torch.randn(320, N, generator=g) * 0.05).half()
+    w3 = (torch.randn(N, 320, generator=g) * 0.05).half()
+    hidden = (x.float() @ w2.float()).half().float()
+    want = hidden @ w3.float()
+    got = swin.swin_fused_feed_mlp(x.cuda(), w2.cuda(), w3.cuda())
+    got = (got[-1] if isinstance(got, (list, tuple)) else got).float().cpu()
+    # a hidden value may round the other way: half an ulp of it, through its column of the weights
+    bound = 2.0 ** -11 * want.abs() + (2.0 ** -10 + N * 2.0 ** -24) * (hidden.abs() @ w3.float().abs()) + 1e-6
+    assert ((got - want).abs() <= bound).all()
