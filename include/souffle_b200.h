@@ -184,8 +184,10 @@ int souffle_bert_plan_info(SouffleBertPlan* plan, int* launches_out, int* grid_o
 /* 1 if the plan's launch runs on CTA pairs (see SouffleBertDesc.pair_mma), else 0. */
 int souffle_bert_plan_uses_pairs(SouffleBertPlan* plan);
 /* The tiling chosen for stage `index` of the program: out[0..5] = {stage type (0 GEMM, 1 attention, 2 LayerNorm),
- * tile rows, tile columns, split-K factor, work items (0: a LayerNorm that the GEMM stage before it does), ring slots}.  The reference fixes these at compile time
- * (cpp/bert/kernels/bert.h:18-52); here they depend on the shape and on the SM count. */
+ * tile rows, tile columns, split-K factor, work items (0: a LayerNorm that the GEMM stage before it does), ring slots}.  The reference
+ * fixes these at compile time (cpp/bert/kernels/bert.h:18-52); here they depend on the shape and on the SM count.  A width or split
+ * that the library chose without timing need not divide the product (the last tile or part is shorter); a setting in the
+ * descriptor has to, and what desc.autotune chooses does. */
 int souffle_bert_plan_stage_info(SouffleBertPlan* plan, int index, int out[6]);
 
 /* ------------------------------------------------------------------------------------------
