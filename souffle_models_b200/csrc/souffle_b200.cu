@@ -938,13 +938,14 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   SF_CUDA(cudaMemset(p->d_status, 0, 64));
 
   // ---- tiling ----
-  TileChoice t_qkv = choose_tiles(M, 3 * H, H, sms, false, false, 1), t_fc1 = choose_tiles(M, F, H, sms, false, false),
-             t_proj = choose_tiles(M, H, H, sms, true, false), t_fc2 = choose_tiles(M, H, F, sms, true, false);
+  std::vector<RankedTile> dividing, *timed = d.autotune ? &dividing : nullptr;      // timed tilings divide (see ragged_width)
+  TileChoice t_qkv = choose_tiles(M, 3 * H, H, sms, false, false, 1), t_fc1 = choose_tiles(M, F, H, sms, false, false, 0, timed),
+             t_proj = choose_tiles(M, H, H, sms, true, false), t_fc2 = choose_tiles(M, H, F, sms, true, false, 0, timed);
   if (pair) {
     t_qkv = choose_tiles_pair(M, 3 * H, H, npairs, false);
-    t_fc1 = choose_tiles_pair(M, F, H, npairs, false);
+    t_fc1 = choose_tiles_pair(M, F, H, npairs, false, false, timed);
     t_proj = choose_tiles_pair(M, H, H, npairs, true);
-    t_fc2 = choose_tiles_pair(M, H, F, npairs, true);
+    t_fc2 = choose_tiles_pair(M, H, F, npairs, true, false, timed);
   }
   if (d.bm_qkv) t_qkv.bm = d.bm_qkv;
   if (d.bn_qkv) t_qkv.bn = d.bn_qkv;

@@ -423,3 +423,8 @@ def test_ffn_of_an_odd_multiple_of_64(B, S, heads, ffn):
     r = so.bert_layer(cfg, x, layers[0], lens)
     assert _err(enc.buffer("fc1"), r["fc1"]) < TOL_LAYER
     assert _err(y, r["out"]) < TOL_LAYER
+    timed = _encoder(cfg, layers, tuning=dict(autotune=1))              # timed tilings can be handed on as settings: they divide
+    f1, f2 = timed.stage_info(4), timed.stage_info(5)
+    assert ffn % f1["bn"] == 0 and (ffn // 64) % f2["splitk"] == 0
+    assert _err(timed.forward(x.cuda(), lens.cuda() if lens is not None else None), r["out"]) < TOL_LAYER
+    timed.status()
