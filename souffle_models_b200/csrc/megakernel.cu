@@ -458,7 +458,7 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
   uint8_t* boxes = smem_raw + kCtlBytes + kRingBytes;
   const int warp = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31;
   const MegaParams& p = ca.p;
-  const int q = warp & 3, cpar = (warp - 2) >> 2, my_col = (int)threadIdx.x - 64;
+  const int q = epi_quarter(warp), cpar = epi_part(warp), my_col = (int)threadIdx.x - 64;
   const int bn = st.bn, chunks = bn >> 5, tiles_n = st.tiles_n, nh = kPair ? 1 : st.bm >> 7, M = st.M;
   const uint32_t rank = kPair ? cluster_cta_rank() : 0u;
   const int first_item = kPair ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, item_step = kPair ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -482,11 +482,11 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
   const bool prof = p.prof != nullptr, affine = st.gamma != nullptr;
   float* bias_s = cs.bias[0];
   __half* gamma_s = reinterpret_cast<__half*>(cs.bias[1]);          // gamma of the tile's columns, then beta
-  // statistics of the warps that have the other chunks of these rows, in their second boxes (written again only once all tiles of the
-  // row have been published, and so after they have been read; plain stores pass through the first)
-  float2* other = reinterpret_cast<float2*>(boxes + ((4 + q) * 2 + 1) * kStageWarp);
+  // Statistics that part 1 of these rows hands to part 0, in part 1's second box: its copies have left it before the tile begins, and
+  // it goes over the statistics behind the barrier that follows their reading (plain stores pass through the first box).
+  float2* other = reinterpret_cast<float2*>(boxes + ln_stats_box(q) * kStageWarp);
   StoreBoxes sb;
-  sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+  sb.base = boxes + epi_box(warp) * kStageWarp;
   sb.box = 0;
   sb.n = 2;
   bool ok = true;            // a warp that has given up goes through the remaining tiles, whose barriers the others wait in
@@ -584,9 +584,7 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
         st_relaxed_2x64(st.stats + ((size_t)(row0 >> 5) * tiles_n + nt) * 32 + lane, (uint64_t)__float_as_uint(mean) | ((uint64_t)tag << 32),
                         (uint64_t)__float_as_uint(dev) | ((uint64_t)tag << 32));
     }
-    // the second half's statistics have been read before the first half's boxes go over them (the first half's have been read before they
-    // are published)
-    if (nh == 2) named_barrier_sync(4 + q, 64);
+    named_barrier_sync(4 + q, 64);          // the statistics have been read: part 1 may store
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
       const uint32_t acc = acc0 + (uint32_t)h, t0 = tmem + acc * kAccStride;
@@ -941,7 +939,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     __syncwarp();
   } else if (warp < 2 + kEpiWarps) {
     // ---------------- epilogue: TMEM -> registers -> global (8 warps: lane quarter x column parity) --
-    const int q = warp & 3, cpar = (warp - 2) >> 2;
+    const int q = epi_quarter(warp), cpar = epi_part(warp);
     const uint32_t tmem = ctl_s.tmem_base + ((uint32_t)(q * 32) << 16);
     const int full_chunks = g.bn >> 5;
     if (kLnEpi && st.epi == EPI_LN) {
@@ -965,7 +963,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     if (prof && warp == 2 && lane == 0)
       for (int i = 6; i < 11; ++i) p.prof[((size_t)st.position * gridDim.x + blockIdx.x) * kProfSlots + i] = 0;
     StoreBoxes sb;
-    sb.base = reinterpret_cast<uint8_t*>(vec_s) + (warp - 2) * 2 * kStageWarp;
+    sb.base = reinterpret_cast<uint8_t*>(vec_s) + epi_box(warp) * kStageWarp;
     sb.box = 0;
     sb.n = 2;
     // The bias of a tile's columns goes to shared memory as fp32 in front of the tile: a thread loads one column's (0 where there is
@@ -1545,7 +1543,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
     __half* probs = reinterpret_cast<__half*>(st.probs);
     const CUtensorMap* tm_out = map_ptr(ca, st.tm_out);
     StoreBoxes sb;                                            // a row's 64 columns are two boxes
-    sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+    sb.base = boxes + epi_box(warp) * kStageWarp;
     sb.box = 0;
     sb.n = 2;
     uint8_t* pbase = ring_ptr + g * kPipeBytes + 3 * kATileBytes + r_in * 128;
@@ -1865,7 +1863,7 @@ __device__ __noinline__ uint32_t attn_swin_stage(const Stage& st, const CallArgs
     float* bias_s = reinterpret_cast<float*>(ring_ptr + 5 * kATileBytes) + grp * 256;      // this head's column of the bias table (x log2 e)
     uint8_t* prow = ring_ptr + (3 + grp) * kATileBytes + r_in * 128;
     StoreBoxes sb;
-    sb.base = boxes + (warp - 2) * 2 * kStageWarp;
+    sb.base = boxes + epi_box(warp) * kStageWarp;
     sb.box = 0;
     sb.n = 2;
     // the table's column of the next item is requested while this one is worked on

@@ -112,6 +112,22 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   uint32_t mg_seq2, mg_win, mg_nwr, mg_nwr2, mg_tok;
 };
 
+#ifdef __CUDACC__
+#define SOUFFLE_HOST_DEVICE __host__ __device__
+#else
+#define SOUFFLE_HOST_DEVICE
+#endif
+
+// The eight epilogue warps of a CTA, numbers 2..9.  The hardware lets a warp read one quarter of tensor memory's lanes, by its number
+// modulo four; the two warps of a quarter have the same rows and take every other 32 columns, the one of part 0 the first.
+SOUFFLE_HOST_DEVICE constexpr int epi_quarter(int warp) { return warp & 3; }
+SOUFFLE_HOST_DEVICE constexpr int epi_part(int warp) { return (warp - 2) >> 2; }
+SOUFFLE_HOST_DEVICE constexpr int epi_warp(int quarter, int part) { return 2 + 4 * part + ((quarter + 2) & 3); }
+// Each has two boxes for its stores; number of a warp's first one.
+SOUFFLE_HOST_DEVICE constexpr int epi_box(int warp) { return (warp - 2) * 2; }
+// The box through which the warps of a quarter exchange the statistics of their rows: the second one of its own part 1.
+SOUFFLE_HOST_DEVICE constexpr int ln_stats_box(int quarter) { return epi_box(epi_warp(quarter, 1)) + 1; }
+
 // q = n / d for n * d < 2^32 as one multiply-high: mg = ceil(2^32 / d); d == 1 has no 32-bit multiplier.
 inline uint32_t fast_div_magic(uint32_t d) { return d <= 1 ? 0u : (uint32_t)((0x100000000ull + d - 1) / d); }
 
