@@ -1499,7 +1499,11 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       for (int k = 0; ok && k < my_items; ++k) {
         const int g = k & 1;
         const uint32_t base = ring + g * kPipeBytes, bit = (bits >> g) & 1u;
-        if (!mbar_wait_hot(bar(g, AB_P_FULL), bit, ctl, 512 + g)) break;
+        if constexpr (kPair) {            // rows of P that warps of the other CTA have written
+          if (!mbar_wait_cluster(bar(g, AB_P_FULL), bit, ctl, 512 + g)) break;
+        } else {
+          if (!mbar_wait_hot(bar(g, AB_P_FULL), bit, ctl, 512 + g)) break;
+        }
         if (!mbar_wait_hot(bar(g, AB_V_FULL), bit, ctl, 514 + g)) break;
         tc_fence_after_sync();
         // O = P V: K = 128 keys = two chunks of 64; V is an MN-major B operand (16 keys = 2048 B per step)
@@ -1645,7 +1649,7 @@ __device__ __forceinline__ void attn_stage_pp(const Stage& st, const CallArgs& c
       tc_fence_before_sync();
       if constexpr (kPair) {                                  // one arrival per warp on the leader's barrier (8 in all)
         __syncwarp();
-        if (lane == 0) mbar_arrive_cluster_relaxed(map_shared_rank(bar(g, AB_P_FULL), 0));      // P is read by this SM's own tensor core
+        if (lane == 0) mbar_arrive_cluster(map_shared_rank(bar(g, AB_P_FULL), 0));
       } else {
         mbar_arrive(bar(g, AB_P_FULL));
       }

@@ -346,10 +346,23 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const void* tmap,
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
-// Arrival on an mbarrier of another CTA of the cluster (`bar` is a shared::cluster address), with the default (CTA-scope) release: for
-// hand-shakes that protect tensor memory, whose reads tcgen05.fence::before_thread_sync has already ordered before the arrival, or
-// shared memory that this SM's own tensor core reads, behind fence.proxy.async.  A cluster-scope release waits for all of the thread's
-// earlier writes, global stores still in flight included: 1.7 k cycles after an epilogue's stores, 1.1 k after a softmax.
+// Arrival on an mbarrier of another CTA of the cluster (`bar` is a shared::cluster address), releasing to the cluster: the thread that
+// waits there with mbar_wait_cluster has this thread's earlier writes, and by them may have the tensor core read.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, const WaitCtl& c, int where) {
+  if (!mbar_wait_hot(bar, parity, c, where)) return false;
+  asm volatile(                       // the phase is complete: this only acquires
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%0], %1;\n\t}"
+      ::"r"(bar), "r"(parity)
+      : "memory");
+  return true;
+}
+// The same arrival with the default (CTA-scope) release, for hand-shakes that protect tensor memory, whose reads
+// tcgen05.fence::before_thread_sync has already ordered before the arrival.  A cluster-scope release waits for all of the thread's
+// earlier writes, plain global stores still in flight included: 1.7 k cycles after those of an epilogue.
 __device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }

@@ -254,6 +254,22 @@ def test_layernorm_in_the_epilogue(B, S, heads, ffn, tuning):
     enc.status()
 
 
+@pytest.mark.parametrize("B,S,heads,tuning", [(64, 128, 12, dict(pair_mma=1)), (21, 112, 12, dict(pair_mma=1)), (64, 80, 4, dict(pair_mma=-1))])
+def test_calls_repeat_themselves_bit_by_bit(B, S, heads, tuning):
+    """Hand-overs between warps and CTAs (probabilities to a pair's tensor cores, row statistics between the tiles of a row): a call in
+    which one came too early or too late would differ from the next with the same input.  No sum depends on timing, so none may."""
+    cfg = so.BertConfig(B, S, heads, 64, 1024, "std")
+    layers = so.make_bert_weights(cfg, 1270, 2, zero_bias=False)
+    enc = _encoder(cfg, layers, tuning=tuning)
+    inputs = [[t.cuda() for t in so.make_bert_input(cfg, 1270 + i, True)] for i in range(2)]
+    first = [enc.forward(x, lens).clone() for x, lens in inputs]
+    assert not torch.equal(first[0], first[1])
+    for _ in range(25):
+        for (x, lens), want in zip(inputs, first):
+            assert torch.equal(enc.forward(x, lens), want)
+    enc.status()
+
+
 @pytest.mark.parametrize("stage", [0, 1, 2, 4])      # in front of attention, proj with LayerNorm 1, FC1, FC2 with LayerNorm 2
 def test_wait_limit_around_layernorm_in_the_epilogue(stage):
     from souffle_models_b200 import _lib
