@@ -78,7 +78,8 @@ typedef struct SouffleBertDesc {
   int32_t debug_skip_arrival; /* failure-detection test hook, 0 = off: CTA (low 16 bits - 1) leaves at the grid
                                  barrier behind stage (high 16 bits) without arriving, so the others run into the
                                  wait limit and the launch ends with SOUFFLE_DEVICE_TIMEOUT (nothing is in flight
-                                 at that point) */
+                                 at that point); -1: the kernel finds its shared memory unaligned and leaves at
+                                 once, which the plan's status reports as SOUFFLE_CUDA_ERROR */
   int32_t autotune;   /* 1: plan creation times the likeliest tilings of every GEMM stage on the device (a few
                          launches each on the plan's own buffers, tens of milliseconds in all) and keeps the
                          fastest; stages with an explicit bm_ / bn_ / split_ setting are left alone.  0: tiles come

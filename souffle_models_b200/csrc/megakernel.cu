@@ -64,7 +64,7 @@ struct MegaParams {
   int* expired;       // host memory or null: set by a CTA that gave up on a wait
   unsigned long long timeout_ns;
   int max_slots;      // experiment knob: cap on operand ring slots, 0 = as many as fit
-  int skip_arrival;   // test hook: CTA (low 16 bits - 1) leaves without arriving after stage (high 16 bits); 0 = off
+  int skip_arrival;   // test hook: CTA (low 16 bits - 1) leaves without arriving after stage (high 16 bits); 0 = off; -1: see kSmemAlign
   long long* prof;    // optional [n_stages][grid][8]: clock64 at stage start, work done, barrier left, then GEMM
                       // role cycles: MMA waiting for operands, MMA waiting for a free accumulator, producer
                       // waiting for a free slot, epilogue waiting for an accumulator, epilogue busy
@@ -83,7 +83,8 @@ __device__ __forceinline__ const CUtensorMap* map_ptr(const CallArgs& a, int idx
   return idx < 0 ? &a.call_maps[-idx - 1] : a.p.maps + idx;
 }
 
-extern __shared__ __align__(1024) uint8_t smem_raw[];      // swizzled tiles need 1024-byte alignment
+constexpr uint32_t kSmemAlign = 1024;        // of swizzled tiles: descriptors and copies take it for granted, so the prologue looks
+extern __shared__ __align__(kSmemAlign) uint8_t smem_raw[];
 
 struct __align__(8) SmemCtl {
   uint64_t full[kMaxSlots];
@@ -2493,6 +2494,14 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[0] = clock64();
     pr[3] = (long long)globaltimer_ns();        // wall clock shared by all SMs: launch skew between CTAs
+  }
+  // The same for all CTAs of a launch: nobody waits for those that leave here.  (Test hook -1: an alignment that no base has.)
+  if (smem_u32(smem_raw) & ((p.skip_arrival == -1 ? 1u << 20 : kSmemAlign) - 1u)) {
+    if (threadIdx.x == 0) {
+      p.status[0] = DEV_SMEM_BASE;
+      if (p.expired) *p.expired = 1;
+    }
+    return;
   }
   SmemCtl& cs = *reinterpret_cast<SmemCtl*>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

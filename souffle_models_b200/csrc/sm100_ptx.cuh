@@ -17,6 +17,7 @@ enum DeviceStatus : int {
   DEV_TIMEOUT_MBAR = 1,   // an mbarrier wait ran out of time
   DEV_TIMEOUT_GRID = 2,   // the grid barrier ran out of time
   DEV_TIMEOUT_FLAG = 3,   // a dataflow flag wait ran out of time
+  DEV_SMEM_BASE = 4,      // shared memory does not begin where the swizzled tiles need it to
 };
 
 struct WaitCtl {

@@ -622,6 +622,7 @@ static int read_status(const int* words, int h[4]) {
 
 static int decode_status(const int* h, const char* what) {
   if (h[0] == DEV_OK) return SOUFFLE_OK;
+  if (h[0] == DEV_SMEM_BASE) return fail(SOUFFLE_CUDA_ERROR, "%s: shared memory does not begin at a multiple of %u bytes", what, kSmemAlign);
   return fail(SOUFFLE_DEVICE_TIMEOUT, "%s: device wait expired (code %d, where %d, cta %d)", what, h[0], h[1], h[2]);
 }
 

@@ -285,6 +285,26 @@ def test_wait_limit_around_layernorm_in_the_epilogue(stage):
     bad.close()
 
 
+@pytest.mark.parametrize("B,pair", [(1, 0), (40, -1), (20, 1)])
+def test_unaligned_shared_memory_is_reported(B, pair):
+    """Swizzled tiles need their base aligned; a launch that does not find it so says so instead of computing with it."""
+    from souffle_models_b200 import _lib
+    cfg = so.BertConfig(B, 128, 12, 64, 128, "std")
+    layers = so.make_bert_weights(cfg, 3, 1)
+    x, _ = so.make_bert_input(cfg, 3)
+    bad = _encoder(cfg, layers, tuning=dict(pair_mma=pair, debug_skip_arrival=-1))
+    for _ in range(2):
+        bad.forward(x.cuda())
+        with pytest.raises(_lib.SouffleError) as ei:
+            bad.status()
+        assert ei.value.code == 5 and "multiple of 1024 bytes" in str(ei.value)
+    bad.close()
+    good = _encoder(cfg, layers, tuning=dict(pair_mma=pair))
+    y = good.forward(x.cuda())
+    good.status()
+    assert _err(y.reshape(B * 128, 768), so.bert_layer(cfg, x, layers[0], None)["out"]) < TOL_LAYER
+
+
 @pytest.mark.parametrize("B,S,heads,ffn", [
     (1, 16, 2, 128),       # rows of 128 columns: one warp, the second block of columns is absent
     (9, 384, 2, 256),      # the same in two passes, the second one ragged
