@@ -41,12 +41,14 @@
 #include <type_traits>
 
 #include "sm100_ptx.cuh"
+#include "stage_program.h"
 
 namespace souffle {
 
 constexpr int kLstmParts = 8;                      // CTAs per layer = cluster size
 constexpr int kLstmXBufs = 4;                      // input vectors the fetch warp may run ahead
 constexpr int kLstmMaxLayers = 18;
+static_assert(kLstmMaxLayers * kLstmParts <= (int)kLaunchSteps, "more CTAs than a launch number has steps for");
 // threads of a CTA: a cell warp per 32 hidden units of the layer (it owns four of the CTA's), and the fetch warp
 __host__ __device__ constexpr int lstm_block(int H) { return (H / 32 + 1) * 32; }
 
@@ -57,7 +59,8 @@ struct LstmParams {
   const float* x;         // [T][H]
   float* y;               // [T][H]: top layer's h per step
   uint64_t* h_all;        // [L][T][H] scratch: every published hidden state (low half) beside the launch's tag
-  unsigned* epoch;        // launches on this scratch so far; the tag is one more, which no word of the scratch holds yet
+  unsigned long long* epoch;      // counter of the launches on this scratch (see launch_step): the tag is one more than this one's
+                                  // number, which no word of the scratch holds yet
   int* status;
   int* expired;           // host memory or null: set by a CTA that gave up on a wait
   int layers, hidden, steps, ref_input_delay;
@@ -370,7 +373,7 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
     sh.abort = 0;
     sh.deadline_ns = globaltimer_ns() + p.timeout_ns;
     sh.pieces = 0;
-    sh.tag = *const_cast<volatile unsigned*>(p.epoch) + 1u;
+    sh.tag = (uint32_t)(atomicAdd(p.epoch, (unsigned long long)launch_step(blockIdx.x, gridDim.x)) / kLaunchSteps) + 1u;
     for (int i = 0; i < kLstmXBufs; ++i) {
       mbar_init(xfull0 + 8 * i, 32);            // the 32 lanes of the fetch warp
       mbar_init(xempty0 + 8 * i, kWarps);       // one lane of every cell warp
@@ -532,8 +535,6 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();
   cluster_sync_all();
-  // the top layer has had every word of the layers below, so every CTA has read the epoch
-  if (layer == L - 1 && part == 0 && tid == 0) *p.epoch = sh.tag;
   if (*const_cast<volatile int*>(&sh.abort)) {   // sent by peers before they came here, and not waited for: 200 us are ample
     if (tid == 0 && p.expired) *p.expired = 1;
     const unsigned long long t0 = globaltimer_ns();

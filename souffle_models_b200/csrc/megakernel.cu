@@ -59,7 +59,7 @@ struct MegaParams {
   const int* lens;
   unsigned* sync;       // [0] arrival count, [1] generation used by this launch
   unsigned* sync_next;  // the pair the next launch will use; cleared by this launch
-  unsigned* epoch;      // plan-owned word that this launch increments at its end (EPI_LN tags), or null
+  unsigned* epoch;      // plan-owned counter (see launch_step) whose launch numbers tag EPI_LN statistics, or null
   int* status;        // [0] code, [1] where, [2] cta
   int* expired;       // host memory or null: set by a CTA that gave up on a wait
   unsigned long long timeout_ns;
@@ -100,7 +100,7 @@ struct __align__(8) SmemCtl {
   int leave[2];                     // a wait has run out: all warps leave the stage loop together
   uint32_t arrived;                 // stages whose arrival this CTA has sent
   uint32_t go;                      // stages that may start, as published by the feeder (publish_go / wait_go / stage_go)
-  uint32_t epoch;                   // of this launch, see RowStat
+  uint32_t epoch;                   // this launch's number x kLaunchSteps, see RowStat
   WaitCtl wait;                     // here and not on the stack: see RoleState
   alignas(16) float bias[2][256];   // of this tile's and the next tile's columns
   alignas(16) Stage stage[2];       // records of this stage and the next, by the parity of their ordinals
@@ -478,7 +478,7 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
     for (int i = 0; i < 4; ++i) rowptr[i] = so[i] != kNoRow ? reinterpret_cast<uint8_t*>(to + (so[i] + (uint32_t)col)) : nullptr;
     staged_store_64B(sbuf, w, rowptr, lane);
   };
-  const uint32_t tag = (cs.epoch << 8) | st.ordinal;
+  const uint32_t tag = cs.epoch | st.ordinal;
   const float inv_n = 1.0f / (float)st.N;
   const bool prof = p.prof != nullptr, affine = st.gamma != nullptr;
   float* bias_s = cs.bias[0];
@@ -2533,7 +2533,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
     cs.abort = 0;
     cs.leave[0] = cs.leave[1] = 0;
     cs.go = cs.arrived = 0u;
-    cs.epoch = p.epoch ? *p.epoch : 0u;
+    cs.epoch = p.epoch ? *const_cast<volatile unsigned*>(p.epoch) & ~(kLaunchSteps - 1u) : 0u;
     cs.wait.abort_smem = &cs.abort;
     cs.wait.status_g = p.status;
     cs.wait.deadline_ns = globaltimer_ns() + p.timeout_ns;      // read once per CTA
@@ -2643,7 +2643,7 @@ souffle_megakernel(const __grid_constant__ CallArgs ca) {
   }
 
   __syncthreads();
-  if (p.epoch && blockIdx.x == 0 && threadIdx.x == 0) *p.epoch = cs.epoch + 1u;      // every CTA has read it: all have been in a grid barrier
+  if (p.epoch && threadIdx.x == 0) atomicAdd(p.epoch, launch_step(blockIdx.x, gridDim.x));
   if (p.prof && threadIdx.x == 0) {
     long long* pr = p.prof + ((size_t)p.n_stages * gridDim.x + blockIdx.x) * kProfSlots;
     pr[2] = clock64();

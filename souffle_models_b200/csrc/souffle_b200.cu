@@ -376,6 +376,7 @@ static int device_info(DeviceInfo** out) {
       if (n < per_sm) per_sm = n;
     }
     d.max_ctas = per_sm * d.sms;
+    if (d.max_ctas > (int)kLaunchSteps) d.max_ctas = (int)kLaunchSteps;
     if (d.max_ctas < 1) return fail(SOUFFLE_NOT_CORESIDENT, "megakernel does not fit on an SM of device %d", dev);
     {   // the build that runs on CTA pairs: how many clusters of two fit the device at once
       const void* pf = (const void*)souffle_megakernel<kFamilyBertPair>;
@@ -2103,7 +2104,7 @@ struct SouffleLstmPlan {
   __half *w_in = nullptr, *w_state = nullptr;
   float* bias = nullptr;
   uint64_t* h_all = nullptr;
-  unsigned* epoch = nullptr;
+  unsigned long long* epoch = nullptr;
   int* status = nullptr;
 };
 
@@ -2248,7 +2249,7 @@ int souffle_lstm_forward_static(const SouffleLstmDesc* desc, const void* w_in, c
   lp.w_state = reinterpret_cast<const __half*>(w_state);
   lp.bias = bias; lp.x = x; lp.y = y;
   lp.h_all = reinterpret_cast<uint64_t*>(sd.scratch);
-  lp.epoch = reinterpret_cast<unsigned*>(sd.scratch + kStaticEpochOffset);
+  lp.epoch = reinterpret_cast<unsigned long long*>(sd.scratch + kStaticEpochOffset);
   lp.expired = nullptr;                  // the words below are read unasked; nothing is allocated here
   lp.status = device_status ? reinterpret_cast<int*>(device_status) : reinterpret_cast<int*>(sd.scratch + kStaticStatusOffset);
   lp.layers = d.layers; lp.hidden = d.hidden; lp.steps = d.steps; lp.ref_input_delay = d.ref_input_delay;

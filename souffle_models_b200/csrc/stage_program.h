@@ -128,6 +128,12 @@ SOUFFLE_HOST_DEVICE constexpr int epi_box(int warp) { return (warp - 2) * 2; }
 // The box through which the warps of a quarter exchange the statistics of their rows: the second one of its own part 1.
 SOUFFLE_HOST_DEVICE constexpr int ln_stats_box(int quarter) { return epi_box(epi_warp(quarter, 1)) + 1; }
 
+// Launches on one scratch are told apart by a counter in it: a launch's number is the counter / kLaunchSteps.  A CTA reads it when it
+// starts and adds its step, then or when it leaves.  The steps of a launch make kLaunchSteps together, so until the last CTA has read it
+// the number stays: a CTA that starts after others have given up and gone still marks its words as this launch's, not as the next one's.
+constexpr uint32_t kLaunchSteps = 256;      // CTAs of a launch at most
+SOUFFLE_HOST_DEVICE constexpr uint32_t launch_step(uint32_t cta, uint32_t ctas) { return cta == 0 ? kLaunchSteps - (ctas - 1) : 1u; }
+
 // q = n / d for n * d < 2^32 as one multiply-high: mg = ceil(2^32 / d); d == 1 has no 32-bit multiplier.
 inline uint32_t fast_div_magic(uint32_t d) { return d <= 1 ? 0u : (uint32_t)((0x100000000ull + d - 1) / d); }
 

@@ -30,3 +30,15 @@ def test_row_statistics_lie_in_a_box_of_a_warp_with_the_same_rows(tmp_path):
     }
   for (int w = 2; w < 10; ++w) CHECK(epi_warp(epi_quarter(w), epi_part(w)) == w);
 """)
+
+
+def test_a_late_cta_reads_the_number_of_its_own_launch(tmp_path):
+    """Whichever other CTAs of a launch have left before it starts; and the next launch's number is the next one."""
+    _run(tmp_path, """
+  for (uint32_t ctas = 1; ctas <= kLaunchSteps; ++ctas) {
+    uint32_t all = 0;
+    for (uint32_t c = 0; c < ctas; ++c) all += launch_step(c, ctas);
+    CHECK(all == kLaunchSteps);
+    for (uint32_t late = 0; late < ctas; ++late) CHECK(launch_step(late, ctas) >= 1 && all - launch_step(late, ctas) < kLaunchSteps);
+  }
+""")
