@@ -1998,6 +1998,10 @@ int souffle_swin_stage_plan_create(const SouffleSwinDesc* desc, const SouffleSwi
     return fail(SOUFFLE_BAD_SHAPE, "dim %d must be 128, 256, 512, 768 or 1024", d.dim);
   if (d.heads < 2 || d.heads % 2 || d.heads * 32 != d.dim) return fail(SOUFFLE_BAD_SHAPE, "heads must be even with dim / heads == 32");
   if (d.mlp_ratio < 1 || d.dim * d.mlp_ratio > 4096) return fail(SOUFFLE_BAD_SHAPE, "dim * mlp_ratio must be in (0, 4096]");
+  // as many windows as 64-row slots of 2^20 rows, and Q, K and V of less than 2^31 values
+  const long long windows = (long long)d.batch * (d.res / d.window) * (d.res / d.window), tokens = windows * d.window * d.window;
+  if (windows > (1 << 14) || tokens * 3 * d.dim >= 0x7FFF8000ll)
+    return fail(SOUFFLE_BAD_SHAPE, "batch %d of %d x %d tokens of %d values is too large", d.batch, d.res, d.res, d.dim);
   for (int i = 0; i < (d.n_blocks > 0 ? d.n_blocks : 1); ++i)
     if (!aligned16(weights[i].qkv_w) || !aligned16(weights[i].proj_w) || !aligned16(weights[i].fc1_w) || !aligned16(weights[i].fc2_w))
       return fail(SOUFFLE_BAD_POINTER, "block %d: weight matrices must be non-null and 16-byte aligned", i);

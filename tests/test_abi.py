@@ -124,3 +124,19 @@ def test_packed_parameter_block_layout():
     assert [off(p) - v for p in (w.qkv_b, w.proj_b, w.ln1_g, w.ln1_b, w.fc1_b, w.fc2_b, w.ln2_g, w.ln2_b)] == \
         [0, 3 * H, 4 * H, 5 * H, 6 * H, 6 * H + F, 7 * H + F, 8 * H + F]
     assert lib.souffle_bert_packed_weights(base, 1, 3, H, F, None, None, None) != 0      # mask would break the alignment
+
+
+@pytest.mark.parametrize("batch,res,dim,window,shape_ok", [
+    (1 << 14, 7, 128, 7, True), ((1 << 14) + 1, 7, 128, 7, False),          # windows
+    (1, 1024, 128, 8, True), (1, 1032, 128, 8, False),
+    (682, 32, 1024, 8, True), (683, 32, 1024, 8, False),                    # values of Q, K and V
+])
+def test_swin_plans_of_too_many_tokens_are_refused(batch, res, dim, window, shape_ok):
+    """The sizes are looked at before the weights, of which there are none here."""
+    lib = _lib.load()
+    d = _lib.SwinDesc(batch=batch, res=res, dim=dim, heads=dim // 32, window=window, mlp_ratio=1, eps=1e-5, n_blocks=1)
+    w, h = (_lib.SwinWeights * 1)(), C.c_void_p()
+    rc = lib.souffle_swin_stage_plan_create(C.byref(d), w, None, C.byref(h))
+    assert rc == (2 if shape_ok else 1), lib.souffle_last_error()
+    assert h.value is None
+    assert (b"too large" in lib.souffle_last_error()) == (not shape_ok)
