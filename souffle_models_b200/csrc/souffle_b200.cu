@@ -415,6 +415,8 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
     s.prev = (uint8_t)(i > 0 ? i - 1 : 0);
     s.next = (uint8_t)(i + 1);
   }
+  // a single stage waits for no CTA, or none outside its pair, unless its tiles exchange row statistics: a plain launch does
+  const bool waits = args.p.n_stages > 1 || (!args.p.stages && args.inline_stages[0].type == STAGE_GEMM && args.inline_stages[0].epi == EPI_LN);
   void* kargs[] = {&args};
   if (family == kFamilyBertPair) {
     // Clusters of two CTAs.  All CTAs must be resident at once (the grid barrier): the grid never exceeds what
@@ -440,7 +442,7 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
     at[1].val.cooperative = 1;
     cfg.attrs = at;
     const void* fn = (const void*)souffle_megakernel<kFamilyBertPair>;
-    if (env_coop && di->pair_coop && args.p.n_stages > 1) {          // (a single stage waits for no CTA outside its pair)
+    if (env_coop && di->pair_coop && waits) {
       cfg.numAttrs = 2;
       if (cudaLaunchKernelExC(&cfg, fn, kargs) == cudaSuccess) return SOUFFLE_OK;
       cudaGetLastError();          // a refused launch configuration is not sticky
@@ -453,8 +455,7 @@ static int launch_mega(const CallArgs& args_in, int grid, cudaStream_t stream, i
   const void* fn = family == kFamilySwin ? (const void*)souffle_megakernel<kFamilySwin>
                    : family == kFamilyBertCoop ? (const void*)souffle_megakernel<kFamilyBertCoop>
                                                : (const void*)souffle_megakernel<kFamilyBert>;
-  // (a single stage waits for no other CTA: a plain launch does)
-  if (args.p.n_stages == 1) {
+  if (!waits) {
     SF_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(kThreads), kargs, (size_t)kSmemBytes, stream));
     return SOUFFLE_OK;
   }
@@ -603,6 +604,7 @@ static int is_captured(cudaStream_t st, bool* captured) {
 // words: the pairs of alternate launches (0-3), a captured launch's pair (4, 5) and the pair it clears for nobody (6, 7).
 constexpr int kCapturedPair = 4;
 constexpr int kEpochWord = 8;          // behind them, in a plan: MegaParams::epoch
+constexpr int kTuneEpochWord = 32;     // in the scratch of autotune_gemm, which clears the words in front before every launch
 static int pick_barrier_words(unsigned* words, unsigned launches, bool captured, cudaStream_t st, MegaParams* mp) {
   if (captured && mp->n_stages > 1) SF_CUDA(cudaMemsetAsync(words + kCapturedPair, 0, 2 * sizeof(unsigned), st));
   const unsigned at = captured ? kCapturedPair : 2u * (launches & 1u);
@@ -816,10 +818,18 @@ static Stage blank_stage(int type) {
 // the plan will build it (shape, epilogue, output pointers) without tile fields; its operands are read through
 // per-call tensor maps over `a` ([M][K]) and `w` ([N][K]), whose contents do not matter for the timing.  A stage
 // that writes split-K planes is timed together with the LayerNorm stage that sums them (`ln_proto`), since more
-// planes make that one slower: in the plan's own build of the kernel (`family`), whose LayerNorm stages differ.  Failures of any
-// kind leave `*choice` as the cycle model set it.
+// planes make that one slower: in the plan's own build of the kernel (`family`), whose LayerNorm stages differ.  Tilings with which the
+// plan normalises in the product's epilogue (`fuse`) are timed so.  Failures of any kind leave `*choice` as the cycle model set it.
+struct TuneFuse {
+  int max_tiles_n = 0;           // see can_fuse in build_bert_plan; 0: none
+  RowStat* stats = nullptr;
+  const void* unit = nullptr;    // 64 x 64
+};
+static bool fuses_layernorm(const TileChoice& t, int N, int max_tiles_n) {
+  return t.split == 1 && t.bn % 32 == 0 && t.bn >= 64 && N / t.bn <= max_tiles_n;
+}
 static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void* a, const void* w, int sms, bool allow_split,
-                          int head_split, int max_split, void* tune_ws, TileChoice* choice, int family) {
+                          int head_split, int max_split, void* tune_ws, TileChoice* choice, int family, const TuneFuse& fuse = TuneFuse()) {
   const bool pair = family == kFamilyBertPair;
   std::vector<RankedTile> ranked;
   if (pair) choose_tiles_pair(proto.M, proto.N, proto.K, sms / 2, allow_split, false, &ranked);
@@ -836,6 +846,13 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
     Stage& g = args.inline_stages[0];
     g = proto;
     g.tm_a = -1; g.tm_b = -2; g.bm = t.bm; g.bn = t.bn; g.splitk = t.split;
+    const bool fused = ln_proto && fuses_layernorm(t, proto.N, fuse.max_tiles_n);
+    if (fused) {
+      g.epi = EPI_LN; g.stats = fuse.stats; g.tm_resid = -4; g.tm_unit = -5; g.out = ln_proto->out; g.eps = ln_proto->eps;
+      if (make_map_uncached(&args.call_maps[3], ln_proto->resid, (uint64_t)proto.M, (uint64_t)proto.N, (uint32_t)(pair ? 128 : t.bm)) ||
+          make_map_uncached(&args.call_maps[4], fuse.unit, 64, 64, pair ? 32u : 64u))
+        continue;
+    }
     if (finalize_stage(g, 0, 1, pair)) continue;
     if (make_map_uncached(&args.call_maps[0], a, (uint64_t)proto.M, (uint64_t)proto.K, (uint32_t)(pair ? 128 : t.bm))) continue;
     if (make_map_uncached(&args.call_maps[1], w, (uint64_t)proto.N, (uint64_t)proto.K, (uint32_t)(pair ? t.bn / 2 : t.bn))) continue;
@@ -852,7 +869,7 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
     g.tm_out = -3;
     int items = stage_items(g) * (pair ? 2 : 1);                // CTAs that have work
     args.p.n_stages = 1;
-    if (ln_proto) {
+    if (ln_proto && !fused) {
       Stage& ln = args.inline_stages[1];
       ln = *ln_proto;
       ln.n_partial = t.split;
@@ -861,8 +878,9 @@ static void autotune_gemm(const Stage& proto, const Stage* ln_proto, const void*
       args.p.n_stages = 2;
     }
     const int grid = items < sms ? items : sms;                 // even for pairs: items and sms both are
-    if (ln_proto && finalize_stage(args.inline_stages[1], 0, grid)) continue;
+    if (args.p.n_stages > 1 && finalize_stage(args.inline_stages[1], 0, grid)) continue;
     args.p.sync = reinterpret_cast<unsigned*>(tune_ws);
+    args.p.epoch = args.p.sync + kTuneEpochWord;           // goes on from launch to launch
     args.p.sync_next = args.p.sync + 2;
     args.p.status = reinterpret_cast<int*>(reinterpret_cast<char*>(tune_ws) + 64);
     args.p.timeout_ns = 200ull * 1000000ull;
@@ -959,15 +977,28 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   if (d.bm_fc2) t_fc2.bm = d.bm_fc2;
   if (d.bn_fc2) t_fc2.bn = d.bn_fc2;
   if (d.split_fc2) t_fc2.split = d.split_fc2;
+  // LayerNorm in the product's epilogue (see gemm_ln_epilogue) where the product is not cut along K, from 2048 rows on: below, products
+  // that are not cut have more tiles per row and shorter LayerNorm stages (twelve layers of 128 tokens, as planes / in the epilogue:
+  // 13 sequences 676 / 675 us, 16 732 / 660, 32 1044 / 946, 64 1795 / 1550; six layers of 30 x 80 at hidden 512 310 / 276).  The
+  // build for few attention items does not have it: it would spill.
+  const int max_tiles_n = M >= 2048 && p->family != kFamilyBertCoop ? (pair ? npairs : sms) : 0;
+  auto can_fuse = [&](const TileChoice& t) { return fuses_layernorm(t, H, max_tiles_n); };
   if (d.autotune) {
     // Scratch for the measurements: a weight-shaped operand, as many fp32 planes as the deepest split tried
-    // (capped at 256 MB), barrier words.  Activation-shaped operands are the plan's own buffers.
+    // (capped at 256 MB), barrier words, row statistics.  Activation-shaped operands are the plan's own buffers.
     const size_t w_bytes = (size_t)(3 * H > F ? 3 * H : F) * H * 2;
     int max_split = (int)((256ull << 20) / ((size_t)M * H * 4));
     max_split = max_split > 16 ? 16 : (max_split < 1 ? 1 : max_split);
-    void *w_tmp = nullptr, *planes = nullptr, *tune_ws = nullptr;
+    void *w_tmp = nullptr, *planes = nullptr, *tune_ws = nullptr, *stats = nullptr;
+    const size_t stats_bytes = (size_t)((M + 255) / 256) * 256 * (H / 64) * sizeof(RowStat);
+    TuneFuse fuse;
     if (cudaMalloc(&w_tmp, w_bytes) == cudaSuccess && cudaMalloc(&planes, (size_t)max_split * M * H * 4) == cudaSuccess &&
-        cudaMalloc(&tune_ws, 256) == cudaSuccess && cudaMemset(w_tmp, 0, w_bytes) == cudaSuccess) {
+        cudaMalloc(&tune_ws, 256) == cudaSuccess && cudaMemset(w_tmp, 0, w_bytes) == cudaSuccess &&
+        cudaMemset(tune_ws, 0, 256) == cudaSuccess && cudaMalloc(&stats, stats_bytes) == cudaSuccess &&
+        cudaMemset(stats, 0xff, stats_bytes) == cudaSuccess) {
+      fuse.max_tiles_n = max_tiles_n;
+      fuse.stats = reinterpret_cast<RowStat*>(stats);
+      fuse.unit = w_tmp;                       // (no unit matrix: what it holds does not matter for the timing either)
       Stage ln = blank_stage(STAGE_LN);
       ln.M = M; ln.N = H; ln.ldo = H; ln.partial = reinterpret_cast<float*>(planes); ln.resid = p->ctx; ln.out = p->ln1;
       ln.eps = d.eps;
@@ -986,12 +1017,12 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
       if (!d.bm_proj && !d.bn_proj && !d.split_proj) {
         Stage f = g;
         f.N = H; f.K = H; f.epi = EPI_PARTIAL; f.partial = reinterpret_cast<float*>(planes); f.ldo = H;
-        autotune_gemm(f, &ln, p->ctx, w_tmp, sms, true, 0, max_split, tune_ws, &t_proj, p->family);
+        autotune_gemm(f, &ln, p->ctx, w_tmp, sms, true, 0, max_split, tune_ws, &t_proj, p->family, fuse);
       }
       if (!d.bm_fc2 && !d.bn_fc2 && !d.split_fc2) {
         Stage f = g;
         f.N = H; f.K = F; f.epi = EPI_PARTIAL; f.partial = reinterpret_cast<float*>(planes); f.ldo = H;
-        autotune_gemm(f, &ln, p->fc1, w_tmp, sms, true, 0, max_split, tune_ws, &t_fc2, p->family);
+        autotune_gemm(f, &ln, p->fc1, w_tmp, sms, true, 0, max_split, tune_ws, &t_fc2, p->family, fuse);
       }
     }
     cudaDeviceSynchronize();
@@ -999,6 +1030,7 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
     if (w_tmp) cudaFree(w_tmp);
     if (planes) cudaFree(planes);
     if (tune_ws) cudaFree(tune_ws);
+    if (stats) cudaFree(stats);
   }
   if (pair) t_qkv.bm = t_fc1.bm = t_proj.bm = t_fc2.bm = 256;      // a pair's tile is 256 rows: 128 per CTA
   auto bad_tile = [pair](const TileChoice& t, int N, bool divides = true) {
@@ -1017,13 +1049,6 @@ static int build_bert_plan(SouffleBertPlan* p, const SouffleBertLayerWeights* la
   const int bn_qkv = t_qkv.bn, bn_fc1 = t_fc1.bn, bn_proj = t_proj.bn, sp_proj = t_proj.split, bn_fc2 = t_fc2.bn,
             sp_fc2 = t_fc2.split;
   const int max_split = sp_proj > sp_fc2 ? sp_proj : sp_fc2;
-  // LayerNorm in the product's epilogue (see gemm_ln_epilogue) where the product is not cut along K, from 2048 rows on: below, products
-  // that are not cut have more tiles per row and shorter LayerNorm stages (twelve layers of 128 tokens, as planes / in the epilogue:
-  // 13 sequences 676 / 675 us, 16 732 / 660, 32 1044 / 946, 64 1795 / 1550; six layers of 30 x 80 at hidden 512 310 / 276).  The
-  // build for few attention items does not have it: it would spill.
-  auto can_fuse = [&](const TileChoice& t) {
-    return M >= 2048 && p->family != kFamilyBertCoop && t.split == 1 && t.bn % 32 == 0 && t.bn >= 64 && H / t.bn <= (pair ? npairs : sms);
-  };
   const bool fuse_proj = can_fuse(t_proj), fuse_fc2 = can_fuse(t_fc2);
   RowStat* stats[2] = {nullptr, nullptr};
   for (int i = 0; i < 2; ++i)

@@ -270,6 +270,25 @@ def test_calls_repeat_themselves_bit_by_bit(B, S, heads, tuning):
     enc.status()
 
 
+@pytest.mark.parametrize("B,S,heads,ffn,settings", [
+    (16, 128, 12, 3072, {}),                                      # single CTAs
+    (24, 128, 12, 3072, dict(pair_mma=1, bn_proj=192, split_proj=1)),
+    (64, 48, 4, 256, {}),                                         # one tile per row
+    (30, 128, 16, 1024, dict(split_fc2=2)),
+])
+def test_autotuned_plans_that_normalise_in_the_epilogue(B, S, heads, ffn, settings):
+    """From 2048 rows on a tiling without a cut along K is timed as the plan runs it; whatever is chosen is the same layer, and its
+    statistics start from a clean array."""
+    cfg = so.BertConfig(B, S, heads, 64, ffn, "std")
+    enc, layers, x, lens, y = _run(cfg, 1280, n_layers=2, ragged=True, zero_bias=False, tuning=dict(autotune=1, **settings))
+    for product, ln in ((2, 3), (5, 6)):
+        t = enc.stage_info(product)
+        assert (enc.stage_info(ln)["items"] == 0) == (t["splitk"] == 1 and t["bn"] >= 64 and t["bn"] % 32 == 0)
+    assert _err(y, so.bert_stack(cfg, x, layers, lens)) < TOL_STACK_FP32
+    assert torch.equal(enc.forward(x.cuda(), lens.cuda()).float().cpu().reshape(y.shape), y)
+    enc.status()
+
+
 @pytest.mark.parametrize("stage", [0, 1, 2, 4])      # in front of attention, proj with LayerNorm 1, FC1, FC2 with LayerNorm 2
 def test_wait_limit_around_layernorm_in_the_epilogue(stage):
     from souffle_models_b200 import _lib
