@@ -129,8 +129,8 @@ SOUFFLE_HOST_DEVICE constexpr int epi_box(int warp) { return (warp - 2) * 2; }
 SOUFFLE_HOST_DEVICE constexpr int ln_stats_box(int quarter) { return epi_box(epi_warp(quarter, 1)) + 1; }
 
 // Launches on one scratch are told apart by a counter in it: a launch's number is the counter / kLaunchSteps.  A CTA reads it when it
-// starts and adds its step, then or when it leaves.  The steps of a launch make kLaunchSteps together, so until the last CTA has read it
-// the number stays: a CTA that starts after others have given up and gone still marks its words as this launch's, not as the next one's.
+// starts, and its step is added when it leaves.  The steps of a launch make kLaunchSteps together, so until the last CTA has read it the
+// number stays: a CTA that starts after others have given up and gone still marks its words as this launch's, not as the next one's.
 constexpr uint32_t kLaunchSteps = 256;      // CTAs of a launch at most
 SOUFFLE_HOST_DEVICE constexpr uint32_t launch_step(uint32_t cta, uint32_t ctas) { return cta == 0 ? kLaunchSteps - (ctas - 1) : 1u; }
 
