@@ -65,7 +65,7 @@ typedef struct SouffleBertDesc {
   int32_t variant;    /* SouffleBertVariant */
   int32_t keep_probs; /* 1: parity mode: the softmax probabilities of the LAST layer are materialised and that layer's
                          stage outputs stay readable (souffle_bert_plan_buffer); 0: they are undefined after the
-                         call (a layer's intermediates of more than half of L2 together are dropped from it once
+                         call (a layer's intermediates of more than a third of L2 together are dropped from it once
                          their last reader has run, so that they need not be written to DRAM) */
   float eps;          /* LayerNorm epsilon (applied in fp32) */
   /* Optional tiling overrides, 0 = choose automatically. */

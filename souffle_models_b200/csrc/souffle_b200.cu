@@ -702,17 +702,19 @@ static int upload_program(SouffleBertPlan* p) {
     s.dead_bytes[0] = s.dead_bytes[1] = 0;
     s.dead_ptr[0] = s.dead_ptr[1] = nullptr;
   }
-  // Buffers are dropped from L2 only where a layer's intermediates are larger than half of it: smaller ones are written anew
+  // Buffers are dropped from L2 only where a layer's intermediates are larger than half of it, or a third where it has no planes: smaller ones are written anew
   // before anything evicts them, and the drops cost time.  Beyond that they keep dead data from being written to DRAM.  128 tokens,
   // inputs that change from call to call, with drops / without: twelve layers of hidden 512 at 24 sequences (41 MB) 681 / 669 us,
   // of hidden 768 at 16 (41 MB) 748 / 740, 24 (61 MB) 895 / 896, 32 (82 MB) 1133 / 1143, 40 (102 MB) 1358 / 1379; one layer at 16
   // 66.0 / 65.9, 32 99.6 / 101.0, 48 (122 MB) 131.7 / 134.9, 64 (163 MB) 172.2 / 176.1.
-  // (With planes.  Where LayerNorm is in the products' epilogues a layer has less, and the drops decide little: twelve layers at 64
-  // sequences, 113 MB, 1426..1466 / 1434..1481 us, at 32, 57 MB, 827..863 / 829..849.)
+  // A layer with planes of 42 to 63 MB loses by them: six of 4 x 384 at hidden 1024 449.9 / 447.6, of 13 x 128 441.7 / 437.3.  One
+  // without planes has no LayerNorm stages to wait for the drops, and wins from a third of L2 on (12 x 32 x 128, 57 MB, moved 753 MB
+  // of DRAM without): 64 sequences 1644 / 1647, 32 913 / 926, 28 (50 MB) 858 / 870, six layers of 34 x 112 (53 MB) 423 / 447, of 60 x
+  // 64 457 / 469, of 36 x 128 at 512 362 / 367; below, 24 x 128 (42 MB) 744 / 748, 16 x 128 (28 MB) 657 / 655, 64 x 128 at 256 250 / 249.
   DeviceInfo* di = nullptr;
   if ((rc = device_info(&di))) return rc;
   for (const SouffleBertPlan::Dead& dd : p->dead_after) {
-    if (p->layer_bytes <= (size_t)di->l2_bytes / 2) break;
+    if (p->layer_bytes <= (size_t)di->l2_bytes / (p->partial ? 2 : 3)) break;
     const size_t next = next_of(dd.after_stage);
     if (next >= n) continue;                                       // nothing runs after it inside the launch
     Stage& nx = p->stages[next];

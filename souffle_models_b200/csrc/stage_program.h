@@ -98,7 +98,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   uint32_t pf_bytes;
   const void* pf_ptr;
   // ---- buffers whose last reader was the stage before this one (multiples of 128 bytes, 128-byte aligned), where a layer's
-  //      intermediates exceed half of L2: their lines are dropped from it at the start of this stage ----
+  //      intermediates take much of L2 (see upload_program): their lines are dropped from it at the start of this stage ----
   uint32_t dead_bytes[2];
   const void* dead_ptr[2];
   // ---- derived on the host by finalize_stage(): the kernel's lone producer / MMA lanes would otherwise

@@ -254,7 +254,8 @@ def test_layernorm_in_the_epilogue(B, S, heads, ffn, tuning):
     enc.status()
 
 
-@pytest.mark.parametrize("B,S,heads,tuning", [(64, 128, 12, dict(pair_mma=1)), (21, 112, 12, dict(pair_mma=1)), (64, 80, 4, dict(pair_mma=-1))])
+@pytest.mark.parametrize("B,S,heads,tuning", [(64, 128, 12, dict(pair_mma=1)), (21, 112, 12, dict(pair_mma=1)), (64, 80, 4, dict(pair_mma=-1)),
+                                              (40, 128, 12, {})])       # 50 MB a layer, without planes: dropped from L2
 def test_calls_repeat_themselves_bit_by_bit(B, S, heads, tuning):
     """Hand-overs between warps and CTAs (probabilities to a pair's tensor cores, row statistics between the tiles of a row): a call in
     which one came too early or too late would differ from the next with the same input.  No sum depends on timing, so none may."""
