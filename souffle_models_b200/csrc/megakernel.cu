@@ -687,7 +687,7 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
 }
 
 // The Swin build's: sums and reordered rows.
-__device__ __noinline__ uint32_t gemm_stage_ool(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<false, true>(ca, acc_bits); }
+__device__ __noinline__ uint32_t swin_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<false, true>(ca, acc_bits); }
 template <bool kPair>
 __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<kPair, false>(ca, acc_bits); }
 
@@ -945,7 +945,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     const int full_chunks = g.bn >> 5;
     if (kLnEpi && st.epi == EPI_LN) {
       const uint32_t which = (uint32_t)(&st == &ctl_s.stage[1]) << 31;
-      if constexpr (kSwin) rs.acc_bits = gemm_stage_ool(ca, rs.acc_bits | which);
+      if constexpr (kSwin) rs.acc_bits = swin_ln_epilogue(ca, rs.acc_bits | which);
       else rs.acc_bits = gemm_ln_epilogue<kPair>(ca, rs.acc_bits | which);
     } else {
     EpiCtx e;
@@ -2474,8 +2474,9 @@ __device__ __noinline__ uint32_t ln_stage_ool(const Stage& st, const MegaParams&
 //                    LayerNorm; every stage inlined into one register allocation (fastest).
 //   kFamilyBertCoop  the same with the attention stage in which all eight softmax warps share one item: S up to
 //                    384, and short sequences at small batch, where a CTA has at most one item anyway.
-//   kFamilySwin      adds the Swin row-permuting epilogues and the window-attention stage; its stages stay out
-//                    of line (inlined as well, the allocation would no longer fit).
+//   kFamilySwin      GEMM stages, whose LayerNorm epilogue can also store the sum and change the order of the rows, the
+//                    window-attention stage and the LayerNorm stages that sum, permute and merge; GEMM stages but for that
+//                    epilogue are inlined, the others stay out of line (the allocation would no longer fit).
 //   kFamilyBertPair  kFamilyBert on CTA pairs: a cluster of two CTAs shares every MMA (cta_group::2), which halves the
 //                    weight-tile traffic per FLOP of the GEMM stages; the attention stage takes two heads per pair.
 //                    Launched with a cluster dimension of two.

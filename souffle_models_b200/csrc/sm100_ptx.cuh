@@ -129,9 +129,7 @@ __device__ __forceinline__ void named_barrier_sync(int id, int nthreads) {
 // proxies and fences
 // ------------------------------------------------------------------------------------
 // Orders generic-proxy writes (st.global / st.shared) before later async-proxy reads (TMA, tcgen05).
-// The form without a state space measured ~900 cycles on a B200, the two restricted forms 3 and 10: hot paths name
-// the spaces they mean.
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
+// The form without a state space measured ~900 cycles on a B200, these two, which name the space they mean, 3 and 10.
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -212,18 +210,6 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {  
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 
-// Shared-memory matrix descriptor for a 128B-swizzled tile whose 8-row groups are 1024 B apart.
-//   bits [0,14) start>>4, [16,30) leading byte offset>>4, [32,46) stride byte offset>>4,
-//   [46,48) version=1 (Blackwell), [61,64) layout type (2 = SWIZZLE_128B).
-__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
 // Instruction descriptor, kind::f16, fp16 x fp16 -> fp32, A K-major, M=128.
 //   [4,6) D format (1=f32), [7,10) A fmt (0=f16), [10,13) B fmt, [15] A major, [16] B major (1 = MN),
 //   [17,23) N>>3, [24,29) M>>4.
@@ -240,8 +226,10 @@ __device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// High word of a SW128 descriptor (stride byte offset 1024, version 1, layout SWIZZLE_128B) and the
-// low word for a tile at `smem_addr` with leading byte offset `lbo_bytes`.
+// Shared-memory matrix descriptor for a 128B-swizzled tile whose 8-row groups are 1024 B apart.
+//   bits [0,14) start>>4, [16,30) leading byte offset>>4, [32,46) stride byte offset>>4,
+//   [46,48) version=1 (Blackwell), [61,64) layout type (2 = SWIZZLE_128B).
+// Its high word, and the low word for a tile at `smem_addr` with leading byte offset `lbo_bytes`.
 constexpr uint32_t kDescHiSw128 = (1024u >> 4) | (1u << 14) | (2u << 29);
 __device__ __forceinline__ uint32_t umma_desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) {
   return ((smem_addr >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
@@ -436,16 +424,8 @@ __device__ __forceinline__ void st_relaxed_tagged(void* p, uint32_t a, uint32_t 
 __device__ __forceinline__ void ld_relaxed_2x64(const void* p, uint64_t& a, uint64_t& b) {
   asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 }
-__device__ __forceinline__ unsigned atom_add_release_u32(unsigned* p, unsigned v) {
-  unsigned old;
-  asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-  return old;
-}
 __device__ __forceinline__ void red_add_release_u32(unsigned* p, unsigned v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
 // ------------------------------------------------------------------------------------
@@ -500,11 +480,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 __device__ __forceinline__ float tanh_fast(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -520,20 +495,9 @@ __device__ __forceinline__ float gelu_tanh(float x) {
   const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
   return 0.5f * x * (1.0f + tanh_fast(u));
 }
-// The same GELU on a pair of fp16 values (the result is stored as fp16 anyway): six packed operations and
-// one packed tanh for two elements.  Overflow of x*x saturates tanh at +-1, which is the right limit.
-__device__ __forceinline__ uint32_t gelu_tanh_h2(uint32_t xw) {
-  const __half2 x = *reinterpret_cast<const __half2*>(&xw);
-  const __half2 c0 = __float2half2_rn(0.7978845608028654f), c1 = __float2half2_rn(0.7978845608028654f * 0.044715f);
-  const __half2 u = __hmul2(x, __hfma2(__hmul2(x, x), c1, c0));
-  uint32_t uw = *reinterpret_cast<const uint32_t*>(&u), tw;
-  asm("tanh.approx.f16x2 %0, %1;" : "=r"(tw) : "r"(uw));
-  const __half2 t = *reinterpret_cast<const __half2*>(&tw);
-  const __half2 hx = __hmul2(x, __float2half2_rn(0.5f));
-  const __half2 y = __hfma2(hx, t, hx);
-  return *reinterpret_cast<const uint32_t*>(&y);
-}
-// Sixteen pairs at once, step by step: each loop is sixteen independent operations (see epilogue_chunk32).
+// The same GELU on pairs of fp16 values (the result is stored as fp16 anyway): six packed operations and one packed tanh for two
+// elements.  Overflow of x*x saturates tanh at +-1, which is the right limit.  Sixteen pairs at once, step by step: each loop is
+// sixteen independent operations (see epilogue_values32).
 __device__ __forceinline__ void gelu_tanh_h2x16(uint32_t (&w)[16]) {
   const __half2 c0 = __float2half2_rn(0.7978845608028654f), c1 = __float2half2_rn(0.7978845608028654f * 0.044715f);
   const __half2 half = __float2half2_rn(0.5f);

@@ -530,6 +530,7 @@ static int finalize_stage(Stage& s, int max_slots, int grid, bool pair = false) 
   }
   s.mg_heads = fast_div_magic((uint32_t)(s.heads > 0 ? s.heads : 1));
   if (s.type != STAGE_GEMM) return SOUFFLE_OK;
+  // (the kernel brings in a tile's bias at a time and has no limit of its own: these are the widths that plans take)
   if (s.bias && s.epi != EPI_PARTIAL && s.N > 4096)
     return fail(SOUFFLE_BAD_SHAPE, "a GEMM stage with a bias vector is limited to 4096 output columns (got %d)", s.N);
   s.tiles_n = (s.N + s.bn - 1) / s.bn;

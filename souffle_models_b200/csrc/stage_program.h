@@ -18,7 +18,7 @@ enum StageType : int {
 };
 
 enum EpilogueKind : int {
-  EPI_F16 = 0,      // out[row, col] = f16(act(acc + bias)) (+ resid)
+  EPI_F16 = 0,      // out[row, col] = f16(act(acc + bias))
   EPI_QKV = 1,      // like EPI_F16 but scattered head-split to [3][B][heads][S][d]
   EPI_PARTIAL = 2,  // raw fp32 accumulators to partial[split][row][col]
   EPI_LN = 3,       // f16(LayerNorm(acc + bias + resid)): the row's statistics come from all tiles that share it; sum_out, eps < 0 and
@@ -50,7 +50,7 @@ struct alignas(16) Stage {      // 16-byte multiples: records are copied 16 byte
   int out_stores;    // copies per box of 32 rows (2 where a sequence ends inside one)
   int M, N, K;
   int bm;            // tile height: 128, or 256 (two 128-row halves that share each B tile); STAGE_ATTN: query rows per item
-  int bn;            // tile width in N (multiple of 16, <= 256, divides N)
+  int bn;            // tile width in N (multiple of 16, <= 256; N may end inside the last tile, see ragged_width)
   int splitk;        // K is cut into this many independent partial products (STAGE_LN: warps that may share a row)
   int b_mn_major;    // 0: B stored [N][K] (K contiguous); 1: B stored [K][N] (N contiguous, bn % 64 == 0)
   int epi;           // EpilogueKind
