@@ -483,8 +483,9 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
   const bool prof = p.prof != nullptr, affine = st.gamma != nullptr;
   float* bias_s = cs.bias[0];
   __half* gamma_s = reinterpret_cast<__half*>(cs.bias[1]);          // gamma of the tile's columns, then beta
-  // Statistics that part 1 of these rows hands to part 0, in part 1's second box: its copies have left it before the tile begins, and
-  // it goes over the statistics behind the barrier that follows their reading (plain stores pass through the first box).
+  // Statistics that part 1 of these rows hands to part 0, in part 1's own second box: its copies have left it before the tile begins, and
+  // the next ones go into it once all tiles of the row have been published, which for this one part 0 does with what it has read here
+  // (plain stores pass through the first box).
   float2* other = reinterpret_cast<float2*>(boxes + ln_stats_box(q) * kStageWarp);
   StoreBoxes sb;
   sb.base = boxes + epi_box(warp) * kStageWarp;
@@ -585,7 +586,9 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
         st_relaxed_2x64(st.stats + ((size_t)(row0 >> 5) * tiles_n + nt) * 32 + lane, (uint64_t)__float_as_uint(mean) | ((uint64_t)tag << 32),
                         (uint64_t)__float_as_uint(dev) | ((uint64_t)tag << 32));
     }
-    named_barrier_sync(4 + q, 64);          // the statistics have been read: part 1 may store
+    // (one half's statistics have been read before they are published, and so before part 1 gets past its wait for them; with two halves
+    // the second one's may not have been)
+    if (nh == 2) named_barrier_sync(4 + q, 64);
 #pragma unroll 1
     for (int h = 0; h < nh; ++h) {
       const uint32_t acc = acc0 + (uint32_t)h, t0 = tmem + acc * kAccStride;
