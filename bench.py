@@ -38,8 +38,8 @@ HIDDEN = HEADS * HEAD_DIM
 #       -k regex:souffle_megakernel -s 4 -c 1 --csv python -m souffle_models_b200.profile_cases bert_base_b<n>
 # (with SOUFFLE_PAIR_COOPERATIVE=0: a launch that is clustered and cooperative cannot be captured)
 # (the library as of the commit that last changed this table; tilings chosen by the cycle model, not timed)
-DRAM_BYTES_PER_LAUNCH = {64: 412_645_632 + 565_328_384, 32: 180_741_888 + 572_626_688, 16: 173_494_528 + 15_390_464,
-                         8: 171_802_112 + 6_097_920}
+DRAM_BYTES_PER_LAUNCH = {64: 425_351_424 + 580_978_688, 32: 177_589_504 + 8_590_848, 16: 173_479_168 + 17_734_656,
+                         8: 171_945_984 + 4_058_880}
 METRIC = "bert_base_12layer_seq128_batch64_sequences_per_second"
 WORKLOAD = "BERT-base 12-layer encoder, batch 64 (sharded by sequence), seq 128, lengths U[32,128]"
 SEED = 1239
