@@ -689,8 +689,8 @@ __device__ __forceinline__ uint32_t gemm_ln_epilogue_of(const CallArgs& ca, uint
   return acc_bits;
 }
 
-// The Swin build's: sums and reordered rows.
-__device__ __noinline__ uint32_t swin_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<false, true>(ca, acc_bits); }
+// The Swin build's, with sums and reordered rows.
+__device__ __noinline__ uint32_t gemm_swin_ln(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<false, true>(ca, acc_bits); }
 template <bool kPair>
 __device__ __noinline__ uint32_t gemm_ln_epilogue(const CallArgs& ca, uint32_t acc_bits) { return gemm_ln_epilogue_of<kPair, false>(ca, acc_bits); }
 
@@ -948,7 +948,7 @@ __device__ __forceinline__ void gemm_stage(const Stage& st, const CallArgs& ca, 
     const int full_chunks = g.bn >> 5;
     if (kLnEpi && st.epi == EPI_LN) {
       const uint32_t which = (uint32_t)(&st == &ctl_s.stage[1]) << 31;
-      if constexpr (kSwin) rs.acc_bits = swin_ln_epilogue(ca, rs.acc_bits | which);
+      if constexpr (kSwin) rs.acc_bits = gemm_swin_ln(ca, rs.acc_bits | which);
       else rs.acc_bits = gemm_ln_epilogue<kPair>(ca, rs.acc_bits | which);
     } else {
     EpiCtx e;

@@ -671,6 +671,7 @@ struct SouffleBertPlan {
   CUtensorMap x_map;
   int x_box_rows = 128;
   int x_res_rows = 0;            // rows of the boxes in which the first layer's input is read as a residual, or 0
+  bool tagged = false;           // a product exchanges row statistics, whose tags come from the launch's number
   bool y_map = false;            // the last stage stores the output through a tensor map of the call's
 };
 
@@ -690,6 +691,7 @@ static int upload_program(SouffleBertPlan* p) {
   for (size_t i = 0; i < n; ++i) {
     Stage& s = p->stages[i];
     s.position = (uint8_t)i;
+    p->tagged = p->tagged || (s.type == STAGE_GEMM && s.epi == EPI_LN);
     const size_t next = next_of(i);
     s.next = (uint8_t)next;
     // the weights of the GEMM stage that comes next are prefetched into L2 while this stage runs
@@ -1329,7 +1331,7 @@ int souffle_bert_forward(SouffleBertPlan* plan, const void* x, const int32_t* se
   if ((rc = expired_word(&mp.expired))) return rc;
   mp.timeout_ns = (unsigned long long)(d.timeout_ms > 0 ? d.timeout_ms : 2000) * 1000000ull;
   mp.prof = plan->d_prof;
-  mp.epoch = plan->d_sync + kEpochWord;
+  mp.epoch = plan->tagged ? plan->d_sync + kEpochWord : nullptr;
   if (plan->x_res_rows && (rc = make_map(&args.call_maps[2], x, M, H, (uint32_t)plan->x_res_rows))) return rc;
   if (plan->y_map && (rc = make_store_map(&args.call_maps[1], y, M, H))) return rc;
   mp.skip_arrival = d.debug_skip_arrival;
@@ -1771,7 +1773,7 @@ static int launch_plan(SouffleBertPlan* plan, const void* x, void* y, const int3
   if ((rc = is_captured(st, &captured)) || (rc = pick_barrier_words(plan->d_sync, plan->launch_id, captured, st, &mp))) return rc;
   mp.status = plan->d_status;
   if ((rc = expired_word(&mp.expired))) return rc;
-  mp.epoch = plan->d_sync + kEpochWord;
+  mp.epoch = plan->tagged ? plan->d_sync + kEpochWord : nullptr;
   mp.timeout_ns = (unsigned long long)(timeout_ms > 0 ? timeout_ms : 2000) * 1000000ull;
   rc = launch_mega(args, plan->grid, st, kFamilySwin);
   if (rc) return rc;

@@ -79,7 +79,7 @@ def test_persistent_kernels_do_not_spill():
     usage = build.resource_usage()
     mega = {k: v for k, v in usage.items() if "souffle_megakernel" in k}
     lstm = {k: v for k, v in usage.items() if "souffle_lstm_wavefront" in k}
-    stages = {k: v for k, v in usage.items() if any(n in k for n in ("swin_ln_epilogue", "gemm_ln_epilogue", "ln_stage_ool", "attn_swin_stage",
+    stages = {k: v for k, v in usage.items() if any(n in k for n in ("gemm_swin_ln", "gemm_ln_epilogue", "ln_stage_ool", "attn_swin_stage",
                                                                      "ln_row_wide", "ln_gather_rows", "ln_stage_direct", "attn_store_probs", "attn_copy_probs"))}
     assert len(mega) == 4 and lstm and len(stages) == 10
     for k, (regs, st, ld) in {**mega, **lstm, **stages}.items():
@@ -95,7 +95,7 @@ def test_megakernels_have_no_stack_frame():
     """Every grid barrier's acquire empties L1, so a word on the stack costs a round trip to L2: neither the four builds nor any
     function that they call may have one, or a spill."""
     usage, frames = build.resource_usage(), build.stack_frames()
-    names = ("souffle_megakernel", "swin_ln_epilogue", "gemm_ln_epilogue", "ln_stage_ool", "ln_stage_direct", "ln_stage_many", "ln_stage_either",
+    names = ("souffle_megakernel", "gemm_swin_ln", "gemm_ln_epilogue", "ln_stage_ool", "ln_stage_direct", "ln_stage_many", "ln_stage_either",
              "drop_dead_buffers", "attn_swin_stage", "ln_row_wide", "ln_gather_rows", "attn_store_probs", "attn_copy_probs",
              "grid_wait_loop", "wait_word_loop", "mbar_wait_loop", "record_timeout")
     for n in names:
