@@ -335,8 +335,9 @@ __device__ __forceinline__ bool lstm_steps(const LstmParams& p, LstmShared<H>& s
             make_float4(__uint_as_float(got[0]), __uint_as_float(got[1]), __uint_as_float(got[2]), __uint_as_float(got[3]));
       } else {                                  // for the next layer
         const uint32_t tag = *const_cast<volatile uint32_t*>(&sh.tag);
-        uint64_t* to = p.h_all + (uint32_t)(t * H + unit0);         // (a 64-bit step index would spill at hidden 256)
-        to += (size_t)(uint32_t)(layer * T) * H;
+        uint64_t* to = p.h_all + (size_t)(uint32_t)(layer * T) * H;
+        to += (size_t)(uint32_t)t * H;
+        to += unit0;
         st_relaxed_tagged(to, got[0], got[1], tag);
         st_relaxed_tagged(to + 2, got[2], got[3], tag);
       }
@@ -535,14 +536,14 @@ __global__ void __launch_bounds__(lstm_block(H), 1) souffle_lstm_wavefront(const
   // Nobody leaves while a peer may still store into its shared memory.
   __syncthreads();
   cluster_sync_all();
-  // The steps of the cluster's CTAs, all of which have read the counter.  (At hidden 256, taking the step with the read leaves a spill in
-  // the prologue, and with one thread per CTA here the loop loses 0.7 %.)
-  if (part == 0 && tid < kLstmParts) atomicAdd(p.epoch, (unsigned long long)launch_step(blockIdx.x + tid, gridDim.x));
   if (*const_cast<volatile int*>(&sh.abort)) {   // sent by peers before they came here, and not waited for: 200 us are ample
     if (tid == 0 && p.expired) *p.expired = 1;
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 200000ull) __nanosleep(1000);
   }
+  // The steps of the cluster's CTAs, all of which have read the counter.  (At hidden 256 the register allocation hangs on this place:
+  // taken with the read, the step leaves a spill in the prologue, behind the barrier or by a thread per CTA the loop is 0.5-0.7 % slower.)
+  if (part == 0 && tid < kLstmParts) atomicAdd(p.epoch, (unsigned long long)launch_step(blockIdx.x + tid, gridDim.x));
 }
 
 }  // namespace souffle
